@@ -38,26 +38,16 @@
 // about 750 cycles each whatever their size), so each ring slot has its own issuing warp.
 // Every mbarrier wait is bounded: when a wait runs out the kernel records a status word, all
 // roles leave their loops, outstanding bulk copies are waited for (bounded) and TMEM is released.
-#include <cuda.h>
-#include <cuda_bf16.h>
-
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <vector>
 
-#include "hb_common.h"
+#include "mlp_common.cuh"
+#include "mlp_wide.h"
 
 namespace {
-
-constexpr int kWidth = 1024;            // layer_size of every Habitat predictor
-constexpr int kMTile = 128;             // output features per MMA (TMEM lanes)
-constexpr int kKBlk = 64;               // bf16 per 128-byte swizzle row
-constexpr int kNumMT = kWidth / kMTile; // 8
-constexpr int kNumKB = kWidth / kKBlk;  // 16
-constexpr int kTileBytes = kMTile * 128;// one weight tile image: 16 KB
-constexpr int kMaxInFeat = 12;          // F + 4 (conv2d: 8 + 4)
 
 struct MlpParams {
   const uint8_t* wpack;      // weight tile images, producer order
@@ -82,143 +72,6 @@ struct MlpParams {
   uint64_t unit_order;       // pair kernel: the 16 (block, K quarter) units of a hidden layer, 4 bits each
   uint32_t unit_gates;       // pair kernel: 4 bits per block j: the block whose completion frees K quarter j
 };
-
-// ---------------------------------------------------------------------------
-// PTX wrappers
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void fence_proxy_async() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t elect_one() {
-  uint32_t pred;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "elect.sync _|p, 0xffffffff;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(pred)::"memory");
-  return pred;
-}
-__device__ __forceinline__ void tc_wait_ld() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-// 32 lanes x 32 consecutive 32-bit columns: thread t of the warp gets lane
-// (quadrant base + t), registers = columns.
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-  tc_wait_ld();
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// 32 lanes x 16 consecutive 32-bit columns.
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// 32 lanes x 64 consecutive 32-bit columns in one instruction: halves the number of
-// load round trips of the epilogue (each tcgen05.ld + wait costs several hundred cycles).
-__device__ __forceinline__ void tc_ld64(uint32_t taddr, float (&v)[64]) {
-  uint32_t r[64];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x64.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, "
-      "%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
-      "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]),
-        "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]),
-        "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]),
-        "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]),
-        "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]),
-        "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]),
-        "=r"(r[62]), "=r"(r[63])
-      : "r"(taddr)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// Byte offset of element (row, col) inside a K-major 128-byte-swizzled block of
-// 128-byte rows: 16-byte chunks are permuted by the row index modulo 8.
-__host__ __device__ __forceinline__ uint32_t swz_off(uint32_t row, uint32_t col) {
-  return row * 128u + ((((col >> 3) ^ row) & 7u) << 4) + ((col & 7u) << 1);
-}
-
-constexpr long long kWaitCycles = 4000000000LL;  // about two seconds
-
-// Bounded wait.  Returns false when the wait ran out or another role gave up.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          int32_t* status, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  for (uint32_t i = 1;; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 63u) == 0u) {
-      if (*abort_flag) return false;
-      if (clock64() - t0 > kWaitCycles) {
-        *abort_flag = 1;
-        atomicCAS(status, 0, code);
-        return false;
-      }
-    }
-  }
-}
 
 // ---------------------------------------------------------------------------
 // The kernel.  A single CTA can only keep 64 queries on chip,
@@ -278,105 +131,6 @@ static_assert(kPairSmemBytes <= 232448, "over the 227 KB shared-memory limit");
 __device__ __forceinline__ void pair_epi_bar_sync() {
   asm volatile("bar.sync 1, 256;" ::: "memory");
 }
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
-                                                  volatile int* abort_flag, int32_t* status,
-                                                  int code) {
-  if (mbar_try_wait_cluster(bar, parity)) return true;
-  const long long t0 = clock64();
-  for (uint32_t i = 1;; ++i) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    if ((i & 63u) == 0u) {
-      if (*abort_flag) return false;
-      if (clock64() - t0 > kWaitCycles) {
-        *abort_flag = 1;
-        atomicCAS(status, 0, code);
-        return false;
-      }
-    }
-  }
-}
-// Asynchronous 16-byte store into a peer CTA's shared memory; completion is counted
-// in bytes on an mbarrier of that CTA.  Unlike st.shared::cluster the issuing
-// thread does not wait for the store to be acknowledged.
-__device__ __forceinline__ void st_async_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c,
-                                            uint32_t d, uint32_t cluster_mbar) {
-  asm volatile(
-      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
-      ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(cluster_mbar)
-      : "memory");
-}
-// Byte offset of element (K row k, query n) of an MN-major, 128-byte-swizzled B
-// operand holding 64 queries per row: rows are 128 B apart, the eight 16-byte
-// groups of a row are permuted by the row index modulo 8.
-__device__ __forceinline__ uint32_t mn_off(uint32_t k, uint32_t n) {
-  return k * 128u + ((((n >> 3) ^ k) & 7u) << 4) + ((n & 7u) << 1);
-}
-__device__ __forceinline__ void st_cluster_f32(uint32_t cluster_addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
-                   : "memory");
-}
-__device__ __forceinline__ unsigned long long global_timer_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-// Tiled TMA load of a box of 128-byte rows into this CTA's shared memory.  With
-// .cta_group::2 the completion may be counted on a barrier of the other CTA of the pair
-// (given as a shared::cluster address): both CTAs' weight copies report to the leader's
-// barrier directly.  No multicast: each CTA fetches its own half of the weights.
-__device__ __forceinline__ void tma_rows_2sm(uint32_t dst, const CUtensorMap* map, int32_t row,
-                                             uint32_t cluster_mbar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(cluster_mbar), "r"(0), "r"(row)
-      : "memory");
-}
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
-      "[%0], %1;" ::"r"(bar),
-      "h"(static_cast<uint16_t>(3))
-      : "memory");
-}
-__device__ __forceinline__ void tc_mma_pair_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                                 uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 // SPLIT = false: bf16 operands, 128 queries per cluster tile (64 per CTA).
 // SPLIT = true (the 1e-4 mode): activations and weights are kept as bf16 hi + lo parts.  A CTA
 // holds 32 queries and lays the hi and lo parts of an activation side by side along N (the 128-byte
@@ -615,7 +369,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
     const uint32_t act_peer = map_to_cta(act, peer);
     uint32_t in_phase = 0, lay = 0, tile_no = 0;
     bool ok = true;
-    float* red = reinterpret_cast<float*>(base_ptr);   // [256][33], aliases activations
+    float* red = reinterpret_cast<float*>(base_ptr);   // [8 warps][queries of the tile], aliases activations
     const bool timed = p.phase_cycles != nullptr && blockIdx.x == 0 && T == 0;
     long long c_wait = 0, c_epi = 0, c_fc2 = 0, c_layers = 0, c_ld = 0, c_bias = 0, c_sync = 0, c_loc = 0, c_rem = 0;
     // named barrier of this group alone (ids 2 and 3; id 1 joins both groups)
@@ -758,57 +512,50 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
           tc_fence_after();
           const long long c1 = timed ? clock64() : 0;
           // fc2 over this CTA's 512 features, 32 queries at a time (bf16: the four column quarters
-          // of the 128 queries; split: the two CTAs' 32 queries, hi and lo columns added first)
+          // of the 128 queries; split: the two CTAs' 32 queries, hi and lo columns added first).
+          // A warp multiplies its 32 features of a block and adds them over its lanes with the
+          // transposing tree (31 shuffles leave one query per lane); the eight warps' sums of a query
+          // meet in shared memory once, after all columns.
+          constexpr int kChunks = SPLIT ? 2 : 4;
 #pragma unroll 1
-          for (int qd = 0; qd < (SPLIT ? 2 : 4); ++qd) {
-            float acc[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
+          for (int qd = 0; qd < kChunks; ++qd) {
+            float part = 0.0f;
 #pragma unroll 1
             for (int jj = 0; jj < 2; ++jj) {
               const int j = grp * 2 + jj;
               const int f = j * 256 + static_cast<int>(rank) * 128 + r;
               const float b = __ldg(bias + f);
               const float w = __ldg(p.fc2_w + f);
+              float v[32];
               if (SPLIT) {
+                float lo[32];
+                tc_ld32(t_lane + static_cast<uint32_t>(j * kPairQ + qd * 64), v);
+                tc_ld32(t_lane + static_cast<uint32_t>(j * kPairQ + qd * 64 + 32), lo);
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                  float vh[16], vl[16];
-                  tc_ld16(t_lane + static_cast<uint32_t>(j * kPairQ + qd * 64 + h * 16), vh);
-                  tc_ld16(t_lane + static_cast<uint32_t>(j * kPairQ + qd * 64 + 32 + h * 16), vl);
-#pragma unroll
-                  for (int i = 0; i < 16; ++i)
-                    acc[h * 16 + i] = fmaf(w, fmaxf((vh[i] + vl[i]) + b, 0.0f), acc[h * 16 + i]);
-                }
+                for (int i = 0; i < 32; ++i) v[i] += lo[i];
               } else {
-                float v[32];
                 tc_ld32(t_lane + static_cast<uint32_t>(j * kPairQ + qd * 32), v);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) acc[i] = fmaf(w, fmaxf(v[i] + b, 0.0f), acc[i]);
               }
-            }
-            const int row = grp * 128 + r;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) red[row * 33 + i] = acc[i];
-            pair_epi_bar_sync();
-            const int n = T & 31, part = T >> 5;       // 8 parts of 32 feature rows each
-            float sum = 0.0f;
-            for (int k2 = 0; k2 < 32; ++k2) sum += red[(part * 32 + k2) * 33 + n];
-            pair_epi_bar_sync();
-            red[part * 32 + n] = sum;
-            pair_epi_bar_sync();
-            if (T < 32) {
-              float tot = 0.0f;
-#pragma unroll
-              for (int k2 = 0; k2 < 8; ++k2) tot += red[k2 * 32 + T];
-              // index among the owner's queries, and which CTA owns them
-              const int slot = SPLIT ? T : (qd & 1) * 32 + T;
-              const uint32_t owner = static_cast<uint32_t>(SPLIT ? qd : qd >> 1);
-              if (owner == rank) fc2_mine[slot] = tot;
-              else st_cluster_f32(map_to_cta(smem_u32(fc2_peer + slot), peer), tot);
+              for (int i = 0; i < 32; ++i) v[i] = __fmul_rn(w, fmaxf(v[i] + b, 0.0f));
+              fold16(v, lane);
+              fold_lanes<2>(v, lane, 16);
+              part += v[0];
             }
-            pair_epi_bar_sync();
+            red[(grp * 4 + quad) * (kChunks * 32) + qd * 32 + fold16_col<32>(lane) + (lane >> 4)] = part;
           }
+          pair_epi_bar_sync();
+          if (T < kChunks * 32) {
+            float tot = 0.0f;
+#pragma unroll
+            for (int k2 = 0; k2 < 8; ++k2) tot += red[k2 * (kChunks * 32) + T];
+            // which CTA owns the query, and its index among the owner's
+            const uint32_t owner = static_cast<uint32_t>(T / kHalfQ);
+            const int slot = T % kHalfQ;
+            if (owner == rank) fc2_mine[slot] = tot;
+            else st_cluster_f32(map_to_cta(smem_u32(fc2_peer + slot), peer), tot);
+          }
+          pair_epi_bar_sync();
           tc_fence_before();
           // hand-over of the partial sums, then the owner finishes its 64 queries
           if (T == 0) {
@@ -877,22 +624,9 @@ void put(uint8_t* tile, int row, int col, uint16_t v) {
 
 }  // namespace
 
-struct hb_mlp {
-  int32_t n_op_feat = 0, layers = 0, precision = 0, n_dev = 0, sm_count = 0, device = 0;
-  float fc2_b = 0.f;
-  uint8_t* wpack = nullptr;
-  CUtensorMap tmap_slot{}, tmap_tile{};
-  float* bias = nullptr;
-  float* fc2_w = nullptr;
-  double* mu = nullptr;
-  double* sigma = nullptr;
-  double* dev_feat = nullptr;
-  int32_t* status = nullptr;
-  long long* phase_cycles = nullptr;
-};
-
 extern "C" void hb_mlp_destroy(hb_mlp* h) {
   if (!h) return;
+  if (h->counted) hb::wide_handle_destroyed(h->device);
   cudaFree(h->wpack); cudaFree(h->bias); cudaFree(h->fc2_w); cudaFree(h->mu);
   cudaFree(h->sigma); cudaFree(h->dev_feat); cudaFree(h->status); cudaFree(h->phase_cycles);
   delete h;
@@ -1036,6 +770,22 @@ extern "C" hb_status hb_mlp_create(hb_mlp** handle, int32_t n_op_features, int32
         return HB_ERR_CUDA;
       }
     }
+    // the same rows by tile image, for blocks that take half of an image's rows (mlp_wide.cu)
+    const cuuint64_t dims3[3] = {128, 128, static_cast<cuuint64_t>(pack.size() / kTileBytes)};
+    const cuuint64_t strides3[2] = {128, kTileBytes};
+    const cuuint32_t elem3[3] = {1, 1, 1};
+    for (int which = 0; which < 2; ++which) {
+      const cuuint32_t box3[3] = {128, 64, which == 0 ? 4u : 1u};
+      const CUresult r = reinterpret_cast<EncodeFn>(fn)(
+          which == 0 ? &h->tmap_wide_slot : &h->tmap_wide_fc1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, h->wpack, dims3,
+          strides3, box3, elem3, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      if (r != CUDA_SUCCESS) {
+        hb::set_error("hb_mlp_create: cuTensorMapEncodeTiled failed (CUresult %d)", static_cast<int>(r));
+        hb_mlp_destroy(h);
+        return HB_ERR_CUDA;
+      }
+    }
   }
   if ((e = cudaMalloc(reinterpret_cast<void**>(&h->status), sizeof(int32_t))) != cudaSuccess)
     return fail(e, "cudaMalloc status");
@@ -1049,6 +799,8 @@ extern "C" hb_status hb_mlp_create(hb_mlp** handle, int32_t n_op_features, int32
   e = cudaFuncSetAttribute(mlp_chain_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            kPairSmemBytes);
   if (e != cudaSuccess) return fail(e, "cudaFuncSetAttribute");
+  hb::wide_handle_created(h->device);
+  h->counted = true;
   *handle = h;
   return HB_OK;
 }
@@ -1068,6 +820,14 @@ extern "C" hb_status hb_mlp_predict(hb_mlp* h, const float* op_features, const u
     return HB_ERR_INVALID_ARGUMENT;
   }
   const bool split = h->precision == HB_PRECISION_BF16X3;
+  // HB_MLP_WIDE=0 keeps every batch on the two-SM kernel
+  static const bool use_wide = [] { const char* e = std::getenv("HB_MLP_WIDE"); return !e || std::atoi(e) != 0; }();
+  if (use_wide) {
+    bool launched = false;
+    const hb_status st = hb::wide_predict(h, hb::wide_plan(Q, split, h->sm_count), op_features, device_row, Q, out,
+                                          static_cast<cudaStream_t>(stream), &launched);
+    if (st != HB_OK || launched) return st;
+  }
   const int tile_q = split ? kPairQ / 2 : kPairQ;
   const int64_t tiles = (Q + tile_q - 1) / tile_q;
   if (tiles > 0x7FFFFFFF) {
@@ -1103,6 +863,7 @@ extern "C" hb_status hb_mlp_status(hb_mlp* h, int32_t* device_status) {
   if (*device_status != 0) {
     // reported once: the word is cleared so that later launches are judged on their own
     HB_CUDA_TRY(cudaMemset(h->status, 0, sizeof(int32_t)));
+    hb::wide_start_over(h->device);
     hb::set_error("mlp kernel: a bounded device-side wait ran out (site 0x%x)", *device_status);
     return HB_ERR_DEVICE_TIMEOUT;
   }

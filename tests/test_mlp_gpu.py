@@ -238,3 +238,65 @@ def test_bf16_mode_against_its_own_arithmetic(op, gain, layers, bound):
     print("%s gain %.2f, %d layers: device vs bf16 replay %.3g of the output scale; replay vs float64 %.3g"
           % (op, gain, layers, diff, np.abs(replay - ref64).max() / scale))
     assert diff <= bound
+
+
+@pytest.mark.parametrize("precision", ["bf16", "bf16x3"])
+def test_small_batches(precision):
+    """Batches below 2,112 (split: 1,056) queries run on groups of 16, 8 or 4 blocks that exchange their
+    activations; the shapes change at 112, 240, 480, 960, 1,056 (split: 56, 120, 240, 528).  Sizes on both
+    sides of every change: each prediction equals, to the last bit, the one the same query gets inside a
+    batch that runs on the two-SM kernel, and that batch is within the mode's tolerance of the oracle
+    (bf16 on variance-preserving weights: 2e-2 of the output scale, as in the input-sensitive test)."""
+    w = workloads.init_mlp_weights("conv2d", seed=9, gain=2.0)
+    feats, dev = workloads.make_queries("conv2d", 6000, 41)
+    mu, sigma = workloads.batch_mu_sigma(feats, dev)
+    h = batched.MLPHandle(feats.shape[1], mu=mu, sigma=sigma, device_features=DEVF, precision=precision, **w)
+    f, r = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()
+    full = h.predict(f, r)
+    ref = omlp.predict(w, feats, dev, DEVF, mu, sigma, np.float64)
+    err = np.abs(full.cpu().numpy() - ref).max() / np.abs(ref).max()
+    assert err <= (2e-2 if precision == "bf16" else 1e-4), err
+    edges = [112, 240, 480, 960, 1056, 2112] if precision == "bf16" else [56, 120, 240, 528, 1056]
+    for Q in [1, 2, 15, 16, 17, 33] + [e + d for e in edges for d in (0, 1)]:
+        lo = 6000 - Q if Q % 2 else 7
+        for _ in range(2):
+            got = h.predict(f[lo:lo + Q].contiguous(), r[lo:lo + Q].contiguous())
+            assert torch.equal(got, full[lo:lo + Q]), Q
+    h.check_status()
+    h.close()
+
+
+def test_small_batches_on_streams_and_in_a_graph():
+    """Small batches keep scratch per stream: interleaved launches of two predictors on more streams than
+    there is scratch for, a captured launch, and a launch after an error status all give the same bits."""
+    from habitat_b200 import _native
+    feats, dev = workloads.make_queries("linear", 500, 43)
+    mu, sigma = workloads.batch_mu_sigma(feats, dev)
+    f, r = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()
+    hs = [batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=DEVF, **workloads.init_mlp_weights(
+        "linear", seed=s, layers=layers, gain=2.0)) for s, layers in ((1, 8), (2, 3))]
+    want = [h.predict(f, r).clone() for h in hs]
+    torch.cuda.synchronize()
+    outs = []
+    streams = [torch.cuda.Stream() for _ in range(20)]
+    for i in range(60):
+        with torch.cuda.stream(streams[i % 20]):
+            outs.append((i % 2, hs[i % 2].predict(f, r)))
+    torch.cuda.synchronize()
+    for k, out in outs:
+        assert torch.equal(out, want[k])
+    g = torch.cuda.CUDAGraph()
+    out = torch.empty_like(want[0])
+    with torch.cuda.graph(g):
+        hs[0].predict(f, r, out=out)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want[0])
+    hs[0].inject_status(0x532)
+    with pytest.raises(_native.HabitatNativeError):
+        hs[0].check_status()
+    for k in (0, 1):
+        assert torch.equal(hs[k].predict(f, r), want[k])
+    for h in hs:
+        h.check_status()
+        h.close()
