@@ -69,8 +69,6 @@ struct MlpParams {
   long long* phase_cycles;   // [16] cluster 0: cycle counters of the roles (diagnostic), or null
   CUtensorMap tmap_slot;     // pair kernel: the pack as [rows][128 B], box of two tile images (32 KB)
   CUtensorMap tmap_tile;     // same tensor, box of one tile image (16 KB, fc1)
-  uint64_t unit_order;       // pair kernel: the 16 (block, K quarter) units of a hidden layer, 4 bits each
-  uint32_t unit_gates;       // pair kernel: 4 bits per block j: the block whose completion frees K quarter j
 };
 
 // ---------------------------------------------------------------------------
@@ -121,7 +119,6 @@ constexpr int kPairActBytes = kNumKB * kPairActKb;    // 128 KB
 // tensor core works on the remaining blocks; the next layer consumes the quarters in the
 // same order.
 constexpr uint64_t kPairOrder = 0xFBEA76D95321C840ull;
-constexpr uint32_t kPairGates = 0x3210u;
 __device__ __forceinline__ int pair_unit_j(uint64_t order, int u) { return static_cast<int>((order >> (4 * u + 2)) & 3u); }
 __device__ __forceinline__ int pair_unit_q(uint64_t order, int u) { return static_cast<int>((order >> (4 * u)) & 3u); }
 constexpr int kPairThreads = 512;              // warps: 0 alloc, 1 MMA, 2-5 + 12-15 epilogue, 6-11 producers
@@ -233,8 +230,8 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
           const uint32_t load_bytes = nkb == 1 ? kTileBytes : kPairStageBytes;
           {
             for (int u = 0; u < n_units && ok; ++u) {
-              const int j = nkb == 1 ? u : pair_unit_j(p.unit_order, u);
-              const int kq = nkb == 1 ? 0 : pair_unit_q(p.unit_order, u);
+              const int j = nkb == 1 ? u : pair_unit_j(kPairOrder, u);
+              const int kq = nkb == 1 ? 0 : pair_unit_q(kPairOrder, u);
               const size_t blk = layer_base + static_cast<size_t>(2 * j + rank) * nkb + kq * 4;
               for (int g = 0; g < n_loads; ++g, ++it) {
                 if (it % kPairStages != w) continue;
@@ -265,10 +262,10 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
   } else if (warp == 1) {
     if (rank == 0) {
       // ------------------------------ MMA issuer (leader) -------------------
-      // The whole warp walks the loop and one elected lane issues: the operands of
-      // tcgen05.mma live in uniform registers, and a loop that only one lane of a
-      // diverged warp executes was measured at 645 cycles per eight MMAs against
-      // 512 (the tensor pipe's own rate) for the warp-uniform form.
+      // One elected lane (elect.sync) runs the whole loop, and no loop depends on what a wait returns
+      // (after a wait that ran out the abort flag is set, and what is issued on stale operands is
+      // discarded), which keeps the descriptors in uniform registers: eight MMAs and their commit are
+      // queued in 150 cycles of the 512 they take.  The barrier of the next slot is tested while they run.
       // D fp32, A/B bf16, A K-major, B MN-major (bit 16), N = 128, M = 256
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
                                  (static_cast<uint32_t>(kPairQ >> 3) << 17) |
@@ -277,82 +274,96 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
                                (static_cast<uint64_t>(2) << 61) | (static_cast<uint64_t>(1) << 16);
       const uint32_t a_lo0 = (stage0 & 0x3FFFF) >> 4;
       const uint32_t b_lo0 = (act & 0x3FFFF) >> 4;
-      // par: bits 0-3 = parity of the next wait on bar_actq[q], bits 4-7 on bar_tfree[j]
-      uint32_t s = 0, ph = 0, par = 0;
-      bool ok = true;
-      const bool mtimed = p.phase_cycles != nullptr && blockIdx.x == 0;
-      long long mc_act = 0, mc_full = 0, mc_tfree = 0, mc_issue = 0, mc_n = 0;
-      auto wait_flip = [&](uint32_t bar0, uint32_t idx, uint32_t bit, long long& acc, int code) -> bool {
-        const long long m0 = mtimed ? clock64() : 0;
-        const bool got = mbar_wait_cluster(bar0 + 8 * idx, (par >> bit) & 1u, abort_flag, p.status, code);
-        par ^= 1u << bit;
-        tc_fence_after();
-        if (mtimed) acc += clock64() - m0;
-        return got;
-      };
-      const long long k0 = clock64();
-      const unsigned long long g0 = global_timer_ns();
-      for (int t = 0; t < my_tiles && ok; ++t) {
-        for (int L = 0; L < n_layers && ok; ++L) {
-          const int nkb = L == 0 ? 1 : kNumKB;
-          const int n_units = nkb == 1 ? kPairMT : 16;
-          const int n_loads = nkb == 1 ? 1 : kLoadsPerUnit;
+      if (elect_one()) {
+        // par: bits 0-3 = parity of the next wait on bar_actq[q], bits 4-7 on bar_tfree[j]
+        uint32_t s = 0, ph = 0, par = 0;
+        const bool mtimed = p.phase_cycles != nullptr && blockIdx.x == 0;
+        long long mc_act = 0, mc_full = 0, mc_tfree = 0, mc_n = 0;
+        auto wait = [&](uint32_t bar, uint32_t parity, long long& acc, int code) {
+          const long long m0 = mtimed ? clock64() : 0;
+          mbar_wait_cluster(bar, parity, abort_flag, p.status, code);
+          tc_fence_after();
+          if (mtimed) acc += clock64() - m0;
+        };
+        const long long k0 = clock64();
+        const unsigned long long g0 = global_timer_ns();
+#pragma unroll 1
+        for (int t = 0; t < my_tiles; ++t) {
           // fc1 reads K block 0, written after the previous tile's TMEM was read out
-          if (nkb == 1 && !wait_flip(bar_actq, 0, 0, mc_act, 0x211)) { ok = false; break; }
-          uint32_t seen = 0;   // bits 0-3: K quarters used, bits 4-7: blocks written, bits 8-15: units done per block
-          for (int u = 0; u < n_units && ok; ++u) {
-            const int j = nkb == 1 ? u : pair_unit_j(p.unit_order, u);
-            const int kq = nkb == 1 ? 0 : pair_unit_q(p.unit_order, u);
-            const bool first_of_block = ((seen >> (4 + j)) & 1u) == 0u;
-            if (nkb > 1) {
-              // first write into TMEM block j of this layer: the previous layer's values must be out
-              if (first_of_block && !wait_flip(bar_tfree, j, 4 + j, mc_tfree, 0x213)) { ok = false; break; }
-              // first use of K quarter kq
-              if (((seen >> kq) & 1u) == 0u && !wait_flip(bar_actq, kq, kq, mc_act, 0x211)) { ok = false; break; }
-            }
-            seen |= (1u << kq) | (16u << j);
-            // two-bit count of the block's earlier units; the fourth unit completes the block
-            const bool last_of_block = nkb == 1 || ((seen >> (8 + 2 * j)) & 3u) == 3u;
-            if (!last_of_block) seen += 1u << (8 + 2 * j);
+          wait(bar_actq, par & 1u, mc_act, 0x211);
+          par ^= 1u;
+#pragma unroll 1
+          for (int j = 0; j < kPairMT; ++j) {
+            wait(bar_full + 8 * s, ph, mc_full, 0x212);
             const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(j * kPairQ);
-            for (int g = 0; g < n_loads; ++g) {
-              const long long m1 = mtimed ? clock64() : 0;
-              if (!mbar_wait_cluster(bar_full + 8 * s, ph, abort_flag, p.status, 0x212)) { ok = false; break; }
-              const long long m2 = mtimed ? clock64() : 0;
-              const uint64_t a0 = desc_hi | (a_lo0 + s * (kPairStageBytes >> 4));
-              const uint64_t b0 = desc_hi | (b_lo0 + static_cast<uint32_t>(kq * 4 + (SPLIT ? 1 : kPairSlotKb) * g) *
-                                                         (kPairActKb >> 4));
-              if (elect_one()) {
-                // a K step of 16: 32 bytes along an A row, 16 K rows (2 KB) of B
-                tc_mma_pair_bf16(d_tmem, a0, b0, idesc, (first_of_block && g == 0) ? 0u : 1u);
-                tc_mma_pair_bf16(d_tmem, a0 + 2, b0 + 128, idesc, 1u);
-                tc_mma_pair_bf16(d_tmem, a0 + 4, b0 + 256, idesc, 1u);
-                tc_mma_pair_bf16(d_tmem, a0 + 6, b0 + 384, idesc, 1u);
-                if (kPairSlotKb == 2 && nkb > 1) {
-                  // second image of the slot (16 KB on): bf16: the next K block, i.e. the next 64 K rows
-                  // of the activations (8 KB on); split: the lo part of the same K block, same activations
-                  const uint64_t a1 = a0 + (kTileBytes >> 4), b1 = SPLIT ? b0 : b0 + (kPairActKb >> 4);
-                  tc_mma_pair_bf16(d_tmem, a1, b1, idesc, 1u);
-                  tc_mma_pair_bf16(d_tmem, a1 + 2, b1 + 128, idesc, 1u);
-                  tc_mma_pair_bf16(d_tmem, a1 + 4, b1 + 256, idesc, 1u);
-                  tc_mma_pair_bf16(d_tmem, a1 + 6, b1 + 384, idesc, 1u);
+            const uint32_t a_lo = a_lo0 + s * (kPairStageBytes >> 4);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              tc_mma_pair_bf16(d_tmem, desc_hi | (a_lo + 2 * k), desc_hi | (b_lo0 + 128 * k), idesc, k ? 1u : 0u);
+            tc_commit_pair(bar_accj + 8 * j);
+            tc_commit_pair(bar_empty + 8 * s);
+            ring_next<kPairStages>(s, ph);
+          }
+#pragma unroll 1
+          for (int L = 1; L < n_layers; ++L) {
+            bool landed = false;            // the barrier of slot s has been seen complete
+#pragma unroll 1
+            for (uint32_t u = 0; u < 16; ++u) {
+              const uint32_t unit = ((u < 8 ? static_cast<uint32_t>(kPairOrder) : static_cast<uint32_t>(kPairOrder >> 32)) >>
+                                     (4 * (u & 7u))) & 15u;
+              const uint32_t j = unit >> 2, kq = unit & 3u;
+              if (u < 7) {
+                // units 0-3 write a TMEM block for the first time (the previous layer's values must be out);
+                // units 0, 4, 5, 6 are the first to read their K quarter
+                if (u < 4) {
+                  wait(bar_tfree + 8 * j, (par >> (4 + j)) & 1u, mc_tfree, 0x213);
+                  par ^= 16u << j;
+                }
+                if (u == 0 || u >= 4) {
+                  wait(bar_actq + 8 * kq, (par >> kq) & 1u, mc_act, 0x211);
+                  par ^= 1u << kq;
+                }
+              }
+              const uint32_t d_tmem = tmem_base + j * kPairQ;
+#pragma unroll
+              for (uint32_t g = 0; g < kLoadsPerUnit; ++g) {
+                uint32_t next = s, next_ph = ph;
+                ring_next<kPairStages>(next, next_ph);
+                const uint32_t a_lo = a_lo0 + s * (kPairStageBytes >> 4);
+                const uint32_t b_lo = b_lo0 + (kq * 4 + (SPLIT ? 1 : kPairSlotKb) * g) * (kPairActKb >> 4);
+                if (!landed) wait(bar_full + 8 * s, ph, mc_full, 0x212);
+#pragma unroll
+                for (int k = 0; k < 4 * kPairSlotKb; ++k) {
+                  // a K step of 16: 32 bytes along an A row, 16 K rows (2 KB) of B.  Second image of the slot
+                  // (16 KB on): bf16: the next K block, i.e. the next 64 K rows of the activations (8 KB on);
+                  // split: the lo part of the same K block, same activations
+                  tc_mma_pair_bf16(d_tmem, desc_hi | (a_lo + (k >> 2) * (kTileBytes >> 4) + 2 * (k & 3)),
+                                   desc_hi | (b_lo + (SPLIT ? 0 : (k >> 2) * (kPairActKb >> 4)) + 128 * (k & 3)), idesc,
+                                   (g == 0 && k == 0) ? u >> 2 : 1u);
+                  if (k == 4) {
+                    landed = mbar_try_wait_cluster(bar_full + 8 * next, next_ph);
+                    tc_fence_after();
+                  }
                 }
                 tc_commit_pair(bar_empty + 8 * s);
-                if (last_of_block && g == n_loads - 1) tc_commit_pair(bar_accj + 8 * j);
+                s = next;
+                ph = next_ph;
               }
-              __syncwarp();
-              if (mtimed) { mc_full += m2 - m1; mc_issue += clock64() - m2; ++mc_n; }
-              if (++s == kPairStages) { s = 0; ph ^= 1u; }
+              // the last units of blocks 0..3 (kPairOrder)
+              if ((0xC840u >> u) & 1u) tc_commit_pair(bar_accj + 8 * j);
             }
+            mc_n += 16 * kLoadsPerUnit;
           }
         }
+        if (mtimed) {
+          p.phase_cycles[4] = mc_act; p.phase_cycles[5] = mc_full; p.phase_cycles[6] = mc_tfree;
+          p.phase_cycles[8] = mc_n;
+          p.phase_cycles[12] = clock64() - k0;
+          p.phase_cycles[7] = p.phase_cycles[12] - mc_act - mc_full - mc_tfree;
+          p.phase_cycles[13] = static_cast<long long>(global_timer_ns() - g0);
+        }
       }
-      if (mtimed && lane == 0) {
-        p.phase_cycles[4] = mc_act; p.phase_cycles[5] = mc_full; p.phase_cycles[6] = mc_tfree;
-        p.phase_cycles[7] = mc_issue; p.phase_cycles[8] = mc_n;
-        p.phase_cycles[12] = clock64() - k0;
-        p.phase_cycles[13] = static_cast<long long>(global_timer_ns() - g0);
-      }
+      __syncwarp();
     }
   } else if (warp >= 2) {
     // ------------------------------ epilogue ------------------------------
@@ -426,7 +437,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
 #pragma unroll 1
           for (int jj = 0; jj < 2; ++jj) {
             const int j = grp + 2 * jj;
-            const int gate = L == 0 ? 3 : static_cast<int>((p.unit_gates >> (4 * j)) & 3u);
+            const int gate = L == 0 ? 3 : j;
             const long long c0 = timed ? clock64() : 0;
             if (e == 0) {
               epi_ok[grp] = mbar_wait(bar_accj + 8 * gate, lay & 1u, abort_flag, p.status, 0x311) ? 1 : 0;
@@ -477,17 +488,28 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
 #pragma unroll
                 for (int i = 0; i < 64; ++i) v[i] = fmaxf(v[i] + b, 0.0f);
               }
+              uint32_t w[32];
 #pragma unroll
-              for (int g = 0; g < 8; ++g) {          // eight values per 16-byte store
-                uint32_t w4[4];
+              for (int i = 0; i < 32; ++i) {
+                const __nv_bfloat162 pk = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                w[i] = *reinterpret_cast<const uint32_t*>(&pk);
+              }
+              if (mine) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                  const __nv_bfloat162 pk = __floats2bfloat162_rn(v[g * 8 + 2 * u], v[g * 8 + 2 * u + 1]);
-                  w4[u] = *reinterpret_cast<const uint32_t*>(&pk);
-                }
-                const uint32_t off = row_off + ((static_cast<uint32_t>(g) ^ sw) << 4);
-                if (mine) *reinterpret_cast<uint4*>(base_ptr + off) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-                else st_async_v4(act_peer + off, w4[0], w4[1], w4[2], w4[3], bar_in_peer);
+                for (uint32_t g = 0; g < 8; ++g)             // eight values per 16-byte store
+                  *reinterpret_cast<uint4*>(base_ptr + row_off + ((g ^ sw) << 4)) =
+                      make_uint4(w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
+              } else {
+                // Into the peer go whole 128-byte rows: eight lanes trade chunks so that each store of theirs
+                // fills one row.  Chunks of 32 different rows per store arrived one by one and held the
+                // peer's shared memory long enough to stall its tensor core (831 -> 740 cycles per slot).
+                trade_chunks<8>(w, lane);
+                const uint32_t c8 = static_cast<uint32_t>(lane) & 7u;
+                const uint32_t row8 = act_peer + (row_off - c8 * 128u);
+#pragma unroll
+                for (uint32_t g = 0; g < 8; ++g)
+                  st_async_v4(row8 + g * 128u + ((c8 ^ g) << 4), w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3],
+                              bar_in_peer);
               }
               if (timed) { if (mine) c_loc += clock64() - d1; else c_rem += clock64() - d1; }
             }
@@ -842,8 +864,6 @@ extern "C" hb_status hb_mlp_predict(hb_mlp* h, const float* op_features, const u
   p.status = h->status;
   p.phase_cycles = h->phase_cycles;
   p.tmap_slot = h->tmap_slot; p.tmap_tile = h->tmap_tile;
-  p.unit_order = kPairOrder;
-  p.unit_gates = kPairGates;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // one cluster of two CTAs per tile (128 queries, 64 in split precision), at most one cluster per SM pair
   const int pairs = static_cast<int>(tiles < h->sm_count / 2 ? tiles : h->sm_count / 2);

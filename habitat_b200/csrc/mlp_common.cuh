@@ -78,6 +78,27 @@ __device__ __forceinline__ void ring_next(uint32_t& s, uint32_t& phase) {
   phase ^= (1u >> s) & 1u;   // back at slot 0
 }
 
+// Transposes N x N chunks of four words over each N neighbouring lanes: lane l of them gives chunk j to lane j.
+template <int N>
+__device__ __forceinline__ void trade_chunks(uint32_t (&w)[4 * N], int lane) {
+#pragma unroll
+  for (int m = 1; m < N; m *= 2) {
+    const bool upper = (lane & m) != 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      if (j & m) continue;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        uint32_t& lo = w[4 * j + i];
+        uint32_t& hi = w[4 * (j + m) + i];
+        const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, upper ? lo : hi, m);
+        if (upper) lo = got;
+        else hi = got;
+      }
+    }
+  }
+}
+
 // One fold of the transposing reduction below: N values per lane and a lane mask become N / 2
 // values, the sums over the pair of lanes that differ in `mask`; lanes with the bit keep the upper half.
 template <int N, int W>

@@ -150,26 +150,6 @@ __device__ __forceinline__ void tc_ld_cols(uint32_t taddr, float (&v)[W]) {
   else if constexpr (W == 16) tc_ld16(taddr, v);
   else tc_ld32(taddr, v);
 }
-// Transposes N x N chunks of four words over each N neighbouring lanes: lane l of them gives chunk j to lane j.
-template <int N>
-__device__ __forceinline__ void trade_chunks(uint32_t (&w)[4 * N], int lane) {
-#pragma unroll
-  for (int m = 1; m < N; m *= 2) {
-    const bool upper = (lane & m) != 0;
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-      if (j & m) continue;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        uint32_t& lo = w[4 * j + i];
-        uint32_t& hi = w[4 * (j + m) + i];
-        const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, upper ? lo : hi, m);
-        if (upper) lo = got;
-        else hi = got;
-      }
-    }
-  }
-}
 // Byte offset of 16-byte chunk `chunk` of K row k in a B operand of W columns (swizzle width 2 W bytes).
 template <int W>
 __device__ __forceinline__ uint32_t b_chunk(uint32_t k, uint32_t chunk) {
