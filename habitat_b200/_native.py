@@ -153,6 +153,34 @@ def load():
     return lib
 
 
+_binding = None
+
+
+def binding():
+    """The CPython binding of the tensor-level entry points (once), bound to the loaded library."""
+    global _binding
+    if _binding is not None:
+        return _binding
+    import importlib.machinery
+    import importlib.util
+    path = os.path.join(_PKG_DIR, "_lib", "_binding.so")
+    if not os.path.exists(path):
+        raise RuntimeError(
+            "habitat_b200: %s is missing. Build it with `python -m habitat_b200.build`; there is no "
+            "fallback." % path)
+    import torch  # noqa: F401  (its shared libraries first)
+    from habitat_b200 import batched, device_table
+    loader = importlib.machinery.ExtensionFileLoader("habitat_b200._binding", path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("habitat_b200._binding", loader))
+    loader.exec_module(module)
+    lib = load()
+    module.setup({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in EXPORTS},
+                 device_table.row_of, check, batched.WaveResult)
+    module.set_generation(device_table.generation())
+    _binding = module
+    return module
+
+
 def check(status):
     if status != HB_OK:
         raise HabitatNativeError(status, load().hb_last_error().decode("utf-8", "replace"))

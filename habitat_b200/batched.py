@@ -30,17 +30,14 @@ def _require_cuda(t, dtype, name):
 _NVTX = os.environ.get("HABITAT_B200_NVTX", "") not in ("", "0")
 
 
-class _Range:
-    def __init__(self, name):
-        self.name = name
-
-    def __enter__(self):
-        if _NVTX:
-            torch.cuda.nvtx.range_push(self.name)
-
-    def __exit__(self, *exc):
-        if _NVTX:
-            torch.cuda.nvtx.range_pop()
+def _call(name, fn, *args):
+    if not _NVTX:
+        return fn(*args)
+    torch.cuda.nvtx.range_push(name)
+    try:
+        return fn(*args)
+    finally:
+        torch.cuda.nvtx.range_pop()
 
 
 def _ptr(t):
@@ -118,15 +115,12 @@ class WavePartials:
 
     def totals(self, out=None):
         """[D] float64 totals of the last wave_scale call that was given this object."""
-        if out is None:
-            out = torch.empty((self.n_planes,), dtype=torch.float64, device=self.buffer.device)
-        _require_cuda(out, torch.float64, "out")
-        if out.numel() != self.n_planes:
+        res = _call("hb_partials_sum", _native.binding().partials_sum, self.buffer, self.per_plane, self.n_planes,
+                    out)
+        if res is None:
+            _require_cuda(out, torch.float64, "out")
             raise ValueError("out must have one entry per destination")
-        with _Range("hb_partials_sum"):
-            _native.check(_native.load().hb_partials_sum(_ptr(self.buffer), self.per_plane, self.n_planes,
-                                                         _ptr(out), _native.current_stream_ptr()))
-        return out
+        return res
 
 
 def wave_scale(kernels: KernelBatch, origin, dests: Sequence, dest_regs=None, metrics=None,
@@ -140,10 +134,16 @@ def wave_scale(kernels: KernelBatch, origin, dests: Sequence, dest_regs=None, me
     With `partials` the call also leaves the first stage of the per-destination totals there.
     Queued on the current stream; does not synchronise.
     """
-    lib = _native.load()
-    K = len(kernels)
-    D = len(dests)
-    dev = kernels.num_blocks.device
+    res = _call("hb_wave_scale", _native.binding().wave_scale, kernels, origin, dests, dest_regs, metrics,
+                want_status, want_limits, out, partials)
+    if res is None:
+        _check_wave_arguments(kernels, dests, dest_regs, metrics, partials)
+    return res
+
+
+def _check_wave_arguments(kernels, dests, dest_regs, metrics, partials):
+    """Says what is wrong with arguments the binding did not take."""
+    K, D = len(kernels), len(dests)
     _require_cuda(kernels.num_blocks, torch.int32, "num_blocks")
     _require_cuda(kernels.block_size, torch.uint16, "block_size")
     _require_cuda(kernels.regs_per_thread, torch.uint16, "regs_per_thread")
@@ -160,51 +160,17 @@ def wave_scale(kernels: KernelBatch, origin, dests: Sequence, dest_regs=None, me
         _require_cuda(dest_regs, torch.int16, "dest_regs")
         if tuple(dest_regs.shape) != (D, K):
             raise ValueError("dest_regs must be [D, K]")
-    rows = device_table.rows_of([origin] + list(dests))
-    if out is None:
-        out = WaveResult(
-            scaled_ns=torch.empty((D, K), dtype=torch.float32, device=dev),
-            dest_occupancy=torch.empty((D, K), dtype=torch.uint8, device=dev),
-            dest_waves=torch.empty((D, K), dtype=torch.uint32, device=dev),
-            origin_occupancy=torch.empty((K,), dtype=torch.uint8, device=dev),
-            origin_waves=torch.empty((K,), dtype=torch.uint32, device=dev),
-            status=torch.empty((D, K), dtype=torch.uint8, device=dev) if want_status else None,
-            limits=torch.empty((D + 1, 4, K), dtype=torch.int32, device=dev) if want_limits else None)
-    soa = _native.KernelSoA(_ptr(kernels.num_blocks), _ptr(kernels.block_size),
-                            _ptr(kernels.regs_per_thread), _ptr(kernels.smem_bytes),
-                            _ptr(kernels.run_time_ns), _ptr(kernels.gamma))
-    wout = _native.WaveOut(_ptr(out.scaled_ns), _ptr(out.dest_occupancy), _ptr(out.dest_waves),
-                           _ptr(out.origin_occupancy), _ptr(out.origin_waves), _ptr(out.status),
-                           _ptr(out.limits))
-    dest_rows = (ctypes.c_int32 * D)(*rows[1:])
-    stream = _native.current_stream_ptr()
     if partials is not None:
         if metrics is not None:
             raise ValueError("partials are not available together with metrics")
         if K > partials.K or D > partials.D:
             raise ValueError("partials were sized for fewer kernels or destinations")
-        per_plane = ctypes.c_int32(0)
-        with _Range("hb_wave_scale_partials"):
-            st = lib.hb_wave_scale_partials(ctypes.byref(soa), K, rows[0], dest_rows, D, _ptr(dest_regs),
-                                            ctypes.byref(wout), _ptr(partials.buffer), ctypes.byref(per_plane),
-                                            stream)
-        partials.per_plane, partials.n_planes = int(per_plane.value), D
-    elif metrics is None:
-        with _Range("hb_wave_scale"):
-            st = lib.hb_wave_scale(ctypes.byref(soa), K, rows[0], dest_rows, D, _ptr(dest_regs),
-                                   ctypes.byref(wout), stream)
-    else:
+    if metrics is not None:
         _require_cuda(metrics.flop_efficiency_pct, torch.float64, "flop_efficiency_pct")
         _require_cuda(metrics.dram_read_bytes, torch.float64, "dram_read_bytes")
         _require_cuda(metrics.dram_write_bytes, torch.float64, "dram_write_bytes")
         _require_cuda(metrics.has_metrics, torch.uint8, "has_metrics")
-        m = _native.KernelMetrics(_ptr(metrics.flop_efficiency_pct), _ptr(metrics.dram_read_bytes),
-                                  _ptr(metrics.dram_write_bytes), _ptr(metrics.has_metrics))
-        with _Range("hb_wave_scale_metrics"):
-            st = lib.hb_wave_scale_metrics(ctypes.byref(soa), ctypes.byref(m), K, rows[0], dest_rows, D,
-                                           _ptr(dest_regs), ctypes.byref(wout), stream)
-    _native.check(st)
-    return out
+    raise ValueError("wave_scale: unsupported arguments (at most %d destinations)" % _native.HB_MAX_DEVICES)
 
 
 WAVE_PATHS = {0: "none", 1: "wave_scale_kernel", 2: "wave_scale_fast_kernel", 4: "wave_scale_lut_kernel"}
@@ -274,20 +240,17 @@ class MLPHandle:
 
     def predict(self, op_features, device_row, out=None):
         """op_features [Q, F] float32 CUDA, device_row [Q] uint8 CUDA -> [Q] float32."""
-        lib = _native.load()
-        _require_cuda(op_features, torch.float32, "op_features")
-        _require_cuda(device_row, torch.uint8, "device_row")
-        Q = op_features.shape[0]
-        if op_features.ndim != 2 or op_features.shape[1] != self.n_op_features:
-            raise ValueError("op_features must be [Q, %d]" % self.n_op_features)
-        if device_row.numel() != Q:
-            raise ValueError("device_row must have Q entries")
-        if out is None:
-            out = torch.empty((Q,), dtype=torch.float32, device=op_features.device)
-        with _Range("hb_mlp_predict"):
-            _native.check(lib.hb_mlp_predict(self._handle, _ptr(op_features), _ptr(device_row), Q,
-                                             _ptr(out), _native.current_stream_ptr()))
-        return out
+        res = _call("hb_mlp_predict", _native.binding().mlp_predict, self._handle.value or 0, self.n_op_features,
+                    op_features, device_row, out)
+        if res is None:
+            _require_cuda(op_features, torch.float32, "op_features")
+            _require_cuda(device_row, torch.uint8, "device_row")
+            if op_features.ndim != 2 or op_features.shape[1] != self.n_op_features:
+                raise ValueError("op_features must be [Q, %d]" % self.n_op_features)
+            if device_row.numel() != op_features.shape[0]:
+                raise ValueError("device_row must have Q entries")
+            raise TypeError("out must be a CUDA tensor")
+        return res
 
     def predict_host(self, op_features, device_row):
         """numpy in / numpy out; transfers and the status check inside the native call."""
@@ -350,47 +313,35 @@ def special_scale(run_time_ms, pred_dest, pred_orig, negative_count=None):
 
 def segment_sum(values, offsets):
     """float64 sums of values[offsets[s]:offsets[s+1]] (float32 / int64 CUDA tensors)."""
-    lib = _native.load()
-    _require_cuda(values, torch.float32, "values")
-    _require_cuda(offsets, torch.int64, "offsets")
-    n = offsets.numel() - 1
-    out = torch.empty((max(n, 0),), dtype=torch.float64, device=values.device)
-    _native.check(lib.hb_segment_sum(_ptr(values), _ptr(offsets), n, _ptr(out),
-                                     _native.current_stream_ptr()))
-    return out
+    res = _native.binding().segment_sum(values, offsets)
+    if res is None:
+        _require_cuda(values, torch.float32, "values")
+        _require_cuda(offsets, torch.int64, "offsets")
+    return res
 
 
 def plane_sum(values, out=None):
     """float64 sum of each row of a [P, L] float32 CUDA tensor, NaN entries skipped."""
-    lib = _native.load()
-    _require_cuda(values, torch.float32, "values")
-    if values.ndim != 2:
-        raise ValueError("values must be [planes, length]")
-    P, L = values.shape
-    if out is None:
-        out = torch.empty((P,), dtype=torch.float64, device=values.device)
-    else:
+    res = _native.binding().plane_sum(values, out)
+    if res is None:
+        _require_cuda(values, torch.float32, "values")
+        if values.ndim != 2:
+            raise ValueError("values must be [planes, length]")
         _require_cuda(out, torch.float64, "out")
-        if out.numel() != P:
-            raise ValueError("out must have one entry per plane")
-    _native.check(lib.hb_plane_sum(_ptr(values), L, P, _ptr(out), _native.current_stream_ptr()))
-    return out
+        raise ValueError("out must have one entry per plane")
+    return res
 
 
 def group_sum(values, keys, n_groups, out=None):
     """float64 sums of a float32 CUDA vector grouped by a uint8 key per element (keys at or above
     n_groups and NaN values are skipped): per-device totals of a batch of MLP predictions."""
-    lib = _native.load()
-    _require_cuda(values, torch.float32, "values")
-    _require_cuda(keys, torch.uint8, "keys")
-    if values.numel() != keys.numel():
-        raise ValueError("values and keys must have the same length")
-    if out is None:
-        out = torch.empty((n_groups,), dtype=torch.float64, device=values.device)
-    else:
-        _require_cuda(out, torch.float64, "out")
-        if out.numel() != n_groups:
-            raise ValueError("out must have one entry per group")
-    _native.check(lib.hb_group_sum(_ptr(values), _ptr(keys), values.numel(), n_groups, _ptr(out),
-                                   _native.current_stream_ptr()))
-    return out
+    res = _native.binding().group_sum(values, keys, n_groups, out)
+    if res is None:
+        _require_cuda(values, torch.float32, "values")
+        _require_cuda(keys, torch.uint8, "keys")
+        if values.numel() != keys.numel():
+            raise ValueError("values and keys must have the same length")
+        if out is not None:
+            _require_cuda(out, torch.float64, "out")
+        raise ValueError("out must have one entry per group")
+    return res

@@ -15,6 +15,7 @@ LIB_DIR = os.path.join(PKG_DIR, "_lib")
 OBJ_DIR = os.path.join(PKG_DIR, "_lib", "obj")
 INCLUDE_DIR = os.path.join(os.path.dirname(PKG_DIR), "include")
 LIB_PATH = os.path.join(LIB_DIR, "libhabitat_b200.so")
+BINDING_PATH = os.path.join(LIB_DIR, "_binding.so")
 
 SOURCES = ["hb_error.cu", "wave_scale.cu", "reduce.cu", "peer_exchange.cu", "mlp_chain.cu", "mlp_wide.cu",
            "device_probe.cu"]
@@ -38,6 +39,30 @@ def _stale(target, deps):
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def build_binding(force=False, verbose=False):
+    """Compiles the CPython binding of the tensor-level entry points (host code only, against the
+    installed torch).  Returns its path."""
+    import sysconfig
+
+    import torch
+    src = os.path.join(SRC_DIR, "binding.cpp")
+    if force or _stale(BINDING_PATH, [src, os.path.join(INCLUDE_DIR, "habitat_b200.h")]):
+        os.makedirs(LIB_DIR, exist_ok=True)
+        root = os.path.dirname(torch.__file__)
+        cuda = os.path.dirname(os.path.dirname(_nvcc()))
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+               "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), "-I", INCLUDE_DIR]
+        for d in (os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                  os.path.join(cuda, "include"), sysconfig.get_paths()["include"]):
+            cmd += ["-isystem", d]
+        cmd += [src, "-o", BINDING_PATH, "-L", os.path.join(root, "lib")]
+        cmd += ["-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+        if verbose:
+            print(" ".join(cmd), file=sys.stderr)
+        subprocess.run(cmd, check=True)
+    return BINDING_PATH
 
 
 # Sources that carry index checks under -DHB_BOUNDS_CHECK (the checked library reuses the
@@ -77,6 +102,7 @@ def build(force=False, verbose=False, ptxas_info=False, checked=False):
         if verbose:
             print(" ".join(cmd), file=sys.stderr)
         subprocess.run(cmd, check=True)
+    build_binding(force=force, verbose=verbose)
     return lib_path
 
 

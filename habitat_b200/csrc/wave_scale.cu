@@ -819,55 +819,72 @@ cudaError_t launch_lut_plain(int np, int ns, unsigned grid, cudaStream_t stream,
   }
 }
 
-// Launches wave_scale_lut_kernel when the launch qualifies; false = nothing launched.  *fused says
-// whether the launch also wrote p.block_sums (one sum per destination and block of the grid).
-bool try_launch_lut(const Ptrs& p, const LaunchParams& lp, int sm_count, cudaStream_t stream, hb_status* st,
-                    bool* fused, unsigned* fused_blocks) {
-  *fused = false;
-  static const bool use_lut = [] { const char* e = std::getenv("HB_WAVE_LUT"); return !e || std::atoi(e) != 0; }();
-  if (!use_lut || p.limits || lp.D > HB_MAX_DEVICES / 2) return false;
-  const int64_t K = lp.K;
-  if (static_cast<int64_t>(lp.D) * K >= (int64_t{1} << 31)) return false;   // 32-bit element indices
+// Everything about a launch that depends on the devices alone.  Callers ask for the same origin and
+// destinations again and again, so a thread keeps its last few plans; a plan is of one version of the
+// device table and holds no results.
+struct LaunchPlan {
+  uint64_t version = 0;
+  LaunchParams lp{};
+  bool lut_ok = false;         // every row can be tabulated
+  bool many_classes = false;   // more than four classes: every row's own tables (extended variant)
+  int n_p = 0, n_s = 0;
   LutParams q{};
-  int rows_p[kMaxClasses] = {}, rows_s[kMaxClasses] = {}, n_p = 0, n_s = 0;
+};
+
+void fill_lut(LaunchPlan* plan) {   // call with g_mu held
+  const LaunchParams& lp = plan->lp;
+  LutParams& q = plan->q;
+  int rows_p[kMaxClasses] = {}, rows_s[kMaxClasses] = {};
+  plan->lut_ok = lp.D <= HB_MAX_DEVICES / 2 && g_tab.lut_ok[lp.origin_row];
+  for (int d = 0; d < lp.D && plan->lut_ok; ++d) plan->lut_ok = g_tab.lut_ok[lp.dest_row[d]];
+  if (!plan->lut_ok) return;
   bool many_classes = false;
-  {
-    std::lock_guard<std::mutex> lock(g_mu);
-    if (!g_tab.lut_ok[lp.origin_row]) return false;
-    for (int d = 0; d < lp.D; ++d)
-      if (!g_tab.lut_ok[lp.dest_row[d]]) return false;
-    for (int d = -1; d < lp.D; ++d) {
-      const int row = d < 0 ? lp.origin_row : lp.dest_row[d];
-      const int pc = many_classes ? -1 : class_of(rows_p, &n_p, row, same_p_class);
-      const int sc = many_classes ? -1 : class_of(rows_s, &n_s, row, same_smem_class);
-      if (pc < 0 || sc < 0) many_classes = true;   // more than four classes: every row's own tables (extended variant)
-      LutDev& o = d < 0 ? q.origin : q.dest[d];
-      o.sel_p = pair_selector(pc < 0 ? 0 : pc);
-      o.sel_s = pair_selector(sc < 0 ? 0 : sc);
-      o.t_off = static_cast<uint32_t>(row * kLutOcc * sizeof(LutOcc));
-      o.p_off = static_cast<uint32_t>(row * kLutP);
-      o.s_off = static_cast<uint32_t>(row * kLutS);
-      o.sms_m1 = static_cast<uint32_t>(g_tab.rows[row].num_sms - 1);
-      o.sms_magic = magic_of(static_cast<uint32_t>(g_tab.rows[row].num_sms));
-      if (d >= 0) {
-        o.a_hi = static_cast<float>(lp.a[d]);
-        o.a_lo = static_cast<float>(lp.a[d] - static_cast<double>(o.a_hi));
-        o.b_hi = static_cast<float>(lp.b[d]);
-        o.b_lo = static_cast<float>(lp.b[d] - static_cast<double>(o.b_hi));
-        q.ridge[d] = lp.ridge[d];
-        q.slope[d] = -0.5 / lp.ridge[d];
-      }
+  for (int d = -1; d < lp.D; ++d) {
+    const int row = d < 0 ? lp.origin_row : lp.dest_row[d];
+    const int pc = many_classes ? -1 : class_of(rows_p, &plan->n_p, row, same_p_class);
+    const int sc = many_classes ? -1 : class_of(rows_s, &plan->n_s, row, same_smem_class);
+    if (pc < 0 || sc < 0) many_classes = true;
+    LutDev& o = d < 0 ? q.origin : q.dest[d];
+    o.sel_p = pair_selector(pc < 0 ? 0 : pc);
+    o.sel_s = pair_selector(sc < 0 ? 0 : sc);
+    o.t_off = static_cast<uint32_t>(row * kLutOcc * sizeof(LutOcc));
+    o.p_off = static_cast<uint32_t>(row * kLutP);
+    o.s_off = static_cast<uint32_t>(row * kLutS);
+    o.sms_m1 = static_cast<uint32_t>(g_tab.rows[row].num_sms - 1);
+    o.sms_magic = magic_of(static_cast<uint32_t>(g_tab.rows[row].num_sms));
+    if (d >= 0) {
+      o.a_hi = static_cast<float>(lp.a[d]);
+      o.a_lo = static_cast<float>(lp.a[d] - static_cast<double>(o.a_hi));
+      o.b_hi = static_cast<float>(lp.b[d]);
+      o.b_lo = static_cast<float>(lp.b[d] - static_cast<double>(o.b_hi));
+      q.ridge[d] = lp.ridge[d];
+      q.slope[d] = -0.5 / lp.ridge[d];
     }
   }
+  plan->many_classes = many_classes;
   // class slots beyond the count repeat class 0 (the kernel variants are built for 1..4 classes,
   // the extended one always loads four)
   for (int c = 0; c < kMaxClasses; ++c) {
-    q.off_p[c] = static_cast<uint32_t>(rows_p[c < n_p ? c : 0] * kLutP);   // unused by the extended variant
-    q.off_s[c] = static_cast<uint32_t>(rows_s[c < n_s ? c : 0] * kLutS);
+    q.off_p[c] = static_cast<uint32_t>(rows_p[c < plan->n_p ? c : 0] * kLutP);   // unused by the extended variant
+    q.off_s[c] = static_cast<uint32_t>(rows_s[c < plan->n_s ? c : 0] * kLutS);
   }
-  q.K = static_cast<uint32_t>(K);
   q.D = lp.D;
   q.origin_peak = lp.origin_peak;
+}
+
+// Launches wave_scale_lut_kernel when the launch qualifies; false = nothing launched.  *fused says
+// whether the launch also wrote p.block_sums (one sum per destination and block of the grid).
+bool try_launch_lut(const Ptrs& p, const LaunchPlan& plan, int64_t K, int sm_count, cudaStream_t stream, hb_status* st,
+                    bool* fused, unsigned* fused_blocks) {
+  *fused = false;
+  static const bool use_lut = [] { const char* e = std::getenv("HB_WAVE_LUT"); return !e || std::atoi(e) != 0; }();
+  const LaunchParams& lp = plan.lp;
+  if (!use_lut || p.limits || !plan.lut_ok) return false;
+  if (static_cast<int64_t>(lp.D) * K >= (int64_t{1} << 31)) return false;   // 32-bit element indices
+  LutParams q = plan.q;
+  q.K = static_cast<uint32_t>(K);
+  const int n_p = plan.n_p, n_s = plan.n_s;
+  const bool many_classes = plan.many_classes;
 
   auto al = [](const void* ptr, uintptr_t a) { return (reinterpret_cast<uintptr_t>(ptr) & (a - 1)) == 0; };
   const bool metrics = p.has_metrics != nullptr;
@@ -911,7 +928,7 @@ bool try_launch_lut(const Ptrs& p, const LaunchParams& lp, int sm_count, cudaStr
 
 // Division-free kernel when every row of the launch is ordinary and only the five standard
 // outputs are wanted; returns false (nothing launched) otherwise.
-bool try_launch_fast(const Ptrs& p, const LaunchParams& lp, cudaStream_t stream, hb_status* st) {
+bool try_launch_fast(const Ptrs& p, const LaunchParams& lp, int64_t K, cudaStream_t stream, hb_status* st) {
   if (p.status || p.limits || lp.D > HB_MAX_DEVICES / 2) return false;
   FastParams fp{};
   {
@@ -920,7 +937,7 @@ bool try_launch_fast(const Ptrs& p, const LaunchParams& lp, cudaStream_t stream,
     for (int d = 0; d < lp.D; ++d)
       if (!fast_row_ok(g_tab.rows[lp.dest_row[d]], g_tab.pre[lp.dest_row[d]])) return false;
     fp.D = lp.D;
-    fp.K = lp.K;
+    fp.K = K;
     fp.origin = fold_fast(g_tab.rows[lp.origin_row], g_tab.pre[lp.origin_row]);
     for (int d = 0; d < lp.D; ++d) {
       FastDev& f = fp.dest[d];
@@ -932,7 +949,6 @@ bool try_launch_fast(const Ptrs& p, const LaunchParams& lp, cudaStream_t stream,
       f.log2_clk = lp.log2_clk[d];
     }
   }
-  const int64_t K = lp.K;
   const bool vec4 = vec4_ok(p, K, true);
   const int threads = 256, vec = vec4 ? 4 : 1;
   const int64_t blocks = ((K + vec - 1) / vec + threads - 1) / threads;
@@ -956,17 +972,18 @@ bool try_launch_fast(const Ptrs& p, const LaunchParams& lp, cudaStream_t stream,
 }
 
 template <bool METRICS>
-hb_status launch_kernel(const Ptrs& p, const LaunchParams& lp, cudaStream_t stream, bool* fused,
+hb_status launch_kernel(const Ptrs& p, const LaunchPlan& plan, int64_t K, cudaStream_t stream, bool* fused,
                         unsigned* fused_blocks) {
   int sm_count = 0;
   const hb_status sync_st = sync_gpu(&sm_count);
   if (sync_st != HB_OK) return sync_st;
-  const int64_t K = lp.K;
   const bool extra = p.status != nullptr || p.limits != nullptr;
   hb_status fast_st = HB_OK;
   *fused = false;
-  if (try_launch_lut(p, lp, sm_count, stream, &fast_st, fused, fused_blocks)) return fast_st;
-  if (!METRICS && try_launch_fast(p, lp, stream, &fast_st)) return fast_st;
+  if (try_launch_lut(p, plan, K, sm_count, stream, &fast_st, fused, fused_blocks)) return fast_st;
+  if (!METRICS && try_launch_fast(p, plan.lp, K, stream, &fast_st)) return fast_st;
+  LaunchParams lp = plan.lp;
+  lp.K = K;
   const bool vec4 = vec4_ok(p, K, !METRICS);
   const int threads = 256;
   const int vec = vec4 ? 4 : 1;
@@ -993,25 +1010,24 @@ hb_status launch_kernel(const Ptrs& p, const LaunchParams& lp, cudaStream_t stre
 // per-destination totals: inside the table kernel when it can (per_plane = blocks of its grid),
 // else by the plane-sum kernel over the results just written (per_plane = kPlaneBlocks).
 template <bool METRICS>
-hb_status launch(const Ptrs& p, const LaunchParams& lp, cudaStream_t stream, int32_t* per_plane = nullptr) {
+hb_status launch(const Ptrs& p, const LaunchPlan& plan, int64_t K, cudaStream_t stream, int32_t* per_plane = nullptr) {
   bool fused = false;
   unsigned fused_blocks = 0;
-  const hb_status st = launch_kernel<METRICS>(p, lp, stream, &fused, &fused_blocks);
+  const hb_status st = launch_kernel<METRICS>(p, plan, K, stream, &fused, &fused_blocks);
   if (st != HB_OK || !p.block_sums) return st;
   if (fused) {
     *per_plane = static_cast<int32_t>(fused_blocks);
     return HB_OK;
   }
-  HB_CUDA_TRY(hb::launch_overlapped(plane_partial_kernel, dim3(lp.D, kPlaneBlocks), dim3(kSumThreads), 0, stream,
-                                    static_cast<const float*>(p.scaled_ns), static_cast<int64_t>(lp.K),
+  HB_CUDA_TRY(hb::launch_overlapped(plane_partial_kernel, dim3(plan.lp.D, kPlaneBlocks), dim3(kSumThreads), 0, stream,
+                                    static_cast<const float*>(p.scaled_ns), K,
                                     p.block_sums));
   *per_plane = kPlaneBlocks;
   return HB_OK;
 }
 
 hb_status fill_params(LaunchParams* lp, int64_t K, int32_t origin_row, const int32_t* dest_rows,
-                      int32_t D) {
-  std::lock_guard<std::mutex> lock(g_mu);
+                      int32_t D) {   // call with g_mu held
   if (g_tab.n == 0) {
     hb::set_error("hb_wave_scale: no device table (call hb_set_devices first)");
     return HB_ERR_INVALID_ARGUMENT;
@@ -1023,7 +1039,6 @@ hb_status fill_params(LaunchParams* lp, int64_t K, int32_t origin_row, const int
   }
   std::memset(lp, 0, sizeof(*lp));
   lp->D = D;
-  lp->K = K;
   lp->origin_row = origin_row;
   const hb_device_spec& o = g_tab.rows[origin_row];
   lp->origin_peak = static_cast<double>(o.peak_gflops_per_second);
@@ -1044,6 +1059,35 @@ hb_status fill_params(LaunchParams* lp, int64_t K, int32_t origin_row, const int
     lp->log2_clk[d] = l_clk;
     lp->ridge[d] = static_cast<double>(t.peak_gflops_per_second) / t.mem_bandwidth_gb;
   }
+  return HB_OK;
+}
+
+// The plan of (origin, destinations), from this thread's last four or made now.
+hb_status plan_for(const LaunchPlan** out, int64_t K, int32_t origin_row, const int32_t* dest_rows, int32_t D) {
+  constexpr int kPlans = 4;
+  thread_local LaunchPlan plans[kPlans];
+  thread_local int oldest = 0;
+  const uint64_t version = g_version.load(std::memory_order_acquire);
+  if (K >= 0 && D >= 1 && D <= HB_MAX_DEVICES && dest_rows) {
+    for (const LaunchPlan& plan : plans) {
+      if (plan.version != version || version == 0 || plan.lp.origin_row != origin_row || plan.lp.D != D) continue;
+      bool same = true;
+      for (int d = 0; d < D && same; ++d) same = dest_rows[d] == plan.lp.dest_row[d];
+      if (same) {
+        *out = &plan;
+        return HB_OK;
+      }
+    }
+  }
+  std::lock_guard<std::mutex> lock(g_mu);
+  LaunchPlan& plan = plans[oldest];
+  plan = LaunchPlan{};
+  const hb_status st = fill_params(&plan.lp, K, origin_row, dest_rows, D);
+  if (st != HB_OK) return st;
+  fill_lut(&plan);
+  plan.version = g_version.load(std::memory_order_acquire);   // changes only under the lock
+  oldest = (oldest + 1) % kPlans;
+  *out = &plan;
   return HB_OK;
 }
 
@@ -1146,11 +1190,11 @@ extern "C" hb_status hb_wave_scale(const hb_kernel_soa* kernels, int64_t K, int3
                                    void* stream) {
   hb_status st = check_io(kernels, out, true, K);
   if (st != HB_OK) return st;
-  LaunchParams lp;
-  st = fill_params(&lp, K, origin_row, dest_rows_host, D);
+  const LaunchPlan* plan = nullptr;
+  st = plan_for(&plan, K, origin_row, dest_rows_host, D);
   if (st != HB_OK) return st;
   if (K == 0) return HB_OK;
-  return launch<false>(make_ptrs(kernels, nullptr, dest_regs, out), lp,
+  return launch<false>(make_ptrs(kernels, nullptr, dest_regs, out), *plan, K,
                        static_cast<cudaStream_t>(stream));
 }
 
@@ -1170,14 +1214,14 @@ extern "C" hb_status hb_wave_scale_partials(const hb_kernel_soa* kernels, int64_
     hb::set_error("hb_wave_scale_partials: partials / per_plane is NULL");
     return HB_ERR_INVALID_ARGUMENT;
   }
-  LaunchParams lp;
-  st = fill_params(&lp, K, origin_row, dest_rows_host, D);
+  const LaunchPlan* plan = nullptr;
+  st = plan_for(&plan, K, origin_row, dest_rows_host, D);
   if (st != HB_OK) return st;
   *per_plane = 0;
   if (K == 0) return HB_OK;
   Ptrs p = make_ptrs(kernels, nullptr, dest_regs, out);
   p.block_sums = partials;
-  return launch<false>(p, lp, static_cast<cudaStream_t>(stream), per_plane);
+  return launch<false>(p, *plan, K, static_cast<cudaStream_t>(stream), per_plane);
 }
 
 extern "C" hb_status hb_wave_scale_metrics(const hb_kernel_soa* kernels,
@@ -1192,11 +1236,11 @@ extern "C" hb_status hb_wave_scale_metrics(const hb_kernel_soa* kernels,
     hb::set_error("hb_wave_scale_metrics: metrics pointer is NULL");
     return HB_ERR_INVALID_ARGUMENT;
   }
-  LaunchParams lp;
-  st = fill_params(&lp, K, origin_row, dest_rows_host, D);
+  const LaunchPlan* plan = nullptr;
+  st = plan_for(&plan, K, origin_row, dest_rows_host, D);
   if (st != HB_OK) return st;
   if (K == 0) return HB_OK;
-  return launch<true>(make_ptrs(kernels, metrics, dest_regs, out), lp,
+  return launch<true>(make_ptrs(kernels, metrics, dest_regs, out), *plan, K,
                       static_cast<cudaStream_t>(stream));
 }
 
@@ -1206,8 +1250,8 @@ extern "C" hb_status hb_wave_scale_host(const hb_kernel_soa* kernels, int64_t K,
                                         const hb_wave_out* out) {
   hb_status st = check_io(kernels, out, true, K);
   if (st != HB_OK) return st;
-  LaunchParams lp;
-  st = fill_params(&lp, K, origin_row, dest_rows_host, D);
+  const LaunchPlan* plan = nullptr;
+  st = plan_for(&plan, K, origin_row, dest_rows_host, D);
   if (st != HB_OK) return st;
   if (K == 0) return HB_OK;
   const size_t k = static_cast<size_t>(K), kd = k * D;
@@ -1251,7 +1295,7 @@ extern "C" hb_status hb_wave_scale_host(const hb_kernel_soa* kernels, int64_t K,
   hb_kernel_soa dk{nb, bs, rg, sm, tm, gm};
   hb_wave_out dout{o_ns, o_occ, o_wav, o_oocc, o_owav, out->status ? o_st : nullptr,
                    out->limits ? o_lim : nullptr};
-  st = launch<false>(make_ptrs(&dk, nullptr, dest_regs ? dr : nullptr, &dout), lp, s);
+  st = launch<false>(make_ptrs(&dk, nullptr, dest_regs ? dr : nullptr, &dout), *plan, K, s);
   if (st != HB_OK) return st;
   HB_CUDA_TRY(cudaMemcpyAsync(out->scaled_ns, o_ns, kd * 4, d2h, s));
   HB_CUDA_TRY(cudaMemcpyAsync(out->dest_occupancy, o_occ, kd, d2h, s));

@@ -15,6 +15,7 @@ _DATA_DIR = os.path.join(os.path.dirname(os.path.abspath(__file__)), "data")
 
 _rows = []        # spec tuples, index = row
 _index = {}       # spec tuple -> row
+_generation = 1   # counts the tables; part of the tokens that devices carry (row_of)
 _uploaded = 0     # number of rows the library has seen
 _uploaded_device = None
 
@@ -56,7 +57,8 @@ def _sync():
 
 
 def row_of(device):
-    """Row index of a DeviceProperties in the library's table (uploading if new)."""
+    """Row index of a DeviceProperties in the library's table (uploading if new).  The device
+    remembers its row (`_row_token`), which is where the native binding looks first."""
     spec = device.spec_tuple()
     row = _index.get(spec)
     if row is None:
@@ -66,7 +68,15 @@ def row_of(device):
         _rows.append(spec)
         _index[spec] = row
     _sync()
+    try:
+        device._row_token = _generation * _native.HB_MAX_DEVICES + row
+    except AttributeError:
+        pass        # an object of another class that takes no attributes
     return row
+
+
+def generation():
+    return _generation
 
 
 def rows_of(devices):
@@ -77,8 +87,11 @@ def rows_of(devices):
 
 def reset():
     """Forgets every row (tests)."""
-    global _uploaded, _uploaded_device
+    global _uploaded, _uploaded_device, _generation
     _rows.clear()
     _index.clear()
+    _generation += 1
+    if _native._binding is not None:
+        _native._binding.set_generation(_generation)
     _uploaded = 0
     _uploaded_device = None
