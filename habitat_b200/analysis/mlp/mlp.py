@@ -156,9 +156,4 @@ class RuntimePredictor:
     def predict(self, kernel_arguments, device_name):
         """One query; same arguments and return type as the reference."""
         row = self.device_row(device_name)
-        feats = torch.tensor([list(kernel_arguments)], dtype=torch.float32, device="cuda")
-        rows = torch.tensor([row], dtype=torch.uint8, device="cuda")
-        out = self._handle.predict(feats, rows)
-        value = float(out.cpu()[0])
-        self._handle.check_status()
-        return value
+        return self._handle.predict_one(kernel_arguments, row)

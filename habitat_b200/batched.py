@@ -252,6 +252,15 @@ class MLPHandle:
             raise TypeError("out must be a CUDA tensor")
         return res
 
+    def predict_one(self, op_features, device_row):
+        """One query, a sequence of F numbers and a device row; returns a float.  The query travels as a
+        kernel parameter and the result comes back through page-locked memory."""
+        value = _native.binding().mlp_predict_one(self._handle.value or 0, self.n_op_features, op_features,
+                                                  device_row)
+        if value is None:
+            raise ValueError("op_features must be [Q, %d]" % self.n_op_features)
+        return value
+
     def predict_host(self, op_features, device_row):
         """numpy in / numpy out; transfers and the status check inside the native call."""
         lib = _native.load()

@@ -24,6 +24,7 @@ struct Api {
   decltype(&hb_wave_scale_partials) wave_scale_partials = nullptr;
   decltype(&hb_partials_sum) partials_sum = nullptr;
   decltype(&hb_mlp_predict) mlp_predict = nullptr;
+  decltype(&hb_mlp_predict_host) mlp_predict_host = nullptr;
   decltype(&hb_group_sum) group_sum = nullptr;
   decltype(&hb_plane_sum) plane_sum = nullptr;
   decltype(&hb_segment_sum) segment_sum = nullptr;
@@ -290,6 +291,30 @@ PyObject* mlp_predict(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// mlp_predict_one(handle address, F, op features of one query, device row) -> float
+PyObject* mlp_predict_one(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 4) Py_RETURN_NONE;
+  hb_mlp* h = static_cast<hb_mlp*>(PyLong_AsVoidPtr(a[0]));
+  const long F = PyLong_AsLong(a[1]), row = PyLong_AsLong(a[3]);
+  Ref seq(PySequence_Fast(a[2], "the operation's features must be a sequence"));
+  if (!seq.p || PyErr_Occurred()) return nullptr;
+  constexpr long kMaxF = 8;
+  if (F > kMaxF || PySequence_Fast_GET_SIZE(seq.p) != F || row < 0 || row > 255) Py_RETURN_NONE;
+  float f[kMaxF], out = 0.0f;
+  for (long i = 0; i < F; ++i) {
+    const double v = PyFloat_AsDouble(PySequence_Fast_GET_ITEM(seq.p, i));
+    if (v == -1.0 && PyErr_Occurred()) return nullptr;
+    f[i] = static_cast<float>(v);
+  }
+  const uint8_t r = static_cast<uint8_t>(row);
+  hb_status st;
+  Py_BEGIN_ALLOW_THREADS
+  st = api.mlp_predict_host(h, f, &r, 1, &out);
+  Py_END_ALLOW_THREADS
+  if (failed(st)) return nullptr;
+  return PyFloat_FromDouble(out);
+}
+
 // partials_sum(buffer, per_plane, n_planes, out)
 PyObject* partials_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -369,7 +394,7 @@ PyObject* setup(PyObject*, PyObject* const* a, Py_ssize_t n) {
   };
   if (!load(api.wave_scale, "hb_wave_scale") || !load(api.wave_scale_metrics, "hb_wave_scale_metrics") ||
       !load(api.wave_scale_partials, "hb_wave_scale_partials") || !load(api.partials_sum, "hb_partials_sum") ||
-      !load(api.mlp_predict, "hb_mlp_predict") || !load(api.group_sum, "hb_group_sum") ||
+      !load(api.mlp_predict, "hb_mlp_predict") || !load(api.mlp_predict_host, "hb_mlp_predict_host") || !load(api.group_sum, "hb_group_sum") ||
       !load(api.plane_sum, "hb_plane_sum") || !load(api.segment_sum, "hb_segment_sum")) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "an entry point is missing");
     return nullptr;
@@ -387,7 +412,7 @@ PyObject* set_generation(PyObject*, PyObject* v) {
 }
 
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {FAST(setup), FAST(wave_scale), FAST(mlp_predict), FAST(partials_sum), FAST(group_sum),
+PyMethodDef methods[] = {FAST(setup), FAST(wave_scale), FAST(mlp_predict), FAST(mlp_predict_one), FAST(partials_sum), FAST(group_sum),
                          FAST(plane_sum), FAST(segment_sum),
                          {"set_generation", set_generation, METH_O, nullptr},
                          {nullptr, nullptr, 0, nullptr}};

@@ -36,11 +36,23 @@ struct HostArena {
   void* base = nullptr;
   size_t bytes = 0;
   cudaStream_t stream = nullptr;
+  uint8_t* pinned = nullptr;   // page-locked, readable and writable by the GPU at the same address
+  size_t pinned_bytes = 0;
 };
 // The arena of the current CUDA device (created, with its stream, on first use).
 hb_status arena_for_current_device(HostArena** out);
 // Makes the block at least `bytes` large.  Call with the arena's mutex held.
 hb_status arena_reserve(HostArena* arena, size_t bytes);
+
+// The same for the page-locked block.
+hb_status arena_reserve_pinned(HostArena* arena, size_t bytes);
+
+// Waits for results that a kernel on `stream` stores straight into page-locked memory: `n` 32-bit words
+// that the caller has filled with kUnwritten (no arithmetic result has this bit pattern).  Watching the
+// words takes about a microsecond after the store; cudaStreamSynchronize, which the wait falls back on
+// when nothing comes (a failed launch, a long kernel), takes several.
+constexpr uint32_t kUnwritten = 0xFFFFFFFFu;
+hb_status wait_written(const void* words, size_t n, cudaStream_t stream);
 
 // Hands out 256-byte aligned pieces of a block; with a null base it only adds up sizes.
 class Carver {

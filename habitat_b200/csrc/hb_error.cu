@@ -1,4 +1,5 @@
 // Error text and version of the library.
+#include <atomic>
 #include <cstdlib>
 
 #include "hb_common.h"
@@ -61,6 +62,36 @@ hb_status arena_reserve(HostArena* a, size_t bytes) {
     return HB_OK;
   }
   a->bytes = want;
+  return HB_OK;
+}
+
+hb_status arena_reserve_pinned(HostArena* a, size_t bytes) {
+  if (bytes <= a->pinned_bytes) return HB_OK;
+  if (a->pinned) cudaFreeHost(a->pinned);
+  a->pinned = nullptr;
+  a->pinned_bytes = 0;
+  const size_t want = bytes < (64u << 10) ? (64u << 10) : bytes + bytes / 4;
+  void* p = nullptr;
+  const cudaError_t e = cudaHostAlloc(&p, want, cudaHostAllocDefault);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaHostAlloc (host-entry staging)");
+  a->pinned = static_cast<uint8_t*>(p);
+  a->pinned_bytes = want;
+  return HB_OK;
+}
+
+hb_status wait_written(const void* words, size_t n, cudaStream_t stream) {
+  const volatile uint32_t* w = static_cast<const volatile uint32_t*>(words);
+  constexpr int kSpins = 200000;   // some hundred microseconds
+  int spins = 0;
+  for (size_t i = 0; i < n; ++i) {
+    while (w[i] == kUnwritten) {
+      if (++spins > kSpins) {
+        const cudaError_t e = cudaStreamSynchronize(stream);
+        return e == cudaSuccess ? HB_OK : cuda_fail(e, "cudaStreamSynchronize");
+      }
+    }
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
   return HB_OK;
 }
 }  // namespace hb

@@ -221,7 +221,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
       if (*abort_flag) return false;
       if (clock64() - t0 > kWaitCycles) {
         *abort_flag = 1;
-        atomicCAS(status, 0, code);
+        *static_cast<volatile int32_t*>(status) = code;
         return false;
       }
     }
@@ -264,7 +264,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
       if (*abort_flag) return false;
       if (clock64() - t0 > kWaitCycles) {
         *abort_flag = 1;
-        atomicCAS(status, 0, code);
+        *static_cast<volatile int32_t*>(status) = code;
         return false;
       }
     }
@@ -340,7 +340,7 @@ struct hb_mlp {
   double* mu = nullptr;
   double* sigma = nullptr;
   double* dev_feat = nullptr;
-  int32_t* status = nullptr;
+  int32_t* status = nullptr;          // page-locked host word that the kernels write when they give up
   long long* phase_cycles = nullptr;
   bool counted = false;      // among the GPU's predictors (mlp_wide.cu)
 };

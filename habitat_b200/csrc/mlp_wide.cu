@@ -32,11 +32,14 @@
 // 8-15 (64 columns: 8-23) receivers.  Every wait is bounded, as in mlp_chain.cu; a launch that gave up
 // leaves a mark in the scratch, and launches that find it report an error instead of a result.
 #include <atomic>
+#include <cstring>
 
 #include "mlp_common.cuh"
 #include "mlp_wide.h"
 
 namespace {
+
+using hb::kWideInline;
 
 struct WideParams {
   const float* bias;
@@ -57,6 +60,9 @@ struct WideParams {
   int32_t* poison;            // set by a launch that gave up
   uint32_t tag;               // of this launch
   unsigned long long parity[2];   // bit g: parity of the next use of group g's buffer 0, 1
+  int32_t inline_q;           // > 0: the queries themselves, below, instead of feats and dev_row
+  float inline_feats[kWideInline * (kMaxInFeat - 4)];
+  uint8_t inline_row[kWideInline];
   CUtensorMap map_slot;       // 32 KB of weight rows: a ring slot
   CUtensorMap map_fc1;        // one K block of the block's rows
 };
@@ -98,7 +104,7 @@ __device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned l
 // Gives up on behalf of the whole block.
 __device__ __forceinline__ void give_up(volatile int* abort_flag, int32_t* status, int32_t* poison, int code) {
   *abort_flag = 1;
-  atomicCAS(status, 0, code);
+  *static_cast<volatile int32_t*>(status) = code;
   atomicExch(poison, 1);
 }
 // mbar_wait that also leaves the mark in the scratch.
@@ -203,7 +209,7 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
   if (threadIdx.x == 64 && *reinterpret_cast<volatile int32_t*>(p.poison) != 0) {
     // an earlier launch left the buffers in an unknown state: report, and touch nothing
     *poisoned = 1;
-    atomicCAS(p.status, 0, 0x5FF);
+    *static_cast<volatile int32_t*>(p.status) = 0x5FF;
   } else if (threadIdx.x == 64) {
     *poisoned = 0;
   }
@@ -416,9 +422,9 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     epi_sync();
     for (int i = T; i < n_q * C_in; i += 128) {
       const int q = i / C_in, f = i - q * C_in;
-      int dr = p.dev_row[q0 + q];
+      int dr = p.inline_q ? p.inline_row[q] : p.dev_row[q0 + q];
       dr = dr < p.n_dev ? dr : p.n_dev - 1;
-      const double x = f < p.n_op_feat ? static_cast<double>(p.feats[(q0 + q) * p.n_op_feat + f])
+      const double x = f < p.n_op_feat ? static_cast<double>(p.inline_q ? p.inline_feats[i - 4 * q] : p.feats[(q0 + q) * p.n_op_feat + f])
                                        : p.dev_feat[dr * 4 + (f - p.n_op_feat)];
       const float xn = static_cast<float>((x - p.mu[f]) / p.sigma[f]);
       const __nv_bfloat16 hi = __float2bfloat16_rn(xn);
@@ -724,9 +730,9 @@ void wide_start_over(int device) {
 }
 
 hb_status wide_predict(hb_mlp* h, const WidePlan& w, const float* feats, const uint8_t* dev_row, int64_t Q, float* out,
-                       cudaStream_t stream, bool* launched) {
+                       cudaStream_t stream, bool* launched, bool host_inputs) {
   *launched = false;
-  if (w.G == 0 || h->device >= kMaxCudaDevices) return HB_OK;
+  if (w.G == 0 || h->device >= kMaxCudaDevices || (host_inputs && Q > kWideInline)) return HB_OK;
   GpuScratch& g = g_wide[h->device];
   std::lock_guard<std::mutex> lock(g.mu);   // held over the launch: parities and tags follow the stream's order
   StreamScratch* s = scratch_of(g, stream);
@@ -737,6 +743,11 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const float* feats, const u
   p.n_dev = h->n_dev; p.n_op_feat = h->n_op_feat; p.layers = h->layers;
   p.feats = feats; p.dev_row = dev_row; p.Q = static_cast<int32_t>(Q); p.per_group = w.per_group; p.out = out;
   p.status = h->status;
+  if (host_inputs) {
+    p.inline_q = static_cast<int32_t>(Q);
+    std::memcpy(p.inline_feats, feats, sizeof(float) * Q * h->n_op_feat);
+    std::memcpy(p.inline_row, dev_row, Q);
+  }
   if (s->fresh) {
     // all words at parity 0, all tags at 0
     HB_CUDA_TRY(cudaMemsetAsync(s->base, 0, kScratchBytes, stream));
