@@ -50,6 +50,22 @@ class WaveOut(ctypes.Structure):
         "status", "limits")]
 
 
+class MlpGrid(ctypes.Structure):
+    _fields_ = [("handle", ctypes.c_void_p), ("op_features", ctypes.c_void_p), ("n", ctypes.c_int64),
+                ("device_rows", ctypes.c_void_p), ("n_device_rows", ctypes.c_int32), ("out", ctypes.c_void_p)]
+
+
+class ScaleGrid(ctypes.Structure):
+    _fields_ = [("run_time_ms", ctypes.c_void_p), ("pred", ctypes.c_void_p), ("n", ctypes.c_int64),
+                ("n_destinations", ctypes.c_int32), ("out_ms", ctypes.c_void_p),
+                ("negative_count", ctypes.c_void_p)]
+
+
+class IterationKind(ctypes.Structure):
+    _fields_ = [("run_time_ms", ctypes.c_void_p), ("pred", ctypes.c_void_p), ("offsets", ctypes.c_void_p),
+                ("n", ctypes.c_int64)]
+
+
 class HabitatNativeError(RuntimeError):
     def __init__(self, status, message):
         super().__init__("habitat_b200 native call failed (status %d): %s" % (status, message))
@@ -88,6 +104,16 @@ EXPORTS = {
     "hb_mlp_predict": (ctypes.c_int32, [
         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
         ctypes.c_void_p]),
+    "hb_mlp_predict_grid": (ctypes.c_int32, [ctypes.POINTER(MlpGrid), ctypes.c_int32, ctypes.c_void_p]),
+    "hb_mlp_poll_status": (ctypes.c_int32, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int32)]),
+    "hb_segment_sum_planes": (ctypes.c_int32, [
+        ctypes.c_void_p, ctypes.c_int64, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
+        ctypes.c_void_p]),
+    "hb_iteration_totals": (ctypes.c_int32, [
+        ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64,
+        ctypes.c_int32, ctypes.c_void_p, ctypes.POINTER(IterationKind), ctypes.c_int32, ctypes.c_void_p,
+        ctypes.c_void_p]),
+    "hb_special_scale_grid": (ctypes.c_int32, [ctypes.POINTER(ScaleGrid), ctypes.c_int32, ctypes.c_void_p]),
     "hb_mlp_status": (ctypes.c_int32, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int32)]),
     "hb_mlp_phase_cycles": (ctypes.c_int32, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int64)]),
     "hb_mlp_predict_host": (ctypes.c_int32, [

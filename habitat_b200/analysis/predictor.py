@@ -16,16 +16,17 @@ import os
 import numpy as np
 import torch
 
-from habitat_b200 import batched
+from habitat_b200 import _native
 from habitat_b200.analysis import SPECIAL_OPERATIONS
-from habitat_b200.analysis.kernels import PredictedKernel
+from habitat_b200.analysis.kernels import MeasuredKernel, PredictedKernel
 from habitat_b200.analysis.mlp.mlp import RuntimePredictor
-from habitat_b200.analysis.operation import PredictedOperation
-from habitat_b200.analysis.run_time import RunTimePrediction, RunTimePurePrediction
+from habitat_b200.analysis.operation import MeasuredOperation, PredictedOperation
+from habitat_b200.analysis.run_time import RunTimeMeasurement, RunTimePrediction, RunTimePurePrediction
 from habitat_b200.analysis.wave_scaling import batch as wave_batch
 from habitat_b200.analysis.wave_scaling.metadata import MetadataManager
 from habitat_b200.analysis.wave_scaling.unified import unified_wave_scaling
 from habitat_b200.data import path_to_data
+from habitat_b200.habitat_cuda import KernelInstance
 from habitat_b200.utils import name_all_arguments
 
 logger = logging.getLogger(__name__)
@@ -152,15 +153,57 @@ class _LazyRunTimePrediction(RunTimePrediction):
         return self._predicted_kernels
 
 
+_METRIC_KEYS = tuple((m, m.value.cupti_name, m.value.legacy_cupti_name) for m in wave_batch._NEEDED)
+_FAST_KINDS = {"conv2d": 0, "linear": 1, "bmm": 2}       # feature_rows of the native binding
+
+
+def _trace_types():
+    return MeasuredOperation, RunTimeMeasurement, MeasuredKernel, KernelInstance
+
+
 class _GroupPlan:
     """Everything about the operations of one origin device that does not depend on the
     destination: which operation is predicted how, the flattened kernels of the wave-scaled
     passes, launch overheads, MLP feature matrices.  Built by the first prediction of a trace
     and kept with it."""
 
-    def __init__(self, operations, indices, mode):
-        self.indices = np.asarray(indices, np.int64)
+    def __init__(self, operations, indices, mode, flat=None):
         self.mode = mode
+        self.mlp_inputs = {}      # op kind -> (features, measured ms) on the GPU, measured ms; filled on first use
+        self._layout = None
+        if flat is None:
+            self._flatten(operations, indices, mode)
+        else:
+            self._take(operations, flat)
+        self.bwd_has = np.flatnonzero(self.bwd_run >= 0)
+        self.bwd_of = self.bwd_run[self.bwd_has]
+
+    @classmethod
+    def of_whole_trace(cls, operations, mode):
+        """The plan of a trace recorded on one device, walked by the native binding; None when the
+        operations are not all of this package's ordinary classes (any object with their surface
+        takes the Python walk), or when a missing metric has to raise (the roofline strategy)."""
+        if mode == wave_batch.ROOFLINE:
+            return None
+        flat = _native.binding().flatten_trace(operations, _trace_types(), SPECIAL_OPERATIONS, _MLP_OPS, _METRIC_KEYS,
+                                               mode != wave_batch.RESIMPLIFIED)
+        return cls(operations, None, mode, flat) if flat is not None else None
+
+    def _take(self, operations, flat):
+        (self.kernels, self.runs, names, wave_idx, fwd, bwd, offsets, overheads, kind_idx, self.passthrough_idx,
+         records, metrics, self.offsets_dev) = flat
+        self.indices = None                      # all operations
+        self.wave_idx, self.fwd_run, self.bwd_run, self.offsets = (
+            np.frombuffer(x, np.int64) for x in (wave_idx, fwd, bwd, offsets))
+        self.overheads = np.frombuffer(overheads, np.float64)
+        self.mlp_idx = dict(zip(_MLP_OPS, kind_idx))
+        for i in self.passthrough_idx:
+            logger.warning("Unhandled special operation: %s", operations[i].name)
+        self.flat = (wave_batch.FlatKernels.from_device(self.mode, names, records, metrics) if self.kernels
+                     else None)
+
+    def _flatten(self, operations, indices, mode):
+        self.indices = np.asarray(indices, np.int64)
         wave_idx, fwd_run, bwd_run, runs = [], [], [], []
         self.mlp_idx = {op: [] for op in _MLP_OPS}
         self.passthrough_idx = []
@@ -198,8 +241,38 @@ class _GroupPlan:
         per_run = np.where(self.offsets[1:] > self.offsets[:-1], per_run, 0.0) if runs else per_run
         wall_ns = np.array([run.run_time_ms for run in runs], np.float64) * 1e6
         self.overheads = np.maximum(wall_ns - per_run, 0.0)
-        self.offsets_dev = None
-        self.mlp_inputs = {}      # op kind -> (feature matrix, measured ms), filled on first use
+        self.offsets_dev = torch.from_numpy(self.offsets).cuda() if self.flat is not None else None
+
+    def layout(self, n):
+        """(kind, a, b) of the n operations of the trace for a destination that predicts this group
+        alone, shared by every such destination (PredictedOperations)."""
+        if self._layout is None:
+            kind, a, b = np.zeros(n, np.int8), np.full(n, -1, np.int64), np.full(n, -1, np.int64)
+            kind[self.wave_idx] = 1
+            a[self.wave_idx], b[self.wave_idx] = self.fwd_run, self.bwd_run
+            for idx in self.mlp_idx.values():
+                kind[idx] = 2
+            kind[self.passthrough_idx] = 3
+            self._layout = kind, a, b
+        return self._layout
+
+    def special_inputs(self, name, operations, order):
+        """Features and measured times of the operations of one MLP kind, on the GPU."""
+        got = self.mlp_inputs.get(name)
+        if got is None:
+            idx = self.mlp_idx[name]
+            if name in _FAST_KINDS:
+                columns = _FAST_ROWS[name][2]
+                got = _native.binding().feature_rows(_FAST_KINDS[name], operations, idx,
+                                                     tuple(columns.index(f) for f in order), _trace_types())
+                if got is not None:
+                    got = got[0], got[1], np.frombuffer(got[2], np.float32)
+            if got is None:
+                ops = [operations[i] for i in idx]
+                rt = np.array([op.run_time_ms for op in ops], np.float32)
+                got = torch.from_numpy(feature_matrix(name, ops, order)).cuda(), torch.from_numpy(rt).cuda(), rt
+            self.mlp_inputs[name] = got
+        return got
 
 
 class PredictedOperations(collections.abc.Sequence):
@@ -208,18 +281,23 @@ class PredictedOperations(collections.abc.Sequence):
     PredictedKernel objects are created when an element is first touched, the per-operation
     times (`run_times_ms`) and their sum (`total_run_time_ms`) are there from the start."""
 
-    def __init__(self, operations, dest):
+    def __init__(self, operations, dest, group=None, layout=None, run_times_ms=None):
         self._operations = operations
         self._dest = dest
-        n = len(operations)
-        self._made = [None] * n
-        self._kind = np.zeros(n, np.int8)       # 0 as measured, 1 wave-scaled, 2 MLP, 3 special passed through
-        self._group = np.zeros(n, np.int32)
-        self._a = np.full(n, -1, np.int64)      # wave: forward run; MLP: position in the group's ms array
-        self._b = np.full(n, -1, np.int64)      # wave: backward run or -1
-        self._groups = []                       # per origin group: dict(plan, times, totals, ms)
-        self.run_times_ms = np.zeros(n, np.float64)
+        self._made = None                           # elements, once one has been touched
+        self._groups = [group] if group else []     # per origin group: dict(plan, times, totals)
         self._total = None
+        self._group = None                          # which group an operation is of; None: the first
+        n = len(operations)
+        if layout is not None:
+            self._kind, self._a, self._b = layout
+            self.run_times_ms = run_times_ms
+        else:
+            self._kind = np.zeros(n, np.int8)       # 0 as measured, 1 wave-scaled, 2 MLP, 3 special passed through
+            self._a = np.full(n, -1, np.int64)      # wave: forward run
+            self._b = np.full(n, -1, np.int64)      # wave: backward run or -1
+            self._group = np.zeros(n, np.int32)
+            self.run_times_ms = np.zeros(n, np.float64)
 
     def __len__(self):
         return len(self._operations)
@@ -229,6 +307,8 @@ class PredictedOperations(collections.abc.Sequence):
             return [self[j] for j in range(*i.indices(len(self)))]
         if i < 0:
             i += len(self)
+        if self._made is None:
+            self._made = [None] * len(self._operations)
         made = self._made[i]
         if made is None:
             made = self._made[i] = self._make(i)
@@ -247,7 +327,7 @@ class PredictedOperations(collections.abc.Sequence):
             return op
         if kind == 3:
             return PredictedOperation(op, op.forward, op.backward, self._dest)
-        g = self._groups[self._group[i]]
+        g = self._groups[self._group[i] if self._group is not None else 0]
         if kind == 2:
             return PredictedOperation(op, RunTimePurePrediction(float(self.run_times_ms[i]), self._dest),
                                       None, self._dest)
@@ -313,6 +393,9 @@ class Predictor:
         records, overheads, MLP features) is stored there and reused by later calls."""
         if not isinstance(operations, (list, tuple)):
             operations = list(operations)
+        whole = self._predict_whole(operations, dest_devices, cache)
+        if whole is not None:
+            return whole
         D = len(dest_devices)
         results = [PredictedOperations(operations, dest) for dest in dest_devices]
         key = ("origins", len(operations))
@@ -335,18 +418,54 @@ class Predictor:
                 self._predict_group(operations, indices, origin, dest_devices, targets, results, cache)
         return results
 
+    def _predict_whole(self, operations, dest_devices, cache):
+        """predict_trace for a trace recorded on one device and predicted for others (what a Trace
+        is); None for anything else."""
+        if not operations or not dest_devices:
+            return None
+        mode = getattr(self._wave_scaling_strategy, "batch_mode", None)
+        origin = operations[0].device
+        key = ("whole", mode, len(operations))
+        plan = cache.get(key) if cache is not None else None
+        if plan is None:
+            if mode is None or any(d.name == origin.name for d in dest_devices):
+                return None
+            plan = _GroupPlan.of_whole_trace(operations, mode)
+            if plan is None:
+                return None
+            if cache is not None:
+                cache[key] = plan
+        elif mode is None or any(d.name == origin.name for d in dest_devices):
+            return None
+        n = len(operations)
+        times, totals, special = self._run_plan(plan, operations, origin, dest_devices)
+        run_ms = (plan.overheads + totals) / 1e6                             # [T, runs]
+        ms = np.empty((len(dest_devices), n), np.float64)
+        if len(plan.wave_idx):
+            wave_ms = run_ms[:, plan.fwd_run]
+            wave_ms[:, plan.bwd_has] += run_ms[:, plan.bwd_of]
+            ms[:, plan.wave_idx] = wave_ms
+        for name, pred_ms in special.items():
+            ms[:, plan.mlp_idx[name]] = pred_ms
+        for i in plan.passthrough_idx:
+            ms[:, i] = operations[i].run_time_ms
+        layout = plan.layout(n)
+        return [PredictedOperations(operations, dest, dict(plan=plan, times=times[t], totals=totals[t]), layout, ms[t])
+                for t, dest in enumerate(dest_devices)]
+
     # ------------------------------------------------------------------
     def _predict_group(self, operations, indices, origin, dest_devices, targets, results, cache=None):
         dests = [dest_devices[d] for d in targets]
         mode = getattr(self._wave_scaling_strategy, "batch_mode", None)
-        key = ("plan", origin.name, mode, len(indices))
+        whole = len(indices) == len(operations)
+        key = ("whole", mode, len(operations)) if whole else ("plan", origin.name, mode, len(indices))
         plan = cache.get(key) if cache is not None else None
         if plan is None:
-            plan = _GroupPlan(operations, indices, mode)
+            plan = _GroupPlan.of_whole_trace(operations, mode) if whole and mode is not None else None
+            plan = plan or _GroupPlan(operations, indices, mode)
             if cache is not None:
                 cache[key] = plan
-        T = len(dests)
-        times, totals = self._wave_scale_plan(plan, origin, dests)
+        times, totals, special = self._run_plan(plan, operations, origin, dests)
         run_ms = (plan.overheads[None, :] + totals) / 1e6                    # [T, runs]
         for t, d in enumerate(targets):
             res = results[d]
@@ -358,69 +477,69 @@ class Predictor:
                 res._a[plan.wave_idx] = plan.fwd_run
                 res._b[plan.wave_idx] = plan.bwd_run
                 ms = run_ms[t][plan.fwd_run]
-                has_bwd = plan.bwd_run >= 0
-                ms = ms + np.where(has_bwd, run_ms[t][np.maximum(plan.bwd_run, 0)], 0.0)
+                ms[plan.bwd_has] += run_ms[t][plan.bwd_of]
                 res.run_times_ms[plan.wave_idx] = ms
             for i in plan.passthrough_idx:
                 res._kind[i] = 3
                 res.run_times_ms[i] = operations[i].run_time_ms
-        for name, idx in plan.mlp_idx.items():
-            if not idx:
-                continue
-            ms = self._special_scale_ops(name, [operations[i] for i in idx], origin, dests, plan)
-            idx = np.asarray(idx, np.int64)
-            for t, d in enumerate(targets):
-                res = results[d]
+            for name, ms in special.items():
+                idx = np.asarray(plan.mlp_idx[name], np.int64)
                 res._kind[idx] = 2
                 res.run_times_ms[idx] = ms[t]
 
-    def _wave_scale_plan(self, plan, origin, dests):
-        """-> (scaled kernel times [T, K], per-pass kernel totals [T, runs]) on the host, float64
-        (predictor.py:111-130 of the reference for every pass and destination at once)."""
+    def _run_plan(self, plan, operations, origin, dests):
+        """One prediction of a flattened group: -> (scaled kernel times [T, K], per-pass kernel totals
+        [T, runs], predicted ms [T, n] by MLP kind) on the host (predictor.py:111-148 of the reference
+        for every pass, special operation and destination at once)."""
         T, K, n_runs = len(dests), len(plan.kernels), len(plan.runs)
-        if plan.mode is None:
-            # a user-supplied strategy: the reference's per-kernel protocol
+        names = [name for name in _MLP_OPS if plan.mlp_idx[name]]
+        kinds, sizes = [], []
+        for name in names:
+            pred = self._predictor(name)
+            rows = bytes([pred.device_row(origin.name)] + [pred.device_row(d.name) for d in dests])
+            feats, rt, _ = plan.special_inputs(name, operations, pred.model.features)
+            kinds.append((pred._handle._handle.value, feats, rt, rows))
+            sizes.append(len(plan.mlp_idx[name]))
+        own = plan.mode is None                  # a user-supplied strategy: the reference's per-kernel protocol
+        flat = None if own else plan.flat
+        regs = None
+        if flat is not None:
+            regs = wave_batch.destination_registers(plan.kernels, flat.names, dests, self._kernel_metadata)
+        data, nan, clamped = _native.binding().run_group(
+            flat.batch if flat is not None else None, flat.metrics if flat is not None else None, origin, dests, regs,
+            plan.offsets_dev if flat is not None else None, kinds)
+        if nan:
+            wave_batch.raise_zero_wave()
+        at = 0
+
+        def take(count, dtype):
+            nonlocal at
+            part = np.frombuffer(data, dtype, count, at)
+            at = (at + count * part.itemsize + 15) & ~15
+            return part
+        if flat is not None:
+            totals = take(T * n_runs, np.float64).reshape(T, n_runs)
+        special = {}
+        for name, n, seen in zip(names, sizes, clamped):
+            special[name] = take(T * n, np.float32).reshape(T, n)
+            pred_ms = take((T + 1) * n, np.float32)
+            if seen:
+                self._warn_negative(name, plan.mlp_inputs[name][2], pred_ms.astype(np.float64), n, T)
+        if flat is not None:
+            times = take(T * K, np.float32).reshape(T, K)
+        elif own:
             times = np.array([[self._wave_scaling_strategy(k, origin, dest, self._kernel_metadata).run_time_ns
                                for k in plan.kernels] for dest in dests], np.float64).reshape(T, K)
             totals = np.zeros((T, n_runs))
             for r in range(n_runs):
                 totals[:, r] = times[:, plan.offsets[r]:plan.offsets[r + 1]].sum(axis=1)
-            return times, totals
-        if K == 0:
-            return np.zeros((T, 0)), np.zeros((T, n_runs))
-        res = wave_batch.scale_kernels(plan.kernels, origin, dests, self._kernel_metadata, plan.mode,
-                                       flat=plan.flat)
-        if plan.offsets_dev is None:
-            plan.offsets_dev = torch.from_numpy(plan.offsets).cuda()
-        # per-pass kernel-time totals on the device: segment sums over the same offsets
-        sums = torch.stack([batched.segment_sum(res.scaled_ns[t], plan.offsets_dev) for t in range(T)])
-        scaled = res.scaled_ns.cpu().numpy()
-        wave_batch.raise_like_reference(scaled)
-        return scaled, sums.cpu().numpy()
+        else:
+            times, totals = np.zeros((T, 0)), np.zeros((T, n_runs))
+        return times, totals, special
 
-    def _special_scale_ops(self, name, ops, origin, dests, plan=None):
-        """-> [T, n] predicted ms (predictor.py:132-148 and the *_scale methods)."""
-        pred = self._predictor(name)
-        order = pred.model.features
-        cached = plan.mlp_inputs.get(name) if plan is not None else None
-        if cached is None:
-            cached = (feature_matrix(name, ops, order), np.array([op.run_time_ms for op in ops], np.float32))
-            if plan is not None:
-                plan.mlp_inputs[name] = cached
-        feats, rt_host = cached
-        n, T = len(ops), len(dests)
-        rows = [pred.device_row(origin.name)] + [pred.device_row(d.name) for d in dests]
-        f = torch.from_numpy(np.tile(feats, (T + 1, 1))).cuda()
-        r = torch.from_numpy(np.repeat(np.asarray(rows, np.uint8), n)).cuda()
-        p = pred.predict_batch(f, r)                      # [(T + 1) n]: origin first
-        rt = torch.from_numpy(rt_host).cuda()
-        neg = torch.zeros(1, dtype=torch.int32, device="cuda").view(torch.uint32)
-        ms = batched.special_scale(rt.repeat(T), p[n:], p[:n].repeat(T), neg).view(T, n).cpu().numpy()
-        pred._handle.check_status()
-        if int(neg.view(torch.int32).cpu()[0]):
-            ph = p.cpu().numpy().astype(np.float64)
-            for t in range(T):
-                raw = rt_host.astype(np.float64) * ph[(t + 1) * n:(t + 2) * n] / ph[:n]
-                for j in np.nonzero(raw < 0)[0]:
-                    logger.warning("Operation %s predicted run time %.2f ms", name, raw[j])
-        return ms
+    @staticmethod
+    def _warn_negative(name, run_time_ms, pred_ms, n, T):
+        for t in range(T):
+            raw = run_time_ms.astype(np.float64) * pred_ms[(t + 1) * n:(t + 2) * n] / pred_ms[:n]
+            for j in np.nonzero(raw < 0)[0]:
+                logger.warning("Operation %s predicted run time %.2f ms", name, raw[j])

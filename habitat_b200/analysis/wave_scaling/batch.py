@@ -74,6 +74,15 @@ class FlatKernels:
     prediction of the same trace (other destinations, another strategy argument) reuses
     instead of walking the kernel objects again."""
 
+    @classmethod
+    def from_device(cls, mode, names, records, metrics):
+        """From CUDA tensors in the order of KernelBatch's and KernelMetricsBatch's fields."""
+        self = cls.__new__(cls)
+        self.mode, self.names, self.count = mode, names, len(names)
+        self.batch = batched.KernelBatch(*records)
+        self.metrics = batched.KernelMetricsBatch(*metrics) if metrics is not None else None
+        return self
+
     def __init__(self, kernels, mode):
         arrays, metrics, self.names = flatten_kernels(kernels, mode)
         self.mode = mode
@@ -95,23 +104,27 @@ def scale_kernels(kernels, origin_device, dest_devices, metadata_manager, mode=U
     Returns a WaveResult whose tensors live on the GPU; nothing is synchronised here."""
     if flat is None or flat.mode != mode or flat.count != len(kernels):
         flat = FlatKernels(kernels, mode)
-    kb, mb, names = flat.batch, flat.metrics, flat.names
-    dest_regs = None
-    if metadata_manager is not None and hasattr(metadata_manager, "registers_matrix"):
+    return batched.wave_scale(flat.batch, origin_device, dest_devices,
+                              dest_regs=destination_registers(kernels, flat.names, dest_devices, metadata_manager),
+                              metrics=flat.metrics)
+
+
+def destination_registers(kernels, names, dest_devices, metadata_manager):
+    """[D, K] int16 CUDA tensor of per-destination register counts (-1: the kernel's own), or None
+    when the register table has nothing to say."""
+    if metadata_manager is None:
+        return None
+    if hasattr(metadata_manager, "registers_matrix"):
         m = metadata_manager.registers_matrix(names, dest_devices)
-        if m is not None:
-            dest_regs = torch.from_numpy(m).cuda()
-    elif metadata_manager is not None:
-        # a foreign manager with only the per-kernel query of the reference
-        m = np.full((len(dest_devices), len(kernels)), -1, np.int16)
-        for d, dev in enumerate(dest_devices):
-            for i, k in enumerate(kernels):
-                r = metadata_manager.kernel_registers_for(k, dev)
-                if r is not None:
-                    m[d, i] = r
-        if (m >= 0).any():
-            dest_regs = torch.from_numpy(m).cuda()
-    return batched.wave_scale(kb, origin_device, dest_devices, dest_regs=dest_regs, metrics=mb)
+        return torch.from_numpy(m).cuda() if m is not None else None
+    # a foreign manager with only the per-kernel query of the reference
+    m = np.full((len(dest_devices), len(kernels)), -1, np.int16)
+    for d, dev in enumerate(dest_devices):
+        for i, k in enumerate(kernels):
+            r = metadata_manager.kernel_registers_for(k, dev)
+            if r is not None:
+                m[d, i] = r
+    return torch.from_numpy(m).cuda() if (m >= 0).any() else None
 
 
 def raise_like_reference(scaled_ns_host):
@@ -119,4 +132,8 @@ def raise_like_reference(scaled_ns_host):
     kernel leaves as NaN (roofline.py:29-45: a kernel the origin cannot run at all, or one
     that fits in an origin wave going to a device that cannot run it)."""
     if np.isnan(scaled_ns_host).any():
-        raise ZeroDivisionError("integer division or modulo by zero")
+        raise_zero_wave()
+
+
+def raise_zero_wave():
+    raise ZeroDivisionError("integer division or modulo by zero")

@@ -8,11 +8,17 @@
 // makes the function return None, and the caller's Python checks then raise the error.
 #include <Python.h>
 
+#include <ATen/EmptyTensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <cuda_runtime_api.h>
+
+#include <cmath>
 #include <cstdint>
+#include <cstring>
+#include <vector>
 
 #include "habitat_b200.h"
 
@@ -28,6 +34,11 @@ struct Api {
   decltype(&hb_group_sum) group_sum = nullptr;
   decltype(&hb_plane_sum) plane_sum = nullptr;
   decltype(&hb_segment_sum) segment_sum = nullptr;
+  decltype(&hb_segment_sum_planes) segment_sum_planes = nullptr;
+  decltype(&hb_mlp_predict_grid) mlp_predict_grid = nullptr;
+  decltype(&hb_mlp_poll_status) mlp_poll_status = nullptr;
+  decltype(&hb_special_scale_grid) special_scale_grid = nullptr;
+  decltype(&hb_iteration_totals) iteration_totals = nullptr;
 } api;
 
 PyObject* g_row_of = nullptr;       // device_table.row_of
@@ -37,7 +48,9 @@ long g_generation = 0;              // of the device table; tokens of an older o
 
 PyObject *s_num_blocks, *s_block_size, *s_regs, *s_smem, *s_time, *s_gamma, *s_row_token, *s_flop, *s_rd, *s_wr,
     *s_has, *s_scaled, *s_docc, *s_dwav, *s_oocc, *s_owav, *s_status, *s_limits, *s_buffer, *s_K, *s_D, *s_per_plane,
-    *s_n_planes;
+    *s_n_planes, *s__name, *s__device, *s__forward, *s__backward, *s__arguments, *s_args, *s_kwargs, *s__kernels,
+    *s__run_time_ms, *s__c, *s__metrics_kernels, *s__cached_metrics, *s__metrics, *s__num_blocks, *s__block_size,
+    *s__regs, *s__smem_static, *s__smem_dynamic, *s__run_time_ns, *s_name;
 
 // A reference that is dropped at the end of the scope.
 struct Ref {
@@ -381,6 +394,549 @@ PyObject* segment_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// ---------------------------------------------------------------------------
+// Traces (habitat_b200/analysis/predictor.py): the walk over recorded objects, and one prediction
+// ---------------------------------------------------------------------------
+// Attribute of an instance, new reference; null (with an error set) when it has none.
+inline PyObject* get(PyObject* o, PyObject* name) { return PyObject_GetAttr(o, name); }
+// The integer attribute `name`; *ok is cleared when it is not a 64-bit integer.
+int64_t int_of(PyObject* o, PyObject* name, bool* ok) {
+  Ref v(get(o, name));
+  if (!v.p || !PyLong_Check(v.p)) {
+    *ok = false;
+    return 0;
+  }
+  const int64_t x = PyLong_AsLongLong(v.p);
+  if (x == -1 && PyErr_Occurred()) *ok = false;
+  return x;
+}
+PyObject* bytes_of(const void* p, size_t n) {
+  return PyBytes_FromStringAndSize(static_cast<const char*>(p), static_cast<Py_ssize_t>(n));
+}
+template <typename T>
+PyObject* bytes_of(const std::vector<T>& v) { return bytes_of(v.data(), v.size() * sizeof(T)); }
+// "Not an ordinary trace": the caller takes the general path, which also raises what there is to raise.
+PyObject* not_ordinary() {
+  PyErr_Clear();
+  Py_RETURN_NONE;
+}
+void* stream_now() { return c10::cuda::getCurrentCUDAStream().stream(); }
+
+// Value of metric `which` among a kernel's metric records: 1 found, 0 absent, -1 not ordinary.  Mirrors
+// MeasuredKernel.get_metric for the three metrics of the roofline rule, whose canonical value is the raw one.
+int find_metric(PyObject* records, PyObject* cached, PyObject* metric, PyObject* name, PyObject* legacy,
+                PyTypeObject* instance_type, double* out) {
+  if (PyDict_GET_SIZE(cached) > 0) {
+    PyObject* hit = PyDict_GetItemWithError(cached, metric);   // borrowed
+    if (hit) {
+      *out = PyFloat_AsDouble(hit);
+      return PyErr_Occurred() ? -1 : 1;
+    }
+    if (PyErr_Occurred()) return -1;
+  }
+  const Py_ssize_t n = PyList_GET_SIZE(records);
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject* rec = PyList_GET_ITEM(records, i);
+    if (Py_TYPE(rec) != instance_type) return -1;
+    Ref list(get(rec, s__metrics));
+    if (!list.p || !PyList_Check(list.p)) return -1;
+    for (Py_ssize_t j = 0; j < PyList_GET_SIZE(list.p); ++j) {
+      PyObject* pair = PyList_GET_ITEM(list.p, j);
+      if (!PyTuple_Check(pair) || PyTuple_GET_SIZE(pair) != 2) return -1;
+      PyObject* key = PyTuple_GET_ITEM(pair, 0);
+      if (key != name && key != legacy) {
+        if (!PyUnicode_Check(key)) return -1;
+        if (PyUnicode_Compare(key, name) != 0 && PyUnicode_Compare(key, legacy) != 0) continue;
+      }
+      *out = PyFloat_AsDouble(PyTuple_GET_ITEM(pair, 1));
+      return PyErr_Occurred() ? -1 : 1;
+    }
+  }
+  return 0;
+}
+
+// flatten_trace(operations, (MeasuredOperation, RunTimeMeasurement, MeasuredKernel, KernelInstance),
+//               special names, MLP kinds, metrics ((Metric, name, legacy name) x 3), with_metrics)
+// -> None when the operations are not all of those very classes or not of one device, else
+//    (kernels, runs, names, wave_idx, fwd_run, bwd_run, offsets, overheads: bytes of int64 / float64,
+//     [indices per MLP kind], passed-through indices,
+//     (num_blocks, block_size, regs, smem, time, gamma), (eff, read, write, has) or None, offsets: CUDA tensors)
+PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  if (n_args != 6) return not_ordinary();
+  Ref ops(PySequence_Fast(a[0], "operations must be a sequence"));
+  if (!ops.p) return nullptr;
+  PyTypeObject* type[4];
+  for (int i = 0; i < 4; ++i) type[i] = reinterpret_cast<PyTypeObject*>(PyTuple_GET_ITEM(a[1], i));
+  PyObject *special = a[2], *kinds = a[3], *metrics = a[4];
+  const bool with_metrics = PyObject_IsTrue(a[5]) == 1;
+  const Py_ssize_t n = PySequence_Fast_GET_SIZE(ops.p), n_kinds = PyTuple_GET_SIZE(kinds);
+
+  Ref kernels(PyList_New(0)), runs(PyList_New(0)), names(PyList_New(0)), passed(PyList_New(0));
+  Ref kind_idx(PyList_New(n_kinds));
+  for (Py_ssize_t k = 0; k < n_kinds; ++k) PyList_SET_ITEM(kind_idx.p, k, PyList_New(0));
+  std::vector<int64_t> wave_idx, fwd, bwd, offsets{0};
+  std::vector<double> overhead, eff, rd, wr;
+  std::vector<int32_t> nb;
+  std::vector<uint16_t> bs, rg;
+  std::vector<uint32_t> sm;
+  std::vector<float> tm;
+  std::vector<uint8_t> has;
+  bool any_metrics = false;
+  Ref first_device(nullptr);
+
+  auto add_run = [&](PyObject* run) -> bool {
+    if (Py_TYPE(run) != type[1]) return false;
+    Ref list(get(run, s__kernels)), ms(get(run, s__run_time_ms));
+    if (!list.p || !ms.p || (!PyList_Check(list.p) && !PyTuple_Check(list.p))) return false;
+    const double wall = PyFloat_AsDouble(ms.p);
+    if (PyErr_Occurred()) return false;
+    double busy = 0.0;
+    const Py_ssize_t count = PySequence_Fast_GET_SIZE(list.p);
+    for (Py_ssize_t i = 0; i < count; ++i) {
+      PyObject* k = PySequence_Fast_GET_ITEM(list.p, i);
+      if (Py_TYPE(k) != type[2]) return false;
+      Ref c(get(k, s__c));
+      if (!c.p || Py_TYPE(c.p) != type[3]) return false;
+      bool ok = true;
+      const int64_t blocks = int_of(c.p, s__num_blocks, &ok), block = int_of(c.p, s__block_size, &ok),
+                    regs = int_of(c.p, s__regs, &ok), time = int_of(c.p, s__run_time_ns, &ok),
+                    stat = int_of(c.p, s__smem_static, &ok), dyn = int_of(c.p, s__smem_dynamic, &ok);
+      Ref name(get(c.p, s__name));
+      if (!ok || !name.p || blocks != static_cast<int32_t>(blocks)) return false;
+      const int64_t smem = stat + dyn;
+      nb.push_back(static_cast<int32_t>(blocks));
+      bs.push_back(static_cast<uint16_t>(block < 0 ? 0 : (block > 0xFFFF ? 0xFFFF : block)));
+      rg.push_back(static_cast<uint16_t>(regs & 0xFFFF));
+      sm.push_back(smem >= 0 && smem <= 0xFFFFFFFFll ? static_cast<uint32_t>(smem) : 0xFFFFFFFFu);
+      tm.push_back(static_cast<float>(static_cast<double>(time)));
+      busy += static_cast<double>(time);
+      if (PyList_Append(kernels.p, k) < 0 || PyList_Append(names.p, name.p) < 0) return false;
+      if (with_metrics) {
+        Ref records(get(k, s__metrics_kernels)), cached(get(k, s__cached_metrics));
+        if (!records.p || !cached.p || !PyList_Check(records.p) || !PyDict_Check(cached.p)) return false;
+        double v[3] = {0.0, 0.0, 0.0};
+        int found = PyList_GET_SIZE(records.p) > 0 || PyDict_GET_SIZE(cached.p) > 0 ? 1 : 0;
+        for (int m = 0; m < 3 && found == 1; ++m) {
+          PyObject* t = PyTuple_GET_ITEM(metrics, m);
+          found = find_metric(records.p, cached.p, PyTuple_GET_ITEM(t, 0), PyTuple_GET_ITEM(t, 1),
+                              PyTuple_GET_ITEM(t, 2), type[3], &v[m]);
+        }
+        if (found < 0) return false;
+        eff.push_back(found ? v[0] : 0.0);
+        rd.push_back(found ? v[1] : 0.0);
+        wr.push_back(found ? v[2] : 0.0);
+        has.push_back(static_cast<uint8_t>(found));
+        any_metrics = any_metrics || found;
+      }
+    }
+    offsets.push_back(static_cast<int64_t>(nb.size()));
+    // launch overhead of a pass (predictor.py:113-116 of the reference): wall time minus kernel time
+    const double rest = wall * 1e6 - busy;
+    overhead.push_back(rest > 0.0 ? rest : 0.0);
+    return PyList_Append(runs.p, run) == 0;
+  };
+
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject* op = PySequence_Fast_GET_ITEM(ops.p, i);
+    if (Py_TYPE(op) != type[0]) return not_ordinary();
+    Ref name(get(op, s__name)), device(get(op, s__device));
+    if (!name.p || !device.p) return not_ordinary();
+    if (!first_device.p) {
+      first_device.p = Py_NewRef(device.p);
+    } else if (device.p != first_device.p) {
+      Ref x(get(device.p, s_name)), y(get(first_device.p, s_name));
+      if (!x.p || !y.p || PyObject_RichCompareBool(x.p, y.p, Py_EQ) != 1) return not_ordinary();
+    }
+    const int is_special = PySet_Contains(special, name.p);
+    if (is_special < 0) return not_ordinary();
+    if (!is_special) {
+      Ref f(get(op, s__forward)), b(get(op, s__backward));
+      if (!f.p || !b.p) return not_ordinary();
+      wave_idx.push_back(i);
+      fwd.push_back(static_cast<int64_t>(overhead.size()));
+      if (!add_run(f.p)) return not_ordinary();
+      bwd.push_back(b.p == Py_None ? -1 : static_cast<int64_t>(overhead.size()));
+      if (b.p != Py_None && !add_run(b.p)) return not_ordinary();
+      continue;
+    }
+    Py_ssize_t kind = 0;
+    while (kind < n_kinds && PyObject_RichCompareBool(PyTuple_GET_ITEM(kinds, kind), name.p, Py_EQ) != 1) ++kind;
+    Ref at(PyLong_FromSsize_t(i));
+    if (PyList_Append(kind < n_kinds ? PyList_GET_ITEM(kind_idx.p, kind) : passed.p, at.p) < 0) return nullptr;
+  }
+  if (PyErr_Occurred()) return not_ordinary();
+
+  // one upload for the records, the metrics and the pass boundaries
+  Ref soa(Py_NewRef(Py_None)), met(Py_NewRef(Py_None)), off(Py_NewRef(Py_None));
+  const int64_t K = static_cast<int64_t>(nb.size());
+  if (K > 0) {
+    std::vector<uint8_t> host;
+    struct Piece { size_t at; int64_t count; at::ScalarType type; };
+    std::vector<Piece> pieces;
+    auto put = [&](const void* p, int64_t count, size_t size, at::ScalarType t) {
+      const size_t at0 = (host.size() + 255) & ~static_cast<size_t>(255);
+      host.resize(at0 + count * size);
+      std::memcpy(host.data() + at0, p, count * size);
+      pieces.push_back(Piece{at0, count, t});
+    };
+    const std::vector<float> gamma(nb.size(), 1.0f);
+    put(nb.data(), K, 4, at::kInt);
+    put(bs.data(), K, 2, at::kUInt16);
+    put(rg.data(), K, 2, at::kUInt16);
+    put(sm.data(), K, 4, at::kUInt32);
+    put(tm.data(), K, 4, at::kFloat);
+    put(gamma.data(), K, 4, at::kFloat);
+    put(offsets.data(), static_cast<int64_t>(offsets.size()), 8, at::kLong);
+    if (any_metrics) {
+      put(eff.data(), K, 8, at::kDouble);
+      put(rd.data(), K, 8, at::kDouble);
+      put(wr.data(), K, 8, at::kDouble);
+      put(has.data(), K, 1, at::kByte);
+    }
+    const int64_t total[1] = {static_cast<int64_t>(host.size())};
+    int current = 0;
+    cudaGetDevice(&current);
+    at::Tensor block = empty(total, at::kByte, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(current)));
+    const cudaError_t e = cudaMemcpyAsync(block.mutable_data_ptr(), host.data(), host.size(), cudaMemcpyHostToDevice,
+                                          static_cast<cudaStream_t>(stream_now()));
+    if (e != cudaSuccess) {
+      PyErr_Format(PyExc_RuntimeError, "upload of the trace: %s", cudaGetErrorString(e));
+      return nullptr;
+    }
+    auto view = [&](size_t i) {
+      const int64_t size[1] = {pieces[i].count};
+      return THPVariable_Wrap(inside(block, pieces[i].at, size, pieces[i].type));
+    };
+    Py_SETREF(soa.p, Py_BuildValue("(NNNNNN)", view(0), view(1), view(2), view(3), view(4), view(5)));
+    Py_SETREF(off.p, view(6));
+    if (any_metrics) Py_SETREF(met.p, Py_BuildValue("(NNNN)", view(7), view(8), view(9), view(10)));
+    if (!soa.p || !off.p || !met.p) return nullptr;
+  }
+  return Py_BuildValue("(OOONNNNNOOOOO)", kernels.p, runs.p, names.p, bytes_of(wave_idx), bytes_of(fwd), bytes_of(bwd),
+                       bytes_of(offsets), bytes_of(overhead), kind_idx.p, passed.p, soa.p, met.p, off.p);
+  END_HANDLE_TH_ERRORS
+}
+
+// Element i of a tuple or list as a double (borrowed access); *ok is cleared when it is no number.
+double item(PyObject* seq, Py_ssize_t i, bool* ok) {
+  if (!*ok || (!PyTuple_Check(seq) && !PyList_Check(seq)) || i >= PySequence_Fast_GET_SIZE(seq)) {
+    *ok = false;
+    return 0.0;
+  }
+  const double v = PyFloat_AsDouble(PySequence_Fast_GET_ITEM(seq, i));
+  if (v == -1.0 && PyErr_Occurred()) *ok = false;
+  return v;
+}
+
+// feature_rows(kind, operations, indices, column order, (MeasuredOperation, RunTimeMeasurement, ...))
+// -> None when an operation is not recorded positionally, else ([n][F] float32 features, [n] float32 measured
+// ms) as CUDA tensors, and the measured ms as bytes.  The rows are those of predictor.py:150-232 of the
+// reference; kind 0 conv2d, 1 linear, 2 bmm.
+PyObject* feature_rows(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  if (n_args != 5) return not_ordinary();
+  const long kind = PyLong_AsLong(a[0]);
+  Ref ops(PySequence_Fast(a[1], "operations must be a sequence"));
+  if (!ops.p || !PyList_Check(a[2]) || !PyTuple_Check(a[3]) || kind < 0 || kind > 2) return not_ordinary();
+  PyTypeObject* op_type = reinterpret_cast<PyTypeObject*>(PyTuple_GET_ITEM(a[4], 0));
+  PyTypeObject* run_type = reinterpret_cast<PyTypeObject*>(PyTuple_GET_ITEM(a[4], 1));
+  const Py_ssize_t n = PyList_GET_SIZE(a[2]), F = PyTuple_GET_SIZE(a[3]);
+  static const Py_ssize_t kArity[3] = {5, 3, 2}, kColumns[3] = {8, 4, 4};
+  if (F > 8) return not_ordinary();
+  long order[8];
+  for (Py_ssize_t c = 0; c < F; ++c) {
+    order[c] = PyLong_AsLong(PyTuple_GET_ITEM(a[3], c));
+    if (order[c] < 0 || order[c] >= kColumns[kind]) return not_ordinary();
+  }
+  std::vector<float> host(static_cast<size_t>(n) * F + n);
+  float* ms = host.data() + static_cast<size_t>(n) * F;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject* op = PySequence_Fast_GET_ITEM(ops.p, PyLong_AsSsize_t(PyList_GET_ITEM(a[2], i)));
+    if (Py_TYPE(op) != op_type) return not_ordinary();
+    Ref arg(get(op, s__arguments)), f(get(op, s__forward)), b(get(op, s__backward));
+    if (!arg.p || !f.p || !b.p || arg.p == Py_None) return not_ordinary();
+    Ref args(get(arg.p, s_args)), kwargs(get(arg.p, s_kwargs));
+    if (!args.p || !kwargs.p || !PyTuple_Check(args.p) || !PyDict_Check(kwargs.p) || PyDict_GET_SIZE(kwargs.p) != 0 ||
+        PyTuple_GET_SIZE(args.p) < kArity[kind])
+      return not_ordinary();
+    PyObject *x = PyTuple_GET_ITEM(args.p, 0), *w = PyTuple_GET_ITEM(args.p, 1);
+    bool ok = true;
+    double v[8] = {};
+    if (kind == 0) {
+      auto first = [&](PyObject* o) {
+        if (PyTuple_Check(o)) return item(o, 0, &ok);
+        const double d = PyFloat_AsDouble(o);
+        if (d == -1.0 && PyErr_Occurred()) ok = false;
+        return d;
+      };
+      v[0] = item(x, 0, &ok); v[1] = item(x, 2, &ok); v[2] = item(x, 1, &ok); v[3] = item(w, 0, &ok);
+      v[4] = item(w, 2, &ok);
+      v[5] = first(PyTuple_GET_ITEM(args.p, 3));
+      v[6] = first(PyTuple_GET_ITEM(args.p, 4));
+      v[7] = PyTuple_GET_ITEM(args.p, 2) == Py_None ? 0.0 : 1.0;
+    } else if (kind == 1) {
+      v[0] = 1.0;
+      const Py_ssize_t dims = PyTuple_Check(x) || PyList_Check(x) ? PySequence_Fast_GET_SIZE(x) : 0;
+      if (dims == 0) return not_ordinary();
+      for (Py_ssize_t d = 0; d + 1 < dims; ++d) v[0] *= item(x, d, &ok);
+      v[1] = item(w, 1, &ok);
+      v[2] = item(w, 0, &ok);
+      v[3] = PyTuple_GET_ITEM(args.p, 2) == Py_None ? 0.0 : 1.0;
+    } else {
+      v[0] = item(x, 0, &ok); v[1] = item(x, 1, &ok); v[2] = item(x, 2, &ok); v[3] = item(w, 2, &ok);
+    }
+    double run = 0.0;
+    for (PyObject* r : {f.p, b.p}) {
+      if (r == Py_None) continue;
+      if (Py_TYPE(r) != run_type) return not_ordinary();
+      Ref t(get(r, s__run_time_ms));
+      run += t.p ? PyFloat_AsDouble(t.p) : 0.0;
+      if (PyErr_Occurred()) return not_ordinary();
+    }
+    if (!ok) return not_ordinary();
+    for (Py_ssize_t c = 0; c < F; ++c) host[i * F + c] = static_cast<float>(v[order[c]]);
+    ms[i] = static_cast<float>(run);
+  }
+  int current = 0;
+  cudaGetDevice(&current);
+  const int64_t total[1] = {static_cast<int64_t>(host.size() * 4)}, nf[2] = {n, F}, n1[1] = {n};
+  at::Tensor block = empty(total, at::kByte, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(current)));
+  const cudaError_t e = cudaMemcpyAsync(block.mutable_data_ptr(), host.data(), host.size() * 4, cudaMemcpyHostToDevice,
+                                        static_cast<cudaStream_t>(stream_now()));
+  if (e != cudaSuccess) {
+    PyErr_Format(PyExc_RuntimeError, "upload of the features: %s", cudaGetErrorString(e));
+    return nullptr;
+  }
+  return Py_BuildValue("(NNN)", THPVariable_Wrap(inside(block, 0, nf, at::kFloat)),
+                       THPVariable_Wrap(inside(block, static_cast<size_t>(n) * F * 4, n1, at::kFloat)),
+                       bytes_of(ms, static_cast<size_t>(n) * 4));
+  END_HANDLE_TH_ERRORS
+}
+
+// run_group(kernels or None, metrics or None, origin, dests, dest_regs or None, offsets or None,
+//           [(handle address, features, measured ms, device rows (bytes: origin, then the destinations))])
+// -> (bytes, NaN seen, [a clamped prediction seen per kind]).  The bytes hold, each part on a 16-byte
+// boundary: [T][passes] float64 kernel-time totals, per kind [T][n] float32 ms and [1 + T][n] float32
+// predictions, [T][K] float32 scaled times.  One prediction of a flattened trace: wave scaling, the sums of
+// its passes, the MLPs of all kinds side by side, their ratios; one download, one wait.
+PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  if (n_args != 7 || !PyList_Check(a[6])) {
+    PyErr_SetString(PyExc_TypeError, "run_group: bad arguments");
+    return nullptr;
+  }
+  Ref dests(PySequence_Fast(a[3], "dests must be a sequence of DeviceProperties"));
+  if (!dests.p) return nullptr;
+  const int64_t T = PySequence_Fast_GET_SIZE(dests.p);
+  int64_t K = 0, n_runs = 0;
+  const at::Tensor* off = nullptr;
+  if (a[5] != Py_None) {
+    off = tensor(a[5], at::kLong);
+    if (!off) {
+      PyErr_SetString(PyExc_TypeError, "run_group: offsets");
+      return nullptr;
+    }
+    n_runs = off->numel() - 1;
+  }
+  auto up16 = [](size_t v) { return (v + 15) & ~static_cast<size_t>(15); };
+  size_t at0 = 0;
+  auto place = [&](size_t bytes) {
+    const size_t here = at0;
+    at0 = up16(at0 + bytes);
+    return here;
+  };
+  const size_t o_totals = place(static_cast<size_t>(T) * n_runs * 8);
+  struct Kind { hb_mlp* h; const at::Tensor *f, *ms; const uint8_t* rows; int64_t n; size_t o_ms, o_pred; };
+  std::vector<Kind> kinds;
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[6]); ++i) {
+    PyObject* t = PyList_GET_ITEM(a[6], i);
+    Kind k{};
+    k.h = static_cast<hb_mlp*>(PyLong_AsVoidPtr(PyTuple_GET_ITEM(t, 0)));
+    k.f = tensor(PyTuple_GET_ITEM(t, 1), at::kFloat);
+    k.ms = tensor(PyTuple_GET_ITEM(t, 2), at::kFloat);
+    PyObject* rows = PyTuple_GET_ITEM(t, 3);
+    if (!k.f || !k.ms || !PyBytes_Check(rows) || PyBytes_GET_SIZE(rows) != T + 1 || k.ms->numel() != k.f->size(0)) {
+      PyErr_SetString(PyExc_TypeError, "run_group: operation kind");
+      return nullptr;
+    }
+    k.rows = reinterpret_cast<const uint8_t*>(PyBytes_AS_STRING(rows));
+    k.n = k.f->size(0);
+    k.o_ms = place(static_cast<size_t>(T) * k.n * 4);
+    k.o_pred = place(static_cast<size_t>(T + 1) * k.n * 4);
+    kinds.push_back(k);
+  }
+  size_t o_scaled = at0, o_rest = 0;
+  if (a[0] != Py_None) {
+    const Field nb(a[0], s_num_blocks, at::kInt);
+    if (!nb.t) {
+      PyErr_SetString(PyExc_TypeError, "run_group: kernels");
+      return nullptr;
+    }
+    K = nb.t->numel();
+  }
+  place(static_cast<size_t>(T) * K * 4);
+  const size_t result = at0;
+  // the planes of the wave-scaling call that stay on the device follow
+  auto plane = [&](size_t bytes) {
+    at0 = (at0 + 255) & ~static_cast<size_t>(255);
+    return place(bytes);
+  };
+  o_rest = plane(static_cast<size_t>(T) * K);
+  const size_t o_waves = plane(static_cast<size_t>(T) * K * 4), o_oocc = plane(K), o_owaves = plane(K * 4);
+
+  int current = 0;
+  cudaGetDevice(&current);
+  const int64_t total[1] = {static_cast<int64_t>(at0 ? at0 : 16)}, host_size[1] = {static_cast<int64_t>(result ? result : 16)};
+  at::Tensor block = empty(total, at::kByte, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(current)));
+  uint8_t* d = static_cast<uint8_t*>(block.mutable_data_ptr());
+  cudaStream_t s = static_cast<cudaStream_t>(stream_now());
+
+  // the predictors first: they take longest, and the wave scaling's host part runs under them
+  std::vector<hb_mlp_grid> grids;
+  std::vector<hb_scale_grid> scales;
+  for (const Kind& k : kinds) {
+    grids.push_back(hb_mlp_grid{k.h, static_cast<const float*>(data(k.f)), k.n, k.rows, static_cast<int32_t>(T + 1),
+                                reinterpret_cast<float*>(d + k.o_pred)});
+    scales.push_back(hb_scale_grid{static_cast<const float*>(data(k.ms)), reinterpret_cast<const float*>(d + k.o_pred), k.n,
+                                   static_cast<int32_t>(T), reinterpret_cast<float*>(d + k.o_ms), nullptr});
+  }
+  if (failed(api.mlp_predict_grid(grids.data(), static_cast<int32_t>(grids.size()), s))) return nullptr;
+  if (K > 0) {
+    const Field nb(a[0], s_num_blocks, at::kInt), bs(a[0], s_block_size, at::kUInt16), rg(a[0], s_regs, at::kUInt16),
+        sm(a[0], s_smem, at::kUInt32), tm(a[0], s_time, at::kFloat), gm(a[0], s_gamma, at::kFloat);
+    const int16_t* regs = nullptr;
+    if (a[4] != Py_None) {
+      const at::Tensor* t = tensor(a[4], at::kShort);
+      if (t && t->numel() == T * K) regs = static_cast<const int16_t*>(data(t));
+      else PyErr_SetString(PyExc_TypeError, "run_group: dest_regs");
+    }
+    if (!bs.t || !rg.t || !sm.t || !tm.t || !gm.t) PyErr_SetString(PyExc_TypeError, "run_group: kernels");
+    int32_t rows[HB_MAX_DEVICES];
+    if (T > HB_MAX_DEVICES) PyErr_SetString(PyExc_ValueError, "too many destinations");
+    if (PyErr_Occurred()) return nullptr;
+    const long origin = row_of(a[2]);
+    if (origin < 0) return nullptr;
+    for (int64_t t = 0; t < T; ++t) {
+      const long r = row_of(PySequence_Fast_GET_ITEM(dests.p, t));
+      if (r < 0) return nullptr;
+      rows[t] = static_cast<int32_t>(r);
+    }
+    hb_kernel_soa soa{static_cast<const int32_t*>(nb.ptr()), static_cast<const uint16_t*>(bs.ptr()),
+                      static_cast<const uint16_t*>(rg.ptr()), static_cast<const uint32_t*>(sm.ptr()),
+                      static_cast<const float*>(tm.ptr()), static_cast<const float*>(gm.ptr())};
+    hb_wave_out o{reinterpret_cast<float*>(d + o_scaled), d + o_rest, reinterpret_cast<uint32_t*>(d + o_waves), d + o_oocc,
+                  reinterpret_cast<uint32_t*>(d + o_owaves), nullptr, nullptr};
+    hb_kernel_metrics m{};
+    const bool with_metrics = a[1] != Py_None;
+    if (with_metrics) {
+      const Field fe(a[1], s_flop, at::kDouble), rd(a[1], s_rd, at::kDouble), wr(a[1], s_wr, at::kDouble),
+          has(a[1], s_has, at::kByte);
+      if (!fe.t || !rd.t || !wr.t || !has.t) {
+        PyErr_SetString(PyExc_TypeError, "run_group: metrics");
+        return nullptr;
+      }
+      m = hb_kernel_metrics{static_cast<const double*>(fe.ptr()), static_cast<const double*>(rd.ptr()),
+                            static_cast<const double*>(wr.ptr()), static_cast<const uint8_t*>(has.ptr())};
+    }
+    if (failed(wave_scale_call(soa, with_metrics ? &m : nullptr, K, static_cast<int32_t>(origin), rows,
+                               static_cast<int32_t>(T), regs, o, nullptr, nullptr, s)))
+      return nullptr;
+    if (off && failed(api.segment_sum_planes(o.scaled_ns, K, static_cast<int32_t>(T), static_cast<const int64_t*>(data(off)),
+                                             n_runs, reinterpret_cast<double*>(d + o_totals), s)))
+      return nullptr;
+  } else if (n_runs > 0) {
+    if (cudaMemsetAsync(d + o_totals, 0, static_cast<size_t>(T) * n_runs * 8, s) != cudaSuccess) {
+      PyErr_SetString(PyExc_RuntimeError, "cudaMemsetAsync");
+      return nullptr;
+    }
+  }
+  if (failed(api.special_scale_grid(scales.data(), static_cast<int32_t>(scales.size()), s))) return nullptr;
+  at::Tensor host(at::detail::empty_cpu(host_size, at::kByte, /*pin_memory=*/true));
+  uint8_t* h = static_cast<uint8_t*>(host.mutable_data_ptr());
+  cudaError_t e;
+  Py_BEGIN_ALLOW_THREADS
+  e = result ? cudaMemcpyAsync(h, d, result, cudaMemcpyDeviceToHost, s) : cudaSuccess;
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  Py_END_ALLOW_THREADS
+  if (e != cudaSuccess) {
+    PyErr_Format(PyExc_RuntimeError, "prediction of a trace: %s", cudaGetErrorString(e));
+    return nullptr;
+  }
+  for (const Kind& k : kinds) {
+    int32_t code = 0;
+    if (failed(api.mlp_poll_status(k.h, &code))) return nullptr;
+  }
+  bool nan = false;
+  const float* scaled = reinterpret_cast<const float*>(h + o_scaled);
+  for (int64_t i = 0; i < T * K; ++i) nan = nan || scaled[i] != scaled[i];
+  Ref clamped(PyList_New(static_cast<Py_ssize_t>(kinds.size())));
+  for (size_t i = 0; i < kinds.size(); ++i) {
+    const float* ms = reinterpret_cast<const float*>(h + kinds[i].o_ms);
+    bool zero = false;
+    for (int64_t j = 0; j < T * kinds[i].n; ++j) zero = zero || ms[j] == 0.0f;
+    PyList_SET_ITEM(clamped.p, static_cast<Py_ssize_t>(i), PyBool_FromLong(zero));
+  }
+  return Py_BuildValue("(NNO)", bytes_of(h, result), PyBool_FromLong(nan), clamped.p);
+  END_HANDLE_TH_ERRORS
+}
+
+// iteration_totals(kernels, scaled_ns, overhead_ns, kernel_offsets, same (bytes per destination),
+//                  [(handle address, features, measured ms, offsets, device rows (bytes))])
+// -> [I, D] float64 totals (habitat_b200/iteration.py), or None when an argument does not fit
+PyObject* iteration_totals(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  if (n_args != 6 || !PyBytes_Check(a[4]) || !PyList_Check(a[5])) return not_ordinary();
+  const Field tm(a[0], s_time, at::kFloat);
+  const at::Tensor *scaled = tensor(a[1], at::kFloat), *over = tensor(a[2], at::kFloat), *off = tensor(a[3], at::kLong);
+  if (!tm.t || !scaled || !over || !off || off->numel() < 1) return not_ordinary();
+  const int64_t K = tm.t->numel(), I = off->numel() - 1, D = PyBytes_GET_SIZE(a[4]);
+  if (over->numel() != K || scaled->numel() != D * K) return not_ordinary();
+  const uint8_t* same = reinterpret_cast<const uint8_t*>(PyBytes_AS_STRING(a[4]));
+  struct Kind { hb_mlp* h; const at::Tensor *f, *ms, *off; const uint8_t* rows; int64_t blocks; };
+  std::vector<Kind> kinds;
+  int64_t floats = 0;
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[5]); ++i) {
+    PyObject* t = PyList_GET_ITEM(a[5], i);
+    Kind k{static_cast<hb_mlp*>(PyLong_AsVoidPtr(PyTuple_GET_ITEM(t, 0))), tensor(PyTuple_GET_ITEM(t, 1), at::kFloat),
+           tensor(PyTuple_GET_ITEM(t, 2), at::kFloat), tensor(PyTuple_GET_ITEM(t, 3), at::kLong),
+           reinterpret_cast<const uint8_t*>(PyBytes_AS_STRING(PyTuple_GET_ITEM(t, 4))),
+           PyBytes_GET_SIZE(PyTuple_GET_ITEM(t, 4))};
+    if (!k.f || !k.ms || !k.off || k.f->dim() != 2 || k.ms->numel() != k.f->size(0) || k.off->numel() != I + 1)
+      return not_ordinary();
+    kinds.push_back(k);
+    if (k.blocks > 1) floats += (k.blocks * k.f->size(0) + 63) & ~int64_t{63};
+  }
+  const int64_t id[2] = {I, D}, fl[1] = {floats};
+  at::Tensor out = empty(id, at::kDouble, tm.t->device()), preds = empty(fl, at::kFloat, tm.t->device());
+  float* p = static_cast<float*>(preds.mutable_data_ptr());
+  void* s = stream_now();
+  std::vector<hb_mlp_grid> grids;
+  std::vector<hb_iteration_kind> its;
+  for (const Kind& k : kinds) {
+    const bool predict = k.blocks > 1;
+    its.push_back(hb_iteration_kind{static_cast<const float*>(data(k.ms)), predict ? p : nullptr,
+                                    static_cast<const int64_t*>(data(k.off)), k.f->size(0)});
+    if (!predict) continue;
+    grids.push_back(hb_mlp_grid{k.h, static_cast<const float*>(data(k.f)), k.f->size(0), k.rows,
+                                static_cast<int32_t>(k.blocks), p});
+    p += (k.blocks * k.f->size(0) + 63) & ~int64_t{63};
+  }
+  hb_status st = HB_OK;
+  Py_BEGIN_ALLOW_THREADS
+  for (size_t i = 0; i < grids.size() && st == HB_OK; i += 4)
+    st = api.mlp_predict_grid(grids.data() + i, static_cast<int32_t>(grids.size() - i < 4 ? grids.size() - i : 4), s);
+  if (st == HB_OK)
+    st = api.iteration_totals(static_cast<const float*>(data(over)), static_cast<const float*>(tm.ptr()),
+                              static_cast<const float*>(data(scaled)), K, static_cast<const int64_t*>(data(off)), I,
+                              static_cast<int32_t>(D), same, its.data(), static_cast<int32_t>(its.size()),
+                              static_cast<double*>(out.mutable_data_ptr()), s);
+  Py_END_ALLOW_THREADS
+  if (failed(st)) return nullptr;
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
 // setup(addresses by name, row_of, check, WaveResult)
 PyObject* setup(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 4 || !PyDict_Check(a[0])) {
@@ -395,7 +951,11 @@ PyObject* setup(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!load(api.wave_scale, "hb_wave_scale") || !load(api.wave_scale_metrics, "hb_wave_scale_metrics") ||
       !load(api.wave_scale_partials, "hb_wave_scale_partials") || !load(api.partials_sum, "hb_partials_sum") ||
       !load(api.mlp_predict, "hb_mlp_predict") || !load(api.mlp_predict_host, "hb_mlp_predict_host") || !load(api.group_sum, "hb_group_sum") ||
-      !load(api.plane_sum, "hb_plane_sum") || !load(api.segment_sum, "hb_segment_sum")) {
+      !load(api.plane_sum, "hb_plane_sum") || !load(api.segment_sum, "hb_segment_sum") ||
+      !load(api.segment_sum_planes, "hb_segment_sum_planes") ||
+      !load(api.mlp_predict_grid, "hb_mlp_predict_grid") || !load(api.mlp_poll_status, "hb_mlp_poll_status") ||
+      !load(api.special_scale_grid, "hb_special_scale_grid") ||
+      !load(api.iteration_totals, "hb_iteration_totals")) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "an entry point is missing");
     return nullptr;
   }
@@ -412,7 +972,7 @@ PyObject* set_generation(PyObject*, PyObject* v) {
 }
 
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {FAST(setup), FAST(wave_scale), FAST(mlp_predict), FAST(mlp_predict_one), FAST(partials_sum), FAST(group_sum),
+PyMethodDef methods[] = {FAST(setup), FAST(wave_scale), FAST(mlp_predict), FAST(mlp_predict_one), FAST(flatten_trace), FAST(feature_rows), FAST(run_group), FAST(iteration_totals), FAST(partials_sum), FAST(group_sum),
                          FAST(plane_sum), FAST(segment_sum),
                          {"set_generation", set_generation, METH_O, nullptr},
                          {nullptr, nullptr, 0, nullptr}};
@@ -427,7 +987,14 @@ PyMODINIT_FUNC PyInit__binding(void) {
       {&s_flop, "flop_efficiency_pct"}, {&s_rd, "dram_read_bytes"}, {&s_wr, "dram_write_bytes"},
       {&s_has, "has_metrics"}, {&s_scaled, "scaled_ns"}, {&s_docc, "dest_occupancy"}, {&s_dwav, "dest_waves"},
       {&s_oocc, "origin_occupancy"}, {&s_owav, "origin_waves"}, {&s_status, "status"}, {&s_limits, "limits"},
-      {&s_buffer, "buffer"}, {&s_K, "K"}, {&s_D, "D"}, {&s_per_plane, "per_plane"}, {&s_n_planes, "n_planes"}};
+      {&s_buffer, "buffer"}, {&s_K, "K"}, {&s_D, "D"}, {&s_per_plane, "per_plane"}, {&s_n_planes, "n_planes"},
+      {&s__name, "_name"}, {&s__device, "_device"}, {&s__forward, "_forward"}, {&s__backward, "_backward"},
+      {&s__arguments, "_arguments"}, {&s_args, "args"}, {&s_kwargs, "kwargs"}, {&s__kernels, "_kernels"},
+      {&s__run_time_ms, "_run_time_ms"}, {&s__c, "_c"}, {&s__metrics_kernels, "_metrics_kernels"},
+      {&s__cached_metrics, "_cached_metrics"}, {&s__metrics, "_metrics"}, {&s__num_blocks, "_num_blocks"},
+      {&s__block_size, "_block_size"}, {&s__regs, "_registers_per_thread"},
+      {&s__smem_static, "_static_shared_memory"}, {&s__smem_dynamic, "_dynamic_shared_memory"},
+      {&s__run_time_ns, "_run_time_ns"}, {&s_name, "name"}};
   for (const auto& n : names)
     if (!(*n.s = PyUnicode_InternFromString(n.name))) return nullptr;
   return PyModule_Create(&module);

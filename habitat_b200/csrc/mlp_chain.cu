@@ -67,6 +67,9 @@ struct MlpParams {
   int32_t num_tiles;
   int32_t* status;           // device word: 0 ok, else (role << 8 | site)
   long long* phase_cycles;   // [16] cluster 0: cycle counters of the roles (diagnostic), or null
+  int32_t beside;            // runs beside the launch before it on the stream: nothing to wait for
+  int32_t grid_n;            // > 0: query q is feature row q % grid_n on device grid_rows[q / grid_n]
+  uint8_t grid_rows[hb::kMaxGridRows];
   CUtensorMap tmap_slot;     // pair kernel: the pack as [rows][128 B], box of two tile images (32 KB)
   CUtensorMap tmap_tile;     // same tensor, box of one tile image (16 KB, fc1)
 };
@@ -194,6 +197,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
+  grid_begin(p.beside != 0);   // the set-up above overlaps the end of the launch before it on the stream
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();
@@ -403,11 +407,19 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
 #pragma unroll
         for (int c = 0; c < kKBlk; ++c) row[c] = __float2bfloat16_rn(0.0f);
         if (T < kHalfQ && q < p.Q) {
-          int dr = p.dev_row[q];
+          int64_t fr = q;
+          int dr;
+          if (p.grid_n) {
+            const uint32_t block = static_cast<uint32_t>(q) / static_cast<uint32_t>(p.grid_n);
+            fr -= static_cast<int64_t>(block) * p.grid_n;
+            dr = p.grid_rows[block];
+          } else {
+            dr = p.dev_row[q];
+          }
           dr = dr < p.n_dev ? dr : p.n_dev - 1;
           for (int c = 0; c < C_in; ++c) {
             const double x = c < p.n_op_feat
-                                 ? static_cast<double>(p.feats[q * p.n_op_feat + c])
+                                 ? static_cast<double>(p.feats[fr * p.n_op_feat + c])
                                  : p.dev_feat[dr * 4 + (c - p.n_op_feat)];
             const float xn = static_cast<float>((x - p.mu[c]) / p.sigma[c]);
             const __nv_bfloat16 hi = __float2bfloat16_rn(xn);
@@ -620,6 +632,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u)
                  : "memory");
   }
+  grid_end(p.beside != 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -828,13 +841,9 @@ extern "C" hb_status hb_mlp_create(hb_mlp** handle, int32_t n_op_features, int32
   return HB_OK;
 }
 
-extern "C" hb_status hb_mlp_predict(hb_mlp* h, const float* op_features, const uint8_t* device_row,
-                                    int64_t Q, float* out, void* stream) {
-  if (!h || Q < 0 || (Q > 0 && (!op_features || !device_row || !out))) {
-    hb::set_error("hb_mlp_predict: bad arguments");
-    return HB_ERR_INVALID_ARGUMENT;
-  }
-  if (Q == 0) return HB_OK;
+namespace {
+// Queues one batch (checked by the callers) on the kernel for its size.
+hb_status queue_batch(hb_mlp* h, const hb::MlpBatch& batch, cudaStream_t s) {
   int cur = -1;
   HB_CUDA_TRY(cudaGetDevice(&cur));
   if (cur != h->device) {
@@ -847,30 +856,81 @@ extern "C" hb_status hb_mlp_predict(hb_mlp* h, const float* op_features, const u
   static const bool use_wide = [] { const char* e = std::getenv("HB_MLP_WIDE"); return !e || std::atoi(e) != 0; }();
   if (use_wide) {
     bool launched = false;
-    const hb_status st = hb::wide_predict(h, hb::wide_plan(Q, split, h->sm_count), op_features, device_row, Q, out,
-                                          static_cast<cudaStream_t>(stream), &launched);
+    const hb_status st = hb::wide_predict(h, hb::wide_plan(batch.Q, split, h->sm_count), batch, s, &launched);
     if (st != HB_OK || launched) return st;
   }
   const int tile_q = split ? kPairQ / 2 : kPairQ;
-  const int64_t tiles = (Q + tile_q - 1) / tile_q;
-  if (tiles > 0x7FFFFFFF) {
+  const int64_t tiles = (batch.Q + tile_q - 1) / tile_q;
+  if (tiles > 0x7FFFFFFF || (batch.grid_n && batch.Q > 0xFFFFFFFFll)) {
     hb::set_error("hb_mlp_predict: Q too large for one launch");
     return HB_ERR_TOO_LARGE;
   }
   MlpParams p{};
   p.wpack = h->wpack; p.bias = h->bias; p.fc2_w = h->fc2_w; p.fc2_b = h->fc2_b;
   p.mu = h->mu; p.sigma = h->sigma; p.dev_feat = h->dev_feat; p.n_dev = h->n_dev;
-  p.n_op_feat = h->n_op_feat; p.layers = h->layers; p.feats = op_features;
-  p.dev_row = device_row; p.Q = Q; p.out = out; p.num_tiles = static_cast<int32_t>(tiles);
+  p.n_op_feat = h->n_op_feat; p.layers = h->layers; p.feats = batch.feats;
+  p.dev_row = batch.dev_row; p.Q = batch.Q; p.out = batch.out; p.num_tiles = static_cast<int32_t>(tiles);
+  p.grid_n = batch.grid_n;
+  if (batch.grid_n) std::memcpy(p.grid_rows, batch.grid_rows, static_cast<size_t>(batch.Q / batch.grid_n));
+  p.beside = batch.beside ? 1 : 0;
   p.status = h->status;
   p.phase_cycles = h->phase_cycles;
   p.tmap_slot = h->tmap_slot; p.tmap_tile = h->tmap_tile;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   // one cluster of two CTAs per tile (128 queries, 64 in split precision), at most one cluster per SM pair
   const int pairs = static_cast<int>(tiles < h->sm_count / 2 ? tiles : h->sm_count / 2);
-  if (split) mlp_chain_pair_kernel<true><<<2 * pairs, kPairThreads, kPairSmemBytes, s>>>(p);
-  else mlp_chain_pair_kernel<false><<<2 * pairs, kPairThreads, kPairSmemBytes, s>>>(p);
-  HB_CUDA_TRY(cudaGetLastError());
+  HB_CUDA_TRY(hb::launch_overlapped(split ? mlp_chain_pair_kernel<true> : mlp_chain_pair_kernel<false>, dim3(2 * pairs),
+                                    dim3(kPairThreads), kPairSmemBytes, s, p));
+  return HB_OK;
+}
+}  // namespace
+
+extern "C" hb_status hb_mlp_predict(hb_mlp* h, const float* op_features, const uint8_t* device_row,
+                                    int64_t Q, float* out, void* stream) {
+  if (!h || Q < 0 || (Q > 0 && (!op_features || !device_row || !out))) {
+    hb::set_error("hb_mlp_predict: bad arguments");
+    return HB_ERR_INVALID_ARGUMENT;
+  }
+  if (Q == 0) return HB_OK;
+  hb::MlpBatch batch;
+  batch.feats = op_features; batch.dev_row = device_row; batch.Q = Q; batch.out = out;
+  return queue_batch(h, batch, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" hb_status hb_mlp_predict_grid(const hb_mlp_grid* items, int32_t n_items, void* stream) {
+  if (n_items < 0 || n_items > hb::kMaxLanes || (n_items > 0 && !items)) {
+    hb::set_error("hb_mlp_predict_grid: 0 to %d batches", hb::kMaxLanes);
+    return HB_ERR_INVALID_ARGUMENT;
+  }
+  for (int i = 0; i < n_items; ++i) {
+    const hb_mlp_grid& g = items[i];
+    if (!g.handle || g.n < 0 || g.n > 0x7FFFFFFF || g.n_device_rows < 0 || g.n_device_rows > hb::kMaxGridRows ||
+        (g.n > 0 && g.n_device_rows > 0 && (!g.op_features || !g.device_rows || !g.out))) {
+      hb::set_error("hb_mlp_predict_grid: bad batch %d (at most %d device rows)", i, hb::kMaxGridRows);
+      return HB_ERR_INVALID_ARGUMENT;
+    }
+  }
+  // The largest first: its launch waits for what is on the stream, the others run beside it on the SMs
+  // that its last wave leaves idle.
+  int order[hb::kMaxLanes] = {0, 1, 2, 3};
+  for (int i = 1; i < n_items; ++i)
+    for (int j = i; j > 0 && items[order[j]].n * items[order[j]].n_device_rows >
+                                 items[order[j - 1]].n * items[order[j - 1]].n_device_rows; --j) {
+      const int t = order[j];
+      order[j] = order[j - 1];
+      order[j - 1] = t;
+    }
+  int lane = 0;
+  for (int i = 0; i < n_items; ++i) {
+    const hb_mlp_grid& g = items[order[i]];
+    if (g.n == 0 || g.n_device_rows == 0) continue;
+    hb::MlpBatch batch;
+    batch.feats = g.op_features; batch.Q = g.n * g.n_device_rows; batch.out = g.out;
+    batch.grid_n = static_cast<int32_t>(g.n); batch.grid_rows = g.device_rows;
+    batch.lane = lane; batch.beside = lane > 0;
+    ++lane;
+    const hb_status st = queue_batch(g.handle, batch, static_cast<cudaStream_t>(stream));
+    if (st != HB_OK) return st;
+  }
   return HB_OK;
 }
 
@@ -894,6 +954,14 @@ extern "C" hb_status hb_mlp_status(hb_mlp* h, int32_t* device_status) {
     return HB_ERR_INVALID_ARGUMENT;
   }
   HB_CUDA_TRY(cudaDeviceSynchronize());   // launches on non-blocking streams included
+  return read_status(h, device_status);
+}
+
+extern "C" hb_status hb_mlp_poll_status(hb_mlp* h, int32_t* device_status) {
+  if (!h || !device_status) {
+    hb::set_error("hb_mlp_poll_status: NULL argument");
+    return HB_ERR_INVALID_ARGUMENT;
+  }
   return read_status(h, device_status);
 }
 
@@ -949,7 +1017,10 @@ extern "C" hb_status hb_mlp_predict_host(hb_mlp* h, const float* op_features,
     const hb::WidePlan plan = hb::wide_plan(Q, h->precision == HB_PRECISION_BF16X3, h->sm_count);
     bool launched = false;
     if (Q <= hb::kWideInline) {
-      st = hb::wide_predict(h, plan, op_features, device_row, Q, p_o, s, &launched, true);
+      hb::MlpBatch batch;
+      batch.feats = op_features; batch.dev_row = device_row; batch.Q = Q; batch.out = p_o;
+      batch.host_inputs = true;
+      st = hb::wide_predict(h, plan, batch, s, &launched);
       if (st != HB_OK) return st;
     }
     if (!launched) {

@@ -61,6 +61,19 @@ __device__ __forceinline__ uint32_t elect_one() {
       : "=r"(pred)::"memory");
   return pred;
 }
+// Programmatic dependent launch of kernels of which some run side by side.  An ordinary one waits for the
+// launch before it and only then lets the next one start; one that runs beside its predecessor does not
+// wait at the start (it can only have started after an ordinary one before it had waited), but one of its
+// blocks waits at the end, so that "this grid is complete" still means "and so are those before it".
+__device__ __forceinline__ void hb_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_begin(bool beside) {
+  if (!beside) hb_grid_wait();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_end(bool beside) {
+  if (beside && blockIdx.x == 0) hb_grid_wait();
+}
+
 // Slot arithmetic of the MMA issue loops.  The descriptors of tcgen05.mma live in uniform registers, and
 // only some operations exist there: a ring position kept by compare and select (or by a remainder)
 // went through vector registers and cost a transfer per MMA, 180 cycles per 16 of them.  Shifts and

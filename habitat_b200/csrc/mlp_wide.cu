@@ -60,6 +60,9 @@ struct WideParams {
   int32_t* poison;            // set by a launch that gave up
   uint32_t tag;               // of this launch
   unsigned long long parity[2];   // bit g: parity of the next use of group g's buffer 0, 1
+  int32_t beside;             // runs beside the launch before it: nothing to wait for
+  int32_t grid_n;             // > 0: query q is feature row q % grid_n on device grid_rows[q / grid_n]
+  uint8_t grid_rows[hb::kMaxGridRows];
   int32_t inline_q;           // > 0: the queries themselves, below, instead of feats and dev_row
   float inline_feats[kWideInline * (kMaxInFeat - 4)];
   uint8_t inline_row[kWideInline];
@@ -206,6 +209,7 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   constexpr uint32_t kTmemCols = kBlocks * W < 32 ? 32 : kBlocks * W;
+  if (threadIdx.x == 64 && !p.beside) hb_grid_wait();   // the mark may be a fresh buffer's
   if (threadIdx.x == 64 && *reinterpret_cast<volatile int32_t*>(p.poison) != 0) {
     // an earlier launch left the buffers in an unknown state: report, and touch nothing
     *poisoned = 1;
@@ -219,6 +223,7 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  grid_begin(p.beside != 0);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -422,9 +427,17 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     epi_sync();
     for (int i = T; i < n_q * C_in; i += 128) {
       const int q = i / C_in, f = i - q * C_in;
-      int dr = p.inline_q ? p.inline_row[q] : p.dev_row[q0 + q];
+      int64_t fr = q0 + q;
+      int dr;
+      if (p.grid_n) {
+        const uint32_t block = static_cast<uint32_t>(fr) / static_cast<uint32_t>(p.grid_n);
+        fr -= static_cast<int64_t>(block) * p.grid_n;
+        dr = p.grid_rows[block];
+      } else {
+        dr = p.inline_q ? p.inline_row[q] : p.dev_row[fr];
+      }
       dr = dr < p.n_dev ? dr : p.n_dev - 1;
-      const double x = f < p.n_op_feat ? static_cast<double>(p.inline_q ? p.inline_feats[i - 4 * q] : p.feats[(q0 + q) * p.n_op_feat + f])
+      const double x = f < p.n_op_feat ? static_cast<double>(p.inline_q ? p.inline_feats[i - 4 * q] : p.feats[fr * p.n_op_feat + f])
                                        : p.dev_feat[dr * 4 + (f - p.n_op_feat)];
       const float xn = static_cast<float>((x - p.mu[f]) / p.sigma[f]);
       const __nv_bfloat16 hi = __float2bfloat16_rn(xn);
@@ -574,6 +587,7 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
   }
+  grid_end(p.beside != 0);
 }
 }  // namespace
 
@@ -582,9 +596,10 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
 // ---------------------------------------------------------------------------
 namespace {
 constexpr int kMaxCudaDevices = 64;
-// Scratch per stream: launches on one stream follow one another, so they can share it.  It is kept
-// between launches, at most kMaxStreams of them per GPU (a launch on yet another stream takes the
-// two-SM kernel, which needs none), and freed with the GPU's last predictor.
+// Scratch per stream: launches on one stream follow one another, so they can share it (those of one call
+// that run side by side have a lane each).  It is kept between launches, at most kMaxStreams of them per
+// GPU (a launch on yet another stream takes the two-SM kernel, which needs none), and freed with the
+// GPU's last predictor.
 constexpr int kMaxStreams = 16;
 constexpr int kMaxGroups = 37;
 constexpr int kWidths = 3;        // W = 16, 32, 64 have their own buffers: a word's parity counts its own uses
@@ -593,6 +608,7 @@ constexpr size_t kHalvesBytes = static_cast<size_t>(kMaxGroups) * 64 * kWideCols
 constexpr size_t kScratchBytes = kActsBytes + kHalvesBytes + 256;   // and the mark of a launch that gave up
 struct StreamScratch {
   unsigned long long stream_id = 0;
+  int lane = 0;
   uint8_t* base = nullptr;
   bool fresh = false;                            // buffers and parities start over at the next launch
   uint32_t tag = 0;
@@ -608,7 +624,7 @@ GpuScratch g_wide[kMaxCudaDevices];
 
 // The scratch of `stream` on GPU `dev`, or null when there is none to be had (a stream that is being
 // captured: a graph may be replayed anywhere; too many streams; no memory).  Call with the mutex held.
-StreamScratch* scratch_of(GpuScratch& g, cudaStream_t stream) {
+StreamScratch* scratch_of(GpuScratch& g, cudaStream_t stream, int lane) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
   if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
@@ -617,7 +633,7 @@ StreamScratch* scratch_of(GpuScratch& g, cudaStream_t stream) {
     return nullptr;
   }
   for (int i = 0; i < g.used; ++i)
-    if (g.s[i].stream_id == id) return &g.s[i];
+    if (g.s[i].stream_id == id && g.s[i].lane == lane) return &g.s[i];
   if (g.used == kMaxStreams) return nullptr;
   StreamScratch& s = g.s[g.used];
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // another stream's capture does not mind this allocation
@@ -630,6 +646,7 @@ StreamScratch* scratch_of(GpuScratch& g, cudaStream_t stream) {
     return nullptr;
   }
   s.stream_id = id;
+  s.lane = lane;
   s.base = static_cast<uint8_t*>(base);
   s.fresh = true;
   ++g.used;
@@ -645,13 +662,15 @@ cudaError_t launch(const WideParams& p, int groups, int device, cudaStream_t str
   cfg.blockDim = dim3(wide_threads<W>());
   cfg.dynamicSmemBytes = wide_smem<W>();
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = G;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 1;   // for the occupancy question
   int n = clusters[device].load(std::memory_order_acquire);
   if (n == 0) {
     cudaError_t e = cudaFuncSetAttribute(mlp_wide_kernel<G, W, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -665,6 +684,7 @@ cudaError_t launch(const WideParams& p, int groups, int device, cudaStream_t str
     clusters[device].store(n, std::memory_order_release);
   }
   *fits = n > 1;
+  cfg.numAttrs = hb::overlapped_launch_enabled() ? 2 : 1;
   return *fits ? cudaLaunchKernelEx(&cfg, mlp_wide_kernel<G, W, SPLIT>, p) : cudaSuccess;
 }
 template <bool SPLIT>
@@ -729,24 +749,27 @@ void wide_start_over(int device) {
   for (int i = 0; i < g.used; ++i) g.s[i].fresh = true;
 }
 
-hb_status wide_predict(hb_mlp* h, const WidePlan& w, const float* feats, const uint8_t* dev_row, int64_t Q, float* out,
-                       cudaStream_t stream, bool* launched, bool host_inputs) {
+hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cudaStream_t stream, bool* launched) {
   *launched = false;
-  if (w.G == 0 || h->device >= kMaxCudaDevices || (host_inputs && Q > kWideInline)) return HB_OK;
+  if (w.G == 0 || h->device >= kMaxCudaDevices || (batch.host_inputs && batch.Q > kWideInline)) return HB_OK;
   GpuScratch& g = g_wide[h->device];
   std::lock_guard<std::mutex> lock(g.mu);   // held over the launch: parities and tags follow the stream's order
-  StreamScratch* s = scratch_of(g, stream);
+  StreamScratch* s = scratch_of(g, stream, batch.lane);
   if (!s) return HB_OK;
   const bool split = h->precision == HB_PRECISION_BF16X3;
   WideParams p{};
   p.bias = h->bias; p.fc2_w = h->fc2_w; p.fc2_b = h->fc2_b; p.mu = h->mu; p.sigma = h->sigma; p.dev_feat = h->dev_feat;
   p.n_dev = h->n_dev; p.n_op_feat = h->n_op_feat; p.layers = h->layers;
-  p.feats = feats; p.dev_row = dev_row; p.Q = static_cast<int32_t>(Q); p.per_group = w.per_group; p.out = out;
+  p.feats = batch.feats; p.dev_row = batch.dev_row; p.Q = static_cast<int32_t>(batch.Q);
+  p.per_group = w.per_group; p.out = batch.out;
   p.status = h->status;
-  if (host_inputs) {
-    p.inline_q = static_cast<int32_t>(Q);
-    std::memcpy(p.inline_feats, feats, sizeof(float) * Q * h->n_op_feat);
-    std::memcpy(p.inline_row, dev_row, Q);
+  p.beside = batch.beside && !s->fresh ? 1 : 0;   // (a fresh buffer's clearing has to be waited for)
+  p.grid_n = batch.grid_n;
+  if (batch.grid_n) std::memcpy(p.grid_rows, batch.grid_rows, batch.Q / batch.grid_n);
+  if (batch.host_inputs) {
+    p.inline_q = static_cast<int32_t>(batch.Q);
+    std::memcpy(p.inline_feats, batch.feats, sizeof(float) * batch.Q * h->n_op_feat);
+    std::memcpy(p.inline_row, batch.dev_row, batch.Q);
   }
   if (s->fresh) {
     // all words at parity 0, all tags at 0

@@ -13,10 +13,26 @@ struct WidePlan {
 WidePlan wide_plan(int64_t Q, bool split, int sm_count);
 // Queries that can travel as kernel parameters: no copy and no read over PCIe for the scalar API.
 constexpr int kWideInline = 16;
-// Queues the launch; *launched stays false when the stream has no scratch (see there).  host_inputs: feats
-// and dev_row are ordinary host memory and Q <= kWideInline.
-hb_status wide_predict(hb_mlp* h, const WidePlan& w, const float* feats, const uint8_t* dev_row, int64_t Q, float* out,
-                       cudaStream_t stream, bool* launched, bool host_inputs = false);
+// A batch of queries.  Either every query has its own row of feats and of dev_row, or (grid_n > 0) the same
+// grid_n feature rows are asked about for each of a list of device rows: query q is row q % grid_n on
+// device grid_rows[q / grid_n], and nothing has to be repeated in memory.
+constexpr int kMaxGridRows = 80;
+struct MlpBatch {
+  const float* feats = nullptr;
+  const uint8_t* dev_row = nullptr;
+  int64_t Q = 0;
+  float* out = nullptr;
+  bool host_inputs = false;          // feats and dev_row are ordinary host memory, Q <= kWideInline
+  int32_t grid_n = 0;
+  const uint8_t* grid_rows = nullptr;   // host, Q / grid_n entries
+  // Launches of one call that read nothing from one another: number `lane` of them (its own scratch), and
+  // whether it may run beside the launch before it on the stream.
+  int lane = 0;
+  bool beside = false;
+};
+constexpr int kMaxLanes = 4;
+// Queues the launch; *launched stays false when the stream has no scratch (see there).
+hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cudaStream_t stream, bool* launched);
 // After a launch that gave up: every stream's scratch on the GPU is set up again before its next use.
 void wide_start_over(int device);
 void wide_handle_created(int device);

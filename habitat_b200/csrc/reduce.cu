@@ -59,6 +59,115 @@ special_scale_kernel(const float* __restrict__ run_time_ms, const float* __restr
   }
 }
 
+// Segment sums over several planes that share the offsets, one warp per (plane, segment): the passes of a
+// trace hold a kernel or a few each, and a block of 256 threads per sum spent its time in barriers.
+__global__ void __launch_bounds__(256)
+segment_sum_planes_kernel(const float* __restrict__ values, int64_t plane_len, const int64_t* __restrict__ offsets,
+                          int64_t n_segments, int64_t n_sums, double* __restrict__ out) {
+  hb_grid_dependency_wait();
+  const int lane = threadIdx.x & 31;
+  for (int64_t w = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5); w < n_sums;
+       w += static_cast<int64_t>(gridDim.x) * 8) {
+    const int64_t plane = w / n_segments, s = w - plane * n_segments;
+    const int64_t lo = offsets[s], hi = offsets[s + 1];
+    const float* v = values + plane * plane_len;
+    double acc = 0.0;
+    for (int64_t i = lo + lane; i < hi; i += 32) acc += static_cast<double>(v[i]);
+    const double t = warp_sum(acc);
+    if (lane == 0) out[w] = t;
+  }
+}
+
+// special_scale_kernel over a grid of predictions [1 + T][n] (row 0: the origin's): ms[t][i] =
+// run_time[i] pred[1 + t][i] / pred[0][i], for up to four operation kinds at a time (blockIdx.y).
+struct ScaleGrid {
+  const float* run_time_ms;
+  const float* pred;
+  float* out_ms;
+  uint32_t* negative_count;
+  int32_t n, T;
+};
+struct ScaleGrids {
+  ScaleGrid g[4];
+};
+__global__ void __launch_bounds__(256) special_scale_grid_kernel(const __grid_constant__ ScaleGrids grids) {
+  hb_grid_dependency_wait();
+  const ScaleGrid& g = grids.g[blockIdx.y];
+  const int64_t total = static_cast<int64_t>(g.n) * g.T;
+  for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * 256; i0 < total; i0 += static_cast<int64_t>(gridDim.x) * 256) {
+    const int64_t i = i0 + threadIdx.x;
+    bool neg = false;
+    if (i < total) {
+      const int64_t k = i % g.n;
+      double v = static_cast<double>(g.run_time_ms[k]) * static_cast<double>(g.pred[g.n + i]) /
+                 static_cast<double>(g.pred[k]);
+      neg = v < 0;
+      if (neg) v = 0.0;
+      g.out_ms[i] = static_cast<float>(v);
+    }
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, neg);
+    if (g.negative_count && (threadIdx.x & 31) == 0 && m) atomicAdd(g.negative_count, __popc(m));
+  }
+}
+
+// Totals of iterations: a warp per (iteration, destination) adds the iteration's overheads, its kernels'
+// times and, kind by kind, its special operations' times (formed here from the prediction grid and rounded to
+// float32 as hb_special_scale stores them).  Nothing in between is written: the separate sums, ratios and
+// repeats took about thirty launches per pass.  Reads each input once per destination, from L2.
+constexpr int kIterKinds = 8;
+struct IterKind {
+  const float* rt;
+  const float* pred;
+  const int64_t* offsets;
+  int64_t n;
+};
+struct IterParams {
+  const float* overhead;
+  const float* measured;
+  const float* scaled;
+  const int64_t* offsets;
+  double* out;
+  int64_t K, I;
+  int32_t D, n_kinds, add;            // add: on top of what out holds
+  int8_t plane[HB_MAX_DEVICES];       // row of the prediction grids, 0 for the origin itself
+  IterKind kind[kIterKinds];
+};
+__global__ void __launch_bounds__(256) iteration_totals_kernel(const __grid_constant__ IterParams p) {
+  hb_grid_dependency_wait();
+  const int lane = threadIdx.x & 31;
+  const int64_t w = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (w >= p.I * p.D) return;
+  const int64_t i = w / p.D;
+  const int d = static_cast<int>(w - i * p.D), plane = p.plane[d];
+  double total = 0.0;
+  if (p.add) {
+    total = p.out[w];
+  } else {
+    const float* t = plane == 0 ? p.measured : p.scaled + d * p.K;
+    double over = 0.0, kern = 0.0;
+    for (int64_t k = p.offsets[i] + lane; k < p.offsets[i + 1]; k += 32) {
+      over += static_cast<double>(p.overhead[k]);
+      kern += static_cast<double>(t[k]);
+    }
+    total = (warp_sum(over) + warp_sum(kern)) / 1e6;   // lane 0
+  }
+  for (int q = 0; q < p.n_kinds; ++q) {
+    const IterKind& kind = p.kind[q];
+    double acc = 0.0;
+    for (int64_t k = kind.offsets[i] + lane; k < kind.offsets[i + 1]; k += 32) {
+      float ms = kind.rt[k];
+      if (plane != 0) {
+        const double v = static_cast<double>(ms) * static_cast<double>(kind.pred[plane * kind.n + k]) /
+                         static_cast<double>(kind.pred[k]);
+        ms = static_cast<float>(v < 0 ? 0.0 : v);
+      }
+      acc += static_cast<double>(ms);
+    }
+    total += warp_sum(acc);
+  }
+  if (lane == 0) p.out[w] = total;
+}
+
 // Per-GPU scratch of the two-stage sums.  A buffer that a launch may still be reading (or
 // that a captured graph refers to) is never freed: when more room is needed a larger buffer
 // is allocated and the old one is kept until the process ends.
@@ -192,6 +301,91 @@ extern "C" hb_status hb_special_scale(const float* run_time_ms, const float* pre
                          static_cast<cudaStream_t>(stream)>>>(run_time_ms, pred_dest, pred_orig, n,
                                                               out_ms, negative_count);
   HB_CUDA_TRY(cudaGetLastError());
+  return HB_OK;
+}
+
+extern "C" hb_status hb_segment_sum_planes(const float* values, int64_t plane_len, int32_t n_planes,
+                                           const int64_t* offsets, int64_t n_segments, double* out, void* stream) {
+  if (n_segments < 0 || n_planes < 0 || plane_len < 0 ||
+      (n_segments > 0 && n_planes > 0 && (!values || !offsets || !out))) {
+    hb::set_error("hb_segment_sum_planes: bad arguments");
+    return HB_ERR_INVALID_ARGUMENT;
+  }
+  const int64_t sums = n_segments * n_planes;
+  if (sums == 0) return HB_OK;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int64_t blocks = (sums + 7) / 8 < 148 * 8 ? (sums + 7) / 8 : 148 * 8;
+  HB_CUDA_TRY(hb::launch_overlapped(segment_sum_planes_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, s,
+                                    values, plane_len, offsets, n_segments, sums, out));
+  return HB_OK;
+}
+
+extern "C" hb_status hb_iteration_totals(const float* overhead_ns, const float* run_time_ns, const float* scaled_ns,
+                                         int64_t n_kernels, const int64_t* kernel_offsets, int64_t n_iterations,
+                                         int32_t n_destinations, const uint8_t* same, const hb_iteration_kind* kinds,
+                                         int32_t n_kinds, double* out, void* stream) {
+  if (n_iterations < 0 || n_destinations < 0 || n_destinations > HB_MAX_DEVICES || n_kinds < 0 || n_kernels < 0 ||
+      (n_kinds > 0 && !kinds) ||
+      (n_iterations > 0 && n_destinations > 0 &&
+       (!kernel_offsets || !same || !out || (n_kernels > 0 && (!overhead_ns || !run_time_ns || !scaled_ns))))) {
+    hb::set_error("hb_iteration_totals: bad arguments");
+    return HB_ERR_INVALID_ARGUMENT;
+  }
+  if (n_iterations == 0 || n_destinations == 0) return HB_OK;
+  IterParams p{};
+  p.overhead = overhead_ns; p.measured = run_time_ns; p.scaled = scaled_ns; p.offsets = kernel_offsets; p.out = out;
+  p.K = n_kernels; p.I = n_iterations; p.D = n_destinations;
+  int other = 0;
+  for (int d = 0; d < n_destinations; ++d) p.plane[d] = static_cast<int8_t>(same[d] ? 0 : ++other);
+  const int64_t blocks = (n_iterations * n_destinations + 7) / 8;
+  if (blocks > 0x7FFFFFFF) {
+    hb::set_error("hb_iteration_totals: too many iterations for one launch");
+    return HB_ERR_TOO_LARGE;
+  }
+  int done = 0;
+  do {
+    p.n_kinds = 0;
+    for (; done < n_kinds && p.n_kinds < kIterKinds; ++done) {
+      const hb_iteration_kind& k = kinds[done];
+      if (k.n == 0) continue;
+      if (k.n < 0 || !k.run_time_ms || !k.offsets || (other > 0 && !k.pred)) {
+        hb::set_error("hb_iteration_totals: bad kind %d", done);
+        return HB_ERR_INVALID_ARGUMENT;
+      }
+      p.kind[p.n_kinds++] = IterKind{k.run_time_ms, k.pred, k.offsets, k.n};
+    }
+    HB_CUDA_TRY(hb::launch_overlapped(iteration_totals_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0,
+                                      static_cast<cudaStream_t>(stream), p));
+    p.add = 1;
+  } while (done < n_kinds);
+  return HB_OK;
+}
+
+extern "C" hb_status hb_special_scale_grid(const hb_scale_grid* items, int32_t n_items, void* stream) {
+  if (n_items < 0 || n_items > 4 || (n_items > 0 && !items)) {
+    hb::set_error("hb_special_scale_grid: 0 to 4 kinds");
+    return HB_ERR_INVALID_ARGUMENT;
+  }
+  ScaleGrids grids{};
+  int kinds = 0;
+  int64_t most = 0;
+  for (int i = 0; i < n_items; ++i) {
+    const hb_scale_grid& g = items[i];
+    if (g.n < 0 || g.n > 0x7FFFFFFF || g.n_destinations < 0 ||
+        (g.n > 0 && g.n_destinations > 0 && (!g.run_time_ms || !g.pred || !g.out_ms))) {
+      hb::set_error("hb_special_scale_grid: bad kind %d", i);
+      return HB_ERR_INVALID_ARGUMENT;
+    }
+    const int64_t total = g.n * g.n_destinations;
+    if (total == 0) continue;
+    grids.g[kinds++] = ScaleGrid{g.run_time_ms, g.pred, g.out_ms, g.negative_count, static_cast<int32_t>(g.n),
+                                 g.n_destinations};
+    most = total > most ? total : most;
+  }
+  if (kinds == 0) return HB_OK;
+  const int64_t blocks = (most + 255) / 256 < 148 * 8 ? (most + 255) / 256 : 148 * 8;
+  HB_CUDA_TRY(hb::launch_overlapped(special_scale_grid_kernel, dim3(static_cast<unsigned>(blocks), kinds), dim3(256), 0,
+                                    static_cast<cudaStream_t>(stream), grids));
   return HB_OK;
 }
 

@@ -6,16 +6,15 @@ every iteration is a list of wave-scaled kernels (one operation each, with its
 launch overhead) and of MLP-predicted operations; the result is the predicted
 iteration time on every destination.  Everything between the inputs and the
 [iterations, destinations] totals stays on the device: the wave-scale kernel,
-the fused MLP chain per operation kind, the ratio/clamp kernel and the
-fixed-order float64 segment sums.
+the fused MLP chain of every operation kind side by side, and one kernel that forms
+the ratios and adds everything up in a fixed order (float64).
 """
 from dataclasses import dataclass
 from typing import Dict, Sequence
 
-import numpy as np
 import torch
 
-from habitat_b200 import batched
+from habitat_b200 import _native, batched
 
 
 @dataclass
@@ -40,37 +39,18 @@ def predict_iteration_totals(kernels: batched.KernelBatch, overhead_ns: torch.Te
 
     A destination with the origin's name keeps the measured times, as
     MeasuredOperation.to_device does (analysis/operation.py:82-85)."""
-    I = kernel_offsets.numel() - 1
-    D = len(dests)
     res = batched.wave_scale(kernels, origin, dests)
-    # sum over kernels of (overhead + scaled) = sum(overhead) + sum(scaled): linear, so the
-    # two segment sums replace a per-kernel add
-    over = batched.segment_sum(overhead_ns, kernel_offsets)                       # [I]
-    measured_kernels = batched.segment_sum(kernels.run_time_ns, kernel_offsets)  # [I]
-    totals = torch.empty((I, D), dtype=torch.float64, device=overhead_ns.device)
-    same = [d.name == origin.name for d in dests]
-    for d in range(D):
-        if same[d]:
-            totals[:, d] = (over + measured_kernels) / 1e6
-        else:
-            totals[:, d] = (over + batched.segment_sum(res.scaled_ns[d], kernel_offsets)) / 1e6
-    for ops in special.values():
-        n = ops.features.shape[0]
-        if n == 0:
-            continue
-        rows = [origin_mlp_row] + [r for r, s in zip(dest_mlp_rows, same) if not s]
-        T = len(rows) - 1
-        measured = batched.segment_sum(ops.run_time_ms, ops.offsets)
-        if T:
-            feats = ops.features.repeat(T + 1, 1)
-            rws = torch.tensor(rows, dtype=torch.uint8, device=feats.device).repeat_interleave(n)
-            pred = ops.handle.predict(feats, rws)
-            ms = batched.special_scale(ops.run_time_ms.repeat(T), pred[n:], pred[:n].repeat(T)).view(T, n)
-        t = 0
-        for d in range(D):
-            if same[d]:
-                totals[:, d] += measured
-            else:
-                totals[:, d] += batched.segment_sum(ms[t].contiguous(), ops.offsets)
-                t += 1
+    same = bytes(d.name == origin.name for d in dests)
+    rows = bytes([origin_mlp_row] + [r for r, s in zip(dest_mlp_rows, same) if not s])
+    kinds = [(ops.handle._handle.value or 0, ops.features, ops.run_time_ms, ops.offsets, rows)
+             for ops in special.values() if ops.features.shape[0]]
+    totals = _native.binding().iteration_totals(kernels, res.scaled_ns, overhead_ns, kernel_offsets, same, kinds)
+    if totals is None:
+        batched._require_cuda(overhead_ns, torch.float32, "overhead_ns")
+        batched._require_cuda(kernel_offsets, torch.int64, "kernel_offsets")
+        for ops in special.values():
+            batched._require_cuda(ops.features, torch.float32, "features")
+            batched._require_cuda(ops.run_time_ms, torch.float32, "run_time_ms")
+            batched._require_cuda(ops.offsets, torch.int64, "offsets")
+        raise ValueError("overheads, features, measured times and offsets have to fit the kernels and iterations")
     return totals, res

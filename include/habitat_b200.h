@@ -227,6 +227,23 @@ void hb_mlp_destroy(hb_mlp* handle);
 hb_status hb_mlp_predict(hb_mlp* handle, const float* op_features, const uint8_t* device_row,
                          int64_t Q, float* out, void* stream);
 
+/* The same n feature rows asked about for each of a few devices (an operation's origin and its candidate
+ * destinations, analysis/predictor.py:132-148 of the reference): out[b * n + i] is row i on the device
+ * device_rows[b] (host array, at most 80 entries).  Up to four batches of different predictors per call;
+ * they read nothing of one another and run side by side on the stream. */
+typedef struct hb_mlp_grid {
+  hb_mlp* handle;
+  const float* op_features;     /* [n][F] */
+  int64_t n;
+  const uint8_t* device_rows;   /* host, [n_device_rows] */
+  int32_t n_device_rows;
+  float* out;                   /* [n_device_rows][n] */
+} hb_mlp_grid;
+hb_status hb_mlp_predict_grid(const hb_mlp_grid* items, int32_t n_items, void* stream);
+
+/* hb_mlp_status without the synchronisation: judges the launches that have ended. */
+hb_status hb_mlp_poll_status(hb_mlp* handle, int32_t* device_status);
+
 /* Synchronises with the device and reports whether any launch on this handle
  * gave up on a bounded device-side wait (HB_ERR_DEVICE_TIMEOUT; *device_status
  * names the waiting role and site) since the last call that reported one: the
@@ -272,6 +289,40 @@ hb_status hb_special_scale(const float* run_time_ms, const float* pred_dest,
  * float64, fixed summation order (results do not depend on the launch). */
 hb_status hb_segment_sum(const float* values, const int64_t* offsets, int64_t n_segments,
                          double* out, void* stream);
+
+/* hb_segment_sum over n_planes planes of plane_len values that share the offsets (the passes of a trace on
+ * every destination): out[p * n_segments + s]. */
+hb_status hb_segment_sum_planes(const float* values, int64_t plane_len, int32_t n_planes, const int64_t* offsets,
+                                int64_t n_segments, double* out, void* stream);
+
+/* hb_special_scale over the predictions hb_mlp_predict_grid leaves when the origin comes first:
+ * out_ms[t * n + i] = max(0, run_time_ms[i] * pred[(1 + t) * n + i] / pred[i]); up to four kinds per call. */
+typedef struct hb_scale_grid {
+  const float* run_time_ms;     /* [n] */
+  const float* pred;            /* [1 + n_destinations][n] */
+  int64_t n;
+  int32_t n_destinations;
+  float* out_ms;                /* [n_destinations][n] */
+  uint32_t* negative_count;     /* incremented per clamped prediction, or NULL */
+} hb_scale_grid;
+hb_status hb_special_scale_grid(const hb_scale_grid* items, int32_t n_items, void* stream);
+
+/* Trace.to_device(...).run_time_ms (analysis/trace.py:26-51 over predictor.py:84-148) for many traces
+ * ("iterations") at once, from predictions that are on the device: out[i * n_destinations + d] = (sum of the
+ * overheads and of the predicted kernel times of iteration i) / 1e6 + the sums of its special operations'
+ * predicted times, float64.  A destination d with same[d] != 0 is the origin itself and keeps the measured
+ * times.  The prediction grids of the kinds (hb_mlp_predict_grid, origin first) hold the other destinations
+ * in order. */
+typedef struct hb_iteration_kind {
+  const float* run_time_ms;     /* [n] measured on the origin */
+  const float* pred;            /* [1 + other destinations][n], or NULL when every destination is the origin */
+  const int64_t* offsets;       /* [n_iterations + 1] */
+  int64_t n;
+} hb_iteration_kind;
+hb_status hb_iteration_totals(const float* overhead_ns, const float* run_time_ns, const float* scaled_ns,
+                              int64_t n_kernels, const int64_t* kernel_offsets, int64_t n_iterations,
+                              int32_t n_destinations, const uint8_t* same /* host */, const hb_iteration_kind* kinds,
+                              int32_t n_kinds, double* out, void* stream);
 
 /* Sum of each of n_planes contiguous planes of plane_len float32 values,
  * skipping NaN entries (pairs the reference would have raised on); used for
