@@ -49,30 +49,42 @@
 
 namespace {
 
-struct MlpParams {
-  const uint8_t* wpack;      // weight tile images, producer order
+// One predictor and its batch of queries.
+struct MlpProblem {
   const float* bias;         // [layers + 1][1024]: fc1, hidden...
   const float* fc2_w;        // [1024]
   float fc2_b;
+  int32_t first_tile;        // of the launch's tiles
   const double* mu;          // [F + 4]
   const double* sigma;       // [F + 4]
   const double* dev_feat;    // [n_dev][4]
   int32_t n_dev;
   int32_t n_op_feat;         // F
   int32_t layers;            // hidden layers
+  int32_t grid_n;            // > 0: query q is feature row q % grid_n on device grid_rows[q / grid_n]
   const float* feats;        // [Q][F]
   const uint8_t* dev_row;    // [Q]
   int64_t Q;
   float* out;                // [Q]
-  int32_t num_tiles;
-  int32_t* status;           // device word: 0 ok, else (role << 8 | site)
-  long long* phase_cycles;   // [16] cluster 0: cycle counters of the roles (diagnostic), or null
-  int32_t beside;            // runs beside the launch before it on the stream: nothing to wait for
-  int32_t grid_n;            // > 0: query q is feature row q % grid_n on device grid_rows[q / grid_n]
+  int32_t* status;           // 0 ok, else (role << 8 | site)
   uint8_t grid_rows[hb::kMaxGridRows];
-  CUtensorMap tmap_slot;     // pair kernel: the pack as [rows][128 B], box of two tile images (32 KB)
+  CUtensorMap tmap_slot;     // the weight pack as [rows][128 B], box of two tile images (32 KB)
   CUtensorMap tmap_tile;     // same tensor, box of one tile image (16 KB, fc1)
 };
+// A launch takes the tiles of up to four predictors, one after the other in one list, so that only the
+// list's end leaves SMs idle.
+struct MlpParams {
+  int32_t num_tiles;
+  int32_t n_problems;
+  int32_t beside;            // runs beside the launch before it on the stream: nothing to wait for
+  long long* phase_cycles;   // [16] cluster 0: cycle counters of the roles (diagnostic), or null
+  MlpProblem prob[hb::kMaxLanes];
+};
+__device__ __forceinline__ const MlpProblem& problem_of(const MlpParams& p, int tile) {
+  int k = 0;
+  for (int i = 1; i < p.n_problems; ++i) k += tile >= p.prob[i].first_tile ? 1 : 0;
+  return p.prob[k];
+}
 
 // ---------------------------------------------------------------------------
 // The kernel.  A single CTA can only keep 64 queries on chip,
@@ -164,9 +176,10 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
   const uint32_t bar_inq = bars + 192;       // [4] peer's half of K quarter q landed here (bytes)
   const uint32_t bar_tfree = bars + 224;     // [4] leader only: TMEM block j read out in both CTAs (8 warps)
   const uint32_t bar_fc2 = bars + 256;       // peer's fc2 partial sums arrived
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_ptr + 264);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + 268);
-  volatile int* epi_ok = reinterpret_cast<volatile int*>(bars_ptr + 272);   // [2], one per epilogue group
+  const uint32_t bar_next = bars + 264;      // the tile is done with the activation buffer (8 warps)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_ptr + 272);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + 276);
+  volatile int* epi_ok = reinterpret_cast<volatile int*>(bars_ptr + 280);   // [5]: per epilogue group, twice; the hand-over of fc2
   float* fc2_mine = reinterpret_cast<float*>(bars_ptr + 512);    // [64] own queries, own features
   float* fc2_peer = reinterpret_cast<float*>(bars_ptr + 768);    // [64] own queries, peer's features
 
@@ -187,6 +200,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
       mbar_init(bar_tfree + 8 * q, 8);  // one arrive per epilogue warp of the block, both CTAs
     }
     mbar_init(bar_fc2, 1);
+    mbar_init(bar_next, 8);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -204,19 +218,23 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const int n_layers = p.layers + 1;
   const int n_pairs = static_cast<int>(gridDim.x >> 1);
   const int pair_id = static_cast<int>(blockIdx.x >> 1);
   int my_tiles = 0;
   if (pair_id < p.num_tiles) my_tiles = (p.num_tiles - 1 - pair_id) / n_pairs + 1;
 
   uint32_t issued = 0;
+  auto publish = [&](uint32_t q) {   // "this CTA's share of K quarter q is in place"
+    const uint32_t bar = bar_actq + 8 * q;
+    if (rank == 0) mbar_arrive(bar);
+    else mbar_arrive_remote(map_to_cta(bar, 0));
+  };
 
-  if (warp >= 6 && warp < 12) {
+  if (warp >= 6 && warp < 6 + kPairStages) {
     // ------------------------------ producers -----------------------------
     // One producer per ring slot.  The pack is laid out per 128-feature block
     // (layer -> block -> K block); this CTA streams blocks 2 j + rank.
-    if (lane == 0 && warp - 6 < kPairStages) {
+    if (lane == 0) {
       const uint32_t w = static_cast<uint32_t>(warp - 6);
       uint32_t it = 0;
       bool ok = true;
@@ -224,6 +242,8 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
       const uint32_t peer_full_leader = map_to_cta(bar_full + 8 * w, 0);
       long long pc_empty = 0, pc_copy = 0, pc_n = 0;
       for (int t = 0; t < my_tiles && ok; ++t) {
+        const MlpProblem& pb = problem_of(p, pair_id + t * n_pairs);
+        const int n_layers = pb.layers + 1;
         size_t layer_base = 0;   // in tile images
         for (int L = 0; L < n_layers && ok; ++L) {
           const int nkb = L == 0 ? 1 : kNumKB;
@@ -241,18 +261,18 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
                 if (it % kPairStages != w) continue;
                 const uint32_t ph = (it / kPairStages) & 1u;
                 const long long q0 = ptimed ? clock64() : 0;
-                if (!mbar_wait(bar_empty + 8 * w, ph ^ 1u, abort_flag, p.status, 0x111)) { ok = false; break; }
+                if (!mbar_wait(bar_empty + 8 * w, ph ^ 1u, abort_flag, pb.status, 0x111)) { ok = false; break; }
                 const long long q1 = ptimed ? clock64() : 0;
                 // both CTAs' boxes are counted on the leader's barrier
                 if (rank == 0) mbar_expect_tx(bar_full + 8 * w, 2 * load_bytes);
                 // bf16: a slot takes two consecutive K blocks (16 KB images); split: the hi and lo
                 // image of one K block (stored back to back)
-                tma_rows_2sm(stage0 + w * kPairStageBytes, nkb == 1 ? &p.tmap_tile : &p.tmap_slot,
+                tma_rows_2sm(stage0 + w * kPairStageBytes, nkb == 1 ? &pb.tmap_tile : &pb.tmap_slot,
                              static_cast<int32_t>((blk + (SPLIT ? 1 : kPairSlotKb) * g) * kRowsPerImage),
                              peer_full_leader);
                 issued = it + 1;
                 if (ptimed) {
-                  mbar_wait(bar_full + 8 * w, ph, abort_flag, p.status, 0x112);
+                  mbar_wait(bar_full + 8 * w, ph, abort_flag, pb.status, 0x112);
                   pc_empty += q1 - q0; pc_copy += clock64() - q1; ++pc_n;
                 }
               }
@@ -283,9 +303,10 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
         uint32_t s = 0, ph = 0, par = 0;
         const bool mtimed = p.phase_cycles != nullptr && blockIdx.x == 0;
         long long mc_act = 0, mc_full = 0, mc_tfree = 0, mc_n = 0;
+        int32_t* status = nullptr;
         auto wait = [&](uint32_t bar, uint32_t parity, long long& acc, int code) {
           const long long m0 = mtimed ? clock64() : 0;
-          mbar_wait_cluster(bar, parity, abort_flag, p.status, code);
+          mbar_wait_cluster(bar, parity, abort_flag, status, code);
           tc_fence_after();
           if (mtimed) acc += clock64() - m0;
         };
@@ -293,6 +314,9 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
         const unsigned long long g0 = global_timer_ns();
 #pragma unroll 1
         for (int t = 0; t < my_tiles; ++t) {
+          const MlpProblem& pb = problem_of(p, pair_id + t * n_pairs);
+          const int n_layers = pb.layers + 1;
+          status = pb.status;
           // fc1 reads K block 0, written after the previous tile's TMEM was read out
           wait(bar_actq, par & 1u, mc_act, 0x211);
           par ^= 1u;
@@ -369,7 +393,63 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
       }
       __syncwarp();
     }
-  } else if (warp >= 2) {
+  } else if (warp == 9 || warp == 10) {
+    // ------------------------------ features ------------------------------
+    // One B column (query) per thread.  The next tile's features are loaded, normalised (float64) and split
+    // into bf16 hi + lo while the tensor core works on the current tile; at the tile's end only the stores
+    // are left.  SPLIT: columns 32..63 are the lo parts of the hidden layers; fc1 carries its own hi/lo
+    // expansion along K, so they are zero here.
+    const int T = static_cast<int>(threadIdx.x) - 9 * 32;
+    for (int t = 0; t < my_tiles; ++t) {
+      const int tile = pair_id + t * n_pairs;
+      const MlpProblem& pb = problem_of(p, tile);
+      const int C_in = pb.n_op_feat + 4;
+      const int64_t q = static_cast<int64_t>(tile - pb.first_tile) * kTileQ + static_cast<int64_t>(rank) * kHalfQ + T;
+      uint32_t x2[kMaxInFeat];             // hi | lo << 16
+#pragma unroll
+      for (int c = 0; c < kMaxInFeat; ++c) x2[c] = 0;
+      if (T < kHalfQ && q < pb.Q) {
+        int64_t fr = q;
+        int dr;
+        if (pb.grid_n) {
+          const uint32_t block = static_cast<uint32_t>(q) / static_cast<uint32_t>(pb.grid_n);
+          fr -= static_cast<int64_t>(block) * pb.grid_n;
+          dr = pb.grid_rows[block];
+        } else {
+          dr = pb.dev_row[q];
+        }
+        dr = dr < pb.n_dev ? dr : pb.n_dev - 1;
+#pragma unroll
+        for (int c = 0; c < kMaxInFeat; ++c) {
+          if (c >= C_in) continue;
+          const double x = c < pb.n_op_feat ? static_cast<double>(pb.feats[fr * pb.n_op_feat + c])
+                                            : pb.dev_feat[dr * 4 + (c - pb.n_op_feat)];
+          const float xn = static_cast<float>((x - pb.mu[c]) / pb.sigma[c]);
+          const __nv_bfloat16 hi = __float2bfloat16_rn(xn);
+          const __nv_bfloat16 lo = __float2bfloat16_rn(xn - __bfloat162float(hi));
+          x2[c] = static_cast<uint32_t>(__bfloat16_as_ushort(hi)) | static_cast<uint32_t>(__bfloat16_as_ushort(lo)) << 16;
+        }
+      }
+      if (t > 0) {
+        if (lane == 0) mbar_wait(bar_next, (t - 1) & 1, abort_flag, pb.status, 0x411);
+        __syncwarp();
+      }
+      // K rows: [hi | lo | hi], then zeros (row k, query n: 128 k + 16 ((n / 8) xor (k mod 8)) + 2 (n mod 8))
+      for (int i = T; i < (kKBlk - 3 * C_in) * 8; i += 64)
+        *reinterpret_cast<uint4*>(base_ptr + 3 * C_in * 128 + 16 * i) = make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int c = 0; c < kMaxInFeat; ++c) {
+        if (c >= C_in) continue;
+        const uint16_t hi = static_cast<uint16_t>(x2[c]), lo = static_cast<uint16_t>(x2[c] >> 16);
+        *reinterpret_cast<uint16_t*>(base_ptr + mn_off(c, T)) = hi;
+        *reinterpret_cast<uint16_t*>(base_ptr + mn_off(C_in + c, T)) = lo;
+        *reinterpret_cast<uint16_t*>(base_ptr + mn_off(2 * C_in + c, T)) = hi;
+      }
+      fence_proxy_async();
+      asm volatile("bar.sync 4, 64;" ::: "memory");
+      if (T == 0) publish(0);
+    }
+  } else if (warp >= 2 && (warp < 6 || warp >= 12)) {
     // ------------------------------ epilogue ------------------------------
     // Two groups of four warps (warps 2-5 and 12-15); a warp may only read the
     // TMEM lane quadrant (warp id mod 4).  Group g drains the 256-feature blocks
@@ -380,7 +460,6 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
     const int quad = warp & 3;
     const int r = quad * 32 + lane;            // feature row inside this CTA's 128-row block
     const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
-    const int C_in = p.n_op_feat + 4;
     const uint32_t act_peer = map_to_cta(act, peer);
     uint32_t in_phase = 0, lay = 0, tile_no = 0;
     bool ok = true;
@@ -389,57 +468,14 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
     long long c_wait = 0, c_epi = 0, c_fc2 = 0, c_layers = 0, c_ld = 0, c_bias = 0, c_sync = 0, c_loc = 0, c_rem = 0;
     // named barrier of this group alone (ids 2 and 3; id 1 joins both groups)
     auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory"); };
-    auto publish = [&](uint32_t q) {   // "this CTA's share of K quarter q is in place"
-      const uint32_t bar = bar_actq + 8 * q;
-      if (rank == 0) mbar_arrive(bar);
-      else mbar_arrive_remote(map_to_cta(bar, 0));
-    };
-
     for (int t = 0; t < my_tiles && ok; ++t, ++tile_no) {
       const int tile = pair_id + t * n_pairs;
-      const int64_t q0 = static_cast<int64_t>(tile) * kTileQ + static_cast<int64_t>(rank) * kHalfQ;
-
-      if (T < kPairHalfQ) {
-        // one B column per thread: a query's split features (SPLIT: columns 32..63 are the lo parts
-        // of the hidden layers; fc1 carries its own hi/lo expansion along K, so they are zero here)
-        const int64_t q = q0 + T;
-        __nv_bfloat16 row[kKBlk];
-#pragma unroll
-        for (int c = 0; c < kKBlk; ++c) row[c] = __float2bfloat16_rn(0.0f);
-        if (T < kHalfQ && q < p.Q) {
-          int64_t fr = q;
-          int dr;
-          if (p.grid_n) {
-            const uint32_t block = static_cast<uint32_t>(q) / static_cast<uint32_t>(p.grid_n);
-            fr -= static_cast<int64_t>(block) * p.grid_n;
-            dr = p.grid_rows[block];
-          } else {
-            dr = p.dev_row[q];
-          }
-          dr = dr < p.n_dev ? dr : p.n_dev - 1;
-          for (int c = 0; c < C_in; ++c) {
-            const double x = c < p.n_op_feat
-                                 ? static_cast<double>(p.feats[fr * p.n_op_feat + c])
-                                 : p.dev_feat[dr * 4 + (c - p.n_op_feat)];
-            const float xn = static_cast<float>((x - p.mu[c]) / p.sigma[c]);
-            const __nv_bfloat16 hi = __float2bfloat16_rn(xn);
-            const __nv_bfloat16 lo = __float2bfloat16_rn(xn - __bfloat162float(hi));
-            row[c] = hi;
-            row[C_in + c] = lo;
-            row[2 * C_in + c] = hi;
-          }
-        }
-        // column T of K rows 0..63 (row k, query n: 128 k + 16 ((n / 8) xor (k mod 8)) + 2 (n mod 8))
-#pragma unroll
-        for (int c = 0; c < kKBlk; ++c)
-          *reinterpret_cast<__nv_bfloat16*>(base_ptr + mn_off(static_cast<uint32_t>(c), static_cast<uint32_t>(T))) = row[c];
-      }
-      fence_proxy_async();
-      pair_epi_bar_sync();
-      if (T == 0) publish(0);
+      const MlpProblem& pb = problem_of(p, tile);
+      const int n_layers = pb.layers + 1;
+      const int64_t q0 = static_cast<int64_t>(tile - pb.first_tile) * kTileQ + static_cast<int64_t>(rank) * kHalfQ;
 
       for (int L = 0; L < n_layers && ok; ++L, ++lay) {
-        const float* bias = p.bias + L * kWidth;
+        const float* bias = pb.bias + L * kWidth;
         const bool last = (L == n_layers - 1);
         if (!last) {
           // Group g drains output blocks g and g + 2.  Block j becomes K quarter j of the next
@@ -452,7 +488,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
             const int gate = L == 0 ? 3 : j;
             const long long c0 = timed ? clock64() : 0;
             if (e == 0) {
-              epi_ok[grp] = mbar_wait(bar_accj + 8 * gate, lay & 1u, abort_flag, p.status, 0x311) ? 1 : 0;
+              epi_ok[grp] = mbar_wait(bar_accj + 8 * gate, lay & 1u, abort_flag, pb.status, 0x311) ? 1 : 0;
               // the peer sends 128 K rows x 128 B of this quarter into this CTA
               mbar_expect_tx(bar_inq + 8 * j, 128u * 128u);
             }
@@ -531,7 +567,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
             group_sync();
             if (e == 0) {
               // own stores are fenced above; the peer's arrive as counted bytes
-              if (mbar_wait_cluster(bar_inq + 8 * j, in_phase, abort_flag, p.status, 0x313))
+              if (mbar_wait_cluster(bar_inq + 8 * j, in_phase, abort_flag, pb.status, 0x313))
                 publish(static_cast<uint32_t>(j));
             }
             if (timed) { c_wait += c1 - c0; c_epi += clock64() - c1; c_sync += clock64() - d2; }
@@ -539,27 +575,34 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
           in_phase ^= 1u;
           if (timed) ++c_layers;
         } else {
-          const long long c0 = timed ? clock64() : 0;
-          if (T == 0) epi_ok[0] = mbar_wait(bar_accj + 8 * 3, lay & 1u, abort_flag, p.status, 0x311) ? 1 : 0;
-          pair_epi_bar_sync();
-          if (epi_ok[0] == 0) { ok = false; break; }
-          tc_fence_after();
-          const long long c1 = timed ? clock64() : 0;
-          // fc2 over this CTA's 512 features, 32 queries at a time (bf16: the four column quarters
-          // of the 128 queries; split: the two CTAs' 32 queries, hi and lo columns added first).
-          // A warp multiplies its 32 features of a block and adds them over its lanes with the
-          // transposing tree (31 shuffles leave one query per lane); the eight warps' sums of a query
-          // meet in shared memory once, after all columns.
+          // fc2 over this CTA's 512 features, a group's two blocks as they complete (the tensor core still
+          // works on the later ones), 32 queries at a time (bf16: the four column quarters of the 128
+          // queries; split: the two CTAs' 32 queries, hi and lo columns added first).  A warp multiplies its
+          // 32 features of a block and adds them over its lanes with the transposing tree (31 shuffles leave
+          // one query per lane); the eight warps' sums of a query meet in shared memory once, after all
+          // columns and blocks.
           constexpr int kChunks = SPLIT ? 2 : 4;
+          float part[kChunks];
+#pragma unroll
+          for (int i = 0; i < kChunks; ++i) part[i] = 0.0f;
+          long long c1 = 0;
 #pragma unroll 1
-          for (int qd = 0; qd < kChunks; ++qd) {
-            float part = 0.0f;
-#pragma unroll 1
-            for (int jj = 0; jj < 2; ++jj) {
-              const int j = grp * 2 + jj;
-              const int f = j * 256 + static_cast<int>(rank) * 128 + r;
-              const float b = __ldg(bias + f);
-              const float w = __ldg(p.fc2_w + f);
+          for (int jj = 0; jj < 3 && ok; ++jj) {
+            // third round: everything has been accumulated, the activation buffer is free
+            const int j = jj < 2 ? grp + 2 * jj : 3;
+            const long long c0 = timed ? clock64() : 0;
+            if (e == 0) epi_ok[grp + 2 * (jj & 1)] = mbar_wait(bar_accj + 8 * j, lay & 1u, abort_flag, pb.status, 0x311) ? 1 : 0;
+            group_sync();
+            if (epi_ok[grp + 2 * (jj & 1)] == 0) { ok = false; break; }
+            tc_fence_after();
+            c1 = timed ? clock64() : 0;
+            if (timed) c_wait += c1 - c0;
+            if (jj == 2) break;
+            const int f = j * 256 + static_cast<int>(rank) * 128 + r;
+            const float b = __ldg(bias + f);
+            const float w = __ldg(pb.fc2_w + f);
+#pragma unroll
+            for (int qd = 0; qd < kChunks; ++qd) {
               float v[32];
               if (SPLIT) {
                 float lo[32];
@@ -574,15 +617,25 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
               for (int i = 0; i < 32; ++i) v[i] = __fmul_rn(w, fmaxf(v[i] + b, 0.0f));
               fold16(v, lane);
               fold_lanes<2>(v, lane, 16);
-              part += v[0];
+              part[qd] += v[0];
             }
-            red[(grp * 4 + quad) * (kChunks * 32) + qd * 32 + fold16_col<32>(lane) + (lane >> 4)] = part;
+            if (timed) c_fc2 += clock64() - c1;
           }
+          if (!ok) break;
+#pragma unroll
+          for (int qd = 0; qd < kChunks; ++qd)
+            red[(grp * 4 + quad) * (kChunks * 32) + qd * 32 + fold16_col<32>(lane) + (lane >> 4)] = part[qd];
           pair_epi_bar_sync();
+          float tot = 0.0f;
           if (T < kChunks * 32) {
-            float tot = 0.0f;
 #pragma unroll
             for (int k2 = 0; k2 < 8; ++k2) tot += red[k2 * (kChunks * 32) + T];
+          }
+          // nothing of this tile is left in the activation buffer or in TMEM: the next tile's features may come
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_next);
+          if (T < kChunks * 32) {
             // which CTA owns the query, and its index among the owner's
             const uint32_t owner = static_cast<uint32_t>(T / kHalfQ);
             const int slot = T % kHalfQ;
@@ -590,20 +643,18 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
             else st_cluster_f32(map_to_cta(smem_u32(fc2_peer + slot), peer), tot);
           }
           pair_epi_bar_sync();
-          tc_fence_before();
           // hand-over of the partial sums, then the owner finishes its 64 queries
           if (T == 0) {
             mbar_arrive_remote(map_to_cta(bar_fc2, peer));
-            epi_ok[0] = mbar_wait_cluster(bar_fc2, tile_no & 1u, abort_flag, p.status, 0x312) ? 1 : 0;
+            epi_ok[4] = mbar_wait_cluster(bar_fc2, tile_no & 1u, abort_flag, pb.status, 0x312) ? 1 : 0;
           }
           pair_epi_bar_sync();
-          if (epi_ok[0] == 0) { ok = false; break; }
+          if (epi_ok[4] == 0) { ok = false; break; }
           if (T < kHalfQ) {
             const int64_t q = q0 + T;
-            if (q < p.Q) p.out[q] = fc2_mine[T] + fc2_peer[T] + p.fc2_b;
+            if (q < pb.Q) pb.out[q] = fc2_mine[T] + fc2_peer[T] + pb.fc2_b;
           }
-          pair_epi_bar_sync();
-          if (timed) { c_wait += c1 - c0; c_fc2 += clock64() - c1; ++c_layers; }
+          if (timed) { c_fc2 += clock64() - c1; ++c_layers; }
         }
       }
     }
@@ -617,7 +668,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
   // ------------------------------ teardown ------------------------------
   tc_fence_before();
   __syncthreads();
-  if (rank == 0 && warp >= 6 && warp < 12 && lane == 0 && *abort_flag && warp - 6 < kPairStages && issued > 0) {
+  if (rank == 0 && warp >= 6 && warp < 6 + kPairStages && lane == 0 && *abort_flag && issued > 0) {
     const uint32_t j = issued - 1;
     const uint32_t ph = (j / kPairStages) & 1u;
     const long long t0 = clock64();
@@ -842,45 +893,70 @@ extern "C" hb_status hb_mlp_create(hb_mlp** handle, int32_t n_op_features, int32
 }
 
 namespace {
-// Queues one batch (checked by the callers) on the kernel for its size.
-hb_status queue_batch(hb_mlp* h, const hb::MlpBatch& batch, cudaStream_t s) {
+// A launch of the two-SM kernel: batches of predictors of one precision.
+class ChainLaunch {
+ public:
+  ChainLaunch(const hb_mlp* h, bool split) : split_(split), pairs_(h->sm_count / 2) { p_.phase_cycles = h->phase_cycles; }
+  int64_t tiles_of(int64_t Q) const { const int q = split_ ? kPairQ / 2 : kPairQ; return (Q + q - 1) / q; }
+  // Rounds of tiles the SMs would walk with `more` tiles on top.
+  int64_t rounds(int64_t more) const { return (p_.num_tiles + more + pairs_ - 1) / pairs_; }
+  bool empty() const { return p_.n_problems == 0; }
+  hb_status add(const hb_mlp* h, const hb::MlpBatch& batch) {
+    const int64_t tiles = tiles_of(batch.Q);
+    if (p_.n_problems == hb::kMaxLanes || tiles + p_.num_tiles > 0x7FFFFFFF || (batch.grid_n && batch.Q > 0xFFFFFFFFll)) {
+      hb::set_error("hb_mlp_predict: Q too large for one launch");
+      return HB_ERR_TOO_LARGE;
+    }
+    MlpProblem& q = p_.prob[p_.n_problems++];
+    q.bias = h->bias; q.fc2_w = h->fc2_w; q.fc2_b = h->fc2_b; q.first_tile = p_.num_tiles;
+    q.mu = h->mu; q.sigma = h->sigma; q.dev_feat = h->dev_feat; q.n_dev = h->n_dev;
+    q.n_op_feat = h->n_op_feat; q.layers = h->layers; q.feats = batch.feats;
+    q.dev_row = batch.dev_row; q.Q = batch.Q; q.out = batch.out; q.status = h->status;
+    q.grid_n = batch.grid_n;
+    if (batch.grid_n) std::memcpy(q.grid_rows, batch.grid_rows, static_cast<size_t>(batch.Q / batch.grid_n));
+    q.tmap_slot = h->tmap_slot; q.tmap_tile = h->tmap_tile;
+    p_.num_tiles += static_cast<int32_t>(tiles);
+    return HB_OK;
+  }
+  hb_status go(bool beside, cudaStream_t s) {
+    p_.beside = beside ? 1 : 0;
+    // one cluster of two CTAs per tile (128 queries, 64 in split precision), at most one cluster per SM pair
+    const int pairs = p_.num_tiles < pairs_ ? p_.num_tiles : pairs_;
+    HB_CUDA_TRY(hb::launch_overlapped(split_ ? mlp_chain_pair_kernel<true> : mlp_chain_pair_kernel<false>,
+                                      dim3(2 * pairs), dim3(kPairThreads), kPairSmemBytes, s, p_));
+    return HB_OK;
+  }
+
+ private:
+  bool split_;
+  int pairs_;
+  MlpParams p_{};
+};
+
+hb_status check_device(const hb_mlp* h) {
   int cur = -1;
   HB_CUDA_TRY(cudaGetDevice(&cur));
-  if (cur != h->device) {
-    // the weight pack, the tensor maps and the status word live on the GPU the handle was created on
-    hb::set_error("hb_mlp_predict: the handle belongs to CUDA device %d but device %d is current", h->device, cur);
-    return HB_ERR_INVALID_ARGUMENT;
-  }
-  const bool split = h->precision == HB_PRECISION_BF16X3;
-  // HB_MLP_WIDE=0 keeps every batch on the two-SM kernel
+  if (cur == h->device) return HB_OK;
+  // the weight pack, the tensor maps and the scratch live on the GPU the handle was created on
+  hb::set_error("hb_mlp_predict: the handle belongs to CUDA device %d but device %d is current", h->device, cur);
+  return HB_ERR_INVALID_ARGUMENT;
+}
+
+// HB_MLP_WIDE=0 keeps every batch on the two-SM kernel
+hb::WidePlan plan_of(const hb_mlp* h, int64_t Q) {
   static const bool use_wide = [] { const char* e = std::getenv("HB_MLP_WIDE"); return !e || std::atoi(e) != 0; }();
-  if (use_wide) {
-    bool launched = false;
-    const hb_status st = hb::wide_predict(h, hb::wide_plan(batch.Q, split, h->sm_count), batch, s, &launched);
-    if (st != HB_OK || launched) return st;
-  }
-  const int tile_q = split ? kPairQ / 2 : kPairQ;
-  const int64_t tiles = (batch.Q + tile_q - 1) / tile_q;
-  if (tiles > 0x7FFFFFFF || (batch.grid_n && batch.Q > 0xFFFFFFFFll)) {
-    hb::set_error("hb_mlp_predict: Q too large for one launch");
-    return HB_ERR_TOO_LARGE;
-  }
-  MlpParams p{};
-  p.wpack = h->wpack; p.bias = h->bias; p.fc2_w = h->fc2_w; p.fc2_b = h->fc2_b;
-  p.mu = h->mu; p.sigma = h->sigma; p.dev_feat = h->dev_feat; p.n_dev = h->n_dev;
-  p.n_op_feat = h->n_op_feat; p.layers = h->layers; p.feats = batch.feats;
-  p.dev_row = batch.dev_row; p.Q = batch.Q; p.out = batch.out; p.num_tiles = static_cast<int32_t>(tiles);
-  p.grid_n = batch.grid_n;
-  if (batch.grid_n) std::memcpy(p.grid_rows, batch.grid_rows, static_cast<size_t>(batch.Q / batch.grid_n));
-  p.beside = batch.beside ? 1 : 0;
-  p.status = h->status;
-  p.phase_cycles = h->phase_cycles;
-  p.tmap_slot = h->tmap_slot; p.tmap_tile = h->tmap_tile;
-  // one cluster of two CTAs per tile (128 queries, 64 in split precision), at most one cluster per SM pair
-  const int pairs = static_cast<int>(tiles < h->sm_count / 2 ? tiles : h->sm_count / 2);
-  HB_CUDA_TRY(hb::launch_overlapped(split ? mlp_chain_pair_kernel<true> : mlp_chain_pair_kernel<false>, dim3(2 * pairs),
-                                    dim3(kPairThreads), kPairSmemBytes, s, p));
-  return HB_OK;
+  return use_wide ? hb::wide_plan(Q, h->precision == HB_PRECISION_BF16X3, h->sm_count) : hb::WidePlan{0, 0, 0, 0};
+}
+
+// Queues one batch (checked by the callers) on the kernel for its size.
+hb_status queue_batch(hb_mlp* h, const hb::MlpBatch& batch, cudaStream_t s) {
+  bool launched = false;
+  hb_status st = check_device(h);
+  if (st == HB_OK) st = hb::wide_predict(h, plan_of(h, batch.Q), batch, s, &launched);
+  if (st != HB_OK || launched) return st;
+  ChainLaunch launch(h, h->precision == HB_PRECISION_BF16X3);
+  st = launch.add(h, batch);
+  return st != HB_OK ? st : launch.go(batch.beside, s);
 }
 }  // namespace
 
@@ -909,26 +985,53 @@ extern "C" hb_status hb_mlp_predict_grid(const hb_mlp_grid* items, int32_t n_ite
       return HB_ERR_INVALID_ARGUMENT;
     }
   }
-  // The largest first: its launch waits for what is on the stream, the others run beside it on the SMs
-  // that its last wave leaves idle.
+  // The largest first: its launch waits for what is on the stream, the others run beside it.  Batches that
+  // fill SM pairs go into one launch per precision, as one list of tiles; a smaller one joins the list when
+  // it fits into the list's last round, else it gets a launch of its own.
   int order[hb::kMaxLanes] = {0, 1, 2, 3};
+  auto queries = [&](int i) { return items[i].n * items[i].n_device_rows; };
   for (int i = 1; i < n_items; ++i)
-    for (int j = i; j > 0 && items[order[j]].n * items[order[j]].n_device_rows >
-                                 items[order[j - 1]].n * items[order[j - 1]].n_device_rows; --j) {
+    for (int j = i; j > 0 && queries(order[j]) > queries(order[j - 1]); --j) {
       const int t = order[j];
       order[j] = order[j - 1];
       order[j - 1] = t;
     }
-  int lane = 0;
+  hb::MlpBatch batches[hb::kMaxLanes];
+  bool queued[hb::kMaxLanes] = {};
   for (int i = 0; i < n_items; ++i) {
-    const hb_mlp_grid& g = items[order[i]];
-    if (g.n == 0 || g.n_device_rows == 0) continue;
-    hb::MlpBatch batch;
-    batch.feats = g.op_features; batch.Q = g.n * g.n_device_rows; batch.out = g.out;
+    const hb_mlp_grid& g = items[i];
+    hb::MlpBatch& batch = batches[i];
+    batch.feats = g.op_features; batch.Q = queries(i); batch.out = g.out;
     batch.grid_n = static_cast<int32_t>(g.n); batch.grid_rows = g.device_rows;
-    batch.lane = lane; batch.beside = lane > 0;
+    queued[i] = batch.Q == 0;
+    const hb_status st = batch.Q ? check_device(g.handle) : HB_OK;
+    if (st != HB_OK) return st;
+  }
+  int lane = 0;
+  for (int k = 0; k < n_items; ++k) {
+    const int i = order[k];
+    if (queued[i]) continue;
+    hb_mlp* h = items[i].handle;
+    batches[i].lane = lane;
+    batches[i].beside = lane > 0;
     ++lane;
-    const hb_status st = queue_batch(g.handle, batch, static_cast<cudaStream_t>(stream));
+    hb_status st = HB_OK;
+    if (plan_of(h, batches[i].Q).G != 0) {
+      st = queue_batch(h, batches[i], static_cast<cudaStream_t>(stream));
+      if (st != HB_OK) return st;
+      continue;
+    }
+    ChainLaunch launch(h, h->precision == HB_PRECISION_BF16X3);
+    for (int m = k; m < n_items && st == HB_OK; ++m) {
+      const int o = order[m];
+      const hb_mlp* other = items[o].handle;
+      if (queued[o] || other->precision != h->precision) continue;
+      const bool fills = plan_of(other, batches[o].Q).G == 0;
+      if (m > k && !fills && launch.rounds(launch.tiles_of(batches[o].Q)) > launch.rounds(0)) continue;
+      st = launch.add(other, batches[o]);
+      queued[o] = true;
+    }
+    if (st == HB_OK) st = launch.go(batches[i].beside, static_cast<cudaStream_t>(stream));
     if (st != HB_OK) return st;
   }
   return HB_OK;

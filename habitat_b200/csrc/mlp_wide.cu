@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     }
     if (c == 0) {
       // the first block of the group adds the 64 sets of 16 features of every query, in mlp_chain.cu's order:
-      // per CTA rank there, eight warps of two 32-feature sets each
+      // per CTA rank there, eight warps (two groups of four) of two 32-feature sets each, 512 features apart
       const int q = T & 63, rank = T >> 6;
       const unsigned long long* h = group_halves + q;
       float tot = 0.0f;
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
 #pragma unroll
             for (int m = 0; m < 16; ++m) {
               const int kk = k + (m >> 2);
-              const int set = ((kk >> 2) * 512 + rank * 128 + (kk & 3) * 32) / 16 + ((m >> 1) & 1) * 16 + (m & 1);
+              const int set = ((kk >> 2) * 256 + rank * 128 + (kk & 3) * 32) / 16 + ((m >> 1) & 1) * 32 + (m & 1);
               const unsigned long long v = ld_relaxed_u64(h + set * kWideCols);
               all = all && static_cast<uint32_t>(v >> 32) == p.tag;
               x[m] = __uint_as_float(static_cast<uint32_t>(v));
