@@ -108,7 +108,7 @@ EXPORTS = {
     "hb_mlp_poll_status": (ctypes.c_int32, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int32)]),
     "hb_segment_sum_planes": (ctypes.c_int32, [
         ctypes.c_void_p, ctypes.c_int64, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
-        ctypes.c_void_p]),
+        ctypes.c_void_p, ctypes.c_void_p]),
     "hb_iteration_totals": (ctypes.c_int32, [
         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64,
         ctypes.c_int32, ctypes.c_void_p, ctypes.POINTER(IterationKind), ctypes.c_int32, ctypes.c_void_p,

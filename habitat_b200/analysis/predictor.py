@@ -19,7 +19,7 @@ import torch
 from habitat_b200 import _native
 from habitat_b200.analysis import SPECIAL_OPERATIONS
 from habitat_b200.analysis.kernels import MeasuredKernel, PredictedKernel
-from habitat_b200.analysis.mlp.mlp import RuntimePredictor
+from habitat_b200.analysis.mlp.mlp import FEATURES, RuntimePredictor
 from habitat_b200.analysis.operation import MeasuredOperation, PredictedOperation
 from habitat_b200.analysis.run_time import RunTimeMeasurement, RunTimePrediction, RunTimePurePrediction
 from habitat_b200.analysis.wave_scaling import batch as wave_batch
@@ -41,7 +41,7 @@ LSTM_PARAMS = ["input", "batch_sizes", "hx", "flat_weights", "bias", "num_layers
                "training", "bidirectional"]
 MATMUL_PARAMS = ["input", "other", "out"]
 
-_MLP_OPS = ("conv2d", "lstm", "linear", "bmm")
+_MLP_OPS = ("conv2d", "linear", "bmm", "lstm")
 
 
 def _first(value):
@@ -154,7 +154,9 @@ class _LazyRunTimePrediction(RunTimePrediction):
 
 
 _METRIC_KEYS = tuple((m, m.value.cupti_name, m.value.legacy_cupti_name) for m in wave_batch._NEEDED)
-_FAST_KINDS = {"conv2d": 0, "linear": 1, "bmm": 2}       # feature_rows of the native binding
+# the kinds whose features the native walk extracts, and the columns it fills: those of the predictors' classes
+_FAST_KINDS = ("conv2d", "linear", "bmm")
+_FAST_ORDERS = tuple(tuple(_FAST_ROWS[k][2].index(f) for f in FEATURES[k]) for k in _FAST_KINDS)
 
 
 def _trace_types():
@@ -169,14 +171,12 @@ class _GroupPlan:
 
     def __init__(self, operations, indices, mode, flat=None):
         self.mode = mode
-        self.mlp_inputs = {}      # op kind -> (features, measured ms) on the GPU, measured ms; filled on first use
+        self.mlp_inputs = {}      # op kind -> (features, measured ms) on the GPU, measured ms, columns; filled on first use
         self._layout = None
         if flat is None:
             self._flatten(operations, indices, mode)
         else:
             self._take(operations, flat)
-        self.bwd_has = np.flatnonzero(self.bwd_run >= 0)
-        self.bwd_of = self.bwd_run[self.bwd_has]
 
     @classmethod
     def of_whole_trace(cls, operations, mode):
@@ -186,17 +186,20 @@ class _GroupPlan:
         if mode == wave_batch.ROOFLINE:
             return None
         flat = _native.binding().flatten_trace(operations, _trace_types(), SPECIAL_OPERATIONS, _MLP_OPS, _METRIC_KEYS,
-                                               mode != wave_batch.RESIMPLIFIED)
+                                               mode != wave_batch.RESIMPLIFIED, _FAST_ORDERS)
         return cls(operations, None, mode, flat) if flat is not None else None
 
     def _take(self, operations, flat):
         (self.kernels, self.runs, names, wave_idx, fwd, bwd, offsets, overheads, kind_idx, self.passthrough_idx,
-         records, metrics, self.offsets_dev) = flat
+         records, metrics, self.offsets_dev, special) = flat
         self.indices = None                      # all operations
         self.wave_idx, self.fwd_run, self.bwd_run, self.offsets = (
             np.frombuffer(x, np.int64) for x in (wave_idx, fwd, bwd, offsets))
         self.overheads = np.frombuffer(overheads, np.float64)
-        self.mlp_idx = dict(zip(_MLP_OPS, kind_idx))
+        self.mlp_idx = {name: np.frombuffer(x, np.int64) for name, x in zip(_MLP_OPS, kind_idx)}
+        for name, got in zip(_FAST_KINDS, special):
+            if got is not None:
+                self.mlp_inputs[name] = (got[0], got[1], np.frombuffer(got[2], np.float32), FEATURES[name])
         for i in self.passthrough_idx:
             logger.warning("Unhandled special operation: %s", operations[i].name)
         self.flat = (wave_batch.FlatKernels.from_device(self.mode, names, records, metrics) if self.kernels
@@ -224,6 +227,7 @@ class _GroupPlan:
             else:
                 logger.warning("Unhandled special operation: %s", name)
                 self.passthrough_idx.append(i)
+        self.mlp_idx = {op: np.asarray(idx, np.int64) for op, idx in self.mlp_idx.items()}
         self.wave_idx = np.asarray(wave_idx, np.int64)
         self.fwd_run = np.asarray(fwd_run, np.int64)
         self.bwd_run = np.asarray(bwd_run, np.int64)
@@ -252,25 +256,18 @@ class _GroupPlan:
             a[self.wave_idx], b[self.wave_idx] = self.fwd_run, self.bwd_run
             for idx in self.mlp_idx.values():
                 kind[idx] = 2
-            kind[self.passthrough_idx] = 3
+            if self.passthrough_idx:
+                kind[self.passthrough_idx] = 3
             self._layout = kind, a, b
         return self._layout
 
     def special_inputs(self, name, operations, order):
         """Features and measured times of the operations of one MLP kind, on the GPU."""
         got = self.mlp_inputs.get(name)
-        if got is None:
-            idx = self.mlp_idx[name]
-            if name in _FAST_KINDS:
-                columns = _FAST_ROWS[name][2]
-                got = _native.binding().feature_rows(_FAST_KINDS[name], operations, idx,
-                                                     tuple(columns.index(f) for f in order), _trace_types())
-                if got is not None:
-                    got = got[0], got[1], np.frombuffer(got[2], np.float32)
-            if got is None:
-                ops = [operations[i] for i in idx]
-                rt = np.array([op.run_time_ms for op in ops], np.float32)
-                got = torch.from_numpy(feature_matrix(name, ops, order)).cuda(), torch.from_numpy(rt).cuda(), rt
+        if got is None or got[3] != order:
+            ops = [operations[i] for i in self.mlp_idx[name]]
+            rt = np.array([op.run_time_ms for op in ops], np.float32)
+            got = torch.from_numpy(feature_matrix(name, ops, order)).cuda(), torch.from_numpy(rt).cuda(), rt, order
             self.mlp_inputs[name] = got
         return got
 
@@ -281,16 +278,16 @@ class PredictedOperations(collections.abc.Sequence):
     PredictedKernel objects are created when an element is first touched, the per-operation
     times (`run_times_ms`) and their sum (`total_run_time_ms`) are there from the start."""
 
-    def __init__(self, operations, dest, group=None, layout=None, run_times_ms=None):
+    def __init__(self, operations, dest, group=None, run_times_ms=None, total_ms=None):
         self._operations = operations
         self._dest = dest
         self._made = None                           # elements, once one has been touched
         self._groups = [group] if group else []     # per origin group: dict(plan, times, totals)
-        self._total = None
+        self._total = total_ms
         self._group = None                          # which group an operation is of; None: the first
         n = len(operations)
-        if layout is not None:
-            self._kind, self._a, self._b = layout
+        if group is not None:                       # all of one group: its layout, when an element is touched
+            self._kind = None
             self.run_times_ms = run_times_ms
         else:
             self._kind = np.zeros(n, np.int8)       # 0 as measured, 1 wave-scaled, 2 MLP, 3 special passed through
@@ -322,6 +319,8 @@ class PredictedOperations(collections.abc.Sequence):
 
     def _make(self, i):
         op = self._operations[i]
+        if self._kind is None:
+            self._kind, self._a, self._b = self._groups[0]["plan"].layout(len(self._operations))
         kind = self._kind[i]
         if kind == 0:
             return op
@@ -437,20 +436,11 @@ class Predictor:
                 cache[key] = plan
         elif mode is None or any(d.name == origin.name for d in dest_devices):
             return None
-        n = len(operations)
-        times, totals, special = self._run_plan(plan, operations, origin, dest_devices)
-        run_ms = (plan.overheads + totals) / 1e6                             # [T, runs]
-        ms = np.empty((len(dest_devices), n), np.float64)
-        if len(plan.wave_idx):
-            wave_ms = run_ms[:, plan.fwd_run]
-            wave_ms[:, plan.bwd_has] += run_ms[:, plan.bwd_of]
-            ms[:, plan.wave_idx] = wave_ms
-        for name, pred_ms in special.items():
-            ms[:, plan.mlp_idx[name]] = pred_ms
+        ms = np.empty((len(dest_devices), len(operations)), np.float64)
         for i in plan.passthrough_idx:
             ms[:, i] = operations[i].run_time_ms
-        layout = plan.layout(n)
-        return [PredictedOperations(operations, dest, dict(plan=plan, times=times[t], totals=totals[t]), layout, ms[t])
+        times, totals, sums = self._run_plan(plan, operations, origin, dest_devices, ms)
+        return [PredictedOperations(operations, dest, dict(plan=plan, times=times[t], totals=totals[t]), ms[t], sums[t])
                 for t, dest in enumerate(dest_devices)]
 
     # ------------------------------------------------------------------
@@ -465,8 +455,10 @@ class Predictor:
             plan = plan or _GroupPlan(operations, indices, mode)
             if cache is not None:
                 cache[key] = plan
-        times, totals, special = self._run_plan(plan, operations, origin, dests)
-        run_ms = (plan.overheads[None, :] + totals) / 1e6                    # [T, runs]
+        ms = np.zeros((len(dests), len(operations)), np.float64)
+        for i in plan.passthrough_idx:
+            ms[:, i] = operations[i].run_time_ms
+        times, totals, _ = self._run_plan(plan, operations, origin, dests, ms)
         for t, d in enumerate(targets):
             res = results[d]
             g = len(res._groups)
@@ -476,69 +468,55 @@ class Predictor:
                 res._group[plan.wave_idx] = g
                 res._a[plan.wave_idx] = plan.fwd_run
                 res._b[plan.wave_idx] = plan.bwd_run
-                ms = run_ms[t][plan.fwd_run]
-                ms[plan.bwd_has] += run_ms[t][plan.bwd_of]
-                res.run_times_ms[plan.wave_idx] = ms
             for i in plan.passthrough_idx:
                 res._kind[i] = 3
-                res.run_times_ms[i] = operations[i].run_time_ms
-            for name, ms in special.items():
-                idx = np.asarray(plan.mlp_idx[name], np.int64)
+            for idx in plan.mlp_idx.values():
                 res._kind[idx] = 2
-                res.run_times_ms[idx] = ms[t]
+            res.run_times_ms[indices] = ms[t, indices]
 
-    def _run_plan(self, plan, operations, origin, dests):
-        """One prediction of a flattened group: -> (scaled kernel times [T, K], per-pass kernel totals
-        [T, runs], predicted ms [T, n] by MLP kind) on the host (predictor.py:111-148 of the reference
-        for every pass, special operation and destination at once)."""
+    def _run_plan(self, plan, operations, origin, dests, ms):
+        """One prediction of a flattened group: fills `ms` [T, operations] for its operations and returns
+        (scaled kernel times [T, K], per-pass kernel totals [T, runs], sums of the rows of `ms`), all on
+        the host (predictor.py:111-148 of the reference for every pass, special operation and destination
+        at once)."""
         T, K, n_runs = len(dests), len(plan.kernels), len(plan.runs)
-        names = [name for name in _MLP_OPS if plan.mlp_idx[name]]
-        kinds, sizes = [], []
+        names = [name for name in _MLP_OPS if len(plan.mlp_idx[name])]
+        kinds = []
         for name in names:
             pred = self._predictor(name)
             rows = bytes([pred.device_row(origin.name)] + [pred.device_row(d.name) for d in dests])
-            feats, rt, _ = plan.special_inputs(name, operations, pred.model.features)
-            kinds.append((pred._handle._handle.value, feats, rt, rows))
-            sizes.append(len(plan.mlp_idx[name]))
-        own = plan.mode is None                  # a user-supplied strategy: the reference's per-kernel protocol
-        flat = None if own else plan.flat
+            feats, rt, _, _ = plan.special_inputs(name, operations, pred.model.features)
+            kinds.append((pred._handle._handle.value, feats, rt, rows, plan.mlp_idx[name]))
+        flat = plan.flat                         # None: no kernels, or a user-supplied strategy
+        times = np.empty((T, K), np.float32 if flat is not None else np.float64)
+        totals = (np.empty if flat is not None else np.zeros)((T, n_runs), np.float64)
+        if flat is None and K:
+            # the reference's per-kernel protocol
+            for t, dest in enumerate(dests):
+                times[t] = [self._wave_scaling_strategy(k, origin, dest, self._kernel_metadata).run_time_ns
+                            for k in plan.kernels]
+            for r in range(n_runs):
+                totals[:, r] = times[:, plan.offsets[r]:plan.offsets[r + 1]].sum(axis=1)
+        if flat is None and len(plan.wave_idx):
+            run_ms = (plan.overheads + totals) / 1e6
+            ms[:, plan.wave_idx] = run_ms[:, plan.fwd_run] + np.where(plan.bwd_run >= 0, run_ms[:, plan.bwd_run], 0.0)
         regs = None
         if flat is not None:
             regs = wave_batch.destination_registers(plan.kernels, flat.names, dests, self._kernel_metadata)
-        data, nan, clamped = _native.binding().run_group(
+        nan, sums, clamped = _native.binding().run_group(
             flat.batch if flat is not None else None, flat.metrics if flat is not None else None, origin, dests, regs,
-            plan.offsets_dev if flat is not None else None, kinds)
+            plan.offsets_dev if flat is not None else None, kinds,
+            (plan.overheads, plan.wave_idx, plan.fwd_run, plan.bwd_run), times, totals, ms)
         if nan:
             wave_batch.raise_zero_wave()
-        at = 0
-
-        def take(count, dtype):
-            nonlocal at
-            part = np.frombuffer(data, dtype, count, at)
-            at = (at + count * part.itemsize + 15) & ~15
-            return part
-        if flat is not None:
-            totals = take(T * n_runs, np.float64).reshape(T, n_runs)
-        special = {}
-        for name, n, seen in zip(names, sizes, clamped):
-            special[name] = take(T * n, np.float32).reshape(T, n)
-            pred_ms = take((T + 1) * n, np.float32)
-            if seen:
-                self._warn_negative(name, plan.mlp_inputs[name][2], pred_ms.astype(np.float64), n, T)
-        if flat is not None:
-            times = take(T * K, np.float32).reshape(T, K)
-        elif own:
-            times = np.array([[self._wave_scaling_strategy(k, origin, dest, self._kernel_metadata).run_time_ns
-                               for k in plan.kernels] for dest in dests], np.float64).reshape(T, K)
-            totals = np.zeros((T, n_runs))
-            for r in range(n_runs):
-                totals[:, r] = times[:, plan.offsets[r]:plan.offsets[r + 1]].sum(axis=1)
-        else:
-            times, totals = np.zeros((T, 0)), np.zeros((T, n_runs))
-        return times, totals, special
+        for name, raw in zip(names, clamped):
+            if raw is not None:
+                self._warn_negative(name, plan.mlp_inputs[name][2], np.frombuffer(raw, np.float32).astype(np.float64), T)
+        return times, totals, sums
 
     @staticmethod
-    def _warn_negative(name, run_time_ms, pred_ms, n, T):
+    def _warn_negative(name, run_time_ms, pred_ms, T):
+        n = len(run_time_ms)
         for t in range(T):
             raw = run_time_ms.astype(np.float64) * pred_ms[(t + 1) * n:(t + 2) * n] / pred_ms[:n]
             for j in np.nonzero(raw < 0)[0]:

@@ -455,15 +455,114 @@ int find_metric(PyObject* records, PyObject* cached, PyObject* metric, PyObject*
   return 0;
 }
 
+// A contiguous buffer (numpy array, bytes) seen as `count` values of T; ok() says whether it is that large.
+template <typename T>
+struct Buffer {
+  Py_buffer view{};
+  bool held = false;
+  Buffer(PyObject* o, bool writable) {
+    held = PyObject_GetBuffer(o, &view, writable ? PyBUF_WRITABLE | PyBUF_C_CONTIGUOUS : PyBUF_C_CONTIGUOUS) == 0;
+    if (!held) PyErr_Clear();
+  }
+  ~Buffer() { if (held) PyBuffer_Release(&view); }
+  Buffer(const Buffer&) = delete;
+  Buffer& operator=(const Buffer&) = delete;
+  bool ok(int64_t count) const { return held && view.len == count * static_cast<int64_t>(sizeof(T)); }
+  T* data() const { return static_cast<T*>(view.buf); }
+  int64_t size() const { return held ? view.len / static_cast<int64_t>(sizeof(T)) : 0; }
+};
+
+// Element i of a tuple or list as a double (borrowed access); *ok is cleared when it is no number.
+double item(PyObject* seq, Py_ssize_t i, bool* ok) {
+  if (!*ok || (!PyTuple_Check(seq) && !PyList_Check(seq)) || i >= PySequence_Fast_GET_SIZE(seq)) {
+    *ok = false;
+    return 0.0;
+  }
+  const double v = PyFloat_AsDouble(PySequence_Fast_GET_ITEM(seq, i));
+  if (v == -1.0 && PyErr_Occurred()) *ok = false;
+  return v;
+}
+
+constexpr Py_ssize_t kFeatureKinds = 3;   // conv2d, linear, bmm: the kinds with positional extractors
+struct Columns {
+  Py_ssize_t n = 0;
+  long at[8];
+};
+// The column order of kind `kind` from a tuple of column numbers.
+bool columns_of(PyObject* t, long kind, Columns* c) {
+  static const Py_ssize_t kColumns[kFeatureKinds] = {8, 4, 4};
+  if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) > 8) return false;
+  c->n = PyTuple_GET_SIZE(t);
+  for (Py_ssize_t i = 0; i < c->n; ++i) {
+    c->at[i] = PyLong_AsLong(PyTuple_GET_ITEM(t, i));
+    if (c->at[i] < 0 || c->at[i] >= kColumns[kind]) return false;
+  }
+  return true;
+}
+// Features of one operation recorded positionally (predictor.py:150-232 of the reference) and its measured ms;
+// false when it was recorded otherwise (an error may be set).
+bool feature_row(long kind, PyObject* op, PyTypeObject* op_type, PyTypeObject* run_type, const Columns& c, float* row,
+                 float* measured) {
+  static const Py_ssize_t kArity[kFeatureKinds] = {5, 3, 2};
+  if (Py_TYPE(op) != op_type) return false;
+  Ref arg(get(op, s__arguments)), f(get(op, s__forward)), b(get(op, s__backward));
+  if (!arg.p || !f.p || !b.p || arg.p == Py_None) return false;
+  Ref args(get(arg.p, s_args)), kwargs(get(arg.p, s_kwargs));
+  if (!args.p || !kwargs.p || !PyTuple_Check(args.p) || !PyDict_Check(kwargs.p) || PyDict_GET_SIZE(kwargs.p) != 0 ||
+      PyTuple_GET_SIZE(args.p) < kArity[kind])
+    return false;
+  PyObject *x = PyTuple_GET_ITEM(args.p, 0), *w = PyTuple_GET_ITEM(args.p, 1);
+  bool ok = true;
+  double v[8] = {};
+  if (kind == 0) {
+    auto first = [&](PyObject* o) {
+      if (PyTuple_Check(o)) return item(o, 0, &ok);
+      const double d = PyFloat_AsDouble(o);
+      if (d == -1.0 && PyErr_Occurred()) ok = false;
+      return d;
+    };
+    v[0] = item(x, 0, &ok); v[1] = item(x, 2, &ok); v[2] = item(x, 1, &ok); v[3] = item(w, 0, &ok);
+    v[4] = item(w, 2, &ok);
+    v[5] = first(PyTuple_GET_ITEM(args.p, 3));
+    v[6] = first(PyTuple_GET_ITEM(args.p, 4));
+    v[7] = PyTuple_GET_ITEM(args.p, 2) == Py_None ? 0.0 : 1.0;
+  } else if (kind == 1) {
+    v[0] = 1.0;
+    const Py_ssize_t dims = PyTuple_Check(x) || PyList_Check(x) ? PySequence_Fast_GET_SIZE(x) : 0;
+    if (dims == 0) return false;
+    for (Py_ssize_t d = 0; d + 1 < dims; ++d) v[0] *= item(x, d, &ok);
+    v[1] = item(w, 1, &ok);
+    v[2] = item(w, 0, &ok);
+    v[3] = PyTuple_GET_ITEM(args.p, 2) == Py_None ? 0.0 : 1.0;
+  } else {
+    v[0] = item(x, 0, &ok); v[1] = item(x, 1, &ok); v[2] = item(x, 2, &ok); v[3] = item(w, 2, &ok);
+  }
+  double run = 0.0;
+  for (PyObject* r : {f.p, b.p}) {
+    if (r == Py_None) continue;
+    if (Py_TYPE(r) != run_type) return false;
+    Ref t(get(r, s__run_time_ms));
+    run += t.p ? PyFloat_AsDouble(t.p) : 0.0;
+    if (PyErr_Occurred()) return false;
+  }
+  if (!ok) return false;
+  for (Py_ssize_t i = 0; i < c.n; ++i) row[i] = static_cast<float>(v[c.at[i]]);
+  *measured = static_cast<float>(run);
+  return true;
+}
+
 // flatten_trace(operations, (MeasuredOperation, RunTimeMeasurement, MeasuredKernel, KernelInstance),
-//               special names, MLP kinds, metrics ((Metric, name, legacy name) x 3), with_metrics)
+//               special names, MLP kinds (conv2d, linear, bmm first), metrics ((Metric, name, legacy name) x 3),
+//               with_metrics, column orders of the first three kinds)
 // -> None when the operations are not all of those very classes or not of one device, else
 //    (kernels, runs, names, wave_idx, fwd_run, bwd_run, offsets, overheads: bytes of int64 / float64,
-//     [indices per MLP kind], passed-through indices,
-//     (num_blocks, block_size, regs, smem, time, gamma), (eff, read, write, has) or None, offsets: CUDA tensors)
+//     (indices per MLP kind: bytes of int64), passed-through indices,
+//     (num_blocks, block_size, regs, smem, time, gamma), (eff, read, write, has) or None, offsets: CUDA tensors,
+//     per kind of the first three: (features, measured ms: CUDA tensors, measured ms as bytes), or None when one of
+//     its operations was not recorded positionally)
 PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  if (n_args != 6) return not_ordinary();
+  if (n_args != 7) return not_ordinary();
   Ref ops(PySequence_Fast(a[0], "operations must be a sequence"));
   if (!ops.p) return nullptr;
   PyTypeObject* type[4];
@@ -473,8 +572,14 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(ops.p), n_kinds = PyTuple_GET_SIZE(kinds);
 
   Ref kernels(PyList_New(0)), runs(PyList_New(0)), names(PyList_New(0)), passed(PyList_New(0));
-  Ref kind_idx(PyList_New(n_kinds));
-  for (Py_ssize_t k = 0; k < n_kinds; ++k) PyList_SET_ITEM(kind_idx.p, k, PyList_New(0));
+  if (n_kinds < kFeatureKinds || n_kinds > 8) return not_ordinary();
+  std::vector<int64_t> kind_idx[8];
+  struct Rows {
+    Columns c;
+    bool ok;
+    std::vector<float> f, ms;
+  } feats[kFeatureKinds];
+  for (long k = 0; k < kFeatureKinds; ++k) feats[k].ok = columns_of(PyTuple_GET_ITEM(a[6], k), k, &feats[k].c);
   std::vector<int64_t> wave_idx, fwd, bwd, offsets{0};
   std::vector<double> overhead, eff, rd, wr;
   std::vector<int32_t> nb;
@@ -562,24 +667,38 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     }
     Py_ssize_t kind = 0;
     while (kind < n_kinds && PyObject_RichCompareBool(PyTuple_GET_ITEM(kinds, kind), name.p, Py_EQ) != 1) ++kind;
-    Ref at(PyLong_FromSsize_t(i));
-    if (PyList_Append(kind < n_kinds ? PyList_GET_ITEM(kind_idx.p, kind) : passed.p, at.p) < 0) return nullptr;
+    if (kind == n_kinds) {
+      Ref at(PyLong_FromSsize_t(i));
+      if (PyList_Append(passed.p, at.p) < 0) return nullptr;
+      continue;
+    }
+    kind_idx[kind].push_back(i);
+    if (kind >= kFeatureKinds || !feats[kind].ok) continue;
+    Rows& r = feats[kind];
+    r.f.resize(r.f.size() + r.c.n);
+    r.ms.resize(r.ms.size() + 1);
+    r.ok = feature_row(static_cast<long>(kind), op, type[0], type[1], r.c, r.f.data() + r.f.size() - r.c.n,
+                       &r.ms.back());
+    if (!r.ok) PyErr_Clear();
   }
   if (PyErr_Occurred()) return not_ordinary();
 
-  // one upload for the records, the metrics and the pass boundaries
-  Ref soa(Py_NewRef(Py_None)), met(Py_NewRef(Py_None)), off(Py_NewRef(Py_None));
+  // one upload for the records, the metrics, the pass boundaries and the features
+  std::vector<uint8_t> host;
+  struct Piece {
+    size_t at;
+    int64_t rows, cols;
+    at::ScalarType type;
+  };
+  std::vector<Piece> pieces;
+  auto put = [&](const void* p, int64_t count, size_t size, at::ScalarType t, int64_t cols = 0) {
+    const size_t at0 = (host.size() + 255) & ~static_cast<size_t>(255);
+    host.resize(at0 + count * size);
+    std::memcpy(host.data() + at0, p, count * size);
+    pieces.push_back(Piece{at0, cols ? count / cols : count, cols, t});
+  };
   const int64_t K = static_cast<int64_t>(nb.size());
   if (K > 0) {
-    std::vector<uint8_t> host;
-    struct Piece { size_t at; int64_t count; at::ScalarType type; };
-    std::vector<Piece> pieces;
-    auto put = [&](const void* p, int64_t count, size_t size, at::ScalarType t) {
-      const size_t at0 = (host.size() + 255) & ~static_cast<size_t>(255);
-      host.resize(at0 + count * size);
-      std::memcpy(host.data() + at0, p, count * size);
-      pieces.push_back(Piece{at0, count, t});
-    };
     const std::vector<float> gamma(nb.size(), 1.0f);
     put(nb.data(), K, 4, at::kInt);
     put(bs.data(), K, 2, at::kUInt16);
@@ -594,290 +713,304 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
       put(wr.data(), K, 8, at::kDouble);
       put(has.data(), K, 1, at::kByte);
     }
+  }
+  for (Rows& r : feats) {
+    r.ok = r.ok && !r.ms.empty();
+    if (!r.ok) continue;
+    put(r.f.data(), static_cast<int64_t>(r.f.size()), 4, at::kFloat, r.c.n);
+    put(r.ms.data(), static_cast<int64_t>(r.ms.size()), 4, at::kFloat);
+  }
+  at::Tensor block;
+  if (!host.empty()) {
     const int64_t total[1] = {static_cast<int64_t>(host.size())};
     int current = 0;
     cudaGetDevice(&current);
-    at::Tensor block = empty(total, at::kByte, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(current)));
+    block = empty(total, at::kByte, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(current)));
     const cudaError_t e = cudaMemcpyAsync(block.mutable_data_ptr(), host.data(), host.size(), cudaMemcpyHostToDevice,
                                           static_cast<cudaStream_t>(stream_now()));
     if (e != cudaSuccess) {
       PyErr_Format(PyExc_RuntimeError, "upload of the trace: %s", cudaGetErrorString(e));
       return nullptr;
     }
-    auto view = [&](size_t i) {
-      const int64_t size[1] = {pieces[i].count};
-      return THPVariable_Wrap(inside(block, pieces[i].at, size, pieces[i].type));
-    };
-    Py_SETREF(soa.p, Py_BuildValue("(NNNNNN)", view(0), view(1), view(2), view(3), view(4), view(5)));
-    Py_SETREF(off.p, view(6));
-    if (any_metrics) Py_SETREF(met.p, Py_BuildValue("(NNNN)", view(7), view(8), view(9), view(10)));
-    if (!soa.p || !off.p || !met.p) return nullptr;
   }
-  return Py_BuildValue("(OOONNNNNOOOOO)", kernels.p, runs.p, names.p, bytes_of(wave_idx), bytes_of(fwd), bytes_of(bwd),
-                       bytes_of(offsets), bytes_of(overhead), kind_idx.p, passed.p, soa.p, met.p, off.p);
-  END_HANDLE_TH_ERRORS
-}
-
-// Element i of a tuple or list as a double (borrowed access); *ok is cleared when it is no number.
-double item(PyObject* seq, Py_ssize_t i, bool* ok) {
-  if (!*ok || (!PyTuple_Check(seq) && !PyList_Check(seq)) || i >= PySequence_Fast_GET_SIZE(seq)) {
-    *ok = false;
-    return 0.0;
+  size_t taken = 0;
+  auto view = [&] {
+    const Piece& p = pieces[taken++];
+    const int64_t size[2] = {p.rows, p.cols};
+    return THPVariable_Wrap(inside(block, p.at, at::IntArrayRef(size, p.cols ? 2 : 1), p.type));
+  };
+  auto views = [&](Py_ssize_t count) {
+    PyObject* t = PyTuple_New(count);
+    for (Py_ssize_t i = 0; t && i < count; ++i) PyTuple_SET_ITEM(t, i, view());
+    return t;
+  };
+  Ref soa(Py_NewRef(Py_None)), met(Py_NewRef(Py_None)), off(Py_NewRef(Py_None)), special_rows(PyTuple_New(kFeatureKinds)),
+      kinds_out(PyTuple_New(n_kinds));
+  if (!special_rows.p || !kinds_out.p) return nullptr;
+  if (K > 0) {
+    Py_SETREF(soa.p, views(6));
+    Py_SETREF(off.p, view());
+    if (any_metrics) Py_SETREF(met.p, views(4));
   }
-  const double v = PyFloat_AsDouble(PySequence_Fast_GET_ITEM(seq, i));
-  if (v == -1.0 && PyErr_Occurred()) *ok = false;
-  return v;
-}
-
-// feature_rows(kind, operations, indices, column order, (MeasuredOperation, RunTimeMeasurement, ...))
-// -> None when an operation is not recorded positionally, else ([n][F] float32 features, [n] float32 measured
-// ms) as CUDA tensors, and the measured ms as bytes.  The rows are those of predictor.py:150-232 of the
-// reference; kind 0 conv2d, 1 linear, 2 bmm.
-PyObject* feature_rows(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
-  HANDLE_TH_ERRORS
-  if (n_args != 5) return not_ordinary();
-  const long kind = PyLong_AsLong(a[0]);
-  Ref ops(PySequence_Fast(a[1], "operations must be a sequence"));
-  if (!ops.p || !PyList_Check(a[2]) || !PyTuple_Check(a[3]) || kind < 0 || kind > 2) return not_ordinary();
-  PyTypeObject* op_type = reinterpret_cast<PyTypeObject*>(PyTuple_GET_ITEM(a[4], 0));
-  PyTypeObject* run_type = reinterpret_cast<PyTypeObject*>(PyTuple_GET_ITEM(a[4], 1));
-  const Py_ssize_t n = PyList_GET_SIZE(a[2]), F = PyTuple_GET_SIZE(a[3]);
-  static const Py_ssize_t kArity[3] = {5, 3, 2}, kColumns[3] = {8, 4, 4};
-  if (F > 8) return not_ordinary();
-  long order[8];
-  for (Py_ssize_t c = 0; c < F; ++c) {
-    order[c] = PyLong_AsLong(PyTuple_GET_ITEM(a[3], c));
-    if (order[c] < 0 || order[c] >= kColumns[kind]) return not_ordinary();
-  }
-  std::vector<float> host(static_cast<size_t>(n) * F + n);
-  float* ms = host.data() + static_cast<size_t>(n) * F;
-  for (Py_ssize_t i = 0; i < n; ++i) {
-    PyObject* op = PySequence_Fast_GET_ITEM(ops.p, PyLong_AsSsize_t(PyList_GET_ITEM(a[2], i)));
-    if (Py_TYPE(op) != op_type) return not_ordinary();
-    Ref arg(get(op, s__arguments)), f(get(op, s__forward)), b(get(op, s__backward));
-    if (!arg.p || !f.p || !b.p || arg.p == Py_None) return not_ordinary();
-    Ref args(get(arg.p, s_args)), kwargs(get(arg.p, s_kwargs));
-    if (!args.p || !kwargs.p || !PyTuple_Check(args.p) || !PyDict_Check(kwargs.p) || PyDict_GET_SIZE(kwargs.p) != 0 ||
-        PyTuple_GET_SIZE(args.p) < kArity[kind])
-      return not_ordinary();
-    PyObject *x = PyTuple_GET_ITEM(args.p, 0), *w = PyTuple_GET_ITEM(args.p, 1);
-    bool ok = true;
-    double v[8] = {};
-    if (kind == 0) {
-      auto first = [&](PyObject* o) {
-        if (PyTuple_Check(o)) return item(o, 0, &ok);
-        const double d = PyFloat_AsDouble(o);
-        if (d == -1.0 && PyErr_Occurred()) ok = false;
-        return d;
-      };
-      v[0] = item(x, 0, &ok); v[1] = item(x, 2, &ok); v[2] = item(x, 1, &ok); v[3] = item(w, 0, &ok);
-      v[4] = item(w, 2, &ok);
-      v[5] = first(PyTuple_GET_ITEM(args.p, 3));
-      v[6] = first(PyTuple_GET_ITEM(args.p, 4));
-      v[7] = PyTuple_GET_ITEM(args.p, 2) == Py_None ? 0.0 : 1.0;
-    } else if (kind == 1) {
-      v[0] = 1.0;
-      const Py_ssize_t dims = PyTuple_Check(x) || PyList_Check(x) ? PySequence_Fast_GET_SIZE(x) : 0;
-      if (dims == 0) return not_ordinary();
-      for (Py_ssize_t d = 0; d + 1 < dims; ++d) v[0] *= item(x, d, &ok);
-      v[1] = item(w, 1, &ok);
-      v[2] = item(w, 0, &ok);
-      v[3] = PyTuple_GET_ITEM(args.p, 2) == Py_None ? 0.0 : 1.0;
-    } else {
-      v[0] = item(x, 0, &ok); v[1] = item(x, 1, &ok); v[2] = item(x, 2, &ok); v[3] = item(w, 2, &ok);
+  for (Py_ssize_t k = 0; k < kFeatureKinds; ++k) {
+    PyObject* got = Py_NewRef(Py_None);
+    if (feats[k].ok) {
+      PyObject *f = view(), *m = view();
+      Py_SETREF(got, Py_BuildValue("(NNN)", f, m, bytes_of(feats[k].ms)));
     }
-    double run = 0.0;
-    for (PyObject* r : {f.p, b.p}) {
-      if (r == Py_None) continue;
-      if (Py_TYPE(r) != run_type) return not_ordinary();
-      Ref t(get(r, s__run_time_ms));
-      run += t.p ? PyFloat_AsDouble(t.p) : 0.0;
-      if (PyErr_Occurred()) return not_ordinary();
-    }
-    if (!ok) return not_ordinary();
-    for (Py_ssize_t c = 0; c < F; ++c) host[i * F + c] = static_cast<float>(v[order[c]]);
-    ms[i] = static_cast<float>(run);
+    PyTuple_SET_ITEM(special_rows.p, k, got);
   }
-  int current = 0;
-  cudaGetDevice(&current);
-  const int64_t total[1] = {static_cast<int64_t>(host.size() * 4)}, nf[2] = {n, F}, n1[1] = {n};
-  at::Tensor block = empty(total, at::kByte, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(current)));
-  const cudaError_t e = cudaMemcpyAsync(block.mutable_data_ptr(), host.data(), host.size() * 4, cudaMemcpyHostToDevice,
-                                        static_cast<cudaStream_t>(stream_now()));
-  if (e != cudaSuccess) {
-    PyErr_Format(PyExc_RuntimeError, "upload of the features: %s", cudaGetErrorString(e));
-    return nullptr;
-  }
-  return Py_BuildValue("(NNN)", THPVariable_Wrap(inside(block, 0, nf, at::kFloat)),
-                       THPVariable_Wrap(inside(block, static_cast<size_t>(n) * F * 4, n1, at::kFloat)),
-                       bytes_of(ms, static_cast<size_t>(n) * 4));
+  for (Py_ssize_t k = 0; k < n_kinds; ++k) PyTuple_SET_ITEM(kinds_out.p, k, bytes_of(kind_idx[k]));
+  if (PyErr_Occurred() || !soa.p || !off.p || !met.p) return nullptr;
+  return Py_BuildValue("(OOONNNNNOOOOOO)", kernels.p, runs.p, names.p, bytes_of(wave_idx), bytes_of(fwd), bytes_of(bwd),
+                       bytes_of(offsets), bytes_of(overhead), kinds_out.p, passed.p, soa.p, met.p, off.p, special_rows.p);
   END_HANDLE_TH_ERRORS
 }
 
 // run_group(kernels or None, metrics or None, origin, dests, dest_regs or None, offsets or None,
-//           [(handle address, features, measured ms, device rows (bytes: origin, then the destinations))])
-// -> (bytes, NaN seen, [a clamped prediction seen per kind]).  The bytes hold, each part on a 16-byte
-// boundary: [T][passes] float64 kernel-time totals, per kind [T][n] float32 ms and [1 + T][n] float32
-// predictions, [T][K] float32 scaled times.  One prediction of a flattened trace: wave scaling, the sums of
-// its passes, the MLPs of all kinds side by side, their ratios; one download, one wait.
+//           [(handle address, features, measured ms, device rows (bytes: origin, then the destinations),
+//             operation indices (int64))],
+//           (overheads, wave_idx, fwd_run, bwd_run: float64 / int64), times [T][K] float32,
+//           totals [T][passes] float64, ms [T][n] float64)
+// -> (NaN seen, total ms per destination, [per kind: None, or [1 + T][n] float32 predictions as bytes when one
+//    may have been clamped]).  One prediction of a flattened trace: fills `times` and `totals` (the kernels' times
+// and their sums per pass) and the entries of `ms` of the wave-scaled and MLP-predicted operations; the other
+// entries of `ms` are the caller's and are part of the totals.
+//
+// Two groups of launches: wave scaling with the sums of its passes, and the MLPs of all kinds side by side with
+// their ratios.  Both leave their results in page-locked memory themselves.  With many kernels the wave scaling
+// goes first, and its results are sorted into the operations while the predictors run; with few it goes last,
+// so that the predictors, which take longest, start first.
 PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  if (n_args != 7 || !PyList_Check(a[6])) {
+  if (n_args != 11 || !PyList_Check(a[6]) || !PyTuple_Check(a[7]) || PyTuple_GET_SIZE(a[7]) != 4) {
     PyErr_SetString(PyExc_TypeError, "run_group: bad arguments");
     return nullptr;
   }
+  auto refuse = [](const char* what) -> PyObject* {
+    PyErr_Format(PyExc_TypeError, "run_group: %s", what);
+    return nullptr;
+  };
   Ref dests(PySequence_Fast(a[3], "dests must be a sequence of DeviceProperties"));
   if (!dests.p) return nullptr;
   const int64_t T = PySequence_Fast_GET_SIZE(dests.p);
+  if (T > HB_MAX_DEVICES) return refuse("too many destinations");
+  const bool scale = a[0] != Py_None;
   int64_t K = 0, n_runs = 0;
   const at::Tensor* off = nullptr;
-  if (a[5] != Py_None) {
+  if (scale) {
+    const Field nb(a[0], s_num_blocks, at::kInt);
     off = tensor(a[5], at::kLong);
-    if (!off) {
-      PyErr_SetString(PyExc_TypeError, "run_group: offsets");
-      return nullptr;
-    }
+    if (!nb.t || !off || off->numel() < 1) return refuse("kernels");
+    K = nb.t->numel();
     n_runs = off->numel() - 1;
   }
-  auto up16 = [](size_t v) { return (v + 15) & ~static_cast<size_t>(15); };
-  size_t at0 = 0;
-  auto place = [&](size_t bytes) {
-    const size_t here = at0;
-    at0 = up16(at0 + bytes);
+  const Buffer<double> overhead(PyTuple_GET_ITEM(a[7], 0), false), totals(a[9], true), ms(a[10], true);
+  const Buffer<int64_t> wave_idx(PyTuple_GET_ITEM(a[7], 1), false), fwd(PyTuple_GET_ITEM(a[7], 2), false),
+      bwd(PyTuple_GET_ITEM(a[7], 3), false);
+  const Buffer<float> times(a[8], true);
+  const int64_t n_wave = wave_idx.size(), n_ops = T ? ms.size() / T : 0;
+  if (scale && (!times.ok(T * K) || !totals.ok(T * n_runs) || !overhead.ok(n_runs))) return refuse("results");
+  if (!ms.ok(T * n_ops) || !fwd.ok(n_wave) || !bwd.ok(n_wave)) return refuse("operations");
+  if (scale)
+    for (int64_t i = 0; i < n_wave; ++i)
+      if (wave_idx.data()[i] < 0 || wave_idx.data()[i] >= n_ops || fwd.data()[i] < 0 || fwd.data()[i] >= n_runs ||
+          bwd.data()[i] >= n_runs)
+        return refuse("operations");
+
+  auto place = [](size_t* at, size_t bytes) {
+    const size_t here = *at;
+    *at = (here + bytes + 255) & ~static_cast<size_t>(255);
     return here;
   };
-  const size_t o_totals = place(static_cast<size_t>(T) * n_runs * 8);
-  struct Kind { hb_mlp* h; const at::Tensor *f, *ms; const uint8_t* rows; int64_t n; size_t o_ms, o_pred; };
+  // in page-locked memory: sums and times of the wave scaling, ms per kind
+  size_t pinned = 0, device = 0;
+  const size_t h_totals = place(&pinned, static_cast<size_t>(T) * n_runs * 8);
+  const size_t h_times = place(&pinned, static_cast<size_t>(T) * K * 4);
+  struct Kind {
+    hb_mlp* h;
+    const at::Tensor *f, *ms;
+    const uint8_t* rows;
+    const int64_t* idx;
+    int64_t n;
+    size_t h_ms, d_pred;
+  };
   std::vector<Kind> kinds;
   for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[6]); ++i) {
     PyObject* t = PyList_GET_ITEM(a[6], i);
+    if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 5) return refuse("operation kind");
     Kind k{};
     k.h = static_cast<hb_mlp*>(PyLong_AsVoidPtr(PyTuple_GET_ITEM(t, 0)));
     k.f = tensor(PyTuple_GET_ITEM(t, 1), at::kFloat);
     k.ms = tensor(PyTuple_GET_ITEM(t, 2), at::kFloat);
     PyObject* rows = PyTuple_GET_ITEM(t, 3);
-    if (!k.f || !k.ms || !PyBytes_Check(rows) || PyBytes_GET_SIZE(rows) != T + 1 || k.ms->numel() != k.f->size(0)) {
-      PyErr_SetString(PyExc_TypeError, "run_group: operation kind");
-      return nullptr;
-    }
+    const Buffer<int64_t> idx(PyTuple_GET_ITEM(t, 4), false);   // the tuple keeps the memory alive
+    if (!k.f || k.f->dim() != 2 || !k.ms || !PyBytes_Check(rows) || PyBytes_GET_SIZE(rows) != T + 1 ||
+        k.ms->numel() != k.f->size(0) || !idx.ok(k.f->size(0)))
+      return refuse("operation kind");
     k.rows = reinterpret_cast<const uint8_t*>(PyBytes_AS_STRING(rows));
+    k.idx = idx.data();
     k.n = k.f->size(0);
-    k.o_ms = place(static_cast<size_t>(T) * k.n * 4);
-    k.o_pred = place(static_cast<size_t>(T + 1) * k.n * 4);
+    for (int64_t j = 0; j < k.n; ++j)
+      if (k.idx[j] < 0 || k.idx[j] >= n_ops) return refuse("operation index");
+    k.h_ms = place(&pinned, static_cast<size_t>(T) * k.n * 4);
+    k.d_pred = place(&device, static_cast<size_t>(T + 1) * k.n * 4);
     kinds.push_back(k);
   }
-  size_t o_scaled = at0, o_rest = 0;
-  if (a[0] != Py_None) {
-    const Field nb(a[0], s_num_blocks, at::kInt);
-    if (!nb.t) {
-      PyErr_SetString(PyExc_TypeError, "run_group: kernels");
-      return nullptr;
-    }
-    K = nb.t->numel();
-  }
-  place(static_cast<size_t>(T) * K * 4);
-  const size_t result = at0;
-  // the planes of the wave-scaling call that stay on the device follow
-  auto plane = [&](size_t bytes) {
-    at0 = (at0 + 255) & ~static_cast<size_t>(255);
-    return place(bytes);
-  };
-  o_rest = plane(static_cast<size_t>(T) * K);
-  const size_t o_waves = plane(static_cast<size_t>(T) * K * 4), o_oocc = plane(K), o_owaves = plane(K * 4);
+  const size_t pairs = static_cast<size_t>(T) * K;
+  const size_t d_scaled = place(&device, pairs * 4), d_occ = place(&device, pairs), d_waves = place(&device, pairs * 4),
+               d_oocc = place(&device, K), d_owaves = place(&device, static_cast<size_t>(K) * 4);
 
   int current = 0;
   cudaGetDevice(&current);
-  const int64_t total[1] = {static_cast<int64_t>(at0 ? at0 : 16)}, host_size[1] = {static_cast<int64_t>(result ? result : 16)};
-  at::Tensor block = empty(total, at::kByte, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(current)));
+  const int64_t dev_size[1] = {static_cast<int64_t>(device ? device : 16)},
+                host_size[1] = {static_cast<int64_t>(pinned ? pinned : 16)};
+  at::Tensor block = empty(dev_size, at::kByte, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(current)));
+  at::Tensor host(at::detail::empty_cpu(host_size, at::kByte, /*pin_memory=*/true));
   uint8_t* d = static_cast<uint8_t*>(block.mutable_data_ptr());
+  uint8_t* h = static_cast<uint8_t*>(host.mutable_data_ptr());
   cudaStream_t s = static_cast<cudaStream_t>(stream_now());
+  // whatever has been launched writes to `host`: nobody leaves before it has ended
+  struct Settle {
+    cudaStream_t s;
+    bool on = true;
+    ~Settle() { if (on) cudaStreamSynchronize(s); }
+  } settle{s};
 
-  // the predictors first: they take longest, and the wave scaling's host part runs under them
-  std::vector<hb_mlp_grid> grids;
-  std::vector<hb_scale_grid> scales;
-  for (const Kind& k : kinds) {
-    grids.push_back(hb_mlp_grid{k.h, static_cast<const float*>(data(k.f)), k.n, k.rows, static_cast<int32_t>(T + 1),
-                                reinterpret_cast<float*>(d + k.o_pred)});
-    scales.push_back(hb_scale_grid{static_cast<const float*>(data(k.ms)), reinterpret_cast<const float*>(d + k.o_pred), k.n,
-                                   static_cast<int32_t>(T), reinterpret_cast<float*>(d + k.o_ms), nullptr});
-  }
-  if (failed(api.mlp_predict_grid(grids.data(), static_cast<int32_t>(grids.size()), s))) return nullptr;
-  if (K > 0) {
+  auto launch_mlps = [&]() -> bool {
+    std::vector<hb_mlp_grid> grids;
+    std::vector<hb_scale_grid> scales;
+    for (const Kind& k : kinds) {
+      float* pred = reinterpret_cast<float*>(d + k.d_pred);
+      grids.push_back(hb_mlp_grid{k.h, static_cast<const float*>(data(k.f)), k.n, k.rows, static_cast<int32_t>(T + 1), pred});
+      scales.push_back(hb_scale_grid{static_cast<const float*>(data(k.ms)), pred, k.n, static_cast<int32_t>(T),
+                                     reinterpret_cast<float*>(h + k.h_ms), nullptr});
+    }
+    return !failed(api.mlp_predict_grid(grids.data(), static_cast<int32_t>(grids.size()), s)) &&
+           !failed(api.special_scale_grid(scales.data(), static_cast<int32_t>(scales.size()), s));
+  };
+  auto launch_waves = [&]() -> bool {
+    if (!scale || K == 0) return true;
     const Field nb(a[0], s_num_blocks, at::kInt), bs(a[0], s_block_size, at::kUInt16), rg(a[0], s_regs, at::kUInt16),
         sm(a[0], s_smem, at::kUInt32), tm(a[0], s_time, at::kFloat), gm(a[0], s_gamma, at::kFloat);
-    const int16_t* regs = nullptr;
-    if (a[4] != Py_None) {
-      const at::Tensor* t = tensor(a[4], at::kShort);
-      if (t && t->numel() == T * K) regs = static_cast<const int16_t*>(data(t));
-      else PyErr_SetString(PyExc_TypeError, "run_group: dest_regs");
-    }
-    if (!bs.t || !rg.t || !sm.t || !tm.t || !gm.t) PyErr_SetString(PyExc_TypeError, "run_group: kernels");
+    const at::Tensor* dr = a[4] == Py_None ? nullptr : tensor(a[4], at::kShort);
+    if (!bs.t || !rg.t || !sm.t || !tm.t || !gm.t || (a[4] != Py_None && (!dr || dr->numel() != T * K)))
+      return refuse("kernel records") != nullptr;
     int32_t rows[HB_MAX_DEVICES];
-    if (T > HB_MAX_DEVICES) PyErr_SetString(PyExc_ValueError, "too many destinations");
-    if (PyErr_Occurred()) return nullptr;
     const long origin = row_of(a[2]);
-    if (origin < 0) return nullptr;
+    if (origin < 0) return false;
     for (int64_t t = 0; t < T; ++t) {
       const long r = row_of(PySequence_Fast_GET_ITEM(dests.p, t));
-      if (r < 0) return nullptr;
+      if (r < 0) return false;
       rows[t] = static_cast<int32_t>(r);
     }
-    hb_kernel_soa soa{static_cast<const int32_t*>(nb.ptr()), static_cast<const uint16_t*>(bs.ptr()),
-                      static_cast<const uint16_t*>(rg.ptr()), static_cast<const uint32_t*>(sm.ptr()),
-                      static_cast<const float*>(tm.ptr()), static_cast<const float*>(gm.ptr())};
-    hb_wave_out o{reinterpret_cast<float*>(d + o_scaled), d + o_rest, reinterpret_cast<uint32_t*>(d + o_waves), d + o_oocc,
-                  reinterpret_cast<uint32_t*>(d + o_owaves), nullptr, nullptr};
+    const hb_kernel_soa soa{static_cast<const int32_t*>(nb.ptr()), static_cast<const uint16_t*>(bs.ptr()),
+                            static_cast<const uint16_t*>(rg.ptr()), static_cast<const uint32_t*>(sm.ptr()),
+                            static_cast<const float*>(tm.ptr()), static_cast<const float*>(gm.ptr())};
+    const hb_wave_out o{reinterpret_cast<float*>(d + d_scaled), d + d_occ, reinterpret_cast<uint32_t*>(d + d_waves),
+                        d + d_oocc, reinterpret_cast<uint32_t*>(d + d_owaves), nullptr, nullptr};
     hb_kernel_metrics m{};
-    const bool with_metrics = a[1] != Py_None;
-    if (with_metrics) {
+    if (a[1] != Py_None) {
       const Field fe(a[1], s_flop, at::kDouble), rd(a[1], s_rd, at::kDouble), wr(a[1], s_wr, at::kDouble),
           has(a[1], s_has, at::kByte);
-      if (!fe.t || !rd.t || !wr.t || !has.t) {
-        PyErr_SetString(PyExc_TypeError, "run_group: metrics");
-        return nullptr;
-      }
+      if (!fe.t || !rd.t || !wr.t || !has.t) return refuse("metrics") != nullptr;
       m = hb_kernel_metrics{static_cast<const double*>(fe.ptr()), static_cast<const double*>(rd.ptr()),
                             static_cast<const double*>(wr.ptr()), static_cast<const uint8_t*>(has.ptr())};
     }
-    if (failed(wave_scale_call(soa, with_metrics ? &m : nullptr, K, static_cast<int32_t>(origin), rows,
-                               static_cast<int32_t>(T), regs, o, nullptr, nullptr, s)))
-      return nullptr;
-    if (off && failed(api.segment_sum_planes(o.scaled_ns, K, static_cast<int32_t>(T), static_cast<const int64_t*>(data(off)),
-                                             n_runs, reinterpret_cast<double*>(d + o_totals), s)))
-      return nullptr;
-  } else if (n_runs > 0) {
-    if (cudaMemsetAsync(d + o_totals, 0, static_cast<size_t>(T) * n_runs * 8, s) != cudaSuccess) {
-      PyErr_SetString(PyExc_RuntimeError, "cudaMemsetAsync");
-      return nullptr;
+    return !failed(wave_scale_call(soa, a[1] != Py_None ? &m : nullptr, K, static_cast<int32_t>(origin), rows,
+                                   static_cast<int32_t>(T), static_cast<const int16_t*>(data(dr)), o, nullptr, nullptr, s)) &&
+           !failed(api.segment_sum_planes(o.scaled_ns, K, static_cast<int32_t>(T), static_cast<const int64_t*>(data(off)),
+                                          n_runs, reinterpret_cast<double*>(h + h_totals),
+                                          reinterpret_cast<float*>(h + h_times), s));
+  };
+  bool nan = false;
+  auto sort_waves = [&] {
+    if (!scale) return;
+    const double* tot = reinterpret_cast<const double*>(h + h_totals);
+    if (K == 0) std::memset(h + h_totals, 0, static_cast<size_t>(T) * n_runs * 8);
+    std::memcpy(totals.data(), tot, static_cast<size_t>(T) * n_runs * 8);
+    std::memcpy(times.data(), h + h_times, pairs * 4);
+    // a NaN time makes its pass's sum NaN, and every kernel is of a pass
+    const double* over = overhead.data();
+    const int64_t *wi = wave_idx.data(), *fw = fwd.data(), *bw = bwd.data();
+    for (int64_t t = 0; t < T; ++t) {
+      const double* q = totals.data() + t * n_runs;
+      for (int64_t r = 0; r < n_runs; ++r) nan = nan || q[r] != q[r];
+      double* out = ms.data() + t * n_ops;
+      for (int64_t i = 0; i < n_wave; ++i) {
+        double v = (over[fw[i]] + q[fw[i]]) / 1e6;
+        if (bw[i] >= 0) v += (over[bw[i]] + q[bw[i]]) / 1e6;
+        out[wi[i]] = v;
+      }
     }
+  };
+
+  constexpr int64_t kManyPairs = 16384;
+  cudaError_t e = cudaSuccess;
+  if (scale && !kinds.empty() && T * K >= kManyPairs) {
+    struct Event {
+      cudaEvent_t ev = nullptr;
+      ~Event() { if (ev) cudaEventDestroy(ev); }
+    } done;
+    e = cudaEventCreateWithFlags(&done.ev, cudaEventDisableTiming);
+    if (!launch_waves()) return nullptr;
+    if (e == cudaSuccess) e = cudaEventRecord(done.ev, s);
+    if (!launch_mlps()) return nullptr;
+    Py_BEGIN_ALLOW_THREADS
+    if (e == cudaSuccess) e = cudaEventSynchronize(done.ev);
+    if (e == cudaSuccess) sort_waves();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    Py_END_ALLOW_THREADS
+  } else {
+    if (!launch_mlps() || !launch_waves()) return nullptr;
+    Py_BEGIN_ALLOW_THREADS
+    e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) sort_waves();
+    Py_END_ALLOW_THREADS
   }
-  if (failed(api.special_scale_grid(scales.data(), static_cast<int32_t>(scales.size()), s))) return nullptr;
-  at::Tensor host(at::detail::empty_cpu(host_size, at::kByte, /*pin_memory=*/true));
-  uint8_t* h = static_cast<uint8_t*>(host.mutable_data_ptr());
-  cudaError_t e;
-  Py_BEGIN_ALLOW_THREADS
-  e = result ? cudaMemcpyAsync(h, d, result, cudaMemcpyDeviceToHost, s) : cudaSuccess;
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  Py_END_ALLOW_THREADS
+  settle.on = false;
   if (e != cudaSuccess) {
     PyErr_Format(PyExc_RuntimeError, "prediction of a trace: %s", cudaGetErrorString(e));
     return nullptr;
   }
-  for (const Kind& k : kinds) {
-    int32_t code = 0;
-    if (failed(api.mlp_poll_status(k.h, &code))) return nullptr;
-  }
-  bool nan = false;
-  const float* scaled = reinterpret_cast<const float*>(h + o_scaled);
-  for (int64_t i = 0; i < T * K; ++i) nan = nan || scaled[i] != scaled[i];
   Ref clamped(PyList_New(static_cast<Py_ssize_t>(kinds.size())));
   for (size_t i = 0; i < kinds.size(); ++i) {
-    const float* ms = reinterpret_cast<const float*>(h + kinds[i].o_ms);
+    const Kind& k = kinds[i];
+    int32_t code = 0;
+    if (failed(api.mlp_poll_status(k.h, &code))) return nullptr;
+    const float* v = reinterpret_cast<const float*>(h + k.h_ms);
     bool zero = false;
-    for (int64_t j = 0; j < T * kinds[i].n; ++j) zero = zero || ms[j] == 0.0f;
-    PyList_SET_ITEM(clamped.p, static_cast<Py_ssize_t>(i), PyBool_FromLong(zero));
+    for (int64_t t = 0; t < T; ++t) {
+      double* out = ms.data() + t * n_ops;
+      for (int64_t j = 0; j < k.n; ++j) {
+        const float x = v[t * k.n + j];
+        zero = zero || x == 0.0f;
+        out[k.idx[j]] = static_cast<double>(x);
+      }
+    }
+    PyObject* pred = Py_NewRef(Py_None);
+    if (zero) {
+      // rare: the raw predictions, for the caller's warnings
+      const size_t bytes = static_cast<size_t>(T + 1) * k.n * 4;
+      Py_DECREF(pred);
+      pred = PyBytes_FromStringAndSize(nullptr, static_cast<Py_ssize_t>(bytes));
+      if (!pred) return nullptr;
+      if (cudaMemcpy(PyBytes_AS_STRING(pred), d + k.d_pred, bytes, cudaMemcpyDeviceToHost) != cudaSuccess) {
+        Py_DECREF(pred);
+        PyErr_SetString(PyExc_RuntimeError, "run_group: cudaMemcpy");
+        return nullptr;
+      }
+    }
+    PyList_SET_ITEM(clamped.p, static_cast<Py_ssize_t>(i), pred);
   }
-  return Py_BuildValue("(NNO)", bytes_of(h, result), PyBool_FromLong(nan), clamped.p);
+  Ref sums(PyList_New(static_cast<Py_ssize_t>(T)));
+  for (int64_t t = 0; t < T; ++t) {
+    double sum[4] = {0.0, 0.0, 0.0, 0.0};
+    const double* q = ms.data() + t * n_ops;
+    for (int64_t i = 0; i < n_ops; ++i) sum[i & 3] += q[i];
+    PyList_SET_ITEM(sums.p, static_cast<Py_ssize_t>(t), PyFloat_FromDouble((sum[0] + sum[1]) + (sum[2] + sum[3])));
+  }
+  return Py_BuildValue("(NOO)", PyBool_FromLong(nan), sums.p, clamped.p);
   END_HANDLE_TH_ERRORS
 }
 
@@ -972,7 +1105,7 @@ PyObject* set_generation(PyObject*, PyObject* v) {
 }
 
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {FAST(setup), FAST(wave_scale), FAST(mlp_predict), FAST(mlp_predict_one), FAST(flatten_trace), FAST(feature_rows), FAST(run_group), FAST(iteration_totals), FAST(partials_sum), FAST(group_sum),
+PyMethodDef methods[] = {FAST(setup), FAST(wave_scale), FAST(mlp_predict), FAST(mlp_predict_one), FAST(flatten_trace), FAST(run_group), FAST(iteration_totals), FAST(partials_sum), FAST(group_sum),
                          FAST(plane_sum), FAST(segment_sum),
                          {"set_generation", set_generation, METH_O, nullptr},
                          {nullptr, nullptr, 0, nullptr}};

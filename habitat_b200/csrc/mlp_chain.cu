@@ -900,7 +900,6 @@ class ChainLaunch {
   int64_t tiles_of(int64_t Q) const { const int q = split_ ? kPairQ / 2 : kPairQ; return (Q + q - 1) / q; }
   // Rounds of tiles the SMs would walk with `more` tiles on top.
   int64_t rounds(int64_t more) const { return (p_.num_tiles + more + pairs_ - 1) / pairs_; }
-  bool empty() const { return p_.n_problems == 0; }
   hb_status add(const hb_mlp* h, const hb::MlpBatch& batch) {
     const int64_t tiles = tiles_of(batch.Q);
     if (p_.n_problems == hb::kMaxLanes || tiles + p_.num_tiles > 0x7FFFFFFF || (batch.grid_n && batch.Q > 0xFFFFFFFFll)) {

@@ -59,23 +59,31 @@ special_scale_kernel(const float* __restrict__ run_time_ms, const float* __restr
   }
 }
 
-// Segment sums over several planes that share the offsets, one warp per (plane, segment): the passes of a
-// trace hold a kernel or a few each, and a block of 256 threads per sum spent its time in barriers.
+// Segment sums over several planes that share the offsets.  The passes of a trace hold a kernel or a few
+// each, and a block of 256 threads per sum (segment_sum_kernel) spent its time in barriers: LANES lanes share
+// a sum, one for short segments (neighbouring threads then read and write neighbouring values), else a warp.
+// `copy`, if given, receives the values themselves: with both outputs in page-locked host memory a caller
+// gets the times and their sums without a copy that the launches behind this one would wait for.
+template <int LANES>
 __global__ void __launch_bounds__(256)
 segment_sum_planes_kernel(const float* __restrict__ values, int64_t plane_len, const int64_t* __restrict__ offsets,
-                          int64_t n_segments, int64_t n_sums, double* __restrict__ out) {
+                          int64_t n_segments, int64_t n_sums, double* __restrict__ out, int64_t n_values,
+                          float* __restrict__ copy) {
   hb_grid_dependency_wait();
-  const int lane = threadIdx.x & 31;
-  for (int64_t w = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5); w < n_sums;
-       w += static_cast<int64_t>(gridDim.x) * 8) {
+  const int lane = threadIdx.x % LANES;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * (256 / LANES);
+  for (int64_t w = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) / LANES; w < n_sums; w += stride) {
     const int64_t plane = w / n_segments, s = w - plane * n_segments;
     const int64_t lo = offsets[s], hi = offsets[s + 1];
     const float* v = values + plane * plane_len;
     double acc = 0.0;
-    for (int64_t i = lo + lane; i < hi; i += 32) acc += static_cast<double>(v[i]);
-    const double t = warp_sum(acc);
-    if (lane == 0) out[w] = t;
+    for (int64_t i = lo + lane; i < hi; i += LANES) acc += static_cast<double>(v[i]);
+    if (LANES == 32) acc = warp_sum(acc);
+    if (lane == 0) out[w] = acc;
   }
+  if (copy)
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; i < n_values; i += gridDim.x * 256ll)
+      copy[i] = values[i];
 }
 
 // special_scale_kernel over a grid of predictions [1 + T][n] (row 0: the origin's): ms[t][i] =
@@ -305,7 +313,8 @@ extern "C" hb_status hb_special_scale(const float* run_time_ms, const float* pre
 }
 
 extern "C" hb_status hb_segment_sum_planes(const float* values, int64_t plane_len, int32_t n_planes,
-                                           const int64_t* offsets, int64_t n_segments, double* out, void* stream) {
+                                           const int64_t* offsets, int64_t n_segments, double* out, float* copy,
+                                           void* stream) {
   if (n_segments < 0 || n_planes < 0 || plane_len < 0 ||
       (n_segments > 0 && n_planes > 0 && (!values || !offsets || !out))) {
     hb::set_error("hb_segment_sum_planes: bad arguments");
@@ -314,9 +323,12 @@ extern "C" hb_status hb_segment_sum_planes(const float* values, int64_t plane_le
   const int64_t sums = n_segments * n_planes;
   if (sums == 0) return HB_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int64_t blocks = (sums + 7) / 8 < 148 * 8 ? (sums + 7) / 8 : 148 * 8;
-  HB_CUDA_TRY(hb::launch_overlapped(segment_sum_planes_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, s,
-                                    values, plane_len, offsets, n_segments, sums, out));
+  const bool small = plane_len <= 8 * n_segments;   // values per sum on average
+  const int64_t want = small ? (sums + 255) / 256 : (sums + 7) / 8;
+  const int64_t blocks = want < 148 * 8 ? want : 148 * 8;
+  HB_CUDA_TRY(hb::launch_overlapped(small ? segment_sum_planes_kernel<1> : segment_sum_planes_kernel<32>,
+                                    dim3(static_cast<unsigned>(blocks)), dim3(256), 0, s, values, plane_len, offsets,
+                                    n_segments, sums, out, plane_len * n_planes, copy));
   return HB_OK;
 }
 

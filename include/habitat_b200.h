@@ -291,9 +291,9 @@ hb_status hb_segment_sum(const float* values, const int64_t* offsets, int64_t n_
                          double* out, void* stream);
 
 /* hb_segment_sum over n_planes planes of plane_len values that share the offsets (the passes of a trace on
- * every destination): out[p * n_segments + s]. */
+ * every destination): out[p * n_segments + s].  copy (or NULL) receives the n_planes * plane_len values. */
 hb_status hb_segment_sum_planes(const float* values, int64_t plane_len, int32_t n_planes, const int64_t* offsets,
-                                int64_t n_segments, double* out, void* stream);
+                                int64_t n_segments, double* out, float* copy, void* stream);
 
 /* hb_special_scale over the predictions hb_mlp_predict_grid leaves when the origin comes first:
  * out_ms[t * n + i] = max(0, run_time_ms[i] * pred[(1 + t) * n + i] / pred[i]); up to four kinds per call. */
