@@ -3,6 +3,7 @@
 There is no fallback: if the shared library has not been built, importing this
 module raises, and so does every API that needs it.
 """
+import atexit
 import ctypes
 import os
 
@@ -203,6 +204,7 @@ def binding():
     module.setup({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in EXPORTS},
                  device_table.row_of, check, batched.WaveResult)
     module.set_generation(device_table.generation())
+    atexit.register(module.release_host_blocks)
     _binding = module
     return module
 

@@ -5,6 +5,7 @@ C ABI (include/habitat_b200.h).  torch is used for device memory and streams
 only; all arithmetic happens in the library's sm_100a kernels.
 """
 import ctypes
+import math
 import os
 from dataclasses import dataclass
 from typing import Optional, Sequence
@@ -12,7 +13,7 @@ from typing import Optional, Sequence
 import numpy as np
 import torch
 
-from habitat_b200 import _native, device_table
+from habitat_b200 import _native
 
 
 def _require_cuda(t, dtype, name):
@@ -182,31 +183,35 @@ def wave_scale_path():
 
 
 def wave_scale_host(arrays, origin, dests, want_status=False, want_limits=False):
-    """Host-buffer path: numpy in, numpy out, transfers inside the native call."""
-    lib = _native.load()
-    nb = np.ascontiguousarray(arrays["num_blocks"], dtype=np.int32)
-    bs = np.ascontiguousarray(arrays["block_size"], dtype=np.uint16)
-    rg = np.ascontiguousarray(arrays["regs_per_thread"], dtype=np.uint16)
-    sm = np.ascontiguousarray(arrays["smem_bytes"], dtype=np.uint32)
-    tm = np.ascontiguousarray(arrays["run_time_ns"], dtype=np.float32)
-    gm = np.ascontiguousarray(arrays["gamma"], dtype=np.float32)
-    K, D = nb.shape[0], len(dests)
-    rows = device_table.rows_of([origin] + list(dests))
-    res = dict(
-        scaled_ns=np.empty((D, K), np.float32), dest_occupancy=np.empty((D, K), np.uint8),
-        dest_waves=np.empty((D, K), np.uint32), origin_occupancy=np.empty((K,), np.uint8),
-        origin_waves=np.empty((K,), np.uint32),
-        status=np.empty((D, K), np.uint8) if want_status else None,
-        limits=np.empty((D + 1, 4, K), np.int32) if want_limits else None)
-    p = lambda a: ctypes.c_void_p(a.ctypes.data) if a is not None else ctypes.c_void_p(0)
-    soa = _native.KernelSoA(p(nb), p(bs), p(rg), p(sm), p(tm), p(gm))
-    wout = _native.WaveOut(p(res["scaled_ns"]), p(res["dest_occupancy"]), p(res["dest_waves"]),
-                           p(res["origin_occupancy"]), p(res["origin_waves"]), p(res["status"]),
-                           p(res["limits"]))
-    dest_rows = (ctypes.c_int32 * D)(*rows[1:])
-    _native.check(lib.hb_wave_scale_host(ctypes.byref(soa), K, rows[0], dest_rows, D,
-                                         ctypes.c_void_p(0), ctypes.byref(wout)))
-    return res
+    """Host-buffer path: numpy in, numpy out, transfers inside the native call.  Results of up to a
+    few megabytes lie in one block of page-locked memory that the kernel writes directly."""
+    binding = _native.binding()
+    ins = [np.ascontiguousarray(arrays[name], dtype=dt) for name, dt in _HOST_IN]
+    K, D = ins[0].shape[0], len(dests)
+    names = ("scaled_ns", "dest_occupancy", "dest_waves", "origin_occupancy", "origin_waves", "status", "limits")
+    pairs = (D, K)
+    planes = [(names[0], np.float32, pairs, 4), (names[1], np.uint8, pairs, 1), (names[2], np.uint32, pairs, 4),
+              (names[3], np.uint8, (K,), 1), (names[4], np.uint32, (K,), 4),
+              (names[5], np.uint8, pairs, 1) if want_status else None,
+              (names[6], np.int32, (D + 1, 4, K), 4) if want_limits else None]
+    at, total = [], 0
+    for p in planes:
+        at.append(total)
+        if p is not None:
+            total += (math.prod(p[2]) * p[3] + 255) & ~255
+    block = binding.host_block(total) if total and not want_limits else None
+    if block is not None:
+        outs = [None if p is None else np.ndarray(p[2], p[1], block, o) for p, o in zip(planes, at)]
+    else:
+        outs = [None if p is None else np.empty(p[2], p[1]) for p in planes]
+    if binding.wave_scale_host(*ins, origin, dests, tuple(outs)) is None:
+        raise ValueError("the kernel arrays must have the same length (at most %d destinations)"
+                         % _native.HB_MAX_DEVICES)
+    return dict(zip(names, outs))
+
+
+_HOST_IN = (("num_blocks", np.int32), ("block_size", np.uint16), ("regs_per_thread", np.uint16),
+            ("smem_bytes", np.uint32), ("run_time_ns", np.float32), ("gamma", np.float32))
 
 
 class MLPHandle:

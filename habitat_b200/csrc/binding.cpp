@@ -9,7 +9,9 @@
 #include <Python.h>
 
 #include <ATen/EmptyTensor.h>
+#include <ATen/core/CachingHostAllocator.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -18,6 +20,8 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
+#include <utility>
 #include <vector>
 
 #include "habitat_b200.h"
@@ -28,6 +32,7 @@ struct Api {
   decltype(&hb_wave_scale) wave_scale = nullptr;
   decltype(&hb_wave_scale_metrics) wave_scale_metrics = nullptr;
   decltype(&hb_wave_scale_partials) wave_scale_partials = nullptr;
+  decltype(&hb_wave_scale_host) wave_scale_host = nullptr;
   decltype(&hb_partials_sum) partials_sum = nullptr;
   decltype(&hb_mlp_predict) mlp_predict = nullptr;
   decltype(&hb_mlp_predict_host) mlp_predict_host = nullptr;
@@ -767,6 +772,221 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   END_HANDLE_TH_ERRORS
 }
 
+// submit_wave(block, device block, kernels, origin, dests, out, partials or None, totals or None,
+//             [(host tensor, device tensor)], (upload, compute, download stream handles),
+//             (uploaded, computed, downloaded event handles), used)
+// One batch of hostio.WaveScaleHost: upload of a record block, wave scaling, download of the wanted results on
+// three streams that events tie together.  `used`: the slot's buffers have held a batch before.
+PyObject* submit_wave(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 12 || !THPVariable_Check(a[0]) || !THPVariable_Check(a[1]) || !PyList_Check(a[8]) || !PyTuple_Check(a[9]) ||
+      !PyTuple_Check(a[10])) {
+    PyErr_SetString(PyExc_TypeError, "submit_wave: bad arguments");
+    return nullptr;
+  }
+  cudaStream_t s[3];
+  cudaEvent_t ev[3];
+  for (int i = 0; i < 3; ++i) {
+    s[i] = static_cast<cudaStream_t>(PyLong_AsVoidPtr(PyTuple_GET_ITEM(a[9], i)));
+    ev[i] = static_cast<cudaEvent_t>(PyLong_AsVoidPtr(PyTuple_GET_ITEM(a[10], i)));
+  }
+  const bool used = PyObject_IsTrue(a[11]) == 1;
+  if (PyErr_Occurred()) return nullptr;
+  auto ok = [](cudaError_t e) {
+    if (e == cudaSuccess) return true;
+    PyErr_Format(PyExc_RuntimeError, "submit_wave: %s", cudaGetErrorString(e));
+    return false;
+  };
+  // a page-locked tensor that its owner drops is not reused before the stream has come this far
+  auto copy = [&](const at::Tensor& dst, const at::Tensor& src, cudaStream_t stream) {
+    if (!ok(cudaMemcpyAsync(dst.mutable_data_ptr(), src.data_ptr(), dst.nbytes(), cudaMemcpyDefault, stream))) return false;
+    const at::Tensor& host = src.is_cuda() ? dst : src;
+    const at::Device dev = (src.is_cuda() ? src : dst).device();
+    if (!host.is_cuda())
+      at::getHostAllocator(at::kCUDA)->record_event(host.mutable_data_ptr(), host.storage().data_ptr().get_context(),
+                                                    c10::cuda::getStreamFromExternal(stream, dev.index()).unwrap());
+    return true;
+  };
+  const at::Tensor &block = THPVariable_Unpack(a[0]), &dev_block = THPVariable_Unpack(a[1]);
+  const c10::DeviceIndex index = dev_block.device().index();
+  // the slot's device inputs were last read by the kernel of batch (i - depth)
+  if (used && !ok(cudaStreamWaitEvent(s[0], ev[1], 0))) return nullptr;
+  if (!copy(dev_block, block, s[0]) || !ok(cudaEventRecord(ev[0], s[0])) || !ok(cudaStreamWaitEvent(s[1], ev[0], 0)))
+    return nullptr;
+  // the kernel of this batch overwrites outputs the download of batch (i - depth) reads
+  if (used && !ok(cudaStreamWaitEvent(s[1], ev[2], 0))) return nullptr;
+  {
+    c10::cuda::CUDAStreamGuard guard(c10::cuda::getStreamFromExternal(s[1], index));
+    PyObject* args[9] = {a[2], a[3], a[4], Py_None, Py_None, Py_False, Py_False, a[5], a[6]};
+    Ref r(wave_scale(nullptr, args, 9));
+    if (!r.p) return nullptr;
+    if (r.p == Py_None) Py_RETURN_NONE;
+    if (a[6] != Py_None) {
+      Ref buffer(PyObject_GetAttr(a[6], s_buffer)), per(PyObject_GetAttr(a[6], s_per_plane)),
+          planes(PyObject_GetAttr(a[6], s_n_planes));
+      if (!buffer.p || !per.p || !planes.p) return nullptr;
+      PyObject* sum[4] = {buffer.p, per.p, planes.p, a[7]};
+      Ref t(partials_sum(nullptr, sum, 4));
+      if (!t.p) return nullptr;
+      if (t.p == Py_None) Py_RETURN_NONE;
+    }
+  }
+  if (!ok(cudaEventRecord(ev[1], s[1])) || !ok(cudaStreamWaitEvent(s[2], ev[1], 0))) return nullptr;
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[8]); ++i) {
+    PyObject* t = PyList_GET_ITEM(a[8], i);
+    if (!copy(THPVariable_Unpack(PyTuple_GET_ITEM(t, 0)), THPVariable_Unpack(PyTuple_GET_ITEM(t, 1)), s[2])) return nullptr;
+  }
+  if (!ok(cudaEventRecord(ev[2], s[2]))) return nullptr;
+  Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------------------
+// Page-locked memory for host results
+// ---------------------------------------------------------------------------
+// Arrays over such blocks are what batched.wave_scale_host returns: the kernel writes them directly.  A block
+// goes back to the pool when the last array over it goes.  Blocks come in quarter steps between powers of two,
+// of at most kMostBlock bytes and kMostTotal in all (page-locking costs about 0.3 ms per MB, so it must not
+// recur); a caller who keeps more results than that gets the rest in ordinary memory, as does one who asks for a
+// larger block.  Room for a few results of a million kernels on eight devices.
+constexpr size_t kMostBlock = 128 << 20, kMostTotal = 256 << 20;
+struct HostBlocks {
+  std::mutex mu;
+  std::vector<std::pair<size_t, void*>> idle;
+  size_t total = 0;
+};
+HostBlocks& host_blocks() {
+  static HostBlocks* b = new HostBlocks();   // never destroyed: arrays may outlive the interpreter's own clean-up
+  return *b;
+}
+struct HostBlock {
+  PyObject_HEAD
+  void* ptr;
+  size_t bytes;      // of the block
+  Py_ssize_t asked;
+};
+void host_block_dealloc(PyObject* o) {
+  HostBlock* b = reinterpret_cast<HostBlock*>(o);
+  if (b->ptr) {
+    HostBlocks& pool = host_blocks();
+    std::lock_guard<std::mutex> lock(pool.mu);
+    pool.idle.emplace_back(b->bytes, b->ptr);
+  }
+  Py_TYPE(o)->tp_free(o);
+}
+int host_block_buffer(PyObject* o, Py_buffer* view, int flags) {
+  HostBlock* b = reinterpret_cast<HostBlock*>(o);
+  return PyBuffer_FillInfo(view, o, b->ptr, b->asked, 0, flags);
+}
+PyBufferProcs host_block_procs = {host_block_buffer, nullptr};
+PyTypeObject host_block_type = [] {
+  PyTypeObject t = {PyVarObject_HEAD_INIT(nullptr, 0)};
+  t.tp_name = "habitat_b200._binding.HostBlock";
+  t.tp_basicsize = sizeof(HostBlock);
+  t.tp_flags = Py_TPFLAGS_DEFAULT;
+  t.tp_dealloc = host_block_dealloc;
+  t.tp_as_buffer = &host_block_procs;
+  return t;
+}();
+
+// host_block(bytes) -> an object with a writable buffer in page-locked memory, or None (see above)
+PyObject* host_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 1) Py_RETURN_NONE;
+  const Py_ssize_t asked = PyLong_AsSsize_t(a[0]);
+  if (PyErr_Occurred()) return nullptr;
+  if (asked < 0 || static_cast<size_t>(asked) > kMostBlock) Py_RETURN_NONE;
+  size_t top = 4096;
+  while (top < static_cast<size_t>(asked)) top *= 2;
+  size_t bytes = top / 2;
+  while (bytes < static_cast<size_t>(asked) || bytes < 4096) bytes += top / 8;
+  HostBlocks& pool = host_blocks();
+  void* ptr = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(pool.mu);
+    for (size_t i = 0; i < pool.idle.size() && !ptr; ++i) {
+      if (pool.idle[i].first != bytes) continue;
+      ptr = pool.idle[i].second;
+      pool.idle.erase(pool.idle.begin() + static_cast<std::ptrdiff_t>(i));
+    }
+    // make room by giving back idle blocks of other sizes
+    while (!ptr && pool.total + bytes > kMostTotal && !pool.idle.empty()) {
+      pool.total -= pool.idle.back().first;
+      cudaFreeHost(pool.idle.back().second);
+      pool.idle.pop_back();
+    }
+    if (!ptr && pool.total + bytes <= kMostTotal) {
+      if (cudaHostAlloc(&ptr, bytes, cudaHostAllocPortable) == cudaSuccess) pool.total += bytes;
+      else cudaGetLastError();
+    }
+  }
+  if (!ptr) Py_RETURN_NONE;
+  HostBlock* b = PyObject_New(HostBlock, &host_block_type);
+  if (!b) return nullptr;
+  b->ptr = ptr;
+  b->bytes = bytes;
+  b->asked = asked;
+  return reinterpret_cast<PyObject*>(b);
+}
+// release_host_blocks(): gives the idle blocks back
+PyObject* release_host_blocks(PyObject*, PyObject* const*, Py_ssize_t) {
+  HostBlocks& pool = host_blocks();
+  std::lock_guard<std::mutex> lock(pool.mu);
+  for (auto& b : pool.idle) {
+    cudaFreeHost(b.second);
+    pool.total -= b.first;
+  }
+  pool.idle.clear();
+  Py_RETURN_NONE;
+}
+
+// wave_scale_host(num_blocks, block_size, regs, smem, time, gamma, origin, dests,
+//                 (scaled, occupancy, waves, origin occupancy, origin waves, status or None, limits or None))
+// -> True, or None when a buffer does not fit
+PyObject* wave_scale_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 9 || !PyTuple_Check(a[8]) || PyTuple_GET_SIZE(a[8]) != 7) Py_RETURN_NONE;
+  Ref dests(PySequence_Fast(a[7], "dests must be a sequence of DeviceProperties"));
+  if (!dests.p) return nullptr;
+  const Py_ssize_t D = PySequence_Fast_GET_SIZE(dests.p);
+  if (D > HB_MAX_DEVICES) Py_RETURN_NONE;
+  const Buffer<int32_t> nb(a[0], false);
+  const Buffer<uint16_t> bs(a[1], false), rg(a[2], false);
+  const Buffer<uint32_t> sm(a[3], false);
+  const Buffer<float> tm(a[4], false), gm(a[5], false);
+  const int64_t K = nb.size();
+  if (!nb.held || !bs.ok(K) || !rg.ok(K) || !sm.ok(K) || !tm.ok(K) || !gm.ok(K)) Py_RETURN_NONE;
+  const long origin = row_of(a[6]);
+  if (origin < 0) return nullptr;
+  int32_t rows[HB_MAX_DEVICES];
+  for (Py_ssize_t d = 0; d < D; ++d) {
+    const long r = row_of(PySequence_Fast_GET_ITEM(dests.p, d));
+    if (r < 0) return nullptr;
+    rows[d] = static_cast<int32_t>(r);
+  }
+  auto result = [&](int i) { return PyTuple_GET_ITEM(a[8], i); };
+  const Buffer<float> ns(result(0), true);
+  const Buffer<uint8_t> occ(result(1), true), oocc(result(3), true);
+  const Buffer<uint32_t> wav(result(2), true), owav(result(4), true);
+  if (!ns.ok(D * K) || !occ.ok(D * K) || !wav.ok(D * K) || !oocc.ok(K) || !owav.ok(K)) Py_RETURN_NONE;
+  hb_wave_out out{ns.data(), occ.data(), wav.data(), oocc.data(), owav.data(), nullptr, nullptr};
+  const Buffer<uint8_t> status(result(5), true);
+  const Buffer<int32_t> limits(result(6), true);
+  if (result(5) != Py_None) {
+    if (!status.ok(D * K)) Py_RETURN_NONE;
+    out.status = status.data();
+  }
+  if (result(6) != Py_None) {
+    if (!limits.ok((D + 1) * 4 * K)) Py_RETURN_NONE;
+    out.limits = limits.data();
+  }
+  const hb_kernel_soa k{nb.data(), bs.data(), rg.data(), sm.data(), tm.data(), gm.data()};
+  hb_status st;
+  Py_BEGIN_ALLOW_THREADS
+  st = api.wave_scale_host(&k, K, static_cast<int32_t>(origin), rows, static_cast<int32_t>(D), nullptr, &out);
+  Py_END_ALLOW_THREADS
+  if (failed(st)) return nullptr;
+  Py_RETURN_TRUE;
+}
+
 // run_group(kernels or None, metrics or None, origin, dests, dest_regs or None, offsets or None,
 //           [(handle address, features, measured ms, device rows (bytes: origin, then the destinations),
 //             operation indices (int64))],
@@ -1082,7 +1302,8 @@ PyObject* setup(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return fn != nullptr;
   };
   if (!load(api.wave_scale, "hb_wave_scale") || !load(api.wave_scale_metrics, "hb_wave_scale_metrics") ||
-      !load(api.wave_scale_partials, "hb_wave_scale_partials") || !load(api.partials_sum, "hb_partials_sum") ||
+      !load(api.wave_scale_partials, "hb_wave_scale_partials") ||
+      !load(api.wave_scale_host, "hb_wave_scale_host") || !load(api.partials_sum, "hb_partials_sum") ||
       !load(api.mlp_predict, "hb_mlp_predict") || !load(api.mlp_predict_host, "hb_mlp_predict_host") || !load(api.group_sum, "hb_group_sum") ||
       !load(api.plane_sum, "hb_plane_sum") || !load(api.segment_sum, "hb_segment_sum") ||
       !load(api.segment_sum_planes, "hb_segment_sum_planes") ||
@@ -1105,7 +1326,7 @@ PyObject* set_generation(PyObject*, PyObject* v) {
 }
 
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {FAST(setup), FAST(wave_scale), FAST(mlp_predict), FAST(mlp_predict_one), FAST(flatten_trace), FAST(run_group), FAST(iteration_totals), FAST(partials_sum), FAST(group_sum),
+PyMethodDef methods[] = {FAST(setup), FAST(wave_scale), FAST(wave_scale_host), FAST(submit_wave), FAST(host_block), FAST(release_host_blocks), FAST(mlp_predict), FAST(mlp_predict_one), FAST(flatten_trace), FAST(run_group), FAST(iteration_totals), FAST(partials_sum), FAST(group_sum),
                          FAST(plane_sum), FAST(segment_sum),
                          {"set_generation", set_generation, METH_O, nullptr},
                          {nullptr, nullptr, 0, nullptr}};
@@ -1130,5 +1351,6 @@ PyMODINIT_FUNC PyInit__binding(void) {
       {&s__run_time_ns, "_run_time_ns"}, {&s_name, "name"}};
   for (const auto& n : names)
     if (!(*n.s = PyUnicode_InternFromString(n.name))) return nullptr;
+  if (PyType_Ready(&host_block_type) < 0) return nullptr;
   return PyModule_Create(&module);
 }

@@ -36,6 +36,7 @@ struct HostArena {
   void* base = nullptr;
   size_t bytes = 0;
   cudaStream_t stream = nullptr;
+  cudaStream_t more[3] = {};   // further streams, created when first asked for (arena_stream)
   uint8_t* pinned = nullptr;   // page-locked, readable and writable by the GPU at the same address
   size_t pinned_bytes = 0;
 };
@@ -44,6 +45,8 @@ hb_status arena_for_current_device(HostArena** out);
 // Makes the block at least `bytes` large.  Call with the arena's mutex held.
 hb_status arena_reserve(HostArena* arena, size_t bytes);
 
+// Stream i (0: arena->stream) of up to four.  Call with the arena's mutex held.
+hb_status arena_stream(HostArena* arena, int i, cudaStream_t* out);
 // The same for the page-locked block.
 hb_status arena_reserve_pinned(HostArena* arena, size_t bytes);
 

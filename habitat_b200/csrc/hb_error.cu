@@ -65,6 +65,16 @@ hb_status arena_reserve(HostArena* a, size_t bytes) {
   return HB_OK;
 }
 
+hb_status arena_stream(HostArena* a, int i, cudaStream_t* out) {
+  cudaStream_t* s = i == 0 ? &a->stream : &a->more[i - 1];
+  if (!*s) {
+    const cudaError_t e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaStreamCreateWithFlags");
+  }
+  *out = *s;
+  return HB_OK;
+}
+
 hb_status arena_reserve_pinned(HostArena* a, size_t bytes) {
   if (bytes <= a->pinned_bytes) return HB_OK;
   if (a->pinned) cudaFreeHost(a->pinned);

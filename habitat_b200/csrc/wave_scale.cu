@@ -18,6 +18,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <string>
+#include <thread>
 #include <vector>
 
 #include "hb_common.h"
@@ -409,6 +411,7 @@ __device__ __forceinline__ LutDevRegs load_lut_dev(const LutDev& d) {
 
 struct LutParams {
   uint32_t K;
+  uint32_t stride;                                   // elements from one output plane to the next
   int32_t D;
   uint32_t off_p[kMaxClasses], off_s[kMaxClasses];   // byte offsets of the class tables
   double origin_peak;                                // metrics mode: origin peak GFLOP/s
@@ -598,7 +601,7 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
 #pragma unroll 1
     for (int d = 0; d < D; ++d) {
       const LutDevRegs dd = load_lut_dev(lp.dest[d]);
-      const uint32_t base = static_cast<uint32_t>(d) * K + k0;   // D K < 2^31
+      const uint32_t base = static_cast<uint32_t>(d) * lp.stride + k0;   // D K < 2^31
       uint32_t occ2;
       if (!EXT) {
         occ2 = __vimin_s16x2_relu(prmt(P[0], P[1], dd.sel.x), prmt(S[0], S[1], dd.sel.y));
@@ -874,15 +877,17 @@ void fill_lut(LaunchPlan* plan) {   // call with g_mu held
 
 // Launches wave_scale_lut_kernel when the launch qualifies; false = nothing launched.  *fused says
 // whether the launch also wrote p.block_sums (one sum per destination and block of the grid).
-bool try_launch_lut(const Ptrs& p, const LaunchPlan& plan, int64_t K, int sm_count, cudaStream_t stream, hb_status* st,
-                    bool* fused, unsigned* fused_blocks) {
+// Output planes (and dest_regs) are `stride` >= K elements apart.
+bool try_launch_lut(const Ptrs& p, const LaunchPlan& plan, int64_t K, int64_t stride, int sm_count, cudaStream_t stream,
+                    hb_status* st, bool* fused, unsigned* fused_blocks, bool to_host = false) {
   *fused = false;
   static const bool use_lut = [] { const char* e = std::getenv("HB_WAVE_LUT"); return !e || std::atoi(e) != 0; }();
   const LaunchParams& lp = plan.lp;
   if (!use_lut || p.limits || !plan.lut_ok) return false;
-  if (static_cast<int64_t>(lp.D) * K >= (int64_t{1} << 31)) return false;   // 32-bit element indices
+  if (static_cast<int64_t>(lp.D) * stride >= (int64_t{1} << 31)) return false;   // 32-bit element indices
   LutParams q = plan.q;
   q.K = static_cast<uint32_t>(K);
+  q.stride = static_cast<uint32_t>(stride);
   const int n_p = plan.n_p, n_s = plan.n_s;
   const bool many_classes = plan.many_classes;
 
@@ -892,8 +897,10 @@ bool try_launch_lut(const Ptrs& p, const LaunchPlan& plan, int64_t K, int sm_cou
   // two records per thread when the inputs sit on 8-byte boundaries; 8-byte stores when the
   // output planes do too (K even)
   const bool vec2 = al(p.num_blocks, 8) && al(p.smem, 8) && al(p.time_ns, 8) && (metrics || al(p.gamma, 8)) &&
-                    al(p.block_size, 4) && al(p.regs, 4) && K >= 2;
-  const bool aligned = vec2 && K % 2 == 0 && al(p.scaled_ns, 8) && al(p.dest_waves, 8) && al(p.origin_waves, 8) &&
+                    al(p.block_size, 4) && al(p.regs, 4) && K >= 2 &&
+                    // over PCIe every warp's store should be one piece: no two-record threads with odd planes
+                    !(to_host && stride % 2 != 0);
+  const bool aligned = vec2 && K % 2 == 0 && stride % 2 == 0 && al(p.scaled_ns, 8) && al(p.dest_waves, 8) && al(p.origin_waves, 8) &&
                        al(p.dest_occ, 2) && al(p.origin_occ, 2) && (!p.status || al(p.status, 2)) &&
                        (!p.dest_regs || al(p.dest_regs, 4));
   const int vec = vec2 ? 2 : 1;
@@ -980,7 +987,7 @@ hb_status launch_kernel(const Ptrs& p, const LaunchPlan& plan, int64_t K, cudaSt
   const bool extra = p.status != nullptr || p.limits != nullptr;
   hb_status fast_st = HB_OK;
   *fused = false;
-  if (try_launch_lut(p, plan, K, sm_count, stream, &fast_st, fused, fused_blocks)) return fast_st;
+  if (try_launch_lut(p, plan, K, K, sm_count, stream, &fast_st, fused, fused_blocks)) return fast_st;
   if (!METRICS && try_launch_fast(p, plan.lp, K, stream, &fast_st)) return fast_st;
   LaunchParams lp = plan.lp;
   lp.K = K;
@@ -1244,6 +1251,197 @@ extern "C" hb_status hb_wave_scale_metrics(const hb_kernel_soa* kernels,
                       static_cast<cudaStream_t>(stream));
 }
 
+// ---------------------------------------------------------------------------
+// Host buffers.  The kernels read staged records from, and write results to, page-locked host memory
+// directly: at 65,536 kernels x 6 destinations (1.3 MB in, 3.9 MB out) that is as fast over PCIe as eleven
+// copies around the launch (114 against 155 us) and for a few kernels it saves all of their latency.  What
+// is left is the host's own copying, 16 GB/s for one core: 82 us to stage those records and 230 us to bring the
+// results to ordinary memory.  So
+//   * records are staged chunk by chunk, and a chunk's launch runs while the next one is staged;
+//   * results in page-locked memory of the caller (batched.wave_scale_host gives such arrays) are written there;
+//   * otherwise large batches go through four threads, each with its part of the staging block and a
+//     stream: stage, launch, wait, copy out, next chunk.
+// ---------------------------------------------------------------------------
+namespace {
+
+// The planes of one call, as (element size, whether per destination).
+struct HostPlanes {
+  static constexpr int kIn = 7, kOut = 7;
+  const uint8_t* in[kIn];
+  uint8_t* out[kOut];
+  size_t in_size[kIn] = {4, 2, 2, 4, 4, 4, 2};     // num_blocks, block, regs, smem, time, gamma | dest_regs [D][K]
+  size_t out_size[kOut] = {4, 1, 4, 1, 4, 1, 4};   // scaled, occ, waves [D][K] | origin occ, waves [K] | status [D][K] | limits
+  int in_rows[kIn], out_rows[kOut];
+  int64_t K;
+
+  HostPlanes(const hb_kernel_soa* k, const int16_t* regs, const hb_wave_out* o, int64_t K_, int D) : K(K_) {
+    const void* i[kIn] = {k->num_blocks, k->block_size, k->regs_per_thread, k->smem_bytes, k->run_time_ns, k->gamma, regs};
+    void* q[kOut] = {o->scaled_ns, o->dest_occupancy, o->dest_waves, o->origin_occupancy, o->origin_waves, o->status, o->limits};
+    for (int j = 0; j < kIn; ++j) {
+      in[j] = static_cast<const uint8_t*>(i[j]);
+      in_rows[j] = in[j] ? (j < 6 ? 1 : D) : 0;
+    }
+    for (int j = 0; j < kOut; ++j) {
+      out[j] = static_cast<uint8_t*>(q[j]);
+      out_rows[j] = !out[j] ? 0 : (j == 3 || j == 4 ? 1 : (j == 6 ? 4 * (D + 1) : D));
+    }
+  }
+  static size_t up(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
+  size_t in_bytes(int64_t n) const {
+    size_t b = 0;
+    for (int j = 0; j < kIn; ++j) b += up(in_size[j] * in_rows[j] * n);
+    return b;
+  }
+  size_t out_bytes(int64_t n) const {
+    size_t b = 0;
+    for (int j = 0; j < kOut; ++j) b += up(out_size[j] * out_rows[j] * n);
+    return b;
+  }
+  // Copies records [lo, lo + n) into `slot` and points p at them; dest_regs rows end up n apart.
+  uint8_t* stage(uint8_t* slot, int64_t lo, int64_t n, Ptrs* p) const {
+    uint8_t* at[kIn];
+    for (int j = 0; j < kIn; ++j) {
+      at[j] = in_rows[j] ? slot : nullptr;
+      const size_t row = in_size[j] * n;
+      for (int r = 0; r < in_rows[j]; ++r) std::memcpy(slot + r * row, in[j] + in_size[j] * (r * K + lo), row);
+      slot += up(row * in_rows[j]);
+    }
+    p->num_blocks = reinterpret_cast<const int32_t*>(at[0]);
+    p->block_size = reinterpret_cast<const uint16_t*>(at[1]);
+    p->regs = reinterpret_cast<const uint16_t*>(at[2]);
+    p->smem = reinterpret_cast<const uint32_t*>(at[3]);
+    p->time_ns = reinterpret_cast<const float*>(at[4]);
+    p->gamma = reinterpret_cast<const float*>(at[5]);
+    p->dest_regs = reinterpret_cast<const int16_t*>(at[6]);
+    return slot;
+  }
+  static void set_out(Ptrs* p, uint8_t* const (&at)[kOut]) {
+    p->scaled_ns = reinterpret_cast<float*>(at[0]);
+    p->dest_occ = at[1];
+    p->dest_waves = reinterpret_cast<uint32_t*>(at[2]);
+    p->origin_occ = at[3];
+    p->origin_waves = reinterpret_cast<uint32_t*>(at[4]);
+    p->status = at[5];
+    p->limits = reinterpret_cast<int32_t*>(at[6]);
+  }
+  // The caller's own result planes from record lo on (rows K apart).
+  void out_there(int64_t lo, Ptrs* p) const {
+    uint8_t* at[kOut];
+    for (int j = 0; j < kOut; ++j) at[j] = out[j] ? out[j] + out_size[j] * lo : nullptr;
+    set_out(p, at);
+  }
+  // Result planes of n records in `slot` (rows n apart).
+  void out_in_slot(uint8_t* slot, int64_t n, Ptrs* p) const {
+    uint8_t* at[kOut];
+    for (int j = 0; j < kOut; ++j) {
+      at[j] = out_rows[j] ? slot : nullptr;
+      slot += up(out_size[j] * out_rows[j] * n);
+    }
+    set_out(p, at);
+  }
+  // ... and from there to the caller's planes.
+  void fetch(const uint8_t* slot, int64_t lo, int64_t n) const {
+    for (int j = 0; j < kOut; ++j) {
+      const size_t row = out_size[j] * n;
+      for (int r = 0; r < out_rows[j]; ++r) std::memcpy(out[j] + out_size[j] * (r * K + lo), slot + r * row, row);
+      slot += up(row * out_rows[j]);
+    }
+  }
+  // Whether the GPU can write every result plane where it is.
+  bool results_page_locked() const {
+    for (int j = 0; j < kOut; ++j) {
+      if (!out[j]) continue;
+      cudaPointerAttributes a{};
+      if (cudaPointerGetAttributes(&a, out[j]) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+      if (a.type != cudaMemoryTypeHost || a.devicePointer != out[j]) return false;
+    }
+    return true;
+  }
+};
+
+constexpr int kHostThreads = 4;
+constexpr size_t kHostDirectBytes = 32u << 20;   // of staged records
+
+// Results to ordinary memory.  Each thread takes every kHostThreads-th chunk.
+hb_status host_in_threads(hb::HostArena* arena, const HostPlanes& io, const LaunchPlan& plan, int64_t K, int64_t chunk,
+                          int threads, int device) {
+  const size_t slot_bytes = io.in_bytes(chunk) + io.out_bytes(chunk);
+  hb_status st = hb::arena_reserve_pinned(arena, slot_bytes * threads);
+  if (st != HB_OK) return st;
+  hb_status got[kHostThreads];
+  std::string text[kHostThreads];
+  auto work = [&](int w) {
+    cudaStream_t s = w == 0 ? arena->stream : arena->more[w - 1];
+    uint8_t* slot = arena->pinned + slot_bytes * w;
+    hb_status mine = cudaSetDevice(device) == cudaSuccess ? HB_OK : HB_ERR_CUDA;
+    for (int64_t lo = chunk * w; lo < K && mine == HB_OK; lo += chunk * threads) {
+      const int64_t n = K - lo < chunk ? K - lo : chunk;
+      Ptrs p{};
+      uint8_t* results = io.stage(slot, lo, n, &p);
+      io.out_in_slot(results, n, &p);
+      mine = launch<false>(p, plan, n, s);
+      const cudaError_t e = cudaStreamSynchronize(s);
+      if (mine == HB_OK && e != cudaSuccess) mine = hb::cuda_fail(e, "hb_wave_scale_host");
+      if (mine == HB_OK) io.fetch(results, lo, n);
+    }
+    got[w] = mine;
+    if (mine != HB_OK) text[w] = hb_last_error();
+  };
+  std::thread helpers[kHostThreads];
+  for (int w = 1; w < threads; ++w) helpers[w] = std::thread(work, w);
+  work(0);
+  for (int w = 1; w < threads; ++w) helpers[w].join();
+  for (int w = 0; w < threads; ++w) {
+    if (got[w] == HB_OK) continue;
+    hb::set_error("%s", text[w].c_str());   // the text of another thread
+    return got[w];
+  }
+  return HB_OK;
+}
+
+// Results straight into the caller's page-locked planes; two streams, so that a chunk's launch does not wait for
+// the last writes of the one before it.  Only the table kernel knows planes that are further apart than its
+// records; other launches take the batch as one chunk.
+hb_status host_direct(hb::HostArena* arena, const HostPlanes& io, const LaunchPlan& plan, int64_t K, int64_t chunk) {
+  hb_status st = hb::arena_reserve_pinned(arena, io.in_bytes(K) + HostPlanes::kIn * 256 * (K / chunk + 1));
+  if (st != HB_OK) return st;
+  int sm_count = 0;
+  st = sync_gpu(&sm_count);
+  if (st != HB_OK) return st;
+  uint8_t* slot = arena->pinned;
+  int used = 0;
+  for (int64_t lo = 0, c = 0; lo < K && st == HB_OK; lo += chunk, ++c) {
+    const int64_t n = K - lo < chunk ? K - lo : chunk;
+    cudaStream_t s = c & 1 ? arena->more[0] : arena->stream;
+    Ptrs p{};
+    slot = io.stage(slot, lo, n, &p);
+    io.out_there(lo, &p);
+    {
+      bool fused = false;
+      unsigned blocks = 0;
+      if (!try_launch_lut(p, plan, n, K, sm_count, s, &st, &fused, &blocks, true)) {
+        // not for the table kernel (the first chunk says so): everything at once
+        slot = io.stage(arena->pinned, 0, K, &p);
+        io.out_there(0, &p);
+        st = launch<false>(p, plan, K, s);
+        lo = K;
+      }
+    }
+    used |= 1 << (c & 1);
+  }
+  for (int i = 0; i < 2; ++i) {
+    if (!(used >> i & 1)) continue;
+    const cudaError_t e = cudaStreamSynchronize(i ? arena->more[0] : arena->stream);
+    if (st == HB_OK && e != cudaSuccess) st = hb::cuda_fail(e, "hb_wave_scale_host");
+  }
+  return st;
+}
+
+}  // namespace
+
 extern "C" hb_status hb_wave_scale_host(const hb_kernel_soa* kernels, int64_t K,
                                         int32_t origin_row, const int32_t* dest_rows_host,
                                         int32_t D, const int16_t* dest_regs,
@@ -1254,58 +1452,39 @@ extern "C" hb_status hb_wave_scale_host(const hb_kernel_soa* kernels, int64_t K,
   st = plan_for(&plan, K, origin_row, dest_rows_host, D);
   if (st != HB_OK) return st;
   if (K == 0) return HB_OK;
-  const size_t k = static_cast<size_t>(K), kd = k * D;
-  // one staging block per GPU, kept between calls, and the library's own stream
+  int device = 0;
+  HB_CUDA_TRY(cudaGetDevice(&device));
+  // one page-locked staging block per GPU, kept between calls, and the library's own streams
   hb::HostArena* arena = nullptr;
   st = hb::arena_for_current_device(&arena);
   if (st != HB_OK) return st;
   std::lock_guard<std::mutex> lock(arena->mu);
-  const size_t lim_bytes = out->limits ? static_cast<size_t>(D + 1) * 4 * k * 4 : 0;
-  hb::Carver sizes(nullptr);
-  sizes.take<uint8_t>(k * 4); sizes.take<uint8_t>(k * 2); sizes.take<uint8_t>(k * 2); sizes.take<uint8_t>(k * 4);
-  sizes.take<uint8_t>(k * 4); sizes.take<uint8_t>(k * 4); sizes.take<uint8_t>(kd * 4); sizes.take<uint8_t>(kd);
-  sizes.take<uint8_t>(kd * 4); sizes.take<uint8_t>(k); sizes.take<uint8_t>(k * 4); sizes.take<uint8_t>(kd * 2);
-  sizes.take<uint8_t>(kd); sizes.take<uint8_t>(lim_bytes);
-  st = hb::arena_reserve(arena, sizes.used());
-  if (st != HB_OK) return st;
-  hb::Carver c(arena->base);
-  int32_t* nb = c.take<int32_t>(k);
-  uint16_t* bs = c.take<uint16_t>(k);
-  uint16_t* rg = c.take<uint16_t>(k);
-  uint32_t* sm = c.take<uint32_t>(k);
-  float* tm = c.take<float>(k);
-  float* gm = c.take<float>(k);
-  float* o_ns = c.take<float>(kd);
-  uint8_t* o_occ = c.take<uint8_t>(kd);
-  uint32_t* o_wav = c.take<uint32_t>(kd);
-  uint8_t* o_oocc = c.take<uint8_t>(k);
-  uint32_t* o_owav = c.take<uint32_t>(k);
-  int16_t* dr = c.take<int16_t>(kd);
-  uint8_t* o_st = c.take<uint8_t>(kd);
-  int32_t* o_lim = reinterpret_cast<int32_t*>(c.take<uint8_t>(lim_bytes));
-  cudaStream_t s = arena->stream;
-  const cudaMemcpyKind h2d = cudaMemcpyHostToDevice, d2h = cudaMemcpyDeviceToHost;
-  HB_CUDA_TRY(cudaMemcpyAsync(nb, kernels->num_blocks, k * 4, h2d, s));
-  HB_CUDA_TRY(cudaMemcpyAsync(bs, kernels->block_size, k * 2, h2d, s));
-  HB_CUDA_TRY(cudaMemcpyAsync(rg, kernels->regs_per_thread, k * 2, h2d, s));
-  HB_CUDA_TRY(cudaMemcpyAsync(sm, kernels->smem_bytes, k * 4, h2d, s));
-  HB_CUDA_TRY(cudaMemcpyAsync(tm, kernels->run_time_ns, k * 4, h2d, s));
-  HB_CUDA_TRY(cudaMemcpyAsync(gm, kernels->gamma, k * 4, h2d, s));
-  if (dest_regs) HB_CUDA_TRY(cudaMemcpyAsync(dr, dest_regs, kd * 2, h2d, s));
-  hb_kernel_soa dk{nb, bs, rg, sm, tm, gm};
-  hb_wave_out dout{o_ns, o_occ, o_wav, o_oocc, o_owav, out->status ? o_st : nullptr,
-                   out->limits ? o_lim : nullptr};
-  st = launch<false>(make_ptrs(&dk, nullptr, dest_regs ? dr : nullptr, &dout), *plan, K, s);
-  if (st != HB_OK) return st;
-  HB_CUDA_TRY(cudaMemcpyAsync(out->scaled_ns, o_ns, kd * 4, d2h, s));
-  HB_CUDA_TRY(cudaMemcpyAsync(out->dest_occupancy, o_occ, kd, d2h, s));
-  HB_CUDA_TRY(cudaMemcpyAsync(out->dest_waves, o_wav, kd * 4, d2h, s));
-  HB_CUDA_TRY(cudaMemcpyAsync(out->origin_occupancy, o_oocc, k, d2h, s));
-  HB_CUDA_TRY(cudaMemcpyAsync(out->origin_waves, o_owav, k * 4, d2h, s));
-  if (out->status) HB_CUDA_TRY(cudaMemcpyAsync(out->status, o_st, kd, d2h, s));
-  if (out->limits) HB_CUDA_TRY(cudaMemcpyAsync(out->limits, o_lim, lim_bytes, d2h, s));
-  HB_CUDA_TRY(cudaStreamSynchronize(s));
-  return HB_OK;
+  const HostPlanes io(kernels, dest_regs, out, K, D);
+  const LaunchPlan mine = *plan;   // other threads' calls replace theirs, not ours; the helpers have none
+  cudaStream_t s;
+  // per-destination registers keep rows of their own, block limits are written by the generic kernel alone
+  if (!dest_regs && !out->limits && io.in_bytes(K) <= kHostDirectBytes && io.results_page_locked()) {
+    // eight chunks or more of 8,192 records: 10 us of staging each
+    int64_t chunk = (K / 8 + 255) & ~int64_t{255};
+    if (chunk < 8192) chunk = 8192;
+    st = hb::arena_stream(arena, 1, &s);
+    return st == HB_OK ? host_direct(arena, io, mine, K, chunk) : st;
+  }
+  // Chunks of 0.5 to 2 MB of records and results, sixteen if the batch is large enough, and no thread for less
+  // than two chunks (starting one costs about 40 us).  1,048,576 kernels x 6: 3.3 ms into memory in use, 5.4 ms
+  // into fresh pages, against 4.1 and 15.8 ms with pageable copies; 65,536: 0.31 against 0.42 ms.
+  const size_t per_record = io.in_bytes(4096) / 4096 + io.out_bytes(4096) / 4096 + 1;
+  const int64_t least = static_cast<int64_t>((512u << 10) / per_record), most = 4 * least;
+  int64_t chunk = K / 16 < least ? least : (K / 16 > most ? most : K / 16);
+  chunk = (chunk + 255) & ~int64_t{255};
+  if (chunk > K) chunk = K;
+  int64_t threads = (K + 2 * chunk - 1) / (2 * chunk);
+  if (threads > kHostThreads) threads = kHostThreads;
+  for (int w = 0; w < threads; ++w) {
+    st = hb::arena_stream(arena, w, &s);
+    if (st != HB_OK) return st;
+  }
+  return host_in_threads(arena, io, mine, K, chunk, static_cast<int>(threads), device);
 }
 
 // The occupancy rules are plain integer code that also compiles for the host

@@ -18,7 +18,7 @@ from typing import Sequence
 import numpy as np
 import torch
 
-from habitat_b200 import batched
+from habitat_b200 import _native, batched
 
 # field order inside a record block: the 4-byte fields first, so that every field starts on an
 # 8-byte boundary whenever K is even
@@ -98,6 +98,13 @@ class _Streams:
         self.computed = [torch.cuda.Event() for _ in range(depth)]
         self.downloaded = [torch.cuda.Event() for _ in range(depth)]
         self.used = [False] * depth
+        # an event gets its native handle when it is first recorded
+        for events, stream in ((self.uploaded, self.s_up), (self.computed, self.s_in), (self.downloaded, self.s_out)):
+            for e in events:
+                e.record(stream)
+        self._stream_handles = tuple(s.cuda_stream for s in (self.s_up, self.s_in, self.s_out))
+        self._event_handles = [tuple(e.cuda_event for e in slot)
+                               for slot in zip(self.uploaded, self.computed, self.downloaded)]
 
     def wait(self, slot):
         """Blocks the host until the results of `slot` are in its pinned buffers."""
@@ -144,35 +151,21 @@ class WaveScaleHost(_Streams):
             if self.want_totals:
                 for h in self.host_out:
                     h["totals"] = torch.zeros((D,), dtype=torch.float64).pin_memory()
+        self._downloads = [[(t, self.dev_totals[i] if k == "totals" else getattr(self.dev_out[i], k))
+                            for k, t in h.items()] for i, h in enumerate(self.host_out)]
         self.h2d_bytes = K * RECORD_BYTES
         self.d2h_bytes = sum(t.numel() * t.element_size() for t in self.host_out[0].values())
 
     def submit(self, block: torch.Tensor, slot: int):
         if block.numel() != self.K * RECORD_BYTES or block.dtype != torch.uint8:
             raise ValueError("block must be a uint8 tensor of K * %d bytes (pack_kernels)" % RECORD_BYTES)
-        with torch.cuda.stream(self.s_up):
-            # the slot's device inputs were last read by the kernel of batch (i - depth)
-            if self.used[slot]:
-                self.s_up.wait_event(self.computed[slot])
-            self.dev_block[slot].copy_(block, non_blocking=True)
-            self.uploaded[slot].record(self.s_up)
-        with torch.cuda.stream(self.s_in):
-            self.s_in.wait_event(self.uploaded[slot])
-            # the kernel of this batch overwrites outputs the download of batch (i - depth) reads
-            if self.used[slot]:
-                self.s_in.wait_event(self.downloaded[slot])
-            if self.want_totals:
-                batched.wave_scale(self.dev_in[slot], self.origin, self.dests, out=self.dev_out[slot],
-                                   partials=self.partials[slot])
-                self.partials[slot].totals(out=self.dev_totals[slot])
-            else:
-                batched.wave_scale(self.dev_in[slot], self.origin, self.dests, out=self.dev_out[slot])
-            self.computed[slot].record(self.s_in)
-        with torch.cuda.stream(self.s_out):
-            self.s_out.wait_event(self.computed[slot])
-            for k, t in self.host_out[slot].items():
-                t.copy_(self.dev_totals[slot] if k == "totals" else getattr(self.dev_out[slot], k), non_blocking=True)
-            self.downloaded[slot].record(self.s_out)
+        with_totals = self.want_totals
+        res = _native.binding().submit_wave(
+            block.contiguous(), self.dev_block[slot], self.dev_in[slot], self.origin, self.dests, self.dev_out[slot],
+            self.partials[slot] if with_totals else None, self.dev_totals[slot] if with_totals else None,
+            self._downloads[slot], self._stream_handles, self._event_handles[slot], self.used[slot])
+        if res is None:
+            raise ValueError("wave_scale: unsupported arguments (at most %d destinations)" % _native.HB_MAX_DEVICES)
         self.used[slot] = True
 
 

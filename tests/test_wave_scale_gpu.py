@@ -385,3 +385,32 @@ def test_second_gpu_gets_its_own_tables(bench_devices):
                                      bench_devices[0], bench_devices)
             tot = batched.plane_sum(res.scaled_ns).cpu().numpy()
             assert np.allclose(tot, np.nansum(to_numpy(res.scaled_ns).astype(np.float64), axis=1), rtol=1e-12)
+
+
+@pytest.mark.parametrize("K", [1, 8192, 8193, 65536, 65537, 150_001])
+@pytest.mark.parametrize("page_locked", [True, False])
+def test_host_entry_in_chunks(bench_devices, K, page_locked, monkeypatch):
+    """The host-buffer entry point stages records in chunks of 8,192 or more and lets the kernel write
+    page-locked results itself (odd counts: planes off the 8-byte boundary, one record per thread), or, into
+    ordinary memory, goes through up to four threads.  Every plane equals the device entry point's to the bit,
+    also the second time (reused blocks), and an earlier result stays as it was."""
+    from habitat_b200 import _native
+    if not page_locked:
+        real = _native.binding()
+
+        class NoBlocks:
+            def __getattr__(self, name):
+                return (lambda n: None) if name == "host_block" else getattr(real, name)
+        monkeypatch.setattr(_native, "binding", lambda: NoBlocks())
+    kernels = workloads.make_kernels(K, seed=K)
+    kernels["run_time_ns"] = kernels["run_time_ns"].astype(np.float32)
+    want = batched.wave_scale(batched.KernelBatch.from_numpy(kernels), bench_devices[0], bench_devices, want_status=True)
+    names = ("scaled_ns", "dest_occupancy", "dest_waves", "origin_occupancy", "origin_waves", "status")
+    want = {n: to_numpy(getattr(want, n)) for n in names}
+    first = batched.wave_scale_host(kernels, bench_devices[0], bench_devices, want_status=True)
+    other = batched.wave_scale_host({n: v[::-1].copy() for n, v in kernels.items()}, bench_devices[0], bench_devices)
+    for n in names:
+        assert np.array_equal(first[n].view(np.uint8), want[n].view(np.uint8)), n
+        if n != "status":
+            assert np.array_equal(other[n][..., ::-1].copy().view(np.uint8), want[n].view(np.uint8)), n
+    assert other["status"] is None and first["limits"] is None
