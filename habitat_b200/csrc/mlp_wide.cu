@@ -714,8 +714,8 @@ namespace hb {
 // (L2 and shared-memory fill bound), wider ones exchange more per layer (L2 latency and bandwidth); the
 // shapes below are those that no other one beats at its capacity.  Measured per launch, conv2d predictor,
 // 8 hidden layers (capacity in queries: time), against 125 us (bf16) and 190 us (split) before:
-//   bf16   112: 29 us   240: 31   480: 37   960: 52   1,056: 54   2,112: 80
-//   split   56: 37       120: 44   240: 52             528: 82     1,056: 138
+//   bf16   112: 25 us   240: 29   480: 32   960: 48   1,056: 48   2,112: 75
+//   split   56: 34       120: 42   240: 46             528: 77     1,056: 128
 // Eight blocks x 64 columns lose to four x 32 in split precision (86 us for 480).  Beyond the last shape
 // the two-SM kernel of mlp_chain.cu is the faster one.
 WidePlan wide_plan(int64_t Q, bool split, int sm_count) {

@@ -13,6 +13,7 @@
 // per-launch (origin, destination) log2 ratios travel as a kernel parameter.
 // The kernel is HBM-bound by design: 20 B read + 5 B written per kernel and
 // 9 B written per pair.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
@@ -365,27 +366,31 @@ bool vec4_ok(const Ptrs& p, int64_t K, bool need_gamma) {
 //   * A = log2(occ) - log2(clock MHz) as float hi + lo: the exponent of the
 //     small-kernel rule (roofline.py:32-45) is (1 - gamma) (A_dest[blocks per SM
 //     on the destination] - A_origin[blocks per SM on the origin]).
-// Rows that agree on everything P (or S) reads form a class; a launch carries at
-// most four classes of each, a record loads one byte per class, and a
-// destination picks its two bytes with a byte permute and takes one 16-bit-pair
-// minimum for the two records a thread owns.  The tables a launch touches
-// (a few KB) stay in L1.  The extended variant (EXT) reads every device's own P and S
+// Rows that agree on everything P (or S) reads form a class.  The tables of four classes lie interleaved in one
+// table of words, so a record's bytes for up to four classes are one load (eight: two), and a destination picks
+// its two bytes with a byte permute and takes one 16-bit-pair minimum for the two records a thread owns.  The
+// tables a launch touches (a few KB) stay in L1.  The extended variant (EXT) reads every device's own P and S
 // bytes per pair instead (no class limit) and adds, under launch-uniform branches,
 // the status plane, per-destination register counts and gamma from raw metrics
 // (one float64 intensity per record, a compare and a multiply-add per pair); it
-// also serves launches with more than four classes.  The grid is persistent:
-// blocks stride over the batch.
+// also serves launches with more than eight classes.
 // Conditions (checked on the host, else wave_scale_fast_kernel or the generic
 // kernel runs): D <= 32, D K < 2^31, and per row 2 <= SMs <= 4096,
 // blocks-per-SM limit <= 32, thread limit per block a multiple of 32 and <= 1024,
 // shared-memory reserve a multiple of 128, shared-memory cap below the table's
 // last step.
 // ---------------------------------------------------------------------------
-constexpr int kMaxClasses = 4;   // table sizes, LutOcc and the table builder: occupancy.cuh
+constexpr int kMaxWords = 2;     // class words per launch; table sizes, LutOcc and the table builder: occupancy.cuh
 
 __device__ uint8_t g_lut_p[HB_MAX_DEVICES * kLutP];
 __device__ uint8_t g_lut_s[HB_MAX_DEVICES * kLutS];
-__device__ LutOcc g_lut_t[HB_MAX_DEVICES * kLutOcc];
+// The P (and S) tables of four classes in one word per index: one load brings a record's bytes of all four.
+// Class c of the device table (classes are numbered as their first rows come) is byte c % 4 of word c / 4.
+constexpr int kWords = HB_MAX_DEVICES / 4;
+__device__ uint32_t g_lut_pw[kWords * kLutP];
+__device__ uint32_t g_lut_sw[kWords * kLutS];
+__device__ uint2 g_lut_m[HB_MAX_DEVICES * kLutOcc];    // {M, sh}
+__device__ float2 g_lut_a[HB_MAX_DEVICES * kLutOcc];   // {A_hi, A_lo}
 
 struct alignas(16) LutDev {       // three 16-byte groups, each fetched with one constant load
   uint32_t sel_p, sel_s;          // permute selectors: class byte of record 0 -> low half, record 1 -> high half
@@ -394,7 +399,7 @@ struct alignas(16) LutDev {       // three 16-byte groups, each fetched with one
   float a_hi, a_lo, b_hi, b_lo;   // large-kernel exponent gamma a + b, split float64 constants
   uint32_t sms_m1, sms_magic;     // SMs - 1 and floor(2^32 / SMs) + 1, for ceil(blocks / SMs)
   uint32_t s_off;                 // byte offset of the row's own S table (extended variant)
-  uint32_t pad;
+  uint32_t words;                 // bit 0 (1): the row's P (S) class is in the launch's second word
 };
 struct LutDevRegs {               // LutDev as read by a thread
   uint4 sel;
@@ -413,7 +418,7 @@ struct LutParams {
   uint32_t K;
   uint32_t stride;                                   // elements from one output plane to the next
   int32_t D;
-  uint32_t off_p[kMaxClasses], off_s[kMaxClasses];   // byte offsets of the class tables
+  uint32_t off_p[kMaxWords], off_s[kMaxWords];       // offsets of the class words' tables, in words
   double origin_peak;                                // metrics mode: origin peak GFLOP/s
   LutDev origin;
   LutDev dest[HB_MAX_DEVICES / 2];
@@ -496,7 +501,7 @@ __device__ __forceinline__ void store_byte_pair(uint8_t* q, uint32_t pair_word, 
 // D <= kTotMaxD.
 constexpr int kTotMaxD = kLutThreads / 16;
 
-template <int VEC, bool EXT, bool ALIGNED, int NP, int NS, bool TOT = false>
+template <int VEC, bool EXT, bool ALIGNED, int NW, bool TOT = false>
 __global__ void __launch_bounds__(kLutThreads, EXT ? 8 : 12)
 wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
   static_assert(!TOT || (VEC == 2 && ALIGNED && !EXT), "fused totals: aligned two-record variant only");
@@ -504,16 +509,17 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
   hb_grid_dependency_wait();
   const uint32_t K = lp.K;
   const int D = lp.D;
-  if (TOT && (blockIdx.x * kLutThreads + threadIdx.x) * VEC >= K) {
+  const uint32_t k0 = (blockIdx.x * kLutThreads + threadIdx.x) * VEC;
+  if (TOT && k0 >= K) {
     for (int d = 0; d < D; ++d) s_tot[d][threadIdx.x] = 0.0;   // threads past the end
   }
-  const uint8_t* __restrict__ tab_t = reinterpret_cast<const uint8_t*>(g_lut_t);
-  const uint32_t stride = gridDim.x * (kLutThreads * VEC);
+  const uint8_t* __restrict__ tab_m = reinterpret_cast<const uint8_t*>(g_lut_m);
+  const uint8_t* __restrict__ tab_a = reinterpret_cast<const uint8_t*>(g_lut_a);
   const bool with_regs = EXT && p.dest_regs != nullptr;
   const bool with_metrics = EXT && p.has_metrics != nullptr;
   const bool with_status = EXT && p.status != nullptr;
 
-  for (uint32_t k0 = (blockIdx.x * kLutThreads + threadIdx.x) * VEC; k0 < K; k0 += stride) {
+  if (k0 < K) {
     const bool pair = VEC == 2 && (ALIGNED || k0 + 1 < K);   // false: the last record of an odd batch
     const Vec<int32_t, VEC> nbv = load_pair<int32_t, VEC, ALIGNED>(p.num_blocks + k0, pair);
     const Vec<uint16_t, VEC> bsv = load_pair<uint16_t, VEC, ALIGNED>(p.block_size + k0, pair);
@@ -523,7 +529,14 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
     Vec<float, VEC> gv;
     if (!with_metrics) gv = load_pair<float, VEC, ALIGNED>(p.gamma + k0, pair);
 
-    uint32_t P[2] = {0u, 0u}, S[2] = {0u, 0u};   // class bytes of the two records
+    uint32_t P[2] = {0u, 0u}, S[2] = {0u, 0u};     // class bytes of the two records
+    uint32_t P2[2] = {0u, 0u}, S2[2] = {0u, 0u};   // ... of the launch's second word
+    // occupancies of the two records on a device, in the halves of a word
+    auto occ_pair = [&](const LutDevRegs& r) {
+      const bool p2 = NW == 2 && (r.sm.w & 1u), s2 = NW == 2 && (r.sm.w & 2u);
+      return __vimin_s16x2_relu(prmt(p2 ? P2[0] : P[0], p2 ? P2[1] : P[1], r.sel.x),
+                                prmt(s2 ? S2[0] : S[0], s2 ? S2[1] : S[1], r.sel.y));
+    };
     uint32_t wrow[2] = {0u, 0u};                 // EXT: warps per block x row length (P index base)
     float omg[2] = {0.0f, 0.0f};
     double xint[2] = {-1.0, -1.0}, xinv[2] = {0.0, 0.0};   // EXT: intensity (< 0: special case) and 1 / intensity
@@ -533,12 +546,12 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
       const uint32_t pidx = HB_IDX(lut_p_index(bsv.v[i], rgv.v[i]), kLutP, 1);
       const uint32_t steps = HB_IDX(lut_s_index(smv.v[i]), kLutS, 2);
       if (!EXT) {
-        uint32_t pw = 0, sw = 0;
-#pragma unroll
-        for (int c = 0; c < NP; ++c) pw |= static_cast<uint32_t>(__ldg(g_lut_p + (lp.off_p[c] + pidx))) << (8 * c);
-#pragma unroll
-        for (int c = 0; c < NS; ++c) sw |= static_cast<uint32_t>(__ldg(g_lut_s + (lp.off_s[c] + steps))) << (8 * c);
-        P[i] = pw; S[i] = sw;
+        P[i] = __ldg(g_lut_pw + (lp.off_p[0] + pidx));
+        S[i] = __ldg(g_lut_sw + (lp.off_s[0] + steps));
+        if (NW == 2) {
+          P2[i] = __ldg(g_lut_pw + (lp.off_p[1] + pidx));
+          S2[i] = __ldg(g_lut_sw + (lp.off_s[1] + steps));
+        }
       } else {
         // extended variant: every device's own tables are indexed directly (no class limit)
         P[i] = pidx; S[i] = steps;
@@ -566,7 +579,7 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
     const LutDevRegs og = load_lut_dev(lp.origin);
     uint32_t o2;
     if (!EXT) {
-      o2 = __vimin_s16x2_relu(prmt(P[0], P[1], og.sel.x), prmt(S[0], S[1], og.sel.y));
+      o2 = occ_pair(og);
     } else {
       o2 = 0;
 #pragma unroll
@@ -583,7 +596,7 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
     for (int i = 0; i < VEC; ++i) {
       const uint32_t occ = i == 0 ? (o2 & 0xFFFFu) : (o2 >> 16);
       const int32_t nb = nbv.v[i];
-      const uint2 w = __ldg(reinterpret_cast<const uint2*>(tab_t + (og.sel.z + HB_IDX(occ, kLutOcc, 3) * 16u)));
+      const uint2 w = __ldg(reinterpret_cast<const uint2*>(tab_m + (og.sel.z + HB_IDX(occ, kLutOcc, 3) * 8u)));
       const uint32_t q = __umulhi(static_cast<uint32_t>(nb), w.x) >> w.y;
       nbok[i] = nb >= 1;
       live[i] = nbok[i] && occ != 0u;
@@ -593,7 +606,7 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
       // the entry read here is never used, and the clamp only keeps the index inside the table.  Not
       // selecting on fits_o keeps this load independent of the one above.
       const uint32_t om = min(__umulhi(static_cast<uint32_t>(nb) + og.sm.x, og.sm.y), static_cast<uint32_t>(kLutOcc - 1));
-      lg_o[i] = __ldg(reinterpret_cast<const float2*>(tab_t + (og.sel.z + HB_IDX(om, kLutOcc, 4) * 16u + 8u)));
+      lg_o[i] = __ldg(reinterpret_cast<const float2*>(tab_a + (og.sel.z + HB_IDX(om, kLutOcc, 4) * 8u)));
     }
     store_byte_pair<VEC, ALIGNED>(p.origin_occ + k0, o2, pair);
     store_pair<uint32_t, VEC, ALIGNED>(p.origin_waves + k0, owav, pair);
@@ -604,7 +617,7 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
       const uint32_t base = static_cast<uint32_t>(d) * lp.stride + k0;   // D K < 2^31
       uint32_t occ2;
       if (!EXT) {
-        occ2 = __vimin_s16x2_relu(prmt(P[0], P[1], dd.sel.x), prmt(S[0], S[1], dd.sel.y));
+        occ2 = occ_pair(dd);
       } else {
         Vec<int16_t, VEC> drv;
         if (with_regs) {
@@ -636,7 +649,7 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
       for (int i = 0; i < VEC; ++i) {
         const uint32_t occ = i == 0 ? (occ2 & 0xFFFFu) : (occ2 >> 16);
         const int32_t nb = nbv.v[i];
-        const uint2 w = __ldg(reinterpret_cast<const uint2*>(tab_t + (dd.sel.z + HB_IDX(occ, kLutOcc, 6) * 16u)));
+        const uint2 w = __ldg(reinterpret_cast<const uint2*>(tab_m + (dd.sel.z + HB_IDX(occ, kLutOcc, 6) * 8u)));
         const uint32_t q = __umulhi(static_cast<uint32_t>(nb), w.x) >> w.y;
         const bool has_wave = occ != 0u;
         wavv.v[i] = (nbok[i] && has_wave) ? q : 0xFFFFFFFFu;
@@ -647,7 +660,7 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
         // blocks per SM on the destination: meaningful (and <= occupancy) when `small`; computed from
         // the record alone so that this table load does not wait for the one above
         const uint32_t dm = min(__umulhi(static_cast<uint32_t>(nb) + dd.sm.x, dd.sm.y), static_cast<uint32_t>(kLutOcc - 1));
-        const float2 lg_d = __ldg(reinterpret_cast<const float2*>(tab_t + (dd.sel.z + HB_IDX(dm, kLutOcc, 7) * 16u + 8u)));
+        const float2 lg_d = __ldg(reinterpret_cast<const float2*>(tab_a + (dd.sel.z + HB_IDX(dm, kLutOcc, 7) * 8u)));
         float gamma, one_minus;
         if (with_metrics) {
           const double x = xint[i];
@@ -717,6 +730,12 @@ struct HostTable {
   std::vector<uint8_t> lut_p = std::vector<uint8_t>(static_cast<size_t>(HB_MAX_DEVICES) * kLutP);
   std::vector<uint8_t> lut_s = std::vector<uint8_t>(static_cast<size_t>(HB_MAX_DEVICES) * kLutS);
   std::vector<LutOcc> lut_t = std::vector<LutOcc>(static_cast<size_t>(HB_MAX_DEVICES) * kLutOcc);
+  // classes of rows that agree on everything P (S) reads, and their tables four to a word
+  FastDev fast[HB_MAX_DEVICES];
+  std::vector<FastDev> p_reps, s_reps;
+  int p_class[HB_MAX_DEVICES] = {}, s_class[HB_MAX_DEVICES] = {};
+  std::vector<uint32_t> words_p = std::vector<uint32_t>(static_cast<size_t>(kWords) * kLutP);
+  std::vector<uint32_t> words_s = std::vector<uint32_t>(static_cast<size_t>(kWords) * kLutS);
 };
 struct GpuCopy {
   std::atomic<bool> constants{false};          // row-independent tables uploaded (read without the lock)
@@ -767,10 +786,22 @@ hb_status sync_gpu(int* sm_count) {
                                    static_cast<size_t>(i) * kLutP));
     HB_CUDA_TRY(cudaMemcpyToSymbol(g_lut_s, &g_tab.lut_s[static_cast<size_t>(i) * kLutS], kLutS,
                                    static_cast<size_t>(i) * kLutS));
-    HB_CUDA_TRY(cudaMemcpyToSymbol(g_lut_t, &g_tab.lut_t[static_cast<size_t>(i) * kLutOcc],
-                                   sizeof(LutOcc) * kLutOcc, sizeof(LutOcc) * kLutOcc * i));
+    uint2 m[kLutOcc];
+    float2 a[kLutOcc];
+    for (int occ = 0; occ < kLutOcc; ++occ) {
+      const LutOcc& e = g_tab.lut_t[static_cast<size_t>(i) * kLutOcc + occ];
+      m[occ] = make_uint2(e.magic, e.shift);
+      a[occ] = make_float2(e.lg_hi, e.lg_lo);
+    }
+    HB_CUDA_TRY(cudaMemcpyToSymbol(g_lut_m, m, sizeof(m), sizeof(m) * i));
+    HB_CUDA_TRY(cudaMemcpyToSymbol(g_lut_a, a, sizeof(a), sizeof(a) * i));
     gc.row_version[i] = g_tab.row_version[i];
     uploaded = true;
+  }
+  if (uploaded) {
+    const size_t p_words = (g_tab.p_reps.size() + 3) / 4, s_words = (g_tab.s_reps.size() + 3) / 4;
+    if (p_words) HB_CUDA_TRY(cudaMemcpyToSymbol(g_lut_pw, g_tab.words_p.data(), sizeof(uint32_t) * kLutP * p_words));
+    if (s_words) HB_CUDA_TRY(cudaMemcpyToSymbol(g_lut_sw, g_tab.words_s.data(), sizeof(uint32_t) * kLutS * s_words));
   }
   if (uploaded) HB_CUDA_TRY(cudaDeviceSynchronize());
   g_gpu_version[dev].store(g_version.load(std::memory_order_acquire), std::memory_order_release);
@@ -787,39 +818,27 @@ bool same_p_class(const FastDev& a, const FastDev& b) {
   return same_regs_class(a, b) && same_warps_class(a, b) && a.blocks_limit == b.blocks_limit;
 }
 
-// Class (index into `rows`, which lists the first row of each class) of `row`; -1 when full.
+// The class of row `row` among `reps` (made now if it is new, its table put into the words); -1 when all
+// numbers are taken.  A class keeps its number and its bytes for good, so a launch that was planned with an older
+// table still finds them.  Call with g_mu held.
 template <typename Same>
-int class_of(int* rows, int* n, int row, Same same) {
-  for (int c = 0; c < *n; ++c)
-    if (same(fold_fast(g_tab.rows[rows[c]], g_tab.pre[rows[c]]), fold_fast(g_tab.rows[row], g_tab.pre[row]))) return c;
-  if (*n >= kMaxClasses) return -1;
-  rows[*n] = row;
-  return (*n)++;
+int class_of(std::vector<FastDev>& reps, std::vector<uint32_t>& words, const std::vector<uint8_t>& rows, int len, int row,
+             Same same) {
+  const FastDev& f = g_tab.fast[row];
+  for (size_t c = 0; c < reps.size(); ++c)
+    if (same(reps[c], f)) return static_cast<int>(c);
+  if (reps.size() == HB_MAX_DEVICES) return -1;
+  const size_t c = reps.size();
+  reps.push_back(f);
+  for (int i = 0; i < len; ++i)
+    words[c / 4 * len + i] |= static_cast<uint32_t>(rows[static_cast<size_t>(row) * len + i]) << (8 * (c % 4));
+  return static_cast<int>(c);
 }
 
-template <int VEC, bool EXT, bool ALIGNED, int NP, int NS, bool TOT = false>
+template <int VEC, bool EXT, bool ALIGNED, int NW, bool TOT = false>
 cudaError_t launch_lut(unsigned grid, cudaStream_t stream, const Ptrs& p, const LutParams& q) {
-  return hb::launch_overlapped(wave_scale_lut_kernel<VEC, EXT, ALIGNED, NP, NS, TOT>, dim3(grid), dim3(kLutThreads),
+  return hb::launch_overlapped(wave_scale_lut_kernel<VEC, EXT, ALIGNED, NW, TOT>, dim3(grid), dim3(kLutThreads),
                                0, stream, p, q);
-}
-
-template <int NP, bool TOT>
-cudaError_t launch_lut_plain(int ns, unsigned grid, cudaStream_t stream, const Ptrs& p, const LutParams& q) {
-  switch (ns) {
-    case 1: return launch_lut<2, false, true, NP, 1, TOT>(grid, stream, p, q);
-    case 2: return launch_lut<2, false, true, NP, 2, TOT>(grid, stream, p, q);
-    case 3: return launch_lut<2, false, true, NP, 3, TOT>(grid, stream, p, q);
-    default: return launch_lut<2, false, true, NP, 4, TOT>(grid, stream, p, q);
-  }
-}
-template <bool TOT>
-cudaError_t launch_lut_plain(int np, int ns, unsigned grid, cudaStream_t stream, const Ptrs& p, const LutParams& q) {
-  switch (np) {
-    case 1: return launch_lut_plain<1, TOT>(ns, grid, stream, p, q);
-    case 2: return launch_lut_plain<2, TOT>(ns, grid, stream, p, q);
-    case 3: return launch_lut_plain<3, TOT>(ns, grid, stream, p, q);
-    default: return launch_lut_plain<4, TOT>(ns, grid, stream, p, q);
-  }
 }
 
 // Everything about a launch that depends on the devices alone.  Callers ask for the same origin and
@@ -829,28 +848,32 @@ struct LaunchPlan {
   uint64_t version = 0;
   LaunchParams lp{};
   bool lut_ok = false;         // every row can be tabulated
-  bool many_classes = false;   // more than four classes: every row's own tables (extended variant)
-  int n_p = 0, n_s = 0;
+  int words = 1;               // class words the rows need; more than kMaxWords: every row's own tables (extended variant)
   LutParams q{};
 };
 
 void fill_lut(LaunchPlan* plan) {   // call with g_mu held
   const LaunchParams& lp = plan->lp;
   LutParams& q = plan->q;
-  int rows_p[kMaxClasses] = {}, rows_s[kMaxClasses] = {};
   plan->lut_ok = lp.D <= HB_MAX_DEVICES / 2 && g_tab.lut_ok[lp.origin_row];
   for (int d = 0; d < lp.D && plan->lut_ok; ++d) plan->lut_ok = g_tab.lut_ok[lp.dest_row[d]];
   if (!plan->lut_ok) return;
-  bool many_classes = false;
+  int words_p[HB_MAX_DEVICES], words_s[HB_MAX_DEVICES], n_p = 0, n_s = 0;
+  auto slot_of = [](int* words, int* n, int word) {
+    for (int i = 0; i < *n; ++i)
+      if (words[i] == word) return i;
+    words[*n] = word;
+    return (*n)++;
+  };
   for (int d = -1; d < lp.D; ++d) {
     const int row = d < 0 ? lp.origin_row : lp.dest_row[d];
-    const int pc = many_classes ? -1 : class_of(rows_p, &plan->n_p, row, same_p_class);
-    const int sc = many_classes ? -1 : class_of(rows_s, &plan->n_s, row, same_smem_class);
-    if (pc < 0 || sc < 0) many_classes = true;
+    const int pc = g_tab.p_class[row], sc = g_tab.s_class[row];
+    if (pc < 0 || sc < 0) plan->words = kMaxWords + 1;
     LutDev& o = d < 0 ? q.origin : q.dest[d];
-    o.sel_p = pair_selector(pc < 0 ? 0 : pc);
-    o.sel_s = pair_selector(sc < 0 ? 0 : sc);
-    o.t_off = static_cast<uint32_t>(row * kLutOcc * sizeof(LutOcc));
+    o.sel_p = pair_selector(pc & 3);
+    o.sel_s = pair_selector(sc & 3);
+    o.words = static_cast<uint32_t>((slot_of(words_p, &n_p, pc >> 2) & 1) | (slot_of(words_s, &n_s, sc >> 2) & 1) << 1);
+    o.t_off = static_cast<uint32_t>(row * kLutOcc * sizeof(uint2));
     o.p_off = static_cast<uint32_t>(row * kLutP);
     o.s_off = static_cast<uint32_t>(row * kLutS);
     o.sms_m1 = static_cast<uint32_t>(g_tab.rows[row].num_sms - 1);
@@ -864,12 +887,10 @@ void fill_lut(LaunchPlan* plan) {   // call with g_mu held
       q.slope[d] = -0.5 / lp.ridge[d];
     }
   }
-  plan->many_classes = many_classes;
-  // class slots beyond the count repeat class 0 (the kernel variants are built for 1..4 classes,
-  // the extended one always loads four)
-  for (int c = 0; c < kMaxClasses; ++c) {
-    q.off_p[c] = static_cast<uint32_t>(rows_p[c < plan->n_p ? c : 0] * kLutP);   // unused by the extended variant
-    q.off_s[c] = static_cast<uint32_t>(rows_s[c < plan->n_s ? c : 0] * kLutS);
+  plan->words = std::max({plan->words, n_p, n_s});
+  for (int w = 0; w < kMaxWords; ++w) {   // a word that is not needed repeats the first
+    q.off_p[w] = static_cast<uint32_t>(std::max(words_p[w < n_p ? w : 0], 0) * kLutP);
+    q.off_s[w] = static_cast<uint32_t>(std::max(words_s[w < n_s ? w : 0], 0) * kLutS);
   }
   q.D = lp.D;
   q.origin_peak = lp.origin_peak;
@@ -888,12 +909,10 @@ bool try_launch_lut(const Ptrs& p, const LaunchPlan& plan, int64_t K, int64_t st
   LutParams q = plan.q;
   q.K = static_cast<uint32_t>(K);
   q.stride = static_cast<uint32_t>(stride);
-  const int n_p = plan.n_p, n_s = plan.n_s;
-  const bool many_classes = plan.many_classes;
 
   auto al = [](const void* ptr, uintptr_t a) { return (reinterpret_cast<uintptr_t>(ptr) & (a - 1)) == 0; };
   const bool metrics = p.has_metrics != nullptr;
-  const bool ext = metrics || p.dest_regs != nullptr || p.status != nullptr || many_classes;
+  const bool ext = metrics || p.dest_regs != nullptr || p.status != nullptr || plan.words > kMaxWords;
   // two records per thread when the inputs sit on 8-byte boundaries; 8-byte stores when the
   // output planes do too (K even)
   const bool vec2 = al(p.num_blocks, 8) && al(p.smem, 8) && al(p.time_ns, 8) && (metrics || al(p.gamma, 8)) &&
@@ -905,27 +924,25 @@ bool try_launch_lut(const Ptrs& p, const LaunchPlan& plan, int64_t K, int64_t st
                        (!p.dest_regs || al(p.dest_regs, 4));
   const int vec = vec2 ? 2 : 1;
   const int64_t blocks = ((K + vec - 1) / vec + kLutThreads - 1) / kLutThreads;
-  // One block per 128 threads' worth of records measured fastest at every batch size (the block
-  // scheduler balances the tail); HB_LUT_BLOCKS_PER_SM = n caps the grid at n blocks per SM, which
-  // then stride over the batch.
-  static const int per_sm = [] { const char* e = std::getenv("HB_LUT_BLOCKS_PER_SM"); return e ? std::atoi(e) : 0; }();
-  const int64_t cap = per_sm > 0 ? static_cast<int64_t>(sm_count) * per_sm : blocks;
-  const unsigned grid = static_cast<unsigned>(blocks < cap ? blocks : cap);
+  // One block per 128 threads' worth of records measured fastest at every batch size: the block scheduler
+  // balances the tail (persistent blocks that stride over the batch were slower throughout).
+  const unsigned grid = static_cast<unsigned>(blocks);
+  const bool two = plan.words == 2;
   cudaError_t le;
   if (ext) {
-    le = !vec2 ? launch_lut<1, true, true, 1, 1>(grid, stream, p, q)
-               : (aligned ? launch_lut<2, true, true, 1, 1>(grid, stream, p, q)
-                          : launch_lut<2, true, false, 1, 1>(grid, stream, p, q));
+    le = !vec2 ? launch_lut<1, true, true, 1>(grid, stream, p, q)
+               : (aligned ? launch_lut<2, true, true, 1>(grid, stream, p, q)
+                          : launch_lut<2, true, false, 1>(grid, stream, p, q));
   } else if (!vec2) {
-    le = launch_lut<1, false, true, 4, 4>(grid, stream, p, q);
+    le = launch_lut<1, false, true, 2>(grid, stream, p, q);
   } else if (!aligned) {
-    le = launch_lut<2, false, false, 4, 4>(grid, stream, p, q);
-  } else if (p.block_sums && lp.D <= kTotMaxD && grid == blocks) {
-    le = launch_lut_plain<true>(n_p, n_s, grid, stream, p, q);
+    le = two ? launch_lut<2, false, false, 2>(grid, stream, p, q) : launch_lut<2, false, false, 1>(grid, stream, p, q);
+  } else if (p.block_sums && lp.D <= kTotMaxD) {
+    le = two ? launch_lut<2, false, true, 2, true>(grid, stream, p, q) : launch_lut<2, false, true, 1, true>(grid, stream, p, q);
     *fused = true;
     *fused_blocks = grid;
   } else {
-    le = launch_lut_plain<false>(n_p, n_s, grid, stream, p, q);
+    le = two ? launch_lut<2, false, true, 2>(grid, stream, p, q) : launch_lut<2, false, true, 1>(grid, stream, p, q);
   }
   t_path = 4;
   const cudaError_t ce = le != cudaSuccess ? le : cudaGetLastError();
@@ -1169,7 +1186,10 @@ extern "C" hb_status hb_set_devices(const hb_device_spec* rows, int32_t n) {
       uint8_t* st = &g_tab.lut_s[static_cast<size_t>(i) * kLutS];
       LutOcc* tt = &g_tab.lut_t[static_cast<size_t>(i) * kLutOcc];
       if (g_tab.lut_ok[i]) {
-        build_row_lut(g_tab.rows[i], fold_fast(g_tab.rows[i], g_tab.pre[i]), pt, st, tt, magic);
+        g_tab.fast[i] = fold_fast(g_tab.rows[i], g_tab.pre[i]);
+        build_row_lut(g_tab.rows[i], g_tab.fast[i], pt, st, tt, magic);
+        g_tab.p_class[i] = class_of(g_tab.p_reps, g_tab.words_p, g_tab.lut_p, kLutP, i, same_p_class);
+        g_tab.s_class[i] = class_of(g_tab.s_reps, g_tab.words_s, g_tab.lut_s, kLutS, i, same_smem_class);
       } else {
         std::memset(pt, 0, kLutP);
         std::memset(st, 0, kLutS);
