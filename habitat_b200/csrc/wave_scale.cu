@@ -21,6 +21,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "hb_common.h"
@@ -369,11 +370,10 @@ bool vec4_ok(const Ptrs& p, int64_t K, bool need_gamma) {
 // Rows that agree on everything P (or S) reads form a class.  The tables of four classes lie interleaved in one
 // table of words, so a record's bytes for up to four classes are one load (eight: two), and a destination picks
 // its two bytes with a byte permute and takes one 16-bit-pair minimum for the two records a thread owns.  The
-// tables a launch touches (a few KB) stay in L1.  The extended variant (EXT) reads every device's own P and S
-// bytes per pair instead (no class limit) and adds, under launch-uniform branches,
-// the status plane, per-destination register counts and gamma from raw metrics
-// (one float64 intensity per record, a compare and a multiply-add per pair); it
-// also serves launches with more than eight classes.
+// tables a launch touches (a few KB) stay in L1.  The extended variant (EXT) adds, under launch-uniform branches,
+// the status plane, per-destination register counts (another P word per pair that has one) and gamma from raw
+// metrics (one float64 intensity per record, a compare and a multiply-add per pair).  Without classes (NW = 0, more
+// than eight in a launch) it reads every device's own P and S bytes per pair.
 // Conditions (checked on the host, else wave_scale_fast_kernel or the generic
 // kernel runs): D <= 32, D K < 2^31, and per row 2 <= SMs <= 4096,
 // blocks-per-SM limit <= 32, thread limit per block a multiple of 32 and <= 1024,
@@ -424,6 +424,7 @@ struct LutParams {
   LutDev dest[HB_MAX_DEVICES / 2];
   double ridge[HB_MAX_DEVICES / 2];                  // metrics mode: destination peak / bandwidth
   double slope[HB_MAX_DEVICES / 2];                  // -0.5 / ridge
+  double half_ridge[HB_MAX_DEVICES / 2];
 };
 
 constexpr int kLutThreads = 128;
@@ -496,16 +497,20 @@ __device__ __forceinline__ void store_byte_pair(uint8_t* q, uint32_t pair_word, 
 // TOT: every block also adds up its own results per destination (float64, fixed order, NaN results
 // skipped like the plane sums do) and leaves the sums in p.block_sums[d * gridDim.x + block], so
 // the totals of a launch need no second pass over the [D x K] plane.  A thread parks the float64
-// sum of its two results per destination in shared memory; at the end sixteen lanes per
-// destination add the block's 128 sums.  Needs a grid that covers the batch in one pass and
-// D <= kTotMaxD.
-constexpr int kTotMaxD = kLutThreads / 16;
+// sum of its two results per destination in shared memory; at the end TOT lanes per destination (sixteen up to eight
+// destinations, eight up to kTotMaxD) add the block's 128 sums.  Needs a grid that covers the batch in one pass.
+constexpr int kTotMaxD = 16;
 
-template <int VEC, bool EXT, bool ALIGNED, int NW, bool TOT = false>
-__global__ void __launch_bounds__(kLutThreads, EXT ? 8 : 12)
+// EXT: 0 plain, 1 with the status plane and per-destination registers, 2 and 3 with gamma from metrics as well,
+// whose float64 values take 20 registers.  With 56 registers (2) nine blocks fit an SM, with 48 (3) ten: the
+// batch that has more blocks than the first can hold at a time is 11 % faster with the second (4 M kernels x 6: 142
+// -> 127 us), a smaller one 6 % slower (250,001: 12.6 -> 13.4 us).
+template <int VEC, int EXT, bool ALIGNED, int NW, int TOT = 0>
+__global__ void __launch_bounds__(kLutThreads, EXT == 2 ? 8 : (EXT == 3 ? 10 : 12))
 wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
-  static_assert(!TOT || (VEC == 2 && ALIGNED && !EXT), "fused totals: aligned two-record variant only");
-  __shared__ double s_tot[TOT ? kTotMaxD : 1][TOT ? kLutThreads : 1];
+  static_assert(!TOT || (VEC == 2 && EXT == 0), "fused totals: plain two-record variants only");
+  extern __shared__ __align__(16) double s_tot_raw[];   // TOT: [D][kLutThreads]
+  double(*s_tot)[kLutThreads] = reinterpret_cast<double(*)[kLutThreads]>(s_tot_raw);
   hb_grid_dependency_wait();
   const uint32_t K = lp.K;
   const int D = lp.D;
@@ -516,7 +521,7 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
   const uint8_t* __restrict__ tab_m = reinterpret_cast<const uint8_t*>(g_lut_m);
   const uint8_t* __restrict__ tab_a = reinterpret_cast<const uint8_t*>(g_lut_a);
   const bool with_regs = EXT && p.dest_regs != nullptr;
-  const bool with_metrics = EXT && p.has_metrics != nullptr;
+  constexpr bool with_metrics = EXT >= 2;
   const bool with_status = EXT && p.status != nullptr;
 
   if (k0 < K) {
@@ -539,13 +544,13 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
     };
     uint32_t wrow[2] = {0u, 0u};                 // EXT: warps per block x row length (P index base)
     float omg[2] = {0.0f, 0.0f};
-    double xint[2] = {-1.0, -1.0}, xinv[2] = {0.0, 0.0};   // EXT: intensity (< 0: special case) and 1 / intensity
+    double xint[2] = {0.0, 0.0}, xinv[2] = {0.0, 0.0};   // EXT: intensity and 1 / intensity
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
       const uint32_t wpb = min((static_cast<uint32_t>(bsv.v[i]) + 31u) >> 5, static_cast<uint32_t>(kLutW - 1));
       const uint32_t pidx = HB_IDX(lut_p_index(bsv.v[i], rgv.v[i]), kLutP, 1);
       const uint32_t steps = HB_IDX(lut_s_index(smv.v[i]), kLutS, 2);
-      if (!EXT) {
+      if (NW > 0) {
         P[i] = __ldg(g_lut_pw + (lp.off_p[0] + pidx));
         S[i] = __ldg(g_lut_sw + (lp.off_s[0] + steps));
         if (NW == 2) {
@@ -553,32 +558,30 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
           S2[i] = __ldg(g_lut_sw + (lp.off_s[1] + steps));
         }
       } else {
-        // extended variant: every device's own tables are indexed directly (no class limit)
-        P[i] = pidx; S[i] = steps;
-        wrow[i] = wpb * kLutU;
+        P[i] = pidx; S[i] = steps;   // every device's own tables are indexed directly (no class limit)
       }
+      if (EXT) wrow[i] = wpb * kLutU;
       if (!with_metrics) omg[i] = 1.0f - gv.v[i];
       if (with_metrics) {
-        // wave_scaling/roofline.py:68-92, float64, same operation order
-        double x = -1.0;   // "no metrics" or next to no floating-point work: gamma = 1
+        // wave_scaling/roofline.py:68-92, float64.  The rule below gives gamma 1 for intensity 0 and gamma 0
+        // for an infinite one, which is how its two special cases are written here: no metrics or next to no
+        // floating-point work, and no memory traffic.
         const uint32_t ki = (i == 0 || pair) ? k0 + i : k0;   // the tail thread's second slot repeats the first
         if (p.has_metrics[ki]) {
           const double total_gb = (p.dram_read[ki] + p.dram_write[ki]) / 1024 / 1024 / 1024;
-          const double gps = p.flop_eff[ki] / 100 * lp.origin_peak;
-          const double gf = gps * static_cast<double>(tv.v[i]) / 1e9;
-          if (gf < 1e-9) x = -1.0;
-          else if (total_gb == 0) x = -2.0;   // gamma = 0
-          else x = gf / total_gb;
+          const double gf = p.flop_eff[ki] * (lp.origin_peak / 100 / 1e9) * static_cast<double>(tv.v[i]);
+          if (!(gf < 1e-9)) {
+            xint[i] = total_gb == 0 ? __longlong_as_double(0x7FF0000000000000ll) : gf / total_gb;
+            xinv[i] = total_gb == 0 ? 0.0 : total_gb / gf;
+          }
         }
-        xint[i] = x;
-        xinv[i] = x > 0.0 ? 1.0 / x : 0.0;
       }
     }
 
     // origin: both records at once
     const LutDevRegs og = load_lut_dev(lp.origin);
     uint32_t o2;
-    if (!EXT) {
+    if (NW > 0) {
       o2 = occ_pair(og);
     } else {
       o2 = 0;
@@ -611,6 +614,20 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
     store_byte_pair<VEC, ALIGNED>(p.origin_occ + k0, o2, pair);
     store_pair<uint32_t, VEC, ALIGNED>(p.origin_waves + k0, owav, pair);
 
+    // per-destination register counts of the two records (-1: the record's own)
+    auto load_regs = [&](uint32_t at) {
+      Vec<int16_t, VEC> r;
+      if (VEC == 1 || ALIGNED) {
+        r = load_vec<int16_t, VEC>(p.dest_regs + at);
+      } else {
+        r.v[0] = p.dest_regs[at];
+        r.v[VEC - 1] = pair ? p.dest_regs[at + 1] : static_cast<int16_t>(-1);
+      }
+      return r;
+    };
+    Vec<int16_t, VEC> drv;
+    if (with_regs) drv = load_regs(k0);
+
 #pragma unroll 1
     for (int d = 0; d < D; ++d) {
       const LutDevRegs dd = load_lut_dev(lp.dest[d]);
@@ -619,27 +636,36 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
       if (!EXT) {
         occ2 = occ_pair(dd);
       } else {
-        Vec<int16_t, VEC> drv;
+        // the next destination's counts are on their way while this one is worked on
+        const Vec<int16_t, VEC> now = drv;
+        if (with_regs && d + 1 < D) drv = load_regs(base + lp.stride);
+        uint32_t over[2] = {0u, 0u};   // P index of a record that MetadataManager.kernel_registers_for gave other registers
+        bool other[2] = {false, false};
         if (with_regs) {
-          if (VEC == 1 || ALIGNED) {
-            drv = load_vec<int16_t, VEC>(p.dest_regs + base);
-          } else {
-            drv.v[0] = p.dest_regs[base];
-            drv.v[VEC - 1] = pair ? p.dest_regs[base + 1] : static_cast<int16_t>(-1);
+#pragma unroll
+          for (int i = 0; i < VEC; ++i) {
+            other[i] = now.v[i] >= 0;
+            const uint32_t units = min((static_cast<uint32_t>(now.v[i]) + 7u) >> 3, static_cast<uint32_t>(kLutU - 1));
+            over[i] = HB_IDX(wrow[i] + units, kLutP, 5);
           }
         }
-        occ2 = 0;
+        if (NW > 0) {
+          const bool p2 = NW == 2 && (dd.sm.w & 1u), s2 = NW == 2 && (dd.sm.w & 2u);
+          uint32_t pw[2] = {p2 ? P2[0] : P[0], p2 ? P2[1] : P[1]};
+          if (with_regs) {
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) {
-          uint32_t pidx = P[i];
-          if (with_regs && drv.v[i] >= 0) {
-            // MetadataManager.kernel_registers_for gave another register count for this destination
-            const uint32_t units = min((static_cast<uint32_t>(drv.v[i]) + 7u) >> 3, static_cast<uint32_t>(kLutU - 1));
-            pidx = HB_IDX(wrow[i] + units, kLutP, 5);
+            for (int i = 0; i < VEC; ++i)
+              if (other[i]) pw[i] = __ldg(g_lut_pw + (lp.off_p[p2 ? 1 : 0] + over[i]));
           }
-          const uint32_t pb = __ldg(g_lut_p + (dd.sel.w + pidx));
-          const uint32_t sb = __ldg(g_lut_s + (dd.sm.z + S[i]));
-          occ2 |= min(pb, sb) << (16 * i);
+          occ2 = __vimin_s16x2_relu(prmt(pw[0], pw[1], dd.sel.x), prmt(s2 ? S2[0] : S[0], s2 ? S2[1] : S[1], dd.sel.y));
+        } else {
+          occ2 = 0;
+#pragma unroll
+          for (int i = 0; i < VEC; ++i) {
+            const uint32_t pb = __ldg(g_lut_p + (dd.sel.w + (other[i] ? over[i] : P[i])));
+            const uint32_t sb = __ldg(g_lut_s + (dd.sm.z + S[i]));
+            occ2 |= min(pb, sb) << (16 * i);
+          }
         }
       }
       Vec<float, VEC> outv;
@@ -663,10 +689,7 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
         const float2 lg_d = __ldg(reinterpret_cast<const float2*>(tab_a + (dd.sel.z + HB_IDX(dm, kLutOcc, 7) * 8u)));
         float gamma, one_minus;
         if (with_metrics) {
-          const double x = xint[i];
-          double gm;
-          if (x < 0.0) gm = x == -1.0 ? 1.0 : 0.0;
-          else gm = x > lp.ridge[d] ? 0.5 * lp.ridge[d] * xinv[i] : fma(lp.slope[d], x, 1.0);
+          const double gm = xint[i] > lp.ridge[d] ? lp.half_ridge[d] * xinv[i] : fma(lp.slope[d], xint[i], 1.0);
           gamma = static_cast<float>(gm);
           one_minus = static_cast<float>(1.0 - gm);
         } else {
@@ -689,25 +712,26 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
       if (with_status) store_byte_pair<VEC, ALIGNED>(p.status + base, st2, pair);
       if (TOT) {
         const float g0 = outv.v[0] == outv.v[0] ? outv.v[0] : 0.0f;                     // NaN: no prediction
-        const float g1 = outv.v[VEC - 1] == outv.v[VEC - 1] ? outv.v[VEC - 1] : 0.0f;
+        const float g1 = pair && outv.v[VEC - 1] == outv.v[VEC - 1] ? outv.v[VEC - 1] : 0.0f;
         s_tot[d][threadIdx.x] = static_cast<double>(g0) + static_cast<double>(g1);   // exact
       }
     }
   }
   if (TOT) {
     __syncthreads();
-    const int d = threadIdx.x >> 4, j = threadIdx.x & 15;
+    constexpr int kLanes = TOT ? TOT : 16;
+    const int d = threadIdx.x / kLanes, j = threadIdx.x % kLanes;
     double acc = 0.0;
     if (d < D) {
       const double2* row = reinterpret_cast<const double2*>(s_tot[d]);
 #pragma unroll
-      for (int i = 0; i < kLutThreads / 32; ++i) {
-        const double2 x = row[j + 16 * i];
+      for (int i = 0; i < kLutThreads / (2 * kLanes); ++i) {
+        const double2 x = row[j + kLanes * i];
         acc += x.x + x.y;
       }
     }
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) acc += __shfl_down_sync(0xFFFFFFFFu, acc, o, 16);
+    for (int o = kLanes / 2; o > 0; o >>= 1) acc += __shfl_down_sync(0xFFFFFFFFu, acc, o, kLanes);
     if (j == 0 && d < D) p.block_sums[static_cast<size_t>(d) * gridDim.x + blockIdx.x] = acc;
   }
 }
@@ -835,10 +859,10 @@ int class_of(std::vector<FastDev>& reps, std::vector<uint32_t>& words, const std
   return static_cast<int>(c);
 }
 
-template <int VEC, bool EXT, bool ALIGNED, int NW, bool TOT = false>
+template <int VEC, int EXT, bool ALIGNED, int NW, int TOT = 0>
 cudaError_t launch_lut(unsigned grid, cudaStream_t stream, const Ptrs& p, const LutParams& q) {
   return hb::launch_overlapped(wave_scale_lut_kernel<VEC, EXT, ALIGNED, NW, TOT>, dim3(grid), dim3(kLutThreads),
-                               0, stream, p, q);
+                               TOT ? sizeof(double) * kLutThreads * q.D : 0, stream, p, q);
 }
 
 // Everything about a launch that depends on the devices alone.  Callers ask for the same origin and
@@ -885,6 +909,7 @@ void fill_lut(LaunchPlan* plan) {   // call with g_mu held
       o.b_lo = static_cast<float>(lp.b[d] - static_cast<double>(o.b_hi));
       q.ridge[d] = lp.ridge[d];
       q.slope[d] = -0.5 / lp.ridge[d];
+      q.half_ridge[d] = 0.5 * lp.ridge[d];
     }
   }
   plan->words = std::max({plan->words, n_p, n_s});
@@ -930,19 +955,38 @@ bool try_launch_lut(const Ptrs& p, const LaunchPlan& plan, int64_t K, int64_t st
   const bool two = plan.words == 2;
   cudaError_t le;
   if (ext) {
-    le = !vec2 ? launch_lut<1, true, true, 1>(grid, stream, p, q)
-               : (aligned ? launch_lut<2, true, true, 1>(grid, stream, p, q)
-                          : launch_lut<2, true, false, 1>(grid, stream, p, q));
+    auto launch_ext = [&](auto words) {
+      constexpr int W = decltype(words)::value;
+      if (metrics && vec2 && blocks > 9ll * sm_count)
+        return aligned ? launch_lut<2, 3, true, W>(grid, stream, p, q) : launch_lut<2, 3, false, W>(grid, stream, p, q);
+      if (metrics)
+        return !vec2 ? launch_lut<1, 2, true, W>(grid, stream, p, q)
+                     : (aligned ? launch_lut<2, 2, true, W>(grid, stream, p, q) : launch_lut<2, 2, false, W>(grid, stream, p, q));
+      return !vec2 ? launch_lut<1, 1, true, W>(grid, stream, p, q)
+                   : (aligned ? launch_lut<2, 1, true, W>(grid, stream, p, q) : launch_lut<2, 1, false, W>(grid, stream, p, q));
+    };
+    le = plan.words > kMaxWords ? launch_ext(std::integral_constant<int, 0>{})
+                                : (two ? launch_ext(std::integral_constant<int, 2>{}) : launch_ext(std::integral_constant<int, 1>{}));
   } else if (!vec2) {
-    le = launch_lut<1, false, true, 2>(grid, stream, p, q);
-  } else if (!aligned) {
-    le = two ? launch_lut<2, false, false, 2>(grid, stream, p, q) : launch_lut<2, false, false, 1>(grid, stream, p, q);
-  } else if (p.block_sums && lp.D <= kTotMaxD) {
-    le = two ? launch_lut<2, false, true, 2, true>(grid, stream, p, q) : launch_lut<2, false, true, 1, true>(grid, stream, p, q);
-    *fused = true;
-    *fused_blocks = grid;
+    le = launch_lut<1, 0, true, 2>(grid, stream, p, q);
   } else {
-    le = two ? launch_lut<2, false, true, 2>(grid, stream, p, q) : launch_lut<2, false, true, 1>(grid, stream, p, q);
+    // Odd batches and nine to sixteen destinations are summed here from 131,073 records on, where reading the
+    // results again is what the plane sum would spend its time on (table kernel and final stage, us, before and
+    // after: 300,001 x 6 16.9 -> 13.4, 1,000,001 x 6 26.5 -> 20.6, 1,000,000 x 12 46.7 -> 34.9).  Smaller ones keep
+    // the plane sum's 256 sums per destination, the number their callers see in per_plane; a launch is all that
+    // would be saved there (70,001 x 6 15.6 -> 13.8).
+    *fused = p.block_sums && ((aligned && lp.D <= 8) || (lp.D <= kTotMaxD && K > (1 << 17)));
+    *fused_blocks = grid;
+    auto launch_plain = [&](auto is_aligned, auto lanes) {
+      constexpr bool A = decltype(is_aligned)::value;
+      constexpr int T = decltype(lanes)::value;
+      return two ? launch_lut<2, 0, A, 2, T>(grid, stream, p, q) : launch_lut<2, 0, A, 1, T>(grid, stream, p, q);
+    };
+    auto launch_totals = [&](auto lanes) {
+      return aligned ? launch_plain(std::true_type{}, lanes) : launch_plain(std::false_type{}, lanes);
+    };
+    le = !*fused ? launch_totals(std::integral_constant<int, 0>{})
+                 : (lp.D <= 8 ? launch_totals(std::integral_constant<int, 16>{}) : launch_totals(std::integral_constant<int, 8>{}));
   }
   t_path = 4;
   const cudaError_t ce = le != cudaSuccess ? le : cudaGetLastError();

@@ -3,7 +3,8 @@ import numpy as np
 import pytest
 import torch
 
-from habitat_b200 import batched, workloads
+from habitat_b200 import batched, device_table, workloads
+from habitat_b200.habitat_cuda import DeviceProperties
 from oracle import wave as owave
 from tests.helpers import assert_wave_equal, run_wave_gpu, run_wave_oracle, to_numpy
 
@@ -414,3 +415,47 @@ def test_host_entry_in_chunks(bench_devices, K, page_locked, monkeypatch):
         if n != "status":
             assert np.array_equal(other[n][..., ::-1].copy().view(np.uint8), want[n].view(np.uint8)), n
     assert other["status"] is None and first["limits"] is None
+
+
+@pytest.mark.parametrize("K,D", [(131_073, 6), (131_074, 9), (200_001, 16), (131_072, 16), (300_000, 17), (1_000_001, 1)])
+def test_totals_of_odd_batches_and_many_destinations(bench_devices, device_file, K, D):
+    """From 131,073 kernels on, odd batches and up to sixteen destinations are summed inside the table kernel as
+    well; sixteen destinations or an even batch at the line itself, and seventeen, are not.  float64 sums in a
+    fixed order: 1e-13 of the exact ones (2^-52 times the 14 levels of additions)."""
+    kernels = workloads.make_kernels(K, seed=K + D)
+    dests = (bench_devices * 3)[:D]
+    out, totals, partials, path = _wave_with_partials(kernels, bench_devices[0], dests)
+    assert path == "wave_scale_lut_kernel"
+    assert partials.per_plane == ((K + 255) // 256 if K > 131_072 and D <= 16 else 256)
+    want = np.nansum(to_numpy(out.scaled_ns).astype(np.float64), axis=1)
+    assert np.allclose(totals, want, rtol=1e-13, atol=0)
+    plain = batched.wave_scale(batched.KernelBatch.from_numpy(kernels), bench_devices[0], dests)
+    for n in ("scaled_ns", "dest_occupancy", "dest_waves"):
+        assert np.array_equal(to_numpy(getattr(out, n)).view(np.uint8), to_numpy(getattr(plain, n)).view(np.uint8))
+
+
+def test_launches_over_many_device_classes(bench_devices):
+    """The class tables hold four classes per word and a launch takes up to two words: rows with ever larger
+    shared memory need one word, two, and then every row's own tables.  Times against the oracle; with metrics the
+    planes of single-destination launches, bit for bit."""
+    device_table.reset()      # the rows of other tests and these may be more than the table holds
+    base = dict(bench_devices[2]._fields)
+    rows = [DeviceProperties("custom%d" % i, **dict(base, shared_mem_per_multiprocessor=65536 + 1024 * i))
+            for i in range(11)]
+    K = 3001
+    kernels = workloads.make_kernels(K, seed=77)
+    regs = workloads.rng(5).integers(-1, 256, size=(11, K)).astype(np.int16)
+    metrics = workloads.make_metrics(K, seed=4)
+    single = [run_wave_gpu(kernels, rows[0], [r], metrics=metrics) for r in rows]
+    for n in (4, 5, 8, 9, 11):
+        for dest_regs in (None, regs[:n]):
+            got = run_wave_gpu(kernels, rows[0], rows[:n], dest_regs=dest_regs)
+            assert got["fast_path"] == "wave_scale_lut_kernel"
+            assert_wave_equal(got, run_wave_oracle(kernels, rows[0], rows[:n], dest_regs=dest_regs))
+        got = run_wave_gpu(kernels, rows[0], rows[:n], metrics=metrics)
+        assert got["plain_path"] == "wave_scale_lut_kernel"
+        for d in range(n):
+            for name in ("fast", "plain"):
+                for plane in ("scaled_ns", "dest_occupancy", "dest_waves"):
+                    assert np.array_equal(got[name][plane][d].view(np.uint8), single[d][name][plane][0].view(np.uint8))
+    device_table.reset()
