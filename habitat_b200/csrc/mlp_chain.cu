@@ -948,10 +948,10 @@ hb::WidePlan plan_of(const hb_mlp* h, int64_t Q) {
 }
 
 // Queues one batch (checked by the callers) on the kernel for its size.
-hb_status queue_batch(hb_mlp* h, const hb::MlpBatch& batch, cudaStream_t s) {
+hb_status queue_batch(hb_mlp* h, const hb::WidePlan& plan, const hb::MlpBatch& batch, cudaStream_t s) {
   bool launched = false;
   hb_status st = check_device(h);
-  if (st == HB_OK) st = hb::wide_predict(h, plan_of(h, batch.Q), batch, s, &launched);
+  if (st == HB_OK) st = hb::wide_predict(h, plan, batch, s, &launched);
   if (st != HB_OK || launched) return st;
   ChainLaunch launch(h, h->precision == HB_PRECISION_BF16X3);
   st = launch.add(h, batch);
@@ -968,7 +968,7 @@ extern "C" hb_status hb_mlp_predict(hb_mlp* h, const float* op_features, const u
   if (Q == 0) return HB_OK;
   hb::MlpBatch batch;
   batch.feats = op_features; batch.dev_row = device_row; batch.Q = Q; batch.out = out;
-  return queue_batch(h, batch, static_cast<cudaStream_t>(stream));
+  return queue_batch(h, plan_of(h, Q), batch, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" hb_status hb_mlp_predict_grid(const hb_mlp_grid* items, int32_t n_items, void* stream) {
@@ -1006,8 +1006,20 @@ extern "C" hb_status hb_mlp_predict_grid(const hb_mlp_grid* items, int32_t n_ite
     const hb_status st = batch.Q ? check_device(g.handle) : HB_OK;
     if (st != HB_OK) return st;
   }
+  hb::WidePlan plans[hb::kMaxLanes];
+  int64_t sizes[hb::kMaxLanes];
+  bool split[hb::kMaxLanes], all_wide = true;
+  int some = 0;   // batches with queries, the first ones in `order`
+  for (; some < n_items && !queued[order[some]]; ++some) {
+    const int i = order[some];
+    plans[some] = plan_of(items[i].handle, batches[i].Q);
+    sizes[some] = batches[i].Q;
+    split[some] = items[i].handle->precision == HB_PRECISION_BF16X3;
+    all_wide = all_wide && plans[some].G != 0;
+  }
+  if (all_wide && some > 1) hb::wide_plans_together(plans, sizes, split, some, items[order[0]].handle->sm_count);
   int lane = 0;
-  for (int k = 0; k < n_items; ++k) {
+  for (int k = 0; k < some; ++k) {
     const int i = order[k];
     if (queued[i]) continue;
     hb_mlp* h = items[i].handle;
@@ -1015,17 +1027,17 @@ extern "C" hb_status hb_mlp_predict_grid(const hb_mlp_grid* items, int32_t n_ite
     batches[i].beside = lane > 0;
     ++lane;
     hb_status st = HB_OK;
-    if (plan_of(h, batches[i].Q).G != 0) {
-      st = queue_batch(h, batches[i], static_cast<cudaStream_t>(stream));
+    if (plans[k].G != 0) {
+      st = queue_batch(h, plans[k], batches[i], static_cast<cudaStream_t>(stream));
       if (st != HB_OK) return st;
       continue;
     }
     ChainLaunch launch(h, h->precision == HB_PRECISION_BF16X3);
-    for (int m = k; m < n_items && st == HB_OK; ++m) {
+    for (int m = k; m < some && st == HB_OK; ++m) {
       const int o = order[m];
       const hb_mlp* other = items[o].handle;
       if (queued[o] || other->precision != h->precision) continue;
-      const bool fills = plan_of(other, batches[o].Q).G == 0;
+      const bool fills = plans[m].G == 0;
       if (m > k && !fills && launch.rounds(launch.tiles_of(batches[o].Q)) > launch.rounds(0)) continue;
       st = launch.add(other, batches[o]);
       queued[o] = true;

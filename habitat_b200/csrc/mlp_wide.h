@@ -31,6 +31,8 @@ struct MlpBatch {
   bool beside = false;
 };
 constexpr int kMaxLanes = 4;
+// Replaces the plans of n <= kMaxLanes batches that are launched side by side, where others finish sooner.
+void wide_plans_together(WidePlan* plans, const int64_t* Q, const bool* split, int n, int sm_count);
 // Queues the launch; *launched stays false when the stream has no scratch (see there).
 hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cudaStream_t stream, bool* launched);
 // After a launch that gave up: every stream's scratch on the GPU is set up again before its next use.

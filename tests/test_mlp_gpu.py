@@ -300,3 +300,38 @@ def test_small_batches_on_streams_and_in_a_graph():
     for h in hs:
         h.check_status()
         h.close()
+
+
+@pytest.mark.parametrize("sizes", [[(1, 1), (1, 1), (1, 1), (1, 1)], [(40, 6), (16, 1)], [(264, 4), (250, 4)],
+                                   [(1056, 1), (4, 4)], [(352, 6), (1, 1)], [(53, 6), (1, 6), (0, 6), (32, 6)],
+                                   [(2112, 1), (2112, 1)], [(2113, 1), (300, 6), (7, 2)], [(9472, 1), (2500, 4), (9, 3)]])
+def test_batches_side_by_side(sizes):
+    """Batches of several predictors in one call take other shapes than alone where they then fit on the GPU
+    together, or one list of tiles; each prediction has the bits it has alone.  Sizes around full shapes, an
+    empty batch, small ones beside one that fills the GPU."""
+    import ctypes
+    from habitat_b200 import _native
+    items, keep, outs, want = (_native.MlpGrid * len(sizes))(), [], [], []
+    for i, (n, devices) in enumerate(sizes):
+        precision = "bf16x3" if i == 1 else "bf16"
+        feats, dev = workloads.make_queries("linear", max(n, 2), 50 + i)
+        mu, sigma = workloads.batch_mu_sigma(feats, dev)
+        h = batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=DEVF, precision=precision,
+                              **workloads.init_mlp_weights("linear", seed=i, layers=3 + i, gain=2.0))
+        f = torch.from_numpy(feats[:n]).cuda()
+        rows = bytes((5 * i + k) % len(DEVF) for k in range(devices))
+        out = torch.full((devices * n,), float("nan"), device="cuda")
+        each = torch.tensor(list(rows), dtype=torch.uint8, device="cuda").repeat_interleave(n)
+        want.append(h.predict(f.repeat(devices, 1).contiguous(), each) if n else out.clone())
+        items[i] = _native.MlpGrid(h._handle.value, f.data_ptr(), n, ctypes.cast(ctypes.c_char_p(rows), ctypes.c_void_p),
+                                   devices, out.data_ptr())
+        keep.append((h, f, rows))
+        outs.append(out)
+    for _ in range(3):
+        _native.check(_native.load().hb_mlp_predict_grid(items, len(sizes), torch.cuda.current_stream().cuda_stream))
+        for k, (got, ref) in enumerate(zip(outs, want)):
+            assert torch.equal(got, ref), k
+            got.fill_(float("nan"))
+    for h, _, _ in keep:
+        h.check_status()
+        h.close()
