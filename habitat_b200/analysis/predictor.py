@@ -179,19 +179,20 @@ class _GroupPlan:
             self._take(operations, flat)
 
     @classmethod
-    def of_whole_trace(cls, operations, mode):
+    def of_whole_trace(cls, operations, mode, with_names):
         """The plan of a trace recorded on one device, walked by the native binding; None when the
         operations are not all of this package's ordinary classes (any object with their surface
         takes the Python walk), or when a missing metric has to raise (the roofline strategy)."""
         if mode == wave_batch.ROOFLINE:
             return None
         flat = _native.binding().flatten_trace(operations, _trace_types(), SPECIAL_OPERATIONS, _MLP_OPS, _METRIC_KEYS,
-                                               mode != wave_batch.RESIMPLIFIED, _FAST_ORDERS)
+                                               mode != wave_batch.RESIMPLIFIED, _FAST_ORDERS, with_names)
         return cls(operations, None, mode, flat) if flat is not None else None
 
     def _take(self, operations, flat):
-        (self.kernels, self.runs, names, wave_idx, fwd, bwd, offsets, overheads, kind_idx, self.passthrough_idx,
+        (self.n_kernels, self.n_runs, self._names, wave_idx, fwd, bwd, offsets, overheads, kind_idx, self.passthrough_idx,
          records, metrics, self.offsets_dev, special) = flat
+        self._kernels, self._operations = None, operations
         self.indices = None                      # all operations
         self.wave_idx, self.fwd_run, self.bwd_run, self.offsets = (
             np.frombuffer(x, np.int64) for x in (wave_idx, fwd, bwd, offsets))
@@ -202,8 +203,23 @@ class _GroupPlan:
                 self.mlp_inputs[name] = (got[0], got[1], np.frombuffer(got[2], np.float32), FEATURES[name])
         for i in self.passthrough_idx:
             logger.warning("Unhandled special operation: %s", operations[i].name)
-        self.flat = (wave_batch.FlatKernels.from_device(self.mode, names, records, metrics) if self.kernels
-                     else None)
+        self.flat = (wave_batch.FlatKernels.from_device(self.mode, self.n_kernels, self._names, records, metrics)
+                     if self.n_kernels else None)
+
+    # The recorded kernels and their names, in the order of the flattened records: only the register table and
+    # user-supplied strategies ask for them.
+    @property
+    def kernels(self):
+        if self._kernels is None:
+            self._kernels = [k for i in self.wave_idx for run in (self._operations[i].forward, self._operations[i].backward)
+                             if run is not None for k in run.kernels]
+        return self._kernels
+
+    @property
+    def names(self):
+        if self._names is None:
+            self._names = [k.name for k in self.kernels]
+        return self._names
 
     def _flatten(self, operations, indices, mode):
         self.indices = np.asarray(indices, np.int64)
@@ -231,14 +247,16 @@ class _GroupPlan:
         self.wave_idx = np.asarray(wave_idx, np.int64)
         self.fwd_run = np.asarray(fwd_run, np.int64)
         self.bwd_run = np.asarray(bwd_run, np.int64)
-        self.runs = runs
-        self.kernels = []
+        self._kernels, self._names = [], None
         offsets = [0]
         for run in runs:
-            self.kernels.extend(run.kernels)
-            offsets.append(len(self.kernels))
+            self._kernels.extend(run.kernels)
+            offsets.append(len(self._kernels))
+        self.n_kernels, self.n_runs = len(self._kernels), len(runs)
         self.offsets = np.asarray(offsets, np.int64)
         self.flat = wave_batch.FlatKernels(self.kernels, mode) if (self.kernels and mode is not None) else None
+        if self.flat is not None:
+            self._names = self.flat.names
         # launch overhead of a pass (predictor.py:113-116 of the reference): wall time minus kernel time
         measured = np.array([k.run_time_ns for k in self.kernels], np.float64)
         per_run = np.add.reduceat(np.concatenate([measured, [0.0]]), self.offsets[:-1]) if runs else np.zeros(0)
@@ -332,12 +350,12 @@ class PredictedOperations(collections.abc.Sequence):
                                       None, self._dest)
         plan = g["plan"]
 
-        def run(r):
+        def run(r, measured):
             lo, hi = plan.offsets[r], plan.offsets[r + 1]
-            return _LazyRunTimePrediction(float(plan.overheads[r]), plan.kernels[lo:hi], g["times"][lo:hi],
+            return _LazyRunTimePrediction(float(plan.overheads[r]), measured.kernels, g["times"][lo:hi],
                                           float(g["totals"][r]), self._dest)
         b = self._b[i]
-        return PredictedOperation(op, run(self._a[i]), run(b) if b >= 0 else None, self._dest)
+        return PredictedOperation(op, run(self._a[i], op.forward), run(b, op.backward) if b >= 0 else None, self._dest)
 
 
 class Predictor:
@@ -429,7 +447,7 @@ class Predictor:
         if plan is None:
             if mode is None or any(d.name == origin.name for d in dest_devices):
                 return None
-            plan = _GroupPlan.of_whole_trace(operations, mode)
+            plan = _GroupPlan.of_whole_trace(operations, mode, self._has_registers())
             if plan is None:
                 return None
             if cache is not None:
@@ -443,6 +461,9 @@ class Predictor:
         return [PredictedOperations(operations, dest, dict(plan=plan, times=times[t], totals=totals[t]), ms[t], sums[t])
                 for t, dest in enumerate(dest_devices)]
 
+    def _has_registers(self):
+        return self._kernel_metadata is not None and not getattr(self._kernel_metadata, "empty", False)
+
     # ------------------------------------------------------------------
     def _predict_group(self, operations, indices, origin, dest_devices, targets, results, cache=None):
         dests = [dest_devices[d] for d in targets]
@@ -451,7 +472,8 @@ class Predictor:
         key = ("whole", mode, len(operations)) if whole else ("plan", origin.name, mode, len(indices))
         plan = cache.get(key) if cache is not None else None
         if plan is None:
-            plan = _GroupPlan.of_whole_trace(operations, mode) if whole and mode is not None else None
+            if whole and mode is not None:
+                plan = _GroupPlan.of_whole_trace(operations, mode, self._has_registers())
             plan = plan or _GroupPlan(operations, indices, mode)
             if cache is not None:
                 cache[key] = plan
@@ -479,7 +501,7 @@ class Predictor:
         (scaled kernel times [T, K], per-pass kernel totals [T, runs], sums of the rows of `ms`), all on
         the host (predictor.py:111-148 of the reference for every pass, special operation and destination
         at once)."""
-        T, K, n_runs = len(dests), len(plan.kernels), len(plan.runs)
+        T, K, n_runs = len(dests), plan.n_kernels, plan.n_runs
         names = [name for name in _MLP_OPS if len(plan.mlp_idx[name])]
         kinds = []
         for name in names:
@@ -501,8 +523,8 @@ class Predictor:
             run_ms = (plan.overheads + totals) / 1e6
             ms[:, plan.wave_idx] = run_ms[:, plan.fwd_run] + np.where(plan.bwd_run >= 0, run_ms[:, plan.bwd_run], 0.0)
         regs = None
-        if flat is not None:
-            regs = wave_batch.destination_registers(plan.kernels, flat.names, dests, self._kernel_metadata)
+        if flat is not None and self._has_registers():
+            regs = wave_batch.destination_registers(plan.kernels, plan.names, dests, self._kernel_metadata)
         nan, sums, clamped = _native.binding().run_group(
             flat.batch if flat is not None else None, flat.metrics if flat is not None else None, origin, dests, regs,
             plan.offsets_dev if flat is not None else None, kinds,

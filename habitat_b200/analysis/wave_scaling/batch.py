@@ -75,10 +75,10 @@ class FlatKernels:
     instead of walking the kernel objects again."""
 
     @classmethod
-    def from_device(cls, mode, names, records, metrics):
-        """From CUDA tensors in the order of KernelBatch's and KernelMetricsBatch's fields."""
+    def from_device(cls, mode, count, names, records, metrics):
+        """From CUDA tensors in the order of KernelBatch's and KernelMetricsBatch's fields; `names` may be None."""
         self = cls.__new__(cls)
-        self.mode, self.names, self.count = mode, names, len(names)
+        self.mode, self.names, self.count = mode, names, count
         self.batch = batched.KernelBatch(*records)
         self.metrics = batched.KernelMetricsBatch(*metrics) if metrics is not None else None
         return self
@@ -104,8 +104,9 @@ def scale_kernels(kernels, origin_device, dest_devices, metadata_manager, mode=U
     Returns a WaveResult whose tensors live on the GPU; nothing is synchronised here."""
     if flat is None or flat.mode != mode or flat.count != len(kernels):
         flat = FlatKernels(kernels, mode)
+    names = flat.names if flat.names is not None else [k.name for k in kernels]
     return batched.wave_scale(flat.batch, origin_device, dest_devices,
-                              dest_regs=destination_registers(kernels, flat.names, dest_devices, metadata_manager),
+                              dest_regs=destination_registers(kernels, names, dest_devices, metadata_manager),
                               metrics=flat.metrics)
 
 

@@ -40,6 +40,10 @@ class MetadataManager:
     def __len__(self):
         return sum(len(v) for v in self._by_name.values())
 
+    @property
+    def empty(self):
+        return not self._by_name
+
     def add(self, name, arch, registers_per_thread):
         entries = self._by_name.setdefault(name, [])
         entries.append((int(arch), int(registers_per_thread)))

@@ -404,9 +404,12 @@ PyObject* segment_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // ---------------------------------------------------------------------------
 // Attribute of an instance, new reference; null (with an error set) when it has none.
 inline PyObject* get(PyObject* o, PyObject* name) { return PyObject_GetAttr(o, name); }
+// The same for an instance of one of the package's recorded classes, which keep their fields in the instance:
+// MeasuredKernel's __getattr__ makes the ordinary look-up go through a Python-level hook's slot.
+inline PyObject* field(PyObject* o, PyObject* name) { return PyObject_GenericGetAttr(o, name); }
 // The integer attribute `name`; *ok is cleared when it is not a 64-bit integer.
 int64_t int_of(PyObject* o, PyObject* name, bool* ok) {
-  Ref v(get(o, name));
+  Ref v(field(o, name));
   if (!v.p || !PyLong_Check(v.p)) {
     *ok = false;
     return 0;
@@ -427,37 +430,47 @@ PyObject* not_ordinary() {
 }
 void* stream_now() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
-// Value of metric `which` among a kernel's metric records: 1 found, 0 absent, -1 not ordinary.  Mirrors
-// MeasuredKernel.get_metric for the three metrics of the roofline rule, whose canonical value is the raw one.
-int find_metric(PyObject* records, PyObject* cached, PyObject* metric, PyObject* name, PyObject* legacy,
-                PyTypeObject* instance_type, double* out) {
-  if (PyDict_GET_SIZE(cached) > 0) {
-    PyObject* hit = PyDict_GetItemWithError(cached, metric);   // borrowed
-    if (hit) {
-      *out = PyFloat_AsDouble(hit);
-      return PyErr_Occurred() ? -1 : 1;
-    }
+// Mirrors MeasuredKernel.get_metric for the three metrics of the roofline rule, whose canonical value is the raw
+// one.  The three metrics of a kernel ((Metric, name, legacy name) each) from the values it has looked up before or the
+// first record that holds them: 1, 0 when one is missing, -1 (perhaps with an error set) when something is not of
+// the ordinary classes.  One walk over the records; names are mostly the very objects that `metrics` holds.
+int find_metrics(PyObject* records, PyObject* cached, PyObject* metrics, PyTypeObject* instance_type, double* out) {
+  const Py_ssize_t n = PyList_GET_SIZE(records);
+  if (n == 0 && PyDict_GET_SIZE(cached) == 0) return 0;
+  PyObject* names[3][2];
+  unsigned missing = 0;
+  for (int m = 0; m < 3; ++m) {
+    PyObject* t = PyTuple_GET_ITEM(metrics, m);
+    names[m][0] = PyTuple_GET_ITEM(t, 1);
+    names[m][1] = PyTuple_GET_ITEM(t, 2);
+    PyObject* hit = PyDict_GET_SIZE(cached) > 0 ? PyDict_GetItemWithError(cached, PyTuple_GET_ITEM(t, 0)) : nullptr;   // borrowed
+    if (hit) out[m] = PyFloat_AsDouble(hit);
+    else missing |= 1u << m;
     if (PyErr_Occurred()) return -1;
   }
-  const Py_ssize_t n = PyList_GET_SIZE(records);
-  for (Py_ssize_t i = 0; i < n; ++i) {
+  for (Py_ssize_t i = 0; i < n && missing; ++i) {
     PyObject* rec = PyList_GET_ITEM(records, i);
     if (Py_TYPE(rec) != instance_type) return -1;
-    Ref list(get(rec, s__metrics));
+    Ref list(field(rec, s__metrics));
     if (!list.p || !PyList_Check(list.p)) return -1;
-    for (Py_ssize_t j = 0; j < PyList_GET_SIZE(list.p); ++j) {
+    for (Py_ssize_t j = 0; j < PyList_GET_SIZE(list.p) && missing; ++j) {
       PyObject* pair = PyList_GET_ITEM(list.p, j);
       if (!PyTuple_Check(pair) || PyTuple_GET_SIZE(pair) != 2) return -1;
       PyObject* key = PyTuple_GET_ITEM(pair, 0);
-      if (key != name && key != legacy) {
+      int m = 0;
+      while (m < 3 && key != names[m][0] && key != names[m][1]) ++m;
+      if (m == 3) {
         if (!PyUnicode_Check(key)) return -1;
-        if (PyUnicode_Compare(key, name) != 0 && PyUnicode_Compare(key, legacy) != 0) continue;
+        for (m = 0; m < 3; ++m)
+          if (PyUnicode_Compare(key, names[m][0]) == 0 || PyUnicode_Compare(key, names[m][1]) == 0) break;
       }
-      *out = PyFloat_AsDouble(PyTuple_GET_ITEM(pair, 1));
-      return PyErr_Occurred() ? -1 : 1;
+      if (m == 3 || !(missing >> m & 1u)) continue;
+      out[m] = PyFloat_AsDouble(PyTuple_GET_ITEM(pair, 1));
+      if (out[m] == -1.0 && PyErr_Occurred()) return -1;
+      missing &= ~(1u << m);
     }
   }
-  return 0;
+  return missing == 0 ? 1 : 0;
 }
 
 // A contiguous buffer (numpy array, bytes) seen as `count` values of T; ok() says whether it is that large.
@@ -477,15 +490,24 @@ struct Buffer {
   int64_t size() const { return held ? view.len / static_cast<int64_t>(sizeof(T)) : 0; }
 };
 
+// A Python number as a double; sizes are integers, which PyFloat_AsDouble makes a float object of.
+double number(PyObject* o, bool* ok) {
+  if (PyLong_CheckExact(o)) {
+    int overflow = 0;
+    const long v = PyLong_AsLongAndOverflow(o, &overflow);
+    if (!overflow) return static_cast<double>(v);
+  }
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) *ok = false;
+  return v;
+}
 // Element i of a tuple or list as a double (borrowed access); *ok is cleared when it is no number.
 double item(PyObject* seq, Py_ssize_t i, bool* ok) {
   if (!*ok || (!PyTuple_Check(seq) && !PyList_Check(seq)) || i >= PySequence_Fast_GET_SIZE(seq)) {
     *ok = false;
     return 0.0;
   }
-  const double v = PyFloat_AsDouble(PySequence_Fast_GET_ITEM(seq, i));
-  if (v == -1.0 && PyErr_Occurred()) *ok = false;
-  return v;
+  return number(PySequence_Fast_GET_ITEM(seq, i), ok);
 }
 
 constexpr Py_ssize_t kFeatureKinds = 3;   // conv2d, linear, bmm: the kinds with positional extractors
@@ -510,7 +532,7 @@ bool feature_row(long kind, PyObject* op, PyTypeObject* op_type, PyTypeObject* r
                  float* measured) {
   static const Py_ssize_t kArity[kFeatureKinds] = {5, 3, 2};
   if (Py_TYPE(op) != op_type) return false;
-  Ref arg(get(op, s__arguments)), f(get(op, s__forward)), b(get(op, s__backward));
+  Ref arg(field(op, s__arguments)), f(field(op, s__forward)), b(field(op, s__backward));
   if (!arg.p || !f.p || !b.p || arg.p == Py_None) return false;
   Ref args(get(arg.p, s_args)), kwargs(get(arg.p, s_kwargs));
   if (!args.p || !kwargs.p || !PyTuple_Check(args.p) || !PyDict_Check(kwargs.p) || PyDict_GET_SIZE(kwargs.p) != 0 ||
@@ -521,10 +543,7 @@ bool feature_row(long kind, PyObject* op, PyTypeObject* op_type, PyTypeObject* r
   double v[8] = {};
   if (kind == 0) {
     auto first = [&](PyObject* o) {
-      if (PyTuple_Check(o)) return item(o, 0, &ok);
-      const double d = PyFloat_AsDouble(o);
-      if (d == -1.0 && PyErr_Occurred()) ok = false;
-      return d;
+      return PyTuple_Check(o) ? item(o, 0, &ok) : number(o, &ok);
     };
     v[0] = item(x, 0, &ok); v[1] = item(x, 2, &ok); v[2] = item(x, 1, &ok); v[3] = item(w, 0, &ok);
     v[4] = item(w, 2, &ok);
@@ -546,7 +565,7 @@ bool feature_row(long kind, PyObject* op, PyTypeObject* op_type, PyTypeObject* r
   for (PyObject* r : {f.p, b.p}) {
     if (r == Py_None) continue;
     if (Py_TYPE(r) != run_type) return false;
-    Ref t(get(r, s__run_time_ms));
+    Ref t(field(r, s__run_time_ms));
     run += t.p ? PyFloat_AsDouble(t.p) : 0.0;
     if (PyErr_Occurred()) return false;
   }
@@ -558,25 +577,25 @@ bool feature_row(long kind, PyObject* op, PyTypeObject* op_type, PyTypeObject* r
 
 // flatten_trace(operations, (MeasuredOperation, RunTimeMeasurement, MeasuredKernel, KernelInstance),
 //               special names, MLP kinds (conv2d, linear, bmm first), metrics ((Metric, name, legacy name) x 3),
-//               with_metrics, column orders of the first three kinds)
+//               with_metrics, column orders of the first three kinds, with_names)
 // -> None when the operations are not all of those very classes or not of one device, else
-//    (kernels, runs, names, wave_idx, fwd_run, bwd_run, offsets, overheads: bytes of int64 / float64,
+//    (number of kernels, number of passes, names or None, wave_idx, fwd_run, bwd_run, offsets, overheads: bytes of int64 / float64,
 //     (indices per MLP kind: bytes of int64), passed-through indices,
 //     (num_blocks, block_size, regs, smem, time, gamma), (eff, read, write, has) or None, offsets: CUDA tensors,
 //     per kind of the first three: (features, measured ms: CUDA tensors, measured ms as bytes), or None when one of
 //     its operations was not recorded positionally)
 PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  if (n_args != 7) return not_ordinary();
+  if (n_args != 8) return not_ordinary();
   Ref ops(PySequence_Fast(a[0], "operations must be a sequence"));
   if (!ops.p) return nullptr;
   PyTypeObject* type[4];
   for (int i = 0; i < 4; ++i) type[i] = reinterpret_cast<PyTypeObject*>(PyTuple_GET_ITEM(a[1], i));
   PyObject *special = a[2], *kinds = a[3], *metrics = a[4];
-  const bool with_metrics = PyObject_IsTrue(a[5]) == 1;
+  const bool with_metrics = PyObject_IsTrue(a[5]) == 1, with_names = PyObject_IsTrue(a[7]) == 1;
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(ops.p), n_kinds = PyTuple_GET_SIZE(kinds);
 
-  Ref kernels(PyList_New(0)), runs(PyList_New(0)), names(PyList_New(0)), passed(PyList_New(0));
+  Ref names(with_names ? PyList_New(0) : Py_NewRef(Py_None)), passed(PyList_New(0));
   if (n_kinds < kFeatureKinds || n_kinds > 8) return not_ordinary();
   std::vector<int64_t> kind_idx[8];
   struct Rows {
@@ -597,7 +616,7 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 
   auto add_run = [&](PyObject* run) -> bool {
     if (Py_TYPE(run) != type[1]) return false;
-    Ref list(get(run, s__kernels)), ms(get(run, s__run_time_ms));
+    Ref list(field(run, s__kernels)), ms(field(run, s__run_time_ms));
     if (!list.p || !ms.p || (!PyList_Check(list.p) && !PyTuple_Check(list.p))) return false;
     const double wall = PyFloat_AsDouble(ms.p);
     if (PyErr_Occurred()) return false;
@@ -606,14 +625,13 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     for (Py_ssize_t i = 0; i < count; ++i) {
       PyObject* k = PySequence_Fast_GET_ITEM(list.p, i);
       if (Py_TYPE(k) != type[2]) return false;
-      Ref c(get(k, s__c));
+      Ref c(field(k, s__c));
       if (!c.p || Py_TYPE(c.p) != type[3]) return false;
       bool ok = true;
       const int64_t blocks = int_of(c.p, s__num_blocks, &ok), block = int_of(c.p, s__block_size, &ok),
                     regs = int_of(c.p, s__regs, &ok), time = int_of(c.p, s__run_time_ns, &ok),
                     stat = int_of(c.p, s__smem_static, &ok), dyn = int_of(c.p, s__smem_dynamic, &ok);
-      Ref name(get(c.p, s__name));
-      if (!ok || !name.p || blocks != static_cast<int32_t>(blocks)) return false;
+      if (!ok || blocks != static_cast<int32_t>(blocks)) return false;
       const int64_t smem = stat + dyn;
       nb.push_back(static_cast<int32_t>(blocks));
       bs.push_back(static_cast<uint16_t>(block < 0 ? 0 : (block > 0xFFFF ? 0xFFFF : block)));
@@ -621,17 +639,15 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
       sm.push_back(smem >= 0 && smem <= 0xFFFFFFFFll ? static_cast<uint32_t>(smem) : 0xFFFFFFFFu);
       tm.push_back(static_cast<float>(static_cast<double>(time)));
       busy += static_cast<double>(time);
-      if (PyList_Append(kernels.p, k) < 0 || PyList_Append(names.p, name.p) < 0) return false;
+      if (with_names) {
+        Ref name(field(c.p, s__name));
+        if (!name.p || PyList_Append(names.p, name.p) < 0) return false;
+      }
       if (with_metrics) {
-        Ref records(get(k, s__metrics_kernels)), cached(get(k, s__cached_metrics));
+        Ref records(field(k, s__metrics_kernels)), cached(field(k, s__cached_metrics));
         if (!records.p || !cached.p || !PyList_Check(records.p) || !PyDict_Check(cached.p)) return false;
         double v[3] = {0.0, 0.0, 0.0};
-        int found = PyList_GET_SIZE(records.p) > 0 || PyDict_GET_SIZE(cached.p) > 0 ? 1 : 0;
-        for (int m = 0; m < 3 && found == 1; ++m) {
-          PyObject* t = PyTuple_GET_ITEM(metrics, m);
-          found = find_metric(records.p, cached.p, PyTuple_GET_ITEM(t, 0), PyTuple_GET_ITEM(t, 1),
-                              PyTuple_GET_ITEM(t, 2), type[3], &v[m]);
-        }
+        const int found = find_metrics(records.p, cached.p, metrics, type[3], v);
         if (found < 0) return false;
         eff.push_back(found ? v[0] : 0.0);
         rd.push_back(found ? v[1] : 0.0);
@@ -644,13 +660,13 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     // launch overhead of a pass (predictor.py:113-116 of the reference): wall time minus kernel time
     const double rest = wall * 1e6 - busy;
     overhead.push_back(rest > 0.0 ? rest : 0.0);
-    return PyList_Append(runs.p, run) == 0;
+    return true;
   };
 
   for (Py_ssize_t i = 0; i < n; ++i) {
     PyObject* op = PySequence_Fast_GET_ITEM(ops.p, i);
     if (Py_TYPE(op) != type[0]) return not_ordinary();
-    Ref name(get(op, s__name)), device(get(op, s__device));
+    Ref name(field(op, s__name)), device(field(op, s__device));
     if (!name.p || !device.p) return not_ordinary();
     if (!first_device.p) {
       first_device.p = Py_NewRef(device.p);
@@ -661,7 +677,7 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const int is_special = PySet_Contains(special, name.p);
     if (is_special < 0) return not_ordinary();
     if (!is_special) {
-      Ref f(get(op, s__forward)), b(get(op, s__backward));
+      Ref f(field(op, s__forward)), b(field(op, s__backward));
       if (!f.p || !b.p) return not_ordinary();
       wave_idx.push_back(i);
       fwd.push_back(static_cast<int64_t>(overhead.size()));
@@ -767,7 +783,7 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   }
   for (Py_ssize_t k = 0; k < n_kinds; ++k) PyTuple_SET_ITEM(kinds_out.p, k, bytes_of(kind_idx[k]));
   if (PyErr_Occurred() || !soa.p || !off.p || !met.p) return nullptr;
-  return Py_BuildValue("(OOONNNNNOOOOOO)", kernels.p, runs.p, names.p, bytes_of(wave_idx), bytes_of(fwd), bytes_of(bwd),
+  return Py_BuildValue("(LLONNNNNOOOOOO)", static_cast<long long>(K), static_cast<long long>(overhead.size()), names.p, bytes_of(wave_idx), bytes_of(fwd), bytes_of(bwd),
                        bytes_of(offsets), bytes_of(overhead), kinds_out.p, passed.p, soa.p, met.p, off.p, special_rows.p);
   END_HANDLE_TH_ERRORS
 }
@@ -1144,7 +1160,7 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
                                           reinterpret_cast<float*>(h + h_times), s));
   };
   bool nan = false;
-  auto sort_waves = [&] {
+  auto sort_passes = [&] {
     if (!scale) return;
     const double* tot = reinterpret_cast<const double*>(h + h_totals);
     if (K == 0) std::memset(h + h_totals, 0, static_cast<size_t>(T) * n_runs * 8);
@@ -1162,6 +1178,19 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
         if (bw[i] >= 0) v += (over[bw[i]] + q[bw[i]]) / 1e6;
         out[wi[i]] = v;
       }
+    }
+  };
+  std::vector<double> sum_ms(static_cast<size_t>(T), 0.0);
+  auto sort_waves = [&] {
+    sort_passes();
+    // the rows' sums but for the predictors' operations, whose times come later
+    for (int64_t t = 0; t < T; ++t) {
+      double sum[4] = {0.0, 0.0, 0.0, 0.0};
+      double* row = ms.data() + t * n_ops;
+      for (const Kind& k : kinds)
+        for (int64_t j = 0; j < k.n; ++j) row[k.idx[j]] = 0.0;
+      for (int64_t i = 0; i < n_ops; ++i) sum[i & 3] += row[i];
+      sum_ms[t] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
     }
   };
 
@@ -1202,11 +1231,14 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     bool zero = false;
     for (int64_t t = 0; t < T; ++t) {
       double* out = ms.data() + t * n_ops;
+      double sum[4] = {0.0, 0.0, 0.0, 0.0};
       for (int64_t j = 0; j < k.n; ++j) {
-        const float x = v[t * k.n + j];
-        zero = zero || x == 0.0f;
-        out[k.idx[j]] = static_cast<double>(x);
+        const double x = static_cast<double>(v[t * k.n + j]);
+        zero = zero || x == 0.0;
+        out[k.idx[j]] = x;
+        sum[j & 3] += x;
       }
+      sum_ms[t] += (sum[0] + sum[1]) + (sum[2] + sum[3]);
     }
     PyObject* pred = Py_NewRef(Py_None);
     if (zero) {
@@ -1225,10 +1257,7 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   }
   Ref sums(PyList_New(static_cast<Py_ssize_t>(T)));
   for (int64_t t = 0; t < T; ++t) {
-    double sum[4] = {0.0, 0.0, 0.0, 0.0};
-    const double* q = ms.data() + t * n_ops;
-    for (int64_t i = 0; i < n_ops; ++i) sum[i & 3] += q[i];
-    PyList_SET_ITEM(sums.p, static_cast<Py_ssize_t>(t), PyFloat_FromDouble((sum[0] + sum[1]) + (sum[2] + sum[3])));
+    PyList_SET_ITEM(sums.p, static_cast<Py_ssize_t>(t), PyFloat_FromDouble(sum_ms[t]));
   }
   return Py_BuildValue("(NOO)", PyBool_FromLong(nan), sums.p, clamped.p);
   END_HANDLE_TH_ERRORS

@@ -171,3 +171,44 @@ def test_trace_to_device(device_file, tmp_path):
     assert not calls
     for pt, first in zip(again, many):
         assert pt.run_time_ms == first.run_time_ms
+
+
+def test_native_walk_over_metric_records(device_file):
+    """The native walk of a trace finds the metrics that MeasuredKernel.get_metric finds: equal names that are
+    other objects, legacy names, several records and entries (the first counts), cached values, one missing, none."""
+    from habitat_b200.analysis import predictor as pr
+    origin = device_file["V100"]
+    infos = [m.value for m in pr.wave_batch._NEEDED]
+    names, legacy = [i.cupti_name for i in infos], [i.legacy_cupti_name for i in infos]
+    other = ["".join(list(n)) for n in names]
+    layouts = [
+        [list(zip(names, (10.0, 1e6, 2e6)))], [list(zip(other, (11.0, 3e6, 4e6)))], [list(zip(legacy, (12.0, 5e6, 6e6)))],
+        [[("x", 1.0), (names[2], 7e6)], [(names[0], 13.0), (names[2], 9e9)], [(legacy[1], 8e6), (names[1], 9e9)]],
+        [[(names[0], 14.0), (names[1], 1e6)]], [[]], [],
+        [[(names[1], 2e6), (names[2], 3e6)]]]
+    runs = []
+    for i, records in enumerate(layouts):
+        parts = [KernelInstance("k%d" % i, 40 + i, 128, 0, 0, 32, 1000 * (i + 1), r) for r in records]
+        k = MeasuredKernel(parts[0] if parts else KernelInstance("k%d" % i, 7, 64, 0, 0, 16, 500), parts, origin)
+        runs.append(RunTimeMeasurement(0.25, [k], origin))
+    runs[7].kernels[0]._cached_metrics[pr.wave_batch._NEEDED[0]] = 15.0
+    runs.append(RunTimeMeasurement(0.5, [r.kernels[0] for r in runs[:3]], origin))
+    runs.append(RunTimeMeasurement(0.5, [], origin))
+    ops = [MeasuredOperation("relu", Arguments((), {}), runs[i], runs[i + 1] if i % 3 else None, origin)
+           for i in range(len(runs) - 1)]
+    for with_names in (True, False):
+        native = pr._GroupPlan.of_whole_trace(ops, "unified", with_names)
+        for i, op in enumerate(ops):
+            for run in (op.forward, op.backward):
+                for k in run.kernels if run is not None else ():
+                    if k is not runs[7].kernels[0]:
+                        k._cached_metrics.clear()
+        python = pr._GroupPlan(ops, range(len(ops)), "unified")
+        for a, b in ((native.flat.batch, python.flat.batch), (native.flat.metrics, python.flat.metrics)):
+            for f, plane in vars(a).items():
+                assert torch.equal(plane, getattr(b, f)), f
+        assert native.names == python.names and native.kernels == python.kernels
+        for f in ("offsets", "wave_idx", "fwd_run", "bwd_run"):
+            assert np.array_equal(getattr(native, f), getattr(python, f))
+        np.testing.assert_allclose(native.overheads, python.overheads, rtol=1e-12)
+        assert (native.n_kernels, native.n_runs) == (python.n_kernels, python.n_runs)
