@@ -897,7 +897,8 @@ namespace {
 class ChainLaunch {
  public:
   ChainLaunch(const hb_mlp* h, bool split) : split_(split), pairs_(h->sm_count / 2) { p_.phase_cycles = h->phase_cycles; }
-  int64_t tiles_of(int64_t Q) const { const int q = split_ ? kPairQ / 2 : kPairQ; return (Q + q - 1) / q; }
+  int tile_q() const { return split_ ? kPairQ / 2 : kPairQ; }
+  int64_t tiles_of(int64_t Q) const { return (Q + tile_q() - 1) / tile_q(); }
   // Rounds of tiles the SMs would walk with `more` tiles on top.
   int64_t rounds(int64_t more) const { return (p_.num_tiles + more + pairs_ - 1) / pairs_; }
   hb_status add(const hb_mlp* h, const hb::MlpBatch& batch) {
@@ -916,6 +917,18 @@ class ChainLaunch {
     q.tmap_slot = h->tmap_slot; q.tmap_tile = h->tmap_tile;
     p_.num_tiles += static_cast<int32_t>(tiles);
     return HB_OK;
+  }
+  // The queries at the end of the first batch without which the list has one round less (0: none).
+  int64_t tail() const {
+    const int64_t over = p_.num_tiles % pairs_, tiles = tiles_of(p_.prob[0].Q);
+    if (over == 0 || over == p_.num_tiles || over >= tiles) return 0;
+    return p_.prob[0].Q - (tiles - over) * tile_q();
+  }
+  void drop(int64_t queries) {
+    const int32_t tiles = static_cast<int32_t>(tiles_of(p_.prob[0].Q) - tiles_of(p_.prob[0].Q - queries));
+    p_.prob[0].Q -= queries;
+    p_.num_tiles -= tiles;
+    for (int i = 1; i < p_.n_problems; ++i) p_.prob[i].first_tile -= tiles;
   }
   hb_status go(bool beside, cudaStream_t s) {
     p_.beside = beside ? 1 : 0;
@@ -947,6 +960,25 @@ hb::WidePlan plan_of(const hb_mlp* h, int64_t Q) {
   return use_wide ? hb::wide_plan(Q, h->precision == HB_PRECISION_BF16X3, h->sm_count) : hb::WidePlan{0, 0, 0, 0};
 }
 
+// A last round of few tiles takes as long as a full one, and the kernel for small batches is quicker: it takes the
+// queries of that round from the first batch of the list (`batch`), the list follows beside it.  9,572 queries:
+// 220 -> 140 us, 28,916: 435 -> 378; split, 5,792: 376 -> 335.
+hb_status queue_tail(ChainLaunch* launch, hb_mlp* h, hb::MlpBatch batch, cudaStream_t s, int* launches) {
+  const int64_t n = launch->tail();
+  const hb::WidePlan plan = n ? plan_of(h, n) : hb::WidePlan{0, 0, 0, 0};
+  if (plan.G == 0) return HB_OK;
+  batch.first = batch.Q - n;
+  batch.Q = n;
+  batch.out += batch.first;
+  bool launched = false;
+  const hb_status st = hb::wide_predict(h, plan, batch, s, &launched);
+  if (st == HB_OK && launched) {
+    launch->drop(n);
+    ++*launches;
+  }
+  return st;
+}
+
 // Queues one batch (checked by the callers) on the kernel for its size.
 hb_status queue_batch(hb_mlp* h, const hb::WidePlan& plan, const hb::MlpBatch& batch, cudaStream_t s) {
   bool launched = false;
@@ -955,7 +987,9 @@ hb_status queue_batch(hb_mlp* h, const hb::WidePlan& plan, const hb::MlpBatch& b
   if (st != HB_OK || launched) return st;
   ChainLaunch launch(h, h->precision == HB_PRECISION_BF16X3);
   st = launch.add(h, batch);
-  return st != HB_OK ? st : launch.go(batch.beside, s);
+  int launches = 0;
+  if (st == HB_OK) st = queue_tail(&launch, h, batch, s, &launches);
+  return st != HB_OK ? st : launch.go(batch.beside || launches > 0, s);
 }
 }  // namespace
 
@@ -1042,7 +1076,8 @@ extern "C" hb_status hb_mlp_predict_grid(const hb_mlp_grid* items, int32_t n_ite
       st = launch.add(other, batches[o]);
       queued[o] = true;
     }
-    if (st == HB_OK) st = launch.go(batches[i].beside, static_cast<cudaStream_t>(stream));
+    if (st == HB_OK) st = queue_tail(&launch, h, batches[i], static_cast<cudaStream_t>(stream), &lane);
+    if (st == HB_OK) st = launch.go(lane > 1, static_cast<cudaStream_t>(stream));
     if (st != HB_OK) return st;
   }
   return HB_OK;

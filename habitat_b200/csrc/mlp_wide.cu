@@ -61,6 +61,7 @@ struct WideParams {
   uint32_t tag;               // of this launch
   unsigned long long parity[2];   // bit g: parity of the next use of group g's buffer 0, 1
   int32_t beside;             // runs beside the launch before it: nothing to wait for
+  int64_t first;              // of feats and dev_row
   int32_t grid_n;             // > 0: query q is feature row q % grid_n on device grid_rows[q / grid_n]
   uint8_t grid_rows[hb::kMaxGridRows];
   int32_t inline_q;           // > 0: the queries themselves, below, instead of feats and dev_row
@@ -434,7 +435,7 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     epi_sync();
     for (int i = T; i < n_q * C_in; i += 128) {
       const int q = i / C_in, f = i - q * C_in;
-      int64_t fr = q0 + q;
+      int64_t fr = p.first + q0 + q;
       int dr;
       if (p.grid_n) {
         const uint32_t block = static_cast<uint32_t>(fr) / static_cast<uint32_t>(p.grid_n);
@@ -823,8 +824,9 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
   p.per_group = w.per_group; p.out = batch.out;
   p.status = h->status;
   p.beside = batch.beside && !s->fresh ? 1 : 0;   // (a fresh buffer's clearing has to be waited for)
+  p.first = batch.first;
   p.grid_n = batch.grid_n;
-  if (batch.grid_n) std::memcpy(p.grid_rows, batch.grid_rows, batch.Q / batch.grid_n);
+  if (batch.grid_n) std::memcpy(p.grid_rows, batch.grid_rows, (batch.first + batch.Q) / batch.grid_n);
   if (batch.host_inputs) {
     p.inline_q = static_cast<int32_t>(batch.Q);
     std::memcpy(p.inline_feats, batch.feats, sizeof(float) * batch.Q * h->n_op_feat);

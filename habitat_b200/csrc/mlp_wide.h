@@ -21,6 +21,7 @@ struct MlpBatch {
   const float* feats = nullptr;
   const uint8_t* dev_row = nullptr;
   int64_t Q = 0;
+  int64_t first = 0;                 // the batch is queries first .. first + Q - 1 of feats, dev_row or the grid
   float* out = nullptr;
   bool host_inputs = false;          // feats and dev_row are ordinary host memory, Q <= kWideInline
   int32_t grid_n = 0;

@@ -335,3 +335,37 @@ def test_batches_side_by_side(sizes):
     for h, _, _ in keep:
         h.check_status()
         h.close()
+
+
+@pytest.mark.parametrize("precision,round_q,most", [("bf16", 9472, 2112), ("bf16x3", 4736, 1056)])
+def test_last_round_of_few_tiles(precision, round_q, most):
+    """Queries beyond full rounds of the two-SM kernel (74 tiles) go to the kernel for small batches while they fit
+    there: on both sides of that, one or two rounds, alone and as a grid with a second batch in the list, each
+    prediction has the bits it has in a small batch."""
+    import ctypes
+    from habitat_b200 import _native
+    n = 2 * round_q + 301
+    feats, dev = workloads.make_queries("bmm", n, 61)
+    mu, sigma = workloads.batch_mu_sigma(feats, dev)
+    h = batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=DEVF, precision=precision,
+                          **workloads.init_mlp_weights("bmm", seed=7, layers=3, gain=2.0))
+    f, r = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()
+    want = torch.cat([h.predict(f[i:i + 2000].contiguous(), r[i:i + 2000].contiguous()) for i in range(0, n, 2000)])
+    for q in (round_q, round_q + 1, round_q + most, round_q + most + 1, 2 * round_q, n):
+        for _ in range(2):
+            assert torch.equal(h.predict(f[:q].contiguous(), r[:q].contiguous()), want[:q]), q
+    # seven devices x m rows: the cut falls inside a device's rows; the second batch keeps its place in the list
+    m, small = (round_q + 900) // 7, (round_q // 4) // 3
+    rows = [bytes(range(6)) + b"\x02", b"\x01\x04\x03"]
+    items, outs = (_native.MlpGrid * 2)(), []
+    for i, k in enumerate((m, small)):
+        outs.append(torch.full((len(rows[i]) * k,), float("nan"), device="cuda"))
+        items[i] = _native.MlpGrid(h._handle.value, f.data_ptr(), k, ctypes.cast(ctypes.c_char_p(rows[i]), ctypes.c_void_p),
+                                   len(rows[i]), outs[i].data_ptr())
+    _native.check(_native.load().hb_mlp_predict_grid(items, 2, torch.cuda.current_stream().cuda_stream))
+    for k, out, devices in zip((m, small), outs, rows):
+        for b, d in enumerate(devices):
+            one = torch.full((k,), d, dtype=torch.uint8, device="cuda")
+            assert torch.equal(out[b * k:(b + 1) * k], h.predict(f[:k].contiguous(), one)), (k, b)
+    h.check_status()
+    h.close()
