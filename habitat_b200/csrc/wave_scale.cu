@@ -474,6 +474,14 @@ __device__ __forceinline__ Vec<T, VEC> load_pair(const T* q, bool pair) {
   }
   return v;
 }
+// The same without vector loads, for arrays of any alignment.
+template <typename T, int VEC>
+__device__ __forceinline__ Vec<T, VEC> load_each(const T* q, bool pair) {
+  Vec<T, VEC> v;
+  v.v[0] = q[0];
+  if (VEC == 2) v.v[VEC - 1] = pair ? q[VEC - 1] : q[0];
+  return v;
+}
 template <typename T, int VEC, bool ALIGNED>
 __device__ __forceinline__ void store_pair(T* q, const Vec<T, VEC>& v, bool pair) {
   if (VEC == 1 || ALIGNED) {
@@ -502,9 +510,9 @@ __device__ __forceinline__ void store_byte_pair(uint8_t* q, uint32_t pair_word, 
 constexpr int kTotMaxD = 16;
 
 // EXT: 0 plain, 1 with the status plane and per-destination registers, 2 and 3 with gamma from metrics as well,
-// whose float64 values take 20 registers.  With 56 registers (2) nine blocks fit an SM, with 48 (3) ten: the
-// batch that has more blocks than the first can hold at a time is 11 % faster with the second (4 M kernels x 6: 142
-// -> 127 us), a smaller one 6 % slower (250,001: 12.6 -> 13.4 us).
+// whose float64 values take 20 registers.  With 56 registers (2) nine blocks fit an SM, with 48 (3) ten: batches
+// of more than two fills of the first are 7 % faster with the second (4,000,000 kernels x 6: 117 -> 109 us),
+// smaller ones 5 to 15 % slower (500,000 x 6: 17.4 -> 18.2 us, 250,000 x 13: 21.0 -> 24.0).
 template <int VEC, int EXT, bool ALIGNED, int NW, int TOT = 0>
 __global__ void __launch_bounds__(kLutThreads, EXT == 2 ? 8 : (EXT == 3 ? 10 : 12))
 wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
@@ -533,6 +541,14 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
     const Vec<float, VEC> tv = load_pair<float, VEC, ALIGNED>(p.time_ns + k0, pair);
     Vec<float, VEC> gv;
     if (!with_metrics) gv = load_pair<float, VEC, ALIGNED>(p.gamma + k0, pair);
+    Vec<double, VEC> fev, rdv, wrv;
+    Vec<uint8_t, VEC> hmv;
+    if (with_metrics) {   // all on their way at once, not the values behind the flag (4,000,000 x 6: 117 -> 109 us)
+      hmv = load_each<uint8_t, VEC>(p.has_metrics + k0, pair);
+      fev = load_each<double, VEC>(p.flop_eff + k0, pair);
+      rdv = load_each<double, VEC>(p.dram_read + k0, pair);
+      wrv = load_each<double, VEC>(p.dram_write + k0, pair);
+    }
 
     uint32_t P[2] = {0u, 0u}, S[2] = {0u, 0u};     // class bytes of the two records
     uint32_t P2[2] = {0u, 0u}, S2[2] = {0u, 0u};   // ... of the launch's second word
@@ -565,14 +581,14 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
       if (with_metrics) {
         // wave_scaling/roofline.py:68-92, float64.  The rule below gives gamma 1 for intensity 0 and gamma 0
         // for an infinite one, which is how its two special cases are written here: no metrics or next to no
-        // floating-point work, and no memory traffic.
-        const uint32_t ki = (i == 0 || pair) ? k0 + i : k0;   // the tail thread's second slot repeats the first
-        if (p.has_metrics[ki]) {
-          const double total_gb = (p.dram_read[ki] + p.dram_write[ki]) / 1024 / 1024 / 1024;
-          const double gf = p.flop_eff[ki] * (lp.origin_peak / 100 / 1e9) * static_cast<double>(tv.v[i]);
+        // floating-point work, and no memory traffic.  Reciprocals, not divisions: two of those per record were
+        // 15 % of the kernel.
+        if (hmv.v[i]) {
+          const double total_gb = (rdv.v[i] + wrv.v[i]) / 1024 / 1024 / 1024;
+          const double gf = fev.v[i] * (lp.origin_peak / 100 / 1e9) * static_cast<double>(tv.v[i]);
           if (!(gf < 1e-9)) {
-            xint[i] = total_gb == 0 ? __longlong_as_double(0x7FF0000000000000ll) : gf / total_gb;
-            xinv[i] = total_gb == 0 ? 0.0 : total_gb / gf;
+            xint[i] = total_gb == 0 ? __longlong_as_double(0x7FF0000000000000ll) : gf * __drcp_rn(total_gb);
+            xinv[i] = total_gb == 0 ? 0.0 : total_gb * __drcp_rn(gf);
           }
         }
       }
@@ -681,7 +697,8 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
         wavv.v[i] = (nbok[i] && has_wave) ? q : 0xFFFFFFFFu;
         // roofline.py:29-30 with its short circuit: the destination is only looked at when the
         // kernel fits in one origin wave
-        const bool small = fits_o[i] && has_wave && q == 0u;
+        // (the two forms say the same; which one schedules better differs: 1 to 2 % either way)
+        const bool small = fits_o[i] && (EXT ? has_wave && q == 0u : wavv.v[i] == 0u);
         const bool ok = live[i] && !(fits_o[i] && !has_wave);
         // blocks per SM on the destination: meaningful (and <= occupancy) when `small`; computed from
         // the record alone so that this table load does not wait for the one above
@@ -957,7 +974,7 @@ bool try_launch_lut(const Ptrs& p, const LaunchPlan& plan, int64_t K, int64_t st
   if (ext) {
     auto launch_ext = [&](auto words) {
       constexpr int W = decltype(words)::value;
-      if (metrics && vec2 && blocks > 9ll * sm_count)
+      if (metrics && vec2 && blocks > 18ll * sm_count)
         return aligned ? launch_lut<2, 3, true, W>(grid, stream, p, q) : launch_lut<2, 3, false, W>(grid, stream, p, q);
       if (metrics)
         return !vec2 ? launch_lut<1, 2, true, W>(grid, stream, p, q)
