@@ -630,6 +630,17 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
     store_byte_pair<VEC, ALIGNED>(p.origin_occ + k0, o2, pair);
     store_pair<uint32_t, VEC, ALIGNED>(p.origin_waves + k0, owav, pair);
 
+    // The plain instances keep what they know about a record in masks: six predicates that live through the loop
+    // leave none for the body, and the masks go into one logic operation per question (11,184,812 x 6 with totals:
+    // 184 -> 174 us, 8,388,608 x 6: 122 -> 116).
+    uint32_t no_blocks[2], not_live[2], not_fit[2];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+      no_blocks[i] = nbok[i] ? 0u : ~0u;
+      not_live[i] = live[i] ? 0u : ~0u;
+      not_fit[i] = fits_o[i] ? 0u : ~0u;
+    }
+
     // per-destination register counts of the two records (-1: the record's own)
     auto load_regs = [&](uint32_t at) {
       Vec<int16_t, VEC> r;
@@ -694,12 +705,19 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
         const uint2 w = __ldg(reinterpret_cast<const uint2*>(tab_m + (dd.sel.z + HB_IDX(occ, kLutOcc, 6) * 8u)));
         const uint32_t q = __umulhi(static_cast<uint32_t>(nb), w.x) >> w.y;
         const bool has_wave = occ != 0u;
-        wavv.v[i] = (nbok[i] && has_wave) ? q : 0xFFFFFFFFu;
         // roofline.py:29-30 with its short circuit: the destination is only looked at when the
         // kernel fits in one origin wave
-        // (the two forms say the same; which one schedules better differs: 1 to 2 % either way)
-        const bool small = fits_o[i] && (EXT ? has_wave && q == 0u : wavv.v[i] == 0u);
-        const bool ok = live[i] && !(fits_o[i] && !has_wave);
+        bool small, ok;
+        if (EXT) {
+          wavv.v[i] = (nbok[i] && has_wave) ? q : 0xFFFFFFFFu;
+          small = fits_o[i] && has_wave && q == 0u;
+          ok = live[i] && !(fits_o[i] && !has_wave);
+        } else {
+          const uint32_t waves = (has_wave ? q : 0xFFFFFFFFu) | no_blocks[i];
+          wavv.v[i] = waves;
+          small = (waves | not_fit[i]) == 0u;
+          ok = (~not_live[i] & (~waves | not_fit[i])) != 0u;
+        }
         // blocks per SM on the destination: meaningful (and <= occupancy) when `small`; computed from
         // the record alone so that this table load does not wait for the one above
         const uint32_t dm = min(__umulhi(static_cast<uint32_t>(nb) + dd.sm.x, dd.sm.y), static_cast<uint32_t>(kLutOcc - 1));
