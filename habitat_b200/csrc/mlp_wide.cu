@@ -435,17 +435,19 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     epi_sync();
     for (int i = T; i < n_q * C_in; i += 128) {
       const int q = i / C_in, f = i - q * C_in;
-      int64_t fr = p.first + q0 + q;
+      const int own = static_cast<int>(q0) + q;                 // of the launch's queries
+      int64_t fr = p.first + own;
       int dr;
       if (p.grid_n) {
         const uint32_t block = static_cast<uint32_t>(fr) / static_cast<uint32_t>(p.grid_n);
         fr -= static_cast<int64_t>(block) * p.grid_n;
         dr = p.grid_rows[block];
       } else {
-        dr = p.inline_q ? p.inline_row[q] : p.dev_row[fr];
+        dr = p.inline_q ? p.inline_row[own] : p.dev_row[fr];
       }
       dr = dr < p.n_dev ? dr : p.n_dev - 1;
-      const double x = f < p.n_op_feat ? static_cast<double>(p.inline_q ? p.inline_feats[i - 4 * q] : p.feats[fr * p.n_op_feat + f])
+      const double x = f < p.n_op_feat ? static_cast<double>(p.inline_q ? p.inline_feats[own * p.n_op_feat + f]
+                                                                             : p.feats[fr * p.n_op_feat + f])
                                        : p.dev_feat[dr * 4 + (f - p.n_op_feat)];
       const float xn = static_cast<float>((x - p.mu[f]) / p.sigma[f]);
       const __nv_bfloat16 hi = __float2bfloat16_rn(xn);

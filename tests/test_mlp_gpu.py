@@ -369,3 +369,24 @@ def test_last_round_of_few_tiles(precision, round_q, most):
             assert torch.equal(out[b * k:(b + 1) * k], h.predict(f[:k].contiguous(), one)), (k, b)
     h.check_status()
     h.close()
+
+
+@pytest.mark.parametrize("precision", ["bf16", "bf16x3"])
+@pytest.mark.parametrize("op", ["conv2d", "bmm"])
+def test_few_host_queries(op, precision):
+    """Up to 16 queries from host memory travel as kernel parameters, in split precision more than eight of them to
+    two groups: every count on both sides of that, each query different, has the bits of the device entry point."""
+    feats, dev = workloads.make_queries(op, 64, 71)
+    mu, sigma = workloads.batch_mu_sigma(feats, dev)
+    h = batched.MLPHandle(feats.shape[1], mu=mu, sigma=sigma, device_features=DEVF, precision=precision,
+                          **workloads.init_mlp_weights(op, seed=3, layers=3, gain=2.0))
+    want = h.predict(torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()).cpu().numpy()
+    assert len(set(want.tolist())) > 48
+    for Q in range(1, 18):
+        lo = 3 * Q
+        if lo + Q > 64:
+            lo = 64 - Q
+        assert np.array_equal(h.predict_host(feats[lo:lo + Q], dev[lo:lo + Q]), want[lo:lo + Q]), Q
+    for q in (0, 9, 63):
+        assert h.predict_one(feats[q].tolist(), int(dev[q])) == want[q]
+    h.close()
