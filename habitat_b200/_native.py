@@ -196,13 +196,13 @@ def binding():
             "habitat_b200: %s is missing. Build it with `python -m habitat_b200.build`; there is no "
             "fallback." % path)
     import torch  # noqa: F401  (its shared libraries first)
-    from habitat_b200 import batched, device_table
+    from habitat_b200 import batched, device_table, habitat_cuda
     loader = importlib.machinery.ExtensionFileLoader("habitat_b200._binding", path)
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader("habitat_b200._binding", loader))
     loader.exec_module(module)
     lib = load()
     module.setup({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in EXPORTS},
-                 device_table.row_of, check, batched.WaveResult)
+                 device_table.row_of, check, batched.WaveResult, habitat_cuda.DeviceProperties)
     module.set_generation(device_table.generation())
     atexit.register(module.release_host_blocks)
     _binding = module

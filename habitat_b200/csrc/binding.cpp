@@ -49,6 +49,7 @@ struct Api {
 PyObject* g_row_of = nullptr;       // device_table.row_of
 PyObject* g_raise = nullptr;        // _native.check
 PyObject* g_wave_result = nullptr;  // batched.WaveResult
+PyObject* g_device_type = nullptr;  // habitat_cuda.DeviceProperties
 long g_generation = 0;              // of the device table; tokens of an older one are looked up again
 
 PyObject *s_num_blocks, *s_block_size, *s_regs, *s_smem, *s_time, *s_gamma, *s_row_token, *s_flop, *s_rd, *s_wr,
@@ -86,15 +87,17 @@ struct Field {
   void* ptr() const { return data(t); }
 };
 
-// Row of a DeviceProperties in the library's table: its token (generation * 64 + row) when it is of the
+// Row of a device in the library's table: a DeviceProperties' token (generation * 64 + row) when it is of the
 // current table, else device_table.row_of.  -1 with a Python error set when that fails.
 long row_of(PyObject* device) {
-  Ref token(PyObject_GetAttr(device, s_row_token));
-  if (token.p && PyLong_Check(token.p)) {
-    const long v = PyLong_AsLong(token.p);
-    if (v >= 0 && v / HB_MAX_DEVICES == g_generation) return v % HB_MAX_DEVICES;
+  if (reinterpret_cast<PyObject*>(Py_TYPE(device)) == g_device_type) {
+    Ref token(PyObject_GetAttr(device, s_row_token));
+    if (token.p && PyLong_Check(token.p)) {
+      const long v = PyLong_AsLong(token.p);
+      if (v >= 0 && v / HB_MAX_DEVICES == g_generation) return v % HB_MAX_DEVICES;
+    }
+    PyErr_Clear();
   }
-  PyErr_Clear();
   Ref row(PyObject_CallOneArg(g_row_of, device));
   if (!row.p) return -1;
   return PyLong_AsLong(row.p);
@@ -1319,10 +1322,10 @@ PyObject* iteration_totals(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   END_HANDLE_TH_ERRORS
 }
 
-// setup(addresses by name, row_of, check, WaveResult)
+// setup(addresses by name, row_of, check, WaveResult, DeviceProperties)
 PyObject* setup(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 4 || !PyDict_Check(a[0])) {
-    PyErr_SetString(PyExc_TypeError, "setup(addresses, row_of, check, WaveResult)");
+  if (n != 5 || !PyDict_Check(a[0])) {
+    PyErr_SetString(PyExc_TypeError, "setup(addresses, row_of, check, WaveResult, DeviceProperties)");
     return nullptr;
   }
   auto load = [&](auto& fn, const char* name) {
@@ -1345,6 +1348,7 @@ PyObject* setup(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Py_XSETREF(g_row_of, Py_NewRef(a[1]));
   Py_XSETREF(g_raise, Py_NewRef(a[2]));
   Py_XSETREF(g_wave_result, Py_NewRef(a[3]));
+  Py_XSETREF(g_device_type, Py_NewRef(a[4]));
   Py_RETURN_NONE;
 }
 

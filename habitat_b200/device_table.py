@@ -58,7 +58,8 @@ def _sync():
 
 def row_of(device):
     """Row index of a DeviceProperties in the library's table (uploading if new).  The device
-    remembers its row (`_row_token`), which is where the native binding looks first."""
+    remembers its row (`_row_token`), which is where the native binding looks first; an object of
+    another class, whose values may change, is looked up by them each time."""
     spec = device.spec_tuple()
     row = _index.get(spec)
     if row is None:
@@ -68,10 +69,8 @@ def row_of(device):
         _rows.append(spec)
         _index[spec] = row
     _sync()
-    try:
+    if type(device) is DeviceProperties:
         device._row_token = _generation * _native.HB_MAX_DEVICES + row
-    except AttributeError:
-        pass        # an object of another class that takes no attributes
     return row
 
 

@@ -9,6 +9,7 @@ reference's bindings keeps working.  Two differences:
     reference runs NVIDIA's occupancy header on the host.
 """
 import ctypes
+import types
 
 from habitat_b200 import _native
 
@@ -39,7 +40,19 @@ class DeviceProperties:
         for key, value in values.items():
             if int(value) != value:
                 raise TypeError("%s must be an integer, got %r" % (key, value))
-        self._fields = {k: int(v) for k, v in values.items()}
+        # read-only: device_table.row_of leaves the row of these values on the object
+        self._fields = types.MappingProxyType({k: int(v) for k, v in values.items()})
+
+    # The remembered row is one of this process's table: it stays out of pickles and copies, and out of
+    # objects whose pickle holds one.
+    def __getstate__(self):
+        state = dict(self.__dict__, _fields=dict(self._fields))
+        state.pop("_row_token", None)
+        return state
+
+    def __setstate__(self, state):
+        self.__dict__.update(state, _fields=types.MappingProxyType(dict(state["_fields"])))
+        self.__dict__.pop("_row_token", None)
 
     def __repr__(self):
         return "DeviceProperties(name=" + self._name + ")"
