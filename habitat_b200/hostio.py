@@ -151,8 +151,6 @@ class WaveScaleHost(_Streams):
             if self.want_totals:
                 for h in self.host_out:
                     h["totals"] = torch.zeros((D,), dtype=torch.float64).pin_memory()
-        self._downloads = [[(t, self.dev_totals[i] if k == "totals" else getattr(self.dev_out[i], k))
-                            for k, t in h.items()] for i, h in enumerate(self.host_out)]
         self.h2d_bytes = K * RECORD_BYTES
         self.d2h_bytes = sum(t.numel() * t.element_size() for t in self.host_out[0].values())
 
@@ -160,12 +158,21 @@ class WaveScaleHost(_Streams):
         if block.numel() != self.K * RECORD_BYTES or block.dtype != torch.uint8:
             raise ValueError("block must be a uint8 tensor of K * %d bytes (pack_kernels)" % RECORD_BYTES)
         with_totals = self.want_totals
+        # what host_out holds now: a caller may have put other tensors there
+        downloads = [(t, self.dev_totals[slot] if k == "totals" else getattr(self.dev_out[slot], k))
+                     for k, t in self.host_out[slot].items()]
+        plain = all(t.dtype is d.dtype and t.shape == d.shape and t.is_contiguous() for t, d in downloads)
         res = _native.binding().submit_wave(
             block.contiguous(), self.dev_block[slot], self.dev_in[slot], self.origin, self.dests, self.dev_out[slot],
             self.partials[slot] if with_totals else None, self.dev_totals[slot] if with_totals else None,
-            self._downloads[slot], self._stream_handles, self._event_handles[slot], self.used[slot])
+            downloads if plain else [], self._stream_handles, self._event_handles[slot], self.used[slot])
         if res is None:
             raise ValueError("wave_scale: unsupported arguments (at most %d destinations)" % _native.HB_MAX_DEVICES)
+        if not plain:       # another type or layout: not a copy of bytes
+            with torch.cuda.stream(self.s_out):
+                for t, d in downloads:
+                    t.copy_(d, non_blocking=True)
+                self.downloaded[slot].record(self.s_out)
         self.used[slot] = True
 
 

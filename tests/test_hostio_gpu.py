@@ -85,3 +85,23 @@ def test_mlp_pipeline():
         assert torch.equal(pipe.host_out[slot][:Q], want)
     h.check_status()
     h.close()
+
+
+def test_wave_scale_pipeline_into_other_tensors(bench_devices):
+    """Results go to what host_out holds when a batch is submitted: another pinned tensor, one of another type,
+    a strided one, a plane that was not asked for at first."""
+    K, D = 3001, len(bench_devices)
+    block = hostio.pack_kernels(workloads.make_kernels(K, seed=310))
+    pipe = hostio.WaveScaleHost(bench_devices[0], bench_devices, K, depth=1, results=("scaled_ns",))
+    pipe.submit(block, 0)
+    pipe.wait(0)
+    want, first = pipe.host_out[0]["scaled_ns"].clone(), pipe.host_out[0]["scaled_ns"]
+    for other in (torch.zeros((D, K)).pin_memory(), torch.zeros((D, K), dtype=torch.float64),
+                  torch.zeros((K, D)).pin_memory().t()):
+        first.fill_(-1.0)
+        pipe.host_out[0] = {"scaled_ns": other, "origin_occupancy": torch.zeros((K,), dtype=torch.uint8).pin_memory()}
+        pipe.submit(block, 0)
+        pipe.wait(0)
+        torch.testing.assert_close(pipe.host_out[0]["scaled_ns"].float(), want, rtol=0, atol=0, equal_nan=True)
+        assert torch.equal(pipe.host_out[0]["origin_occupancy"], pipe.dev_out[0].origin_occupancy.cpu())
+        assert bool((first == -1.0).all())
