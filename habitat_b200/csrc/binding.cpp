@@ -1278,6 +1278,8 @@ PyObject* iteration_totals(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   const int64_t K = tm.t->numel(), I = off->numel() - 1, D = PyBytes_GET_SIZE(a[4]);
   if (over->numel() != K || scaled->numel() != D * K) return not_ordinary();
   const uint8_t* same = reinterpret_cast<const uint8_t*>(PyBytes_AS_STRING(a[4]));
+  int64_t others = 0;   // destinations that the kinds are predicted for
+  for (int64_t d = 0; d < D; ++d) others += same[d] == 0;
   struct Kind { hb_mlp* h; const at::Tensor *f, *ms, *off; const uint8_t* rows; int64_t blocks; };
   std::vector<Kind> kinds;
   int64_t floats = 0;
@@ -1287,7 +1289,8 @@ PyObject* iteration_totals(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
            tensor(PyTuple_GET_ITEM(t, 2), at::kFloat), tensor(PyTuple_GET_ITEM(t, 3), at::kLong),
            reinterpret_cast<const uint8_t*>(PyBytes_AS_STRING(PyTuple_GET_ITEM(t, 4))),
            PyBytes_GET_SIZE(PyTuple_GET_ITEM(t, 4))};
-    if (!k.f || !k.ms || !k.off || k.f->dim() != 2 || k.ms->numel() != k.f->size(0) || k.off->numel() != I + 1)
+    if (!k.f || !k.ms || !k.off || k.f->dim() != 2 || k.ms->numel() != k.f->size(0) || k.off->numel() != I + 1 ||
+        k.blocks != 1 + others)
       return not_ordinary();
     kinds.push_back(k);
     if (k.blocks > 1) floats += (k.blocks * k.f->size(0) + 63) & ~int64_t{63};

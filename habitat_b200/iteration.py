@@ -39,11 +39,18 @@ def predict_iteration_totals(kernels: batched.KernelBatch, overhead_ns: torch.Te
 
     A destination with the origin's name keeps the measured times, as
     MeasuredOperation.to_device does (analysis/operation.py:82-85)."""
-    res = batched.wave_scale(kernels, origin, dests)
     same = bytes(d.name == origin.name for d in dests)
     rows = bytes([origin_mlp_row] + [r for r, s in zip(dest_mlp_rows, same) if not s])
-    kinds = [(ops.handle._handle.value or 0, ops.features, ops.run_time_ms, ops.offsets, rows)
-             for ops in special.values() if ops.features.shape[0]]
+    if len(rows) != 1 + same.count(0):
+        raise ValueError("dest_mlp_rows must have an entry per destination")
+    kinds = []
+    for ops in special.values():
+        if ops.features.shape[0] == 0:
+            continue
+        if ops.features.ndim != 2 or (len(rows) > 1 and ops.features.shape[1] != ops.handle.n_op_features):
+            raise ValueError("op_features must be [Q, %d]" % ops.handle.n_op_features)
+        kinds.append((ops.handle._handle.value or 0, ops.features, ops.run_time_ms, ops.offsets, rows))
+    res = batched.wave_scale(kernels, origin, dests)
     totals = _native.binding().iteration_totals(kernels, res.scaled_ns, overhead_ns, kernel_offsets, same, kinds)
     if totals is None:
         batched._require_cuda(overhead_ns, torch.float32, "overhead_ns")
