@@ -1276,7 +1276,7 @@ PyObject* iteration_totals(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   const at::Tensor *scaled = tensor(a[1], at::kFloat), *over = tensor(a[2], at::kFloat), *off = tensor(a[3], at::kLong);
   if (!tm.t || !scaled || !over || !off || off->numel() < 1) return not_ordinary();
   const int64_t K = tm.t->numel(), I = off->numel() - 1, D = PyBytes_GET_SIZE(a[4]);
-  if (over->numel() != K || scaled->numel() != D * K) return not_ordinary();
+  if (over->numel() < K || scaled->numel() != D * K) return not_ordinary();
   const uint8_t* same = reinterpret_cast<const uint8_t*>(PyBytes_AS_STRING(a[4]));
   int64_t others = 0;   // destinations that the kinds are predicted for
   for (int64_t d = 0; d < D; ++d) others += same[d] == 0;

@@ -49,14 +49,14 @@ def predict_iteration_totals(kernels: batched.KernelBatch, overhead_ns: torch.Te
             continue
         if ops.features.ndim != 2 or (len(rows) > 1 and ops.features.shape[1] != ops.handle.n_op_features):
             raise ValueError("op_features must be [Q, %d]" % ops.handle.n_op_features)
-        kinds.append((ops.handle._handle.value or 0, ops.features, ops.run_time_ms, ops.offsets, rows))
+        kinds.append((ops.handle._handle.value or 0, ops.features.contiguous(), ops.run_time_ms, ops.offsets, rows))
     res = batched.wave_scale(kernels, origin, dests)
     totals = _native.binding().iteration_totals(kernels, res.scaled_ns, overhead_ns, kernel_offsets, same, kinds)
     if totals is None:
         batched._require_cuda(overhead_ns, torch.float32, "overhead_ns")
         batched._require_cuda(kernel_offsets, torch.int64, "kernel_offsets")
         for ops in special.values():
-            batched._require_cuda(ops.features, torch.float32, "features")
+            batched._require_cuda(ops.features.contiguous(), torch.float32, "features")
             batched._require_cuda(ops.run_time_ms, torch.float32, "run_time_ms")
             batched._require_cuda(ops.offsets, torch.int64, "offsets")
         raise ValueError("overheads, features, measured times and offsets have to fit the kernels and iterations")

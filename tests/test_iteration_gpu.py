@@ -80,3 +80,28 @@ def test_iteration_totals(bench_devices, I):
     assert np.abs(got - want).max() <= 2e-2 * np.abs(want).min()
     assert np.abs(got[:, 0] - want[:, 0]).max() <= 1e-6 * want[:, 0].max()   # identity column
     print("config-4 style totals, max rel err %.3g" % (np.abs(got - want) / want).max())
+
+
+def test_strided_features_and_longer_overheads(bench_devices):
+    """Features of any layout and overheads beyond the kernels are taken; the totals are those of plain arrays."""
+    I, origin, dests = 3, bench_devices[0], bench_devices
+    kernels, overhead, ops = _make(I, 77, origin.spec_tuple())
+    feats, rt = ops["bmm"]
+    mu, sigma = workloads.batch_mu_sigma(feats, np.tile(np.arange(6, dtype=np.uint8), len(feats))[:len(feats)])
+    h = batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=workloads.BENCH_DEVICE_FEATURES,
+                          **workloads.torch_init_mlp_weights("bmm"))
+    off = torch.arange(I + 1, device="cuda") * PER_ITER["bmm"]
+    koff = torch.arange(I + 1, device="cuda") * KERNELS_PER_ITER
+    f = torch.from_numpy(feats).cuda()
+    over = torch.from_numpy(overhead).cuda()
+
+    def totals(features, overheads):
+        special = {"bmm": iteration.SpecialOps(h, features, torch.from_numpy(rt).cuda(), off)}
+        return iteration.predict_iteration_totals(batched.KernelBatch.from_numpy(kernels), overheads, koff, special,
+                                                  origin, dests, 0, list(range(6)))[0]
+    want = totals(f, over)
+    strided = f.t().contiguous().t()
+    assert not strided.is_contiguous()
+    assert torch.equal(totals(strided, over), want)
+    assert torch.equal(totals(f, torch.cat([over, torch.full((5,), float("nan"), device="cuda")])), want)
+    h.close()
