@@ -979,7 +979,7 @@ hb_status queue_tail(ChainLaunch* launch, hb_mlp* h, hb::MlpBatch batch, cudaStr
   return st;
 }
 
-// Queues one batch (checked by the callers) on the kernel for its size.
+// Queues one batch (checked by the callers) on the kernel for its size.  Call under wide_queue.
 hb_status queue_batch(hb_mlp* h, const hb::WidePlan& plan, const hb::MlpBatch& batch, cudaStream_t s) {
   bool launched = false;
   hb_status st = check_device(h);
@@ -1002,6 +1002,7 @@ extern "C" hb_status hb_mlp_predict(hb_mlp* h, const float* op_features, const u
   if (Q == 0) return HB_OK;
   hb::MlpBatch batch;
   batch.feats = op_features; batch.dev_row = device_row; batch.Q = Q; batch.out = out;
+  const auto queue = hb::wide_queue(h->device);
   return queue_batch(h, plan_of(h, Q), batch, static_cast<cudaStream_t>(stream));
 }
 
@@ -1051,6 +1052,8 @@ extern "C" hb_status hb_mlp_predict_grid(const hb_mlp_grid* items, int32_t n_ite
     split[some] = items[i].handle->precision == HB_PRECISION_BF16X3;
     all_wide = all_wide && plans[some].G != 0;
   }
+  if (some == 0) return HB_OK;
+  const auto queue = hb::wide_queue(items[order[0]].handle->device);   // the current device, as are the others'
   if (all_wide && some > 1) hb::wide_plans_together(plans, sizes, split, some, items[order[0]].handle->sm_count);
   int lane = 0;
   for (int k = 0; k < some; ++k) {
@@ -1169,6 +1172,7 @@ extern "C" hb_status hb_mlp_predict_host(hb_mlp* h, const float* op_features,
       hb::MlpBatch batch;
       batch.feats = op_features; batch.dev_row = device_row; batch.Q = Q; batch.out = p_o;
       batch.host_inputs = true;
+      const auto queue = hb::wide_queue(h->device);
       st = hb::wide_predict(h, plan, batch, s, &launched);
       if (st != HB_OK) return st;
     }

@@ -811,12 +811,16 @@ void wide_start_over(int device) {
   for (int i = 0; i < g.used; ++i) g.s[i].fresh = true;
 }
 
+std::unique_lock<std::mutex> wide_queue(int device) {
+  if (device < 0 || device >= kMaxCudaDevices) return {};   // wide_predict launches nothing there
+  return std::unique_lock<std::mutex>(g_wide[device].mu);
+}
+
 hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cudaStream_t stream, bool* launched) {
   *launched = false;
   if (w.G == 0 || h->device >= kMaxCudaDevices || (batch.host_inputs && batch.Q > kWideInline)) return HB_OK;
-  GpuScratch& g = g_wide[h->device];
-  std::lock_guard<std::mutex> lock(g.mu);   // held over the launch: parities and tags follow the stream's order
-  StreamScratch* s = scratch_of(g, stream, batch.lane);
+  // parities and tags follow the stream's order: the caller holds the queue's lock
+  StreamScratch* s = scratch_of(g_wide[h->device], stream, batch.lane);
   if (!s) return HB_OK;
   const bool split = h->precision == HB_PRECISION_BF16X3;
   WideParams p{};

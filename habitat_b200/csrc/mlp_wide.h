@@ -1,6 +1,8 @@
 // Host interface of the kernel for batches that do not fill the GPU (mlp_wide.cu).
 #pragma once
 
+#include <mutex>
+
 #include "hb_common.h"
 
 struct hb_mlp;
@@ -34,7 +36,11 @@ struct MlpBatch {
 constexpr int kMaxLanes = 4;
 // Replaces the plans of n <= kMaxLanes batches that are launched side by side, where others finish sooner.
 void wide_plans_together(WidePlan* plans, const int64_t* Q, const bool* split, int n, int sm_count);
-// Queues the launch; *launched stays false when the stream has no scratch (see there).
+// One call's launches on `device` follow one another on their stream: the caller holds this from the first to the
+// last of them.  A launch that runs beside the one before it relies on what its own call has queued; another
+// thread's launch in between, on the same stream, could still be using the lane's scratch.
+std::unique_lock<std::mutex> wide_queue(int device);
+// Queues the launch; *launched stays false when the stream has no scratch (see there).  Call under wide_queue.
 hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cudaStream_t stream, bool* launched);
 // After a launch that gave up: every stream's scratch on the GPU is set up again before its next use.
 void wide_start_over(int device);

@@ -390,3 +390,58 @@ def test_few_host_queries(op, precision):
     for q in (0, 9, 63):
         assert h.predict_one(feats[q].tolist(), int(dev[q])) == want[q]
     h.close()
+
+
+def test_two_threads_with_batches_side_by_side_on_one_stream():
+    """Calls of two threads on one stream, each with launches that run side by side or with a last round of its own:
+    the launches of a call stay together, so that every call has the bits it has alone."""
+    import ctypes
+    import threading
+    from habitat_b200 import _native
+    lib, stream = _native.load(), torch.cuda.current_stream().cuda_stream
+    n, devices = (53, 32, 9), 6
+    feats, dev = workloads.make_queries("bmm", 9900, 81)
+    mu, sigma = workloads.batch_mu_sigma(feats, dev)
+    hs = [batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=DEVF, **workloads.init_mlp_weights(
+        "bmm", seed=s, layers=4, gain=2.0)) for s in range(3)]
+    f, r = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()
+    rows = bytes(range(devices))
+    calls = 60
+    outs = [[[torch.full((devices * k,), float("nan"), device="cuda") for k in n] for _ in range(calls)] for _ in range(2)]
+    tails = [[torch.full((9900,), float("nan"), device="cuda") for _ in range(calls // 10)] for _ in range(2)]
+    errors = []
+
+    def grid(mine):
+        items = (_native.MlpGrid * 3)()
+        for i in range(3):
+            items[i] = _native.MlpGrid(hs[i]._handle.value, f.data_ptr(), n[i],
+                                       ctypes.cast(ctypes.c_char_p(rows), ctypes.c_void_p), devices, mine[i].data_ptr())
+        return lib.hb_mlp_predict_grid(items, 3, stream)
+
+    def work(t):
+        for c in range(calls):
+            errors.append(grid(outs[t][c]))
+            if c % 10 == t:
+                errors.append(lib.hb_mlp_predict(hs[t]._handle, ctypes.c_void_p(f.data_ptr()), ctypes.c_void_p(r.data_ptr()),
+                                                 9900, ctypes.c_void_p(tails[t][c // 10].data_ptr()), stream))
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not any(errors)
+    for i in range(3):
+        each = torch.arange(devices, device="cuda").to(torch.uint8).repeat_interleave(n[i])
+        want = hs[i].predict(f[:n[i]].repeat(devices, 1).contiguous(), each)
+        for t in range(2):
+            for c in range(calls):
+                assert torch.equal(outs[t][c][i], want), (t, c, i)
+    for t in range(2):
+        want = hs[t].predict(f, r)
+        for out in tails[t]:
+            assert torch.equal(out, want), t
+    for h in hs:
+        h.check_status()
+        h.close()
