@@ -37,7 +37,7 @@
 // weight producers.  Bulk copies issued by one thread complete one after the other (measured:
 // about 750 cycles each whatever their size), so each ring slot has its own issuing warp.
 // Every mbarrier wait is bounded: when a wait runs out the kernel records a status word, all
-// roles leave their loops, outstanding bulk copies are waited for (bounded) and TMEM is released.
+// roles leave their loops, outstanding bulk copies and MMAs are waited for (bounded) and TMEM is released.
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -180,6 +180,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_ptr + 272);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + 276);
   volatile int* epi_ok = reinterpret_cast<volatile int*>(bars_ptr + 280);   // [5]: per epilogue group, twice; the hand-over of fc2
+  const uint32_t bar_drain = bars + 304;     // leader only, after giving up: the MMAs have ended
   float* fc2_mine = reinterpret_cast<float*>(bars_ptr + 512);    // [64] own queries, own features
   float* fc2_peer = reinterpret_cast<float*>(bars_ptr + 768);    // [64] own queries, peer's features
 
@@ -201,6 +202,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
     }
     mbar_init(bar_fc2, 1);
     mbar_init(bar_next, 8);
+    mbar_init(bar_drain, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -675,6 +677,12 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
     while (!mbar_try_wait(bar_full + 8 * (warp - 6), ph)) {
       if (clock64() - t0 > kWaitCycles) break;
     }
+  }
+  if (rank == 0 && warp == 1 && *abort_flag && elect_one()) {
+    // and the MMAs, before the TMEM they write is somebody else's (the lane that issued them)
+    tc_commit_pair(bar_drain);
+    const long long t0 = clock64();
+    while (!mbar_try_wait_cluster(bar_drain, 0) && clock64() - t0 <= kWaitCycles) {}
   }
   __syncthreads();
   cluster_sync_all();   // neither CTA leaves while the other may still touch its memory

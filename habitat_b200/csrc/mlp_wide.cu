@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_ptr + 200);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + 204);
   volatile int* poisoned = reinterpret_cast<volatile int*>(bars_ptr + 208);
+  const uint32_t bar_drain = bars + 216;                      // after giving up: the MMAs have ended
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = static_cast<int>(blockIdx.x) / G, c = static_cast<int>(blockIdx.x) % G;   // group = cluster
@@ -206,6 +207,7 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     for (int q = 0; q < 4; ++q) mbar_init(bar_act + 8 * q, kReceivers);
     for (int b = 0; b < kBlocks; ++b) mbar_init(bar_acc + 8 * b, 1);
     mbar_init(bar_tfree, 4);
+    mbar_init(bar_drain, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -591,6 +593,12 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     const long long t0 = clock64();
     for (uint32_t i = issued > kSlots ? issued - kSlots : 0; i < issued; ++i)
       while (!mbar_try_wait(bar_full + 8 * (i % kSlots), (i / kSlots) & 1u) && clock64() - t0 <= kWaitCycles) {}
+  }
+  if (*abort_flag && warp == 0 && elect_one()) {
+    // and the MMAs, before the TMEM they write is somebody else's (the lane that issued them)
+    commit_one(bar_drain);
+    const long long t0 = clock64();
+    while (!mbar_try_wait(bar_drain, 0) && clock64() - t0 <= kWaitCycles) {}
   }
   __syncthreads();
   if (warp == 0) {
