@@ -36,8 +36,9 @@
 // warps 2-5 and 12-15 = two epilogue groups (one TMEM lane quadrant per warp), warps 6-11 =
 // weight producers.  Bulk copies issued by one thread complete one after the other (measured:
 // about 750 cycles each whatever their size), so each ring slot has its own issuing warp.
-// Every mbarrier wait is bounded: when a wait runs out the kernel records a status word, all
-// roles leave their loops, outstanding bulk copies and MMAs are waited for (bounded) and TMEM is released.
+// Every mbarrier wait is bounded: when a wait runs out the kernel records a status word, the roles
+// leave their loops or run them empty (the two epilogue groups keep meeting at their common barriers, which
+// have no limit of their own), outstanding bulk copies and MMAs are waited for (bounded) and TMEM is released.
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -470,16 +471,17 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
     long long c_wait = 0, c_epi = 0, c_fc2 = 0, c_layers = 0, c_ld = 0, c_bias = 0, c_sync = 0, c_loc = 0, c_rem = 0;
     // named barrier of this group alone (ids 2 and 3; id 1 joins both groups)
     auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory"); };
-    for (int t = 0; t < my_tiles && ok; ++t, ++tile_no) {
+    for (int t = 0; t < my_tiles; ++t, ++tile_no) {
       const int tile = pair_id + t * n_pairs;
       const MlpProblem& pb = problem_of(p, tile);
       const int n_layers = pb.layers + 1;
       const int64_t q0 = static_cast<int64_t>(tile - pb.first_tile) * kTileQ + static_cast<int64_t>(rank) * kHalfQ;
 
-      for (int L = 0; L < n_layers && ok; ++L, ++lay) {
+      for (int L = 0; L < n_layers; ++L, ++lay) {
         const float* bias = pb.bias + L * kWidth;
         const bool last = (L == n_layers - 1);
         if (!last) {
+          if (!ok) continue;
           // Group g drains output blocks g and g + 2.  Block j becomes K quarter j of the next
           // layer and is written over the current activations in place: in the unit order of a
           // hidden layer nothing reads quarter j once block j is complete.  Under fc1 the input
@@ -623,10 +625,12 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
             }
             if (timed) c_fc2 += clock64() - c1;
           }
-          if (!ok) break;
+          // from here on both groups take part, also one that gave up
+          if (ok) {
 #pragma unroll
-          for (int qd = 0; qd < kChunks; ++qd)
-            red[(grp * 4 + quad) * (kChunks * 32) + qd * 32 + fold16_col<32>(lane) + (lane >> 4)] = part[qd];
+            for (int qd = 0; qd < kChunks; ++qd)
+              red[(grp * 4 + quad) * (kChunks * 32) + qd * 32 + fold16_col<32>(lane) + (lane >> 4)] = part[qd];
+          }
           pair_epi_bar_sync();
           float tot = 0.0f;
           if (T < kChunks * 32) {
@@ -637,7 +641,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(bar_next);
-          if (T < kChunks * 32) {
+          if (ok && T < kChunks * 32) {
             // which CTA owns the query, and its index among the owner's
             const uint32_t owner = static_cast<uint32_t>(T / kHalfQ);
             const int slot = T % kHalfQ;
@@ -647,12 +651,13 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
           pair_epi_bar_sync();
           // hand-over of the partial sums, then the owner finishes its 64 queries
           if (T == 0) {
-            mbar_arrive_remote(map_to_cta(bar_fc2, peer));
-            epi_ok[4] = mbar_wait_cluster(bar_fc2, tile_no & 1u, abort_flag, pb.status, 0x312) ? 1 : 0;
+            const bool all = *abort_flag == 0;   // both groups' sums are there
+            if (all) mbar_arrive_remote(map_to_cta(bar_fc2, peer));
+            epi_ok[4] = all && mbar_wait_cluster(bar_fc2, tile_no & 1u, abort_flag, pb.status, 0x312) ? 1 : 0;
           }
           pair_epi_bar_sync();
-          if (epi_ok[4] == 0) { ok = false; break; }
-          if (T < kHalfQ) {
+          ok = epi_ok[4] != 0;
+          if (ok && T < kHalfQ) {
             const int64_t q = q0 + T;
             if (q < pb.Q) pb.out[q] = fc2_mine[T] + fc2_peer[T] + pb.fc2_b;
           }
