@@ -138,11 +138,21 @@ def wave_scale(kernels: KernelBatch, origin, dests: Sequence, dest_regs=None, me
     res = _call("hb_wave_scale", _native.binding().wave_scale, kernels, origin, dests, dest_regs, metrics,
                 want_status, want_limits, out, partials)
     if res is None:
-        _check_wave_arguments(kernels, dests, dest_regs, metrics, partials)
+        _check_wave_arguments(kernels, dests, dest_regs, metrics, out, partials)
     return res
 
 
-def _check_wave_arguments(kernels, dests, dest_regs, metrics, partials):
+def _check_result(t, size, count, name):
+    """A given result: contiguous memory that the GPU can write, of `size`-byte elements, at least `count`."""
+    if not isinstance(t, torch.Tensor) or not (t.is_cuda or t.is_pinned()):
+        raise TypeError("%s must be a CUDA tensor" % name)
+    if t.element_size() != size:
+        raise TypeError("%s must have elements of %d bytes" % (name, size))
+    if not t.is_contiguous() or t.numel() < count:
+        raise ValueError("%s must be contiguous, of at least %d elements" % (name, count))
+
+
+def _check_wave_arguments(kernels, dests, dest_regs, metrics, out, partials):
     """Says what is wrong with arguments the binding did not take."""
     K, D = len(kernels), len(dests)
     _require_cuda(kernels.num_blocks, torch.int32, "num_blocks")
@@ -157,6 +167,8 @@ def _check_wave_arguments(kernels, dests, dest_regs, metrics, partials):
         if kernels.gamma is None:
             raise ValueError("gamma is required unless metrics are given")
         _require_cuda(kernels.gamma, torch.float32, "gamma")
+        if kernels.gamma.numel() < K:
+            raise ValueError("gamma has a different length")
     if dest_regs is not None:
         _require_cuda(dest_regs, torch.int16, "dest_regs")
         if tuple(dest_regs.shape) != (D, K):
@@ -167,10 +179,17 @@ def _check_wave_arguments(kernels, dests, dest_regs, metrics, partials):
         if K > partials.K or D > partials.D:
             raise ValueError("partials were sized for fewer kernels or destinations")
     if metrics is not None:
-        _require_cuda(metrics.flop_efficiency_pct, torch.float64, "flop_efficiency_pct")
-        _require_cuda(metrics.dram_read_bytes, torch.float64, "dram_read_bytes")
-        _require_cuda(metrics.dram_write_bytes, torch.float64, "dram_write_bytes")
-        _require_cuda(metrics.has_metrics, torch.uint8, "has_metrics")
+        for name, dtype in (("flop_efficiency_pct", torch.float64), ("dram_read_bytes", torch.float64),
+                            ("dram_write_bytes", torch.float64), ("has_metrics", torch.uint8)):
+            _require_cuda(getattr(metrics, name), dtype, name)
+            if getattr(metrics, name).numel() < K:
+                raise ValueError("%s has a different length" % name)
+    if out is not None:
+        for name, size, count in (("scaled_ns", 4, D * K), ("dest_occupancy", 1, D * K), ("dest_waves", 4, D * K),
+                                  ("origin_occupancy", 1, K), ("origin_waves", 4, K), ("status", 1, D * K),
+                                  ("limits", 4, (D + 1) * 4 * K)):
+            if getattr(out, name) is not None:
+                _check_result(getattr(out, name), size, count, name)
     raise ValueError("wave_scale: unsupported arguments (at most %d destinations)" % _native.HB_MAX_DEVICES)
 
 
@@ -254,7 +273,7 @@ class MLPHandle:
                 raise ValueError("op_features must be [Q, %d]" % self.n_op_features)
             if device_row.numel() != op_features.shape[0]:
                 raise ValueError("device_row must have Q entries")
-            raise TypeError("out must be a CUDA tensor")
+            _check_result(out, 4, op_features.shape[0], "out")
         return res
 
     def predict_one(self, op_features, device_row):

@@ -74,6 +74,13 @@ const at::Tensor* tensor(PyObject* o, at::ScalarType type) {
   return t.is_cuda() && t.scalar_type() == type && t.is_contiguous() ? &t : nullptr;
 }
 void* data(const at::Tensor* t) { return t ? t->mutable_data_ptr() : nullptr; }
+// A given result plane of at least `count` elements of `size` bytes that the GPU can write: its data, or null.
+void* result_data(PyObject* o, size_t size, int64_t count) {
+  if (!o || !THPVariable_Check(o)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  return (t.is_cuda() || t.is_pinned()) && t.element_size() == size && t.is_contiguous() && t.numel() >= count
+             ? t.mutable_data_ptr() : nullptr;
+}
 
 // Attribute `name` of `o` as tensor data; the tensor stays alive through its owner.
 struct Field {
@@ -83,8 +90,8 @@ struct Field {
     if (!ref.p) PyErr_Clear();
     else t = tensor(ref.p, type);
   }
-  bool none() const { return ref.p == Py_None; }
   void* ptr() const { return data(t); }
+  bool covers(int64_t count) const { return t && t->numel() >= count; }
 };
 
 // Row of a device in the library's table: a DeviceProperties' token (generation * 64 + row) when it is of the
@@ -148,8 +155,9 @@ PyObject* wave_scale(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Field nb(kernels, s_num_blocks, at::kInt), bs(kernels, s_block_size, at::kUInt16),
       rg(kernels, s_regs, at::kUInt16), sm(kernels, s_smem, at::kUInt32), tm(kernels, s_time, at::kFloat),
       gm(kernels, s_gamma, at::kFloat);
-  if (!nb.t || !bs.t || !rg.t || !sm.t || !tm.t || (metrics == Py_None && !gm.t)) Py_RETURN_NONE;
+  if (!nb.t || !bs.t || !rg.t || !sm.t || !tm.t) Py_RETURN_NONE;
   const int64_t K = nb.t->numel();
+  if (metrics == Py_None && !gm.covers(K)) Py_RETURN_NONE;
   if (bs.t->numel() != K || rg.t->numel() != K || sm.t->numel() != K || tm.t->numel() != K) Py_RETURN_NONE;
 
   Ref dests(PySequence_Fast(a[2], "dests must be a sequence of DeviceProperties"));
@@ -176,7 +184,7 @@ PyObject* wave_scale(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (partials != Py_None) Py_RETURN_NONE;
     const Field fe(metrics, s_flop, at::kDouble), rd(metrics, s_rd, at::kDouble), wr(metrics, s_wr, at::kDouble),
         has(metrics, s_has, at::kByte);
-    if (!fe.t || !rd.t || !wr.t || !has.t) Py_RETURN_NONE;
+    if (!fe.covers(K) || !rd.covers(K) || !wr.covers(K) || !has.covers(K)) Py_RETURN_NONE;
     m.flop_efficiency_pct = static_cast<const double*>(fe.ptr());
     m.dram_read_bytes = static_cast<const double*>(rd.ptr());
     m.dram_write_bytes = static_cast<const double*>(wr.ptr());
@@ -239,14 +247,16 @@ PyObject* wave_scale(PyObject*, PyObject* const* a, Py_ssize_t n) {
                     static_cast<uint8_t*>(ptr[3]),  static_cast<uint32_t*>(ptr[4]), static_cast<uint8_t*>(ptr[5]),
                     static_cast<int32_t*>(ptr[6])};
   } else {
-    // given results are taken as they are (their pointers), like the planes of any earlier call
+    // given results: at least as large as this call's planes
+    const int64_t dk = D * K, counts[7] = {dk, dk, dk, K, K, dk, (D + 1) * 4 * K};
+    constexpr size_t kSizes[7] = {4, 1, 4, 1, 4, 1, 4};
     PyObject* names[7] = {s_scaled, s_docc, s_dwav, s_oocc, s_owav, s_status, s_limits};
     void* ptr[7];
     for (int i = 0; i < 7; ++i) {
       Ref f(PyObject_GetAttr(out, names[i]));
       if (!f.p) return nullptr;
-      if (f.p != Py_None && !THPVariable_Check(f.p)) Py_RETURN_NONE;
-      ptr[i] = f.p == Py_None ? nullptr : THPVariable_Unpack(f.p).mutable_data_ptr();
+      ptr[i] = f.p == Py_None ? nullptr : result_data(f.p, kSizes[i], counts[i]);
+      if (f.p != Py_None && !ptr[i] && counts[i] > 0) Py_RETURN_NONE;
     }
     o = hb_wave_out{static_cast<float*>(ptr[0]),    static_cast<uint8_t*>(ptr[1]),  static_cast<uint32_t*>(ptr[2]),
                     static_cast<uint8_t*>(ptr[3]),  static_cast<uint32_t*>(ptr[4]), static_cast<uint8_t*>(ptr[5]),
@@ -297,8 +307,8 @@ PyObject* mlp_predict(PyObject*, PyObject* const* a, Py_ssize_t n) {
     made = empty(size, at::kFloat, f->device());
     out = made.mutable_data_ptr();
   } else {
-    if (!THPVariable_Check(a[4])) Py_RETURN_NONE;
-    out = THPVariable_Unpack(a[4]).mutable_data_ptr();
+    out = result_data(a[4], 4, Q);
+    if (!out && Q > 0) Py_RETURN_NONE;
   }
   void* stream = c10::cuda::getCurrentCUDAStream().stream();
   const float* pf = static_cast<const float*>(data(f));
@@ -1133,7 +1143,8 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const Field nb(a[0], s_num_blocks, at::kInt), bs(a[0], s_block_size, at::kUInt16), rg(a[0], s_regs, at::kUInt16),
         sm(a[0], s_smem, at::kUInt32), tm(a[0], s_time, at::kFloat), gm(a[0], s_gamma, at::kFloat);
     const at::Tensor* dr = a[4] == Py_None ? nullptr : tensor(a[4], at::kShort);
-    if (!bs.t || !rg.t || !sm.t || !tm.t || !gm.t || (a[4] != Py_None && (!dr || dr->numel() != T * K)))
+    if (!bs.covers(K) || !rg.covers(K) || !sm.covers(K) || !tm.covers(K) || !gm.covers(K) ||
+        (a[4] != Py_None && (!dr || dr->numel() != T * K)))
       return refuse("kernel records") != nullptr;
     int32_t rows[HB_MAX_DEVICES];
     const long origin = row_of(a[2]);
@@ -1152,7 +1163,7 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (a[1] != Py_None) {
       const Field fe(a[1], s_flop, at::kDouble), rd(a[1], s_rd, at::kDouble), wr(a[1], s_wr, at::kDouble),
           has(a[1], s_has, at::kByte);
-      if (!fe.t || !rd.t || !wr.t || !has.t) return refuse("metrics") != nullptr;
+      if (!fe.covers(K) || !rd.covers(K) || !wr.covers(K) || !has.covers(K)) return refuse("metrics") != nullptr;
       m = hb_kernel_metrics{static_cast<const double*>(fe.ptr()), static_cast<const double*>(rd.ptr()),
                             static_cast<const double*>(wr.ptr()), static_cast<const uint8_t*>(has.ptr())};
     }

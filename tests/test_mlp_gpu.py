@@ -445,3 +445,20 @@ def test_two_threads_with_batches_side_by_side_on_one_stream():
     for h in hs:
         h.check_status()
         h.close()
+
+
+def test_given_result_has_to_cover_the_queries():
+    feats, dev = workloads.make_queries("bmm", 100, 91)
+    mu, sigma = workloads.batch_mu_sigma(feats, dev)
+    h = batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=DEVF, **workloads.torch_init_mlp_weights("bmm", layers=2))
+    f, r = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()
+    want = h.predict(f, r)
+    for out in (torch.empty(99, device="cuda"), torch.empty(100), torch.empty(100, dtype=torch.float64, device="cuda"),
+                torch.empty(200, device="cuda")[::2]):
+        with pytest.raises((ValueError, TypeError)):
+            h.predict(f, r, out=out)
+    for out in (torch.empty(120, device="cuda"), torch.empty(100).pin_memory()):
+        h.predict(f, r, out=out)
+        torch.cuda.synchronize()
+        assert torch.equal(out[:100].cpu(), want.cpu())
+    h.close()

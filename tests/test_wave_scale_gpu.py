@@ -459,3 +459,49 @@ def test_launches_over_many_device_classes(bench_devices):
                 for plane in ("scaled_ns", "dest_occupancy", "dest_waves"):
                     assert np.array_equal(got[name][plane][d].view(np.uint8), single[d][name][plane][0].view(np.uint8))
     device_table.reset()
+
+
+def test_arrays_that_are_too_short_are_refused(bench_devices):
+    """gamma, metrics and given results that do not cover the kernels are an error of the call; longer ones are
+    taken, and so are results in page-locked memory."""
+    K, origin, dests = 300, bench_devices[0], bench_devices[:3]
+    kb = batched.KernelBatch.from_numpy(workloads.make_kernels(K, seed=5))
+    g = torch.Generator(device="cuda").manual_seed(5)
+    planes = [torch.rand(K, generator=g, device="cuda", dtype=torch.float64) * 1e9 + 1 for _ in range(3)]
+    has = torch.ones(K, dtype=torch.uint8, device="cuda")
+    want, want_m = (batched.wave_scale(kb, origin, dests, metrics=m) for m in
+                    (None, batched.KernelMetricsBatch(*planes, has)))
+
+    def with_gamma(t):
+        return batched.KernelBatch(kb.num_blocks, kb.block_size, kb.regs_per_thread, kb.smem_bytes, kb.run_time_ns, t)
+    with pytest.raises(ValueError):
+        batched.wave_scale(with_gamma(kb.gamma[:-1].clone()), origin, dests)
+    for i in range(4):
+        short = [t[:-1].clone() if i == j else t for j, t in enumerate(planes + [has])]
+        with pytest.raises(ValueError):
+            batched.wave_scale(kb, origin, dests, metrics=batched.KernelMetricsBatch(*short))
+
+    def equal(a, b):
+        torch.testing.assert_close(a.scaled_ns.cpu().flatten()[:3 * K], b.scaled_ns.cpu().flatten(), rtol=0, atol=0,
+                                   equal_nan=True)
+    longer = [torch.cat([t, t[:7]]) for t in planes + [has]]
+    equal(batched.wave_scale(with_gamma(torch.cat([kb.gamma, kb.gamma])), origin, dests), want)
+    equal(batched.wave_scale(kb, origin, dests, metrics=batched.KernelMetricsBatch(*longer)), want_m)
+
+    def result(**other):
+        dk = (3, K)
+        fields = dict(scaled_ns=torch.empty(dk, device="cuda"), dest_occupancy=torch.empty(dk, dtype=torch.uint8, device="cuda"),
+                      dest_waves=torch.empty(dk, dtype=torch.uint32, device="cuda"),
+                      origin_occupancy=torch.empty(K, dtype=torch.uint8, device="cuda"),
+                      origin_waves=torch.empty(K, dtype=torch.int32, device="cuda"), status=None, limits=None)
+        return batched.WaveResult(**dict(fields, **other))
+    for other in (dict(scaled_ns=torch.empty((3, K - 1), device="cuda")), dict(origin_waves=torch.empty(K, dtype=torch.uint8, device="cuda")),
+                  dict(scaled_ns=torch.empty((K, 3), device="cuda").t()), dict(scaled_ns=torch.empty((3, K))),
+                  dict(status=torch.empty((2, K), dtype=torch.uint8, device="cuda")),
+                  dict(limits=torch.empty((3, 4, K), dtype=torch.int32, device="cuda"))):
+        with pytest.raises((ValueError, TypeError)):
+            batched.wave_scale(kb, origin, dests, out=result(**other))
+    for other in ({}, dict(scaled_ns=torch.empty((4, K), device="cuda")), dict(scaled_ns=torch.empty((3, K)).pin_memory())):
+        res = batched.wave_scale(kb, origin, dests, out=result(**other))
+        torch.cuda.synchronize()
+        equal(res, want)
