@@ -522,6 +522,8 @@ class Predictor:
         if flat is None and len(plan.wave_idx):
             run_ms = (plan.overheads + totals) / 1e6
             ms[:, plan.wave_idx] = run_ms[:, plan.fwd_run] + np.where(plan.bwd_run >= 0, run_ms[:, plan.bwd_run], 0.0)
+        if flat is None and not kinds:           # nothing for the GPU, and none needed
+            return times, totals, ms.sum(axis=1).tolist()
         regs = None
         if flat is not None and self._has_registers():
             regs = wave_batch.destination_registers(plan.kernels, plan.names, dests, self._kernel_metadata)

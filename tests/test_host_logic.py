@@ -213,3 +213,28 @@ def test_precision_knob(monkeypatch):
     monkeypatch.setenv("HABITAT_B200_PRECISION", "fp64")
     with pytest.raises(ValueError):
         Predictor()
+
+
+@pytest.mark.parametrize("strategy", ["own", "unified"])
+def test_traces_without_work_for_the_gpu_need_none(strategy):
+    """A user's wave scaling strategy, and operations without kernels, are predicted on the host alone."""
+    from habitat_b200.analysis.predictor import Predictor
+    from habitat_b200.analysis.trace import Trace
+    origin, dests = Device.V100, [Device.T4, Device.P100]
+    kernel = MeasuredKernel(KernelInstance("k", 10, 128, 0, 0, 32, 1000), [], origin)
+    kernels = [kernel, kernel] if strategy == "own" else []
+    run = RunTimeMeasurement(0.005, kernels, origin)
+    ops = [MeasuredOperation("relu", Arguments((), {}), run, None, origin),
+           MeasuredOperation("add", Arguments((), {}), run, run, origin),
+           MeasuredOperation("rnn_tanh", Arguments((), {}), run, None, origin)]
+    factor = {d.name: 2.0 + i for i, d in enumerate(dests)}
+    own = lambda k, o, dest, metadata: PredictedKernel(k, k.run_time_ns * factor[dest.name])
+    predictor = Predictor(wave_scaling_strategy=own) if strategy == "own" else Predictor()
+    trace = Trace(origin, ops)
+    for _ in range(2):
+        for dest, got in zip(dests, trace.to_devices(dests, predictor)):
+            one = (3000 + 2000 * factor[dest.name]) / 1e6 if kernels else 0.005
+            passed = ops[2].run_time_ms if ops[2].name in SPECIAL_OPERATIONS else one
+            assert np.allclose(got.operations.run_times_ms, [one, 2 * one, passed], rtol=1e-12)
+            assert got.run_time_ms == pytest.approx(3 * one + passed, rel=1e-12)
+            assert got.operations[1].forward.run_time_ms == pytest.approx(one, rel=1e-12)
