@@ -16,7 +16,7 @@ import os
 import numpy as np
 import torch
 
-from habitat_b200 import _native
+from habitat_b200 import _native, batched
 from habitat_b200.analysis import SPECIAL_OPERATIONS
 from habitat_b200.analysis.kernels import MeasuredKernel, PredictedKernel
 from habitat_b200.analysis.mlp.mlp import FEATURES, RuntimePredictor
@@ -503,12 +503,16 @@ class Predictor:
         at once)."""
         T, K, n_runs = len(dests), plan.n_kernels, plan.n_runs
         names = [name for name in _MLP_OPS if len(plan.mlp_idx[name])]
-        kinds = []
+        kinds, native = [], []
         for name in names:
             pred = self._predictor(name)
             rows = bytes([pred.device_row(origin.name)] + [pred.device_row(d.name) for d in dests])
-            feats, rt, _, _ = plan.special_inputs(name, operations, pred.model.features)
-            kinds.append((pred._handle._handle.value, feats, rt, rows, plan.mlp_idx[name]))
+            feats, rt, rt_host, _ = plan.special_inputs(name, operations, pred.model.features)
+            if getattr(pred.predict_batch, "__func__", None) is RuntimePredictor.predict_batch:
+                kinds.append((pred._handle._handle.value, feats, rt, rows, plan.mlp_idx[name]))
+                native.append(name)
+            else:
+                ms[:, plan.mlp_idx[name]] = self._special_scale_ops(name, pred, rows, feats, rt, rt_host, T)
         flat = plan.flat                         # None: no kernels, or a user-supplied strategy
         times = np.empty((T, K), np.float32 if flat is not None else np.float64)
         totals = (np.empty if flat is not None else np.zeros)((T, n_runs), np.float64)
@@ -533,10 +537,24 @@ class Predictor:
             (plan.overheads, plan.wave_idx, plan.fwd_run, plan.bwd_run), times, totals, ms)
         if nan:
             wave_batch.raise_zero_wave()
-        for name, raw in zip(names, clamped):
+        for name, raw in zip(native, clamped):
             if raw is not None:
                 self._warn_negative(name, plan.mlp_inputs[name][2], np.frombuffer(raw, np.float32).astype(np.float64), T)
         return times, totals, sums
+
+    def _special_scale_ops(self, name, pred, rows, feats, rt, rt_host, T):
+        """-> [T, n] predicted ms of the operations of one kind (predictor.py:132-148 of the reference) from a
+        predictor with a predict_batch of its own."""
+        n = len(rt_host)
+        p = pred.predict_batch(feats.repeat(T + 1, 1), torch.tensor(list(rows), dtype=torch.uint8,
+                                                                    device="cuda").repeat_interleave(n))
+        neg = torch.zeros(1, dtype=torch.int32, device="cuda")
+        ms = batched.special_scale(rt.repeat(T), p[n:], p[:n].repeat(T), neg.view(torch.uint32)).view(T, n).cpu().numpy()
+        if getattr(pred, "_handle", None) is not None:
+            pred._handle.check_status()
+        if int(neg.cpu()[0]):
+            self._warn_negative(name, rt_host, p.cpu().numpy().astype(np.float64), T)
+        return ms
 
     @staticmethod
     def _warn_negative(name, run_time_ms, pred_ms, T):

@@ -43,9 +43,12 @@ def predict_iteration_totals(kernels: batched.KernelBatch, overhead_ns: torch.Te
     rows = bytes([origin_mlp_row] + [r for r, s in zip(dest_mlp_rows, same) if not s])
     if len(rows) != 1 + same.count(0):
         raise ValueError("dest_mlp_rows must have an entry per destination")
-    kinds = []
+    kinds, own = [], []                       # own: handles with a predict of their own
     for ops in special.values():
         if ops.features.shape[0] == 0:
+            continue
+        if getattr(ops.handle.predict, "__func__", None) is not batched.MLPHandle.predict:
+            own.append(ops)
             continue
         if ops.features.ndim != 2 or (len(rows) > 1 and ops.features.shape[1] != ops.handle.n_op_features):
             raise ValueError("op_features must be [Q, %d]" % ops.handle.n_op_features)
@@ -60,4 +63,19 @@ def predict_iteration_totals(kernels: batched.KernelBatch, overhead_ns: torch.Te
             batched._require_cuda(ops.run_time_ms, torch.float32, "run_time_ms")
             batched._require_cuda(ops.offsets, torch.int64, "offsets")
         raise ValueError("overheads, features, measured times and offsets have to fit the kernels and iterations")
+    for ops in own:
+        _add_special(totals, ops, rows, same)
     return totals, res
+
+
+def _add_special(totals, ops, rows, same):
+    """Adds the operations of one kind from the predictions of ops.handle.predict."""
+    n, T = ops.features.shape[0], len(rows) - 1
+    if T:
+        pred = ops.handle.predict(ops.features.repeat(T + 1, 1), torch.tensor(
+            list(rows), dtype=torch.uint8, device=totals.device).repeat_interleave(n))
+        ms = batched.special_scale(ops.run_time_ms.repeat(T), pred[n:], pred[:n].repeat(T)).view(T, n)
+    t = 0
+    for d, measured in enumerate(same):
+        totals[:, d] += batched.segment_sum(ops.run_time_ms if measured else ms[t], ops.offsets)
+        t += not measured

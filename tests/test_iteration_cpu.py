@@ -11,7 +11,9 @@ def _call(bench_devices, width=4, rows=range(6), dims=2):
     zeros = lambda dtype: torch.zeros(10, dtype=dtype)
     kernels = batched.KernelBatch(zeros(torch.int32), zeros(torch.uint16), zeros(torch.uint16), zeros(torch.uint32),
                                   zeros(torch.float32), zeros(torch.float32))
-    handle = types.SimpleNamespace(n_op_features=4, _handle=types.SimpleNamespace(value=0))
+    handle = object.__new__(batched.MLPHandle)
+    handle.n_op_features, handle._handle = 4, types.SimpleNamespace(value=0)
+    handle.close = lambda: None
     features = torch.zeros((4, width) if dims == 2 else (4,))
     special = {"bmm": iteration.SpecialOps(handle, features, torch.zeros(4), torch.tensor([0, 4]))}
     return iteration.predict_iteration_totals(kernels, torch.zeros(10), torch.tensor([0, 10]), special,

@@ -105,3 +105,56 @@ def test_strided_features_and_longer_overheads(bench_devices):
     assert torch.equal(totals(strided, over), want)
     assert torch.equal(totals(f, torch.cat([over, torch.full((5,), float("nan"), device="cuda")])), want)
     h.close()
+
+
+def test_predictors_with_a_predict_of_their_own(bench_devices):
+    """Handles and runtime predictors that predict otherwise are asked, side by side with ordinary ones: totals and
+    traces follow their predictions."""
+    from habitat_b200.analysis.arguments import Arguments
+    from habitat_b200.analysis.mlp.mlp import RuntimePredictor
+    from habitat_b200.analysis.operation import MeasuredOperation
+    from habitat_b200.analysis.predictor import Predictor
+    from habitat_b200.analysis.run_time import RunTimeMeasurement
+    from habitat_b200.analysis.trace import Trace
+    I, origin, dests = 3, bench_devices[0], bench_devices
+    kernels, overhead, ops = _make(I, 78, origin.spec_tuple())
+    koff = torch.arange(I + 1, device="cuda") * KERNELS_PER_ITER
+
+    class Slower(batched.MLPHandle):
+        def predict(self, op_features, device_row, out=None):
+            return op_features[:, 0] * (1.0 + device_row.float())       # of device r: 1 + r times device 0's
+
+    special = {}
+    for op, cls in (("linear", batched.MLPHandle), ("bmm", Slower)):
+        feats, rt = ops[op]
+        mu, sigma = workloads.batch_mu_sigma(feats, np.tile(np.arange(6, dtype=np.uint8), len(feats))[:len(feats)])
+        h = cls(4, mu=mu, sigma=sigma, device_features=workloads.BENCH_DEVICE_FEATURES,
+                **workloads.torch_init_mlp_weights(op))
+        special[op] = iteration.SpecialOps(h, torch.from_numpy(feats).cuda(), torch.from_numpy(rt).cuda(),
+                                           torch.arange(I + 1, device="cuda") * PER_ITER[op])
+
+    def totals(which):
+        return iteration.predict_iteration_totals(batched.KernelBatch.from_numpy(kernels), torch.from_numpy(overhead).cuda(),
+                                                  koff, which, origin, dests, 0, list(range(6)))[0].cpu().numpy()
+    added = totals(special) - totals({"linear": special["linear"]})
+    measured = ops["bmm"][1].astype(np.float64).reshape(I, -1).sum(axis=1)
+    np.testing.assert_allclose(added, measured[:, None] * np.arange(1, 7), rtol=1e-6)
+
+    class Slow(RuntimePredictor):
+        def predict_batch(self, op_features, device_rows):
+            return op_features[:, 1] * torch.where(device_rows == self.device_row(origin.name), 1.0, 5.0)
+
+    predictor = Predictor()
+    for cls, op in ((Slow, "linear"), (RuntimePredictor, "bmm")):
+        pred = cls(op, 2, 1024)
+        with torch.no_grad():
+            pred.model.fc2.bias.fill_(1.0)
+        pred.mu, pred.sigma = np.zeros(8), np.full(8, 1e4)
+        setattr(predictor, op + "_pred", pred)
+    run = RunTimeMeasurement(0.5, [], origin)
+    trace = Trace(origin, [MeasuredOperation("linear", Arguments(((8, 16), (32, 16), None), {}), run, None, origin),
+                           MeasuredOperation("bmm", Arguments(((4, 8, 16), (4, 16, 8)), {}), run, run, origin)])
+    for got in trace.to_devices(dests[1:], predictor):
+        times = got.operations.run_times_ms
+        assert times[0] == pytest.approx(2.5, rel=1e-6) and 0 < times[1] < 10
+        assert got.run_time_ms == pytest.approx(times.sum(), rel=1e-12)
