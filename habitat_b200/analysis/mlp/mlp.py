@@ -116,9 +116,8 @@ class RuntimePredictor:
         torch.save({"mu": self.mu, "sigma": self.sigma, "model": self.model.state_dict()}, path)
 
     def invalidate(self):
-        """Drops the device-side weight pack (call after changing weights, mu or sigma)."""
-        if self._handle is not None:
-            self._handle.close()
+        """Drops the device-side weight pack (call after changing weights, mu or sigma).  A prediction that another
+        thread is making keeps it until it has ended."""
         self._handle = None
         self._device_rows = None
 

@@ -503,13 +503,14 @@ class Predictor:
         at once)."""
         T, K, n_runs = len(dests), plan.n_kernels, plan.n_runs
         names = [name for name in _MLP_OPS if len(plan.mlp_idx[name])]
-        kinds, native = [], []
+        kinds, native, held = [], [], []
         for name in names:
             pred = self._predictor(name)
             rows = bytes([pred.device_row(origin.name)] + [pred.device_row(d.name) for d in dests])
             feats, rt, rt_host, _ = plan.special_inputs(name, operations, pred.model.features)
             if getattr(pred.predict_batch, "__func__", None) is RuntimePredictor.predict_batch:
-                kinds.append((pred._handle._handle.value, feats, rt, rows, plan.mlp_idx[name]))
+                held.append(pred._handle)        # the call below knows its address only
+                kinds.append((held[-1]._handle.value or 0, feats, rt, rows, plan.mlp_idx[name]))
                 native.append(name)
             else:
                 ms[:, plan.mlp_idx[name]] = self._special_scale_ops(name, pred, rows, feats, rt, rt_host, T)

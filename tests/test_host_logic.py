@@ -238,3 +238,38 @@ def test_traces_without_work_for_the_gpu_need_none(strategy):
             assert np.allclose(got.operations.run_times_ms, [one, 2 * one, passed], rtol=1e-12)
             assert got.run_time_ms == pytest.approx(3 * one + passed, rel=1e-12)
             assert got.operations[1].forward.run_time_ms == pytest.approx(one, rel=1e-12)
+
+
+def test_weights_dropped_during_a_prediction_live_until_it_ends(monkeypatch):
+    """RuntimePredictor.invalidate in another thread (a checkpoint is loaded, a device row appears) while a trace is
+    being predicted: the native call has the handle's address only."""
+    import types
+    from habitat_b200.analysis import predictor as module
+    closed = []
+
+    class Handle:
+        def __init__(self):
+            self._handle = types.SimpleNamespace(value=77)
+
+        def close(self):
+            closed.append(self._handle.value)
+
+        __del__ = close
+
+    pred = RuntimePredictor("linear", 1, 16)
+    pred._handle, pred._device_rows = Handle(), {"V100": 0, "T4": 1}
+    predictor = module.Predictor()
+    predictor.linear_pred = pred
+
+    def run_group(kernels, metrics, origin, dests, regs, offsets, kinds, passes, times, totals, ms):
+        pred.invalidate()
+        assert [k[0] for k in kinds] == [77] and not closed
+        return False, [0.0], [None]
+    monkeypatch.setattr(module._native, "binding", lambda: types.SimpleNamespace(run_group=run_group))
+    none = np.zeros(0, np.int64)
+    plan = types.SimpleNamespace(
+        n_kernels=0, n_runs=0, flat=None, wave_idx=none, overheads=none.astype(np.float64), fwd_run=none, bwd_run=none,
+        mlp_idx=dict(conv2d=none, linear=np.zeros(1, np.int64), bmm=none, lstm=none),
+        special_inputs=lambda name, operations, order: (None, None, np.ones(1, np.float32), order))
+    predictor._run_plan(plan, [], Device.V100, [Device.T4], np.zeros((1, 1)))
+    assert closed == [77] and pred._handle is None
