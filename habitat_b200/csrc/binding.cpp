@@ -11,6 +11,7 @@
 #include <ATen/EmptyTensor.h>
 #include <ATen/core/CachingHostAllocator.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -121,6 +122,20 @@ bool failed(hb_status st) {
 at::Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const at::Device& dev) {
   return at::Tensor(at::detail::empty_cuda(sizes, type, dev, c10::nullopt));
 }
+// The same beside tensors that are on the GPU already: with its device current, straight from torch's allocator
+// (the general form looks up and switches devices, a tenth of a microsecond each time).
+at::Tensor empty_beside(at::IntArrayRef sizes, at::ScalarType type, const at::Device& dev, bool current) {
+  if (!current) return empty(sizes, type, dev);
+  size_t bytes = c10::elementSize(type);
+  for (const int64_t n : sizes) bytes *= static_cast<size_t>(n);
+  c10::Allocator* allocator = c10::cuda::CUDACachingAllocator::get();
+  at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(
+      c10::Storage(c10::make_intrusive<c10::StorageImpl>(c10::StorageImpl::use_byte_size_t(), bytes, allocator->allocate(bytes),
+                                                         allocator, /*resizable=*/true)),
+      c10::DispatchKeySet(c10::DispatchKey::CUDA), c10::scalarTypeToTypeMeta(type));
+  t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+  return t;
+}
 // A contiguous tensor of `type` at byte `offset` of another one's storage.
 at::Tensor inside(const at::Tensor& block, size_t offset, at::IntArrayRef sizes, at::ScalarType type) {
   at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(block.storage()),
@@ -133,7 +148,10 @@ at::Tensor inside(const at::Tensor& block, size_t offset, at::IntArrayRef sizes,
 
 // Results up to this size share one allocation (each plane on a 256-byte boundary): an allocation costs
 // about a microsecond.  Larger ones are separate, so that a caller who keeps one plane keeps only that.
+// Only bytes and uint32 share: torch.save refuses tensors that see one storage as different types, and counts
+// those two as one.
 constexpr size_t kOneBlock = 1 << 20;
+constexpr bool shares_block(at::ScalarType t) { return t == at::kByte || t == at::kUInt32; }
 
 hb_status wave_scale_call(const hb_kernel_soa& k, const hb_kernel_metrics* m, int64_t K, int32_t origin,
                           const int32_t* rows, int32_t D, const int16_t* regs, const hb_wave_out& out, double* partials,
@@ -219,13 +237,13 @@ PyObject* wave_scale(PyObject*, PyObject* const* a, Py_ssize_t n) {
     size_t offset[7], total = 0;
     for (int i = 0; i < 7; ++i) {
       offset[i] = total;
-      if (planes[i].want) total += (planes[i].bytes + 255) & ~static_cast<size_t>(255);
+      if (planes[i].want && shares_block(planes[i].type)) total += (planes[i].bytes + 255) & ~static_cast<size_t>(255);
     }
-    const bool one = total <= kOneBlock;
+    const bool one = total <= kOneBlock, current = dev.index() == c10::cuda::current_device();
     at::Tensor block;
     if (one) {
       const int64_t size[1] = {static_cast<int64_t>(total)};
-      block = empty(size, at::kByte, dev);
+      block = empty_beside(size, at::kByte, dev, current);
     }
     void* ptr[7];
     PyObject* args[8] = {nullptr};
@@ -235,8 +253,8 @@ PyObject* wave_scale(PyObject*, PyObject* const* a, Py_ssize_t n) {
         args[1 + i] = Py_NewRef(Py_None);
         continue;
       }
-      at::Tensor t = one ? inside(block, offset[i], planes[i].sizes, planes[i].type)
-                         : empty(planes[i].sizes, planes[i].type, dev);
+      at::Tensor t = one && shares_block(planes[i].type) ? inside(block, offset[i], planes[i].sizes, planes[i].type)
+                                                         : empty_beside(planes[i].sizes, planes[i].type, dev, current);
       ptr[i] = t.mutable_data_ptr();
       args[1 + i] = THPVariable_Wrap(std::move(t));
     }

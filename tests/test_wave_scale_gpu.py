@@ -505,3 +505,13 @@ def test_arrays_that_are_too_short_are_refused(bench_devices):
         res = batched.wave_scale(kb, origin, dests, out=result(**other))
         torch.cuda.synchronize()
         equal(res, want)
+
+
+@pytest.mark.parametrize("K", [333, 200_000])
+def test_results_can_be_saved(bench_devices, K, tmp_path):
+    kb = batched.KernelBatch.from_numpy(workloads.make_kernels(K, seed=6))
+    res = batched.wave_scale(kb, bench_devices[0], bench_devices, want_status=True, want_limits=True)
+    torch.save(res, str(tmp_path / "res.pt"))
+    back = torch.load(str(tmp_path / "res.pt"), weights_only=False)
+    for name, t in vars(res).items():
+        assert np.array_equal(to_numpy(getattr(back, name)), to_numpy(t), equal_nan=name == "scaled_ns"), name
