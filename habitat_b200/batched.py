@@ -224,7 +224,7 @@ def wave_scale_host(arrays, origin, dests, want_status=False, want_limits=False)
     else:
         outs = [None if p is None else np.empty(p[2], p[1]) for p in planes]
     if binding.wave_scale_host(*ins, origin, dests, tuple(outs)) is None:
-        raise ValueError("the kernel arrays must have the same length (at most %d destinations)"
+        raise ValueError("the kernel arrays must cover the entries of num_blocks (at most %d destinations)"
                          % _native.HB_MAX_DEVICES)
     return dict(zip(names, outs))
 

@@ -504,7 +504,8 @@ int find_metrics(PyObject* records, PyObject* cached, PyObject* metrics, PyTypeO
   return missing == 0 ? 1 : 0;
 }
 
-// A contiguous buffer (numpy array, bytes) seen as `count` values of T; ok() says whether it is that large.
+// A contiguous buffer (numpy array, bytes) seen as values of T; ok() says whether it holds `count` of them, covers()
+// whether at least as many.
 template <typename T>
 struct Buffer {
   Py_buffer view{};
@@ -516,6 +517,7 @@ struct Buffer {
   ~Buffer() { if (held) PyBuffer_Release(&view); }
   Buffer(const Buffer&) = delete;
   Buffer& operator=(const Buffer&) = delete;
+  bool covers(int64_t count) const { return held && view.len >= count * static_cast<int64_t>(sizeof(T)); }
   bool ok(int64_t count) const { return held && view.len == count * static_cast<int64_t>(sizeof(T)); }
   T* data() const { return static_cast<T*>(view.buf); }
   int64_t size() const { return held ? view.len / static_cast<int64_t>(sizeof(T)) : 0; }
@@ -1000,7 +1002,7 @@ PyObject* wave_scale_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Buffer<uint32_t> sm(a[3], false);
   const Buffer<float> tm(a[4], false), gm(a[5], false);
   const int64_t K = nb.size();
-  if (!nb.held || !bs.ok(K) || !rg.ok(K) || !sm.ok(K) || !tm.ok(K) || !gm.ok(K)) Py_RETURN_NONE;
+  if (!nb.held || !bs.covers(K) || !rg.covers(K) || !sm.covers(K) || !tm.covers(K) || !gm.covers(K)) Py_RETURN_NONE;
   const long origin = row_of(a[6]);
   if (origin < 0) return nullptr;
   int32_t rows[HB_MAX_DEVICES];
