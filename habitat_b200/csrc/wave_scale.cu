@@ -1446,16 +1446,20 @@ struct HostPlanes {
       slot += up(row * out_rows[j]);
     }
   }
-  // Whether the GPU can write every result plane where it is.
+  // Whether the GPU can write every result plane where it is: page-locked at both ends (a caller may have registered
+  // the beginning of an array only).
   bool results_page_locked() const {
     for (int j = 0; j < kOut; ++j) {
       if (!out[j]) continue;
-      cudaPointerAttributes a{};
-      if (cudaPointerGetAttributes(&a, out[j]) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
+      uint8_t* const last = out[j] + out_size[j] * out_rows[j] * K - 1;
+      for (uint8_t* p : {out[j], last}) {
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+          cudaGetLastError();
+          return false;
+        }
+        if (a.type != cudaMemoryTypeHost || a.devicePointer != p) return false;
       }
-      if (a.type != cudaMemoryTypeHost || a.devicePointer != out[j]) return false;
     }
     return true;
   }

@@ -515,3 +515,34 @@ def test_results_can_be_saved(bench_devices, K, tmp_path):
     back = torch.load(str(tmp_path / "res.pt"), weights_only=False)
     for name, t in vars(res).items():
         assert np.array_equal(to_numpy(getattr(back, name)), to_numpy(t), equal_nan=name == "scaled_ns"), name
+
+
+def test_host_results_that_are_page_locked_in_part(bench_devices):
+    """A result array whose beginning alone has been registered is ordinary memory to the host entry point."""
+    import ctypes
+    from habitat_b200 import _native
+    K, D = 40_000, len(bench_devices)
+    made = workloads.make_kernels(K, seed=8)
+    types = (np.int32, np.uint16, np.uint16, np.uint32, np.float32, np.float32)
+    names = ("num_blocks", "block_size", "regs_per_thread", "smem_bytes", "run_time_ns", "gamma")
+    ins = [np.ascontiguousarray(made[n], t) for n, t in zip(names, types)]
+    want = batched.wave_scale_host(made, bench_devices[0], bench_devices)
+    outs = {n: torch.zeros(v.nbytes, dtype=torch.uint8).pin_memory().numpy().view(v.dtype).reshape(v.shape)
+            for n, v in want.items() if v is not None}
+    scaled = np.zeros((D * K + 4096,), np.float32)
+    at = (-scaled.ctypes.data % 4096) // 4                   # from a page boundary on
+    outs["scaled_ns"] = scaled[at:at + D * K].reshape(D, K)
+    address = outs["scaled_ns"].ctypes.data
+    p = lambda a: ctypes.c_void_p(a.ctypes.data if a is not None else 0)
+    soa = _native.KernelSoA(*[p(a) for a in ins])
+    out = _native.WaveOut(*[p(outs.get(n)) for n in ("scaled_ns", "dest_occupancy", "dest_waves", "origin_occupancy",
+                                                     "origin_waves", "status", "limits")])
+    rows = device_table.rows_of([bench_devices[0]] + list(bench_devices))
+    assert int(torch.cuda.cudart().cudaHostRegister(address, 65536, 0)) == 0
+    try:
+        _native.check(_native.load().hb_wave_scale_host(ctypes.byref(soa), K, rows[0], (ctypes.c_int32 * D)(*rows[1:]), D,
+                                                        ctypes.c_void_p(0), ctypes.byref(out)))
+    finally:
+        torch.cuda.cudart().cudaHostUnregister(address)
+    for n, v in outs.items():
+        assert np.array_equal(v.view(np.uint8), want[n].view(np.uint8)), n
