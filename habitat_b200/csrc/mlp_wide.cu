@@ -615,10 +615,13 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
 namespace {
 constexpr int kMaxCudaDevices = 64;
 // Scratch per stream: launches on one stream follow one another, so they can share it (those of one call
-// that run side by side have a lane each).  It is kept between launches, at most kMaxStreams of them per
-// GPU (a launch on yet another stream takes the two-SM kernel, which needs none), and freed with the
-// GPU's last predictor.
-constexpr int kMaxStreams = 16;
+// that run side by side have a lane each).  It is kept between launches and freed with the GPU's last predictor.
+// The first kMaxStreams streams and lanes keep theirs.  Later ones (a program with a stream per request) share
+// kMoreStreams: each launch of theirs is followed by an event, and a new stream takes over what has been out of
+// use for longest.  The events keep a launch from overlapping the end of the one before it, which is why
+// the first streams go without.  While none of the shared ones is out of use, a launch takes the two-SM kernel,
+// which needs no scratch.
+constexpr int kMaxStreams = 16, kMoreStreams = 16;
 constexpr int kMaxGroups = 37;
 constexpr int kWidths = 3;        // W = 16, 32, 64 have their own buffers: a word's parity counts its own uses
 constexpr size_t kActsBytes = static_cast<size_t>(kMaxGroups) * 2 * 2048 * (16 + 32 + 64);
@@ -631,17 +634,27 @@ struct StreamScratch {
   bool fresh = false;                            // buffers and parities start over at the next launch
   uint32_t tag = 0;
   unsigned long long parity[kWidths][2] = {};    // bit g: parity of the next use of group g's buffers
+  cudaEvent_t done = nullptr;                    // shared ones: behind the last launch
+  uint64_t last_use = 0;
 };
 struct GpuScratch {
   std::mutex mu;
   int handles = 0;
   int used = 0;
-  StreamScratch s[kMaxStreams];
+  uint64_t uses = 0;
+  StreamScratch s[kMaxStreams + kMoreStreams];
 };
 GpuScratch g_wide[kMaxCudaDevices];
 
+// A thread's own calls while another stream is being captured: that capture does not mind them.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // The scratch of `stream` on GPU `dev`, or null when there is none to be had (a stream that is being
-// captured: a graph may be replayed anywhere; too many streams; no memory).  Call with the mutex held.
+// captured: a graph may be replayed anywhere; too many streams at work; no memory).  Call with the mutex held.
 StreamScratch* scratch_of(GpuScratch& g, cudaStream_t stream, int lane) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
@@ -652,15 +665,28 @@ StreamScratch* scratch_of(GpuScratch& g, cudaStream_t stream, int lane) {
   }
   for (int i = 0; i < g.used; ++i)
     if (g.s[i].stream_id == id && g.s[i].lane == lane) return &g.s[i];
-  if (g.used == kMaxStreams) return nullptr;
+  const RelaxedCapture relaxed;
+  if (g.used == kMaxStreams + kMoreStreams) {
+    StreamScratch* oldest = nullptr;
+    for (int i = kMaxStreams; i < g.used; ++i) {
+      StreamScratch& s = g.s[i];
+      if (s.done && (!oldest || s.last_use < oldest->last_use) && cudaEventQuery(s.done) == cudaSuccess) oldest = &s;
+    }
+    cudaGetLastError();   // not an error of this call: some event is still ahead
+    if (oldest) {
+      oldest->stream_id = id;   // the buffers, their parities and their tag go on
+      oldest->lane = lane;
+    }
+    return oldest;
+  }
   StreamScratch& s = g.s[g.used];
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // another stream's capture does not mind this allocation
-  cudaThreadExchangeStreamCaptureMode(&mode);
+  s = StreamScratch{};
   void* base = nullptr;
-  const bool ok = cudaMalloc(&base, kScratchBytes) == cudaSuccess;
-  cudaThreadExchangeStreamCaptureMode(&mode);
-  if (!ok) {
+  if ((g.used >= kMaxStreams && cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming) != cudaSuccess) ||
+      cudaMalloc(&base, kScratchBytes) != cudaSuccess) {
     cudaGetLastError();
+    if (s.done) cudaEventDestroy(s.done);
+    s.done = nullptr;
     return nullptr;
   }
   s.stream_id = id;
@@ -808,7 +834,11 @@ void wide_handle_destroyed(int device) {
   GpuScratch& g = g_wide[device];
   std::lock_guard<std::mutex> lock(g.mu);
   if (--g.handles > 0) return;
-  for (int i = 0; i < g.used; ++i) cudaFree(g.s[i].base);   // waits for launches that still use it
+  for (int i = 0; i < g.used; ++i) {
+    cudaFree(g.s[i].base);   // waits for launches that still use it
+    if (g.s[i].done) cudaEventDestroy(g.s[i].done);
+    g.s[i].done = nullptr;
+  }
   g.used = 0;
 }
 
@@ -828,8 +858,10 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
   *launched = false;
   if (w.G == 0 || h->device >= kMaxCudaDevices || (batch.host_inputs && batch.Q > kWideInline)) return HB_OK;
   // parities and tags follow the stream's order: the caller holds the queue's lock
-  StreamScratch* s = scratch_of(g_wide[h->device], stream, batch.lane);
+  GpuScratch& g = g_wide[h->device];
+  StreamScratch* s = scratch_of(g, stream, batch.lane);
   if (!s) return HB_OK;
+  s->last_use = ++g.uses;
   const bool split = h->precision == HB_PRECISION_BF16X3;
   WideParams p{};
   p.bias = h->bias; p.fc2_w = h->fc2_w; p.fc2_b = h->fc2_b; p.mu = h->mu; p.sigma = h->sigma; p.dev_feat = h->dev_feat;
@@ -871,6 +903,11 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
   const cudaError_t e = split ? launch<true>(w, p, h->device, stream, &fits)
                               : launch<false>(w, p, h->device, stream, &fits);
   s->fresh = e != cudaSuccess || !fits;   // not launched: the parities above did not happen
+  if (s->done && cudaEventRecord(s->done, stream) != cudaSuccess) {
+    cudaGetLastError();
+    cudaEventDestroy(s->done);
+    s->done = nullptr;         // nobody can tell any more when it is out of use: it stays with its stream
+  }
   if (e != cudaSuccess) return cuda_fail(e, "mlp_wide_kernel launch");
   *launched = fits;
   return HB_OK;

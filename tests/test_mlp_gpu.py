@@ -462,3 +462,51 @@ def test_given_result_has_to_cover_the_queries():
         torch.cuda.synchronize()
         assert torch.equal(out[:100].cpu(), want.cpu())
     h.close()
+
+
+def test_small_batches_on_ever_new_streams():
+    """A program with a stream per request keeps the kernel for small batches (the two-SM kernel would leave its cycle
+    counters) and its bits: 64 streams one after the other, some with three predictors side by side, then all of
+    them at once."""
+    import ctypes
+    from habitat_b200 import _native
+    feats, dev = workloads.make_queries("linear", 300, 95)
+    mu, sigma = workloads.batch_mu_sigma(feats, dev)
+    f, r = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()
+    hs = [batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=DEVF, **workloads.init_mlp_weights(
+        "linear", seed=s, layers=3, gain=2.0)) for s in range(3)]
+    want = [h.predict(f, r) for h in hs]
+    n, rows = 40, bytes([1, 4, 2])
+    each = torch.tensor(list(rows), dtype=torch.uint8, device="cuda").repeat_interleave(n)
+    want_grid = [h.predict(f[:n].repeat(3, 1).contiguous(), each) for h in hs]
+    outs = [torch.empty((3 * n,), device="cuda") for _ in hs]
+    items = (_native.MlpGrid * 3)(*[
+        _native.MlpGrid(h._handle.value, f.data_ptr(), n, ctypes.cast(ctypes.c_char_p(rows), ctypes.c_void_p), 3,
+                        out.data_ptr()) for h, out in zip(hs, outs)])
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(priority=-(i % 2)) for i in range(64)]
+    assert len({s.cuda_stream for s in streams}) > 40
+    for turn in range(2):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                if i % 3 == turn:
+                    for out in outs:
+                        out.fill_(float("nan"))
+                    _native.check(_native.load().hb_mlp_predict_grid(items, 3, s.cuda_stream))
+                got = hs[i % 2].predict(f, r)
+            s.synchronize()
+            assert torch.equal(got, want[i % 2])
+            if i % 3 == turn:
+                for out, ref in zip(outs, want_grid):
+                    assert torch.equal(out, ref)
+    assert [h.phase_cycles()["slots"] for h in hs] == [0, 0, 0]
+    results = []
+    for i in range(256):
+        with torch.cuda.stream(streams[i % 64]):
+            results.append(hs[i % 3].predict(f, r))
+    torch.cuda.synchronize()
+    for i, got in enumerate(results):
+        assert torch.equal(got, want[i % 3]), i
+    for h in hs:
+        h.check_status()
+        h.close()
