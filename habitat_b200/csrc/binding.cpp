@@ -22,6 +22,7 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <utility>
 #include <vector>
 
@@ -895,14 +896,21 @@ PyObject* submit_wave(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // ---------------------------------------------------------------------------
 // Arrays over such blocks are what batched.wave_scale_host returns: the kernel writes them directly.  A block
 // goes back to the pool when the last array over it goes.  Blocks come in quarter steps between powers of two,
-// of at most kMostBlock bytes and kMostTotal in all (page-locking costs about 0.3 ms per MB, so it must not
-// recur); a caller who keeps more results than that gets the rest in ordinary memory, as does one who asks for a
-// larger block.  Room for a few results of a million kernels on eight devices.
+// of at most kMostBlock bytes and kMostTotal in all, room for a few results of a million kernels on eight devices;
+// a caller who keeps more results than that gets the rest in ordinary memory, as does one who asks for a
+// larger block.
+//
+// Page-locking costs about 0.3 ms per MB, so it must not recur: 65,536 kernels on six devices take 0.16 ms into a
+// block that has come back, 1.0 ms into fresh pages and 2.2 ms with a new block.  So a new one needs credit: two to begin with (a loop that keeps one result while the next
+// is made), one more for each time a block is used again, kMostCredit at most.  A caller who keeps every result
+// pays for two blocks and then gets ordinary memory; so does one whose sizes push one another out of the pool.
 constexpr size_t kMostBlock = 128 << 20, kMostTotal = 256 << 20;
+constexpr int kFirstCredit = 2, kMostCredit = 8;
 struct HostBlocks {
   std::mutex mu;
   std::vector<std::pair<size_t, void*>> idle;
-  size_t total = 0;
+  size_t total = 0, blocks = 0;
+  int credit = kFirstCredit;
 };
 HostBlocks& host_blocks() {
   static HostBlocks* b = new HostBlocks();   // never destroyed: arrays may outlive the interpreter's own clean-up
@@ -952,25 +960,47 @@ PyObject* host_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
   void* ptr = nullptr;
   {
     std::lock_guard<std::mutex> lock(pool.mu);
-    for (size_t i = 0; i < pool.idle.size() && !ptr; ++i) {
-      if (pool.idle[i].first != bytes) continue;
-      ptr = pool.idle[i].second;
-      pool.idle.erase(pool.idle.begin() + static_cast<std::ptrdiff_t>(i));
-    }
-    // make room by giving back idle blocks of other sizes
-    while (!ptr && pool.total + bytes > kMostTotal && !pool.idle.empty()) {
-      pool.total -= pool.idle.back().first;
-      cudaFreeHost(pool.idle.back().second);
-      pool.idle.pop_back();
-    }
-    if (!ptr && pool.total + bytes <= kMostTotal) {
-      if (cudaHostAlloc(&ptr, bytes, cudaHostAllocPortable) == cudaSuccess) pool.total += bytes;
-      else cudaGetLastError();
+    // the smallest idle block that is large enough, and not more than twice as large
+    auto best = pool.idle.end();
+    for (auto it = pool.idle.begin(); it != pool.idle.end(); ++it)
+      if (it->first >= bytes && it->first <= 2 * bytes && (best == pool.idle.end() || it->first < best->first)) best = it;
+    if (best != pool.idle.end()) {
+      bytes = best->first;
+      ptr = best->second;
+      pool.idle.erase(best);
+      if (pool.credit < kMostCredit) ++pool.credit;
+    } else if (pool.credit > 0) {
+      // make room by giving back idle blocks of other sizes
+      while (pool.total + bytes > kMostTotal && !pool.idle.empty()) {
+        pool.total -= pool.idle.back().first;
+        --pool.blocks;
+        cudaFreeHost(pool.idle.back().second);
+        pool.idle.pop_back();
+      }
+      try {
+        pool.idle.reserve(pool.blocks + 1);   // a block that comes back needs no memory
+      } catch (const std::bad_alloc&) {
+        Py_RETURN_NONE;
+      }
+      if (pool.total + bytes <= kMostTotal) {
+        if (cudaHostAlloc(&ptr, bytes, cudaHostAllocPortable) == cudaSuccess) {
+          pool.total += bytes;
+          ++pool.blocks;
+          --pool.credit;
+        } else {
+          cudaGetLastError();
+          ptr = nullptr;
+        }
+      }
     }
   }
   if (!ptr) Py_RETURN_NONE;
   HostBlock* b = PyObject_New(HostBlock, &host_block_type);
-  if (!b) return nullptr;
+  if (!b) {
+    std::lock_guard<std::mutex> lock(pool.mu);
+    pool.idle.emplace_back(bytes, ptr);
+    return nullptr;
+  }
   b->ptr = ptr;
   b->bytes = bytes;
   b->asked = asked;
@@ -983,6 +1013,7 @@ PyObject* release_host_blocks(PyObject*, PyObject* const*, Py_ssize_t) {
   for (auto& b : pool.idle) {
     cudaFreeHost(b.second);
     pool.total -= b.first;
+    --pool.blocks;
   }
   pool.idle.clear();
   Py_RETURN_NONE;

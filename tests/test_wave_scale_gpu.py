@@ -546,3 +546,44 @@ def test_host_results_that_are_page_locked_in_part(bench_devices):
         torch.cuda.cudart().cudaHostUnregister(address)
     for n, v in outs.items():
         assert np.array_equal(v.view(np.uint8), want[n].view(np.uint8)), n
+
+
+def test_host_results_that_are_kept(bench_devices):
+    """Page-locked blocks are made for results that come back: a caller who keeps every result gets at most a few of
+    them, one who drops them soon has nothing else, and all results are those of the device entry point."""
+    import subprocess
+    import sys
+    import os
+    code = """
+import numpy as np, torch
+from habitat_b200 import batched, device_table, workloads
+from tests.helpers import to_numpy
+devs = device_table.load_device_file()
+bench = [devs[n] for n in workloads.BENCH_DEVICES]
+def make(K):
+    kernels = workloads.make_kernels(K, seed=K)
+    kernels["run_time_ns"] = kernels["run_time_ns"].astype(np.float32)
+    return kernels
+pinned = lambda res: torch.from_numpy(res["scaled_ns"]).is_pinned()
+kernels = make(9000)
+want = to_numpy(batched.wave_scale(batched.KernelBatch.from_numpy(kernels), bench[0], bench).scaled_ns)
+kept = [batched.wave_scale_host(kernels, bench[0], bench) for _ in range(12)]
+assert 1 <= sum(pinned(r) for r in kept) <= 3, [pinned(r) for r in kept]
+for r in kept:
+    assert np.array_equal(r["scaled_ns"].view(np.uint8), want.view(np.uint8))
+del kept, r
+for i in range(12):                     # a result lives while the next one is made
+    res = batched.wave_scale_host(kernels, bench[0], bench)
+    assert pinned(res)
+del res
+seen = []
+for K in [9000, 20000, 60000] * 8:      # other sizes follow
+    res = batched.wave_scale_host(make(K), bench[0], bench)
+    seen.append(pinned(res))
+    del res
+assert all(seen[6:]), seen
+print("kept results ok")
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and "kept results ok" in r.stdout, r.stdout + r.stderr
