@@ -16,10 +16,11 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <string>
 #include <thread>
 #include <type_traits>
 #include <vector>
@@ -1468,19 +1469,21 @@ struct HostPlanes {
 constexpr int kHostThreads = 4;
 constexpr size_t kHostDirectBytes = 32u << 20;   // of staged records
 
-// Results to ordinary memory.  Each thread takes every kHostThreads-th chunk.
+// Results to ordinary memory.  Each thread takes the next chunk, so it works with as many threads as start (where
+// a limit on threads is reached, with this one alone).
 hb_status host_in_threads(hb::HostArena* arena, const HostPlanes& io, const LaunchPlan& plan, int64_t K, int64_t chunk,
                           int threads, int device) {
   const size_t slot_bytes = io.in_bytes(chunk) + io.out_bytes(chunk);
   hb_status st = hb::arena_reserve_pinned(arena, slot_bytes * threads);
   if (st != HB_OK) return st;
-  hb_status got[kHostThreads];
-  std::string text[kHostThreads];
+  hb_status got[kHostThreads] = {};
+  char text[kHostThreads][256];
+  std::atomic<int64_t> next{0};
   auto work = [&](int w) {
     cudaStream_t s = w == 0 ? arena->stream : arena->more[w - 1];
     uint8_t* slot = arena->pinned + slot_bytes * w;
     hb_status mine = cudaSetDevice(device) == cudaSuccess ? HB_OK : HB_ERR_CUDA;
-    for (int64_t lo = chunk * w; lo < K && mine == HB_OK; lo += chunk * threads) {
+    for (int64_t lo = next.fetch_add(chunk); lo < K && mine == HB_OK; lo = next.fetch_add(chunk)) {
       const int64_t n = K - lo < chunk ? K - lo : chunk;
       Ptrs p{};
       uint8_t* results = io.stage(slot, lo, n, &p);
@@ -1491,15 +1494,19 @@ hb_status host_in_threads(hb::HostArena* arena, const HostPlanes& io, const Laun
       if (mine == HB_OK) io.fetch(results, lo, n);
     }
     got[w] = mine;
-    if (mine != HB_OK) text[w] = hb_last_error();
+    if (mine != HB_OK) std::snprintf(text[w], sizeof(text[w]), "%s", hb_last_error());
   };
   std::thread helpers[kHostThreads];
-  for (int w = 1; w < threads; ++w) helpers[w] = std::thread(work, w);
+  int started = 1;
+  try {
+    for (; started < threads; ++started) helpers[started] = std::thread(work, started);
+  } catch (const std::exception&) {   // no further thread to be had
+  }
   work(0);
-  for (int w = 1; w < threads; ++w) helpers[w].join();
-  for (int w = 0; w < threads; ++w) {
+  for (int w = 1; w < started; ++w) helpers[w].join();
+  for (int w = 0; w < started; ++w) {
     if (got[w] == HB_OK) continue;
-    hb::set_error("%s", text[w].c_str());   // the text of another thread
+    hb::set_error("%s", text[w]);   // the text of another thread
     return got[w];
   }
   return HB_OK;

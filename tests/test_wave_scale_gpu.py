@@ -587,3 +587,50 @@ print("kept results ok")
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
                        cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert r.returncode == 0 and "kept results ok" in r.stdout, r.stdout + r.stderr
+
+
+def test_host_entry_without_further_threads(tmp_path):
+    """Where no thread can be started (the process's limit), the host entry point does the work itself: a library
+    in front of the C library's lets none, one or two through."""
+    import os
+    import subprocess
+    import sys
+    (tmp_path / "threads.c").write_text("""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <errno.h>
+#include <pthread.h>
+int threads_left = -1, threads_refused = 0;
+int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* x) {
+  int (*real)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*) = dlsym(RTLD_NEXT, "pthread_create");
+  if (threads_left == 0) { ++threads_refused; return EAGAIN; }
+  if (threads_left > 0) --threads_left;
+  return real(t, a, f, x);
+}
+""")
+    shim = str(tmp_path / "threads.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-o", shim, str(tmp_path / "threads.c"), "-ldl"], check=True)
+    code = """
+import ctypes, sys
+import numpy as np
+from habitat_b200 import batched, device_table, workloads
+shim = ctypes.CDLL(sys.argv[1])
+left, refused = (ctypes.c_int.in_dll(shim, n) for n in ("threads_left", "threads_refused"))
+devs = device_table.load_device_file()
+bench = [devs[n] for n in workloads.BENCH_DEVICES]
+kernels = workloads.make_kernels(200_001, seed=12)
+call = lambda: batched.wave_scale_host(kernels, bench[0], bench, want_limits=True)    # results in ordinary memory
+want = call()
+for n in (0, 1, 2):
+    refused.value, left.value = 0, n
+    got = call()
+    left.value = -1
+    assert refused.value == 1, (n, refused.value)
+    for name, plane in want.items():
+        if plane is not None:
+            assert np.array_equal(got[name].view(np.uint8), plane.view(np.uint8)), (n, name)
+print("few threads ok")
+"""
+    r = subprocess.run([sys.executable, "-c", code, shim], env=dict(os.environ, LD_PRELOAD=shim), capture_output=True, text=True,
+                       timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and "few threads ok" in r.stdout, r.stdout + r.stderr
