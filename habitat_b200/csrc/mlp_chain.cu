@@ -1179,31 +1179,39 @@ extern "C" hb_status hb_mlp_predict_host(hb_mlp* h, const float* op_features,
     std::memset(p_o, 0xFF, 4 * q);
     float* p_f = p_o + q;
     uint8_t* p_r = reinterpret_cast<uint8_t*>(p_f) + f_bytes;
-    const hb::WidePlan plan = hb::wide_plan(Q, h->precision == HB_PRECISION_BF16X3, h->sm_count);
-    bool launched = false;
-    if (Q <= hb::kWideInline) {
-      hb::MlpBatch batch;
-      batch.feats = op_features; batch.dev_row = device_row; batch.Q = Q; batch.out = p_o;
-      batch.host_inputs = true;
-      const auto queue = hb::wide_queue(h->device);
-      st = hb::wide_predict(h, plan, batch, s, &launched);
-      if (st != HB_OK) return st;
-    }
-    if (!launched) {
+    hb::MlpBatch batch;
+    batch.Q = Q; batch.out = p_o;
+    const hb::WidePlan plan = plan_of(h, Q);
+    batch.host_inputs = plan.G != 0 && Q <= hb::kWideInline;
+    if (batch.host_inputs) {
+      batch.feats = op_features;
+      batch.dev_row = device_row;
+    } else {
       std::memcpy(p_f, op_features, f_bytes);
       std::memcpy(p_r, device_row, q);
-      float* d_f = p_f;
-      uint8_t* d_r = p_r;
-      if (plan.G == 0) {
+      batch.feats = p_f;
+      batch.dev_row = p_r;
+    }
+    {
+      const auto queue = hb::wide_queue(h->device);
+      bool launched = false;
+      st = hb::wide_predict(h, plan, batch, s, &launched);
+      if (st != HB_OK) return st;
+      if (!launched) {
         // the two-SM kernel reads a tile's features when it gets to the tile: they have to be near
+        if (batch.host_inputs) {
+          std::memcpy(p_f, op_features, f_bytes);
+          std::memcpy(p_r, device_row, q);
+          batch.host_inputs = false;
+        }
         st = hb::arena_reserve(arena, f_bytes + q);
         if (st != HB_OK) return st;
-        d_f = static_cast<float*>(arena->base);
-        d_r = static_cast<uint8_t*>(arena->base) + f_bytes;
-        HB_CUDA_TRY(cudaMemcpyAsync(d_f, p_f, f_bytes + q, cudaMemcpyHostToDevice, s));
+        batch.feats = static_cast<float*>(arena->base);
+        batch.dev_row = static_cast<uint8_t*>(arena->base) + f_bytes;
+        HB_CUDA_TRY(cudaMemcpyAsync(arena->base, p_f, f_bytes + q, cudaMemcpyHostToDevice, s));
+        st = queue_batch(h, hb::WidePlan{}, batch, s);
+        if (st != HB_OK) return st;
       }
-      st = hb_mlp_predict(h, d_f, d_r, Q, p_o, s);
-      if (st != HB_OK) return st;
     }
     st = hb::wait_written(p_o, q, s);
     if (st != HB_OK) return st;

@@ -510,3 +510,35 @@ def test_small_batches_on_ever_new_streams():
     for h in hs:
         h.check_status()
         h.close()
+
+
+def test_small_batches_switched_off():
+    """HB_MLP_WIDE=0 keeps every batch on the two-SM kernel, which leaves its cycle counters; without it small batches
+    from host memory leave none.  The predictions are the same."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import os
+import numpy as np, torch
+from habitat_b200 import batched, workloads
+feats, dev = workloads.make_queries("bmm", 300, 97)
+mu, sigma = workloads.batch_mu_sigma(feats, dev)
+w = workloads.init_mlp_weights("bmm", seed=2, layers=2, gain=2.0)
+want = None
+for Q in (300, 17, 16, 1):
+    h = batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=workloads.BENCH_DEVICE_FEATURES, **w)
+    got = h.predict_host(feats[:Q], dev[:Q])
+    want = got if want is None else want
+    assert np.array_equal(got, want[:Q]), Q
+    assert (h.phase_cycles()["slots"] > 0) == ("HB_MLP_WIDE" in os.environ), Q
+    h.close()
+print(want.tobytes().hex()[:200])
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    outs = []
+    for env in (dict(os.environ), dict(os.environ, HB_MLP_WIDE="0")):
+        r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300, cwd=root)
+        assert r.returncode == 0, r.stderr
+        outs.append(r.stdout)
+    assert outs[0] == outs[1]
