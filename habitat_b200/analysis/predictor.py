@@ -532,8 +532,9 @@ class Predictor:
         regs = None
         if flat is not None and self._has_registers():
             regs = wave_batch.destination_registers(plan.kernels, plan.names, dests, self._kernel_metadata)
-        nan, sums, clamped = _native.binding().run_group(
-            flat.batch if flat is not None else None, flat.metrics if flat is not None else None, origin, dests, regs,
+        nan, sums, clamped = batched._call(
+            "run_group", _native.binding().run_group, flat.batch if flat is not None else None,
+            flat.metrics if flat is not None else None, origin, dests, regs,
             plan.offsets_dev if flat is not None else None, kinds,
             (plan.overheads, plan.wave_idx, plan.fwd_run, plan.bwd_run), times, totals, ms)
         if nan:

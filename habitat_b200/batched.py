@@ -135,7 +135,9 @@ def wave_scale(kernels: KernelBatch, origin, dests: Sequence, dest_regs=None, me
     With `partials` the call also leaves the first stage of the per-destination totals there.
     Queued on the current stream; does not synchronise.
     """
-    res = _call("hb_wave_scale", _native.binding().wave_scale, kernels, origin, dests, dest_regs, metrics,
+    name = ("hb_wave_scale_partials" if partials is not None else
+            "hb_wave_scale" if metrics is None else "hb_wave_scale_metrics")
+    res = _call(name, _native.binding().wave_scale, kernels, origin, dests, dest_regs, metrics,
                 want_status, want_limits, out, partials)
     if res is None:
         _check_wave_arguments(kernels, dests, dest_regs, metrics, out, partials)
@@ -279,8 +281,8 @@ class MLPHandle:
     def predict_one(self, op_features, device_row):
         """One query, a sequence of F numbers and a device row; returns a float.  The query travels as a
         kernel parameter and the result comes back through page-locked memory."""
-        value = _native.binding().mlp_predict_one(self._handle.value or 0, self.n_op_features, op_features,
-                                                  device_row)
+        value = _call("hb_mlp_predict_host", _native.binding().mlp_predict_one, self._handle.value or 0,
+                      self.n_op_features, op_features, device_row)
         if value is None:
             raise ValueError("op_features must be [Q, %d]" % self.n_op_features)
         return value

@@ -54,7 +54,8 @@ def predict_iteration_totals(kernels: batched.KernelBatch, overhead_ns: torch.Te
             raise ValueError("op_features must be [Q, %d]" % ops.handle.n_op_features)
         kinds.append((ops.handle._handle.value or 0, ops.features.contiguous(), ops.run_time_ms, ops.offsets, rows))
     res = batched.wave_scale(kernels, origin, dests)
-    totals = _native.binding().iteration_totals(kernels, res.scaled_ns, overhead_ns, kernel_offsets, same, kinds)
+    totals = batched._call("iteration_totals", _native.binding().iteration_totals, kernels, res.scaled_ns, overhead_ns,
+                           kernel_offsets, same, kinds)
     if totals is None:
         batched._require_cuda(overhead_ns, torch.float32, "overhead_ns")
         batched._require_cuda(kernel_offsets, torch.int64, "kernel_offsets")

@@ -273,3 +273,27 @@ def test_weights_dropped_during_a_prediction_live_until_it_ends(monkeypatch):
         special_inputs=lambda name, operations, order: (None, None, np.ones(1, np.float32), order))
     predictor._run_plan(plan, [], Device.V100, [Device.T4], np.zeros((1, 1)))
     assert closed == [77] and pred._handle is None
+
+
+def test_ranges_on_a_timeline(monkeypatch):
+    """With HABITAT_B200_NVTX every native call stands in a range of its own name, closed also when it fails."""
+    import torch
+    from habitat_b200 import batched
+    opened, closed = [], []
+    monkeypatch.setattr(batched, "_NVTX", True)
+    monkeypatch.setattr(torch.cuda.nvtx, "range_push", opened.append)
+    monkeypatch.setattr(torch.cuda.nvtx, "range_pop", lambda: closed.append(1))
+    zeros = lambda dtype: torch.zeros(4, dtype=dtype)
+    kernels = batched.KernelBatch(zeros(torch.int32), zeros(torch.uint16), zeros(torch.uint16), zeros(torch.uint32),
+                                  zeros(torch.float32), zeros(torch.float32))
+    metrics = batched.KernelMetricsBatch(*[zeros(torch.float64)] * 3, zeros(torch.uint8))
+    for more in ({}, dict(metrics=metrics), dict(partials=batched.WavePartials(4, 1, device="cpu"))):
+        with pytest.raises(TypeError):                      # CPU tensors
+            batched.wave_scale(kernels, Device.V100, [Device.T4], **more)
+    handle = object.__new__(batched.MLPHandle)
+    handle.n_op_features, handle._handle = 4, type("Closed", (), {"value": None})()
+    handle.close = lambda: None
+    with pytest.raises(ValueError):
+        handle.predict_one([1.0, 2.0], 0)
+    assert opened == ["hb_wave_scale", "hb_wave_scale_metrics", "hb_wave_scale_partials", "hb_mlp_predict_host"]
+    assert len(closed) == 4
