@@ -3,9 +3,9 @@
 // A small launch is bound by the host: through ctypes, wave_scale spent 45 us on argument objects, five
 // allocations, device look-ups and structure building for a kernel of 5 us.  This module reads the torch
 // tensors directly, makes small results in one allocation and calls the C ABI through function addresses
-// that _native.py hands over (so that another build of the library can stand in).  It holds no arithmetic
-// and no state but those addresses.  Every argument is checked as batched.py documents; a check that fails
-// makes the function return None, and the caller's Python checks then raise the error.
+// that _native.py hands over (so that another build of the library can stand in).  Its state is those addresses
+// and the pool of page-locked blocks for host results.  Every argument is checked as batched.py documents; a check
+// that fails makes the function return None, and the caller's Python checks then raise the error.
 #include <Python.h>
 
 #include <ATen/EmptyTensor.h>
@@ -901,9 +901,10 @@ PyObject* submit_wave(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // larger block.
 //
 // Page-locking costs about 0.3 ms per MB, so it must not recur: 65,536 kernels on six devices take 0.16 ms into a
-// block that has come back, 1.0 ms into fresh pages and 2.2 ms with a new block.  So a new one needs credit: two to begin with (a loop that keeps one result while the next
-// is made), one more for each time a block is used again, kMostCredit at most.  A caller who keeps every result
-// pays for two blocks and then gets ordinary memory; so does one whose sizes push one another out of the pool.
+// block that has come back, 1.0 ms into fresh pages and 2.2 ms with a new block.  So a new one needs credit: two to
+// begin with (a loop that keeps one result while the next is made), one more for each time a block is used again,
+// kMostCredit at most.  A caller who keeps every result pays for two blocks and then gets ordinary memory; so does
+// one whose sizes push one another out of the pool.
 constexpr size_t kMostBlock = 128 << 20, kMostTotal = 256 << 20;
 constexpr int kFirstCredit = 2, kMostCredit = 8;
 struct HostBlocks {

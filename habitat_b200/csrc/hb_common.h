@@ -26,9 +26,11 @@ inline hb_status cuda_fail(cudaError_t e, const char* what) {
 // ---------------------------------------------------------------------------
 // Staging for the `_host` entry points: one device block per GPU that only ever
 // grows, and one non-blocking stream per GPU, both kept for the life of the
-// process.  A `_host` call holds the arena's mutex from its first copy to its
-// final synchronise, so calls on one GPU run one after the other and the block
-// can be re-carved (and, when too small, replaced) without anything in flight.
+// process.  A `_host` call holds the arena's mutex from its first copy until it has
+// synchronised, or (hb_mlp_predict_host) has seen every result that its launches
+// write: what they read is read by then.  So calls on one GPU run one after the
+// other, and the block can be re-carved (and, when too small, replaced) with nothing
+// in flight that still uses it.
 // ---------------------------------------------------------------------------
 namespace hb {
 struct HostArena {

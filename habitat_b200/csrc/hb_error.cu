@@ -49,7 +49,7 @@ hb_status arena_for_current_device(HostArena** out) {
 
 hb_status arena_reserve(HostArena* a, size_t bytes) {
   if (bytes <= a->bytes) return HB_OK;
-  // nothing of an earlier call is in flight: every `_host` call ends with a synchronise
+  // nothing in flight still uses the block (see HostArena)
   if (a->base) cudaFree(a->base);
   a->base = nullptr;
   a->bytes = 0;

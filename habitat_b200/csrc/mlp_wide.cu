@@ -367,7 +367,10 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
       bool ok = true;
       const long long t0 = clock64();
       if (W == 32) {
-        // what is asked for before the others can have written it only delays what they write
+        // What is asked for before the others can have written it only delays what they write.  The two shapes of 32
+        // columns gain (without and with, us: 300 queries 32.9 / 32.1, 480 32.6 / 32.2, 1,056 48.6 / 48.0; split, 150
+        // 48.0 / 46.4, 500 77.9 / 77.2; 200 cycles gain less, 500 about as much).  With 16 columns the values come
+        // sooner (one query 23.3 / 23.7), with 64 later than any pause (960 48.0 / 48.0).
         while (clock64() - t0 < 350) {}
       }
 #pragma unroll
@@ -782,7 +785,7 @@ WidePlan wide_plan(int64_t Q, bool split, int sm_count) {
 // rarely fit on the GPU together: the second then waits for the first.  A shape takes the same time with few
 // groups as with many, so the shortest way through is the lowest time at which all batches fit when each takes
 // the narrowest shape of that time or less, unless one after the other is shorter.  What is left of the GPU goes
-// to cheaper shapes for the batches that start last.  Three predictors with 318, 192 and 6 queries: 60 -> 48 us.
+// to cheaper shapes for the batches that start last.  Three predictors with 318, 192 and 6 queries: 60 -> 51 us.
 void wide_plans_together(WidePlan* plans, const int64_t* Q, const bool* split, int n, int sm_count) {
   auto us_of = [&](const Shape& s, int b) { return split[b] ? s.us_split : s.us; };
   auto share_of = [&](const WidePlan& w, const Shape& s) {   // of the clusters that run at a time

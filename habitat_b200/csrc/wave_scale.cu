@@ -511,9 +511,11 @@ __device__ __forceinline__ void store_byte_pair(uint8_t* q, uint32_t pair_word, 
 constexpr int kTotMaxD = 16;
 
 // EXT: 0 plain, 1 with the status plane and per-destination registers, 2 and 3 with gamma from metrics as well,
-// whose float64 values take 20 registers.  With 56 registers (2) nine blocks fit an SM, with 48 (3) ten: batches
-// of more than two fills of the first are 7 % faster with the second (4,000,000 kernels x 6: 117 -> 109 us),
-// smaller ones 5 to 15 % slower (500,000 x 6: 17.4 -> 18.2 us, 250,000 x 13: 21.0 -> 24.0).
+// whose float64 values take 20 registers.  With 56 registers (2) nine blocks fit an SM, with 48 (3) ten.  Batches of
+// more than two fills of the first take the second: with register counts it is 4 to 8 % faster (4,000,000 kernels x 6:
+// 113.7 -> 105.4 us, 11,184,812 x 6: 310 -> 287), without them up to 5 % faster with one or two destinations (8,000,000
+// x 1: 73.7 -> 69.9) and 1 to 4 % slower with more (4,000,000 x 6: 81.8 -> 84.8).  Smaller batches are slower with the
+// second (500,000 x 6: 17.4 -> 18.2 us, 250,000 x 13: 21.0 -> 24.0, with register counts).
 template <int VEC, int EXT, bool ALIGNED, int NW, int TOT = 0>
 __global__ void __launch_bounds__(kLutThreads, EXT == 2 ? 8 : (EXT == 3 ? 10 : 12))
 wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
@@ -544,7 +546,7 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
     if (!with_metrics) gv = load_pair<float, VEC, ALIGNED>(p.gamma + k0, pair);
     Vec<double, VEC> fev, rdv, wrv;
     Vec<uint8_t, VEC> hmv;
-    if (with_metrics) {   // all on their way at once, not the values behind the flag (4,000,000 x 6: 117 -> 109 us)
+    if (with_metrics) {   // all on their way at once, not the values behind the flag (3,000,000 x 2: 39.1 -> 35.7 us)
       hmv = load_each<uint8_t, VEC>(p.has_metrics + k0, pair);
       fev = load_each<double, VEC>(p.flop_eff + k0, pair);
       rdv = load_each<double, VEC>(p.dram_read + k0, pair);
@@ -633,7 +635,7 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
 
     // The plain instances keep what they know about a record in masks: six predicates that live through the loop
     // leave none for the body, and the masks go into one logic operation per question (11,184,812 x 6 with totals:
-    // 184 -> 174 us, 8,388,608 x 6: 122 -> 116).
+    // 175 -> 173.8 us, 8,388,608 x 6: 117.5 -> 116.3).
     uint32_t no_blocks[2], not_live[2], not_fit[2];
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
@@ -1574,7 +1576,7 @@ extern "C" hb_status hb_wave_scale_host(const hb_kernel_soa* kernels, int64_t K,
   cudaStream_t s;
   // per-destination registers keep rows of their own, block limits are written by the generic kernel alone
   if (!dest_regs && !out->limits && io.in_bytes(K) <= kHostDirectBytes && io.results_page_locked()) {
-    // eight chunks or more of 8,192 records: 10 us of staging each
+    // at most eight chunks, of at least 8,192 records: 10 us of staging each
     int64_t chunk = (K / 8 + 255) & ~int64_t{255};
     if (chunk < 8192) chunk = 8192;
     st = hb::arena_stream(arena, 1, &s);

@@ -163,7 +163,8 @@ class WaveScaleHost(_Streams):
                      for k, t in self.host_out[slot].items()]
         plain = all(t.dtype is d.dtype and t.shape == d.shape and t.is_contiguous() for t, d in downloads)
         res = batched._call(
-            "submit_wave", _native.binding().submit_wave, block.contiguous(), self.dev_block[slot], self.dev_in[slot], self.origin, self.dests, self.dev_out[slot],
+            "submit_wave", _native.binding().submit_wave, block.contiguous(), self.dev_block[slot], self.dev_in[slot],
+            self.origin, self.dests, self.dev_out[slot],
             self.partials[slot] if with_totals else None, self.dev_totals[slot] if with_totals else None,
             downloads if plain else [], self._stream_handles, self._event_handles[slot], self.used[slot])
         if res is None:
