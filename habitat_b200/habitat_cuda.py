@@ -46,13 +46,15 @@ class DeviceProperties:
     # The remembered row is one of this process's table: it stays out of pickles and copies, and out of
     # objects whose pickle holds one.
     def __getstate__(self):
-        state = dict(self.__dict__, _fields=dict(self._fields))
-        state.pop("_row_token", None)
+        state = {k: v for k, v in self.__dict__.items() if k != "_row_token"}
+        if "_fields" in state:                   # a subclass may keep its values otherwise
+            state["_fields"] = dict(state["_fields"])
         return state
 
     def __setstate__(self, state):
-        self.__dict__.update(state, _fields=types.MappingProxyType(dict(state["_fields"])))
-        self.__dict__.pop("_row_token", None)
+        self.__dict__.update((k, v) for k, v in state.items() if k != "_row_token")
+        if "_fields" in state:
+            self._fields = types.MappingProxyType(dict(state["_fields"]))
 
     def __repr__(self):
         return "DeviceProperties(name=" + self._name + ")"

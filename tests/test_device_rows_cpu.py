@@ -92,3 +92,13 @@ def test_copies_and_other_classes_are_looked_up(device_file):
         changing.spec = device_file[name].spec_tuple()
         assert device_table.row_of(changing) == device_table.row_of(device_file[name])
         assert not hasattr(changing, "_row_token")
+
+    class Elsewhere(DeviceProperties):
+        def __init__(self, spec):
+            self._name, self.spec = "y", spec
+
+        def spec_tuple(self):
+            return self.spec
+
+    kept = copy.deepcopy(Elsewhere(device.spec_tuple()))
+    assert kept.spec_tuple() == device.spec_tuple() and device_table.row_of(kept) == device_table.row_of(device)
