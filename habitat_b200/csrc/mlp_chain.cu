@@ -33,9 +33,8 @@
 // one ring slot: see the comment at the kernel).
 //
 // Warp roles: warp 0 = TMEM allocation, warp 1 = barrier set-up + MMA issuer (leader CTA),
-// warps 2-5 and 12-15 = two epilogue groups (one TMEM lane quadrant per warp), warps 6-11 =
-// weight producers.  Bulk copies issued by one thread complete one after the other (measured:
-// about 750 cycles each whatever their size), so each ring slot has its own issuing warp.
+// warps 2-5 and 12-15 = two epilogue groups (one TMEM lane quadrant per warp), warps 6-8 =
+// weight producers, warps 9 and 10 = features.
 // Every mbarrier wait is bounded: when a wait runs out the kernel records a status word, the roles
 // leave their loops or run them empty (the two epilogue groups keep meeting at their common barriers, which
 // have no limit of their own), outstanding bulk copies and MMAs are waited for (bounded) and TMEM is released.
@@ -69,8 +68,7 @@ struct MlpProblem {
   float* out;                // [Q]
   int32_t* status;           // 0 ok, else (role << 8 | site)
   uint8_t grid_rows[hb::kMaxGridRows];
-  CUtensorMap tmap_slot;     // the weight pack as [rows][128 B], box of two tile images (32 KB)
-  CUtensorMap tmap_tile;     // same tensor, box of one tile image (16 KB, fc1)
+  CUtensorMap tmap_tile;     // the weight pack as [rows][128 B], box of one tile image (16 KB)
 };
 // A launch takes the tiles of up to four predictors, one after the other in one list, so that only the
 // list's end leaves SMs idle.
@@ -121,10 +119,14 @@ __device__ __forceinline__ const MlpProblem& problem_of(const MlpParams& p, int 
 constexpr int kPairQ = 128;                 // queries per cluster tile
 constexpr int kPairHalfQ = 64;              // activation rows resident per CTA
 constexpr int kPairMT = kWidth / 256;       // 4 MMA row blocks per layer
-constexpr int kPairSlotKb = 2;               // weight tiles (K blocks of 64) per ring slot
-constexpr int kPairStages = 6 / kPairSlotKb; // ring slots: 96 KB in all
-constexpr int kPairStageBytes = kPairSlotKb * kTileBytes;
-static_assert(kPairStages <= 6, "one producer warp per ring slot, warps 6-11");
+// Ring of weight tiles, 96 KB in all.  From the commit that frees a slot to its next tile in place it takes 1,100 to
+// 1,300 cycles (710 to 900 of them the copy), while a tile lasts the tensor core 256.  Three slots of 32 KB with a
+// producer each did not cover that; six of 16 KB do, just: 65,536 split queries 3,251 -> 3,084 us, 4,194,304 of
+// bf16 57.0 -> 55.8 ms.
+constexpr int kPairStages = 6;
+constexpr int kPairProducers = 3;            // warps 6-8, two slots each; six measured the same, two 2 % slower (split)
+constexpr int kPairStageBytes = kTileBytes;
+static_assert(kPairStages == 2 * kPairProducers && kPairProducers == 3, "warps 6-8, two slots each");
 constexpr int kPairActKb = kPairHalfQ * 128;          // 8 KB per K block
 constexpr int kPairActBytes = kNumKB * kPairActKb;    // 128 KB
 // Order of the 16 (output block j, K quarter q) units of a hidden layer, four bits each
@@ -135,9 +137,7 @@ constexpr int kPairActBytes = kNumKB * kPairActKb;    // 128 KB
 // tensor core works on the remaining blocks; the next layer consumes the quarters in the
 // same order.
 constexpr uint64_t kPairOrder = 0xFBEA76D95321C840ull;
-__device__ __forceinline__ int pair_unit_j(uint64_t order, int u) { return static_cast<int>((order >> (4 * u + 2)) & 3u); }
-__device__ __forceinline__ int pair_unit_q(uint64_t order, int u) { return static_cast<int>((order >> (4 * u)) & 3u); }
-constexpr int kPairThreads = 512;              // warps: 0 alloc, 1 MMA, 2-5 + 12-15 epilogue, 6-11 producers
+constexpr int kPairThreads = 512;              // warps: 0 alloc, 1 MMA, 2-5 + 12-15 epilogue, 6-8 producers, 9-10 features
 constexpr int kPairSmemBytes = kPairActBytes + kPairStages * kPairStageBytes + 1024 + 1024;
 static_assert(kPairSmemBytes <= 232448, "over the 227 KB shared-memory limit");
 
@@ -148,8 +148,8 @@ __device__ __forceinline__ void pair_epi_bar_sync() {
 // SPLIT = true (the 1e-4 mode): activations and weights are kept as bf16 hi + lo parts.  A CTA
 // holds 32 queries and lays the hi and lo parts of an activation side by side along N (the 128-byte
 // B row of K index k is [hi of 32 queries | lo of 32 queries]), so the same M = 256, N = 128 MMA
-// multiplies a weight tile with both parts at once, at full rate; a ring slot carries the hi and the
-// lo image of one K block of weights and both accumulate into the same TMEM columns:
+// multiplies a weight tile with both parts at once, at full rate; the hi and the lo image of a K block
+// of weights follow one another through the ring and accumulate into the same TMEM columns:
 // D = (W_hi + W_lo) [x_hi | x_lo], and the epilogue adds the two column halves of a query (all four
 // partial products, fp32 accumulation).  Two MMAs per K step and 64 queries instead of one and 128:
 // a quarter of the bf16 rate.
@@ -158,7 +158,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
   constexpr int kTileQ = SPLIT ? kPairQ / 2 : kPairQ;          // queries per cluster tile
   constexpr int kHalfQ = kTileQ / 2;                           // queries per CTA
-  constexpr int kLoadsPerUnit = SPLIT ? 4 : 4 / kPairSlotKb;   // ring slots per (block, K quarter) unit
+  constexpr int kLoadsPerUnit = SPLIT ? 8 : 4;                 // ring slots per (block, K quarter) unit
   constexpr int kRowsPerImage = (SPLIT ? 2 : 1) * (kTileBytes / 128);   // 128-byte rows per packed K block
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -233,66 +233,62 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
     else mbar_arrive_remote(map_to_cta(bar, 0));
   };
 
-  if (warp >= 6 && warp < 6 + kPairStages) {
+  if (warp >= 6 && warp < 6 + kPairProducers) {
     // ------------------------------ producers -----------------------------
-    // One producer per ring slot.  The pack is laid out per 128-feature block
-    // (layer -> block -> K block); this CTA streams blocks 2 j + rank.
+    // The pack is laid out per 128-feature block (layer -> block -> K block); this CTA streams blocks 2 j + rank,
+    // a hidden layer as 16 (block, K quarter) units of four K blocks each (fc1 has only one).  What a load needs
+    // is worked out before the wait for its slot, so that only the request stands between the two (a dozen
+    // instructions more there cost the split mode 4 %).
     if (lane == 0) {
+      constexpr int kLayerLoads = 16 * kLoadsPerUnit;
       const uint32_t w = static_cast<uint32_t>(warp - 6);
-      uint32_t it = 0;
+      uint32_t s = w, ph = 1;
+      uint32_t n = w;              // load of the tile
       bool ok = true;
-      const bool ptimed = p.phase_cycles != nullptr && blockIdx.x == 0 && w == 0;
-      const uint32_t peer_full_leader = map_to_cta(bar_full + 8 * w, 0);
-      long long pc_empty = 0, pc_copy = 0, pc_n = 0;
+      const bool timed = p.phase_cycles != nullptr && blockIdx.x == 0 && w == 0;
+      long long c_empty = 0, c_first = 0;
       for (int t = 0; t < my_tiles && ok; ++t) {
         const MlpProblem& pb = problem_of(p, pair_id + t * n_pairs);
-        const int n_layers = pb.layers + 1;
-        size_t layer_base = 0;   // in tile images
-        for (int L = 0; L < n_layers && ok; ++L) {
-          const int nkb = L == 0 ? 1 : kNumKB;
-          // A ring slot takes two consecutive K blocks of one output block (fc1 has only one);
-          // a hidden layer is streamed as 16 (block, K quarter) units of two slots each.
-          const int n_units = nkb == 1 ? kPairMT : 16;
-          const int n_loads = nkb == 1 ? 1 : kLoadsPerUnit;
-          const uint32_t load_bytes = nkb == 1 ? kTileBytes : kPairStageBytes;
-          {
-            for (int u = 0; u < n_units && ok; ++u) {
-              const int j = nkb == 1 ? u : pair_unit_j(kPairOrder, u);
-              const int kq = nkb == 1 ? 0 : pair_unit_q(kPairOrder, u);
-              const size_t blk = layer_base + static_cast<size_t>(2 * j + rank) * nkb + kq * 4;
-              for (int g = 0; g < n_loads; ++g, ++it) {
-                if (it % kPairStages != w) continue;
-                const uint32_t ph = (it / kPairStages) & 1u;
-                const long long q0 = ptimed ? clock64() : 0;
-                if (!mbar_wait(bar_empty + 8 * w, ph ^ 1u, abort_flag, pb.status, 0x111)) { ok = false; break; }
-                const long long q1 = ptimed ? clock64() : 0;
-                // both CTAs' boxes are counted on the leader's barrier
-                if (rank == 0) mbar_expect_tx(bar_full + 8 * w, 2 * load_bytes);
-                // bf16: a slot takes two consecutive K blocks (16 KB images); split: the hi and lo
-                // image of one K block (stored back to back)
-                tma_rows_2sm(stage0 + w * kPairStageBytes, nkb == 1 ? &pb.tmap_tile : &pb.tmap_slot,
-                             static_cast<int32_t>((blk + (SPLIT ? 1 : kPairSlotKb) * g) * kRowsPerImage),
-                             peer_full_leader);
-                issued = it + 1;
-                if (ptimed) {
-                  mbar_wait(bar_full + 8 * w, ph, abort_flag, pb.status, 0x112);
-                  pc_empty += q1 - q0; pc_copy += clock64() - q1; ++pc_n;
-                }
-              }
+        const uint32_t tile_loads = static_cast<uint32_t>(kPairMT + pb.layers * kLayerLoads);
+        for (; n < tile_loads; n += kPairProducers) {
+          uint32_t image = 2 * n + rank, g = 0;              // fc1: block n
+          if (n >= kPairMT) {
+            const uint32_t m = n - kPairMT, L = m / kLayerLoads, u = m % kLayerLoads / kLoadsPerUnit;
+            const uint32_t unit = static_cast<uint32_t>(kPairOrder >> (4 * u)) & 15u;
+            g = m % kLoadsPerUnit;
+            image = kNumMT + (L * kNumMT + 2 * (unit >> 2) + rank) * kNumKB + (unit & 3u) * 4;
+          }
+          // split: a K block's hi and lo image are stored back to back
+          const int32_t row = static_cast<int32_t>(image * kRowsPerImage + g * (kTileBytes / 128));
+          const uint32_t dst = stage0 + s * kPairStageBytes, full = bar_full + 8 * s;
+          const uint32_t full_leader = map_to_cta(full, 0);   // both CTAs' boxes are counted there
+          const long long c0 = timed ? clock64() : 0;
+          if (!mbar_wait(bar_empty + 8 * s, ph, abort_flag, pb.status, 0x111)) { ok = false; break; }
+          if (rank == 0) mbar_expect_tx(full, 2 * kPairStageBytes);
+          tma_rows_2sm(dst, &pb.tmap_tile, row, full_leader);
+          if (timed) {
+            // (waiting for every copy here, to time it, held up the ring: 2 % of the launch)
+            c_empty += clock64() - c0;
+            if (issued == 0) {
+              mbar_wait(full, 0, abort_flag, pb.status, 0x112);
+              c_first = clock64() - c0;
             }
           }
-          layer_base += static_cast<size_t>(kNumMT) * nkb;
+          ++issued;
+          s += kPairProducers;
+          if (s >= kPairStages) { s = w; ph ^= 1u; }
         }
+        n -= tile_loads;
       }
-      if (ptimed) { p.phase_cycles[9] = pc_empty; p.phase_cycles[10] = pc_copy; p.phase_cycles[11] = pc_n; }
+      if (timed) { p.phase_cycles[9] = c_empty; p.phase_cycles[10] = c_first; p.phase_cycles[11] = issued; }
     }
   } else if (warp == 1) {
     if (rank == 0) {
       // ------------------------------ MMA issuer (leader) -------------------
       // One elected lane (elect.sync) runs the whole loop, and no loop depends on what a wait returns
       // (after a wait that ran out the abort flag is set, and what is issued on stale operands is
-      // discarded), which keeps the descriptors in uniform registers: eight MMAs and their commit are
-      // queued in 150 cycles of the 512 they take.  The barrier of the next slot is tested while they run.
+      // discarded), which keeps the descriptors in uniform registers: four MMAs and their commit are
+      // queued in about 100 cycles of the 256 they take.  The barrier of the next slot is tested while they run.
       // D fp32, A/B bf16, A K-major, B MN-major (bit 16), N = 128, M = 256
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
                                  (static_cast<uint32_t>(kPairQ >> 3) << 17) |
@@ -361,17 +357,14 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
                 uint32_t next = s, next_ph = ph;
                 ring_next<kPairStages>(next, next_ph);
                 const uint32_t a_lo = a_lo0 + s * (kPairStageBytes >> 4);
-                const uint32_t b_lo = b_lo0 + (kq * 4 + (SPLIT ? 1 : kPairSlotKb) * g) * (kPairActKb >> 4);
+                const uint32_t b_lo = b_lo0 + (kq * 4 + (SPLIT ? g >> 1 : g)) * (kPairActKb >> 4);
                 if (!landed) wait(bar_full + 8 * s, ph, mc_full, 0x212);
 #pragma unroll
-                for (int k = 0; k < 4 * kPairSlotKb; ++k) {
-                  // a K step of 16: 32 bytes along an A row, 16 K rows (2 KB) of B.  Second image of the slot
-                  // (16 KB on): bf16: the next K block, i.e. the next 64 K rows of the activations (8 KB on);
-                  // split: the lo part of the same K block, same activations
-                  tc_mma_pair_bf16(d_tmem, desc_hi | (a_lo + (k >> 2) * (kTileBytes >> 4) + 2 * (k & 3)),
-                                   desc_hi | (b_lo + (SPLIT ? 0 : (k >> 2) * (kPairActKb >> 4)) + 128 * (k & 3)), idesc,
+                for (int k = 0; k < 4; ++k) {
+                  // a K step of 16: 32 bytes along an A row, 16 K rows (2 KB) of B
+                  tc_mma_pair_bf16(d_tmem, desc_hi | (a_lo + 2 * k), desc_hi | (b_lo + 128 * k), idesc,
                                    (g == 0 && k == 0) ? u >> 2 : 1u);
-                  if (k == 4) {
+                  if (k == 1) {
                     landed = mbar_try_wait_cluster(bar_full + 8 * next, next_ph);
                     tc_fence_after();
                   }
@@ -675,12 +668,14 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
   // ------------------------------ teardown ------------------------------
   tc_fence_before();
   __syncthreads();
-  if (rank == 0 && warp >= 6 && warp < 6 + kPairStages && lane == 0 && *abort_flag && issued > 0) {
-    const uint32_t j = issued - 1;
-    const uint32_t ph = (j / kPairStages) & 1u;
+  if (rank == 0 && warp >= 6 && warp < 6 + kPairProducers && lane == 0 && *abort_flag && issued > 0) {
+    // this producer's last copies, one per slot of its own
     const long long t0 = clock64();
-    while (!mbar_try_wait(bar_full + 8 * (warp - 6), ph)) {
-      if (clock64() - t0 > kWaitCycles) break;
+    for (uint32_t i = 0; i < 2 && i < issued; ++i) {
+      const uint32_t own = issued - 1 - i;
+      const uint32_t s = static_cast<uint32_t>(warp - 6) + own % 2 * kPairProducers;
+      while (!mbar_try_wait(bar_full + 8 * s, (own / 2) & 1u))
+        if (clock64() - t0 > kWaitCycles) break;
     }
   }
   if (rank == 0 && warp == 1 && *abort_flag && elect_one()) {
@@ -859,7 +854,7 @@ extern "C" hb_status hb_mlp_create(hb_mlp** handle, int32_t n_op_features, int32
     const cuuint64_t strides[1] = {128};
     const cuuint32_t elem[2] = {1, 1};
     for (int which = 0; which < 2; ++which) {
-      const cuuint32_t box[2] = {128, static_cast<cuuint32_t>((which == 0 ? kPairStageBytes : kTileBytes) / 128)};
+      const cuuint32_t box[2] = {128, static_cast<cuuint32_t>((which == 0 ? 2 : 1) * kTileBytes / 128)};
       const CUresult r = reinterpret_cast<EncodeFn>(fn)(
           which == 0 ? &h->tmap_slot : &h->tmap_tile, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, h->wpack, dims, strides,
           box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -927,7 +922,7 @@ class ChainLaunch {
     q.dev_row = batch.dev_row; q.Q = batch.Q; q.out = batch.out; q.status = h->status;
     q.grid_n = batch.grid_n;
     if (batch.grid_n) std::memcpy(q.grid_rows, batch.grid_rows, static_cast<size_t>(batch.Q / batch.grid_n));
-    q.tmap_slot = h->tmap_slot; q.tmap_tile = h->tmap_tile;
+    q.tmap_tile = h->tmap_tile;
     p_.num_tiles += static_cast<int32_t>(tiles);
     return HB_OK;
   }

@@ -260,8 +260,8 @@ hb_status hb_mlp_inject_status(hb_mlp* handle, int32_t device_status);
  * for the most recent launch.  out[0..3] first epilogue group: waiting for its
  * output blocks, draining them, fc2, layers counted.  out[4..8] MMA issuer:
  * waiting for activations, for weights, for TMEM blocks to be read out, issuing,
- * ring slots counted.  out[9..11] first producer: waiting for a free slot, copy
- * latency, copies counted.  out[12], out[13]: the MMA issuer's whole loop in SM
+ * ring slots counted.  out[9..11] first producer: waiting for a free slot and
+ * requesting a copy, latency of the launch's first copy, copies counted.  out[12], out[13]: the MMA issuer's whole loop in SM
  * cycles and in nanoseconds (their ratio is the SM clock under load).
  * out[14], out[15] first epilogue group: hand-over of a drained block, stores
  * into the peer CTA.  Synchronises.  No reference counterpart. */
