@@ -131,12 +131,18 @@ constexpr int kPairActKb = kPairHalfQ * 128;          // 8 KB per K block
 constexpr int kPairActBytes = kNumKB * kPairActKb;    // 128 KB
 // Order of the 16 (output block j, K quarter q) units of a hidden layer, four bits each
 // (4 j + q), first unit in the low bits:
-//   (0,0) (1,0) (2,0) (3,0) | (0,1) (0,2) (0,3) | (1,1) (2,1) (3,1) | (1,2) (1,3) | (2,2) (3,2) | (2,3) | (3,3)
-// Block j completes after 7, 12, 15, 16 units, and by then no later unit reads quarter j,
+//   (0,0) (0,1) (1,0) (1,1) (2,0) (3,0) (0,2) (0,3) | (2,1) (3,1) (1,2) (1,3) | (2,2) (3,2) (2,3) | (3,3)
+// Block j completes after 8, 12, 15, 16 units, and by then no later unit reads quarter j,
 // so the epilogue of block j can replace quarter j of the activations in place while the
 // tensor core works on the remaining blocks; the next layer consumes the quarters in the
-// same order.
-constexpr uint64_t kPairOrder = 0xFBEA76D95321C840ull;
+// same order.  What the last epilogues of a layer hold up, TMEM blocks 2 and 3 and quarters 2 and 3, comes
+// as late as that allows in the next one, after five to seven units of 1,024 cycles.
+// 109.1 -> 106.3 us for one round of tiles (with (1,0) (2,0) (3,0) in units 1 to 3 the issuer waited 2,700 cycles a
+// layer for TMEM blocks); split precision, whose units last twice as long, takes the same time either way.
+constexpr uint64_t kPairOrder = 0xFBEA76D932C85410ull;
+constexpr uint32_t kPairFirstOfBlock = 0x35;     // units that write a TMEM block for the first time in the layer
+constexpr uint32_t kPairFirstOfQuarter = 0xC3;   // ... that read a K quarter for the first time
+constexpr uint32_t kPairLastOfBlock = 0xC880;    // ... that complete a block
 constexpr int kPairThreads = 512;              // warps: 0 alloc, 1 MMA, 2-5 + 12-15 epilogue, 6-8 producers, 9-10 features
 constexpr int kPairSmemBytes = kPairActBytes + kPairStages * kPairStageBytes + 1024 + 1024;
 static_assert(kPairSmemBytes <= 232448, "over the 227 KB shared-memory limit");
@@ -339,14 +345,13 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
               const uint32_t unit = ((u < 8 ? static_cast<uint32_t>(kPairOrder) : static_cast<uint32_t>(kPairOrder >> 32)) >>
                                      (4 * (u & 7u))) & 15u;
               const uint32_t j = unit >> 2, kq = unit & 3u;
-              if (u < 7) {
-                // units 0-3 write a TMEM block for the first time (the previous layer's values must be out);
-                // units 0, 4, 5, 6 are the first to read their K quarter
-                if (u < 4) {
+              if (u < 8) {
+                // (the previous layer's values must be out)
+                if ((kPairFirstOfBlock >> u) & 1u) {
                   wait(bar_tfree + 8 * j, (par >> (4 + j)) & 1u, mc_tfree, 0x213);
                   par ^= 16u << j;
                 }
-                if (u == 0 || u >= 4) {
+                if ((kPairFirstOfQuarter >> u) & 1u) {
                   wait(bar_actq + 8 * kq, (par >> kq) & 1u, mc_act, 0x211);
                   par ^= 1u << kq;
                 }
@@ -363,7 +368,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
                 for (int k = 0; k < 4; ++k) {
                   // a K step of 16: 32 bytes along an A row, 16 K rows (2 KB) of B
                   tc_mma_pair_bf16(d_tmem, desc_hi | (a_lo + 2 * k), desc_hi | (b_lo + 128 * k), idesc,
-                                   (g == 0 && k == 0) ? u >> 2 : 1u);
+                                   (g == 0 && k == 0) ? kq : 1u);
                   if (k == 1) {
                     landed = mbar_try_wait_cluster(bar_full + 8 * next, next_ph);
                     tc_fence_after();
@@ -373,8 +378,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
                 s = next;
                 ph = next_ph;
               }
-              // the last units of blocks 0..3 (kPairOrder)
-              if ((0xC840u >> u) & 1u) tc_commit_pair(bar_accj + 8 * j);
+              if ((kPairLastOfBlock >> u) & 1u) tc_commit_pair(bar_accj + 8 * j);
             }
             mc_n += 16 * kLoadsPerUnit;
           }
