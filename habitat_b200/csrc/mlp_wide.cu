@@ -240,6 +240,52 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     return static_cast<uint32_t>(((p.parity[use & 1] >> group) + static_cast<unsigned>(use >> 1)) & 1ull) << 31;
   };
 
+  const int64_t q0 = static_cast<int64_t>(group) * p.per_group;
+  const int n_q = static_cast<int>(min(static_cast<int64_t>(p.per_group), static_cast<int64_t>(p.Q) - q0));
+  // fc1's B operand: K rows 0..63 hold [hi | lo | hi] of the normalised features, one query per column.  Epilogue
+  // and receivers, who have nothing else to do yet, share the work: a value takes two dependent loads and a float64
+  // division, 1,100 cycles, and the epilogue's 128 threads alone took three rounds with 32 queries, six with 64
+  // (100 queries 25.1 -> 24.3 us, 900 48.2 -> 46.5, 2,000 75.1 -> 74.1).  A function that both roles call: as a step
+  // before the roles part it made every layer 30 % slower.  In split precision, with half the queries, it gained
+  // nothing and cost 1 to 2 % from 150 queries on: epilogue alone.
+  constexpr bool kAllFeatures = !SPLIT;
+  auto features = [&]() {
+    constexpr int kThreads = kAllFeatures ? wide_threads<W>() - 128 : 128;
+    auto feat_sync = [] { asm volatile("bar.sync 2, %0;" ::"n"(kThreads) : "memory"); };
+    const int T = static_cast<int>(threadIdx.x) - 128;
+    const int C_in = p.n_op_feat + 4;
+    for (int i = T; i < 64 * 2 * W / 16; i += kThreads) *reinterpret_cast<uint4*>(base_ptr + 16 * i) = make_uint4(0, 0, 0, 0);
+    feat_sync();
+    for (int i = T; i < n_q * C_in; i += kThreads) {
+      const int q = i / C_in, f = i - q * C_in;
+      const int own = static_cast<int>(q0) + q;                 // of the launch's queries
+      int64_t fr = p.first + own;
+      int dr;
+      if (p.grid_n) {
+        const uint32_t block = static_cast<uint32_t>(fr) / static_cast<uint32_t>(p.grid_n);
+        fr -= static_cast<int64_t>(block) * p.grid_n;
+        dr = p.grid_rows[block];
+      } else {
+        dr = p.inline_q ? p.inline_row[own] : p.dev_row[fr];
+      }
+      dr = dr < p.n_dev ? dr : p.n_dev - 1;
+      const double x = f < p.n_op_feat ? static_cast<double>(p.inline_q ? p.inline_feats[own * p.n_op_feat + f]
+                                                                             : p.feats[fr * p.n_op_feat + f])
+                                       : p.dev_feat[dr * 4 + (f - p.n_op_feat)];
+      const float xn = static_cast<float>((x - p.mu[f]) / p.sigma[f]);
+      const __nv_bfloat16 hi = __float2bfloat16_rn(xn);
+      const __nv_bfloat16 lo = __float2bfloat16_rn(xn - __bfloat162float(hi));
+      const uint32_t ch = static_cast<uint32_t>(q) >> 3, in = 2u * (static_cast<uint32_t>(q) & 7u);
+      *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<W>(f, ch) + in) = hi;
+      *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<W>(C_in + f, ch) + in) = lo;
+      *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<W>(2 * C_in + f, ch) + in) = hi;
+    }
+    fence_proxy_async();
+    feat_sync();
+    if (T < kReceivers) mbar_arrive(bar_act);
+    __syncwarp();
+  };
+
   if (*poisoned) {
     // nothing has been started
   } else if (warp == 1) {
@@ -355,6 +401,7 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     constexpr int kLoads = SPLIT ? 2 : 1;
     constexpr int kUnits = static_cast<int>(kQuarterBytes) / (16 * kLoads) / (32 * kReceivers);   // per thread
     static_assert(kUnits >= 1, "a unit per thread and quarter");
+    if (kAllFeatures) features();
     for (int L = 1; L < n_layers; ++L) {
       // the tensor core has read the previous layer's input
       if (!warp_wait(bar_acc + 8 * (kBlocks - 1), (L - 1) & 1, lane, abort_flag, p, 0x531)) break;
@@ -431,41 +478,7 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     const int quad = warp & 3;
     const int T = static_cast<int>(threadIdx.x) - 128;          // 0..127
     auto epi_sync = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
-    const int64_t q0 = static_cast<int64_t>(group) * p.per_group;
-    const int n_q = static_cast<int>(min(static_cast<int64_t>(p.per_group), static_cast<int64_t>(p.Q) - q0));
-    const int C_in = p.n_op_feat + 4;
-
-    // fc1's B operand: K rows 0..63 hold [hi | lo | hi] of the normalised features, one query per column
-    for (int i = T; i < 64 * 2 * W / 16; i += 128) *reinterpret_cast<uint4*>(base_ptr + 16 * i) = make_uint4(0, 0, 0, 0);
-    epi_sync();
-    for (int i = T; i < n_q * C_in; i += 128) {
-      const int q = i / C_in, f = i - q * C_in;
-      const int own = static_cast<int>(q0) + q;                 // of the launch's queries
-      int64_t fr = p.first + own;
-      int dr;
-      if (p.grid_n) {
-        const uint32_t block = static_cast<uint32_t>(fr) / static_cast<uint32_t>(p.grid_n);
-        fr -= static_cast<int64_t>(block) * p.grid_n;
-        dr = p.grid_rows[block];
-      } else {
-        dr = p.inline_q ? p.inline_row[own] : p.dev_row[fr];
-      }
-      dr = dr < p.n_dev ? dr : p.n_dev - 1;
-      const double x = f < p.n_op_feat ? static_cast<double>(p.inline_q ? p.inline_feats[own * p.n_op_feat + f]
-                                                                             : p.feats[fr * p.n_op_feat + f])
-                                       : p.dev_feat[dr * 4 + (f - p.n_op_feat)];
-      const float xn = static_cast<float>((x - p.mu[f]) / p.sigma[f]);
-      const __nv_bfloat16 hi = __float2bfloat16_rn(xn);
-      const __nv_bfloat16 lo = __float2bfloat16_rn(xn - __bfloat162float(hi));
-      const uint32_t ch = static_cast<uint32_t>(q) >> 3, in = 2u * (static_cast<uint32_t>(q) & 7u);
-      *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<W>(f, ch) + in) = hi;
-      *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<W>(C_in + f, ch) + in) = lo;
-      *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<W>(2 * C_in + f, ch) + in) = hi;
-    }
-    fence_proxy_async();
-    epi_sync();
-    if (T < kReceivers) mbar_arrive(bar_act);
-
+    features();
     // M = 64 leaves 16 rows in the low lanes of every quadrant, M = 128 all 32
     const bool row_ok = kM == 128 || lane < 16;
     const int row = kM == 128 ? quad * 32 + lane : quad * 16 + (lane & 15);
