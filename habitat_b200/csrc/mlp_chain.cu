@@ -969,7 +969,7 @@ hb_status check_device(const hb_mlp* h) {
 // HB_MLP_WIDE=0 keeps every batch on the two-SM kernel
 hb::WidePlan plan_of(const hb_mlp* h, int64_t Q) {
   static const bool use_wide = [] { const char* e = std::getenv("HB_MLP_WIDE"); return !e || std::atoi(e) != 0; }();
-  return use_wide ? hb::wide_plan(Q, h->precision == HB_PRECISION_BF16X3, h->sm_count) : hb::WidePlan{0, 0, 0, 0};
+  return use_wide ? hb::wide_plan(Q, h->precision == HB_PRECISION_BF16X3, h->sm_count) : hb::WidePlan{};
 }
 
 // A last round of few tiles takes as long as a full one, and the kernel for small batches is quicker: it takes the
@@ -977,7 +977,7 @@ hb::WidePlan plan_of(const hb_mlp* h, int64_t Q) {
 // 220 -> 140 us, 28,916: 435 -> 378; split, 5,792: 376 -> 335.
 hb_status queue_tail(ChainLaunch* launch, hb_mlp* h, hb::MlpBatch batch, cudaStream_t s, int* launches) {
   const int64_t n = launch->tail();
-  const hb::WidePlan plan = n ? plan_of(h, n) : hb::WidePlan{0, 0, 0, 0};
+  const hb::WidePlan plan = n ? plan_of(h, n) : hb::WidePlan{};
   if (plan.G == 0) return HB_OK;
   batch.first = batch.Q - n;
   batch.Q = n;

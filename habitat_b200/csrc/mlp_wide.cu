@@ -74,16 +74,19 @@ struct WideParams {
 // Receiver warps: enough that 64 columns, too, need only four 16-byte loads per thread and K quarter.
 template <int W>
 constexpr int wide_receivers() { return W == 64 ? 16 : 8; }
-template <int W>
-constexpr int wide_threads() { return 256 + 32 * wide_receivers<W>(); }
+template <int W, bool NEAR>
+constexpr int wide_threads() { return 256 + (NEAR ? 0 : 32 * wide_receivers<W>()); }
 constexpr int kWideSlotBytes = 2 * kTileBytes;
 constexpr int kWideCols = 64;    // queries per group at most
 
-template <int W>
-constexpr int wide_slots() { return W == 64 ? 3 : (W == 32 ? 5 : 6); }
-template <int W>
-constexpr int wide_smem() { return 2048 * W + wide_slots<W>() * kWideSlotBytes + 1024 + 512; }
-static_assert(wide_smem<64>() <= 232448 && wide_smem<32>() <= 232448 && wide_smem<16>() <= 232448, "shared memory");
+template <int W, bool NEAR>
+constexpr int wide_slots() { return W == 64 ? 3 : (W == 32 || NEAR ? 5 : 6); }
+template <int W, bool NEAR>
+constexpr int wide_act_bytes() { return (NEAR ? 2 : 1) * 2048 * W; }
+template <int W, bool NEAR>
+constexpr int wide_smem() { return wide_act_bytes<W, NEAR>() + wide_slots<W, NEAR>() * kWideSlotBytes + 1024 + 512; }
+static_assert(wide_smem<64, false>() <= 232448 && wide_smem<32, false>() <= 232448 &&
+              wide_smem<16, false>() <= 232448 && wide_smem<16, true>() <= 232448, "shared memory");
 
 __device__ __forceinline__ uint4 ld_relaxed_v4(const void* p) {
   uint4 v;
@@ -167,12 +170,20 @@ __device__ __forceinline__ uint32_t b_chunk(uint32_t k, uint32_t chunk) {
   return k * (2u * W) + ((chunk ^ x) << 4);
 }
 
-template <int G, int W, bool SPLIT>
-__global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __grid_constant__ WideParams p) {
+// NEAR: groups of up to six queries (split: three) exchange through distributed shared memory instead.  B is K-major,
+// so that a block's share of a query is 128 contiguous bytes, which eight threads store into each of the other
+// blocks (st.async, counted in bytes on the barrier of the buffer); two buffers alternate by layer, for the reason
+// given above.  An all-gather of 128 bytes per block takes 750 cycles, of 1 KB 1,500, of 2 KB 2,400 (about 14 bytes
+// a cycle), while the way through L2 moves whole rows of columns, filled or not: 1,140 cycles to the first K quarter and
+// 600 to each further one.  One query 23.6 -> 19.1 us, 14: 23.6 -> 20.5, 42: 23.9 -> 23.8, 56: 24.0 -> 25.5
+// (not taken); split, one 33.1 -> 28.9, 14: 33.4 -> 31.0, 28: 33.9 either way (not taken).
+template <int G, int W, bool SPLIT, bool NEAR>
+__global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(const __grid_constant__ WideParams p) {
+  static_assert(!NEAR || (G == 16 && W == 16), "one K block of 64 features per block");
   constexpr int kM = G == 16 ? 64 : 128;              // weight rows per MMA
   constexpr int kBlocks = kWidth / G / kM;            // row blocks per thread block
-  constexpr int kCols = SPLIT ? W / 2 : W;            // queries a group can hold
-  constexpr int kSlots = wide_slots<W>();
+  constexpr int kCols = SPLIT || NEAR ? W / 2 : W;    // queries a group can hold
+  constexpr int kSlots = wide_slots<W, NEAR>();
   constexpr int kReceivers = wide_receivers<W>();
   constexpr int kParts = SPLIT ? 2 : 1;               // images per packed K block
   constexpr int kUnitBytes = kM * 128;                // one K block of the rows
@@ -184,11 +195,11 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - raw);
   const uint32_t act = base;
-  const uint32_t ring = base + 2048u * W;
+  const uint32_t ring = base + wide_act_bytes<W, NEAR>();
   const uint32_t bars = ring + kSlots * kWideSlotBytes;
   uint8_t* bars_ptr = base_ptr + (bars - base);
   const uint32_t bar_full = bars, bar_empty = bars + 64;      // [kSlots]
-  const uint32_t bar_act = bars + 128;                        // [4] K quarter in place
+  const uint32_t bar_act = bars + 128;                        // [4] K quarter in place; NEAR: [2] buffer in place
   const uint32_t bar_acc = bars + 160;                        // [kBlocks] row block accumulated
   const uint32_t bar_tfree = bars + 192;                      // TMEM read out (4 warps)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_ptr + 200);
@@ -204,13 +215,15 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
       mbar_init(bar_full + 8 * s, 1);
       mbar_init(bar_empty + 8 * s, 1);
     }
-    for (int q = 0; q < 4; ++q) mbar_init(bar_act + 8 * q, kReceivers);
+    for (int q = 0; q < 4; ++q) mbar_init(bar_act + 8 * q, NEAR ? 1 : kReceivers);
     for (int b = 0; b < kBlocks; ++b) mbar_init(bar_acc + 8 * b, 1);
     mbar_init(bar_tfree, 4);
     mbar_init(bar_drain, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // (before the peers' first stores)
+  if (NEAR) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   constexpr uint32_t kTmemCols = kBlocks * W < 32 ? 32 : kBlocks * W;
   if (threadIdx.x == 64 && !p.beside) hb_grid_wait();   // the mark may be a fresh buffer's
   if (threadIdx.x == 64 && *reinterpret_cast<volatile int32_t*>(p.poison) != 0) {
@@ -227,6 +240,7 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   grid_begin(p.beside != 0);
+  if (NEAR) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -248,9 +262,9 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
   // (100 queries 25.1 -> 24.3 us, 900 48.2 -> 46.5, 2,000 75.1 -> 74.1).  A function that both roles call: as a step
   // before the roles part it made every layer 30 % slower.  In split precision, with half the queries, it gained
   // nothing and cost 1 to 2 % from 150 queries on: epilogue alone.
-  constexpr bool kAllFeatures = !SPLIT;
+  constexpr bool kAllFeatures = !SPLIT && !NEAR;
   auto features = [&]() {
-    constexpr int kThreads = kAllFeatures ? wide_threads<W>() - 128 : 128;
+    constexpr int kThreads = kAllFeatures ? wide_threads<W, NEAR>() - 128 : 128;
     auto feat_sync = [] { asm volatile("bar.sync 2, %0;" ::"n"(kThreads) : "memory"); };
     const int T = static_cast<int>(threadIdx.x) - 128;
     const int C_in = p.n_op_feat + 4;
@@ -276,13 +290,14 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
       const __nv_bfloat16 hi = __float2bfloat16_rn(xn);
       const __nv_bfloat16 lo = __float2bfloat16_rn(xn - __bfloat162float(hi));
       const uint32_t ch = static_cast<uint32_t>(q) >> 3, in = 2u * (static_cast<uint32_t>(q) & 7u);
-      *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<W>(f, ch) + in) = hi;
-      *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<W>(C_in + f, ch) + in) = lo;
-      *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<W>(2 * C_in + f, ch) + in) = hi;
+      auto at = [&](int k) { return NEAR ? swz_off(q, k) : b_chunk<W>(k, ch) + in; };
+      *reinterpret_cast<__nv_bfloat16*>(base_ptr + at(f)) = hi;
+      *reinterpret_cast<__nv_bfloat16*>(base_ptr + at(C_in + f)) = lo;
+      *reinterpret_cast<__nv_bfloat16*>(base_ptr + at(2 * C_in + f)) = hi;
     }
     fence_proxy_async();
     feat_sync();
-    if (T < kReceivers) mbar_arrive(bar_act);
+    if (T < (NEAR ? 1 : kReceivers)) mbar_arrive(bar_act);
     __syncwarp();
   };
 
@@ -315,16 +330,18 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     }
   } else if (warp == 0) {
     // ------------------------------ MMA issuer ------------------------------
-    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (static_cast<uint32_t>(W >> 3) << 17) |
-                               (static_cast<uint32_t>(kM >> 4) << 24);
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (NEAR ? 0u : 1u << 16) |
+                               (static_cast<uint32_t>(W >> 3) << 17) | (static_cast<uint32_t>(kM >> 4) << 24);
     // A: K-major, 128-byte swizzle, 8-row groups 1024 B apart; B: MN-major, one swizzle atom wide, 8-row
-    // groups of K 16 W bytes apart
+    // groups of K 16 W bytes apart; NEAR: K-major like A, 16 rows (queries) of 128 bytes per K block
     const uint64_t desc_a = (static_cast<uint64_t>(1024 >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
                             (static_cast<uint64_t>(2) << 61) | (static_cast<uint64_t>(1) << 16);
-    const uint64_t desc_b = (static_cast<uint64_t>((16 * W) >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
-                            (static_cast<uint64_t>(W == 64 ? 2 : (W == 32 ? 4 : 6)) << 61) |
-                            (static_cast<uint64_t>(1) << 16);
-    constexpr uint32_t kStepB = (32 * W) >> 4;                 // 16 K rows of B, in 16-byte units
+    const uint64_t desc_b = NEAR ? desc_a
+                                 : (static_cast<uint64_t>((16 * W) >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
+                                       (static_cast<uint64_t>(W == 64 ? 2 : (W == 32 ? 4 : 6)) << 61) |
+                                       (static_cast<uint64_t>(1) << 16);
+    // in 16-byte units: 16 K values of B, a K block of 64
+    constexpr uint32_t kStepB = NEAR ? 2 : (32 * W) >> 4, kBlockB = (128 * W) >> 4;
     const uint32_t a_lo0 = (ring & 0x3FFFF) >> 4, b_lo0 = (act & 0x3FFFF) >> 4;
     // One elected lane runs the whole loop.  An MMA of these shapes takes 24 to 49 cycles and only a
     // couple of them queue up, so what stands between two MMAs shows: the wait for the next slot goes
@@ -337,9 +354,20 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
         wide_wait(bar, parity, abort_flag, p, code);
         tc_fence_after();
       };
+      // layer L's input: its first K quarter (which has one phase more than the others, fc1's input); NEAR: the whole
+      // of buffer L & 1, written by the peers
+      auto wait_input = [&](int L) {
+        if (!NEAR) {
+          wait(bar_act, L & 1, 0x521);
+          return;
+        }
+        if (!mbar_wait_cluster(bar_act + 8 * (L & 1), (L >> 1) & 1, abort_flag, p.status, 0x521)) atomicExch(p.poison, 1);
+        fence_proxy_async();
+        tc_fence_after();
+      };
       uint32_t s = 0, ph = 0;
       for (int b = 0; b < kBlocks; ++b) {                        // fc1: one K block
-        if (b == 0) wait(bar_act, 0, 0x521);
+        if (b == 0) wait_input(0);
         wait(bar_full + 8 * s, ph, 0x522);
         const uint32_t d = tmem_base + static_cast<uint32_t>(b * W);
         const uint32_t a_lo = a_lo0 + s * (kWideSlotBytes >> 4);
@@ -359,24 +387,24 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
         for (int b = 0; b < kBlocks; ++b) {
           const uint32_t d = tmem_base + static_cast<uint32_t>(b * W);
           wait(bar_full + 8 * s, ph, 0x522);
-          if (b == 0) wait(bar_act, L & 1, 0x521);
+          if (b == 0) wait_input(L);
           uint32_t prev = 0;
 #pragma unroll 1
           for (int g = 0; g < kSlotsPerBlock; ++g) {
             uint32_t next = s, next_ph = ph;
             ring_next<kSlots>(next, next_ph);
             const uint32_t a_lo = a_lo0 + s * (kWideSlotBytes >> 4);
-            const uint32_t b_lo = b_lo0 + static_cast<uint32_t>(g) * (4 * kStepB * kUnitsPerSlot / kParts);
+            const uint32_t b_lo = b_lo0 + (NEAR ? static_cast<uint32_t>(L & 1) * (kNumKB * kBlockB) : 0u) +
+                                  static_cast<uint32_t>(g) * (kBlockB * kUnitsPerSlot / kParts);
 #pragma unroll
             for (int u = 0; u < kMmas; ++u) {
               mma_one_bf16(d, desc_a | (a_lo + (u >> 2) * (kUnitBytes >> 4) + 2 * (u & 3)),
-                           desc_b | (b_lo + ((u >> 2) / kParts * 4 + (u & 3)) * kStepB), idesc,
+                           desc_b | (b_lo + (u >> 2) / kParts * kBlockB + (u & 3) * kStepB), idesc,
                            u == 0 ? static_cast<uint32_t>(g) : 1u);
               if (u == 1 && g > 0) commit_one(bar_empty + 8 * prev);
               if (u == kMmas / 2 && g + 1 < kSlotsPerBlock) {
                 wait(bar_full + 8 * next, next_ph, 0x522);
-                // quarter 0 has one phase more than the others (fc1's input)
-                if (b == 0 && (g + 1) % kPerQuarter == 0)
+                if (!NEAR && b == 0 && (g + 1) % kPerQuarter == 0)
                   wait(bar_act + 8 * ((g + 1) / kPerQuarter), (L - 1) & 1, 0x521);
               }
             }
@@ -495,10 +523,13 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
         const float bias = __ldg(p.bias + L * kWidth + f);
         const float w2 = last ? __ldg(p.fc2_w + f) : 0.0f;
         ok = ok && warp_wait(bar_acc + 8 * b, L & 1, lane, abort_flag, p, 0x541);
-        if (!ok) break;
+        if (!ok) {
+          if (NEAR && !last) epi_sync();
+          break;
+        }
         tc_fence_after();
         // up to 32 columns at a time (split: 16 queries, their hi and their lo column)
-        constexpr int kPiece = SPLIT ? (W == 16 ? 8 : 16) : (W < 32 ? W : 32);
+        constexpr int kPiece = kCols < 16 ? 8 : (SPLIT || W < 32 ? 16 : 32);
         const uint32_t t_block = t_lane + static_cast<uint32_t>(b * W);
 #pragma unroll 1
         for (int q1 = 0; q1 < kCols; q1 += kPiece) {
@@ -519,7 +550,35 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
           }
 #pragma unroll
           for (int i = 0; i < kPiece; ++i) v[i] = fmaxf(v[i] + bias, 0.0f);
-          if (!last) {
+          if (NEAR && !last) {
+            // own features first, then the group's other blocks: 128 bytes of every query
+            const uint32_t mine = static_cast<uint32_t>((L + 1) & 1) * (2048u * W) + static_cast<uint32_t>(c) * (128u * W);
+            const uint32_t in_bar = bar_act + 8 * ((L + 1) & 1);
+#pragma unroll
+            for (int q = 0; q < kPiece; ++q) {
+              if (!row_ok || q >= n_q) continue;
+              const __nv_bfloat16 hi = __float2bfloat16_rn(v[q]);
+              *reinterpret_cast<__nv_bfloat16*>(base_ptr + mine + swz_off(q, row)) = hi;
+              if (SPLIT)
+                *reinterpret_cast<__nv_bfloat16*>(base_ptr + mine + swz_off(W / 2 + q, row)) =
+                    __float2bfloat16_rn(v[q] - __bfloat162float(hi));
+            }
+            fence_proxy_async();
+            epi_sync();
+            if (T == 0) mbar_expect_tx(in_bar, static_cast<uint32_t>((G - 1) * kParts * 128 * n_q));
+            const uint32_t chunk = static_cast<uint32_t>(T) & 7u, to = static_cast<uint32_t>(c + (T >> 3)) % G;
+            if (T >= 8) {   // eight threads per peer, 16 bytes of each query
+              const uint32_t there = map_to_cta(base + mine, to), bar = map_to_cta(in_bar, to);
+              for (uint32_t q = 0; q < static_cast<uint32_t>(n_q); ++q)
+#pragma unroll
+                for (uint32_t part = 0; part < kParts; ++part) {
+                  const uint32_t at = (part * (W / 2) + q) * 128u + (((chunk ^ q) & 7u) << 4);
+                  const uint4 x = *reinterpret_cast<const uint4*>(base_ptr + mine + at);
+                  st_async_v4(there + at, x.x, x.y, x.z, x.w, bar);
+                }
+            }
+            __syncwarp();
+          } else if (!last) {
             constexpr int kWords = SPLIT ? kPiece : kPiece / 2;
             uint32_t w[kWords];
 #pragma unroll
@@ -621,6 +680,13 @@ __global__ void __launch_bounds__(wide_threads<W>(), 1) mlp_wide_kernel(const __
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
   }
+  if (NEAR && (*abort_flag || *poisoned)) {
+    // A block that has everything it waited for has been sent all that will be.  One that gave up may still be
+    // written to: it stays until the others have left or given up as well (their waits are bounded), and a
+    // little longer for what is on its way.
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    for (const long long t0 = clock64(); clock64() - t0 < 100000;) {}
+  }
   grid_end(p.beside != 0);
 }
 }  // namespace
@@ -714,13 +780,13 @@ StreamScratch* scratch_of(GpuScratch& g, cudaStream_t stream, int lane) {
 }
 
 // Launches one shape; *fits = false (nothing launched) where the GPU cannot hold one such cluster.
-template <int G, int W, bool SPLIT>
+template <int G, int W, bool SPLIT, bool NEAR = false>
 cudaError_t launch(const WideParams& p, int groups, int device, cudaStream_t stream, bool* fits) {
   static std::atomic<int> clusters[kMaxCudaDevices];   // 1 + clusters the GPU runs at a time, 0: not asked yet
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(groups * G));
-  cfg.blockDim = dim3(wide_threads<W>());
-  cfg.dynamicSmemBytes = wide_smem<W>();
+  cfg.blockDim = dim3(wide_threads<W, NEAR>());
+  cfg.dynamicSmemBytes = wide_smem<W, NEAR>();
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -733,22 +799,23 @@ cudaError_t launch(const WideParams& p, int groups, int device, cudaStream_t str
   cfg.numAttrs = 1;   // for the occupancy question
   int n = clusters[device].load(std::memory_order_acquire);
   if (n == 0) {
-    cudaError_t e = cudaFuncSetAttribute(mlp_wide_kernel<G, W, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         wide_smem<W>());
+    cudaError_t e = cudaFuncSetAttribute(mlp_wide_kernel<G, W, SPLIT, NEAR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         wide_smem<W, NEAR>());
     if (e == cudaSuccess && G > 8)
-      e = cudaFuncSetAttribute(mlp_wide_kernel<G, W, SPLIT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      e = cudaFuncSetAttribute(mlp_wide_kernel<G, W, SPLIT, NEAR>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     int active = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&active, mlp_wide_kernel<G, W, SPLIT>, &cfg);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&active, mlp_wide_kernel<G, W, SPLIT, NEAR>, &cfg);
     if (e != cudaSuccess) return e;
     n = 1 + active;
     clusters[device].store(n, std::memory_order_release);
   }
   *fits = n > 1;
   cfg.numAttrs = hb::overlapped_launch_enabled() ? 2 : 1;
-  return *fits ? cudaLaunchKernelEx(&cfg, mlp_wide_kernel<G, W, SPLIT>, p) : cudaSuccess;
+  return *fits ? cudaLaunchKernelEx(&cfg, mlp_wide_kernel<G, W, SPLIT, NEAR>, p) : cudaSuccess;
 }
 template <bool SPLIT>
 cudaError_t launch(const hb::WidePlan& w, const WideParams& p, int device, cudaStream_t s, bool* fits) {
+  if (w.near) return launch<16, 16, SPLIT, true>(p, w.groups, device, s, fits);
   switch (w.G * 100 + w.W) {
     case 1616: return launch<16, 16, SPLIT>(p, w.groups, device, s, fits);
     case 816: return launch<8, 16, SPLIT>(p, w.groups, device, s, fits);
@@ -767,19 +834,22 @@ namespace hb {
 // (L2 and shared-memory fill bound), wider ones exchange more per layer (L2 latency and bandwidth); the
 // shapes below are those that no other one beats at its capacity.  Measured per launch, conv2d predictor,
 // 8 hidden layers (capacity in queries: time), against 125 us (bf16) and 190 us (split) before:
-//   bf16   112: 25 us   240: 29   480: 32   960: 48   1,056: 48   2,112: 75
+//   bf16    42: 24 us (one: 19)   112: 24 us   240: 28   480: 32   960: 48   1,056: 48   2,112: 75
 //   split   56: 34       120: 42   240: 46             528: 77     1,056: 128
 // Eight blocks x 64 columns lose to four x 32 in split precision (86 us for 480).  Beyond the last shape
 // the two-SM kernel of mlp_chain.cu is the faster one.
 namespace {
-struct Shape { int G, W, clusters, us, us_split; };   // us: what a launch of the shape takes, full or not
-constexpr Shape kShapes[] = {{16, 16, 7, 25, 34},  {8, 16, 15, 29, 42},  {8, 32, 15, 32, 46},
-                             {8, 64, 15, 48, 1000}, {4, 32, 33, 48, 77}, {4, 64, 33, 75, 128}};
+// us: what a launch of the shape takes, full or not
+struct Shape { int G, W, clusters, us, us_split; bool near; };
+constexpr Shape kShapes[] = {{16, 16, 7, 22, 31, true},  {16, 16, 7, 25, 34, false}, {8, 16, 15, 29, 42, false},
+                             {8, 32, 15, 32, 46, false}, {8, 64, 15, 48, 1000, false}, {4, 32, 33, 48, 77, false},
+                             {4, 64, 33, 75, 128, false}};
 int clusters_of(const Shape& s, int sm_count) { return sm_count >= 148 ? s.clusters : s.clusters * sm_count / 148; }
-WidePlan plan_in(const Shape& s, int64_t Q, bool split) {
+int cols_of(const Shape& s, bool split) { return s.near ? (split ? 3 : 6) : (split ? s.W / 2 : s.W); }
+WidePlan plan_in(const Shape& s, int64_t Q, bool split, int cols = 0) {
   // full groups while they last: fewer groups move the weights fewer times
-  const int cols = split ? s.W / 2 : s.W;
-  WidePlan w{s.G, s.W, static_cast<int>((Q + cols - 1) / cols), 0};
+  if (cols == 0) cols = cols_of(s, split);
+  WidePlan w{s.G, s.W, static_cast<int>((Q + cols - 1) / cols), 0, s.near};
   w.per_group = static_cast<int>((Q + w.groups - 1) / w.groups);
   w.groups = static_cast<int>((Q + w.per_group - 1) / w.per_group);
   return w;
@@ -789,9 +859,11 @@ WidePlan plan_in(const Shape& s, int64_t Q, bool split) {
 WidePlan wide_plan(int64_t Q, bool split, int sm_count) {
   for (const Shape& s : kShapes) {
     if (split && s.G == 8 && s.W == 64) continue;
-    if (Q <= static_cast<int64_t>(clusters_of(s, sm_count)) * (split ? s.W / 2 : s.W)) return plan_in(s, Q, split);
+    const int clusters = clusters_of(s, sm_count);
+    if (Q > static_cast<int64_t>(clusters) * cols_of(s, split)) continue;
+    return plan_in(s, Q, split, s.near ? static_cast<int>((Q + clusters - 1) / clusters) : 0);
   }
-  return WidePlan{0, 0, 0, 0};
+  return WidePlan{};
 }
 
 // Shapes for batches that run side by side.  The cheapest shape of each is the most spread out, and two of them
@@ -808,7 +880,7 @@ void wide_plans_together(WidePlan* plans, const int64_t* Q, const bool* split, i
   int in_turn = 0;
   for (int b = 0; b < n; ++b)
     for (const Shape& s : kShapes)
-      if (s.G == plans[b].G && s.W == plans[b].W) in_turn += us_of(s, b);
+      if (s.G == plans[b].G && s.W == plans[b].W && s.near == plans[b].near) in_turn += us_of(s, b);
   for (const Shape& level : kShapes) {
     WidePlan take[kMaxLanes];
     double least[kMaxLanes], all = 0.0;
@@ -911,7 +983,7 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
   const unsigned long long groups = (1ull << w.groups) - 1;
   for (int b = 0; b < 2; ++b) {
     p.parity[b] = s->parity[width][b];
-    if (((h->layers + 1 - b) / 2) & 1) s->parity[width][b] ^= groups;
+    if (!w.near && (((h->layers + 1 - b) / 2) & 1)) s->parity[width][b] ^= groups;
   }
   p.map_slot = w.G == 16 ? h->tmap_wide_slot : h->tmap_slot;
   p.map_fc1 = w.G == 16 ? h->tmap_wide_fc1 : h->tmap_tile;

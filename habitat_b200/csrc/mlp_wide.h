@@ -8,9 +8,11 @@
 struct hb_mlp;
 
 namespace hb {
-// G blocks per group (0: not for this batch), W columns per group, groups, queries per group.
+// G blocks per group (0: not for this batch), W columns per group, groups, queries per group; near: the exchange
+// goes through distributed shared memory.
 struct WidePlan {
   int G, W, groups, per_group;
+  bool near;
 };
 WidePlan wide_plan(int64_t Q, bool split, int sm_count);
 // Queries that can travel as kernel parameters: no copy and no read over PCIe for the scalar API.

@@ -266,6 +266,26 @@ def test_small_batches(precision):
     h.close()
 
 
+@pytest.mark.parametrize("precision", ["bf16", "bf16x3"])
+@pytest.mark.parametrize("layers", [1, 2, 3, 8])
+def test_few_queries(precision, layers):
+    """Up to 42 queries (split: 21) run on at most seven groups of up to six (three), which exchange their activations
+    through distributed shared memory, two buffers in turn: odd and even numbers of layers, every size up to the first
+    that runs otherwise, each prediction with the bits it has inside a batch of the two-SM kernel."""
+    w = workloads.init_mlp_weights("lstm", seed=29, gain=2.0, layers=layers)
+    feats, dev = workloads.make_queries("lstm", 3000, 47)
+    mu, sigma = workloads.batch_mu_sigma(feats, dev)
+    h = batched.MLPHandle(feats.shape[1], mu=mu, sigma=sigma, device_features=DEVF, precision=precision, **w)
+    f, r = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()
+    full = h.predict(f, r)
+    for Q in range(1, 45):
+        lo = 61 * Q
+        got = h.predict(f[lo:lo + Q].contiguous(), r[lo:lo + Q].contiguous())
+        assert torch.equal(got, full[lo:lo + Q]), Q
+    h.check_status()
+    h.close()
+
+
 def test_small_batches_on_streams_and_in_a_graph():
     """Small batches keep scratch per stream: interleaved launches of two predictors on more streams than
     there is scratch for, a captured launch, and a launch after an error status all give the same bits."""
