@@ -204,7 +204,6 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
   const uint32_t bar_tfree = bars + 192;                      // TMEM read out (4 warps)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_ptr + 200);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + 204);
-  volatile int* poisoned = reinterpret_cast<volatile int*>(bars_ptr + 208);
   const uint32_t bar_drain = bars + 216;                      // after giving up: the MMAs have ended
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -225,14 +224,6 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
   // (before the peers' first stores)
   if (NEAR) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   constexpr uint32_t kTmemCols = kBlocks * W < 32 ? 32 : kBlocks * W;
-  if (threadIdx.x == 64 && !p.beside) hb_grid_wait();   // the mark may be a fresh buffer's
-  if (threadIdx.x == 64 && *reinterpret_cast<volatile int32_t*>(p.poison) != 0) {
-    // an earlier launch left the buffers in an unknown state: report, and touch nothing
-    *poisoned = 1;
-    *static_cast<volatile int32_t*>(p.status) = 0x5FF;
-  } else if (threadIdx.x == 64) {
-    *poisoned = 0;
-  }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(kTmemCols)
@@ -301,8 +292,13 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
     __syncwarp();
   };
 
-  if (*poisoned) {
-    // nothing has been started
+  if (warp == 2) {
+    // An earlier launch that gave up left the buffers in an unknown state: report, and give up as well (no result is
+    // stored then).  Nobody waits for the mark, whose load takes 700 cycles.
+    if (lane == 0 && *reinterpret_cast<volatile int32_t*>(p.poison) != 0) {
+      *static_cast<volatile int32_t*>(p.status) = 0x5FF;
+      *abort_flag = 1;
+    }
   } else if (warp == 1) {
     // ------------------------------ weight producer ------------------------------
     if (lane == 0) {
@@ -680,7 +676,7 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
   }
-  if (NEAR && (*abort_flag || *poisoned)) {
+  if (NEAR && *abort_flag) {
     // A block that has everything it waited for has been sent all that will be.  One that gave up may still be
     // written to: it stays until the others have left or given up as well (their waits are bounded), and a
     // little longer for what is on its way.
