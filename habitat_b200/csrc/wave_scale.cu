@@ -459,47 +459,50 @@ __device__ __forceinline__ uint32_t hb_checked(uint32_t idx, uint32_t limit, uin
 #define HB_IDX(idx, limit, site) (idx)
 #endif
 
-// Two records per thread (VEC = 2) need the inputs on 8-byte boundaries; ALIGNED says that the
-// output planes are too (K even), so results leave as 8-byte stores.  Otherwise (odd K: every
-// other plane starts on an odd element) the same two-record arithmetic ends in scalar stores,
-// and the thread that owns the last, single record loads it alone.
-template <typename T, int VEC, bool ALIGNED>
+// Two records per thread (VEC = 2) need the inputs on 8-byte boundaries; GAP = 0 says that the output planes are
+// too (K even), so results leave as 8-byte stores.  Otherwise (odd K: every other plane starts on an odd element) the
+// same two-record arithmetic ends in scalar stores, and a thread with a single record loads it alone.  The records of
+// a thread are then neighbours (GAP = 1), or (GAP = 32) so far apart that each of a warp's accesses is one piece
+// of 32 elements: with metrics, four arrays of which are loaded one element at a time in any case, that is 2 to 5 %
+// faster up to eight destinations (1,000,001 x 6: 33.6 -> 32.6 us, x 1: 14.9 -> 14.3; 4,000,001 x 6: 113.3 -> 111.5) and
+// 1 % slower with thirteen; without metrics the vector loads are worth more (1,000,001 x 6: 19.4 against 21.1).
+template <typename T, int VEC, uint32_t GAP>
 __device__ __forceinline__ Vec<T, VEC> load_pair(const T* q, bool pair) {
-  if (VEC == 1 || ALIGNED) return load_vec<T, VEC>(q);
+  if (VEC == 1 || GAP == 0) return load_vec<T, VEC>(q);
   Vec<T, VEC> v;
-  if (pair) {
+  if (GAP == 1 && pair) {
     v = load_vec<T, VEC>(q);
   } else {
     v.v[0] = q[0];
-    v.v[VEC - 1] = q[0];
+    v.v[VEC - 1] = GAP > 1 && pair ? q[GAP] : q[0];
   }
   return v;
 }
 // The same without vector loads, for arrays of any alignment.
-template <typename T, int VEC>
+template <typename T, int VEC, uint32_t GAP>
 __device__ __forceinline__ Vec<T, VEC> load_each(const T* q, bool pair) {
   Vec<T, VEC> v;
   v.v[0] = q[0];
-  if (VEC == 2) v.v[VEC - 1] = pair ? q[VEC - 1] : q[0];
+  if (VEC == 2) v.v[VEC - 1] = pair ? q[GAP ? GAP : 1] : q[0];
   return v;
 }
-template <typename T, int VEC, bool ALIGNED>
+template <typename T, int VEC, uint32_t GAP>
 __device__ __forceinline__ void store_pair(T* q, const Vec<T, VEC>& v, bool pair) {
-  if (VEC == 1 || ALIGNED) {
+  if (VEC == 1 || GAP == 0) {
     store_vec<T, VEC>(q, v);
   } else {
     q[0] = v.v[0];
-    if (pair) q[VEC - 1] = v.v[VEC - 1];
+    if (pair) q[GAP] = v.v[VEC - 1];
   }
 }
 // The low bytes of the two 16-bit halves of `pair_word` as one or two bytes at q.
-template <int VEC, bool ALIGNED>
+template <int VEC, uint32_t GAP>
 __device__ __forceinline__ void store_byte_pair(uint8_t* q, uint32_t pair_word, bool pair) {
-  if (VEC == 2 && ALIGNED) {
+  if (VEC == 2 && GAP == 0) {
     *reinterpret_cast<uint16_t*>(q) = static_cast<uint16_t>(__byte_perm(pair_word, 0u, 0x4420u));
   } else {
     q[0] = static_cast<uint8_t>(pair_word);
-    if (VEC == 2 && pair) q[1] = static_cast<uint8_t>(pair_word >> 16);
+    if (VEC == 2 && pair) q[GAP] = static_cast<uint8_t>(pair_word >> 16);
   }
 }
 
@@ -516,7 +519,7 @@ constexpr int kTotMaxD = 16;
 // 113.7 -> 105.4 us, 11,184,812 x 6: 310 -> 287), without them up to 5 % faster with one or two destinations (8,000,000
 // x 1: 73.7 -> 69.9) and 1 to 4 % slower with more (4,000,000 x 6: 81.8 -> 84.8).  Smaller batches are slower with the
 // second (500,000 x 6: 17.4 -> 18.2 us, 250,000 x 13: 21.0 -> 24.0, with register counts).
-template <int VEC, int EXT, bool ALIGNED, int NW, int TOT = 0>
+template <int VEC, int EXT, bool ALIGNED, int NW, int TOT = 0, bool FAR = false>
 __global__ void __launch_bounds__(kLutThreads, EXT == 2 ? 8 : (EXT == 3 ? 10 : 12))
 wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
   static_assert(!TOT || (VEC == 2 && EXT == 0), "fused totals: plain two-record variants only");
@@ -525,7 +528,11 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
   hb_grid_dependency_wait();
   const uint32_t K = lp.K;
   const int D = lp.D;
-  const uint32_t k0 = (blockIdx.x * kLutThreads + threadIdx.x) * VEC;
+  static_assert(!FAR || (VEC == 2 && !ALIGNED), "two records per thread, scalar stores");
+  constexpr uint32_t GAP = ALIGNED ? 0 : (FAR ? 32 : 1);
+  // a warp owns 32 VEC records in a row
+  const uint32_t k0 = GAP > 1 ? (blockIdx.x * kLutThreads + (threadIdx.x & ~31u)) * VEC + (threadIdx.x & 31u)
+                              : (blockIdx.x * kLutThreads + threadIdx.x) * VEC;
   if (TOT && k0 >= K) {
     for (int d = 0; d < D; ++d) s_tot[d][threadIdx.x] = 0.0;   // threads past the end
   }
@@ -536,21 +543,21 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
   const bool with_status = EXT && p.status != nullptr;
 
   if (k0 < K) {
-    const bool pair = VEC == 2 && (ALIGNED || k0 + 1 < K);   // false: the last record of an odd batch
-    const Vec<int32_t, VEC> nbv = load_pair<int32_t, VEC, ALIGNED>(p.num_blocks + k0, pair);
-    const Vec<uint16_t, VEC> bsv = load_pair<uint16_t, VEC, ALIGNED>(p.block_size + k0, pair);
-    const Vec<uint16_t, VEC> rgv = load_pair<uint16_t, VEC, ALIGNED>(p.regs + k0, pair);
-    const Vec<uint32_t, VEC> smv = load_pair<uint32_t, VEC, ALIGNED>(p.smem + k0, pair);
-    const Vec<float, VEC> tv = load_pair<float, VEC, ALIGNED>(p.time_ns + k0, pair);
+    const bool pair = VEC == 2 && (ALIGNED || k0 + GAP < K);   // false: a single record at the end of an odd batch
+    const Vec<int32_t, VEC> nbv = load_pair<int32_t, VEC, GAP>(p.num_blocks + k0, pair);
+    const Vec<uint16_t, VEC> bsv = load_pair<uint16_t, VEC, GAP>(p.block_size + k0, pair);
+    const Vec<uint16_t, VEC> rgv = load_pair<uint16_t, VEC, GAP>(p.regs + k0, pair);
+    const Vec<uint32_t, VEC> smv = load_pair<uint32_t, VEC, GAP>(p.smem + k0, pair);
+    const Vec<float, VEC> tv = load_pair<float, VEC, GAP>(p.time_ns + k0, pair);
     Vec<float, VEC> gv;
-    if (!with_metrics) gv = load_pair<float, VEC, ALIGNED>(p.gamma + k0, pair);
+    if (!with_metrics) gv = load_pair<float, VEC, GAP>(p.gamma + k0, pair);
     Vec<double, VEC> fev, rdv, wrv;
     Vec<uint8_t, VEC> hmv;
     if (with_metrics) {   // all on their way at once, not the values behind the flag (3,000,000 x 2: 39.1 -> 35.7 us)
-      hmv = load_each<uint8_t, VEC>(p.has_metrics + k0, pair);
-      fev = load_each<double, VEC>(p.flop_eff + k0, pair);
-      rdv = load_each<double, VEC>(p.dram_read + k0, pair);
-      wrv = load_each<double, VEC>(p.dram_write + k0, pair);
+      hmv = load_each<uint8_t, VEC, GAP>(p.has_metrics + k0, pair);
+      fev = load_each<double, VEC, GAP>(p.flop_eff + k0, pair);
+      rdv = load_each<double, VEC, GAP>(p.dram_read + k0, pair);
+      wrv = load_each<double, VEC, GAP>(p.dram_write + k0, pair);
     }
 
     uint32_t P[2] = {0u, 0u}, S[2] = {0u, 0u};     // class bytes of the two records
@@ -630,8 +637,8 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
       const uint32_t om = min(__umulhi(static_cast<uint32_t>(nb) + og.sm.x, og.sm.y), static_cast<uint32_t>(kLutOcc - 1));
       lg_o[i] = __ldg(reinterpret_cast<const float2*>(tab_a + (og.sel.z + HB_IDX(om, kLutOcc, 4) * 8u)));
     }
-    store_byte_pair<VEC, ALIGNED>(p.origin_occ + k0, o2, pair);
-    store_pair<uint32_t, VEC, ALIGNED>(p.origin_waves + k0, owav, pair);
+    store_byte_pair<VEC, GAP>(p.origin_occ + k0, o2, pair);
+    store_pair<uint32_t, VEC, GAP>(p.origin_waves + k0, owav, pair);
 
     // The plain instances keep what they know about a record in masks: six predicates that live through the loop
     // leave none for the body, and the masks go into one logic operation per question (11,184,812 x 6 with totals:
@@ -651,7 +658,7 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
         r = load_vec<int16_t, VEC>(p.dest_regs + at);
       } else {
         r.v[0] = p.dest_regs[at];
-        r.v[VEC - 1] = pair ? p.dest_regs[at + 1] : static_cast<int16_t>(-1);
+        r.v[VEC - 1] = pair ? p.dest_regs[at + GAP] : static_cast<int16_t>(-1);
       }
       return r;
     };
@@ -744,10 +751,10 @@ wave_scale_lut_kernel(const Ptrs p, const __grid_constant__ LutParams lp) {
           st2 |= st << (16 * i);
         }
       }
-      store_pair<float, VEC, ALIGNED>(p.scaled_ns + base, outv, pair);
-      store_pair<uint32_t, VEC, ALIGNED>(p.dest_waves + base, wavv, pair);
-      store_byte_pair<VEC, ALIGNED>(p.dest_occ + base, occ2, pair);
-      if (with_status) store_byte_pair<VEC, ALIGNED>(p.status + base, st2, pair);
+      store_pair<float, VEC, GAP>(p.scaled_ns + base, outv, pair);
+      store_pair<uint32_t, VEC, GAP>(p.dest_waves + base, wavv, pair);
+      store_byte_pair<VEC, GAP>(p.dest_occ + base, occ2, pair);
+      if (with_status) store_byte_pair<VEC, GAP>(p.status + base, st2, pair);
       if (TOT) {
         const float g0 = outv.v[0] == outv.v[0] ? outv.v[0] : 0.0f;                     // NaN: no prediction
         const float g1 = pair && outv.v[VEC - 1] == outv.v[VEC - 1] ? outv.v[VEC - 1] : 0.0f;
@@ -897,9 +904,9 @@ int class_of(std::vector<FastDev>& reps, std::vector<uint32_t>& words, const std
   return static_cast<int>(c);
 }
 
-template <int VEC, int EXT, bool ALIGNED, int NW, int TOT = 0>
+template <int VEC, int EXT, bool ALIGNED, int NW, int TOT = 0, bool FAR = false>
 cudaError_t launch_lut(unsigned grid, cudaStream_t stream, const Ptrs& p, const LutParams& q) {
-  return hb::launch_overlapped(wave_scale_lut_kernel<VEC, EXT, ALIGNED, NW, TOT>, dim3(grid), dim3(kLutThreads),
+  return hb::launch_overlapped(wave_scale_lut_kernel<VEC, EXT, ALIGNED, NW, TOT, FAR>, dim3(grid), dim3(kLutThreads),
                                TOT ? sizeof(double) * kLutThreads * q.D : 0, stream, p, q);
 }
 
@@ -995,7 +1002,10 @@ bool try_launch_lut(const Ptrs& p, const LaunchPlan& plan, int64_t K, int64_t st
   if (ext) {
     auto launch_ext = [&](auto words) {
       constexpr int W = decltype(words)::value;
-      if (metrics && vec2 && blocks > 18ll * sm_count)
+      const bool large = blocks > 18ll * sm_count;
+      if (metrics && vec2 && !aligned && lp.D <= 8)   // see GAP
+        return large ? launch_lut<2, 3, false, W, 0, true>(grid, stream, p, q) : launch_lut<2, 2, false, W, 0, true>(grid, stream, p, q);
+      if (metrics && vec2 && large)
         return aligned ? launch_lut<2, 3, true, W>(grid, stream, p, q) : launch_lut<2, 3, false, W>(grid, stream, p, q);
       if (metrics)
         return !vec2 ? launch_lut<1, 2, true, W>(grid, stream, p, q)

@@ -113,6 +113,36 @@ def test_metrics_mode(device_file):
         assert_wave_equal(one, ref, rel=2e-6)
 
 
+@pytest.mark.parametrize("D", [1, 6, 8, 9])
+@pytest.mark.parametrize("K", [1, 3, 31, 33, 63, 65, 191, 255, 257, 511, 4097, 700001])
+def test_metrics_of_odd_batches(device_file, K, D):
+    """Odd batches with metrics: a thread's two records are 32 apart (up to eight destinations) and the last warps hold
+    one or none.  Every result is, bit for bit, that of an even batch which has the same records first."""
+    names = sorted(device_file)
+    devs = [device_file[names[i % len(names)]] for i in range(D)]
+    origin = device_file["V100"]
+    g = workloads.rng(K + D)
+    kernels = workloads.make_kernels(K + 1, seed=K)
+    metrics = workloads.make_metrics(K + 1, seed=K + 1)
+    regs = torch.from_numpy(g.integers(-1, 256, size=(D, K + 1)).astype(np.int16)).cuda()
+
+    def run(n):
+        kb = batched.KernelBatch.from_numpy({k: v[:n] for k, v in kernels.items()})
+        mb = batched.KernelMetricsBatch(
+            *(torch.from_numpy(metrics[f][:n].astype(t)).cuda() for f, t in
+              (("flop_efficiency_pct", np.float64), ("dram_read_bytes", np.float64), ("dram_write_bytes", np.float64),
+               ("has_metrics", np.uint8))))
+        res = batched.wave_scale(kb, origin, devs, dest_regs=regs[:, :n].contiguous(), metrics=mb, want_status=True)
+        torch.cuda.synchronize()
+        assert batched.wave_scale_path() == "wave_scale_lut_kernel"
+        return {k: to_numpy(getattr(res, k))[..., :K] for k in
+                ("scaled_ns", "dest_occupancy", "dest_waves", "origin_occupancy", "origin_waves", "status")}
+
+    got, want = run(K), run(K + 1)
+    for name in got:
+        assert got[name].tobytes() == np.ascontiguousarray(want[name]).tobytes(), name
+
+
 def test_host_buffer_entry_point(bench_devices):
     kernels = workloads.make_kernels(10001, seed=31)
     res = batched.wave_scale_host(kernels, bench_devices[0], bench_devices, want_status=True,
