@@ -173,25 +173,28 @@ class _GroupPlan:
         self.mode = mode
         self.mlp_inputs = {}      # op kind -> (features, measured ms) on the GPU, measured ms, columns; filled on first use
         self._layout = None
+        self.started = None       # predictors that were started during the walk,
+        self.staged = None        # and memory that the first prediction's upload reads
         if flat is None:
             self._flatten(operations, indices, mode)
         else:
             self._take(operations, flat)
 
     @classmethod
-    def of_whole_trace(cls, operations, mode, with_names):
+    def of_whole_trace(cls, operations, mode, with_names, early=None):
         """The plan of a trace recorded on one device, walked by the native binding; None when the
         operations are not all of this package's ordinary classes (any object with their surface
-        takes the Python walk), or when a missing metric has to raise (the roofline strategy)."""
+        takes the Python walk), or when a missing metric has to raise (the roofline strategy).
+        early(inputs of the MLP kinds, indices of their operations) is called before the kernels are walked."""
         if mode == wave_batch.ROOFLINE:
             return None
         flat = _native.binding().flatten_trace(operations, _trace_types(), SPECIAL_OPERATIONS, _MLP_OPS, _METRIC_KEYS,
-                                               mode != wave_batch.RESIMPLIFIED, _FAST_ORDERS, with_names)
+                                               mode != wave_batch.RESIMPLIFIED, _FAST_ORDERS, with_names, early)
         return cls(operations, None, mode, flat) if flat is not None else None
 
     def _take(self, operations, flat):
         (self.n_kernels, self.n_runs, self._names, wave_idx, fwd, bwd, offsets, overheads, kind_idx, self.passthrough_idx,
-         records, metrics, self.offsets_dev, special) = flat
+         records, metrics, self.offsets_dev, special, self.started, self.staged) = flat
         self._kernels, self._operations = None, operations
         self.indices = None                      # all operations
         self.wave_idx, self.fwd_run, self.bwd_run, self.offsets = (
@@ -447,7 +450,9 @@ class Predictor:
         if plan is None:
             if mode is None or any(d.name == origin.name for d in dest_devices):
                 return None
-            plan = _GroupPlan.of_whole_trace(operations, mode, self._has_registers())
+            plan = _GroupPlan.of_whole_trace(
+                operations, mode, self._has_registers(),
+                lambda special, indices: self._start_kinds(special, indices, origin, dest_devices, len(operations)))
             if plan is None:
                 return None
             if cache is not None:
@@ -457,9 +462,36 @@ class Predictor:
         ms = np.empty((len(dest_devices), len(operations)), np.float64)
         for i in plan.passthrough_idx:
             ms[:, i] = operations[i].run_time_ms
-        times, totals, sums = self._run_plan(plan, operations, origin, dest_devices, ms)
+        started, plan.started = plan.started, None          # for this prediction; the plan is used again
+        times, totals, sums = self._run_plan(plan, operations, origin, dest_devices, ms, started)
+        plan.staged = None
         return [PredictedOperations(operations, dest, dict(plan=plan, times=times[t], totals=totals[t]), ms[t], sums[t])
                 for t, dest in enumerate(dest_devices)]
+
+    def _start_kinds(self, special, indices, origin, dests, n_operations):
+        """Starts the predictors of a trace whose kernels are still being walked: what run_group takes as their
+        results, with the kinds it is for and the handles in use, or None when they cannot be started now (`_run_plan`
+        then runs them, and raises what there is to raise)."""
+        try:
+            kinds, names, held = [], [], []
+            for name, idx in zip(_MLP_OPS, indices):
+                if not idx:
+                    continue
+                got = special[_FAST_KINDS.index(name)] if name in _FAST_KINDS else None
+                pred = self._predictor(name)
+                if got is None or FEATURES[name] != pred.model.features or not self._is_plain(pred):
+                    return None
+                rows = bytes([pred.device_row(origin.name)] + [pred.device_row(d.name) for d in dests])
+                held.append(pred._handle)
+                kinds.append((held[-1]._handle.value or 0, got[0], got[1], rows, idx))
+                names.append(name)
+            return _native.binding().start_kinds(kinds, len(dests), n_operations), kinds, names, held
+        except Exception:
+            return None
+
+    @staticmethod
+    def _is_plain(pred):
+        return getattr(pred.predict_batch, "__func__", None) is RuntimePredictor.predict_batch
 
     def _has_registers(self):
         return self._kernel_metadata is not None and not getattr(self._kernel_metadata, "empty", False)
@@ -496,19 +528,22 @@ class Predictor:
                 res._kind[idx] = 2
             res.run_times_ms[indices] = ms[t, indices]
 
-    def _run_plan(self, plan, operations, origin, dests, ms):
+    def _run_plan(self, plan, operations, origin, dests, ms, started=None):
         """One prediction of a flattened group: fills `ms` [T, operations] for its operations and returns
         (scaled kernel times [T, K], per-pass kernel totals [T, runs], sums of the rows of `ms`), all on
         the host (predictor.py:111-148 of the reference for every pass, special operation and destination
-        at once)."""
+        at once).  `started`: what _start_kinds returned for these operations and destinations."""
         T, K, n_runs = len(dests), plan.n_kernels, plan.n_runs
         names = [name for name in _MLP_OPS if len(plan.mlp_idx[name])]
         kinds, native, held = [], [], []
+        if started is not None:
+            started, kinds, native, held = started
+            names = []
         for name in names:
             pred = self._predictor(name)
             rows = bytes([pred.device_row(origin.name)] + [pred.device_row(d.name) for d in dests])
             feats, rt, rt_host, _ = plan.special_inputs(name, operations, pred.model.features)
-            if getattr(pred.predict_batch, "__func__", None) is RuntimePredictor.predict_batch:
+            if self._is_plain(pred):
                 held.append(pred._handle)        # the call below knows its address only
                 kinds.append((held[-1]._handle.value or 0, feats, rt, rows, plan.mlp_idx[name]))
                 native.append(name)
@@ -536,7 +571,7 @@ class Predictor:
             "run_group", _native.binding().run_group, flat.batch if flat is not None else None,
             flat.metrics if flat is not None else None, origin, dests, regs,
             plan.offsets_dev if flat is not None else None, kinds,
-            (plan.overheads, plan.wave_idx, plan.fwd_run, plan.bwd_run), times, totals, ms)
+            (plan.overheads, plan.wave_idx, plan.fwd_run, plan.bwd_run), times, totals, ms, *(() if started is None else (started,)))
         if nan:
             wave_batch.raise_zero_wave()
         for name, raw in zip(native, clamped):

@@ -611,16 +611,20 @@ bool feature_row(long kind, PyObject* op, PyTypeObject* op_type, PyTypeObject* r
 
 // flatten_trace(operations, (MeasuredOperation, RunTimeMeasurement, MeasuredKernel, KernelInstance),
 //               special names, MLP kinds (conv2d, linear, bmm first), metrics ((Metric, name, legacy name) x 3),
-//               with_metrics, column orders of the first three kinds, with_names)
+//               with_metrics, column orders of the first three kinds, with_names, early or None)
 // -> None when the operations are not all of those very classes or not of one device, else
 //    (number of kernels, number of passes, names or None, wave_idx, fwd_run, bwd_run, offsets, overheads: bytes of int64 / float64,
 //     (indices per MLP kind: bytes of int64), passed-through indices,
 //     (num_blocks, block_size, regs, smem, time, gamma), (eff, read, write, has) or None, offsets: CUDA tensors,
 //     per kind of the first three: (features, measured ms: CUDA tensors, measured ms as bytes), or None when one of
-//     its operations was not recorded positionally)
+//     its operations was not recorded positionally, what `early` returned or None, page-locked memory that has to be
+//     kept until the stream has got to the end of the upload, or None)
+// The operations of the MLP kinds are walked first.  early(the entries per kind of the first three, indices per MLP kind)
+// is called when their features are on the GPU, before the walk over the kernels, which takes longer than the
+// predictors do: what it launches runs meanwhile.
 PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  if (n_args != 8) return not_ordinary();
+  if (n_args != 9) return not_ordinary();
   Ref ops(PySequence_Fast(a[0], "operations must be a sequence"));
   if (!ops.p) return nullptr;
   PyTypeObject* type[4];
@@ -639,6 +643,7 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   } feats[kFeatureKinds];
   for (long k = 0; k < kFeatureKinds; ++k) feats[k].ok = columns_of(PyTuple_GET_ITEM(a[6], k), k, &feats[k].c);
   std::vector<int64_t> wave_idx, fwd, bwd, offsets{0};
+  std::vector<PyObject*> wave_ops;   // borrowed from `ops`
   std::vector<double> overhead, eff, rd, wr;
   std::vector<int32_t> nb;
   std::vector<uint16_t> bs, rg;
@@ -711,13 +716,8 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const int is_special = PySet_Contains(special, name.p);
     if (is_special < 0) return not_ordinary();
     if (!is_special) {
-      Ref f(field(op, s__forward)), b(field(op, s__backward));
-      if (!f.p || !b.p) return not_ordinary();
       wave_idx.push_back(i);
-      fwd.push_back(static_cast<int64_t>(overhead.size()));
-      if (!add_run(f.p)) return not_ordinary();
-      bwd.push_back(b.p == Py_None ? -1 : static_cast<int64_t>(overhead.size()));
-      if (b.p != Py_None && !add_run(b.p)) return not_ordinary();
+      wave_ops.push_back(op);
       continue;
     }
     Py_ssize_t kind = 0;
@@ -738,87 +738,128 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   }
   if (PyErr_Occurred()) return not_ordinary();
 
-  // one upload for the records, the metrics, the pass boundaries and the features
-  std::vector<uint8_t> host;
-  struct Piece {
-    size_t at;
-    int64_t rows, cols;
-    at::ScalarType type;
+  // what goes to the GPU in one piece, and the tensors in it
+  struct Upload {
+    struct Piece {
+      size_t at;
+      int64_t rows, cols;
+      at::ScalarType type;
+    };
+    std::vector<uint8_t> host;
+    std::vector<Piece> pieces;
+    at::Tensor block;
+    size_t taken = 0;
+    void put(const void* p, int64_t count, size_t size, at::ScalarType t, int64_t cols = 0) {
+      const size_t at0 = (host.size() + 255) & ~static_cast<size_t>(255);
+      host.resize(at0 + count * size);
+      std::memcpy(host.data() + at0, p, count * size);
+      pieces.push_back(Piece{at0, cols ? count / cols : count, cols, t});
+    }
+    // A copy from pageable memory first waits for what is on the stream; behind `early`'s launches it goes from a
+    // page-locked block.
+    at::Tensor staged;
+    bool go(bool behind) {
+      if (host.empty()) return true;
+      const int64_t total[1] = {static_cast<int64_t>(host.size())};
+      int current = 0;
+      cudaGetDevice(&current);
+      block = empty(total, at::kByte, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(current)));
+      const void* from = host.data();
+      if (behind) {
+        staged = at::Tensor(at::detail::empty_cpu(total, at::kByte, /*pin_memory=*/true));
+        from = std::memcpy(staged.mutable_data_ptr(), host.data(), host.size());
+      }
+      const cudaError_t e = cudaMemcpyAsync(block.mutable_data_ptr(), from, host.size(), cudaMemcpyHostToDevice,
+                                            static_cast<cudaStream_t>(stream_now()));
+      if (e != cudaSuccess) PyErr_Format(PyExc_RuntimeError, "upload of the trace: %s", cudaGetErrorString(e));
+      return e == cudaSuccess;
+    }
+    PyObject* view() {
+      const Piece& p = pieces[taken++];
+      const int64_t size[2] = {p.rows, p.cols};
+      return THPVariable_Wrap(inside(block, p.at, at::IntArrayRef(size, p.cols ? 2 : 1), p.type));
+    }
+    PyObject* views(Py_ssize_t count) {
+      PyObject* t = PyTuple_New(count);
+      for (Py_ssize_t i = 0; t && i < count; ++i) PyTuple_SET_ITEM(t, i, view());
+      return t;
+    }
   };
-  std::vector<Piece> pieces;
-  auto put = [&](const void* p, int64_t count, size_t size, at::ScalarType t, int64_t cols = 0) {
-    const size_t at0 = (host.size() + 255) & ~static_cast<size_t>(255);
-    host.resize(at0 + count * size);
-    std::memcpy(host.data() + at0, p, count * size);
-    pieces.push_back(Piece{at0, cols ? count / cols : count, cols, t});
+  Upload records, features;
+  Ref special_rows(PyTuple_New(kFeatureKinds)), kinds_out(PyTuple_New(n_kinds)), started(Py_NewRef(Py_None));
+  if (!special_rows.p || !kinds_out.p) return nullptr;
+  for (Py_ssize_t k = 0; k < n_kinds; ++k) PyTuple_SET_ITEM(kinds_out.p, k, bytes_of(kind_idx[k]));
+  // the features go on their own when something is to start with them, else with the records
+  const bool early = a[8] != Py_None;
+  Upload& with = early ? features : records;
+  auto put_features = [&] {
+    for (Rows& r : feats) {
+      r.ok = r.ok && !r.ms.empty();
+      if (!r.ok) continue;
+      with.put(r.f.data(), static_cast<int64_t>(r.f.size()), 4, at::kFloat, r.c.n);
+      with.put(r.ms.data(), static_cast<int64_t>(r.ms.size()), 4, at::kFloat);
+    }
   };
+  auto take_features = [&] {
+    for (Py_ssize_t k = 0; k < kFeatureKinds; ++k) {
+      PyObject* got = Py_NewRef(Py_None);
+      if (feats[k].ok) {
+        PyObject *f = with.view(), *m = with.view();
+        Py_SETREF(got, Py_BuildValue("(NNN)", f, m, bytes_of(feats[k].ms)));
+      }
+      PyTuple_SET_ITEM(special_rows.p, k, got);
+    }
+  };
+  if (early) {
+    put_features();
+    if (!features.go(false)) return nullptr;
+    take_features();
+    if (PyErr_Occurred()) return nullptr;
+    if (!features.host.empty()) Py_SETREF(started.p, PyObject_CallFunctionObjArgs(a[8], special_rows.p, kinds_out.p, nullptr));
+    if (!started.p) return nullptr;
+  }
+
+  for (PyObject* op : wave_ops) {
+    Ref f(field(op, s__forward)), b(field(op, s__backward));
+    if (!f.p || !b.p) return not_ordinary();
+    fwd.push_back(static_cast<int64_t>(overhead.size()));
+    if (!add_run(f.p)) return not_ordinary();
+    bwd.push_back(b.p == Py_None ? -1 : static_cast<int64_t>(overhead.size()));
+    if (b.p != Py_None && !add_run(b.p)) return not_ordinary();
+  }
+  if (PyErr_Occurred()) return not_ordinary();
+
   const int64_t K = static_cast<int64_t>(nb.size());
   if (K > 0) {
     const std::vector<float> gamma(nb.size(), 1.0f);
-    put(nb.data(), K, 4, at::kInt);
-    put(bs.data(), K, 2, at::kUInt16);
-    put(rg.data(), K, 2, at::kUInt16);
-    put(sm.data(), K, 4, at::kUInt32);
-    put(tm.data(), K, 4, at::kFloat);
-    put(gamma.data(), K, 4, at::kFloat);
-    put(offsets.data(), static_cast<int64_t>(offsets.size()), 8, at::kLong);
+    records.put(nb.data(), K, 4, at::kInt);
+    records.put(bs.data(), K, 2, at::kUInt16);
+    records.put(rg.data(), K, 2, at::kUInt16);
+    records.put(sm.data(), K, 4, at::kUInt32);
+    records.put(tm.data(), K, 4, at::kFloat);
+    records.put(gamma.data(), K, 4, at::kFloat);
+    records.put(offsets.data(), static_cast<int64_t>(offsets.size()), 8, at::kLong);
     if (any_metrics) {
-      put(eff.data(), K, 8, at::kDouble);
-      put(rd.data(), K, 8, at::kDouble);
-      put(wr.data(), K, 8, at::kDouble);
-      put(has.data(), K, 1, at::kByte);
+      records.put(eff.data(), K, 8, at::kDouble);
+      records.put(rd.data(), K, 8, at::kDouble);
+      records.put(wr.data(), K, 8, at::kDouble);
+      records.put(has.data(), K, 1, at::kByte);
     }
   }
-  for (Rows& r : feats) {
-    r.ok = r.ok && !r.ms.empty();
-    if (!r.ok) continue;
-    put(r.f.data(), static_cast<int64_t>(r.f.size()), 4, at::kFloat, r.c.n);
-    put(r.ms.data(), static_cast<int64_t>(r.ms.size()), 4, at::kFloat);
-  }
-  at::Tensor block;
-  if (!host.empty()) {
-    const int64_t total[1] = {static_cast<int64_t>(host.size())};
-    int current = 0;
-    cudaGetDevice(&current);
-    block = empty(total, at::kByte, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(current)));
-    const cudaError_t e = cudaMemcpyAsync(block.mutable_data_ptr(), host.data(), host.size(), cudaMemcpyHostToDevice,
-                                          static_cast<cudaStream_t>(stream_now()));
-    if (e != cudaSuccess) {
-      PyErr_Format(PyExc_RuntimeError, "upload of the trace: %s", cudaGetErrorString(e));
-      return nullptr;
-    }
-  }
-  size_t taken = 0;
-  auto view = [&] {
-    const Piece& p = pieces[taken++];
-    const int64_t size[2] = {p.rows, p.cols};
-    return THPVariable_Wrap(inside(block, p.at, at::IntArrayRef(size, p.cols ? 2 : 1), p.type));
-  };
-  auto views = [&](Py_ssize_t count) {
-    PyObject* t = PyTuple_New(count);
-    for (Py_ssize_t i = 0; t && i < count; ++i) PyTuple_SET_ITEM(t, i, view());
-    return t;
-  };
-  Ref soa(Py_NewRef(Py_None)), met(Py_NewRef(Py_None)), off(Py_NewRef(Py_None)), special_rows(PyTuple_New(kFeatureKinds)),
-      kinds_out(PyTuple_New(n_kinds));
-  if (!special_rows.p || !kinds_out.p) return nullptr;
+  if (!early) put_features();
+  if (!records.go(started.p != Py_None)) return nullptr;
+  Ref soa(Py_NewRef(Py_None)), met(Py_NewRef(Py_None)), off(Py_NewRef(Py_None));
   if (K > 0) {
-    Py_SETREF(soa.p, views(6));
-    Py_SETREF(off.p, view());
-    if (any_metrics) Py_SETREF(met.p, views(4));
+    Py_SETREF(soa.p, records.views(6));
+    Py_SETREF(off.p, records.view());
+    if (any_metrics) Py_SETREF(met.p, records.views(4));
   }
-  for (Py_ssize_t k = 0; k < kFeatureKinds; ++k) {
-    PyObject* got = Py_NewRef(Py_None);
-    if (feats[k].ok) {
-      PyObject *f = view(), *m = view();
-      Py_SETREF(got, Py_BuildValue("(NNN)", f, m, bytes_of(feats[k].ms)));
-    }
-    PyTuple_SET_ITEM(special_rows.p, k, got);
-  }
-  for (Py_ssize_t k = 0; k < n_kinds; ++k) PyTuple_SET_ITEM(kinds_out.p, k, bytes_of(kind_idx[k]));
+  if (!early) take_features();
   if (PyErr_Occurred() || !soa.p || !off.p || !met.p) return nullptr;
-  return Py_BuildValue("(LLONNNNNOOOOOO)", static_cast<long long>(K), static_cast<long long>(overhead.size()), names.p, bytes_of(wave_idx), bytes_of(fwd), bytes_of(bwd),
-                       bytes_of(offsets), bytes_of(overhead), kinds_out.p, passed.p, soa.p, met.p, off.p, special_rows.p);
+  Ref staged(records.staged.defined() ? THPVariable_Wrap(records.staged) : Py_NewRef(Py_None));
+  if (!staged.p) return nullptr;
+  return Py_BuildValue("(LLONNNNNOOOOOOOO)", static_cast<long long>(K), static_cast<long long>(overhead.size()), names.p, bytes_of(wave_idx), bytes_of(fwd), bytes_of(bwd),
+                       bytes_of(offsets), bytes_of(overhead), kinds_out.p, passed.p, soa.p, met.p, off.p, special_rows.p, started.p, staged.p);
   END_HANDLE_TH_ERRORS
 }
 
@@ -1068,11 +1109,115 @@ PyObject* wave_scale_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Py_RETURN_TRUE;
 }
 
+// The operations of one MLP kind of a trace: the predictor, its inputs, and where its raw predictions (device) and
+// the operations' times (page-locked) go.
+struct Kind {
+  hb_mlp* h;
+  const at::Tensor *f, *ms;
+  const uint8_t* rows;
+  const int64_t* idx;
+  int64_t n;
+  float *pred, *times;
+};
+size_t place(size_t* at, size_t bytes) {
+  const size_t here = *at;
+  *at = (here + bytes + 255) & ~static_cast<size_t>(255);
+  return here;
+}
+// Kinds of a list of (handle address, features, measured ms, device rows (bytes: origin, then T destinations), operation
+// indices (int64, below n_ops)), without their places; null or what is wrong with it.
+const char* kinds_of(PyObject* list, int64_t T, int64_t n_ops, std::vector<Kind>* kinds) {
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(list); ++i) {
+    PyObject* t = PyList_GET_ITEM(list, i);
+    if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 5) return "operation kind";
+    Kind k{};
+    k.h = static_cast<hb_mlp*>(PyLong_AsVoidPtr(PyTuple_GET_ITEM(t, 0)));
+    k.f = tensor(PyTuple_GET_ITEM(t, 1), at::kFloat);
+    k.ms = tensor(PyTuple_GET_ITEM(t, 2), at::kFloat);
+    PyObject* rows = PyTuple_GET_ITEM(t, 3);
+    const Buffer<int64_t> idx(PyTuple_GET_ITEM(t, 4), false);   // the tuple keeps the memory alive
+    if (!k.f || k.f->dim() != 2 || !k.ms || !PyBytes_Check(rows) || PyBytes_GET_SIZE(rows) != T + 1 ||
+        k.ms->numel() != k.f->size(0) || !idx.ok(k.f->size(0)))
+      return "operation kind";
+    k.rows = reinterpret_cast<const uint8_t*>(PyBytes_AS_STRING(rows));
+    k.idx = idx.data();
+    k.n = k.f->size(0);
+    for (int64_t j = 0; j < k.n; ++j)
+      if (k.idx[j] < 0 || k.idx[j] >= n_ops) return "operation index";
+    kinds->push_back(k);
+  }
+  return nullptr;
+}
+bool launch_kinds(const std::vector<Kind>& kinds, int64_t T, cudaStream_t s) {
+  std::vector<hb_mlp_grid> grids;
+  std::vector<hb_scale_grid> scales;
+  for (const Kind& k : kinds) {
+    grids.push_back(hb_mlp_grid{k.h, static_cast<const float*>(data(k.f)), k.n, k.rows, static_cast<int32_t>(T + 1), k.pred});
+    scales.push_back(hb_scale_grid{static_cast<const float*>(data(k.ms)), k.pred, k.n, static_cast<int32_t>(T), k.times, nullptr});
+  }
+  return !failed(api.mlp_predict_grid(grids.data(), static_cast<int32_t>(grids.size()), s)) &&
+         !failed(api.special_scale_grid(scales.data(), static_cast<int32_t>(scales.size()), s));
+}
+size_t pred_bytes(const Kind& k, int64_t T) { return static_cast<size_t>(T + 1) * k.n * 4; }
+size_t times_bytes(const Kind& k, int64_t T) { return static_cast<size_t>(T) * k.n * 4; }
+
+// Predictors that were started ahead of the rest of a trace: start_kinds makes one, run_group takes its results.  Whoever
+// lets go of it waits for what has been launched, which writes to its memory.
+constexpr const char* kStartedName = "habitat_b200.started";
+struct Started {
+  at::Tensor block, host;
+  cudaStream_t s = nullptr;
+  int64_t T = 0;
+  std::vector<Kind> kinds;
+  bool launched = false;
+  ~Started() {
+    if (launched) cudaStreamSynchronize(s);
+  }
+};
+// start_kinds([as for run_group], destinations, operations) -> capsule.  The caller keeps the list's objects alive.
+PyObject* start_kinds(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  if (n_args != 3 || !PyList_Check(a[0])) {
+    PyErr_SetString(PyExc_TypeError, "start_kinds: bad arguments");
+    return nullptr;
+  }
+  std::unique_ptr<Started> st(new Started);
+  st->T = PyLong_AsLongLong(a[1]);
+  const int64_t n_ops = PyLong_AsLongLong(a[2]);
+  if (PyErr_Occurred()) return nullptr;
+  if (const char* wrong = kinds_of(a[0], st->T, n_ops, &st->kinds)) {
+    PyErr_Format(PyExc_TypeError, "start_kinds: %s", wrong);
+    return nullptr;
+  }
+  size_t pinned = 0, device = 0;
+  std::vector<std::pair<size_t, size_t>> at;
+  for (const Kind& k : st->kinds) at.emplace_back(place(&device, pred_bytes(k, st->T)), place(&pinned, times_bytes(k, st->T)));
+  int current = 0;
+  cudaGetDevice(&current);
+  const int64_t dev_size[1] = {static_cast<int64_t>(device ? device : 16)},
+                host_size[1] = {static_cast<int64_t>(pinned ? pinned : 16)};
+  st->block = empty(dev_size, at::kByte, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(current)));
+  st->host = at::Tensor(at::detail::empty_cpu(host_size, at::kByte, /*pin_memory=*/true));
+  for (size_t i = 0; i < st->kinds.size(); ++i) {
+    st->kinds[i].pred = reinterpret_cast<float*>(static_cast<uint8_t*>(st->block.mutable_data_ptr()) + at[i].first);
+    st->kinds[i].times = reinterpret_cast<float*>(static_cast<uint8_t*>(st->host.mutable_data_ptr()) + at[i].second);
+  }
+  st->s = static_cast<cudaStream_t>(stream_now());
+  st->launched = true;
+  if (!launch_kinds(st->kinds, st->T, st->s)) return nullptr;
+  PyObject* capsule = PyCapsule_New(st.get(), kStartedName, [](PyObject* c) {
+    delete static_cast<Started*>(PyCapsule_GetPointer(c, kStartedName));
+  });
+  if (capsule) st.release();
+  return capsule;
+  END_HANDLE_TH_ERRORS
+}
+
 // run_group(kernels or None, metrics or None, origin, dests, dest_regs or None, offsets or None,
 //           [(handle address, features, measured ms, device rows (bytes: origin, then the destinations),
 //             operation indices (int64))],
 //           (overheads, wave_idx, fwd_run, bwd_run: float64 / int64), times [T][K] float32,
-//           totals [T][passes] float64, ms [T][n] float64)
+//           totals [T][passes] float64, ms [T][n] float64 [, what start_kinds returned for these kinds])
 // -> (NaN seen, total ms per destination, [per kind: None, or [1 + T][n] float32 predictions as bytes when one
 //    may have been clamped]).  One prediction of a flattened trace: fills `times` and `totals` (the kernels' times
 // and their sums per pass) and the entries of `ms` of the wave-scaled and MLP-predicted operations; the other
@@ -1084,7 +1229,7 @@ PyObject* wave_scale_host(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // so that the predictors, which take longest, start first.
 PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  if (n_args != 11 || !PyList_Check(a[6]) || !PyTuple_Check(a[7]) || PyTuple_GET_SIZE(a[7]) != 4) {
+  if ((n_args != 11 && n_args != 12) || !PyList_Check(a[6]) || !PyTuple_Check(a[7]) || PyTuple_GET_SIZE(a[7]) != 4) {
     PyErr_SetString(PyExc_TypeError, "run_group: bad arguments");
     return nullptr;
   }
@@ -1119,45 +1264,24 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
           bwd.data()[i] >= n_runs)
         return refuse("operations");
 
-  auto place = [](size_t* at, size_t bytes) {
-    const size_t here = *at;
-    *at = (here + bytes + 255) & ~static_cast<size_t>(255);
-    return here;
-  };
   // in page-locked memory: sums and times of the wave scaling, ms per kind
   size_t pinned = 0, device = 0;
   const size_t h_totals = place(&pinned, static_cast<size_t>(T) * n_runs * 8);
   const size_t h_times = place(&pinned, static_cast<size_t>(T) * K * 4);
-  struct Kind {
-    hb_mlp* h;
-    const at::Tensor *f, *ms;
-    const uint8_t* rows;
-    const int64_t* idx;
-    int64_t n;
-    size_t h_ms, d_pred;
-  };
   std::vector<Kind> kinds;
-  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(a[6]); ++i) {
-    PyObject* t = PyList_GET_ITEM(a[6], i);
-    if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 5) return refuse("operation kind");
-    Kind k{};
-    k.h = static_cast<hb_mlp*>(PyLong_AsVoidPtr(PyTuple_GET_ITEM(t, 0)));
-    k.f = tensor(PyTuple_GET_ITEM(t, 1), at::kFloat);
-    k.ms = tensor(PyTuple_GET_ITEM(t, 2), at::kFloat);
-    PyObject* rows = PyTuple_GET_ITEM(t, 3);
-    const Buffer<int64_t> idx(PyTuple_GET_ITEM(t, 4), false);   // the tuple keeps the memory alive
-    if (!k.f || k.f->dim() != 2 || !k.ms || !PyBytes_Check(rows) || PyBytes_GET_SIZE(rows) != T + 1 ||
-        k.ms->numel() != k.f->size(0) || !idx.ok(k.f->size(0)))
-      return refuse("operation kind");
-    k.rows = reinterpret_cast<const uint8_t*>(PyBytes_AS_STRING(rows));
-    k.idx = idx.data();
-    k.n = k.f->size(0);
-    for (int64_t j = 0; j < k.n; ++j)
-      if (k.idx[j] < 0 || k.idx[j] >= n_ops) return refuse("operation index");
-    k.h_ms = place(&pinned, static_cast<size_t>(T) * k.n * 4);
-    k.d_pred = place(&device, static_cast<size_t>(T + 1) * k.n * 4);
-    kinds.push_back(k);
+  if (const char* wrong = kinds_of(a[6], T, n_ops, &kinds)) return refuse(wrong);
+  Started* started = nullptr;
+  if (n_args == 12) {
+    started = static_cast<Started*>(PyCapsule_GetPointer(a[11], kStartedName));
+    if (!started) return nullptr;
+    bool same = started->T == T && started->kinds.size() == kinds.size();
+    for (size_t i = 0; same && i < kinds.size(); ++i)
+      same = kinds[i].h == started->kinds[i].h && kinds[i].n == started->kinds[i].n && kinds[i].f == started->kinds[i].f;
+    if (!same) return refuse("other kinds than were started");
   }
+  std::vector<std::pair<size_t, size_t>> at;
+  if (!started)
+    for (const Kind& k : kinds) at.emplace_back(place(&device, pred_bytes(k, T)), place(&pinned, times_bytes(k, T)));
   const size_t pairs = static_cast<size_t>(T) * K;
   const size_t d_scaled = place(&device, pairs * 4), d_occ = place(&device, pairs), d_waves = place(&device, pairs * 4),
                d_oocc = place(&device, K), d_owaves = place(&device, static_cast<size_t>(K) * 4);
@@ -1178,18 +1302,11 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     ~Settle() { if (on) cudaStreamSynchronize(s); }
   } settle{s};
 
-  auto launch_mlps = [&]() -> bool {
-    std::vector<hb_mlp_grid> grids;
-    std::vector<hb_scale_grid> scales;
-    for (const Kind& k : kinds) {
-      float* pred = reinterpret_cast<float*>(d + k.d_pred);
-      grids.push_back(hb_mlp_grid{k.h, static_cast<const float*>(data(k.f)), k.n, k.rows, static_cast<int32_t>(T + 1), pred});
-      scales.push_back(hb_scale_grid{static_cast<const float*>(data(k.ms)), pred, k.n, static_cast<int32_t>(T),
-                                     reinterpret_cast<float*>(h + k.h_ms), nullptr});
-    }
-    return !failed(api.mlp_predict_grid(grids.data(), static_cast<int32_t>(grids.size()), s)) &&
-           !failed(api.special_scale_grid(scales.data(), static_cast<int32_t>(scales.size()), s));
-  };
+  for (size_t i = 0; i < kinds.size(); ++i) {
+    kinds[i].pred = started ? started->kinds[i].pred : reinterpret_cast<float*>(d + at[i].first);
+    kinds[i].times = started ? started->kinds[i].times : reinterpret_cast<float*>(h + at[i].second);
+  }
+  auto launch_mlps = [&]() -> bool { return started || launch_kinds(kinds, T, s); };
   auto launch_waves = [&]() -> bool {
     if (!scale || K == 0) return true;
     const Field nb(a[0], s_num_blocks, at::kInt), bs(a[0], s_block_size, at::kUInt16), rg(a[0], s_regs, at::kUInt16),
@@ -1262,7 +1379,7 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 
   constexpr int64_t kManyPairs = 16384;
   cudaError_t e = cudaSuccess;
-  if (scale && !kinds.empty() && T * K >= kManyPairs) {
+  if (scale && !kinds.empty() && !started && T * K >= kManyPairs) {
     struct Event {
       cudaEvent_t ev = nullptr;
       ~Event() { if (ev) cudaEventDestroy(ev); }
@@ -1280,10 +1397,12 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (!launch_mlps() || !launch_waves()) return nullptr;
     Py_BEGIN_ALLOW_THREADS
     e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && started && started->s != s) e = cudaStreamSynchronize(started->s);
     if (e == cudaSuccess) sort_waves();
     Py_END_ALLOW_THREADS
   }
   settle.on = false;
+  if (started && e == cudaSuccess) started->launched = false;   // ended
   if (e != cudaSuccess) {
     PyErr_Format(PyExc_RuntimeError, "prediction of a trace: %s", cudaGetErrorString(e));
     return nullptr;
@@ -1293,7 +1412,7 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     const Kind& k = kinds[i];
     int32_t code = 0;
     if (failed(api.mlp_poll_status(k.h, &code))) return nullptr;
-    const float* v = reinterpret_cast<const float*>(h + k.h_ms);
+    const float* v = k.times;
     bool zero = false;
     for (int64_t t = 0; t < T; ++t) {
       double* out = ms.data() + t * n_ops;
@@ -1309,11 +1428,11 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     PyObject* pred = Py_NewRef(Py_None);
     if (zero) {
       // rare: the raw predictions, for the caller's warnings
-      const size_t bytes = static_cast<size_t>(T + 1) * k.n * 4;
+      const size_t bytes = pred_bytes(k, T);
       Py_DECREF(pred);
       pred = PyBytes_FromStringAndSize(nullptr, static_cast<Py_ssize_t>(bytes));
       if (!pred) return nullptr;
-      if (cudaMemcpy(PyBytes_AS_STRING(pred), d + k.d_pred, bytes, cudaMemcpyDeviceToHost) != cudaSuccess) {
+      if (cudaMemcpy(PyBytes_AS_STRING(pred), k.pred, bytes, cudaMemcpyDeviceToHost) != cudaSuccess) {
         Py_DECREF(pred);
         PyErr_SetString(PyExc_RuntimeError, "run_group: cudaMemcpy");
         return nullptr;
@@ -1425,7 +1544,7 @@ PyObject* set_generation(PyObject*, PyObject* v) {
 }
 
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {FAST(setup), FAST(wave_scale), FAST(wave_scale_host), FAST(submit_wave), FAST(host_block), FAST(release_host_blocks), FAST(mlp_predict), FAST(mlp_predict_one), FAST(flatten_trace), FAST(run_group), FAST(iteration_totals), FAST(partials_sum), FAST(group_sum),
+PyMethodDef methods[] = {FAST(setup), FAST(wave_scale), FAST(wave_scale_host), FAST(submit_wave), FAST(host_block), FAST(release_host_blocks), FAST(mlp_predict), FAST(mlp_predict_one), FAST(flatten_trace), FAST(start_kinds), FAST(run_group), FAST(iteration_totals), FAST(partials_sum), FAST(group_sum),
                          FAST(plane_sum), FAST(segment_sum),
                          {"set_generation", set_generation, METH_O, nullptr},
                          {nullptr, nullptr, 0, nullptr}};

@@ -158,3 +158,99 @@ def test_predictors_with_a_predict_of_their_own(bench_devices):
         times = got.operations.run_times_ms
         assert times[0] == pytest.approx(2.5, rel=1e-6) and 0 < times[1] < 10
         assert got.run_time_ms == pytest.approx(times.sum(), rel=1e-12)
+
+
+def _recorded(origin, n, seed, odd=None):
+    """A trace of n conv2d, linear and bmm operations each among 2 n others of one or two kernels; `odd` replaces the
+    arguments of one linear operation."""
+    from habitat_b200.analysis.arguments import Arguments
+    from habitat_b200.analysis.kernels import MeasuredKernel
+    from habitat_b200.analysis.operation import MeasuredOperation
+    from habitat_b200.analysis.run_time import RunTimeMeasurement
+    from habitat_b200.analysis.trace import Trace
+    from habitat_b200.habitat_cuda import KernelInstance
+    g = workloads.rng(seed)
+
+    def run(with_kernels):
+        kernels = []
+        for _ in range(int(g.integers(1, 3)) if with_kernels else 0):
+            c = KernelInstance("k%d" % g.integers(0, 9), int(g.integers(1, 5000)), 128, 0, 1024, 32,
+                               int(g.integers(2000, 10 ** 6)), [])
+            kernels.append(MeasuredKernel(c, [], origin))
+        return RunTimeMeasurement(float(g.uniform(0.5, 40.0)), kernels, origin)
+
+    ops = []
+    for i in range(n):
+        b, f = int(g.integers(1, 64)), int(g.integers(16, 512))
+        linear = Arguments(((b, f), (f, f), None), {}) if odd is None or i else odd
+        for name, args in (("conv2d", Arguments(((b, 3, 32, 32), (f, 3, 3, 3), (f,), (1, 1), (1, 1), (1, 1), 1), {})),
+                           ("linear", linear), ("bmm", Arguments(((b, f, 16), (b, 16, f)), {}))):
+            ops.append(MeasuredOperation(name, args, run(False), run(False) if i % 2 else None, origin))
+            ops.append(MeasuredOperation("relu", Arguments((), {}), run(True), run(True) if i % 3 else None, origin))
+    return Trace(origin, ops)
+
+
+@pytest.mark.parametrize("n", [1, 7, 200])
+def test_predictors_started_during_the_walk(bench_devices, monkeypatch, n):
+    """The first prediction of a trace starts its predictors before the kernels are walked; a later one, or one whose
+    predictors cannot be started then (an operation recorded by keyword), runs them afterwards.  All of them give the
+    same bits, for other destinations than the first ones as well, and with predictors changed in between."""
+    from habitat_b200 import _native
+    from habitat_b200.analysis.arguments import Arguments
+    from habitat_b200.analysis.mlp.mlp import RuntimePredictor
+    from habitat_b200.analysis.predictor import Predictor
+    origin, dests = bench_devices[0], bench_devices[1:]
+
+    def predictor(seed):
+        p = Predictor()
+        for k, op in enumerate(("conv2d", "linear", "bmm")):
+            torch.manual_seed(seed + k)
+            pred = RuntimePredictor(op, 2, 1024)
+            F = len(pred.model.features)
+            pred.mu, pred.sigma = np.full(F + 4, 10.0), np.full(F + 4, 50.0)
+            pred.model.fc2.bias.data.fill_(1.0)
+            setattr(p, op + "_pred", pred)
+        return p
+
+    def result(trace, targets, p):
+        return [(t.run_time_ms, t.operations.run_times_ms.tobytes()) for t in trace.to_devices(targets, p)]
+
+    started = []
+    real = Predictor._start_kinds
+    monkeypatch.setattr(Predictor, "_start_kinds", lambda self, *a: started.append(real(self, *a)) or started[-1])
+    p, q = predictor(1), predictor(5)
+    trace = _recorded(origin, n, 3)
+    first = result(trace, dests, p)
+    assert started.pop() is not None
+    assert result(trace, dests, p) == first and result(trace, dests[:2], p) == first[:2] and not started
+    other = result(trace, dests, q)
+    assert other != first and result(_recorded(origin, n, 3), dests, q) == other and started.pop() is not None
+    # not started: the same results
+    monkeypatch.setattr(Predictor, "_start_kinds", lambda self, *a: None)
+    assert result(_recorded(origin, n, 3), dests, p) == first
+    monkeypatch.setattr(Predictor, "_start_kinds", lambda self, *a: started.append(real(self, *a)) or started[-1])
+    by_keyword = Arguments(((4, 32), (64, 32)), {"bias": None})
+    result(_recorded(origin, n, 3, by_keyword), dests, p)
+    assert started.pop() is None
+    # started, and the walk then finds something that is not ordinary: the general path has the same results
+    class Named(type(trace.operations[1].forward.kernels[0])):
+        pass
+    strange = _recorded(origin, n, 3)
+    kernel = strange.operations[-1].forward.kernels[0]
+    kernel.__class__ = Named
+    got = result(strange, dests, p)
+    assert started.pop() is not None
+    for (a, b), (c, d) in zip(got, first):
+        assert np.allclose(np.frombuffer(b), np.frombuffer(d), rtol=1e-12) and np.isclose(a, c, rtol=1e-12)
+    # results of other kinds than were started are refused
+    with pytest.raises(TypeError):
+        _native.binding().run_group(None, None, origin, dests, None, None, [], (b"", b"", b"", b""),
+                                    np.empty((5, 0), np.float32), np.empty((5, 0)), np.empty((5, 0)),
+                                    real(p, *_special_of(trace), origin, dests, len(trace.operations))[0])
+
+
+def _special_of(trace):
+    """What the walk hands over before it looks at the kernels."""
+    plan = next(v for k, v in trace._prediction_cache.items() if k[0] == "whole")
+    return ([plan.mlp_inputs[k][:2] for k in ("conv2d", "linear", "bmm")],
+            [plan.mlp_idx[k].tobytes() for k in ("conv2d", "linear", "bmm")])
