@@ -205,6 +205,7 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_ptr + 200);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + 204);
   const uint32_t bar_drain = bars + 216;                      // after giving up: the MMAs have ended
+  volatile int* mark_seen = reinterpret_cast<volatile int*>(bars_ptr + 208);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = static_cast<int>(blockIdx.x) / G, c = static_cast<int>(blockIdx.x) % G;   // group = cluster
@@ -219,6 +220,7 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
     mbar_init(bar_tfree, 4);
     mbar_init(bar_drain, 1);
     *abort_flag = 0;
+    *mark_seen = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // (before the peers' first stores)
@@ -294,10 +296,14 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
 
   if (warp == 2) {
     // An earlier launch that gave up left the buffers in an unknown state: report, and give up as well (no result is
-    // stored then).  Nobody waits for the mark, whose load takes 700 cycles.
-    if (lane == 0 && *reinterpret_cast<volatile int32_t*>(p.poison) != 0) {
-      *static_cast<volatile int32_t*>(p.status) = 0x5FF;
-      *abort_flag = 1;
+    // stored then).  Only that result waits for the mark, whose load takes 700 cycles.
+    if (lane == 0) {
+      if (*reinterpret_cast<volatile int32_t*>(p.poison) != 0) {
+        *static_cast<volatile int32_t*>(p.status) = 0x5FF;
+        *abort_flag = 1;
+      }
+      __threadfence_block();
+      *mark_seen = 1;
     }
   } else if (warp == 1) {
     // ------------------------------ weight producer ------------------------------
@@ -652,7 +658,9 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
       float* tots = reinterpret_cast<float*>(base_ptr);        // the tensor core is done with the activations
       tots[T] = tot;
       epi_sync();
-      if (T < n_q && *abort_flag == 0) p.out[q0 + T] = tots[T] + tots[64 + T] + p.fc2_b;
+      // (the mark is long there)
+      for (const long long t0 = clock64(); *mark_seen == 0 && clock64() - t0 <= kWaitCycles;) {}
+      if (T < n_q && *mark_seen != 0 && *abort_flag == 0) p.out[q0 + T] = tots[T] + tots[64 + T] + p.fc2_b;
     }
   }
 
