@@ -1,11 +1,12 @@
 // MLP inference for batches that do not fill the GPU: the layers' features are spread over the SMs.
 //
-// mlp_chain.cu gives 128 queries to two SMs, which stream all 16.8 MB of weights past them: 125 us
+// mlp_chain.cu gives 128 queries to two SMs, which stream all 16.8 MB of weights past them: 118 us
 // whether the batch has one query or 9,472.  What bounds that is the weight stream of one SM pair, so
 // here G = 16, 8 or 4 thread blocks form a group that owns up to 64 queries (32 in split precision);
 // block c computes output features 1024 / G * c .. of every layer for all of the group's queries and
 // streams only their weights.  Between layers a group's blocks exchange their activations through
-// global memory (L2): an all-gather of 2 KB per query.
+// global memory (L2): an all-gather of 2 KB per query.  Groups of few queries use distributed shared memory
+// instead (NEAR, see there).
 //
 // Formulation as in mlp_chain.cu, H^T = W . X^T with tcgen05.mma (cta_group::1): A = weight rows
 // (M = 64 with 16 blocks, else 128), B = activations (MN-major, W = 16, 32 or 64 columns, swizzle width
@@ -28,8 +29,8 @@
 // Weights arrive through a ring of 32 KB slots, 3 to 6 of them; they do not depend on the activations,
 // so the ring is full again when an exchange ends.
 //
-// Warp roles: 0 MMA issuer (and TMEM), 1 weight producer, 4-7 epilogue (one TMEM lane quadrant each),
-// 8-15 (64 columns: 8-23) receivers.  Every wait is bounded, as in mlp_chain.cu; a launch that gave up
+// Warp roles: 0 MMA issuer (and TMEM), 1 weight producer, 2 the mark, 4-7 epilogue (one TMEM lane quadrant each),
+// 8-15 (64 columns: 8-23, NEAR: none) receivers.  Every wait is bounded, as in mlp_chain.cu; a launch that gave up
 // leaves a mark in the scratch, and launches that find it report an error instead of a result.
 #include <atomic>
 #include <cstring>
@@ -837,9 +838,9 @@ namespace hb {
 // 33 of 16, 8 or 4 blocks.  Smaller groups hold more queries in all but stream more weights per block
 // (L2 and shared-memory fill bound), wider ones exchange more per layer (L2 latency and bandwidth); the
 // shapes below are those that no other one beats at its capacity.  Measured per launch, conv2d predictor,
-// 8 hidden layers (capacity in queries: time), against 125 us (bf16) and 190 us (split) before:
-//   bf16    42: 24 us (one: 19)   112: 24 us   240: 28   480: 32   960: 48   1,056: 48   2,112: 75
-//   split   56: 34       120: 42   240: 46             528: 77     1,056: 128
+// 8 hidden layers (capacity in queries: time), against 118 us (bf16) and 195 us (split) of the two-SM kernel:
+//   bf16    42: 23 us (one: 19)   112: 24   240: 28   480: 32   960: 46   1,056: 47   2,112: 73
+//   split   21: 32 (one: 28)       56: 34   120: 42   240: 46             528: 77     1,056: 127
 // Eight blocks x 64 columns lose to four x 32 in split precision (86 us for 480).  Beyond the last shape
 // the two-SM kernel of mlp_chain.cu is the faster one.
 namespace {
@@ -849,7 +850,7 @@ constexpr Shape kShapes[] = {{16, 16, 7, 22, 31, true},  {16, 16, 7, 25, 34, fal
                              {8, 32, 15, 32, 46, false}, {8, 64, 15, 48, 1000, false}, {4, 32, 33, 48, 77, false},
                              {4, 64, 33, 75, 128, false}};
 int clusters_of(const Shape& s, int sm_count) { return sm_count >= 148 ? s.clusters : s.clusters * sm_count / 148; }
-int cols_of(const Shape& s, bool split) { return s.near ? (split ? 3 : 6) : (split ? s.W / 2 : s.W); }
+int cols_of(const Shape& s, bool split) { return s.near ? (split ? 3 : 6) : (split ? s.W / 2 : s.W); }   // near: see NEAR
 WidePlan plan_in(const Shape& s, int64_t Q, bool split, int cols = 0) {
   // full groups while they last: fewer groups move the weights fewer times
   if (cols == 0) cols = cols_of(s, split);
