@@ -967,9 +967,9 @@ hb_status check_device(const hb_mlp* h) {
 }
 
 // HB_MLP_WIDE=0 keeps every batch on the two-SM kernel
-hb::WidePlan plan_of(const hb_mlp* h, int64_t Q) {
+hb::WidePlan plan_of(const hb_mlp* h, int64_t Q, bool alone = true) {
   static const bool use_wide = [] { const char* e = std::getenv("HB_MLP_WIDE"); return !e || std::atoi(e) != 0; }();
-  return use_wide ? hb::wide_plan(Q, h->precision == HB_PRECISION_BF16X3, h->sm_count) : hb::WidePlan{};
+  return use_wide ? hb::wide_plan(Q, h->precision == HB_PRECISION_BF16X3, h->sm_count, alone) : hb::WidePlan{};
 }
 
 // A last round of few tiles takes as long as a full one, and the kernel for small batches is quicker: it takes the
@@ -1059,7 +1059,7 @@ extern "C" hb_status hb_mlp_predict_grid(const hb_mlp_grid* items, int32_t n_ite
   int some = 0;   // batches with queries, the first ones in `order`
   for (; some < n_items && !queued[order[some]]; ++some) {
     const int i = order[some];
-    plans[some] = plan_of(items[i].handle, batches[i].Q);
+    plans[some] = plan_of(items[i].handle, batches[i].Q, n_items < 2 || queued[order[1]]);
     sizes[some] = batches[i].Q;
     split[some] = items[i].handle->precision == HB_PRECISION_BF16X3;
     all_wide = all_wide && plans[some].G != 0;

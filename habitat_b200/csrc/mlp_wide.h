@@ -14,7 +14,8 @@ struct WidePlan {
   int G, W, groups, per_group;
   bool near;
 };
-WidePlan wide_plan(int64_t Q, bool split, int sm_count);
+// alone: no other batches of the call run beside it
+WidePlan wide_plan(int64_t Q, bool split, int sm_count, bool alone);
 // Queries that can travel as kernel parameters: no copy and no read over PCIe for the scalar API.
 constexpr int kWideInline = 16;
 // A batch of queries.  Either every query has its own row of feats and of dev_row, or (grid_n > 0) the same
