@@ -256,7 +256,9 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
   // (100 queries 25.1 -> 24.3 us, 900 48.2 -> 46.5, 2,000 75.1 -> 74.1).  A function that both roles call: as a step
   // before the roles part it made every layer 30 % slower.  In split precision, with half the queries, it gained
   // nothing and cost 1 to 2 % from 150 queries on: epilogue alone.
-  constexpr bool kAllFeatures = !SPLIT && !NEAR;
+  // So too in four blocks of 32 columns, which three batches that fill the GPU take: 636, 384 and 12 queries side by
+  // side in an iteration batch 68.0 -> 66.0 us, while 1,056 alone give back 47.9 -> 48.6 (48.9 before any of this).
+  constexpr bool kAllFeatures = !SPLIT && !NEAR && !(G == 4 && W == 32);
   auto features = [&]() {
     constexpr int kThreads = kAllFeatures ? wide_threads<W, NEAR>() - 128 : 128;
     auto feat_sync = [] { asm volatile("bar.sync 2, %0;" ::"n"(kThreads) : "memory"); };
