@@ -173,28 +173,32 @@ class _GroupPlan:
         self.mode = mode
         self.mlp_inputs = {}      # op kind -> (features, measured ms) on the GPU, measured ms, columns; filled on first use
         self._layout = None
-        self.started = None       # predictors that were started during the walk,
-        self.staged = None        # and memory that the first prediction's upload reads
         if flat is None:
             self._flatten(operations, indices, mode)
         else:
             self._take(operations, flat)
 
     @classmethod
-    def of_whole_trace(cls, operations, mode, with_names, early=None):
+    def of_whole_trace(cls, operations, mode, with_names, early=None, first=None):
         """The plan of a trace recorded on one device, walked by the native binding; None when the
         operations are not all of this package's ordinary classes (any object with their surface
         takes the Python walk), or when a missing metric has to raise (the roofline strategy).
-        early(inputs of the MLP kinds, indices of their operations) is called before the kernels are walked."""
+        early(inputs of the MLP kinds, indices of their operations) is called before the kernels are walked.
+        What belongs to the prediction that asks and not to the plan goes into the list `first`: what `early`
+        returned, and memory to be kept until that prediction has ended."""
         if mode == wave_batch.ROOFLINE:
             return None
         flat = _native.binding().flatten_trace(operations, _trace_types(), SPECIAL_OPERATIONS, _MLP_OPS, _METRIC_KEYS,
                                                mode != wave_batch.RESIMPLIFIED, _FAST_ORDERS, with_names, early)
-        return cls(operations, None, mode, flat) if flat is not None else None
+        if flat is None:
+            return None
+        if first is not None:
+            first.extend(flat[-2:])
+        return cls(operations, None, mode, flat[:-2])
 
     def _take(self, operations, flat):
         (self.n_kernels, self.n_runs, self._names, wave_idx, fwd, bwd, offsets, overheads, kind_idx, self.passthrough_idx,
-         records, metrics, self.offsets_dev, special, self.started, self.staged) = flat
+         records, metrics, self.offsets_dev, special) = flat
         self._kernels, self._operations = None, operations
         self.indices = None                      # all operations
         self.wave_idx, self.fwd_run, self.bwd_run, self.offsets = (
@@ -446,34 +450,33 @@ class Predictor:
         mode = getattr(self._wave_scaling_strategy, "batch_mode", None)
         origin = operations[0].device
         key = ("whole", mode, len(operations))
-        plan = cache.get(key) if cache is not None else None
+        known = cache.get(key) if cache is not None else None
+        plan, first = known, [None]              # first: of this prediction alone, whoever else finds the plan
+        if mode is None or any(d.name == origin.name for d in dest_devices):
+            return None
         if plan is None:
-            if mode is None or any(d.name == origin.name for d in dest_devices):
-                return None
+            first = []
             plan = _GroupPlan.of_whole_trace(
                 operations, mode, self._has_registers(),
-                lambda special, indices: self._start_kinds(special, indices, origin, dest_devices, len(operations)))
+                lambda special, indices: self._start_kinds(special, indices, origin, dest_devices, len(operations)),
+                first)
             if plan is None:
                 return None
-            if cache is not None:
-                cache[key] = plan
-        elif mode is None or any(d.name == origin.name for d in dest_devices):
-            return None
         ms = np.empty((len(dest_devices), len(operations)), np.float64)
         for i in plan.passthrough_idx:
             ms[:, i] = operations[i].run_time_ms
-        started, plan.started = plan.started, None          # for this prediction; the plan is used again
-        times, totals, sums = self._run_plan(plan, operations, origin, dest_devices, ms, started)
-        plan.staged = None
+        times, totals, sums = self._run_plan(plan, operations, origin, dest_devices, ms, first[0])
+        if known is None and cache is not None:
+            cache[key] = plan                    # not before its records are on the GPU, for other streams as well
         return [PredictedOperations(operations, dest, dict(plan=plan, times=times[t], totals=totals[t]), ms[t], sums[t])
                 for t, dest in enumerate(dest_devices)]
 
     def _start_kinds(self, special, indices, origin, dests, n_operations):
         """Starts the predictors of a trace whose kernels are still being walked: what run_group takes as their
-        results, with the kinds it is for and the handles in use, or None when they cannot be started now (`_run_plan`
+        results, with the kinds it is for, or None when they cannot be started now (`_run_plan`
         then runs them, and raises what there is to raise)."""
         try:
-            kinds, names, held = [], [], []
+            kinds, held = [], []
             for name, idx in zip(_MLP_OPS, indices):
                 if not idx:
                     continue
@@ -484,8 +487,7 @@ class Predictor:
                 rows = bytes([pred.device_row(origin.name)] + [pred.device_row(d.name) for d in dests])
                 held.append(pred._handle)
                 kinds.append((held[-1]._handle.value or 0, got[0], got[1], rows, idx))
-                names.append(name)
-            return _native.binding().start_kinds(kinds, len(dests), n_operations), kinds, names, held
+            return _native.binding().start_kinds(kinds, len(dests), n_operations, held), kinds
         except Exception:
             return None
 
@@ -507,12 +509,12 @@ class Predictor:
             if whole and mode is not None:
                 plan = _GroupPlan.of_whole_trace(operations, mode, self._has_registers())
             plan = plan or _GroupPlan(operations, indices, mode)
-            if cache is not None:
-                cache[key] = plan
         ms = np.zeros((len(dests), len(operations)), np.float64)
         for i in plan.passthrough_idx:
             ms[:, i] = operations[i].run_time_ms
         times, totals, _ = self._run_plan(plan, operations, origin, dests, ms)
+        if cache is not None:
+            cache[key] = plan                    # as in _predict_whole
         for t, d in enumerate(targets):
             res = results[d]
             g = len(res._groups)
@@ -537,8 +539,7 @@ class Predictor:
         names = [name for name in _MLP_OPS if len(plan.mlp_idx[name])]
         kinds, native, held = [], [], []
         if started is not None:
-            started, kinds, native, held = started
-            names = []
+            kinds, native, names = started[1], names, []
         for name in names:
             pred = self._predictor(name)
             rows = bytes([pred.device_row(origin.name)] + [pred.device_row(d.name) for d in dests])
@@ -571,7 +572,8 @@ class Predictor:
             "run_group", _native.binding().run_group, flat.batch if flat is not None else None,
             flat.metrics if flat is not None else None, origin, dests, regs,
             plan.offsets_dev if flat is not None else None, kinds,
-            (plan.overheads, plan.wave_idx, plan.fwd_run, plan.bwd_run), times, totals, ms, *(() if started is None else (started,)))
+            (plan.overheads, plan.wave_idx, plan.fwd_run, plan.bwd_run), times, totals, ms,
+            *(() if started is None else started[:1]))
         if nan:
             wave_batch.raise_zero_wave()
         for name, raw in zip(native, clamped):

@@ -1168,16 +1168,17 @@ struct Started {
   at::Tensor block, host;
   cudaStream_t s = nullptr;
   int64_t T = 0;
+  Ref held{nullptr};          // the predictors, and what `kinds` points into
   std::vector<Kind> kinds;
   bool launched = false;
   ~Started() {
     if (launched) cudaStreamSynchronize(s);
   }
 };
-// start_kinds([as for run_group], destinations, operations) -> capsule.  The caller keeps the list's objects alive.
+// start_kinds([as for run_group], destinations, operations, objects that keep the handles alive) -> capsule
 PyObject* start_kinds(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  if (n_args != 3 || !PyList_Check(a[0])) {
+  if (n_args != 4 || !PyList_Check(a[0])) {
     PyErr_SetString(PyExc_TypeError, "start_kinds: bad arguments");
     return nullptr;
   }
@@ -1189,6 +1190,10 @@ PyObject* start_kinds(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     PyErr_Format(PyExc_TypeError, "start_kinds: %s", wrong);
     return nullptr;
   }
+  Ref list(PySequence_Tuple(a[0])), handles(PySequence_Tuple(a[3]));
+  if (!list.p || !handles.p) return nullptr;
+  st->held.p = PyTuple_Pack(2, list.p, handles.p);
+  if (!st->held.p) return nullptr;
   size_t pinned = 0, device = 0;
   std::vector<std::pair<size_t, size_t>> at;
   for (const Kind& k : st->kinds) at.emplace_back(place(&device, pred_bytes(k, st->T)), place(&pinned, times_bytes(k, st->T)));
@@ -1276,7 +1281,8 @@ PyObject* run_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (!started) return nullptr;
     bool same = started->T == T && started->kinds.size() == kinds.size();
     for (size_t i = 0; same && i < kinds.size(); ++i)
-      same = kinds[i].h == started->kinds[i].h && kinds[i].n == started->kinds[i].n && kinds[i].f == started->kinds[i].f;
+      same = kinds[i].h == started->kinds[i].h && kinds[i].n == started->kinds[i].n && kinds[i].f == started->kinds[i].f &&
+             kinds[i].ms == started->kinds[i].ms && std::memcmp(kinds[i].rows, started->kinds[i].rows, T + 1) == 0;
     if (!same) return refuse("other kinds than were started");
   }
   std::vector<std::pair<size_t, size_t>> at;

@@ -297,3 +297,80 @@ def test_ranges_on_a_timeline(monkeypatch):
         handle.predict_one([1.0, 2.0], 0)
     assert opened == ["hb_wave_scale", "hb_wave_scale_metrics", "hb_wave_scale_partials", "hb_mlp_predict_host"]
     assert len(closed) == 4
+
+
+class _StandIns:
+    """Stand-ins for the native walk over a trace (a linear and a gru operation, no kernels), for the predictors that are
+    started during it and for the run; they keep what they were asked for."""
+
+    def __init__(self, monkeypatch):
+        import types
+        from habitat_b200.analysis import predictor as module
+        self.started, self.ran, self.fail = [], [], None
+
+        def flatten_trace(operations, classes, special, kinds, metrics, with_metrics, orders, with_names, early):
+            idx = [b"", np.zeros(1, np.int64).tobytes(), b"", b""]
+            inputs = [None, ("features", "ms", np.ones(1, np.float32).tobytes()), None]
+            got = early(inputs, idx) if early is not None else None
+            return 0, 0, None, b"", b"", bytes(8), b"", b"", idx, [1], None, None, None, inputs, got, "staged"
+
+        def start_kinds(kinds, T, n_operations, handles):
+            self.started.append(kinds[0][3])
+            if self.fail is not None:
+                raise self.fail
+            return "started for %s" % list(kinds[0][3])
+
+        def run_group(kernels, metrics, origin, dests, regs, offsets, kinds, passes, times, totals, ms, *started):
+            self.ran.append((kinds[0][3], started))
+            ms[:, 0] = list(kinds[0][3])[1:]
+            return False, [0.0] * len(dests), [None]
+
+        self.handle = types.SimpleNamespace(_handle=types.SimpleNamespace(value=77))
+        self.pred = RuntimePredictor("linear", 1, 16)
+        self.pred._handle, self.pred._device_rows = self.handle, {"V100": 0, "T4": 1, "P100": 2, "P4000": 3}
+        self.predictor = module.Predictor()
+        self.predictor.linear_pred = self.pred
+        self.binding = types.SimpleNamespace(flatten_trace=flatten_trace, start_kinds=start_kinds, run_group=run_group)
+        monkeypatch.setattr(module._native, "binding", lambda: self.binding)
+
+
+def test_started_predictors_are_of_one_prediction(monkeypatch):
+    """What the first prediction of a trace has started is for its destinations and weights alone: not for the next
+    prediction after one that was interrupted, and not for one that comes as soon as the plan is in the cache."""
+    from habitat_b200.analysis.trace import Trace
+    stand_ins = _StandIns(monkeypatch)
+
+    class Run:
+        run_time_ms = 2.0
+
+        def interrupt(self):
+            raise KeyboardInterrupt
+
+    class Interrupted(Run):
+        run_time_ms = property(Run.interrupt)
+
+    ops = [MeasuredOperation("linear", Arguments(((2, 4), (3, 4), None), {}), Run(), None, Device.V100),
+           MeasuredOperation("gru", Arguments((), {}), Interrupted(), None, Device.V100)]
+    rows = {d: bytes([0, stand_ins.pred._device_rows[d.name]]) for d in (Device.T4, Device.P100, Device.P4000)}
+    trace = Trace(Device.V100, ops)
+    with pytest.raises(KeyboardInterrupt):
+        trace.to_devices([Device.T4], stand_ins.predictor)
+    ops[1]._forward = Run()
+    assert trace.to_devices([Device.P100], stand_ins.predictor)[0].operations.run_times_ms.tolist() == [2.0, 2.0]
+    assert stand_ins.started == [rows[Device.T4], rows[Device.P100]]
+    assert stand_ins.ran == [(rows[Device.P100], ("started for [0, 2]",))]
+
+    # one that comes as soon as the plan can be found
+    class Cache(dict):
+        def __setitem__(self, key, plan):
+            super().__setitem__(key, plan)
+            if key[0] == "whole" and not seen:
+                seen.append(list(stand_ins.ran))       # by then the first one has ended
+                seen.append(trace.to_devices([Device.P4000], stand_ins.predictor))
+    seen, stand_ins.started, stand_ins.ran = [], [], []
+    trace = Trace(Device.V100, ops)
+    trace._prediction_cache = Cache()
+    assert trace.to_devices([Device.T4], stand_ins.predictor)[0].operations.run_times_ms.tolist() == [1.0, 2.0]
+    assert seen[0] == [(rows[Device.T4], ("started for [0, 1]",))]
+    assert seen[1][0].operations.run_times_ms.tolist() == [3.0, 2.0]
+    assert stand_ins.ran[1:] == [(rows[Device.P4000], ())] and stand_ins.started == [rows[Device.T4]]

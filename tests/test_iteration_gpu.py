@@ -242,11 +242,92 @@ def test_predictors_started_during_the_walk(bench_devices, monkeypatch, n):
     assert started.pop() is not None
     for (a, b), (c, d) in zip(got, first):
         assert np.allclose(np.frombuffer(b), np.frombuffer(d), rtol=1e-12) and np.isclose(a, c, rtol=1e-12)
-    # results of other kinds than were started are refused
-    with pytest.raises(TypeError):
-        _native.binding().run_group(None, None, origin, dests, None, None, [], (b"", b"", b"", b""),
-                                    np.empty((5, 0), np.float32), np.empty((5, 0)), np.empty((5, 0)),
-                                    real(p, *_special_of(trace), origin, dests, len(trace.operations))[0])
+    # results of other kinds than were started are refused, and of other devices
+    capsule, kinds = real(p, *_special_of(trace), origin, dests, len(trace.operations))
+    turned = [(h, f, ms, rows[:1] + rows[:0:-1], idx) for h, f, ms, rows, idx in kinds]
+    for wrong in ([], turned):
+        with pytest.raises(TypeError, match="other kinds"):
+            _native.binding().run_group(None, None, origin, dests, None, None, wrong, (b"", b"", b"", b""),
+                                        np.empty((5, 0), np.float32), np.empty((5, 0)),
+                                        np.empty((5, len(trace.operations))), capsule)
+
+
+def test_started_predictors_are_of_one_prediction(bench_devices):
+    """Predictions of one trace that come between the first one's start of its predictors and its end, in the same thread
+    after an interruption, from another stream as soon as the plan can be found, and from other threads: each has the
+    results of its own destinations."""
+    import threading
+    from habitat_b200.analysis.arguments import Arguments
+    from habitat_b200.analysis.mlp.mlp import RuntimePredictor
+    from habitat_b200.analysis.operation import MeasuredOperation
+    from habitat_b200.analysis.predictor import Predictor
+    from habitat_b200.analysis.run_time import RunTimeMeasurement
+    origin, dests = bench_devices[0], bench_devices[1:]
+    p = Predictor()
+    for k, op in enumerate(("conv2d", "linear", "bmm")):
+        torch.manual_seed(k)
+        pred = RuntimePredictor(op, 2, 1024)
+        F = len(pred.model.features)
+        pred.mu, pred.sigma = np.full(F + 4, 10.0), np.full(F + 4, 50.0)
+        pred.model.fc2.bias.data.fill_(1.0)
+        setattr(p, op + "_pred", pred)
+
+    def result(trace, targets):
+        return [t.operations.run_times_ms.tobytes() for t in trace.to_devices(targets, p)]
+
+    class Meanwhile(dict):
+        """Calls a function as soon as a plan can be found."""
+        def __setitem__(self, key, plan):
+            super().__setitem__(key, plan)
+            if key[0] == "whole" and self.then is not None:
+                then, self.then = self.then, None
+                then()
+
+    class Interrupted(RunTimeMeasurement):
+        @property
+        def run_time_ms(self):
+            if raising:
+                raise raising.pop()
+            return 2.0
+
+    raising = []
+
+    def recorded():
+        trace = _recorded(origin, 60, 11)
+        trace.operations.append(MeasuredOperation("gru", Arguments((), {}), Interrupted(2.0, [], origin), None, origin))
+        return trace
+
+    want, turned = result(recorded(), dests), result(recorded(), dests[::-1])
+    assert want == turned[::-1] and want != turned
+    trace = recorded()
+    raising.append(KeyboardInterrupt())
+    with pytest.raises(KeyboardInterrupt):
+        trace.to_devices(dests, p)
+    assert result(trace, dests[::-1]) == turned
+
+    trace, seen, other = recorded(), [], torch.cuda.Stream()
+    trace._prediction_cache = Meanwhile()
+
+    def on_another_stream():
+        with torch.cuda.stream(other):
+            seen.append(result(trace, dests[::-1]))
+    trace._prediction_cache.then = on_another_stream
+    assert result(trace, dests) == want and seen == [turned]
+
+    for _ in range(10):
+        trace, results = recorded(), {}
+        start = threading.Barrier(4)
+
+        def predict(i):
+            with torch.cuda.stream(torch.cuda.Stream()):
+                start.wait()
+                results[i] = result(trace, dests if i % 2 else dests[::-1])
+        threads = [threading.Thread(target=predict, args=(i,)) for i in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert results == {i: want if i % 2 else turned for i in range(4)}
 
 
 def _special_of(trace):
