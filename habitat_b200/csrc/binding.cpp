@@ -625,13 +625,13 @@ bool feature_row(long kind, PyObject* op, PyTypeObject* op_type, PyTypeObject* r
 PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
   if (n_args != 9) return not_ordinary();
-  Ref ops(PySequence_Fast(a[0], "operations must be a sequence"));
+  Ref ops(PySequence_Tuple(a[0]));   // `early` runs Python, other threads as well: a list may change meanwhile
   if (!ops.p) return nullptr;
   PyTypeObject* type[4];
   for (int i = 0; i < 4; ++i) type[i] = reinterpret_cast<PyTypeObject*>(PyTuple_GET_ITEM(a[1], i));
   PyObject *special = a[2], *kinds = a[3], *metrics = a[4];
   const bool with_metrics = PyObject_IsTrue(a[5]) == 1, with_names = PyObject_IsTrue(a[7]) == 1;
-  const Py_ssize_t n = PySequence_Fast_GET_SIZE(ops.p), n_kinds = PyTuple_GET_SIZE(kinds);
+  const Py_ssize_t n = PyTuple_GET_SIZE(ops.p), n_kinds = PyTuple_GET_SIZE(kinds);
 
   Ref names(with_names ? PyList_New(0) : Py_NewRef(Py_None)), passed(PyList_New(0));
   if (n_kinds < kFeatureKinds || n_kinds > 8) return not_ordinary();
@@ -703,7 +703,7 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   };
 
   for (Py_ssize_t i = 0; i < n; ++i) {
-    PyObject* op = PySequence_Fast_GET_ITEM(ops.p, i);
+    PyObject* op = PyTuple_GET_ITEM(ops.p, i);
     if (Py_TYPE(op) != type[0]) return not_ordinary();
     Ref name(field(op, s__name)), device(field(op, s__device));
     if (!name.p || !device.p) return not_ordinary();

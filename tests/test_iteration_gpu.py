@@ -335,3 +335,24 @@ def _special_of(trace):
     plan = next(v for k, v in trace._prediction_cache.items() if k[0] == "whole")
     return ([plan.mlp_inputs[k][:2] for k in ("conv2d", "linear", "bmm")],
             [plan.mlp_idx[k].tobytes() for k in ("conv2d", "linear", "bmm")])
+
+
+def test_operations_removed_during_the_walk(bench_devices):
+    """A list of operations that is emptied while the predictors are started (another thread can): the walk over their
+    kernels still has them, and records what it would have."""
+    import gc
+    import weakref
+    from habitat_b200.analysis.predictor import _GroupPlan
+    want = _GroupPlan.of_whole_trace(_recorded(bench_devices[0], 20, 5).operations, "unified", False)
+    operations = _recorded(bench_devices[0], 20, 5).operations
+    alive = [weakref.ref(op) for op in operations]
+
+    def early(inputs, indices):
+        operations.clear()
+        gc.collect()
+        assert all(ref() is not None for ref in alive)     # (before the walk goes on to them)
+    got = _GroupPlan.of_whole_trace(operations, "unified", False, early)
+    assert not operations and got.n_kernels == want.n_kernels > 0
+    for name, plane in vars(want.flat.batch).items():
+        assert torch.equal(plane, getattr(got.flat.batch, name)), name
+    assert np.array_equal(got.overheads, want.overheads) and np.array_equal(got.wave_idx, want.wave_idx)
