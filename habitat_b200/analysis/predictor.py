@@ -183,7 +183,8 @@ class _GroupPlan:
         """The plan of a trace recorded on one device, walked by the native binding; None when the
         operations are not all of this package's ordinary classes (any object with their surface
         takes the Python walk), or when a missing metric has to raise (the roofline strategy).
-        early(inputs of the MLP kinds, indices of their operations) is called before the kernels are walked.
+        early(inputs of the MLP kinds, indices of their operations) is called before the kernels are walked, with None
+        for the inputs when some kind's are not known by then.
         What belongs to the prediction that asks and not to the plan goes into the list `first`: what `early`
         returned, and memory to be kept until that prediction has ended."""
         if mode == wave_batch.ROOFLINE:
@@ -475,14 +476,16 @@ class Predictor:
         """Starts the predictors of a trace whose kernels are still being walked: what run_group takes as their
         results, with the kinds it is for, or None when they cannot be started now (`_run_plan`
         then runs them, and raises what there is to raise)."""
+        if special is None:
+            return None
         try:
             kinds, held = [], []
             for name, idx in zip(_MLP_OPS, indices):
                 if not idx:
                     continue
-                got = special[_FAST_KINDS.index(name)] if name in _FAST_KINDS else None
+                got = special[_FAST_KINDS.index(name)]
                 pred = self._predictor(name)
-                if got is None or FEATURES[name] != pred.model.features or not self._is_plain(pred):
+                if FEATURES[name] != pred.model.features or not self._is_plain(pred):
                     return None
                 rows = bytes([pred.device_row(origin.name)] + [pred.device_row(d.name) for d in dests])
                 held.append(pred._handle)

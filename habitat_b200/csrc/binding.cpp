@@ -621,7 +621,8 @@ bool feature_row(long kind, PyObject* op, PyTypeObject* op_type, PyTypeObject* r
 //     kept until the stream has got to the end of the upload, or None)
 // The operations of the MLP kinds are walked first.  early(the entries per kind of the first three, indices per MLP kind)
 // is called when their features are on the GPU, before the walk over the kernels, which takes longer than the
-// predictors do: what it launches runs meanwhile.
+// predictors do: what it launches runs meanwhile.  Where a kind has no features yet (it is not of the first three, or one
+// of its operations was not recorded positionally) the features go with the records, and `early` gets None for the entries.
 PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
   if (n_args != 9) return not_ordinary();
@@ -789,8 +790,18 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   Ref special_rows(PyTuple_New(kFeatureKinds)), kinds_out(PyTuple_New(n_kinds)), started(Py_NewRef(Py_None));
   if (!special_rows.p || !kinds_out.p) return nullptr;
   for (Py_ssize_t k = 0; k < n_kinds; ++k) PyTuple_SET_ITEM(kinds_out.p, k, bytes_of(kind_idx[k]));
-  // the features go on their own when something is to start with them, else with the records
-  const bool early = a[8] != Py_None;
+  // the features go on their own when all kinds can start with them, else with the records
+  bool early = a[8] != Py_None, any = false, all = true;
+  for (Py_ssize_t k = 0; k < n_kinds; ++k) {
+    if (kind_idx[k].empty()) continue;
+    any = true;
+    all = all && k < kFeatureKinds && feats[k].ok;
+  }
+  if (early && any && !all) {
+    Ref none(PyObject_CallFunctionObjArgs(a[8], Py_None, kinds_out.p, nullptr));
+    if (!none.p) return nullptr;
+  }
+  early = early && any && all;
   Upload& with = early ? features : records;
   auto put_features = [&] {
     for (Rows& r : feats) {
@@ -815,7 +826,7 @@ PyObject* flatten_trace(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (!features.go(false)) return nullptr;
     take_features();
     if (PyErr_Occurred()) return nullptr;
-    if (!features.host.empty()) Py_SETREF(started.p, PyObject_CallFunctionObjArgs(a[8], special_rows.p, kinds_out.p, nullptr));
+    Py_SETREF(started.p, PyObject_CallFunctionObjArgs(a[8], special_rows.p, kinds_out.p, nullptr));
     if (!started.p) return nullptr;
   }
 

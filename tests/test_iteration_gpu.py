@@ -356,3 +356,23 @@ def test_operations_removed_during_the_walk(bench_devices):
     for name, plane in vars(want.flat.batch).items():
         assert torch.equal(plane, getattr(got.flat.batch, name)), name
     assert np.array_equal(got.overheads, want.overheads) and np.array_equal(got.wave_idx, want.wave_idx)
+
+
+def test_traces_whose_predictors_cannot_start_go_up_in_one_piece(bench_devices):
+    """An lstm operation, or one recorded by keyword, keeps the predictors from starting during the walk: features and
+    records then are one upload, and nothing has to be kept for it."""
+    from habitat_b200.analysis.arguments import Arguments
+    from habitat_b200.analysis.operation import MeasuredOperation
+    from habitat_b200.analysis.predictor import _GroupPlan
+    from habitat_b200.analysis.run_time import RunTimeMeasurement
+    origin = bench_devices[0]
+    lstm = MeasuredOperation("lstm", Arguments(((12, 4, 64), ((2, 4, 128),), (), True, 2, 0.0, False, False, False), {}),
+                             RunTimeMeasurement(1.5, [], origin), None, origin)
+    plain, keyword = _recorded(origin, 5, 9), _recorded(origin, 5, 9, Arguments(((4, 32), (64, 32)), {"bias": None}))
+    for operations, together in ((plain.operations, False), (plain.operations + [lstm], True), (keyword.operations, True)):
+        asked, first = [], []
+        plan = _GroupPlan.of_whole_trace(operations, "unified", False, lambda *a: asked.append(a) or "started", first)
+        one = plan.mlp_inputs["conv2d"][0].untyped_storage().data_ptr() == \
+            plan.flat.batch.num_blocks.untyped_storage().data_ptr()
+        assert one == together and [a[0] is None for a in asked] == [together]
+        assert first[0] == (None if together else "started") and (first[1] is None) == together
