@@ -490,7 +490,8 @@ class Predictor:
                 rows = bytes([pred.device_row(origin.name)] + [pred.device_row(d.name) for d in dests])
                 held.append(pred._handle)
                 kinds.append((held[-1]._handle.value or 0, got[0], got[1], rows, idx))
-            return _native.binding().start_kinds(kinds, len(dests), n_operations, held), kinds
+            return batched._call("start_kinds", _native.binding().start_kinds, kinds, len(dests), n_operations,
+                                 held), kinds
         except Exception:
             return None
 

@@ -334,28 +334,30 @@ class _StandIns:
         monkeypatch.setattr(module._native, "binding", lambda: self.binding)
 
 
+def _linear_and_gru():
+    run = RunTimeMeasurement(2.0, [], Device.V100)
+    return [MeasuredOperation("linear", Arguments(((2, 4), (3, 4), None), {}), run, None, Device.V100),
+            MeasuredOperation("gru", Arguments((), {}), run, None, Device.V100)]
+
+
 def test_started_predictors_are_of_one_prediction(monkeypatch):
     """What the first prediction of a trace has started is for its destinations and weights alone: not for the next
     prediction after one that was interrupted, and not for one that comes as soon as the plan is in the cache."""
     from habitat_b200.analysis.trace import Trace
     stand_ins = _StandIns(monkeypatch)
 
-    class Run:
-        run_time_ms = 2.0
-
-        def interrupt(self):
+    class Interrupted:
+        @property
+        def run_time_ms(self):
             raise KeyboardInterrupt
 
-    class Interrupted(Run):
-        run_time_ms = property(Run.interrupt)
-
-    ops = [MeasuredOperation("linear", Arguments(((2, 4), (3, 4), None), {}), Run(), None, Device.V100),
-           MeasuredOperation("gru", Arguments((), {}), Interrupted(), None, Device.V100)]
+    ops = _linear_and_gru()
+    measured, ops[1]._forward = ops[1].forward, Interrupted()
     rows = {d: bytes([0, stand_ins.pred._device_rows[d.name]]) for d in (Device.T4, Device.P100, Device.P4000)}
     trace = Trace(Device.V100, ops)
     with pytest.raises(KeyboardInterrupt):
         trace.to_devices([Device.T4], stand_ins.predictor)
-    ops[1]._forward = Run()
+    ops[1]._forward = measured
     assert trace.to_devices([Device.P100], stand_ins.predictor)[0].operations.run_times_ms.tolist() == [2.0, 2.0]
     assert stand_ins.started == [rows[Device.T4], rows[Device.P100]]
     assert stand_ins.ran == [(rows[Device.P100], ("started for [0, 2]",))]
@@ -374,3 +376,17 @@ def test_started_predictors_are_of_one_prediction(monkeypatch):
     assert seen[0] == [(rows[Device.T4], ("started for [0, 1]",))]
     assert seen[1][0].operations.run_times_ms.tolist() == [3.0, 2.0]
     assert stand_ins.ran[1:] == [(rows[Device.P4000], ())] and stand_ins.started == [rows[Device.T4]]
+
+
+def test_ranges_of_a_first_prediction(monkeypatch):
+    """The predictors that a first prediction starts during the walk stand in a range of their own, closed also when the
+    launch fails."""
+    import torch
+    from habitat_b200 import batched
+    from habitat_b200.analysis.trace import Trace
+    stand_ins, opened, closed = _StandIns(monkeypatch), [], []
+    monkeypatch.setattr(batched, "_NVTX", True)
+    monkeypatch.setattr(torch.cuda.nvtx, "range_push", opened.append)
+    monkeypatch.setattr(torch.cuda.nvtx, "range_pop", lambda: closed.append(1))
+    Trace(Device.V100, _linear_and_gru()).to_devices([Device.T4], stand_ins.predictor)
+    assert opened == ["start_kinds", "run_group"] and len(closed) == 2
