@@ -475,8 +475,8 @@ class Predictor:
     def _start_kinds(self, special, indices, origin, dests, n_operations):
         """Starts the predictors of a trace whose kernels are still being walked: what run_group takes as their
         results, with the kinds it is for, or None when they cannot be started now (`_run_plan`
-        then runs them, and raises what there is to raise)."""
-        if special is None:
+        then prepares them again and raises what there is to raise).  What a launch raises is raised here."""
+        if special is None or len(dests) > _native.HB_MAX_DEVICES:
             return None
         try:
             kinds, held = [], []
@@ -490,10 +490,9 @@ class Predictor:
                 rows = bytes([pred.device_row(origin.name)] + [pred.device_row(d.name) for d in dests])
                 held.append(pred._handle)
                 kinds.append((held[-1]._handle.value or 0, got[0], got[1], rows, idx))
-            return batched._call("start_kinds", _native.binding().start_kinds, kinds, len(dests), n_operations,
-                                 held), kinds
         except Exception:
             return None
+        return batched._call("start_kinds", _native.binding().start_kinds, kinds, len(dests), n_operations, held), kinds
 
     @staticmethod
     def _is_plain(pred):

@@ -390,3 +390,22 @@ def test_ranges_of_a_first_prediction(monkeypatch):
     monkeypatch.setattr(torch.cuda.nvtx, "range_pop", lambda: closed.append(1))
     Trace(Device.V100, _linear_and_gru()).to_devices([Device.T4], stand_ins.predictor)
     assert opened == ["start_kinds", "run_group"] and len(closed) == 2
+
+
+def test_errors_of_predictors_that_start_during_the_walk(monkeypatch):
+    """What keeps a predictor from being started is raised by the run that follows the walk, as ever; what its launch
+    raises is raised at once, and nothing is launched again."""
+    from habitat_b200 import _native
+    from habitat_b200.analysis.trace import Trace
+    stand_ins = _StandIns(monkeypatch)
+    predict = lambda dests: Trace(Device.V100, _linear_and_gru()).to_devices(dests, stand_ins.predictor)
+    stand_ins.fail = _native.HabitatNativeError(_native.HB_ERR_CUDA, "out of memory")
+    with pytest.raises(_native.HabitatNativeError, match="out of memory"):
+        predict([Device.T4])
+    assert len(stand_ins.started) == 1 and not stand_ins.ran
+    many = [Device.T4] * (_native.HB_MAX_DEVICES + 1)      # refused by the run
+    assert len(predict(many)) == len(many) and len(stand_ins.started) == 1 and len(stand_ins.ran) == 1
+    stand_ins.pred.invalidate()                             # no mu and sigma to make the handle from
+    with pytest.raises(RuntimeError, match="mu/sigma"):
+        predict([Device.T4])
+    assert len(stand_ins.started) == 1 and len(stand_ins.ran) == 1
