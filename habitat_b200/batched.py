@@ -308,6 +308,11 @@ class MLPHandle:
         """Writes the device status word from the host (tests of the error path)."""
         _native.check(_native.load().hb_mlp_inject_status(self._handle, int(code)))
 
+    def inject_mark(self):
+        """Leaves, from the host, the mark of a small-batch launch that gave up (tests of the error path): the next
+        such launch on this GPU reports an error instead of results."""
+        _native.check(_native.load().hb_mlp_inject_mark(self._handle))
+
     def phase_cycles(self):
         """Cycle counters of the first cluster in the last bf16 launch (synchronises): epilogue group 0
         (wait, epilogue, fc2, layers, epi_publish, epi_remote), the MMA issuer (mma_wait_act,

@@ -1139,6 +1139,15 @@ extern "C" hb_status hb_mlp_inject_status(hb_mlp* h, int32_t device_status) {
   return HB_OK;
 }
 
+extern "C" hb_status hb_mlp_inject_mark(hb_mlp* h) {
+  if (!h) {
+    hb::set_error("hb_mlp_inject_mark: NULL handle");
+    return HB_ERR_INVALID_ARGUMENT;
+  }
+  const hb_status st = check_device(h);
+  return st != HB_OK ? st : hb::wide_set_mark(h->device);
+}
+
 extern "C" hb_status hb_mlp_phase_cycles(hb_mlp* h, int64_t out[16]) {
   if (!h || !out) {
     hb::set_error("hb_mlp_phase_cycles: NULL argument");

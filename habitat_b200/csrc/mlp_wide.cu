@@ -32,6 +32,10 @@
 // Warp roles: 0 MMA issuer (and TMEM), 1 weight producer, 2 the mark, 4-7 epilogue (one TMEM lane quadrant each),
 // 8-15 (64 columns: 8-23, NEAR: none) receivers.  Every wait is bounded, as in mlp_chain.cu; a launch that gave up
 // leaves a mark in the scratch, and launches that find it report an error instead of a result.
+//
+// After giving up no ring slot may be requested again that nobody has waited for: its copy could still be under way,
+// and its barrier would be armed a second time in one phase.  So the MMA issuer, whose commits free the slots, waits
+// for the producer to leave before it issues anything past a wait that ran out, and goes no further than the layer's end.
 #include <atomic>
 #include <cstring>
 
@@ -205,8 +209,9 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
   const uint32_t bar_tfree = bars + 192;                      // TMEM read out (4 warps)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_ptr + 200);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + 204);
-  const uint32_t bar_drain = bars + 216;                      // after giving up: the MMAs have ended
   volatile int* mark_seen = reinterpret_cast<volatile int*>(bars_ptr + 208);
+  volatile int* producer_left = reinterpret_cast<volatile int*>(bars_ptr + 212);
+  const uint32_t bar_drain = bars + 216;                      // after giving up: the MMAs have ended
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = static_cast<int>(blockIdx.x) / G, c = static_cast<int>(blockIdx.x) % G;   // group = cluster
@@ -222,6 +227,7 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
     mbar_init(bar_drain, 1);
     *abort_flag = 0;
     *mark_seen = 0;
+    *producer_left = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // (before the peers' first stores)
@@ -332,6 +338,7 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
           }
         }
       }
+      *producer_left = 1;
     }
   } else if (warp == 0) {
     // ------------------------------ MMA issuer ------------------------------
@@ -355,8 +362,11 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
     // on uniform values alone (a wait that ran out has set the abort flag; what is issued after it reads
     // stale shared memory and is discarded).  16 MMAs of 64 x 16 took 1,150 cycles in the plain form.
     if (elect_one()) {
+      auto gave_up = [&] {   // (the producer looks at the abort flag when a slot does not come)
+        for (const long long t0 = clock64(); *producer_left == 0 && clock64() - t0 <= kWaitCycles;) {}
+      };
       auto wait = [&](uint32_t bar, uint32_t parity, int code) {
-        wide_wait(bar, parity, abort_flag, p, code);
+        if (!mbar_try_wait(bar, parity) && (*abort_flag || !wide_wait(bar, parity, abort_flag, p, code))) gave_up();
         tc_fence_after();
       };
       // layer L's input: its first K quarter (which has one phase more than the others, fc1's input); NEAR: the whole
@@ -366,7 +376,10 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
           wait(bar_act, L & 1, 0x521);
           return;
         }
-        if (!mbar_wait_cluster(bar_act + 8 * (L & 1), (L >> 1) & 1, abort_flag, p.status, 0x521)) atomicExch(p.poison, 1);
+        if (!mbar_wait_cluster(bar_act + 8 * (L & 1), (L >> 1) & 1, abort_flag, p.status, 0x521)) {
+          atomicExch(p.poison, 1);
+          gave_up();
+        }
         fence_proxy_async();
         tc_fence_after();
       };
@@ -386,7 +399,7 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
       constexpr int kMmas = 4 * kUnitsPerSlot;                   // per slot
       constexpr int kPerQuarter = kSlotsPerBlock / 4;            // slots; none spans two K quarters
 #pragma unroll 1
-      for (int L = 1; L < n_layers; ++L) {
+      for (int L = 1; L < n_layers && *abort_flag == 0; ++L) {
         wait(bar_tfree, (L - 1) & 1, 0x523);
 #pragma unroll 1
         for (int b = 0; b < kBlocks; ++b) {
@@ -570,7 +583,8 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
             }
             fence_proxy_async();
             epi_sync();
-            if (T == 0) mbar_expect_tx(in_bar, static_cast<uint32_t>((G - 1) * kParts * 128 * n_q));
+            // (after giving up the buffer's last phase may be incomplete: it is not armed again)
+            if (T == 0 && *abort_flag == 0) mbar_expect_tx(in_bar, static_cast<uint32_t>((G - 1) * kParts * 128 * n_q));
             const uint32_t chunk = static_cast<uint32_t>(T) & 7u, to = static_cast<uint32_t>(c + (T >> 3)) % G;
             if (T >= 8) {   // eight threads per peer, 16 bytes of each query
               const uint32_t there = map_to_cta(base + mine, to), bar = map_to_cta(in_bar, to);
@@ -946,6 +960,17 @@ void wide_start_over(int device) {
   GpuScratch& g = g_wide[device];
   std::lock_guard<std::mutex> lock(g.mu);
   for (int i = 0; i < g.used; ++i) g.s[i].fresh = true;
+}
+
+hb_status wide_set_mark(int device) {
+  if (device < 0 || device >= kMaxCudaDevices) return HB_OK;
+  GpuScratch& g = g_wide[device];
+  std::lock_guard<std::mutex> lock(g.mu);
+  HB_CUDA_TRY(cudaDeviceSynchronize());
+  for (int i = 0; i < g.used; ++i)
+    HB_CUDA_TRY(cudaMemset(g.s[i].base + kActsBytes + kHalvesBytes, 1, sizeof(int32_t)));
+  HB_CUDA_TRY(cudaDeviceSynchronize());
+  return HB_OK;
 }
 
 std::unique_lock<std::mutex> wide_queue(int device) {

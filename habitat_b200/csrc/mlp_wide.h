@@ -47,6 +47,8 @@ std::unique_lock<std::mutex> wide_queue(int device);
 hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cudaStream_t stream, bool* launched);
 // After a launch that gave up: every stream's scratch on the GPU is set up again before its next use.
 void wide_start_over(int device);
+// Leaves the mark of a launch that gave up in the GPU's scratch (tests of the error path); synchronises.
+hb_status wide_set_mark(int device);
 void wide_handle_created(int device);
 void wide_handle_destroyed(int device);
 }  // namespace hb

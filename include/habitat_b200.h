@@ -256,6 +256,12 @@ hb_status hb_mlp_status(hb_mlp* handle, int32_t* device_status);
  * kernel is made to wait or fail).  No reference counterpart. */
 hb_status hb_mlp_inject_status(hb_mlp* handle, int32_t device_status);
 
+/* Leaves, from the host, the mark that a launch of the small-batch kernel leaves in its
+ * scratch when it gives up (test hook, as above): small-batch launches on the handle's GPU
+ * then store no result and report device status 0x5ff, until a status has been read.
+ * Synchronises.  No reference counterpart. */
+hb_status hb_mlp_inject_mark(hb_mlp* handle);
+
 /* Profiling aid (bf16 kernel): SM cycle counters of the first cluster's leader CTA
  * for the most recent launch.  out[0..3] first epilogue group: waiting for its
  * output blocks, draining them, fc2, layers counted.  out[4..8] MMA issuer:
