@@ -38,6 +38,9 @@
 // Every mbarrier wait is bounded: when a wait runs out the kernel records a status word, the roles
 // leave their loops or run them empty (the two epilogue groups keep meeting at their common barriers, which
 // have no limit of their own), outstanding bulk copies and MMAs are waited for (bounded) and TMEM is released.
+// No ring slot is requested again that nobody has waited for: its copy could still be under way, and its barrier would be
+// armed a second time in one phase.  So the MMA issuer, whose commits free the slots of both CTAs, waits for all
+// producers to leave before it issues anything past a wait that ran out, and goes no further than the tile's end.
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -188,6 +191,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + 276);
   volatile int* epi_ok = reinterpret_cast<volatile int*>(bars_ptr + 280);   // [5]: per epilogue group, twice; the hand-over of fc2
   const uint32_t bar_drain = bars + 304;     // leader only, after giving up: the MMAs have ended
+  volatile int* producers_left = reinterpret_cast<volatile int*>(bars_ptr + 312);   // [2 * kPairProducers] leader only
   float* fc2_mine = reinterpret_cast<float*>(bars_ptr + 512);    // [64] own queries, own features
   float* fc2_peer = reinterpret_cast<float*>(bars_ptr + 768);    // [64] own queries, peer's features
 
@@ -211,6 +215,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
     mbar_init(bar_next, 8);
     mbar_init(bar_drain, 1);
     *abort_flag = 0;
+    for (int i = 0; i < 2 * kPairProducers; ++i) producers_left[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -286,6 +291,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
         }
         n -= tile_loads;
       }
+      st_cluster_u32(map_to_cta(bars + 312 + 4 * (kPairProducers * rank + w), 0), 1u);
       if (timed) { p.phase_cycles[9] = c_empty; p.phase_cycles[10] = c_first; p.phase_cycles[11] = issued; }
     }
   } else if (warp == 1) {
@@ -309,16 +315,22 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
         const bool mtimed = p.phase_cycles != nullptr && blockIdx.x == 0;
         long long mc_act = 0, mc_full = 0, mc_tfree = 0, mc_n = 0;
         int32_t* status = nullptr;
+        auto gave_up = [&] {   // (the producers look at their CTA's abort flag when a slot does not come)
+          st_cluster_u32(map_to_cta(bars + 276, 1), 1u);
+          const long long t0 = clock64();
+          for (int i = 0; i < 2 * kPairProducers; ++i)
+            while (producers_left[i] == 0 && clock64() - t0 <= kWaitCycles) {}
+        };
         auto wait = [&](uint32_t bar, uint32_t parity, long long& acc, int code) {
           const long long m0 = mtimed ? clock64() : 0;
-          mbar_wait_cluster(bar, parity, abort_flag, status, code);
+          if (!mbar_wait_cluster(bar, parity, abort_flag, status, code)) gave_up();
           tc_fence_after();
           if (mtimed) acc += clock64() - m0;
         };
         const long long k0 = clock64();
         const unsigned long long g0 = global_timer_ns();
 #pragma unroll 1
-        for (int t = 0; t < my_tiles; ++t) {
+        for (int t = 0; t < my_tiles && *abort_flag == 0; ++t) {
           const MlpProblem& pb = problem_of(p, pair_id + t * n_pairs);
           const int n_layers = pb.layers + 1;
           status = pb.status;
@@ -462,7 +474,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
     const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     const uint32_t act_peer = map_to_cta(act, peer);
     uint32_t in_phase = 0, lay = 0, tile_no = 0;
-    bool ok = true;
+    bool ok = true, in_order = true;           // in_order (e == 0): no wait for the peer's half of a quarter has run out
     float* red = reinterpret_cast<float*>(base_ptr);   // [8 warps][queries of the tile], aliases activations
     const bool timed = p.phase_cycles != nullptr && blockIdx.x == 0 && T == 0;
     long long c_wait = 0, c_epi = 0, c_fc2 = 0, c_layers = 0, c_ld = 0, c_bias = 0, c_sync = 0, c_loc = 0, c_rem = 0;
@@ -489,9 +501,10 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
             const int gate = L == 0 ? 3 : j;
             const long long c0 = timed ? clock64() : 0;
             if (e == 0) {
-              epi_ok[grp] = mbar_wait(bar_accj + 8 * gate, lay & 1u, abort_flag, pb.status, 0x311) ? 1 : 0;
+              const bool go = in_order && mbar_wait(bar_accj + 8 * gate, lay & 1u, abort_flag, pb.status, 0x311);
+              epi_ok[grp] = go ? 1 : 0;
               // the peer sends 128 K rows x 128 B of this quarter into this CTA
-              mbar_expect_tx(bar_inq + 8 * j, 128u * 128u);
+              if (go) mbar_expect_tx(bar_inq + 8 * j, 128u * 128u);
             }
             group_sync();
             if (epi_ok[grp] == 0) { ok = false; break; }
@@ -568,8 +581,8 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
             group_sync();
             if (e == 0) {
               // own stores are fenced above; the peer's arrive as counted bytes
-              if (mbar_wait_cluster(bar_inq + 8 * j, in_phase, abort_flag, pb.status, 0x313))
-                publish(static_cast<uint32_t>(j));
+              in_order = mbar_wait_cluster(bar_inq + 8 * j, in_phase, abort_flag, pb.status, 0x313);
+              if (in_order) publish(static_cast<uint32_t>(j));
             }
             if (timed) { c_wait += c1 - c0; c_epi += clock64() - c1; c_sync += clock64() - d2; }
           }
@@ -687,6 +700,10 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
     tc_commit_pair(bar_drain);
     const long long t0 = clock64();
     while (!mbar_try_wait_cluster(bar_drain, 0) && clock64() - t0 <= kWaitCycles) {}
+  }
+  if (*abort_flag && threadIdx.x == 0) {
+    // copies that the peer requested and the leader did not count
+    for (const long long t0 = clock64(); clock64() - t0 < 100000;) {}
   }
   __syncthreads();
   cluster_sync_all();   // neither CTA leaves while the other may still touch its memory
