@@ -314,10 +314,12 @@ class MLPHandle:
         _native.check(_native.load().hb_mlp_inject_mark(self._handle))
 
     def phase_cycles(self):
-        """Cycle counters of the first cluster in the last bf16 launch (synchronises): epilogue group 0
-        (wait, epilogue, fc2, layers, epi_publish, epi_remote), the MMA issuer (mma_wait_act,
-        mma_wait_weights, mma_wait_tmem, mma_issue, slots; mma_total_cycles and mma_total_ns over the
-        same interval, whose ratio is the SM clock under load) and the first producer."""
+        """Cycle counters of the first cluster in the last launch of the two-SM kernel (synchronises): epilogue
+        group 0 (wait, epilogue, fc2, layers, epi_publish, epi_remote), the MMA issuer (mma_wait_act,
+        mma_wait_weights, mma_wait_tmem, mma_issue, slots of 16 KB; mma_total_cycles and mma_total_ns over the
+        same interval, whose ratio is the SM clock under load) and the first of three producers
+        (producer_wait_slot: waiting for its slots and requesting copies, copies: how many of them;
+        producer_copy: the launch's first copy alone, not a sum over `copies`)."""
         out = (ctypes.c_int64 * 16)()
         _native.check(_native.load().hb_mlp_phase_cycles(self._handle, out))
         names = ("wait", "epilogue", "fc2", "layers", "mma_wait_act", "mma_wait_weights", "mma_wait_tmem",

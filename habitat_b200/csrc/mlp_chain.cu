@@ -34,7 +34,7 @@
 //
 // Warp roles: warp 0 = TMEM allocation, warp 1 = barrier set-up + MMA issuer (leader CTA),
 // warps 2-5 and 12-15 = two epilogue groups (one TMEM lane quadrant per warp), warps 6-8 =
-// weight producers, warps 9 and 10 = features.
+// weight producers, warps 9 and 10 = features (warp 11 times a copy).
 // Every mbarrier wait is bounded: when a wait runs out the kernel records a status word, the roles
 // leave their loops or run them empty (the two epilogue groups keep meeting at their common barriers, which
 // have no limit of their own), outstanding bulk copies and MMAs are waited for (bounded) and TMEM is released.
@@ -257,7 +257,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
       uint32_t n = w;              // load of the tile
       bool ok = true;
       const bool timed = p.phase_cycles != nullptr && blockIdx.x == 0 && w == 0;
-      long long c_empty = 0, c_first = 0;
+      long long c_empty = 0;
       for (int t = 0; t < my_tiles && ok; ++t) {
         const MlpProblem& pb = problem_of(p, pair_id + t * n_pairs);
         const uint32_t tile_loads = static_cast<uint32_t>(kPairMT + pb.layers * kLayerLoads);
@@ -277,14 +277,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
           if (!mbar_wait(bar_empty + 8 * s, ph, abort_flag, pb.status, 0x111)) { ok = false; break; }
           if (rank == 0) mbar_expect_tx(full, 2 * kPairStageBytes);
           tma_rows_2sm(dst, &pb.tmap_tile, row, full_leader);
-          if (timed) {
-            // (waiting for every copy here, to time it, held up the ring: 2 % of the launch)
-            c_empty += clock64() - c0;
-            if (issued == 0) {
-              mbar_wait(full, 0, abort_flag, pb.status, 0x112);
-              c_first = clock64() - c0;
-            }
-          }
+          if (timed) c_empty += clock64() - c0;   // (a copy that is waited for here, to time it, holds up the ring)
           ++issued;
           s += kPairProducers;
           if (s >= kPairStages) { s = w; ph ^= 1u; }
@@ -292,7 +285,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
         n -= tile_loads;
       }
       st_cluster_u32(map_to_cta(bars + 312 + 4 * (kPairProducers * rank + w), 0), 1u);
-      if (timed) { p.phase_cycles[9] = c_empty; p.phase_cycles[10] = c_first; p.phase_cycles[11] = issued; }
+      if (timed) { p.phase_cycles[9] = c_empty; p.phase_cycles[11] = issued; }
     }
   } else if (warp == 1) {
     if (rank == 0) {
@@ -404,6 +397,13 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
         }
       }
       __syncwarp();
+    }
+  } else if (warp == 11) {
+    // diagnostic: how long the first copy takes, requested about now
+    if (lane == 0 && p.phase_cycles != nullptr && blockIdx.x == 0 && my_tiles > 0) {
+      const long long t0 = clock64();
+      mbar_wait(bar_full, 0, abort_flag, problem_of(p, pair_id).status, 0x112);
+      p.phase_cycles[10] = clock64() - t0;
     }
   } else if (warp == 9 || warp == 10) {
     // ------------------------------ features ------------------------------

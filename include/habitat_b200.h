@@ -266,9 +266,10 @@ hb_status hb_mlp_inject_mark(hb_mlp* handle);
  * for the most recent launch.  out[0..3] first epilogue group: waiting for its
  * output blocks, draining them, fc2, layers counted.  out[4..8] MMA issuer:
  * waiting for activations, for weights, for TMEM blocks to be read out, issuing,
- * ring slots counted.  out[9..11] first producer: waiting for a free slot and
- * requesting a copy, latency of the launch's first copy, copies counted.  out[12], out[13]: the MMA issuer's whole loop in SM
- * cycles and in nanoseconds (their ratio is the SM clock under load).
+ * ring slots (16 KB) counted.  out[9..11] first of three producers: waiting for a
+ * free slot and requesting a copy; the launch's first copy alone; copies counted.
+ * out[12], out[13]: the MMA issuer's whole loop in SM cycles and in nanoseconds
+ * (their ratio is the SM clock under load).
  * out[14], out[15] first epilogue group: hand-over of a drained block, stores
  * into the peer CTA.  Synchronises.  No reference counterpart. */
 hb_status hb_mlp_phase_cycles(hb_mlp* handle, int64_t out[16]);

@@ -573,6 +573,26 @@ def test_small_batches_on_ever_new_streams():
         h.close()
 
 
+def test_cycle_counters():
+    """The counters of the two-SM kernel's first cluster: slots and copies of whole tiles, a first copy of plausible
+    length, and the issuer's waits within its whole loop."""
+    w = workloads.init_mlp_weights("bmm", seed=2, layers=3, gain=2.0)
+    feats, dev = workloads.make_queries("bmm", 74 * 128 * 2, 9)
+    mu, sigma = workloads.batch_mu_sigma(feats, dev)
+    for precision, parts in (("bf16", 1), ("bf16x3", 2)):
+        h = batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=DEVF, precision=precision, **w)
+        Q = len(feats) // parts                                  # two rounds of tiles
+        h.predict(torch.from_numpy(feats[:Q]).cuda(), torch.from_numpy(dev[:Q]).cuda())
+        h.check_status()
+        c = h.phase_cycles()
+        slots = 2 * 3 * 64 * parts                               # (fc1's four are not counted)
+        assert c["slots"] == slots
+        assert 0 <= c["copies"] - (slots + 2 * 4) / 3 < 1        # one producer of three
+        assert 300 < c["producer_copy"] < c["mma_total_cycles"] / 4
+        assert 0 < c["mma_wait_act"] + c["mma_wait_weights"] + c["mma_wait_tmem"] < c["mma_total_cycles"]
+        h.close()
+
+
 def test_small_batches_switched_off():
     """HB_MLP_WIDE=0 keeps every batch on the two-SM kernel, which leaves its cycle counters; without it small batches
     from host memory leave none.  The predictions are the same."""
