@@ -29,8 +29,8 @@
 //
 // Precision modes: HB_PRECISION_BF16 rounds hidden activations and weights to bf16 (128
 // queries per tile); HB_PRECISION_BF16X3 keeps hi + lo parts of both (64 queries per tile,
-// the two parts of an activation side by side along N, the two parts of a weight tile in
-// one ring slot: see the comment at the kernel).
+// the two parts of an activation side by side along N, the two parts of a weight tile one
+// after the other in the ring: see the comment at the kernel).
 //
 // Warp roles: warp 0 = TMEM allocation, warp 1 = barrier set-up + MMA issuer (leader CTA),
 // warps 2-5 and 12-15 = two epilogue groups (one TMEM lane quadrant per warp), warps 6-8 =

@@ -1,6 +1,6 @@
 // MLP inference for batches that do not fill the GPU: the layers' features are spread over the SMs.
 //
-// mlp_chain.cu gives 128 queries to two SMs, which stream all 16.8 MB of weights past them: 118 us
+// mlp_chain.cu gives 128 queries to two SMs, which stream all 16.8 MB of weights past them: 103 to 110 us
 // whether the batch has one query or 9,472.  What bounds that is the weight stream of one SM pair, so
 // here G = 16, 8 or 4 thread blocks form a group that owns up to 64 queries (32 in split precision);
 // block c computes output features 1024 / G * c .. of every layer for all of the group's queries and
@@ -180,8 +180,9 @@ __device__ __forceinline__ uint32_t b_chunk(uint32_t k, uint32_t chunk) {
 // blocks (st.async, counted in bytes on the barrier of the buffer); two buffers alternate by layer, for the reason
 // given above.  An all-gather of 128 bytes per block takes 750 cycles, of 1 KB 1,500, of 2 KB 2,400 (about 14 bytes
 // a cycle), while the way through L2 moves whole rows of columns, filled or not: 1,140 cycles to the first K quarter and
-// 600 to each further one.  One query 23.6 -> 19.1 us, 14: 23.6 -> 20.5, 42: 23.9 -> 23.8, 56: 24.0 -> 25.5
-// (not taken); split, one 33.1 -> 28.9, 14: 33.4 -> 31.0, 28: 33.9 either way (not taken).
+// 600 to each further one.  At first one query 23.6 -> 19.1 us, 14: 23.6 -> 20.5, 42: 23.9 -> 23.8, 56: 24.0 -> 25.5
+// (not taken); split, one 33.1 -> 28.9, 14: 33.4 -> 31.0, 28: 33.9 either way (not taken).  Now 18.9, 20.2 and 23.3, split
+// 28.8 and 30.6.
 template <int G, int W, bool SPLIT, bool NEAR>
 __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(const __grid_constant__ WideParams p) {
   static_assert(!NEAR || (G == 16 && W == 16), "one K block of 64 features per block");
@@ -262,8 +263,9 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
   // (100 queries 25.1 -> 24.3 us, 900 48.2 -> 46.5, 2,000 75.1 -> 74.1).  A function that both roles call: as a step
   // before the roles part it made every layer 30 % slower.  In split precision, with half the queries, it gained
   // nothing and cost 1 to 2 % from 150 queries on: epilogue alone.
-  // So too in four blocks of 32 columns, which three batches that fill the GPU take: 636, 384 and 12 queries side by
-  // side in an iteration batch 68.0 -> 66.0 us, while 1,056 alone give back 47.9 -> 48.6 (48.9 before any of this).
+  // So too in four blocks of 32 columns, which batches that fill the GPU side by side take: shared, the features made 480,
+  // 480 and 6 queries 58.9 -> 61.0 us and an iteration batch with 636, 384 and 12 66.0 -> 68.0 (those three alone 50.0 ->
+  // 49.8), 960 beside 96, 1,000 beside 12 and 800 beside 200 the same within 0.2, 961 to 1,056 alone 47.9 -> 47.7.
   constexpr bool kAllFeatures = !SPLIT && !NEAR && !(G == 4 && W == 32);
   auto features = [&]() {
     constexpr int kThreads = kAllFeatures ? wide_threads<W, NEAR>() - 128 : 128;
@@ -854,9 +856,9 @@ namespace hb {
 // 33 of 16, 8 or 4 blocks.  Smaller groups hold more queries in all but stream more weights per block
 // (L2 and shared-memory fill bound), wider ones exchange more per layer (L2 latency and bandwidth); the
 // shapes below are those that no other one beats at its capacity.  Measured per launch, conv2d predictor,
-// 8 hidden layers (capacity in queries: time), against 118 us (bf16) and 195 us (split) of the two-SM kernel:
-//   bf16    42: 23 us (one: 19)   112: 24   240: 28   480: 32   960: 46   1,056: 47   2,112: 73
-//   split   21: 32 (one: 28)       56: 34   120: 42   240: 46             528: 77     1,056: 127
+// 8 hidden layers (capacity in queries: time), against 103 us (bf16) and 168 us (split) of one tile of the two-SM kernel:
+//   bf16    42: 23 us (one: 19)   112: 24   240: 28   480: 32   960: 46   1,056: 48   2,112: 73
+//   split   21: 32 (one: 29)       56: 34   120: 42   240: 46             528: 78     1,056: 126
 // Eight blocks x 64 columns lose to four x 32 in split precision (86 us for 480).  Beyond the last shape
 // the two-SM kernel of mlp_chain.cu is the faster one.
 namespace {

@@ -14,7 +14,8 @@ struct WidePlan {
   int G, W, groups, per_group;
   bool near;
 };
-// alone: no other batches of the call run beside it
+// alone: no other batch that this kernel takes runs beside it (queries beyond full rounds of mlp_chain.cu's tiles are
+// alone in this sense)
 WidePlan wide_plan(int64_t Q, bool split, int sm_count, bool alone);
 // Queries that can travel as kernel parameters: no copy and no read over PCIe for the scalar API.
 constexpr int kWideInline = 16;

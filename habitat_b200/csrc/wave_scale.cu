@@ -465,7 +465,10 @@ __device__ __forceinline__ uint32_t hb_checked(uint32_t idx, uint32_t limit, uin
 // a thread are then neighbours (GAP = 1), or (GAP = 32) so far apart that each of a warp's accesses is one piece
 // of 32 elements: with metrics, four arrays of which are loaded one element at a time in any case, that is 2 to 5 %
 // faster up to eight destinations (1,000,001 x 6: 33.6 -> 32.6 us, x 1: 14.9 -> 14.3; 4,000,001 x 6: 113.3 -> 111.5) and
-// 1 % slower with thirteen; without metrics the vector loads are worth more (1,000,001 x 6: 19.4 against 21.1).
+// 1 % slower with thirteen; without metrics the vector loads are worth more (1,000,001 x 6: 19.4 against 21.1).  The line
+// lies where middle batches change sides (every destination with a register count of its own: 1,000,001 x 8: 44.4 ->
+// 44.2, x 9: 48.6 -> 48.4, x 10: 52.1 -> 52.3, x 13: 63.7 -> 64.3); small ones gain beyond it too (250,001 x 8: 15.2 ->
+// 14.7, x 16: 24.4 -> 24.0), large ones lose below it already (4,000,001 x 6: 121.3 -> 121.8, x 8: 149.8 -> 150.9).
 template <typename T, int VEC, uint32_t GAP>
 __device__ __forceinline__ Vec<T, VEC> load_pair(const T* q, bool pair) {
   if (VEC == 1 || GAP == 0) return load_vec<T, VEC>(q);

@@ -435,8 +435,8 @@ def test_last_round_of_few_tiles(precision, round_q, most):
 @pytest.mark.parametrize("precision", ["bf16", "bf16x3"])
 @pytest.mark.parametrize("op", ["conv2d", "bmm"])
 def test_few_host_queries(op, precision):
-    """Up to 16 queries from host memory travel as kernel parameters, in split precision more than eight of them to
-    two groups: every count on both sides of that, each query different, has the bits of the device entry point."""
+    """Up to 16 queries from host memory travel as kernel parameters, to as many groups as there are (up to seven): every
+    count on both sides of that, each query different, has the bits of the device entry point."""
     feats, dev = workloads.make_queries(op, 64, 71)
     mu, sigma = workloads.batch_mu_sigma(feats, dev)
     h = batched.MLPHandle(feats.shape[1], mu=mu, sigma=sigma, device_features=DEVF, precision=precision,
