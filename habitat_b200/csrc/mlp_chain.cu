@@ -290,7 +290,7 @@ mlp_chain_pair_kernel(const __grid_constant__ MlpParams p) {
   } else if (warp == 1) {
     if (rank == 0) {
       // ------------------------------ MMA issuer (leader) -------------------
-      // One elected lane (elect.sync) runs the whole loop, and no loop depends on what a wait returns
+      // One elected lane (elect.sync) runs the whole loop, and no loop of a tile depends on what a wait returns
       // (after a wait that ran out the abort flag is set, and what is issued on stale operands is
       // discarded), which keeps the descriptors in uniform registers: four MMAs and their commit are
       // queued in about 100 cycles of the 256 they take.  The barrier of the next slot is tested while they run.

@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(wide_threads<W, NEAR>(), 1) mlp_wide_kernel(co
     // One elected lane runs the whole loop.  An MMA of these shapes takes 24 to 49 cycles and only a
     // couple of them queue up, so what stands between two MMAs shows: the wait for the next slot goes
     // between the MMAs of the current one, the commit that frees a slot behind the next slot's first
-    // MMAs, and every loop runs its full count whatever the waits say, so that the descriptors depend
+    // MMAs, and every loop of a layer runs its full count whatever the waits say, so that the descriptors depend
     // on uniform values alone (a wait that ran out has set the abort flag; what is issued after it reads
     // stale shared memory and is discarded).  16 MMAs of 64 x 16 took 1,150 cycles in the plain form.
     if (elect_one()) {
