@@ -313,6 +313,11 @@ class MLPHandle:
         such launch on this GPU reports an error instead of results."""
         _native.check(_native.load().hb_mlp_inject_mark(self._handle))
 
+    def inject_stale(self):
+        """Makes the next small-batch launch of each stream on this GPU take what its blocks exchange for stale (tests):
+        it runs the network once more, and the predictions are the same."""
+        _native.check(_native.load().hb_mlp_inject_stale(self._handle))
+
     def phase_cycles(self):
         """Cycle counters of the first cluster in the last launch of the two-SM kernel (synchronises): epilogue
         group 0 (wait, epilogue, fc2, layers, epi_publish, epi_remote), the MMA issuer (mma_wait_act,

@@ -18,7 +18,7 @@ LIB_PATH = os.path.join(LIB_DIR, "libhabitat_b200.so")
 BINDING_PATH = os.path.join(LIB_DIR, "_binding.so")
 
 SOURCES = ["hb_error.cu", "wave_scale.cu", "reduce.cu", "peer_exchange.cu", "mlp_chain.cu", "mlp_wide.cu",
-           "device_probe.cu"]
+           "mlp_pairs.cu", "device_probe.cu"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

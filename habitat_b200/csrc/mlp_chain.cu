@@ -45,6 +45,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "mlp_common.cuh"
@@ -739,6 +740,41 @@ void put(uint8_t* tile, int row, int col, uint16_t v) {
 
 }  // namespace
 
+namespace {
+// A tensor map of unswizzled bytes; dims, strides and box as cuTensorMapEncodeTiled takes them.
+cudaError_t encode_bytes(CUtensorMap* map, void* base, uint32_t rank, const cuuint64_t* dims, const cuuint64_t* strides,
+                         const cuuint32_t* box) {
+  using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                                CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
+                                CUtensorMapFloatOOBfill);
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult found;
+  const cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found);
+  if (e != cudaSuccess) return e;
+  if (fn == nullptr || found != cudaDriverEntryPointSuccess) return cudaErrorNotSupported;
+  const cuuint32_t elem[3] = {1, 1, 1};
+  return reinterpret_cast<EncodeFn>(fn)(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, rank, base, dims, strides, box, elem,
+                                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+             ? cudaSuccess
+             : cudaErrorInvalidValue;
+}
+}  // namespace
+
+cudaError_t hb::encode_rows(CUtensorMap* map, void* base, uint32_t row_bytes, uint64_t rows, uint32_t box_rows) {
+  const cuuint64_t dims[2] = {row_bytes, rows}, strides[1] = {row_bytes};
+  const cuuint32_t box[2] = {row_bytes, box_rows};
+  return encode_bytes(map, base, 2, dims, strides, box);
+}
+
+cudaError_t hb::encode_images(CUtensorMap* map, void* base, uint64_t rows, uint32_t box_rows, uint32_t box_images) {
+  const cuuint64_t dims[3] = {128, kTileBytes / 128, rows / (kTileBytes / 128)}, strides[2] = {128, kTileBytes};
+  const cuuint32_t box[3] = {128, box_rows, box_images};
+  return encode_bytes(map, base, 3, dims, strides, box);
+}
+
 extern "C" void hb_mlp_destroy(hb_mlp* h) {
   if (!h) return;
   if (h->counted) hb::wide_handle_destroyed(h->device);
@@ -855,54 +891,13 @@ extern "C" hb_status hb_mlp_create(hb_mlp** handle, int32_t n_op_features, int32
   HB_UP(sigma, sigma, sizeof(double) * C_in);
   HB_UP(dev_feat, device_features, sizeof(double) * 4 * n_device_rows);
 #undef HB_UP
-  {
-    // The pack as a 2-D tensor of 128-byte rows for the tiled TMA loads of the pair kernel.  The
-    // tile images are stored already swizzled, so the maps use no swizzle of their own.
-    using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if ((e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres)) != cudaSuccess)
-      return fail(e, "cudaGetDriverEntryPoint(cuTensorMapEncodeTiled)");
-    if (fn == nullptr || qres != cudaDriverEntryPointSuccess) {
-      hb::set_error("hb_mlp_create: the driver does not export cuTensorMapEncodeTiled");
-      hb_mlp_destroy(h);
-      return HB_ERR_CUDA;
-    }
-    const cuuint64_t dims[2] = {128, static_cast<cuuint64_t>(pack.size() / 128)};
-    const cuuint64_t strides[1] = {128};
-    const cuuint32_t elem[2] = {1, 1};
-    for (int which = 0; which < 2; ++which) {
-      const cuuint32_t box[2] = {128, static_cast<cuuint32_t>((which == 0 ? 2 : 1) * kTileBytes / 128)};
-      const CUresult r = reinterpret_cast<EncodeFn>(fn)(
-          which == 0 ? &h->tmap_slot : &h->tmap_tile, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, h->wpack, dims, strides,
-          box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r != CUDA_SUCCESS) {
-        hb::set_error("hb_mlp_create: cuTensorMapEncodeTiled failed (CUresult %d)", static_cast<int>(r));
-        hb_mlp_destroy(h);
-        return HB_ERR_CUDA;
-      }
-    }
-    // the same rows by tile image, for blocks that take half of an image's rows (mlp_wide.cu)
-    const cuuint64_t dims3[3] = {128, 128, static_cast<cuuint64_t>(pack.size() / kTileBytes)};
-    const cuuint64_t strides3[2] = {128, kTileBytes};
-    const cuuint32_t elem3[3] = {1, 1, 1};
-    for (int which = 0; which < 2; ++which) {
-      const cuuint32_t box3[3] = {128, 64, which == 0 ? 4u : 1u};
-      const CUresult r = reinterpret_cast<EncodeFn>(fn)(
-          which == 0 ? &h->tmap_wide_slot : &h->tmap_wide_fc1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, h->wpack, dims3,
-          strides3, box3, elem3, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r != CUDA_SUCCESS) {
-        hb::set_error("hb_mlp_create: cuTensorMapEncodeTiled failed (CUresult %d)", static_cast<int>(r));
-        hb_mlp_destroy(h);
-        return HB_ERR_CUDA;
-      }
-    }
-  }
+  // The pack as rows of 128 bytes for the tiled TMA loads.  The tile images are stored already swizzled, so the maps use
+  // no swizzle of their own.
+  const uint64_t pack_rows = pack.size() / 128;
+  if ((e = hb::encode_rows(&h->tmap_tile, h->wpack, 128, pack_rows, kTileBytes / 128)) != cudaSuccess ||
+      (e = hb::encode_images(&h->tmap_slot, h->wpack, pack_rows, 64, 4)) != cudaSuccess ||
+      (e = hb::encode_images(&h->tmap_half_tile, h->wpack, pack_rows, 64, 1)) != cudaSuccess)
+    return fail(e, "cuTensorMapEncodeTiled");
   if ((e = cudaHostAlloc(reinterpret_cast<void**>(&h->status), sizeof(int32_t), cudaHostAllocDefault)) != cudaSuccess)
     return fail(e, "cudaHostAlloc status");
   *h->status = 0;
@@ -1083,7 +1078,15 @@ extern "C" hb_status hb_mlp_predict_grid(const hb_mlp_grid* items, int32_t n_ite
   }
   if (some == 0) return HB_OK;
   const auto queue = hb::wide_queue(items[order[0]].handle->device);   // the current device, as are the others'
-  if (all_wide && some > 1) hb::wide_plans_together(plans, sizes, split, some, items[order[0]].handle->sm_count);
+  if (all_wide && some > 1) {
+    hb::wide_plans_together(plans, sizes, split, some, items[order[0]].handle->sm_count);
+    // large clusters first: small ones spread over all GPCs and would leave no room for them
+    for (int i = 1; i < some; ++i)
+      for (int j = i; j > 0 && plans[j].G > plans[j - 1].G; --j) {
+        std::swap(plans[j], plans[j - 1]);
+        std::swap(order[j], order[j - 1]);
+      }
+  }
   int lane = 0;
   for (int k = 0; k < some; ++k) {
     const int i = order[k];
@@ -1163,6 +1166,15 @@ extern "C" hb_status hb_mlp_inject_mark(hb_mlp* h) {
   }
   const hb_status st = check_device(h);
   return st != HB_OK ? st : hb::wide_set_mark(h->device);
+}
+
+extern "C" hb_status hb_mlp_inject_stale(hb_mlp* h) {
+  if (!h) {
+    hb::set_error("hb_mlp_inject_stale: NULL handle");
+    return HB_ERR_INVALID_ARGUMENT;
+  }
+  hb::wide_expect_stale(h->device);
+  return HB_OK;
 }
 
 extern "C" hb_status hb_mlp_phase_cycles(hb_mlp* h, int64_t out[16]) {

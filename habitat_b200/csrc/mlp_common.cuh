@@ -353,8 +353,8 @@ struct hb_mlp {
   int32_t n_op_feat = 0, layers = 0, precision = 0, n_dev = 0, sm_count = 0, device = 0;
   float fc2_b = 0.f;
   uint8_t* wpack = nullptr;
-  CUtensorMap tmap_slot{}, tmap_tile{};            // two tile images, one tile image
-  CUtensorMap tmap_wide_slot{}, tmap_wide_fc1{};   // 64 rows of four consecutive tile images, of one
+  CUtensorMap tmap_tile{};                         // one tile image
+  CUtensorMap tmap_slot{}, tmap_half_tile{};       // 64 rows of four consecutive tile images, of one
   float* bias = nullptr;
   float* fc2_w = nullptr;
   double* mu = nullptr;

@@ -1,5 +1,7 @@
-// Host interface of the kernel for batches that do not fill the GPU (mlp_wide.cu).
+// Host interface of the kernels for batches that do not fill the GPU (mlp_wide.cu, mlp_pairs.cu).
 #pragma once
+
+#include <cuda.h>
 
 #include <mutex>
 
@@ -8,8 +10,12 @@
 struct hb_mlp;
 
 namespace hb {
-// G blocks per group (0: not for this batch), W columns per group, groups, queries per group; near: the exchange
-// goes through distributed shared memory.
+// Tensor maps of unswizzled bytes: a box of `box_rows` rows of `row_bytes`; a box of `box_rows` rows, at most 128, of
+// `box_images` consecutive 16 KB images of 128-byte rows.
+cudaError_t encode_rows(CUtensorMap* map, void* base, uint32_t row_bytes, uint64_t rows, uint32_t box_rows);
+cudaError_t encode_images(CUtensorMap* map, void* base, uint64_t rows, uint32_t box_rows, uint32_t box_images);
+// G blocks per group (0: not for this batch), W columns (mlp_pairs.cu: per CTA), groups, queries per group; near: the
+// exchange goes through distributed shared memory.
 struct WidePlan {
   int G, W, groups, per_group;
   bool near;
@@ -50,6 +56,8 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
 void wide_start_over(int device);
 // Leaves the mark of a launch that gave up in the GPU's scratch (tests of the error path); synchronises.
 hb_status wide_set_mark(int device);
+// The next launch on each stream of the GPU that tries to do without releases takes what it exchanges for stale (tests).
+void wide_expect_stale(int device);
 void wide_handle_created(int device);
 void wide_handle_destroyed(int device);
 }  // namespace hb

@@ -262,6 +262,11 @@ hb_status hb_mlp_inject_status(hb_mlp* handle, int32_t device_status);
  * Synchronises.  No reference counterpart. */
 hb_status hb_mlp_inject_mark(hb_mlp* handle);
 
+/* The next small-batch launch on each stream that has had one, on the handle's GPU, takes what its
+ * blocks exchange for stale and runs the network once more, the slower way (test hook; the
+ * predictions are the same).  No reference counterpart. */
+hb_status hb_mlp_inject_stale(hb_mlp* handle);
+
 /* Profiling aid (bf16 kernel): SM cycle counters of the first cluster's leader CTA
  * for the most recent launch.  out[0..3] first epilogue group: waiting for its
  * output blocks, draining them, fc2, layers counted.  out[4..8] MMA issuer:

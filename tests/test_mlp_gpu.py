@@ -623,3 +623,30 @@ print(want.tobytes().hex()[:200])
         assert r.returncode == 0, r.stderr
         outs.append(r.stdout)
     assert outs[0] == outs[1]
+
+
+@pytest.mark.parametrize("precision,edges", [("bf16", (28, 224, 448, 960, 1920, 4224)),
+                                             ("bf16x3", (14, 112, 224, 480, 960, 2112))])
+@pytest.mark.parametrize("layers", [1, 2, 3, 8])
+def test_clusters_of_pairs(precision, edges, layers):
+    """Each shape of the kernel for clusters of SM pairs at both ends of its range, with groups that are not
+    full and halves of different lengths, and the size past the last shape: each prediction has the bits it has in a full
+    round of the two-SM kernel's tiles (two buffers alternate by layer, so odd and even numbers of layers).  Once with
+    what the blocks exchange taken for stale, so that the network runs a second time, and as usual after that."""
+    n = 9472 if precision == "bf16" else 4736
+    w = workloads.init_mlp_weights("conv2d", seed=37, gain=2.0, layers=layers)
+    feats, dev = workloads.make_queries("conv2d", n, 59)
+    mu, sigma = workloads.batch_mu_sigma(feats, dev)
+    h = batched.MLPHandle(feats.shape[1], mu=mu, sigma=sigma, device_features=DEVF, precision=precision, **w)
+    f, r = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()
+    full = h.predict(f, r)
+    for e in edges:
+        for Q in (e, e + 1, e - 1, e - 13):
+            lo = (17 * Q) % (n - Q)
+            for turn in range(4):
+                if turn == 1:
+                    h.inject_stale()
+                got = h.predict(f[lo:lo + Q].contiguous(), r[lo:lo + Q].contiguous())
+                assert torch.equal(got, full[lo:lo + Q]), (Q, turn)
+    h.check_status()
+    h.close()
