@@ -40,11 +40,12 @@ constexpr int kNearM = 64;                            // weight rows per block
 constexpr int kNearThreads = 256;
 constexpr int kNearQ = 4;                             // queries per group at most; split: half as many
 constexpr int kNearActBytes = 2 * 2048 * kNearCols;   // two buffers
-// Ring of weights.
+// Ring of weights.  bf16: few slots, each wait holds up the issue of MMAs for 90 cycles (one query 18.9 -> 17.8 us against five
+// of 32 KB); a layer in split precision does not fit, and there two large ones are refilled too late (28.9 -> 34.7).
 template <bool SPLIT>
-constexpr int kNearSlots = 5;
+constexpr int kNearSlots = SPLIT ? 5 : 2;
 template <bool SPLIT>
-constexpr int kNearSlotBytes = 2 * kTileBytes;
+constexpr int kNearSlotBytes = (SPLIT ? 2 : 4) * kTileBytes;
 template <bool SPLIT>
 constexpr int kNearSmem = kNearActBytes + kNearSlots<SPLIT> * kNearSlotBytes<SPLIT> + 1024 + 512;
 static_assert(kNearSmem<false> <= 232448 && kNearSmem<true> <= 232448, "shared memory");
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
             tma_3d(ring + s * kSlotBytes, &p.map_fc1, row, image0, full);
           } else {   // four images each
             tma_3d(ring + s * kSlotBytes, &p.map_slot, row, image0 + g * kUnitsPerSlot, full);
+            if (!SPLIT) tma_3d(ring + s * kSlotBytes + kSlotBytes / 2, &p.map_slot, row, image0 + g * kUnitsPerSlot + 4, full);
           }
           ++issued;
           ring_next<kSlots>(s, ph);
@@ -518,7 +520,7 @@ namespace hb {
 // 33 of 16, 8 or 4 blocks.  Smaller clusters hold more queries in all but stream more weights per block, wider ones
 // exchange more per layer.  Measured per launch, conv2d predictor, 8 hidden layers (capacity in queries: us), against 103 us
 // (bf16) and 168 us (split) of one tile of mlp_chain.cu's kernel, which is the faster one beyond the last shape:
-//   near               28: 21 (one: 18.9)      split    14: 29.6 (one: 27.8)
+//   near               28: 19.6 (one: 17.8)   split    14: 29.6 (one: 27.8)
 //   8 pairs x 16      224: 25.4 (one: 22.7)           112: 33.0 (one: 30.2)
 //   8 pairs x 32      448: 27.3                       224: 36.4
 //   4 pairs x 32      960: 35.2                       480: 49.5
