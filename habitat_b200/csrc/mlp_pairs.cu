@@ -6,7 +6,7 @@
 // weights, and after each layer the cluster exchanges its activations.
 //
 // Formulation as in mlp_chain.cu, H^T = W . X^T with tcgen05.mma.cta_group::2: A = weight rows, half of them in each CTA
-// of the pair (P = 8: M = 128, else 256), B = activations, N = 2 NC columns, half of them in each CTA (MN-major, rows of 2 NC
+// of the pair (M = 128 or 256), B = activations, N = 2 NC columns, half of them in each CTA (MN-major, rows of 2 NC
 // bytes), D = fp32 in TMEM.  Each CTA keeps, and each exchange moves, the activations of one half of the
 // queries only: blocks that share no MMAs move twice as much for the same number.
 // K is walked in the same order and fc2 adds in the same order as in mlp_chain.cu, so all kernels give the same bits
@@ -32,15 +32,16 @@
 // (448 queries: 27.3 us so, 26.5 if nobody looked; with releases 32; by ordinary loads that poll the data in L2, 32 bytes a
 // cycle, 34; bulk copies that are looked at before they are used 30.  With NC = 64 looking takes as long as releasing.)
 //
-// P = 2: a pair's 512 features are two row blocks, of K quarters i and 2 + i.  The units (block b, K quarter q) of a layer
-// are issued in the order (0,0) (0,1) (1,0) (0,2) (0,3) | (1,1) (1,2) (1,3): quarters 0 and 1 are exchanged under the last
-// three units and quarters 2 and 3 under the first three of the next layer.  D alternates between two sets of TMEM columns.
+// NC = 64: a pair's features are two row blocks, one in K quarters 0 and 1 and one in 2 and 3.  The units (block b, K quarter
+// q) of a layer are issued in the order (0,0) (0,1) (1,0) (0,2) (0,3) | (1,1) (1,2) (1,3): quarters 0 and 1 are
+// exchanged under the last three units and quarters 2 and 3 under the first three of the next layer.  D alternates between two
+// sets of TMEM columns.
 //
-// What bounds it: P = 8 the latency of one exchange per layer (2,300 to 2,700 cycles from the last MMA to the next layer's first,
-// of which 300 to 500 until the accumulators are there, 350 to take them and write them out, 400 for the store, 400 for the
-// arrivals, 700 for the loads) next to 1,500 of MMAs; P = 2, 4 shared memory besides: a CTA's weights are written and read
-// once per layer, B is read once per row block, and the exchange writes it, 1.5 MB a layer and CTA for P = 2, NC = 64 at
-// 128 bytes a cycle.
+// What bounds it: NC = 16, 32 the latency of one exchange per layer (P = 8: 2,300 to 2,700 cycles from the last MMA to the next
+// layer's first, of which 300 to 500 until the accumulators are there, 350 to take them and write them out, 400 for the
+// store, 400 for the arrivals, 700 for the loads) next to 1,500 of MMAs; NC = 64 shared memory besides: a CTA's weights are
+// written and read once per layer, B is read once per row block, and the exchange writes it, 1.5 MB a layer and CTA for P = 2
+// and 1 MB for P = 4 at 128 bytes a cycle, and what the order of units leaves of the exchange.
 //
 // The blocks of a cluster are scheduled as a whole: that is what makes waiting for one another safe, and a launch may
 // have more clusters than fit at a time.
@@ -54,7 +55,7 @@
 
 namespace {
 
-// P = 2: the units of a layer, four bits each (4 b + q), first unit in the low bits
+// Two row blocks: the units of a layer, four bits each (4 b + q), first unit in the low bits
 constexpr uint32_t kQuadOrder = 0x76532410u;
 constexpr uint32_t kQuadFirstOfQuarter = 0x1Bu;   // units that read a K quarter for the first time
 constexpr uint32_t kQuadLastOfQuarter1 = 5;       // the one that reads quarter 1 for the last time
@@ -62,29 +63,31 @@ constexpr uint32_t kQuadLastOfQuarter1 = 5;       // the one that reads quarter 
 template <int P, int NC, bool SPLIT>
 struct PairShape {
   static constexpr int kCtas = 2 * P;
-  static constexpr int kBlocks = P == 2 ? 2 : 1;           // row blocks per pair
-  static constexpr int kRows = P == 8 ? 64 : 128;          // A rows per CTA and block
+  static constexpr int kBlocks = NC == 64 ? 2 : 1;         // row blocks per pair
+  static constexpr int kRows = 512 / P / kBlocks;          // A rows per CTA and block
+  static constexpr bool kNarrow = kRows == 64;             // M = 128: D's second half of the columns is in TMEM lanes 64 and up
   static constexpr int kN = 2 * NC;
   static constexpr int kHalfQ = SPLIT ? NC / 2 : NC;       // queries per CTA at most
   static constexpr int kRowBytes = 2 * NC;
   static constexpr int kActBytes = kWidth * kRowBytes;
-  static constexpr int kSlots = P == 8 ? 4 : (NC == 64 ? 6 : 8);
-  static constexpr int kSlotBytes = P == 8 ? 2 * kTileBytes : kTileBytes;
+  static constexpr int kSlotBytes = kNarrow ? 2 * kTileBytes : kTileBytes;
+  static constexpr int kSlots = (NC == 64 ? 6 : 8) * kTileBytes / kSlotBytes;
   static constexpr int kUnitBytes = kRows * 128;           // one K block of the rows
   static constexpr int kImages = kSlotBytes / kUnitBytes;  // per slot
   static constexpr int kParts = SPLIT ? 2 : 1;             // images per packed K block
   static constexpr int kUnits = 4 * kBlocks;               // (block, K quarter) per layer
   static constexpr int kUnitSlots = 4 * kParts / kImages;
   // A K quarter of the activations is counted on the barrier of the slot that it is used with.
-  static constexpr bool kJoint = P == 8 && !SPLIT;
-  static constexpr bool kTry = P != 2 && NC < 64;          // see above
+  static constexpr bool kTry = kBlocks == 1;               // see above
+  static constexpr bool kJoint = kTry && kNarrow && !SPLIT;
   static constexpr int kColGroups = NC == 64 ? 2 : 1;      // epilogue warps that share 32 rows
-  static constexpr int kEpiWarps = (P == 8 ? 4 : 8) * kColGroups;
-  static constexpr int kStores = P == 8 ? 4 : 8;           // bulk stores per block and CTA
+  static constexpr int kEpiWarps = (kNarrow ? 4 : 8) * kColGroups;
+  static constexpr int kStores = kNarrow ? 4 : 8;          // bulk stores per block and CTA
   static constexpr int kLookWarps = kTry ? 8 : 0;          // those that look at what has come
   static constexpr int kThreads = 128 + 32 * (kEpiWarps + kLookWarps);
-  static constexpr uint32_t kTmemCols = P == 2 ? 4 * kN : (P == 8 ? 32 : kN);
-  static_assert(P == 8 ? NC <= 32 : NC >= 32, "shapes");
+  static constexpr int kDCols = kNarrow ? NC : kN;          // TMEM columns of a block
+  static constexpr uint32_t kTmemCols = kBlocks == 2 ? 4 * kDCols : (kDCols < 32 ? 32 : kDCols);
+  static_assert(kRows == 64 || kRows == 128, "shapes");
   static_assert(!kJoint || (kUnitSlots == 1 && kSlots == kUnits), "a slot per quarter, each its own");
   static constexpr int kStageBytes = kTry ? 2 * kRows * kRowBytes : 0;   // this CTA's rows on their way out
   static constexpr int kSmem = kActBytes + kSlots * kSlotBytes + kStageBytes + 1024 + 1024;
@@ -156,7 +159,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
   const uint32_t bar_acc = bars + 192;      // [kBlocks] row block accumulated
   const uint32_t bar_stored = bars + 208;   // [kBlocks] this CTA's rows of the block are in global memory
   const uint32_t bar_feat = bars + 224;     // leader only: fc1's input in place in both CTAs
-  const uint32_t bar_q1 = bars + 232;       // P = 2: quarter 1 has been read
+  const uint32_t bar_q1 = bars + 232;       // two blocks: quarter 1 has been read
   const uint32_t bar_seen = bars + 240;     // kTry: the layer's input has been looked at
   const uint32_t bar_drain = bars + 248;    // leader only, after giving up: the MMAs have ended
   const uint32_t bar_out = bars + 256;      // kTry: the layer's output is on its way (kEpiWarps)
@@ -213,7 +216,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
   const int n_q = r ? in_group - first_half : first_half;
   constexpr uint32_t kHalfBytes = S::kActBytes;
   // first output feature of the pair's row block b, as a K index of the next layer
-  auto block_feature = [&](int b) { return P == 2 ? (2 * b + pair) * 256 : pair * (2 * S::kRows); };
+  auto block_feature = [&](int b) { return b * 512 + pair * (2 * S::kRows); };
   auto saw_stale = [&] {
     for (uint32_t c = 0; c < S::kCtas; ++c) st_cluster_u32(map_to_cta(bars + 296, c), 1u);
     __threadfence();
@@ -246,16 +249,16 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
           const int u = L - 1, buf = u & 1;
 #pragma unroll 1
           for (int q = 0; q < 4; ++q) {
-            if (q == 0 || (P == 2 && q == 2)) {
+            if (q == 0 || (S::kBlocks == 2 && q == 2)) {
               // the buffer has been read, this CTA's rows copied from it (kTry: they are not in it), and it has been looked at;
               // then the rows of all CTAs
-              const int b = P == 2 ? q >> 1 : 0;
+              const int b = S::kBlocks == 2 ? q >> 1 : 0;
               ok = S::kTry ? pairs_wait(bar_acc, u & 1, abort_flag, p, 0x531)
                              : pairs_wait(bar_stored + 8 * b, u & 1, abort_flag, p, 0x531);
               if (!sure && u > 0) ok = ok && pairs_wait(bar_seen, (u - 1) & 1, abort_flag, p, 0x534);
               ok = ok && pairs_wait(bar_sig + 8 * (buf * S::kBlocks + b), (u >> 1) & 1, abort_flag, p, 0x532);
               asm volatile("fence.proxy.async.global;" ::: "memory");
-            } else if (P == 2 && q == 1 && u > 0) {
+            } else if (S::kBlocks == 2 && q == 1 && u > 0) {
               ok = pairs_wait(bar_q1, (u - 1) & 1, abort_flag, p, 0x533);
             }
             if (!ok) break;
@@ -277,7 +280,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
           const uint32_t m = n - S::kBlocks, L = m / kLayerLoads, u = m % kLayerLoads / S::kUnitSlots, g = m % S::kUnitSlots;
           const uint32_t unit = S::kBlocks == 2 ? (kQuadOrder >> (4 * u)) & 15u : u, kq = unit & 3u;
           const uint32_t b = fc1 ? n : unit >> 2;
-          const uint32_t mt = P == 8 ? pair : static_cast<uint32_t>(block_feature(b)) / kMTile + r;
+          const uint32_t mt = static_cast<uint32_t>(block_feature(b)) / kMTile + (S::kNarrow ? 0u : r);
           const uint32_t image =
               fc1 ? S::kParts * mt
                   : S::kParts * (kNumMT + (L * kNumMT + mt) * kNumKB + kq * 4) + g * S::kImages;
@@ -286,7 +289,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
           if (!pairs_wait(bar_empty + 8 * s, ph, abort_flag, p, 0x511)) break;
           if (r == 0) mbar_expect_tx(full, 2 * (fc1 ? S::kUnitBytes : S::kSlotBytes));
           if (S::kJoint && r == 0 && fc1) mbar_arrive(full);
-          if (P == 8) tma_3d_pair(dst, fc1 ? &p.map_fc1 : &p.map_slot, r * S::kRows, image, full_leader);
+          if (S::kNarrow) tma_3d_pair(dst, fc1 ? &p.map_fc1 : &p.map_slot, r * S::kRows, image, full_leader);
           else tma_2d_pair(dst, &p.map_slot, image * kMTile, full_leader);
         }
         st_cluster_u32(map_to_cta(bars + 304 + 4 * (2 * r + w), leader), 1u);
@@ -329,7 +332,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
 #pragma unroll 1
         for (int b = 0; b < S::kBlocks; ++b) {                     // fc1: one K block
           wait(bar_full + 8 * s, ph, 0x522);
-          const uint32_t d = tmem_base + static_cast<uint32_t>(b * S::kN);
+          const uint32_t d = tmem_base + static_cast<uint32_t>(b * S::kDCols);
           const uint32_t a_lo = a_lo0 + s * (S::kSlotBytes >> 4);
 #pragma unroll
           for (int k = 0; k < 4; ++k)
@@ -348,7 +351,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
             const uint32_t unit = S::kBlocks == 2 ? (kQuadOrder >> (4 * u)) & 15u : u, b = unit >> 2, kq = unit & 3u;
             if (!S::kJoint && (S::kBlocks == 1 || (kQuadFirstOfQuarter >> u) & 1u))
               wait(bar_actq + 8 * kq, (L - 1) & 1, 0x523);
-            const uint32_t d = tmem_base + (S::kBlocks == 2 ? ((L & 1) * 2 + b) * S::kN : 0u);
+            const uint32_t d = tmem_base + (S::kBlocks == 2 ? ((L & 1) * 2 + b) * S::kDCols : 0u);
 #pragma unroll
             for (uint32_t g = 0; g < S::kUnitSlots; ++g) {
               uint32_t next = s, next_ph = ph;
@@ -430,20 +433,19 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         }
         __syncwarp();
       }
-      // A warp drains 32 rows (features) of one half of the columns, or a part of them (kColGroups).  M = 128 keeps D's
-      // second half of the columns in TMEM lanes 64 and up (64 rows per CTA), M = 256 has 128 rows.  Split precision: a
+      // A warp drains 32 rows (features) of one half of the columns, or a part of them (kColGroups).  Split precision: a
       // query has two columns, of the lo and the hi part of its activations: one 32-bit word in a row of B.
       const int quad = warp & 3, rest = (warp - 4) >> 2;
-      const uint32_t half = P == 8 ? quad >> 1 : rest & 1;
-      const int part = P == 8 ? rest : rest >> 1;
-      const int row0 = P == 8 ? (quad & 1) * 32 : quad * 32;
+      const uint32_t half = S::kNarrow ? quad >> 1 : rest & 1;
+      const int part = S::kNarrow ? rest : rest >> 1;
+      const int row0 = S::kNarrow ? (quad & 1) * 32 : quad * 32;
       constexpr int kPiece = S::kHalfQ / S::kColGroups;      // queries per warp
       constexpr int kCols = S::kParts * kPiece;
-      const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (P == 8 ? 0u : half * NC) +
+      const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (S::kNarrow ? 0u : half * NC) +
                               static_cast<uint32_t>(part * kCols);
       unsigned long long* const group_halves = p.halves + static_cast<size_t>(group) * 64 * hb::kGroupCols;
       auto rows_sync = [&] {   // the warps of these rows
-        if (S::kColGroups == 2) asm volatile("bar.sync %0, 64;" ::"r"(2 + quad + (P == 8 ? 0 : 4 * static_cast<int>(half))) : "memory");
+        if (S::kColGroups == 2) asm volatile("bar.sync %0, 64;" ::"r"(2 + quad + (S::kNarrow ? 0 : 4 * static_cast<int>(half))) : "memory");
         else __syncwarp();
       };
       bool ok = start;
@@ -463,13 +465,12 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
             ok = __shfl_sync(0xFFFFFFFFu, go ? 1 : 0, 0) != 0;
           }
           // where the rows are kept for the copy: in a place of their own, or the activation buffer, where it has been read
-          // (P = 2: quarter 2 b has) and is loaded over after they have been copied
-          const int at0 = S::kTry ? static_cast<int>(half) * S::kRows + row0
-                                  : (P == 2 ? b * 512 + static_cast<int>(half * 128) + row0 : (half == r ? f0 : f0 ^ 512));
+          // (quarter 2 b) and is loaded over after they have been copied
+          const int at0 = (S::kTry ? 0 : b * 512) + static_cast<int>(half) * S::kRows + row0;
           const uint32_t rows = S::kTry ? stage : act;
           if (ok) {
             tc_fence_after();
-            const uint32_t t_block = t_lane + (S::kBlocks == 2 ? static_cast<uint32_t>(((L & 1) * 2 + b) * S::kN) : 0u);
+            const uint32_t t_block = t_lane + (S::kBlocks == 2 ? static_cast<uint32_t>(((L & 1) * 2 + b) * S::kDCols) : 0u);
             float v[kPiece];
             if (SPLIT) {
               float d[kCols];

@@ -524,16 +524,16 @@ namespace hb {
 //   8 pairs x 16      224: 25.4 (one: 22.7)           112: 33.0 (one: 30.2)
 //   8 pairs x 32      448: 27.3                       224: 36.4
 //   4 pairs x 32      960: 35.2                       480: 49.5
-//   4 pairs x 64    1,920: 51.5                       960: 73.8
+//   4 pairs x 64    1,920: 49.2                       960: 62.2   (in one row block, exchanged at once, 51.5 and 73.6)
 //   2 pairs x 64    4,224: 68.7                     2,112: 103
 // Blocks without partners (M = 64 or 128 each, all queries of a group in every block; data polled in L2) took 24 for 112,
 // 28 for 240, 32 for 480, 46 for 960, 48 for 1,056 and 73 for 2,112 queries, split 34 for 56, 46 for 240, 78 for 528 and 126
-// for 1,056: better than these only from 100 to 112, 449 to 480 and 961 to 1,056 queries, by 3, 7 and 7 %.
+// for 1,056: better than these only from 100 to 112, 449 to 480 and 961 to 1,056 queries, by 3, 9 and 2 % (split: 225 to 240, 8 %).
 namespace {
 // us: what a launch of the shape takes, full or not
 struct Shape { int pairs, NC, clusters, us, us_split; };   // pairs 0: mlp_near_kernel
 constexpr Shape kShapes[] = {{0, 16, 7, 20, 30}, {8, 16, 7, 25, 33}, {8, 32, 7, 27, 36}, {4, 32, 15, 35, 49},
-                             {4, 64, 15, 51, 74}, {2, 64, 33, 69, 103}};
+                             {4, 64, 15, 49, 62}, {2, 64, 33, 69, 103}};
 int clusters_of(const Shape& s, int sm_count) { return sm_count >= 148 ? s.clusters : s.clusters * sm_count / 148; }
 int cols_of(const Shape& s, bool split) { return s.pairs == 0 ? (split ? kNearQ / 2 : kNearQ) : (split ? s.NC : 2 * s.NC); }
 WidePlan plan_in(const Shape& s, int64_t Q, bool split, int cols = 0) {
@@ -705,8 +705,9 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
   p.poison = reinterpret_cast<int32_t*>(s->base + kActsBytes + kHalvesBytes);
   s->tag = s->tag % 0x7FFFFFFFu + 1;   // the high bit is the second run's (mlp_pairs.cu)
   p.tag = s->tag;
-  p.map_slot = w.G == 16 ? h->tmap_slot : h->tmap_tile;
-  p.map_fc1 = w.G == 16 ? h->tmap_half_tile : h->tmap_tile;
+  const bool narrow = w.G == 16 || (w.G == 8 && w.W == 64);   // blocks of 64 weight rows
+  p.map_slot = narrow ? h->tmap_slot : h->tmap_tile;
+  p.map_fc1 = narrow ? h->tmap_half_tile : h->tmap_tile;
   bool fits = false;
   const cudaError_t e =
       !w.near ? launch_pairs(w.G / 2, w.W, split, p, w.groups, h->device, stream, &fits)
