@@ -18,9 +18,9 @@
 // store), waits until they are there and arrives at a barrier of each CTA that wants them; a CTA requests its K quarters (256
 // rows, one tiled load each) when all have arrived.  32 KB are there 730 cycles after the request, 128 KB after 1,540.
 //
-// The arrival is a release: one more round trip to L2, 1,300 cycles in each layer, 5.5 us of a launch.  Where the exchange
-// stands between the layers (P = 8, 4) and there is not much to look at (NC = 16, 32), the network is tried without (kTry).  The arrival is a relaxed one, what has
-// come is used at once, and other warps look at it afterwards, while the next layer's is on its way.  An activation is never
+// The arrival should be a release: one more round trip to L2, 1,300 to 2,300 cycles in each layer.  The network is tried
+// without first.  The arrival is a relaxed one, what has come is used at once, and warps look at it afterwards, while the
+// next layer's is on its way.  An activation is never
 // negative, so the high sign bit of every 32-bit word (two bf16 activations, or the lo and the hi part of one in
 // split precision) carries the parity of the buffer's use; with the parity 1 both halves are negated, and the instruction
 // negates B.  A word of an earlier use with the same parity cannot come: the use in between has been looked at in the
@@ -30,7 +30,8 @@
 // has read all of layer L - 1, which every CTA wrote after reading L - 2.  The host keeps the parity each group's buffers
 // have reached.
 // (448 queries: 27.3 us so, 26.5 if nobody looked; with releases 32; by ordinary loads that poll the data in L2, 32 bytes a
-// cycle, 34; bulk copies that are looked at before they are used 30.  With NC = 64 looking takes as long as releasing.)
+// cycle, 34; bulk copies that are looked at before they are used 30.  1,920 queries 45.6, with releases 49.2; 4,224 65.1 and
+// 68.2.)
 //
 // NC = 64: a pair's features are two row blocks, one in K quarters 0 and 1 and one in 2 and 3.  The units (block b, K quarter
 // q) of a layer are issued in the order (0,0) (0,1) (1,0) (0,2) (0,3) | (1,1) (1,2) (1,3): quarters 0 and 1 are
@@ -47,7 +48,7 @@
 // have more clusters than fit at a time.
 //
 // Warp roles: 0 TMEM, the mark, activation loads; 1 MMA issuer (the pair's leader); 2-3 weight producers; 4 and more:
-// epilogue; kTry: eight more that look at what has come.  Every wait is bounded, as in mlp_chain.cu; a launch that gave up leaves a mark in the scratch, and
+// epilogue; NC = 16, 32: eight more that look at what has come.  Every wait is bounded, as in mlp_chain.cu; a launch that gave up leaves a mark in the scratch, and
 // launches that find it report an error instead of a result.  After giving up no ring slot is requested again whose
 // copy could be under way: the MMA issuer, whose commits free the slots, waits for the producers of both CTAs to leave
 // before it issues anything past a wait that ran out, and goes no further than the layer's end.
@@ -78,18 +79,18 @@ struct PairShape {
   static constexpr int kUnits = 4 * kBlocks;               // (block, K quarter) per layer
   static constexpr int kUnitSlots = 4 * kParts / kImages;
   // A K quarter of the activations is counted on the barrier of the slot that it is used with.
-  static constexpr bool kTry = kBlocks == 1;               // see above
-  static constexpr bool kJoint = kTry && kNarrow && !SPLIT;
+  static constexpr bool kApart = kBlocks == 1;             // there is room for the rows on their way out
+  static constexpr bool kJoint = kApart && kNarrow && !SPLIT;
   static constexpr int kColGroups = NC == 64 ? 2 : 1;      // epilogue warps that share 32 rows
   static constexpr int kEpiWarps = (kNarrow ? 4 : 8) * kColGroups;
   static constexpr int kStores = kNarrow ? 4 : 8;          // bulk stores per block and CTA
-  static constexpr int kLookWarps = kTry ? 8 : 0;          // those that look at what has come
+  static constexpr int kLookWarps = kApart ? 8 : 0;        // those that look at what has come; else the epilogue's do
   static constexpr int kThreads = 128 + 32 * (kEpiWarps + kLookWarps);
   static constexpr int kDCols = kNarrow ? NC : kN;          // TMEM columns of a block
   static constexpr uint32_t kTmemCols = kBlocks == 2 ? 4 * kDCols : (kDCols < 32 ? 32 : kDCols);
   static_assert(kRows == 64 || kRows == 128, "shapes");
   static_assert(!kJoint || (kUnitSlots == 1 && kSlots == kUnits), "a slot per quarter, each its own");
-  static constexpr int kStageBytes = kTry ? 2 * kRows * kRowBytes : 0;   // this CTA's rows on their way out
+  static constexpr int kStageBytes = kApart ? 2 * kRows * kRowBytes : 0;   // this CTA's rows on their way out
   static constexpr int kSmem = kActBytes + kSlots * kSlotBytes + kStageBytes + 1024 + 1024;
   static_assert(kSmem <= 232448, "shared memory");
 };
@@ -160,9 +161,9 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
   const uint32_t bar_stored = bars + 208;   // [kBlocks] this CTA's rows of the block are in global memory
   const uint32_t bar_feat = bars + 224;     // leader only: fc1's input in place in both CTAs
   const uint32_t bar_q1 = bars + 232;       // two blocks: quarter 1 has been read
-  const uint32_t bar_seen = bars + 240;     // kTry: the layer's input has been looked at
+  const uint32_t bar_seen = bars + 240;     // first run: the layer's input has been looked at
   const uint32_t bar_drain = bars + 248;    // leader only, after giving up: the MMAs have ended
-  const uint32_t bar_out = bars + 256;      // kTry: the layer's output is on its way (kEpiWarps)
+  const uint32_t bar_out = bars + 256;      // kApart: the layer's output is on its way (kEpiWarps)
   constexpr int kBars = 33;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_ptr + 288);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + 292);
@@ -182,7 +183,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
     for (int i = 0; i < 2 * S::kBlocks; ++i) mbar_init(bar_sig + 8 * i, 32 / S::kBlocks);
     for (int b = 0; b < S::kBlocks; ++b) mbar_init(bar_stored + 8 * b, S::kStores);
     mbar_init(bar_feat, 2);
-    mbar_init(bar_seen, S::kTry ? S::kLookWarps : 1);
+    mbar_init(bar_seen, S::kApart ? S::kLookWarps : S::kEpiWarps);
     mbar_init(bar_out, S::kEpiWarps);
     for (int i = 0; i < 4; ++i) producers_left[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -224,9 +225,9 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
   constexpr uint32_t kSigns = SPLIT ? 0x80000000u : 0x80008000u;   // those that carry the parity
   float result = 0.0f;
 
-  // sure: with releases; the first run of kTry goes without
+  // sure: with releases; the first run goes without
 #pragma unroll 1
-  for (bool sure = !S::kTry;; sure = true) {
+  for (bool sure = false;; sure = true) {
     uint8_t* const group_acts = (sure ? p.sure_acts : p.acts) + static_cast<size_t>(group) * (4u * kHalfBytes);
     // both signs of the words of the `use`-th exchange
     auto signs_of = [&](int use) -> uint32_t {
@@ -250,12 +251,12 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
 #pragma unroll 1
           for (int q = 0; q < 4; ++q) {
             if (q == 0 || (S::kBlocks == 2 && q == 2)) {
-              // the buffer has been read, this CTA's rows copied from it (kTry: they are not in it), and it has been looked at;
+              // the buffer has been read, this CTA's rows copied from it (kApart: they are not in it), and it has been looked at;
               // then the rows of all CTAs
               const int b = S::kBlocks == 2 ? q >> 1 : 0;
-              ok = S::kTry ? pairs_wait(bar_acc, u & 1, abort_flag, p, 0x531)
+              ok = S::kApart ? pairs_wait(bar_acc, u & 1, abort_flag, p, 0x531)
                              : pairs_wait(bar_stored + 8 * b, u & 1, abort_flag, p, 0x531);
-              if (!sure && u > 0) ok = ok && pairs_wait(bar_seen, (u - 1) & 1, abort_flag, p, 0x534);
+              if (!sure && u > 0 && q == 0) ok = ok && pairs_wait(bar_seen, (u - 1) & 1, abort_flag, p, 0x534);
               ok = ok && pairs_wait(bar_sig + 8 * (buf * S::kBlocks + b), (u >> 1) & 1, abort_flag, p, 0x532);
               asm volatile("fence.proxy.async.global;" ::: "memory");
             } else if (S::kBlocks == 2 && q == 1 && u > 0) {
@@ -380,9 +381,9 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         }
       }
       __syncwarp();
-    } else if (S::kTry && warp >= 4 + S::kEpiWarps) {
+    } else if (S::kApart && warp >= 4 + S::kEpiWarps) {
       // ------------------------------ looking at what has been used ------------------------------
-      constexpr int kShare = S::kTry ? S::kActBytes / S::kLookWarps : 0, kBatch = 8;
+      constexpr int kShare = S::kApart ? S::kActBytes / S::kLookWarps : 0, kBatch = 8;
       const uint8_t* const mine = base_ptr + (warp - 4 - S::kEpiWarps) * kShare + 16 * lane;
 #pragma unroll 1
       for (int L = 0; L < n_layers && start && !sure; ++L) {
@@ -448,12 +449,29 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         if (S::kColGroups == 2) asm volatile("bar.sync %0, 64;" ::"r"(2 + quad + (S::kNarrow ? 0 : 4 * static_cast<int>(half))) : "memory");
         else __syncwarp();
       };
+      // This warp's share of the input, without the first `from` rows of quarters 0 and 2.
+      auto look = [&](uint32_t want, uint32_t from) {
+        constexpr uint32_t kStep = 4096;              // 32 rows
+        uint32_t bad = 0;
+#pragma unroll 1
+        for (uint32_t at = (warp - 4) * kStep; at < S::kActBytes; at += S::kEpiWarps * kStep) {
+          if ((at / S::kRowBytes & 511u) < from) continue;
+          uint4 x[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) x[k] = *reinterpret_cast<const uint4*>(base_ptr + at + 512 * k + 16 * lane);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) bad |= (x[k].x ^ want) | (x[k].y ^ want) | (x[k].z ^ want) | (x[k].w ^ want);
+        }
+        if (bad & kSigns) saw_stale();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_seen);
+      };
       bool ok = start;
       // a wait that ran out skips the work that is left but none of the barriers
 #pragma unroll 1
       for (int L = 0; L < n_layers; ++L) {
         const bool last = L == n_layers - 1;
-        const uint32_t signs = signs_of(L);
+        const uint32_t signs = signs_of(L), want = L > 0 ? signs_of(L - 1) ^ p.expect_stale : 0u;
 #pragma unroll 1
         for (int b = 0; b < S::kBlocks; ++b) {
           const int f0 = block_feature(b) + static_cast<int>(r) * S::kRows + row0, f = f0 + lane;
@@ -466,8 +484,8 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
           }
           // where the rows are kept for the copy: in a place of their own, or the activation buffer, where it has been read
           // (quarter 2 b) and is loaded over after they have been copied
-          const int at0 = (S::kTry ? 0 : b * 512) + static_cast<int>(half) * S::kRows + row0;
-          const uint32_t rows = S::kTry ? stage : act;
+          const int at0 = (S::kApart ? 0 : b * 512) + static_cast<int>(half) * S::kRows + row0;
+          const uint32_t rows = S::kApart ? stage : act;
           if (ok) {
             tc_fence_after();
             const uint32_t t_block = t_lane + (S::kBlocks == 2 ? static_cast<uint32_t>(((L & 1) * 2 + b) * S::kDCols) : 0u);
@@ -498,13 +516,20 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
                 }
                 w[i] = (w[i] & (SPLIT ? 0x7FFFFFFFu : 0x7FFF7FFFu)) ^ signs;
               }
+              uint32_t bad = 0;
 #pragma unroll
-              for (int c = 0; c < kWords / 4; ++c)
-                *reinterpret_cast<uint4*>(
+              for (int c = 0; c < kWords / 4; ++c) {
+                uint4* const to = reinterpret_cast<uint4*>(
                     base_ptr + (rows - base) +
-                    b_chunk<NC>(static_cast<uint32_t>(at0 + lane), static_cast<uint32_t>(part * (kWords / 4) + c))) =
-                    make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+                    b_chunk<NC>(static_cast<uint32_t>(at0 + lane), static_cast<uint32_t>(part * (kWords / 4) + c)));
+                if (!S::kApart && !sure && L > 0) {   // looked at before it goes
+                  const uint4 x = *to;
+                  bad |= (x.x ^ want) | (x.y ^ want) | (x.z ^ want) | (x.w ^ want);
+                }
+                *to = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+              }
               fence_proxy_async();
+              if (bad & kSigns) saw_stale();
             } else {
               constexpr int kFold = kPiece < 16 ? 16 : kPiece;
               float sum[kFold];
@@ -518,7 +543,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
                 st_relaxed_u64(h + i, static_cast<unsigned long long>(tag) << 32 | __float_as_uint(sum[i]));
             }
           }
-          if (S::kTry) {
+          if (S::kApart) {
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_out);
           }
@@ -540,7 +565,10 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
             }
             __syncwarp();
           }
+          // Block 0 has used all of the layer's input.  What the blocks' rows are not written over is looked at now.
+          if (!S::kApart && b == 0 && L > 0 && ok && !sure) look(want, 2 * S::kRows);
         }
+        if (!S::kApart && last && ok && !sure) look(want, 0);
       }
       if (cta < 2 && warp < 8) {
         // the first CTA of each half adds the 64 sets of 16 features of its queries

@@ -411,12 +411,12 @@ using hb::kMaxCudaDevices;
 // the first streams go without.  While none of the shared ones is out of use, a launch takes the two-SM kernel,
 // which needs no scratch.
 constexpr int kMaxStreams = 16, kMoreStreams = 16;
-constexpr int kMaxGroups = 37;
-// Activation buffers of mlp_pairs.cu: one per shape that exchanges by parity (a word's parity counts its own uses), and one
-// that all shapes use with releases.
-constexpr int kTryShapes = 3;                           // eight pairs, NC = 16 and 32; four pairs, NC = 32
+constexpr int kMaxGroups = 34;
+// Activation buffers of mlp_pairs.cu: one for the first runs of each shape (a word's parity counts its own uses), and one that
+// all shapes use for second runs.
+constexpr int kTryShapes = 5;                           // of kShapes, after the first
 constexpr size_t acts_bytes(int groups, int row_bytes) { return static_cast<size_t>(groups) * 4 * kWidth * row_bytes; }
-constexpr int kTryGroups[kTryShapes] = {8, 8, 16}, kTryRow[kTryShapes] = {32, 64, 64};
+constexpr int kTryGroups[kTryShapes] = {8, 8, 16, 16, kMaxGroups}, kTryRow[kTryShapes] = {32, 64, 64, 128, 128};
 constexpr size_t try_offset(int shape) { return shape ? try_offset(shape - 1) + acts_bytes(kTryGroups[shape - 1], kTryRow[shape - 1]) : 0; }
 constexpr size_t kSureOffset = try_offset(kTryShapes), kActsBytes = kSureOffset + acts_bytes(kMaxGroups, 128);
 constexpr size_t kHalvesBytes = static_cast<size_t>(kMaxGroups) * 64 * hb::kGroupCols * sizeof(unsigned long long);
@@ -524,16 +524,16 @@ namespace hb {
 //   8 pairs x 16      224: 25.4 (one: 22.7)           112: 33.0 (one: 30.2)
 //   8 pairs x 32      448: 27.3                       224: 36.4
 //   4 pairs x 32      960: 35.2                       480: 49.5
-//   4 pairs x 64    1,920: 49.2                       960: 62.2   (in one row block, exchanged at once, 51.5 and 73.6)
-//   2 pairs x 64    4,224: 68.7                     2,112: 103
+//   4 pairs x 64    1,920: 45.6                       960: 62.2   (in one row block, exchanged at once, 51.5 and 73.6)
+//   2 pairs x 64    4,224: 65.1                     2,112: 105
 // Blocks without partners (M = 64 or 128 each, all queries of a group in every block; data polled in L2) took 24 for 112,
 // 28 for 240, 32 for 480, 46 for 960, 48 for 1,056 and 73 for 2,112 queries, split 34 for 56, 46 for 240, 78 for 528 and 126
-// for 1,056: better than these only from 100 to 112, 449 to 480 and 961 to 1,056 queries, by 3, 9 and 2 % (split: 225 to 240, 8 %).
+// for 1,056: better than these only from 100 to 112 and 449 to 480 queries, by 3 and 9 % (split: 225 to 240, 8 %).
 namespace {
 // us: what a launch of the shape takes, full or not
 struct Shape { int pairs, NC, clusters, us, us_split; };   // pairs 0: mlp_near_kernel
 constexpr Shape kShapes[] = {{0, 16, 7, 20, 30}, {8, 16, 7, 25, 33}, {8, 32, 7, 27, 36}, {4, 32, 15, 35, 49},
-                             {4, 64, 15, 49, 62}, {2, 64, 33, 69, 103}};
+                             {4, 64, 15, 46, 62}, {2, 64, 33, 65, 105}};
 int clusters_of(const Shape& s, int sm_count) { return sm_count >= 148 ? s.clusters : s.clusters * sm_count / 148; }
 int cols_of(const Shape& s, bool split) { return s.pairs == 0 ? (split ? kNearQ / 2 : kNearQ) : (split ? s.NC : 2 * s.NC); }
 WidePlan plan_in(const Shape& s, int64_t Q, bool split, int cols = 0) {
@@ -685,20 +685,18 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
     s->fresh = false;
   }
   if (!w.near) {
+    const int i = w.W == 16 ? 0 : (w.G == 16 ? 1 : (w.G == 4 ? 4 : (w.W == 32 ? 2 : 3)));   // of the shapes with buffers
+    p.acts = s->base + try_offset(i);
+    p.map_acts = s->map_try[i];
     p.sure_acts = s->base + kSureOffset;
-    p.map_sure = s->map_sure[w.W == 16 ? 0 : (w.W == 32 ? 1 : 2)];
-    if (w.G > 4 && w.W < 64) {   // the others use releases only
-      const int i = w.W == 16 ? 0 : (w.G == 16 ? 1 : 2);
-      p.acts = s->base + try_offset(i);
-      p.map_acts = s->map_try[i];
-      p.expect_stale = s->expect_stale ? 0x80008000u : 0u;
-      s->expect_stale = false;
-      // exchange `use` (0 .. layers - 1) takes buffer use & 1; every group of the launch flips with it
-      const unsigned long long groups = (1ull << w.groups) - 1;
-      for (int b = 0; b < 2; ++b) {
-        p.parity[b] = s->parity[i][b];
-        if (((h->layers + 1 - b) / 2) & 1) s->parity[i][b] ^= groups;
-      }
+    p.map_sure = s->map_sure[w.W / 32];
+    p.expect_stale = s->expect_stale ? 0x80008000u : 0u;
+    s->expect_stale = false;
+    // exchange `use` (0 .. layers - 1) takes buffer use & 1; every group of the launch flips with it
+    const unsigned long long groups = (1ull << w.groups) - 1;
+    for (int b = 0; b < 2; ++b) {
+      p.parity[b] = s->parity[i][b];
+      if (((h->layers + 1 - b) / 2) & 1) s->parity[i][b] ^= groups;
     }
   }
   p.halves = reinterpret_cast<unsigned long long*>(s->base + kActsBytes);
