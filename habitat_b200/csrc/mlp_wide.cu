@@ -5,7 +5,7 @@
 // output features 64 c .. of every layer for them and streams only their weights.
 //
 // Formulation as in mlp_chain.cu, H^T = W . X^T with tcgen05.mma (cta_group::1): A = weight rows (M = 64), B =
-// activations (K-major, 16 columns), D = fp32 in TMEM.  K is walked in the same order and fc2 adds in the same order as
+// activations (K-major, 8 or 16 columns), D = fp32 in TMEM.  K is walked in the same order and fc2 adds in the same order as
 // there, so all kernels give the same bits and the choice of kernel never shows in a result.
 //
 // Exchange.  B is K-major, so that a block's share of a query is 128 contiguous bytes, which eight threads store into each
@@ -35,11 +35,14 @@
 namespace {
 
 constexpr int kNearBlocks = 16;                       // of a group
-constexpr int kNearCols = 16;                         // of B; split: hi and lo of eight queries
+// Columns of B: eight queries, split: their hi and their lo parts (with eight too many 14 queries took 19.1 instead of 18.7 us)
+template <bool SPLIT>
+constexpr int kNearCols = SPLIT ? 16 : 8;
 constexpr int kNearM = 64;                            // weight rows per block
 constexpr int kNearThreads = 256;
 constexpr int kNearQ = 4;                             // queries per group at most; split: half as many
-constexpr int kNearActBytes = 2 * 2048 * kNearCols;   // two buffers
+template <bool SPLIT>
+constexpr int kNearActBytes = 2 * 2048 * kNearCols<SPLIT>;   // two buffers
 // Ring of weights.  bf16: few slots, each wait holds up the issue of MMAs for 90 cycles (one query 18.9 -> 17.8 us against five
 // of 32 KB); a layer in split precision does not fit, and there two large ones are refilled too late (28.9 -> 34.7).
 template <bool SPLIT>
@@ -47,7 +50,7 @@ constexpr int kNearSlots = SPLIT ? 5 : 2;
 template <bool SPLIT>
 constexpr int kNearSlotBytes = (SPLIT ? 2 : 4) * kTileBytes;
 template <bool SPLIT>
-constexpr int kNearSmem = kNearActBytes + kNearSlots<SPLIT> * kNearSlotBytes<SPLIT> + 1024 + 512;
+constexpr int kNearSmem = kNearActBytes<SPLIT> + kNearSlots<SPLIT> * kNearSlotBytes<SPLIT> + 1024 + 512;
 static_assert(kNearSmem<false> <= 232448 && kNearSmem<true> <= 232448, "shared memory");
 
 // mbar_wait that also leaves the mark in the scratch.
@@ -93,13 +96,13 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
   constexpr int kUnitBytes = kNearM * 128;            // one K block of the rows
   constexpr int kUnitsPerSlot = kSlotBytes / kUnitBytes;
   constexpr int kSlotsPerLayer = kNumKB * kParts / kUnitsPerSlot;
-  constexpr int kBufferBytes = 2048 * kNearCols;
+  constexpr int kCols = kNearCols<SPLIT>, kBufferBytes = 2048 * kCols;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - raw);
   const uint32_t act = base;
-  const uint32_t ring = base + kNearActBytes;
+  const uint32_t ring = base + kNearActBytes<SPLIT>;
   const uint32_t bars = ring + kSlots * kSlotBytes;
   uint8_t* bars_ptr = base_ptr + (bars - base);
   const uint32_t bar_full = bars, bar_empty = bars + 64;      // [kSlots]
@@ -189,13 +192,13 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
     }
   } else if (warp == 0) {
     // ------------------------------ MMA issuer ------------------------------
-    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kNearCols >> 3) << 17) |
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kCols >> 3) << 17) |
                                (static_cast<uint32_t>(kNearM >> 4) << 24);
-    // A and B: K-major, 128-byte swizzle, 8-row groups 1024 B apart; B: 16 rows (queries) of 128 bytes per K block
+    // A and B: K-major, 128-byte swizzle, 8-row groups 1024 B apart; B: kCols rows of 128 bytes per K block
     const uint64_t desc = (static_cast<uint64_t>(1024 >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
                           (static_cast<uint64_t>(2) << 61) | (static_cast<uint64_t>(1) << 16);
     // in 16-byte units: 16 K values of B, a K block of 64
-    constexpr uint32_t kStepB = 2, kBlockB = (128 * kNearCols) >> 4;
+    constexpr uint32_t kStepB = 2, kBlockB = (128 * kCols) >> 4;
     const uint32_t a_lo0 = (ring & 0x3FFFF) >> 4, b_lo0 = (act & 0x3FFFF) >> 4;
     // One elected lane runs the whole loop.  An MMA of this shape takes 23 cycles and only a
     // couple of them queue up, so what stands between two MMAs shows: the wait for the next slot goes
@@ -270,7 +273,7 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
     auto epi_sync = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
     // fc1's B operand: K columns 0..63 hold [hi | lo | hi] of the normalised features, one query per row
     const int C_in = p.n_op_feat + 4;
-    for (int i = T; i < 64 * 2 * kNearCols / 16; i += 128) *reinterpret_cast<uint4*>(base_ptr + 16 * i) = make_uint4(0, 0, 0, 0);
+    for (int i = T; i < 64 * 2 * kCols / 16; i += 128) *reinterpret_cast<uint4*>(base_ptr + 16 * i) = make_uint4(0, 0, 0, 0);
     epi_sync();
     for (int i = T; i < n_q * C_in; i += 128) {
       const int q = i / C_in, f = i - q * C_in;
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
     const bool row_ok = lane < 16;
     const int row = quad * 16 + (lane & 15), f = c * kNearM + row;
     const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
-    constexpr int kPiece = kNearCols / 2;                       // queries
+    constexpr int kPiece = 8;                                   // columns, queries
     bool ok = true;
     // a wait that ran out skips the work that is left but none of the block-wide barriers
     for (int L = 0; L < n_layers; ++L) {
@@ -305,7 +308,7 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
       tc_ld8(t_lane, v);
       if (SPLIT) {   // columns 8 to 15 are the lo parts
         float lo[kPiece];
-        tc_ld8(t_lane + kNearCols / 2, lo);
+        tc_ld8(t_lane + 8, lo);
 #pragma unroll
         for (int i = 0; i < kPiece; ++i) v[i] += lo[i];
       }
@@ -316,7 +319,7 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
       for (int i = 0; i < kPiece; ++i) v[i] = fmaxf(v[i] + bias, 0.0f);
       if (!last) {
         // own features first, then the group's other blocks: 128 bytes of every query
-        const uint32_t mine = static_cast<uint32_t>((L + 1) & 1) * kBufferBytes + static_cast<uint32_t>(c) * (128u * kNearCols);
+        const uint32_t mine = static_cast<uint32_t>((L + 1) & 1) * kBufferBytes + static_cast<uint32_t>(c) * (128u * kCols);
         const uint32_t in_bar = bar_act + 8 * ((L + 1) & 1);
 #pragma unroll
         for (int q = 0; q < kNearQ / kParts; ++q) {
@@ -324,7 +327,7 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
           const __nv_bfloat16 hi = __float2bfloat16_rn(v[q]);
           *reinterpret_cast<__nv_bfloat16*>(base_ptr + mine + swz_off(q, row)) = hi;
           if (SPLIT)
-            *reinterpret_cast<__nv_bfloat16*>(base_ptr + mine + swz_off(kNearCols / 2 + q, row)) =
+            *reinterpret_cast<__nv_bfloat16*>(base_ptr + mine + swz_off(8 + q, row)) =
                 __float2bfloat16_rn(v[q] - __bfloat162float(hi));
         }
         fence_proxy_async();
@@ -337,7 +340,7 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
           for (uint32_t q = 0; q < static_cast<uint32_t>(n_q); ++q)
 #pragma unroll
             for (uint32_t part = 0; part < kParts; ++part) {
-              const uint32_t at = (part * (kNearCols / 2) + q) * 128u + (((chunk ^ q) & 7u) << 4);
+              const uint32_t at = (part * 8 + q) * 128u + (((chunk ^ q) & 7u) << 4);
               const uint4 x = *reinterpret_cast<const uint4*>(base_ptr + mine + at);
               st_async_v4(there + at, x.x, x.y, x.z, x.w, bar);
             }
@@ -520,7 +523,7 @@ namespace hb {
 // 33 of 16, 8 or 4 blocks.  Smaller clusters hold more queries in all but stream more weights per block, wider ones
 // exchange more per layer.  Measured per launch, conv2d predictor, 8 hidden layers (capacity in queries: us), against 103 us
 // (bf16) and 168 us (split) of one tile of mlp_chain.cu's kernel, which is the faster one beyond the last shape:
-//   near               28: 19.6 (one: 17.8)   split    14: 29.6 (one: 27.8)
+//   near               28: 19.9 (one: 17.6)   split    14: 29.8 (one: 27.4)
 //   8 pairs x 16      224: 25.4 (one: 22.7)           112: 33.0 (one: 30.2)
 //   8 pairs x 32      448: 27.3                       224: 36.4
 //   4 pairs x 32      960: 35.2                       480: 49.5
