@@ -1,4 +1,4 @@
-// Shared by the MLP kernels (mlp_chain.cu, mlp_wide.cu): sizes, PTX wrappers, the handle.
+// Shared by the MLP kernels (mlp_chain.cu, mlp_pairs.cu, mlp_wide.cu): sizes, PTX wrappers, the handle.
 #pragma once
 
 #include <cuda.h>

@@ -20,13 +20,12 @@
 //
 // The arrival should be a release: one more round trip to L2, 1,300 to 2,300 cycles in each layer.  The network is tried
 // without first.  The arrival is a relaxed one, what has come is used at once, and warps look at it afterwards, while the
-// next layer's is on its way.  An activation is never
-// negative, so the high sign bit of every 32-bit word (two bf16 activations, or the lo and the hi part of one in
+// next layer's is on its way.  An activation is never negative, so the high sign bit of every 32-bit word (two bf16 activations, or the lo and the hi part of one in
 // split precision) carries the parity of the buffer's use; with the parity 1 both halves are negated, and the instruction
 // negates B.  A word of an earlier use with the same parity cannot come: the use in between has been looked at in the
-// same place.  Where a word does not show the parity (in one launch of 4,000 while other streams kept L2 busy), all CTAs of
-// the cluster run the network once more, with releases and buffers without parities.  No result is stored
-// before all CTAs have looked at everything.  Two buffers alternate by layer: a CTA writes layer L only after its pair
+// same place.  Where a word does not show the parity (in one launch of 40,000 while other streams kept L2 busy, never
+// alone), all CTAs of the cluster run the network once more, with releases and buffers without parities.  No result is
+// stored before all CTAs have looked at everything.  Two buffers alternate by layer: a CTA writes layer L only after its pair
 // has read all of layer L - 1, which every CTA wrote after reading L - 2.  The host keeps the parity each group's buffers
 // have reached.
 // (448 queries: 27.3 us so, 26.5 if nobody looked; with releases 32; by ordinary loads that poll the data in L2, 32 bytes a
@@ -48,8 +47,8 @@
 // have more clusters than fit at a time.
 //
 // Warp roles: 0 TMEM, the mark, activation loads; 1 MMA issuer (the pair's leader); 2-3 weight producers; 4 and more:
-// epilogue; NC = 16, 32: eight more that look at what has come.  Every wait is bounded, as in mlp_chain.cu; a launch that gave up leaves a mark in the scratch, and
-// launches that find it report an error instead of a result.  After giving up no ring slot is requested again whose
+// epilogue; NC = 16, 32: eight more that look at what has come.  Every wait is bounded, as in mlp_chain.cu; a launch that
+// gave up leaves a mark in the scratch, and launches that find it report an error instead of a result.  After giving up no ring slot is requested again whose
 // copy could be under way: the MMA issuer, whose commits free the slots, waits for the producers of both CTAs to leave
 // before it issues anything past a wait that ran out, and goes no further than the layer's end.
 #include "mlp_small.cuh"
@@ -225,6 +224,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
   constexpr uint32_t kSigns = SPLIT ? 0x80000000u : 0x80008000u;   // those that carry the parity
   float result = 0.0f;
 
+  bool start = true;     // a CTA that gave up takes no part in a second run
   // sure: with releases; the first run goes without
 #pragma unroll 1
   for (bool sure = false;; sure = true) {
@@ -234,7 +234,6 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
       return !sure && (((p.parity[use & 1] >> group) + static_cast<unsigned>(use >> 1)) & 1ull) ? 0x80008000u : 0u;
     };
     const uint32_t tag = sure ? p.tag | 0x80000000u : p.tag;
-    const bool start = *abort_flag == 0;       // a CTA that gave up takes no part in a second run
     if (warp == 0) {
       // ------------------------------ the mark; activation loads ------------------------------
       if (lane == 0 && start) {
@@ -586,6 +585,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     tc_fence_after();
     if (sure || *stale == 0) break;
+    start = *abort_flag == 0;   // (nobody sets it between the two barriers)
     if (threadIdx.x == 0) {
       for (int i = 0; i < kBars; ++i) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bars + 8 * i) : "memory");
       init_barriers();
