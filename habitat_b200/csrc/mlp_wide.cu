@@ -1,7 +1,7 @@
 // MLP inference for few queries: the layers' features are spread over the SMs, and sixteen thread blocks exchange them
 // through distributed shared memory; and the choice of kernel for every batch that does not fill the GPU.
 //
-// Sixteen thread blocks form a group (one cluster) that owns up to four queries (two in split precision); block c computes
+// Sixteen thread blocks form a group (one cluster) that owns up to six queries (two in split precision); block c computes
 // output features 64 c .. of every layer for them and streams only their weights.
 //
 // Formulation as in mlp_chain.cu, H^T = W . X^T with tcgen05.mma (cta_group::1): A = weight rows (M = 64), B =
@@ -40,7 +40,8 @@ template <bool SPLIT>
 constexpr int kNearCols = SPLIT ? 16 : 8;
 constexpr int kNearM = 64;                            // weight rows per block
 constexpr int kNearThreads = 256;
-constexpr int kNearQ = 4;                             // queries per group at most; split: half as many
+template <bool SPLIT>
+constexpr int kNearQ = SPLIT ? 2 : 6;                 // queries per group at most (with eight 0.3 us more for all, 56: 22.9)
 template <bool SPLIT>
 constexpr int kNearActBytes = 2 * 2048 * kNearCols<SPLIT>;   // two buffers
 // Ring of weights.  bf16: few slots, each wait holds up the issue of MMAs for 90 cycles (one query 18.9 -> 17.8 us against five
@@ -322,7 +323,7 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
         const uint32_t mine = static_cast<uint32_t>((L + 1) & 1) * kBufferBytes + static_cast<uint32_t>(c) * (128u * kCols);
         const uint32_t in_bar = bar_act + 8 * ((L + 1) & 1);
 #pragma unroll
-        for (int q = 0; q < kNearQ / kParts; ++q) {
+        for (int q = 0; q < kNearQ<SPLIT>; ++q) {
           if (!row_ok || q >= n_q) continue;
           const __nv_bfloat16 hi = __float2bfloat16_rn(v[q]);
           *reinterpret_cast<__nv_bfloat16*>(base_ptr + mine + swz_off(q, row)) = hi;
@@ -420,7 +421,9 @@ constexpr int kMaxGroups = 34;
 constexpr int kTryShapes = 5;                           // of kShapes, after the first
 constexpr size_t acts_bytes(int groups, int row_bytes) { return static_cast<size_t>(groups) * 4 * kWidth * row_bytes; }
 constexpr int kTryGroups[kTryShapes] = {8, 8, 16, 16, kMaxGroups}, kTryRow[kTryShapes] = {32, 64, 64, 128, 128};
-constexpr size_t try_offset(int shape) { return shape ? try_offset(shape - 1) + acts_bytes(kTryGroups[shape - 1], kTryRow[shape - 1]) : 0; }
+constexpr size_t try_offset(int shape) {
+  return shape ? try_offset(shape - 1) + acts_bytes(kTryGroups[shape - 1], kTryRow[shape - 1]) : 0;
+}
 constexpr size_t kSureOffset = try_offset(kTryShapes), kActsBytes = kSureOffset + acts_bytes(kMaxGroups, 128);
 constexpr size_t kHalvesBytes = static_cast<size_t>(kMaxGroups) * 64 * hb::kGroupCols * sizeof(unsigned long long);
 constexpr size_t kScratchBytes = kActsBytes + kHalvesBytes + 256;   // and the mark of a launch that gave up
@@ -523,7 +526,7 @@ namespace hb {
 // 33 of 16, 8 or 4 blocks.  Smaller clusters hold more queries in all but stream more weights per block, wider ones
 // exchange more per layer.  Measured per launch, conv2d predictor, 8 hidden layers (capacity in queries: us), against 103 us
 // (bf16) and 168 us (split) of one tile of mlp_chain.cu's kernel, which is the faster one beyond the last shape:
-//   near               28: 19.9 (one: 17.6)   split    14: 29.8 (one: 27.4)
+//   near               42: 21.5 (one: 17.6)   split    14: 29.5 (one: 27.2)
 //   8 pairs x 16      224: 25.4 (one: 22.7)           112: 33.0 (one: 30.2)
 //   8 pairs x 32      448: 27.3                       224: 36.4
 //   4 pairs x 32      960: 35.2                       480: 49.5
@@ -538,7 +541,9 @@ struct Shape { int pairs, NC, clusters, us, us_split; };   // pairs 0: mlp_near_
 constexpr Shape kShapes[] = {{0, 16, 7, 20, 30}, {8, 16, 7, 25, 33}, {8, 32, 7, 27, 36}, {4, 32, 15, 35, 49},
                              {4, 64, 15, 46, 62}, {2, 64, 33, 65, 105}};
 int clusters_of(const Shape& s, int sm_count) { return sm_count >= 148 ? s.clusters : s.clusters * sm_count / 148; }
-int cols_of(const Shape& s, bool split) { return s.pairs == 0 ? (split ? kNearQ / 2 : kNearQ) : (split ? s.NC : 2 * s.NC); }
+int cols_of(const Shape& s, bool split) {
+  return s.pairs == 0 ? (split ? kNearQ<true> : kNearQ<false>) : (split ? s.NC : 2 * s.NC);
+}
 WidePlan plan_in(const Shape& s, int64_t Q, bool split, int cols = 0) {
   // full groups while they last: fewer groups move the weights fewer times
   if (cols == 0) cols = cols_of(s, split);
