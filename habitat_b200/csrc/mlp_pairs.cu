@@ -94,8 +94,16 @@ struct PairShape {
   static_assert(kSmem <= 232448, "shared memory");
 };
 
+// A bounded wait that leaves the mark in the scratch: what this CTA's threads, copies and MMAs have done.
 __device__ __forceinline__ bool pairs_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, const SmallParams& p,
                                            int code) {
+  if (mbar_wait(bar, parity, abort_flag, p.status, code)) return true;
+  atomicExch(p.poison, 1);
+  return false;
+}
+// ... what other CTAs' threads have done.
+__device__ __forceinline__ bool cluster_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, const SmallParams& p,
+                                             int code) {
   if (mbar_wait_cluster(bar, parity, abort_flag, p.status, code)) return true;
   atomicExch(p.poison, 1);
   return false;
@@ -256,7 +264,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
               ok = S::kApart ? pairs_wait(bar_acc, u & 1, abort_flag, p, 0x531)
                              : pairs_wait(bar_stored + 8 * b, u & 1, abort_flag, p, 0x531);
               if (!sure && u > 0 && q == 0) ok = ok && pairs_wait(bar_seen, (u - 1) & 1, abort_flag, p, 0x534);
-              ok = ok && pairs_wait(bar_sig + 8 * (buf * S::kBlocks + b), (u >> 1) & 1, abort_flag, p, 0x532);
+              ok = ok && cluster_wait(bar_sig + 8 * (buf * S::kBlocks + b), (u >> 1) & 1, abort_flag, p, 0x532);
               asm volatile("fence.proxy.async.global;" ::: "memory");
             } else if (S::kBlocks == 2 && q == 1 && u > 0) {
               ok = pairs_wait(bar_q1, (u - 1) & 1, abort_flag, p, 0x533);
@@ -317,7 +325,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
       // last 16 MMAs: with 8 an MMA took 33 cycles whatever N, with 16 it takes 23 to 25.
       if (r == 0 && start && elect_one()) {
         auto wait = [&](uint32_t bar, uint32_t parity, int code) {
-          if (!pairs_wait(bar, parity, abort_flag, p, code)) {
+          if (!mbar_try_wait(bar, parity) && (*abort_flag || !pairs_wait(bar, parity, abort_flag, p, code))) {
             // (the producers look at their CTA's abort flag when a slot does not come)
             st_cluster_u32(map_to_cta(bars + 292, leader + 1), 1u);
             __threadfence();
@@ -328,7 +336,8 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
           tc_fence_after();
         };
         uint32_t s = 0, ph = 0;
-        wait(bar_feat, 0, 0x521);
+        if (!cluster_wait(bar_feat, 0, abort_flag, p, 0x521)) wait(bar_feat, 0, 0x521);
+        tc_fence_after();
 #pragma unroll 1
         for (int b = 0; b < S::kBlocks; ++b) {                     // fc1: one K block
           wait(bar_full + 8 * s, ph, 0x522);

@@ -527,19 +527,19 @@ namespace hb {
 // exchange more per layer.  Measured per launch, conv2d predictor, 8 hidden layers (capacity in queries: us), against 103 us
 // (bf16) and 168 us (split) of one tile of mlp_chain.cu's kernel, which is the faster one beyond the last shape:
 //   near               42: 21.5 (one: 17.6)   split    14: 29.5 (one: 27.2)
-//   8 pairs x 16      224: 25.4 (one: 22.7)           112: 33.0 (one: 30.2)
-//   8 pairs x 32      448: 27.3                       224: 36.4
-//   4 pairs x 32      960: 35.2                       480: 49.5
-//   4 pairs x 64    1,920: 45.6                       960: 62.2   (in one row block, exchanged at once, 51.5 and 73.6)
-//   2 pairs x 64    4,224: 65.1                     2,112: 105
+//   8 pairs x 16      224: 25.2 (one: 22.5)           112: 32.2 (one: 29.8)
+//   8 pairs x 32      448: 27.2                       224: 35.9
+//   4 pairs x 32      960: 34.8                       480: 49.2   (in two row blocks 38.8 and 49.9)
+//   4 pairs x 64    1,920: 44.8                       960: 61.5   (in one row block, exchanged at once, 51.5 and 73.6)
+//   2 pairs x 64    4,224: 64.2                     2,112: 105
 // Blocks without partners (M = 64 or 128 each, all queries of a group in every block; data polled in L2) took 24 for 112,
 // 28 for 240, 32 for 480, 46 for 960, 48 for 1,056 and 73 for 2,112 queries, split 34 for 56, 46 for 240, 78 for 528 and 126
 // for 1,056: better than these only from 100 to 112 and 449 to 480 queries, by 3 and 9 % (split: 225 to 240, 8 %).
 namespace {
 // us: what a launch of the shape takes, full or not
 struct Shape { int pairs, NC, clusters, us, us_split; };   // pairs 0: mlp_near_kernel
-constexpr Shape kShapes[] = {{0, 16, 7, 20, 30}, {8, 16, 7, 25, 33}, {8, 32, 7, 27, 36}, {4, 32, 15, 35, 49},
-                             {4, 64, 15, 46, 62}, {2, 64, 33, 65, 105}};
+constexpr Shape kShapes[] = {{0, 16, 7, 21, 30}, {8, 16, 7, 25, 32}, {8, 32, 7, 27, 36}, {4, 32, 15, 35, 49},
+                             {4, 64, 15, 45, 62}, {2, 64, 33, 64, 105}};
 int clusters_of(const Shape& s, int sm_count) { return sm_count >= 148 ? s.clusters : s.clusters * sm_count / 148; }
 int cols_of(const Shape& s, bool split) {
   return s.pairs == 0 ? (split ? kNearQ<true> : kNearQ<false>) : (split ? s.NC : 2 * s.NC);
