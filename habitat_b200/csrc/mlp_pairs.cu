@@ -1,7 +1,7 @@
 // MLP inference for batches between a few queries and full rounds of mlp_chain.cu's tiles: clusters of two-SM pairs.
 //
 // mlp_chain.cu gives a pair of SMs 128 queries and streams all weights past them: 103 to 110 us whether the batch has one
-// query or 9,472.  Here P = 8, 4 or 2 pairs form a cluster that owns up to 2 NC queries (NC = 16, 32 or 64; split
+// query or 9,472.  Here P = 8, 4 or 2 pairs form a cluster that owns up to 2 NC queries (NC = 16, 32, 40 or 64; split
 // precision: NC).  Pair i computes 1024 / P output features of every layer for all of them and streams only their
 // weights, and after each layer the cluster exchanges its activations.
 //
@@ -32,12 +32,16 @@
 // cycle, 34; bulk copies that are looked at before they are used 30.  1,920 queries 45.6, with releases 49.2; 4,224 65.1 and
 // 68.2.)
 //
+// NC = 40: rows of 80 bytes fit no swizzle, so B lies in panels of eight columns, 16 bytes a row, and a warp's rows go out as
+// five copies of 512 bytes.  N is a multiple of 32, so the MMAs read a sixth panel per CTA, which is whatever lies behind the
+// fifth; nobody reads the columns of D that come of it.  480 queries: 29.1 us; 34.8 in groups of four pairs.
+//
 // NC = 64: a pair's features are two row blocks, one in K quarters 0 and 1 and one in 2 and 3.  The units (block b, K quarter
 // q) of a layer are issued in the order (0,0) (0,1) (1,0) (0,2) (0,3) | (1,1) (1,2) (1,3): quarters 0 and 1 are
 // exchanged under the last three units and quarters 2 and 3 under the first three of the next layer.  D alternates between two
 // sets of TMEM columns.
 //
-// What bounds it: NC = 16, 32 the latency of one exchange per layer (P = 8: 2,300 to 2,700 cycles from the last MMA to the next
+// What bounds it: NC = 16 to 40 the latency of one exchange per layer (P = 8: 2,300 to 2,700 cycles from the last MMA to the next
 // layer's first, of which 300 to 500 until the accumulators are there, 350 to take them and write them out, 400 for the
 // store, 400 for the arrivals, 700 for the loads) next to 1,500 of MMAs; NC = 64 shared memory besides: a CTA's weights are
 // written and read once per layer, B is read once per row block, and the exchange writes it, 1.5 MB a layer and CTA for P = 2
@@ -47,7 +51,7 @@
 // have more clusters than fit at a time.
 //
 // Warp roles: 0 TMEM, the mark, activation loads; 1 MMA issuer (the pair's leader); 2-3 weight producers; 4 and more:
-// epilogue; NC = 16, 32: eight more that look at what has come.  Every wait is bounded, as in mlp_chain.cu; a launch that
+// epilogue; NC = 16 to 40: eight more that look at what has come.  Every wait is bounded, as in mlp_chain.cu; a launch that
 // gave up leaves a mark in the scratch, and launches that find it report an error instead of a result.  After giving up no ring slot is requested again whose
 // copy could be under way: the MMA issuer, whose commits free the slots, waits for the producers of both CTAs to leave
 // before it issues anything past a wait that ran out, and goes no further than the layer's end.
@@ -66,7 +70,8 @@ struct PairShape {
   static constexpr int kBlocks = NC == 64 ? 2 : 1;         // row blocks per pair
   static constexpr int kRows = 512 / P / kBlocks;          // A rows per CTA and block
   static constexpr bool kNarrow = kRows == 64;             // M = 128: D's second half of the columns is in TMEM lanes 64 and up
-  static constexpr int kN = 2 * NC;
+  static constexpr bool kPanels = NC == 40;                // B without swizzle, in panels of eight columns
+  static constexpr int kN = (2 * NC + 31) / 32 * 32;
   static constexpr int kHalfQ = SPLIT ? NC / 2 : NC;       // queries per CTA at most
   static constexpr int kRowBytes = 2 * NC;
   static constexpr int kActBytes = kWidth * kRowBytes;
@@ -85,8 +90,8 @@ struct PairShape {
   static constexpr int kStores = kNarrow ? 4 : 8;          // bulk stores per block and CTA
   static constexpr int kLookWarps = kApart ? 8 : 0;        // those that look at what has come; else the epilogue's do
   static constexpr int kThreads = 128 + 32 * (kEpiWarps + kLookWarps);
-  static constexpr int kDCols = kNarrow ? NC : kN;          // TMEM columns of a block
-  static constexpr uint32_t kTmemCols = kBlocks == 2 ? 4 * kDCols : (kDCols < 32 ? 32 : kDCols);
+  static constexpr int kDCols = kNarrow ? kN / 2 : kN;      // TMEM columns of a block
+  static constexpr uint32_t kTmemCols = kBlocks == 2 ? 4 * kDCols : (kDCols <= 32 ? 32 : (kDCols <= 64 ? 64 : 128));
   static_assert(kRows == 64 || kRows == 128, "shapes");
   static_assert(!kJoint || (kUnitSlots == 1 && kSlots == kUnits), "a slot per quarter, each its own");
   static constexpr int kStageBytes = kApart ? 2 * kRows * kRowBytes : 0;   // this CTA's rows on their way out
@@ -141,9 +146,11 @@ __device__ __forceinline__ void commit_pair(uint32_t bar, uint16_t ctas) {
       "h"(ctas)
       : "memory");
 }
-// Byte offset of 16-byte chunk `chunk` of K row k in a B operand of NC columns per CTA (swizzle width 2 NC bytes).
+// Byte offset of 16-byte chunk `chunk` of K row k in a B operand of NC columns per CTA (swizzle width 2 NC bytes); NC = 40: in
+// panels of `rows` K rows of 16 bytes, 256 in a K quarter.
 template <int NC>
-__device__ __forceinline__ uint32_t b_chunk(uint32_t k, uint32_t chunk) {
+__device__ __forceinline__ uint32_t b_chunk(uint32_t k, uint32_t chunk, uint32_t rows = 256) {
+  if (NC == 40) return (chunk * rows + k) * 16u;
   const uint32_t x = NC == 64 ? (k & 7u) : (NC == 32 ? ((k >> 1) & 3u) : ((k >> 2) & 1u));
   return k * (2u * NC) + ((chunk ^ x) << 4);
 }
@@ -251,7 +258,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
           *abort_flag = 1;
         }
         bool ok = true;
-        const int32_t row0 = (group * 4 + static_cast<int>(r)) * kWidth;
+        const int32_t row0 = (group * 4 + static_cast<int>(r)) * 4;   // in K quarters
         const CUtensorMap* const map = sure ? &p.map_sure : &p.map_acts;
         for (int L = 1; L < n_layers && ok; ++L) {
           const int u = L - 1, buf = u & 1;
@@ -272,7 +279,8 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
             if (!ok) break;
             const uint32_t bar = S::kJoint ? bar_full + 8 * ((S::kBlocks + q) % S::kSlots) : bar_actq + 8 * q;
             if (r == 0) mbar_expect_tx(bar, 2u * 256u * S::kRowBytes);
-            tma_2d_pair(act + q * 256 * S::kRowBytes, map, row0 + buf * 2 * kWidth + q * 256, map_to_cta(bar, leader));
+            tma_2d_pair(act + q * 256 * S::kRowBytes, map, (row0 + buf * 8 + q) * static_cast<int32_t>(hb::act_map_box(NC)),
+                        map_to_cta(bar, leader));
           }
         }
       }
@@ -313,11 +321,16 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
       // groups of K 16 NC bytes apart
       const uint64_t desc_a = (static_cast<uint64_t>(1024 >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
                               (static_cast<uint64_t>(2) << 61) | (static_cast<uint64_t>(1) << 16);
-      const uint64_t desc_b = (static_cast<uint64_t>((16 * NC) >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
-                              (static_cast<uint64_t>(NC == 64 ? 2 : (NC == 32 ? 4 : 6)) << 61) |
-                              (static_cast<uint64_t>(1) << 16);
-      // in 16-byte units: 16 K values of B, a K block of 64
-      constexpr uint32_t kStepB = (32 * NC) >> 4, kBlockB = (128 * NC) >> 4;
+      // (panels: no swizzle, 8-row groups 128 B apart and 8-column ones 4 KB)
+      const uint64_t desc_b =
+          S::kPanels ? (static_cast<uint64_t>(4096 >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
+                           (static_cast<uint64_t>(128 >> 4) << 16)
+                     : (static_cast<uint64_t>((16 * NC) >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
+                           (static_cast<uint64_t>(NC == 64 ? 2 : (NC == 32 ? 4 : 6)) << 61) |
+                           (static_cast<uint64_t>(1) << 16);
+      // in 16-byte units: 16 K values of B, a K block of 64, a K quarter
+      constexpr uint32_t kStepB = (S::kPanels ? 256 : 32 * NC) >> 4, kBlockB = 4 * kStepB;
+      constexpr uint32_t kQuarterB = (256 * S::kRowBytes) >> 4;
       const uint32_t a_lo0 = (ring & 0x3FFFF) >> 4, b_lo0 = (act & 0x3FFFF) >> 4;
       // One elected lane runs the whole loop, and no loop of a layer depends on what a wait returns (after a wait that
       // ran out the abort flag is set, and what is issued on stale operands is discarded), which keeps the descriptors in
@@ -371,7 +384,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
               for (uint32_t i = 0; i < 4 * S::kImages; ++i) {
                 const uint32_t kb = (g * S::kImages + (i >> 2)) / S::kParts, k = i & 3u;
                 tc_mma_pair_bf16(d, desc_a | (a_lo + (i >> 2) * (S::kUnitBytes >> 4) + 2 * k),
-                                 desc_b | (b_lo0 + (kq * 4 + kb) * kBlockB + k * kStepB), id,
+                                 desc_b | (b_lo0 + kq * kQuarterB + kb * kBlockB + k * kStepB), id,
                                  (g == 0 && i == 0) ? kq : 1u);
                 if (i == 2 * S::kImages - 1) {
                   // (not past the layer's end: a try_wait that has to wait holds up the MMAs behind it)
@@ -391,7 +404,8 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
       __syncwarp();
     } else if (S::kApart && warp >= 4 + S::kEpiWarps) {
       // ------------------------------ looking at what has been used ------------------------------
-      constexpr int kShare = S::kApart ? S::kActBytes / S::kLookWarps : 0, kBatch = 8;
+      constexpr int kShare = S::kApart ? S::kActBytes / S::kLookWarps : 0, kBatch = S::kPanels ? 10 : 8;
+      static_assert(kShare % (512 * kBatch) == 0, "all of it");
       const uint8_t* const mine = base_ptr + (warp - 4 - S::kEpiWarps) * kShare + 16 * lane;
 #pragma unroll 1
       for (int L = 0; L < n_layers && start && !sure; ++L) {
@@ -423,7 +437,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         auto feat_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory"); };
         const int C_in = p.n_op_feat + 4;
         for (int i = T; i < 64 * S::kRowBytes / 16; i += kEpiThreads)
-          *reinterpret_cast<uint4*>(base_ptr + 16 * i) = make_uint4(0, 0, 0, 0);
+          *reinterpret_cast<uint4*>(base_ptr + (S::kPanels ? b_chunk<NC>(i & 63, i >> 6) : 16 * i)) = make_uint4(0, 0, 0, 0);
         feat_sync();
         for (int i = T; i < n_q * C_in; i += kEpiThreads) {
           const int q = i / C_in, f = i - q * C_in;
@@ -498,7 +512,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
             tc_fence_after();
             const uint32_t t_block = t_lane + (S::kBlocks == 2 ? static_cast<uint32_t>(((L & 1) * 2 + b) * S::kDCols) : 0u);
             float v[kPiece];
-            if (SPLIT) {
+            if constexpr (SPLIT) {
               float d[kCols];
               tc_ld_cols<kCols>(t_block, d);
 #pragma unroll
@@ -529,7 +543,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
               for (int c = 0; c < kWords / 4; ++c) {
                 uint4* const to = reinterpret_cast<uint4*>(
                     base_ptr + (rows - base) +
-                    b_chunk<NC>(static_cast<uint32_t>(at0 + lane), static_cast<uint32_t>(part * (kWords / 4) + c)));
+                    b_chunk<NC>(static_cast<uint32_t>(at0 + lane), static_cast<uint32_t>(part * (kWords / 4) + c), 2 * S::kRows));
                 if (!S::kApart && !sure && L > 0) {   // looked at before it goes
                   const uint4 x = *to;
                   bad |= (x.x ^ want) | (x.y ^ want) | (x.z ^ want) | (x.w ^ want);
@@ -539,7 +553,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
               fence_proxy_async();
               if (bad & kSigns) saw_stale();
             } else {
-              constexpr int kFold = kPiece < 16 ? 16 : kPiece;
+              constexpr int kFold = (kPiece + 15) / 16 * 16;
               float sum[kFold];
 #pragma unroll
               for (int i = 0; i < kFold; ++i) sum[i] = i < kPiece ? __fmul_rn(w2, v[i % kPiece]) : 0.0f;
@@ -547,7 +561,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
               const int set = (f0 + (lane & 16)) / 16, col = fold16_col<kFold>(lane);
               unsigned long long* h = group_halves + set * hb::kGroupCols + half * 64 + part * kPiece + col;
 #pragma unroll
-              for (int i = 0; i < kFold / 16 && (kPiece >= 16 || col < kPiece); ++i)
+              for (int i = 0; i < kFold / 16 && (kPiece == kFold || col + i < kPiece); ++i)
                 st_relaxed_u64(h + i, static_cast<unsigned long long>(tag) << 32 | __float_as_uint(sum[i]));
             }
           }
@@ -559,10 +573,15 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
           rows_sync();
           if (part == 0) {
             if (ok) {
-              if (lane == 0) {
-                store_rows(group_acts + ((L & 1) * 2 + half) * kHalfBytes + static_cast<uint32_t>(f0) * S::kRowBytes,
-                           rows + static_cast<uint32_t>(at0) * S::kRowBytes, 32 * S::kRowBytes);
-                mbar_arrive(bar_stored + 8 * b);
+              uint8_t* const to = group_acts + ((L & 1) * 2 + half) * kHalfBytes;
+              if (S::kPanels) {
+                if (lane < NC / 8)
+                  store_rows(to + (f0 >> 8) * (256 * S::kRowBytes) + b_chunk<NC>(f0 & 255, lane),
+                             rows + b_chunk<NC>(at0, lane, 2 * S::kRows), 32 * 16);
+              } else if (lane == 0) {
+                store_rows(to + static_cast<uint32_t>(f0) * S::kRowBytes, rows + static_cast<uint32_t>(at0) * S::kRowBytes,
+                           32 * S::kRowBytes);
+                if (!S::kApart) mbar_arrive(bar_stored + 8 * b);
               }
               __syncwarp();
               if (lane < P) {
@@ -640,6 +659,7 @@ template <bool SPLIT>
 cudaError_t launch(int P, int NC, const SmallParams& p, int groups, int device, cudaStream_t stream, bool* fits) {
   switch (P * 100 + NC) {
     case 816: return launch<8, 16, SPLIT>(p, groups, device, stream, fits);
+    case 840: return launch<8, 40, SPLIT>(p, groups, device, stream, fits);
     case 832: return launch<8, 32, SPLIT>(p, groups, device, stream, fits);
     case 432: return launch<4, 32, SPLIT>(p, groups, device, stream, fits);
     case 464: return launch<4, 64, SPLIT>(p, groups, device, stream, fits);

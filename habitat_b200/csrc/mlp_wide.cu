@@ -418,11 +418,11 @@ constexpr int kMaxStreams = 16, kMoreStreams = 16;
 constexpr int kMaxGroups = 34;
 // Activation buffers of mlp_pairs.cu: one for the first runs of each shape (a word's parity counts its own uses), and one that
 // all shapes use for second runs.
-constexpr int kTryShapes = 5;                           // of kShapes, after the first
+constexpr int kTryShapes = 6;                           // of kShapes, after the first
 constexpr size_t acts_bytes(int groups, int row_bytes) { return static_cast<size_t>(groups) * 4 * kWidth * row_bytes; }
-constexpr int kTryGroups[kTryShapes] = {8, 8, 16, 16, kMaxGroups}, kTryRow[kTryShapes] = {32, 64, 64, 128, 128};
+constexpr int kTryGroups[kTryShapes] = {8, 8, 8, 16, 16, kMaxGroups}, kTryNC[kTryShapes] = {16, 32, 40, 32, 64, 64};
 constexpr size_t try_offset(int shape) {
-  return shape ? try_offset(shape - 1) + acts_bytes(kTryGroups[shape - 1], kTryRow[shape - 1]) : 0;
+  return shape ? try_offset(shape - 1) + acts_bytes(kTryGroups[shape - 1], 2 * kTryNC[shape - 1]) : 0;
 }
 constexpr size_t kSureOffset = try_offset(kTryShapes), kActsBytes = kSureOffset + acts_bytes(kMaxGroups, 128);
 constexpr size_t kHalvesBytes = static_cast<size_t>(kMaxGroups) * 64 * hb::kGroupCols * sizeof(unsigned long long);
@@ -435,7 +435,7 @@ struct StreamScratch {
   uint32_t tag = 0;
   unsigned long long parity[kTryShapes][2] = {};   // bit g: parity of the next use of group g's buffers
   bool expect_stale = false;                     // at the next launch that could (tests)
-  CUtensorMap map_try[kTryShapes]{}, map_sure[3]{};   // NC = 16, 32, 64
+  CUtensorMap map_try[kTryShapes]{}, map_sure[kTryShapes]{};
   cudaEvent_t done = nullptr;                    // shared ones: behind the last launch
   uint64_t last_use = 0;
 };
@@ -493,10 +493,11 @@ StreamScratch* scratch_of(GpuScratch& g, cudaStream_t stream, int lane) {
   }
   cudaError_t maps = cudaSuccess;
   uint8_t* const acts = static_cast<uint8_t*>(base);
-  for (int i = 0; i < kTryShapes && maps == cudaSuccess; ++i)
-    maps = hb::encode_rows(&s.map_try[i], acts + try_offset(i), kTryRow[i], acts_bytes(kTryGroups[i], 1), 256);
-  for (int i = 0; i < 3 && maps == cudaSuccess; ++i)
-    maps = hb::encode_rows(&s.map_sure[i], acts + kSureOffset, 32u << i, acts_bytes(kMaxGroups, 128) / (32u << i), 256);
+  for (int i = 0; i < 2 * kTryShapes && maps == cudaSuccess; ++i) {
+    const int shape = i / 2, NC = kTryNC[shape];
+    maps = hb::encode_rows(i % 2 ? &s.map_sure[shape] : &s.map_try[shape], acts + (i % 2 ? kSureOffset : try_offset(shape)),
+                           hb::act_map_row(NC), acts_bytes(kTryGroups[shape], 2 * NC) / hb::act_map_row(NC), hb::act_map_box(NC));
+  }
   if (maps != cudaSuccess) {
     cudaGetLastError();
     cudaFree(base);
@@ -529,17 +530,18 @@ namespace hb {
 //   near               42: 21.5 (one: 17.6)   split    14: 29.5 (one: 27.2)
 //   8 pairs x 16      224: 25.2 (one: 22.5)           112: 32.2 (one: 29.8)
 //   8 pairs x 32      448: 27.2                       224: 35.9
+//   8 pairs x 40      560: 29.2                       280: 38.3   (what 4 pairs x 32 take is 5.6 and 11 more)
 //   4 pairs x 32      960: 34.8                       480: 49.2   (in two row blocks 38.8 and 49.9)
 //   4 pairs x 64    1,920: 44.8                       960: 61.5   (in one row block, exchanged at once, 51.5 and 73.6)
 //   2 pairs x 64    4,224: 64.2                     2,112: 105
 // Blocks without partners (M = 64 or 128 each, all queries of a group in every block; data polled in L2) took 24 for 112,
 // 28 for 240, 32 for 480, 46 for 960, 48 for 1,056 and 73 for 2,112 queries, split 34 for 56, 46 for 240, 78 for 528 and 126
-// for 1,056: better than these only from 100 to 112 and 449 to 480 queries, by 3 and 9 % (split: 225 to 240, 8 %).
+// for 1,056: better than these only from 100 to 112 queries, by 3 %.
 namespace {
 // us: what a launch of the shape takes, full or not
 struct Shape { int pairs, NC, clusters, us, us_split; };   // pairs 0: mlp_near_kernel
-constexpr Shape kShapes[] = {{0, 16, 7, 21, 30}, {8, 16, 7, 25, 32}, {8, 32, 7, 27, 36}, {4, 32, 15, 35, 49},
-                             {4, 64, 15, 45, 62}, {2, 64, 33, 64, 105}};
+constexpr Shape kShapes[] = {{0, 16, 7, 21, 30}, {8, 16, 7, 25, 32}, {8, 32, 7, 27, 36}, {8, 40, 7, 29, 38},
+                             {4, 32, 15, 35, 49}, {4, 64, 15, 45, 62}, {2, 64, 33, 64, 105}};
 int clusters_of(const Shape& s, int sm_count) { return sm_count >= 148 ? s.clusters : s.clusters * sm_count / 148; }
 int cols_of(const Shape& s, bool split) {
   return s.pairs == 0 ? (split ? kNearQ<true> : kNearQ<false>) : (split ? s.NC : 2 * s.NC);
@@ -693,11 +695,11 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
     s->fresh = false;
   }
   if (!w.near) {
-    const int i = w.W == 16 ? 0 : (w.G == 16 ? 1 : (w.G == 4 ? 4 : (w.W == 32 ? 2 : 3)));   // of the shapes with buffers
+    const int i = w.G == 16 ? (w.W == 16 ? 0 : (w.W == 32 ? 1 : 2)) : (w.G == 4 ? 5 : (w.W == 32 ? 3 : 4));   // of the shapes with buffers
     p.acts = s->base + try_offset(i);
     p.map_acts = s->map_try[i];
     p.sure_acts = s->base + kSureOffset;
-    p.map_sure = s->map_sure[w.W / 32];
+    p.map_sure = s->map_sure[i];
     p.expect_stale = s->expect_stale ? 0x80008000u : 0u;
     s->expect_stale = false;
     // exchange `use` (0 .. layers - 1) takes buffer use & 1; every group of the launch flips with it
