@@ -1,7 +1,7 @@
 // MLP inference for batches between a few queries and full rounds of mlp_chain.cu's tiles: clusters of two-SM pairs.
 //
 // mlp_chain.cu gives a pair of SMs 128 queries and streams all weights past them: 103 to 110 us whether the batch has one
-// query or 9,472.  Here P = 8, 4 or 2 pairs form a cluster that owns up to 2 NC queries (NC = 16, 32, 40 or 64; split
+// query or 9,472.  Here P = 8, 4 or 2 pairs form a cluster that owns up to 2 NC queries (NC = 16, 32, 40, 48 or 64; split
 // precision: NC).  Pair i computes 1024 / P output features of every layer for all of them and streams only their
 // weights, and after each layer the cluster exchanges its activations.
 //
@@ -32,16 +32,17 @@
 // cycle, 34; bulk copies that are looked at before they are used 30.  1,920 queries 45.6, with releases 49.2; 4,224 65.1 and
 // 68.2.)
 //
-// NC = 40: rows of 80 bytes fit no swizzle, so B lies in panels of eight columns, 16 bytes a row, and a warp's rows go out as
-// five copies of 512 bytes.  N is a multiple of 32, so the MMAs read a sixth panel per CTA, which is whatever lies behind the
-// fifth; nobody reads the columns of D that come of it.  480 queries: 29.1 us; 34.8 in groups of four pairs.
+// NC = 40, 48: rows of 80 or 96 bytes fit no swizzle, so B lies in panels of eight columns, 16 bytes a row, and a warp's rows go out as
+// five or six copies of 512 bytes.  N is a multiple of 32, so with 40 the MMAs read a sixth panel per CTA, which is whatever
+// lies behind the fifth; nobody reads the columns of D that come of it.  480 queries: 29.1 us in eight pairs with 40, 34.8 in
+// four with 32; 1,056: 41.1 in four pairs with 48, 45.1 with 64.
 //
 // NC = 64: a pair's features are two row blocks, one in K quarters 0 and 1 and one in 2 and 3.  The units (block b, K quarter
 // q) of a layer are issued in the order (0,0) (0,1) (1,0) (0,2) (0,3) | (1,1) (1,2) (1,3): quarters 0 and 1 are
 // exchanged under the last three units and quarters 2 and 3 under the first three of the next layer.  D alternates between two
 // sets of TMEM columns.
 //
-// What bounds it: NC = 16 to 40 the latency of one exchange per layer (P = 8: 2,300 to 2,700 cycles from the last MMA to the next
+// What bounds it: NC = 16 to 48 the latency of one exchange per layer (P = 8: 2,300 to 2,700 cycles from the last MMA to the next
 // layer's first, of which 300 to 500 until the accumulators are there, 350 to take them and write them out, 400 for the
 // store, 400 for the arrivals, 700 for the loads) next to 1,500 of MMAs; NC = 64 shared memory besides: a CTA's weights are
 // written and read once per layer, B is read once per row block, and the exchange writes it, 1.5 MB a layer and CTA for P = 2
@@ -51,7 +52,7 @@
 // have more clusters than fit at a time.
 //
 // Warp roles: 0 TMEM, the mark, activation loads; 1 MMA issuer (the pair's leader); 2-3 weight producers; 4 and more:
-// epilogue; NC = 16 to 40: eight more that look at what has come.  Every wait is bounded, as in mlp_chain.cu; a launch that
+// epilogue; NC = 16 to 48: eight more that look at what has come.  Every wait is bounded, as in mlp_chain.cu; a launch that
 // gave up leaves a mark in the scratch, and launches that find it report an error instead of a result.  After giving up no ring slot is requested again whose
 // copy could be under way: the MMA issuer, whose commits free the slots, waits for the producers of both CTAs to leave
 // before it issues anything past a wait that ran out, and goes no further than the layer's end.
@@ -70,13 +71,13 @@ struct PairShape {
   static constexpr int kBlocks = NC == 64 ? 2 : 1;         // row blocks per pair
   static constexpr int kRows = 512 / P / kBlocks;          // A rows per CTA and block
   static constexpr bool kNarrow = kRows == 64;             // M = 128: D's second half of the columns is in TMEM lanes 64 and up
-  static constexpr bool kPanels = NC == 40;                // B without swizzle, in panels of eight columns
+  static constexpr bool kPanels = NC == 40 || NC == 48;    // B without swizzle, in panels of eight columns
   static constexpr int kN = (2 * NC + 31) / 32 * 32;
   static constexpr int kHalfQ = SPLIT ? NC / 2 : NC;       // queries per CTA at most
   static constexpr int kRowBytes = 2 * NC;
   static constexpr int kActBytes = kWidth * kRowBytes;
   static constexpr int kSlotBytes = kNarrow ? 2 * kTileBytes : kTileBytes;
-  static constexpr int kSlots = (NC == 64 ? 6 : 8) * kTileBytes / kSlotBytes;
+  static constexpr int kSlots = (NC >= 48 ? 6 : 8) * kTileBytes / kSlotBytes;
   static constexpr int kUnitBytes = kRows * 128;           // one K block of the rows
   static constexpr int kImages = kSlotBytes / kUnitBytes;  // per slot
   static constexpr int kParts = SPLIT ? 2 : 1;             // images per packed K block
@@ -146,11 +147,11 @@ __device__ __forceinline__ void commit_pair(uint32_t bar, uint16_t ctas) {
       "h"(ctas)
       : "memory");
 }
-// Byte offset of 16-byte chunk `chunk` of K row k in a B operand of NC columns per CTA (swizzle width 2 NC bytes); NC = 40: in
+// Byte offset of 16-byte chunk `chunk` of K row k in a B operand of NC columns per CTA (swizzle width 2 NC bytes); NC = 40, 48: in
 // panels of `rows` K rows of 16 bytes, 256 in a K quarter.
 template <int NC>
 __device__ __forceinline__ uint32_t b_chunk(uint32_t k, uint32_t chunk, uint32_t rows = 256) {
-  if (NC == 40) return (chunk * rows + k) * 16u;
+  if (NC == 40 || NC == 48) return (chunk * rows + k) * 16u;
   const uint32_t x = NC == 64 ? (k & 7u) : (NC == 32 ? ((k >> 1) & 3u) : ((k >> 2) & 1u));
   return k * (2u * NC) + ((chunk ^ x) << 4);
 }
@@ -404,7 +405,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
       __syncwarp();
     } else if (S::kApart && warp >= 4 + S::kEpiWarps) {
       // ------------------------------ looking at what has been used ------------------------------
-      constexpr int kShare = S::kApart ? S::kActBytes / S::kLookWarps : 0, kBatch = S::kPanels ? 10 : 8;
+      constexpr int kShare = S::kApart ? S::kActBytes / S::kLookWarps : 0, kBatch = NC == 40 ? 10 : 8;
       static_assert(kShare % (512 * kBatch) == 0, "all of it");
       const uint8_t* const mine = base_ptr + (warp - 4 - S::kEpiWarps) * kShare + 16 * lane;
 #pragma unroll 1
@@ -464,7 +465,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
       const int row0 = S::kNarrow ? (quad & 1) * 32 : quad * 32;
       constexpr int kPiece = S::kHalfQ / S::kColGroups;      // queries per warp
       constexpr int kCols = S::kParts * kPiece;
-      const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (S::kNarrow ? 0u : half * NC) +
+      const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (S::kNarrow ? 0u : half * (S::kN / 2)) +
                               static_cast<uint32_t>(part * kCols);
       unsigned long long* const group_halves = p.halves + static_cast<size_t>(group) * 64 * hb::kGroupCols;
       auto rows_sync = [&] {   // the warps of these rows
@@ -661,6 +662,7 @@ cudaError_t launch(int P, int NC, const SmallParams& p, int groups, int device, 
     case 816: return launch<8, 16, SPLIT>(p, groups, device, stream, fits);
     case 840: return launch<8, 40, SPLIT>(p, groups, device, stream, fits);
     case 832: return launch<8, 32, SPLIT>(p, groups, device, stream, fits);
+    case 448: return launch<4, 48, SPLIT>(p, groups, device, stream, fits);
     case 432: return launch<4, 32, SPLIT>(p, groups, device, stream, fits);
     case 464: return launch<4, 64, SPLIT>(p, groups, device, stream, fits);
     default: return launch<2, 64, SPLIT>(p, groups, device, stream, fits);

@@ -8,8 +8,8 @@
 
 namespace hb {
 
-// Tensor maps of mlp_pairs.cu's activations: bytes per row, and rows of a K quarter (256 rows of NC columns; NC = 40 in panels).
-constexpr uint32_t act_map_row(int NC) { return NC == 40 ? 256u : 2u * NC; }
+// Tensor maps of mlp_pairs.cu's activations: bytes per row, and rows of a K quarter (256 rows of NC columns; 40 and 48 in panels).
+constexpr uint32_t act_map_row(int NC) { return NC == 40 || NC == 48 ? 256u : 2u * NC; }
 constexpr uint32_t act_map_box(int NC) { return 512u * NC / act_map_row(NC); }
 constexpr int kGroupCols = 128;    // columns of a group's fc2 sums
 
@@ -106,13 +106,14 @@ __device__ __forceinline__ void give_up(volatile int* abort_flag, int32_t* statu
 }
 template <int W>
 __device__ __forceinline__ void tc_ld_cols(uint32_t taddr, float (&v)[W]) {
-  static_assert(W == 8 || W == 16 || W == 32 || W == 40, "columns per load");
+  static_assert(W == 8 || W == 16 || W == 32 || W == 40 || W == 48, "columns per load");
   if constexpr (W > 32) {
-    float x[32], y[8];
+    float x[32], y[W - 32];
     tc_ld32(taddr, x);
-    tc_ld8(taddr + 32, y);
+    if constexpr (W == 40) tc_ld8(taddr + 32, y);
+    else tc_ld16(taddr + 32, y);
 #pragma unroll
-    for (int i = 0; i < W; ++i) v[i] = i < 32 ? x[i % 32] : y[i % 8];
+    for (int i = 0; i < W; ++i) v[i] = i < 32 ? x[i % 32] : y[i % (W - 32)];
   } else if constexpr (W == 8) tc_ld8(taddr, v);
   else if constexpr (W == 16) tc_ld16(taddr, v);
   else tc_ld32(taddr, v);
