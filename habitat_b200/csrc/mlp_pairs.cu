@@ -35,7 +35,7 @@
 // NC = 40, 48: rows of 80 or 96 bytes fit no swizzle, so B lies in panels of eight columns, 16 bytes a row, and a warp's rows go out as
 // five or six copies of 512 bytes.  N is a multiple of 32, so with 40 the MMAs read a sixth panel per CTA, which is whatever
 // lies behind the fifth; nobody reads the columns of D that come of it.  480 queries: 29.1 us in eight pairs with 40, 34.8 in
-// four with 32; 1,056: 41.1 in four pairs with 48, 45.1 with 64.
+// four with 32; 600: 32.4 in eight with 48; 1,056: 41.1 in four pairs with 48, 45.1 with 64.
 //
 // NC = 64: a pair's features are two row blocks, one in K quarters 0 and 1 and one in 2 and 3.  The units (block b, K quarter
 // q) of a layer are issued in the order (0,0) (0,1) (1,0) (0,2) (0,3) | (1,1) (1,2) (1,3): quarters 0 and 1 are
@@ -85,7 +85,7 @@ struct PairShape {
   static constexpr int kUnitSlots = 4 * kParts / kImages;
   // A K quarter of the activations is counted on the barrier of the slot that it is used with.
   static constexpr bool kApart = kBlocks == 1;             // there is room for the rows on their way out
-  static constexpr bool kJoint = kApart && kNarrow && !SPLIT;
+  static constexpr bool kJoint = kApart && kNarrow && !SPLIT && kSlots == kUnits;
   static constexpr int kColGroups = NC == 64 ? 2 : 1;      // epilogue warps that share 32 rows
   static constexpr int kEpiWarps = (kNarrow ? 4 : 8) * kColGroups;
   static constexpr int kStores = kNarrow ? 4 : 8;          // bulk stores per block and CTA
@@ -661,6 +661,7 @@ cudaError_t launch(int P, int NC, const SmallParams& p, int groups, int device, 
   switch (P * 100 + NC) {
     case 816: return launch<8, 16, SPLIT>(p, groups, device, stream, fits);
     case 840: return launch<8, 40, SPLIT>(p, groups, device, stream, fits);
+    case 848: return launch<8, 48, SPLIT>(p, groups, device, stream, fits);
     case 832: return launch<8, 32, SPLIT>(p, groups, device, stream, fits);
     case 448: return launch<4, 48, SPLIT>(p, groups, device, stream, fits);
     case 432: return launch<4, 32, SPLIT>(p, groups, device, stream, fits);

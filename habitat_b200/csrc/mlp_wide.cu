@@ -418,9 +418,10 @@ constexpr int kMaxStreams = 16, kMoreStreams = 16;
 constexpr int kMaxGroups = 34;
 // Activation buffers of mlp_pairs.cu: one for the first runs of each shape (a word's parity counts its own uses), and one that
 // all shapes use for second runs.
-constexpr int kTryShapes = 7;                           // of kShapes, after the first
+constexpr int kTryShapes = 8;                           // of kShapes, after the first
 constexpr size_t acts_bytes(int groups, int row_bytes) { return static_cast<size_t>(groups) * 4 * kWidth * row_bytes; }
-constexpr int kTryGroups[kTryShapes] = {8, 8, 8, 16, 16, 16, kMaxGroups}, kTryNC[kTryShapes] = {16, 32, 40, 32, 48, 64, 64};
+constexpr int kTryGroups[kTryShapes] = {8, 8, 8, 8, 16, 16, 16, kMaxGroups};
+constexpr int kTryNC[kTryShapes] = {16, 32, 40, 48, 32, 48, 64, 64};
 constexpr size_t try_offset(int shape) {
   return shape ? try_offset(shape - 1) + acts_bytes(kTryGroups[shape - 1], 2 * kTryNC[shape - 1]) : 0;
 }
@@ -531,6 +532,7 @@ namespace hb {
 //   8 pairs x 16      224: 25.2 (one: 22.5)           112: 32.2 (one: 29.8)
 //   8 pairs x 32      448: 27.2                       224: 35.9
 //   8 pairs x 40      560: 29.2                       280: 38.3   (what 4 pairs x 32 take is 5.6 and 11 more)
+//   8 pairs x 48      672: 32.4                       336: 42.6
 //   4 pairs x 32      960: 34.8                       480: 49.2   (in two row blocks 38.8 and 49.9)
 //   4 pairs x 48    1,440: 41.1                       720: 59.4
 //   4 pairs x 64    1,920: 44.8                       960: 61.5   (in one row block, exchanged at once, 51.5 and 73.6)
@@ -539,9 +541,9 @@ namespace hb {
 // 28 for 240, 32 for 480, 46 for 960, 48 for 1,056 and 73 for 2,112 queries, split 34 for 56, 46 for 240, 78 for 528 and 126
 // for 1,056: better than these only from 100 to 112 queries, by 3 %.
 namespace {
-// us: what a launch of the shape takes, full or not
+// us: what a launch of the shape takes, full or not.  The ones with pairs are in the order of kTryNC.
 struct Shape { int pairs, NC, clusters, us, us_split; };   // pairs 0: mlp_near_kernel
-constexpr Shape kShapes[] = {{0, 16, 7, 21, 30}, {8, 16, 7, 25, 32}, {8, 32, 7, 27, 36}, {8, 40, 7, 29, 38},
+constexpr Shape kShapes[] = {{0, 16, 7, 21, 30}, {8, 16, 7, 25, 32}, {8, 32, 7, 27, 36}, {8, 40, 7, 29, 38}, {8, 48, 7, 32, 42},
                              {4, 32, 15, 35, 49}, {4, 48, 15, 41, 59},
                              {4, 64, 15, 45, 62}, {2, 64, 33, 64, 105}};
 int clusters_of(const Shape& s, int sm_count) { return sm_count >= 148 ? s.clusters : s.clusters * sm_count / 148; }
@@ -697,8 +699,8 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
     s->fresh = false;
   }
   if (!w.near) {
-    // of the shapes with buffers
-    const int i = w.G == 16 ? (w.W == 16 ? 0 : (w.W == 32 ? 1 : 2)) : (w.G == 4 ? 6 : (w.W == 32 ? 3 : (w.W == 48 ? 4 : 5)));
+    int i = 0;   // of the shapes with buffers
+    while (i < kTryShapes - 1 && (2 * kShapes[i + 1].pairs != w.G || kShapes[i + 1].NC != w.W)) ++i;
     p.acts = s->base + try_offset(i);
     p.map_acts = s->map_try[i];
     p.sure_acts = s->base + kSureOffset;

@@ -625,8 +625,8 @@ print(want.tobytes().hex()[:200])
     assert outs[0] == outs[1]
 
 
-@pytest.mark.parametrize("precision,edges", [("bf16", (28, 224, 448, 560, 960, 1440, 1920, 4224)),
-                                             ("bf16x3", (14, 112, 224, 280, 480, 720, 960, 2112))])
+@pytest.mark.parametrize("precision,edges", [("bf16", (28, 224, 448, 560, 672, 960, 1440, 1920, 4224)),
+                                             ("bf16x3", (14, 112, 224, 280, 336, 480, 720, 960, 2112))])
 @pytest.mark.parametrize("layers", [1, 2, 3, 8])
 def test_clusters_of_pairs(precision, edges, layers):
     """Each shape of the kernel for clusters of SM pairs at both ends of its range, with groups that are not
