@@ -32,9 +32,9 @@
 // cycle, 34; bulk copies that are looked at before they are used 30.  1,920 queries 45.6, with releases 49.2; 4,224 65.1 and
 // 68.2.)
 //
-// NC = 40, 48: rows of 80 or 96 bytes fit no swizzle, so B lies in panels of eight columns, 16 bytes a row, and a warp's rows go out as
-// five or six copies of 512 bytes.  N is a multiple of 32, so with 40 the MMAs read a sixth panel per CTA, which is whatever
-// lies behind the fifth; nobody reads the columns of D that come of it.  480 queries: 29.1 us in eight pairs with 40, 34.8 in
+// NC = 40, 48: rows of 80 or 96 bytes fit no swizzle, so B lies in panels of eight columns, 16 bytes a row, and a warp's rows go
+// out as five or six copies of 512 bytes.  N is a multiple of 32, so with 40 the MMAs read a sixth panel per CTA, which is
+// whatever lies behind the fifth; nobody reads the columns of D that come of it.  480 queries: 29.1 us in eight pairs with 40, 34.8 in
 // four with 32; 600: 32.4 in eight with 48; 1,056: 41.1 in four pairs with 48, 45.1 with 64.
 //
 // NC = 64: a pair's features are two row blocks, one in K quarters 0 and 1 and one in 2 and 3.  The units (block b, K quarter
