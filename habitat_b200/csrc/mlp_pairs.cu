@@ -178,7 +178,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
   const uint32_t bar_q1 = bars + 232;       // two blocks: quarter 1 has been read
   const uint32_t bar_seen = bars + 240;     // first run: the layer's input has been looked at
   const uint32_t bar_drain = bars + 248;    // leader only, after giving up: the MMAs have ended
-  const uint32_t bar_out = bars + 256;      // kApart: the layer's output is on its way (kEpiWarps)
+  const uint32_t bar_out = bars + 256;      // kApart: the output of a layer after the first is on its way (kEpiWarps)
   constexpr int kBars = 33;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_ptr + 288);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + 292);
@@ -409,10 +409,9 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
       static_assert(kShare % (512 * kBatch) == 0, "all of it");
       const uint8_t* const mine = base_ptr + (warp - 4 - S::kEpiWarps) * kShare + 16 * lane;
 #pragma unroll 1
-      for (int L = 0; L < n_layers && start && !sure; ++L) {
+      for (int L = 1; L < n_layers && start && !sure; ++L) {
         // (not while the epilogue is at it: it took 500 cycles instead of 220)
-        if (!pairs_wait(bar_out, L & 1, abort_flag, p, 0x551)) break;
-        if (L == 0) continue;
+        if (!pairs_wait(bar_out, (L - 1) & 1, abort_flag, p, 0x551)) break;
         const uint32_t want = signs_of(L - 1) ^ p.expect_stale;
         uint32_t bad = 0;
 #pragma unroll 1
@@ -566,7 +565,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
                 st_relaxed_u64(h + i, static_cast<unsigned long long>(tag) << 32 | __float_as_uint(sum[i]));
             }
           }
-          if (S::kApart) {
+          if (S::kApart && L > 0) {   // (each phase waits for the look of the one before: no parity comes round unseen)
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_out);
           }

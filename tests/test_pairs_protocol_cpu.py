@@ -1,0 +1,84 @@
+"""The barriers of the kernel for clusters of SM pairs (habitat_b200/csrc/mlp_pairs.cu), as a model: every order in which
+the roles of a block can run and copies and commits can land, for a block with rows of its own for what goes out.
+
+A wait on a barrier's parity passes while the phase under way has the other parity, so a role that sleeps through two
+phases waits for a third one.  No order may leave the roles waiting."""
+import pytest
+
+SLOTS, SLOTS_PER_LAYER = 2, 2
+
+
+def _roles(layers, looked_from):
+    """What each role does, in order: ("wait", barrier, phase), ("arrive", barrier), or ("later", barrier) for an arrival
+    that comes when a copy has landed or the MMAs have ended.  looked_from: the first layer whose output is announced
+    to the warps that look at what has come."""
+    n_layers, loads = layers + 1, 1 + layers * SLOTS_PER_LAYER
+    producer, issuer, loader, epilogue, look = [], [], [], [], []
+    for n in range(loads):
+        if n >= SLOTS:
+            producer.append(("wait", "empty%d" % (n % SLOTS), n // SLOTS - 1))
+        producer.append(("later", "full%d" % (n % SLOTS)))
+    n = 0
+    for L in range(n_layers):
+        if L > 0:
+            issuer.append(("wait", "act", L - 1))
+        for _ in range(1 if L == 0 else SLOTS_PER_LAYER):
+            issuer += [("wait", "full%d" % (n % SLOTS), n // SLOTS), ("later", "empty%d" % (n % SLOTS))]
+            n += 1
+        issuer.append(("later", "acc"))
+        epilogue.append(("wait", "acc", L))
+        if L >= looked_from:
+            epilogue.append(("arrive", "out"))
+            look.append(("wait", "out", L - looked_from))
+        if L > 0:
+            look.append(("arrive", "seen"))
+        if L < layers:
+            epilogue.append(("later", "signal%d" % (L & 1)))
+            loader.append(("wait", "acc", L))
+            if L > 0:
+                loader.append(("wait", "seen", L - 1))
+            loader += [("wait", "signal%d" % (L & 1), L // 2), ("later", "act")]
+    return producer, issuer, loader, epilogue, look
+
+
+def _stuck(roles):
+    """A state from which nothing can go on although some role has not ended, or None."""
+    start = ((0,) * len(roles), (), ())
+    seen, todo = {start}, [start]
+    while todo:
+        at, phases, coming = todo.pop()
+        done = dict(phases)
+        steps = []
+        for i, ops in enumerate(roles):
+            if at[i] == len(ops):
+                continue
+            op = ops[at[i]]
+            if op[0] == "wait" and (done.get(op[1], 0) & 1) == (op[2] & 1):
+                continue
+            moved = at[:i] + (at[i] + 1,) + at[i + 1:]
+            if op[0] == "arrive":
+                steps.append((moved, {**done, op[1]: done.get(op[1], 0) + 1}, coming))
+            else:
+                steps.append((moved, done, tuple(sorted(coming + (op[1],))) if op[0] == "later" else coming))
+        for bar in set(coming):
+            left = list(coming)
+            left.remove(bar)
+            steps.append((at, {**done, bar: done.get(bar, 0) + 1}, tuple(left)))
+        if not steps and any(a < len(ops) for a, ops in zip(at, roles)):
+            return at
+        for moved, done, left in steps:
+            state = (moved, tuple(sorted(done.items())), left)
+            if state not in seen:
+                seen.add(state)
+                todo.append(state)
+    return None
+
+
+@pytest.mark.parametrize("layers", [1, 2, 3, 4])
+def test_no_order_leaves_the_roles_waiting(layers):
+    assert _stuck(_roles(layers, looked_from=1)) is None
+
+
+def test_an_announcement_that_nobody_answers_can_be_missed():
+    """The output of fc1 is not announced: nothing waits for a look at it, so the next announcement could come first."""
+    assert _stuck(_roles(3, looked_from=0)) is not None
