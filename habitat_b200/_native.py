@@ -117,6 +117,7 @@ EXPORTS = {
     "hb_special_scale_grid": (ctypes.c_int32, [ctypes.POINTER(ScaleGrid), ctypes.c_int32, ctypes.c_void_p]),
     "hb_mlp_status": (ctypes.c_int32, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int32)]),
     "hb_mlp_inject_mark": (ctypes.c_int32, [ctypes.c_void_p]),
+    "hb_mlp_inject_mark_at": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_int32]),
     "hb_mlp_inject_stale": (ctypes.c_int32, [ctypes.c_void_p]),
     "hb_mlp_phase_cycles": (ctypes.c_int32, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int64)]),
     "hb_mlp_predict_host": (ctypes.c_int32, [

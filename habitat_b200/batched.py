@@ -308,10 +308,13 @@ class MLPHandle:
         """Writes the device status word from the host (tests of the error path)."""
         _native.check(_native.load().hb_mlp_inject_status(self._handle, int(code)))
 
-    def inject_mark(self):
+    def inject_mark(self, block=None):
         """Leaves, from the host, the mark of a small-batch launch that gave up (tests of the error path): the next
-        such launch on this GPU reports an error instead of results."""
-        _native.check(_native.load().hb_mlp_inject_mark(self._handle))
+        such launch on this GPU reports an error instead of results.  With `block` only the block of that rank in each
+        cluster heeds it."""
+        lib = _native.load()
+        _native.check(lib.hb_mlp_inject_mark(self._handle) if block is None
+                      else lib.hb_mlp_inject_mark_at(self._handle, int(block)))
 
     def inject_stale(self):
         """Makes the next small-batch launch of each stream on this GPU take what its blocks exchange for stale (tests):

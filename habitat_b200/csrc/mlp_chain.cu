@@ -1165,7 +1165,16 @@ extern "C" hb_status hb_mlp_inject_mark(hb_mlp* h) {
     return HB_ERR_INVALID_ARGUMENT;
   }
   const hb_status st = check_device(h);
-  return st != HB_OK ? st : hb::wide_set_mark(h->device);
+  return st != HB_OK ? st : hb::wide_set_mark(h->device, 1);
+}
+
+extern "C" hb_status hb_mlp_inject_mark_at(hb_mlp* h, int32_t block) {
+  if (!h || block < 0) {
+    hb::set_error("hb_mlp_inject_mark_at: bad arguments");
+    return HB_ERR_INVALID_ARGUMENT;
+  }
+  const hb_status st = check_device(h);
+  return st != HB_OK ? st : hb::wide_set_mark(h->device, ~block);
 }
 
 extern "C" hb_status hb_mlp_inject_stale(hb_mlp* h) {

@@ -240,7 +240,6 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
   constexpr uint32_t kSigns = SPLIT ? 0x80000000u : 0x80008000u;   // those that carry the parity
   float result = 0.0f;
 
-  bool start = true;     // a CTA that gave up takes no part in a second run
   // sure: with releases; the first run goes without
 #pragma unroll 1
   for (bool sure = false;; sure = true) {
@@ -252,9 +251,9 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
     const uint32_t tag = sure ? p.tag | 0x80000000u : p.tag;
     if (warp == 0) {
       // ------------------------------ the mark; activation loads ------------------------------
-      if (lane == 0 && start) {
+      if (lane == 0) {
         // An earlier launch that gave up may still be writing: report, and give up as well (no result is stored then).
-        if (*reinterpret_cast<volatile int32_t*>(p.poison) != 0) {
+        if (hb::concerns(*reinterpret_cast<volatile int32_t*>(p.poison), cta)) {
           *static_cast<volatile int32_t*>(p.status) = 0x5FF;
           *abort_flag = 1;
         }
@@ -288,7 +287,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
       __syncwarp();
     } else if (warp == 2 || warp == 3) {
       // ------------------------------ weight producers ------------------------------
-      if (lane == 0 && start) {
+      if (lane == 0) {
         const uint32_t w = static_cast<uint32_t>(warp - 2);
         constexpr uint32_t kLayerLoads = S::kUnits * S::kUnitSlots;
         const uint32_t loads = S::kBlocks + static_cast<uint32_t>(p.layers) * kLayerLoads;
@@ -334,10 +333,10 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
       constexpr uint32_t kQuarterB = (256 * S::kRowBytes) >> 4;
       const uint32_t a_lo0 = (ring & 0x3FFFF) >> 4, b_lo0 = (act & 0x3FFFF) >> 4;
       // One elected lane runs the whole loop, and no loop of a layer depends on what a wait returns (after a wait that
-      // ran out the abort flag is set, and what is issued on stale operands is discarded), which keeps the descriptors in
+      // ran out the abort flag is set, and nothing that comes of stale operands is stored as a result), which keeps the descriptors in
       // uniform registers.  A try_wait holds up the issue for 90 cycles, so with M = 128 (21 to 32 cycles per MMA) slots
       // last 16 MMAs: with 8 an MMA took 33 cycles whatever N, with 16 it takes 23 to 25.
-      if (r == 0 && start && elect_one()) {
+      if (r == 0 && elect_one()) {
         auto wait = [&](uint32_t bar, uint32_t parity, int code) {
           if (!mbar_try_wait(bar, parity) && (*abort_flag || !pairs_wait(bar, parity, abort_flag, p, code))) {
             // (the producers look at their CTA's abort flag when a slot does not come)
@@ -409,7 +408,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
       static_assert(kShare % (512 * kBatch) == 0, "all of it");
       const uint8_t* const mine = base_ptr + (warp - 4 - S::kEpiWarps) * kShare + 16 * lane;
 #pragma unroll 1
-      for (int L = 1; L < n_layers && start && !sure; ++L) {
+      for (int L = 1; L < n_layers && !sure; ++L) {
         // (not while the epilogue is at it: it took 500 cycles instead of 220)
         if (!pairs_wait(bar_out, (L - 1) & 1, abort_flag, p, 0x551)) break;
         const uint32_t want = signs_of(L - 1) ^ p.expect_stale;
@@ -431,31 +430,29 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
       // ------------------------------ epilogue ------------------------------
       constexpr int kEpiThreads = 32 * S::kEpiWarps;
       const int T = static_cast<int>(threadIdx.x) - 128;
-      if (start) {
-        // fc1's B operand: K rows 0..63 hold [hi | lo | hi] of the normalised features, one query per column (split: the
-        // second of its two, see below)
-        auto feat_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory"); };
-        const int C_in = p.n_op_feat + 4;
-        for (int i = T; i < 64 * S::kRowBytes / 16; i += kEpiThreads)
-          *reinterpret_cast<uint4*>(base_ptr + (S::kPanels ? b_chunk<NC>(i & 63, i >> 6) : 16 * i)) = make_uint4(0, 0, 0, 0);
-        feat_sync();
-        for (int i = T; i < n_q * C_in; i += kEpiThreads) {
-          const int q = i / C_in, f = i - q * C_in;
-          __nv_bfloat16 hi, lo;
-          load_feature(p, static_cast<int>(q0) + q, f, hi, lo);
-          const uint32_t col = static_cast<uint32_t>(SPLIT ? 2 * q + 1 : q), ch = col >> 3, in = 2u * (col & 7u);
-          *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<NC>(f, ch) + in) = hi;
-          *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<NC>(C_in + f, ch) + in) = lo;
-          *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<NC>(2 * C_in + f, ch) + in) = hi;
-        }
-        fence_proxy_async();
-        feat_sync();
-        if (T == 0) {
-          if (r == 0) mbar_arrive(bar_feat);
-          else mbar_arrive_remote(map_to_cta(bar_feat, leader));
-        }
-        __syncwarp();
+      // fc1's B operand: K rows 0..63 hold [hi | lo | hi] of the normalised features, one query per column (split: the
+      // second of its two, see below)
+      auto feat_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory"); };
+      const int C_in = p.n_op_feat + 4;
+      for (int i = T; i < 64 * S::kRowBytes / 16; i += kEpiThreads)
+        *reinterpret_cast<uint4*>(base_ptr + (S::kPanels ? b_chunk<NC>(i & 63, i >> 6) : 16 * i)) = make_uint4(0, 0, 0, 0);
+      feat_sync();
+      for (int i = T; i < n_q * C_in; i += kEpiThreads) {
+        const int q = i / C_in, f = i - q * C_in;
+        __nv_bfloat16 hi, lo;
+        load_feature(p, static_cast<int>(q0) + q, f, hi, lo);
+        const uint32_t col = static_cast<uint32_t>(SPLIT ? 2 * q + 1 : q), ch = col >> 3, in = 2u * (col & 7u);
+        *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<NC>(f, ch) + in) = hi;
+        *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<NC>(C_in + f, ch) + in) = lo;
+        *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<NC>(2 * C_in + f, ch) + in) = hi;
       }
+      fence_proxy_async();
+      feat_sync();
+      if (T == 0) {
+        if (r == 0) mbar_arrive(bar_feat);
+        else mbar_arrive_remote(map_to_cta(bar_feat, leader));
+      }
+      __syncwarp();
       // A warp drains 32 rows (features) of one half of the columns, or a part of them (kColGroups).  Split precision: a
       // query has two columns, of the lo and the hi part of its activations: one 32-bit word in a row of B.
       const int quad = warp & 3, rest = (warp - 4) >> 2;
@@ -488,7 +485,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_seen);
       };
-      bool ok = start;
+      bool ok = true;
       // a wait that ran out skips the work that is left but none of the barriers
 #pragma unroll 1
       for (int L = 0; L < n_layers; ++L) {
@@ -606,14 +603,19 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         result = tots[T & 63] + tots[64 + (T & 63)] + p.fc2_b;
       }
     }
-    // No CTA leaves while another may still signal to it, and all have looked at everything.  (Flags that another CTA
-    // has to see were followed by a fence.)
+    // No CTA leaves while another may still signal to it, all have looked at everything, and all know whether one gave up: what
+    // it has sent since may be anything, a last layer with its sums included, so then no CTA stores a result or runs again, and all
+    // go through the teardown.  (Flags that another CTA has to see were followed by a fence.)
     tc_fence_before();
+    __syncwarp();
+    if (lane == 0 && *abort_flag) {
+      for (uint32_t c = 0; c < S::kCtas; ++c) st_cluster_u32(map_to_cta(bars + 292, c), 1u);
+      __threadfence();
+    }
     __syncwarp();
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     tc_fence_after();
-    if (sure || *stale == 0) break;
-    start = *abort_flag == 0;   // (nobody sets it between the two barriers)
+    if (sure || *abort_flag || *stale == 0) break;   // (nobody sets them between the two barriers)
     if (threadIdx.x == 0) {
       for (int i = 0; i < kBars; ++i) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bars + 8 * i) : "memory");
       init_barriers();

@@ -30,7 +30,7 @@ struct SmallParams {
   uint8_t* acts;              // [groups][2 buffers][2 halves][1024 K rows][row bytes] with parities, and another without
   uint8_t* sure_acts;         // (mlp_pairs.cu)
   unsigned long long* halves; // [groups][64 sets of 16 features][kGroupCols]: fc2 sum, tag
-  int32_t* poison;            // set by a launch that gave up
+  int32_t* poison;            // set by a launch that gave up; below zero: block ~poison of each group alone heeds it (tests)
   uint32_t tag;               // of this launch
   uint32_t expect_stale;      // 0x80008000: every word of the first run is taken for stale (tests)
   unsigned long long parity[2];   // bit g: parity of the next use of group g's buffer 0, 1 (mlp_pairs.cu)
@@ -45,6 +45,8 @@ struct SmallParams {
   CUtensorMap map_fc1;        // one K block of the block's rows
   CUtensorMap map_acts, map_sure;   // 256 rows of acts, of sure_acts
 };
+
+inline __device__ bool concerns(int32_t poison, uint32_t block) { return poison > 0 || (poison < 0 && ~poison == static_cast<int32_t>(block)); }
 
 // Launches `groups` clusters of `ctas` blocks; *fits = false (nothing launched) where the GPU cannot hold one.
 template <typename Kernel>

@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
     // An earlier launch that gave up may still be writing: report, and give up as well (no result is
     // stored then).  Only that result waits for the mark, whose load takes 700 cycles.
     if (lane == 0) {
-      if (*reinterpret_cast<volatile int32_t*>(p.poison) != 0) {
+      if (hb::concerns(*reinterpret_cast<volatile int32_t*>(p.poison), static_cast<uint32_t>(c))) {
         *static_cast<volatile int32_t*>(p.status) = 0x5FF;
         *abort_flag = 1;
       }
@@ -644,13 +644,13 @@ void wide_start_over(int device) {
   for (int i = 0; i < g.used; ++i) g.s[i].fresh = true;
 }
 
-hb_status wide_set_mark(int device) {
+hb_status wide_set_mark(int device, int32_t mark) {
   if (device < 0 || device >= kMaxCudaDevices) return HB_OK;
   GpuScratch& g = g_wide[device];
   std::lock_guard<std::mutex> lock(g.mu);
   HB_CUDA_TRY(cudaDeviceSynchronize());
   for (int i = 0; i < g.used; ++i)
-    HB_CUDA_TRY(cudaMemset(g.s[i].base + kActsBytes + kHalvesBytes, 1, sizeof(int32_t)));
+    HB_CUDA_TRY(cudaMemcpy(g.s[i].base + kActsBytes + kHalvesBytes, &mark, sizeof(mark), cudaMemcpyHostToDevice));
   HB_CUDA_TRY(cudaDeviceSynchronize());
   return HB_OK;
 }

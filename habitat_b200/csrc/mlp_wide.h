@@ -54,8 +54,9 @@ std::unique_lock<std::mutex> wide_queue(int device);
 hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cudaStream_t stream, bool* launched);
 // After a launch that gave up: every stream's scratch on the GPU is set up again before its next use.
 void wide_start_over(int device);
-// Leaves the mark of a launch that gave up in the GPU's scratch (tests of the error path); synchronises.
-hb_status wide_set_mark(int device);
+// Leaves the mark of a launch that gave up in the GPU's scratch (tests of the error path): 1, or ~b for block b of each group
+// alone; synchronises.
+hb_status wide_set_mark(int device, int32_t mark);
 // The next launch on each stream of the GPU that tries to do without releases takes what it exchanges for stale (tests).
 void wide_expect_stale(int device);
 void wide_handle_created(int device);

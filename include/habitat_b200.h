@@ -261,6 +261,9 @@ hb_status hb_mlp_inject_status(hb_mlp* handle, int32_t device_status);
  * then store no result and report device status 0x5ff, until a status has been read.
  * Synchronises.  No reference counterpart. */
 hb_status hb_mlp_inject_mark(hb_mlp* handle);
+/* The same mark, but heeded by one thread block (its rank in each cluster) alone, as if that block
+ * had given up by itself. */
+hb_status hb_mlp_inject_mark_at(hb_mlp* handle, int32_t block);
 
 /* The next small-batch launch on each stream that has had one, on the handle's GPU, takes what its
  * blocks exchange for stale and runs the network once more, the slower way (test hook; the

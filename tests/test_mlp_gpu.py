@@ -233,6 +233,34 @@ def test_launches_that_find_the_mark_of_one_that_gave_up(precision, sizes):
     h.close()
 
 
+@pytest.mark.parametrize("precision,sizes", [("bf16", (100, 300, 500, 600, 900, 1200, 1700, 2000)),
+                                             ("bf16x3", (50, 200, 250, 300, 400, 600, 900, 1000))])
+def test_no_result_when_one_block_has_given_up(precision, sizes):
+    """Each shape of the kernel for clusters of SM pairs: one block gives up, the second one
+    of a pair without queries of the last sums, so that everybody else goes on to the end.  No block stores a result, and
+    the launch ends as a whole."""
+    from habitat_b200 import _native
+    w = workloads.init_mlp_weights("linear", seed=31, gain=2.0, layers=2)
+    feats, dev = workloads.make_queries("linear", max(sizes), 53)
+    mu, sigma = workloads.batch_mu_sigma(feats, dev)
+    h = batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=DEVF, precision=precision, **w)
+    d_f, d_r = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()
+    for Q in sizes:
+        f, r, out = d_f[:Q].contiguous(), d_r[:Q].contiguous(), torch.empty((Q,), device="cuda")
+        want = h.predict(f, r).clone()
+        h.check_status()
+        h.inject_mark(block=3)
+        out.fill_(-7.0)
+        h.predict(f, r, out=out)
+        torch.cuda.synchronize()
+        assert (out == -7.0).all(), Q
+        with pytest.raises(_native.HabitatNativeError):
+            h.check_status()
+        assert torch.equal(h.predict(f, r), want), Q
+        h.check_status()
+    h.close()
+
+
 @pytest.mark.parametrize("width,layers", [(256, 3), (1000, 2), (64, 1)])
 def test_other_layer_sizes(width, layers):
     """RuntimePredictor(model_name, layers, layer_size) takes any size in the reference
