@@ -300,6 +300,8 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
       const float bias = __ldg(p.bias + L * kWidth + f);
       const float w2 = last ? __ldg(p.fc2_w + f) : 0.0f;
       ok = ok && warp_wait(bar_acc, L & 1, lane, abort_flag, p, 0x541);
+      // (an issuer that gave up has gone on to the layer's end: sums that are not there stop the block that adds them)
+      if (last) ok = __shfl_sync(0xFFFFFFFFu, ok && *abort_flag == 0 ? 1 : 0, 0) != 0;
       if (!ok) {
         if (!last) epi_sync();
         continue;
