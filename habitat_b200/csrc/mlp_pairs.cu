@@ -283,6 +283,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
                         map_to_cta(bar, leader));
           }
         }
+        if (S::kBlocks == 2 && ok) pairs_wait(bar_q1, (p.layers - 1) & 1, abort_flag, p, 0x533);   // as the last slots below
       }
       __syncwarp();
     } else if (warp == 2 || warp == 3) {
@@ -291,7 +292,9 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         const uint32_t w = static_cast<uint32_t>(warp - 2);
         constexpr uint32_t kLayerLoads = S::kUnits * S::kUnitSlots;
         const uint32_t loads = S::kBlocks + static_cast<uint32_t>(p.layers) * kLayerLoads;
-        for (uint32_t n = w; n < loads; n += 2) {
+        // and at the end every slot's last commit: it may still be on its way to this CTA when the layer's is there, and the
+        // barriers start over, or the shared memory is somebody else's
+        for (uint32_t n = w; n < loads + S::kSlots; n += 2) {
           const bool fc1 = n < S::kBlocks;
           const uint32_t m = n - S::kBlocks, L = m / kLayerLoads, u = m % kLayerLoads / S::kUnitSlots, g = m % S::kUnitSlots;
           const uint32_t unit = S::kBlocks == 2 ? (kQuadOrder >> (4 * u)) & 15u : u, kq = unit & 3u;
@@ -303,6 +306,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
           const uint32_t s = n % S::kSlots, ph = (n / S::kSlots & 1u) ^ 1u;
           const uint32_t full = bar_full + 8 * s, full_leader = map_to_cta(full, leader), dst = ring + s * S::kSlotBytes;
           if (!pairs_wait(bar_empty + 8 * s, ph, abort_flag, p, 0x511)) break;
+          if (n >= loads) continue;
           if (r == 0) mbar_expect_tx(full, 2 * (fc1 ? S::kUnitBytes : S::kSlotBytes));
           if (S::kJoint && r == 0 && fc1) mbar_arrive(full);
           if (S::kNarrow) tma_3d_pair(dst, fc1 ? &p.map_fc1 : &p.map_slot, r * S::kRows, image, full_leader);
