@@ -234,6 +234,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
   // first output feature of the pair's row block b, as a K index of the next layer
   auto block_feature = [&](int b) { return b * 512 + pair * (2 * S::kRows); };
   auto saw_stale = [&] {
+#pragma unroll 1
     for (uint32_t c = 0; c < S::kCtas; ++c) st_cluster_u32(map_to_cta(bars + 296, c), 1u);
     __threadfence();
   };
@@ -292,9 +293,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         const uint32_t w = static_cast<uint32_t>(warp - 2);
         constexpr uint32_t kLayerLoads = S::kUnits * S::kUnitSlots;
         const uint32_t loads = S::kBlocks + static_cast<uint32_t>(p.layers) * kLayerLoads;
-        // and at the end every slot's last commit: it may still be on its way to this CTA when the layer's is there, and the
-        // barriers start over, or the shared memory is somebody else's
-        for (uint32_t n = w; n < loads + S::kSlots; n += 2) {
+        for (uint32_t n = w; n < loads; n += 2) {
           const bool fc1 = n < S::kBlocks;
           const uint32_t m = n - S::kBlocks, L = m / kLayerLoads, u = m % kLayerLoads / S::kUnitSlots, g = m % S::kUnitSlots;
           const uint32_t unit = S::kBlocks == 2 ? (kQuadOrder >> (4 * u)) & 15u : u, kq = unit & 3u;
@@ -306,12 +305,15 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
           const uint32_t s = n % S::kSlots, ph = (n / S::kSlots & 1u) ^ 1u;
           const uint32_t full = bar_full + 8 * s, full_leader = map_to_cta(full, leader), dst = ring + s * S::kSlotBytes;
           if (!pairs_wait(bar_empty + 8 * s, ph, abort_flag, p, 0x511)) break;
-          if (n >= loads) continue;
           if (r == 0) mbar_expect_tx(full, 2 * (fc1 ? S::kUnitBytes : S::kSlotBytes));
           if (S::kJoint && r == 0 && fc1) mbar_arrive(full);
           if (S::kNarrow) tma_3d_pair(dst, fc1 ? &p.map_fc1 : &p.map_slot, r * S::kRows, image, full_leader);
           else tma_2d_pair(dst, &p.map_slot, image * kMTile, full_leader);
         }
+        // Every slot's last commit: it may still be on its way to this CTA when the layer's is there, and the barriers start over,
+        // or the shared memory is somebody else's.
+        for (uint32_t n = loads + w; n < loads + S::kSlots && *abort_flag == 0; n += 2)
+          pairs_wait(bar_empty + 8 * (n % S::kSlots), (n / S::kSlots & 1u) ^ 1u, abort_flag, p, 0x512);
         st_cluster_u32(map_to_cta(bars + 304 + 4 * (2 * r + w), leader), 1u);
       }
       __syncwarp();
@@ -596,7 +598,6 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
           // Block 0 has used all of the layer's input.  What the blocks' rows are not written over is looked at now.
           if (!S::kApart && b == 0 && L > 0 && ok && !sure) look(want, 2 * S::kRows);
         }
-        if (!S::kApart && last && ok && !sure) look(want, 0);
       }
       if (cta < 2 && warp < 8) {
         // the first CTA of each half adds the 64 sets of 16 features of its queries
@@ -613,6 +614,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
     tc_fence_before();
     __syncwarp();
     if (lane == 0 && *abort_flag) {
+#pragma unroll 1
       for (uint32_t c = 0; c < S::kCtas; ++c) st_cluster_u32(map_to_cta(bars + 292, c), 1u);
       __threadfence();
     }

@@ -300,8 +300,6 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
       const float bias = __ldg(p.bias + L * kWidth + f);
       const float w2 = last ? __ldg(p.fc2_w + f) : 0.0f;
       ok = ok && warp_wait(bar_acc, L & 1, lane, abort_flag, p, 0x541);
-      // (an issuer that gave up has gone on to the layer's end: sums that are not there stop the block that adds them)
-      if (last) ok = __shfl_sync(0xFFFFFFFFu, ok && *abort_flag == 0 ? 1 : 0, 0) != 0;
       if (!ok) {
         if (!last) epi_sync();
         continue;
@@ -350,11 +348,12 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
         }
         __syncwarp();
       } else {
+        const int gave_up = *abort_flag;   // an issuer that did has gone on to the layer's end
         float s[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) s[i] = i < kPiece ? __fmul_rn(w2, v[i % kPiece]) : 0.0f;
         fold16(s, lane);
-        if (row_ok) {
+        if (row_ok && gave_up == 0) {   // (without the sums the block that adds them gives up as well)
           const int set = (c * kNearM + quad * 16) / 16;
           st_relaxed_u64(group_halves + set * hb::kGroupCols + fold16_col<16>(lane),
                          static_cast<unsigned long long>(p.tag) << 32 | __float_as_uint(s[0]));
