@@ -22,8 +22,10 @@
 // without first.  The arrival is a relaxed one, what has come is used at once, and warps look at it afterwards, while the
 // next layer's is on its way.  An activation is never negative, so the high sign bit of every 32-bit word (two bf16 activations, or the lo and the hi part of one in
 // split precision) carries the parity of the buffer's use; with the parity 1 both halves are negated, and the instruction
-// negates B.  A word of an earlier use with the same parity cannot come: the use in between has been looked at in the
-// same place.  Where a word does not show the parity (in one launch of 40,000 while other streams kept L2 busy, never
+// negates B.  A word of an earlier use with the same parity cannot come: the use in between, n, is ordered before the load of use
+// n + 2, for in every second layer an epilogue warp passes a fence between two arrivals that the loader waits for first, while the
+// MMAs run (371 queries 27.1 us without, 27.4 so, 27.6 with a fence in each layer; 4,224 63.7, 63.9, 64.5).  That
+// a word comes whole, new or old, is what copies of 16 bytes and more do; nothing else is taken for granted.  Where a word does not show the parity (in one launch of 40,000 while other streams kept L2 busy, never
 // alone), all CTAs of the cluster run the network once more, with releases and buffers without parities.  No result is
 // stored before all CTAs have looked at everything.  Two buffers alternate by layer: a CTA writes layer L only after its pair
 // has read all of layer L - 1, which every CTA wrote after reading L - 2.  The host keeps the parity each group's buffers
@@ -598,6 +600,10 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
           // Block 0 has used all of the layer's input.  What the blocks' rows are not written over is looked at now.
           if (!S::kApart && b == 0 && L > 0 && ok && !sure) look(want, 2 * S::kRows);
         }
+        // With the arrivals after it a release of this layer's and the last one's rows, before those places are read again; while
+        // the next layer's MMAs run.
+        if (!sure && (L & 1) && L + 2 < n_layers) asm volatile("fence.acq_rel.cluster;" ::: "memory");
+        if (!S::kApart && last && ok && !sure) look(want, 0);
       }
       if (cta < 2 && warp < 8) {
         // the first CTA of each half adds the 64 sets of 16 features of its queries

@@ -95,3 +95,15 @@ def test_commits_of_the_last_slots_can_come_late():
     """The last layer's MMAs have ended when its commit is there, but the commits that free its slots may come after it."""
     at, coming = _fault(_roles(2, last_slots=False))
     assert coming and all(bar.startswith("empty") for bar in coming)
+
+
+@pytest.mark.parametrize("layers", range(1, 10))
+@pytest.mark.parametrize("fence", ["odd layers", "none"])
+def test_rows_are_ordered_before_their_place_is_read_again(layers, fence):
+    """Without releases a load may find the rows of an earlier use of its place.  It must not find those of two uses ago, which
+    carry the same parity: the rows of the use in between have to be ordered before it.  A fence after exchange u and
+    the arrival for a later one order what was written up to u; the loader waits for the arrivals of each exchange."""
+    fenced = [u for u in range(layers) if fence == "odd layers" and u % 2 == 1 and u + 2 < layers + 1]
+    for u in range(layers - 2):                       # written in exchange u, the place is read again in u + 2
+        ordered = any(u <= f < f + 1 <= u + 2 for f in fenced)
+        assert ordered == (fence == "odd layers"), u
