@@ -26,7 +26,7 @@
 // n + 2, for in every second layer an epilogue warp passes a fence between two arrivals that the loader waits for first, while the
 // MMAs run (371 queries 27.1 us without, 27.4 so, 27.6 with a fence in each layer; 4,224 63.7, 63.9, 64.5).  That
 // a word comes whole, new or old, is what copies of 16 bytes and more do; nothing else is taken for granted.  Where a word does not show the parity (in one launch of 40,000 while other streams kept L2 busy, never
-// alone), all CTAs of the cluster run the network once more, with releases and buffers without parities.  No result is
+// alone), all CTAs of the cluster run the network once more, with releases; the words and their parities are those of the first run.  No result is
 // stored before all CTAs have looked at everything.  Two buffers alternate by layer: a CTA writes layer L only after its pair
 // has read all of layer L - 1, which every CTA wrote after reading L - 2.  The host keeps the parity each group's buffers
 // have reached.
@@ -246,10 +246,10 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
   // sure: with releases; the first run goes without
 #pragma unroll 1
   for (bool sure = false;; sure = true) {
-    uint8_t* const group_acts = (sure ? p.sure_acts : p.acts) + static_cast<size_t>(group) * (4u * kHalfBytes);
+    uint8_t* const group_acts = p.acts + static_cast<size_t>(group) * (4u * kHalfBytes);
     // both signs of the words of the `use`-th exchange
     auto signs_of = [&](int use) -> uint32_t {
-      return !sure && (((p.parity[use & 1] >> group) + static_cast<unsigned>(use >> 1)) & 1ull) ? 0x80008000u : 0u;
+      return (((p.parity[use & 1] >> group) + static_cast<unsigned>(use >> 1)) & 1ull) ? 0x80008000u : 0u;
     };
     const uint32_t tag = sure ? p.tag | 0x80000000u : p.tag;
     if (warp == 0) {
@@ -262,7 +262,6 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         }
         bool ok = true;
         const int32_t row0 = (group * 4 + static_cast<int>(r)) * 4;   // in K quarters
-        const CUtensorMap* const map = sure ? &p.map_sure : &p.map_acts;
         for (int L = 1; L < n_layers && ok; ++L) {
           const int u = L - 1, buf = u & 1;
 #pragma unroll 1
@@ -282,7 +281,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
             if (!ok) break;
             const uint32_t bar = S::kJoint ? bar_full + 8 * ((S::kBlocks + q) % S::kSlots) : bar_actq + 8 * q;
             if (r == 0) mbar_expect_tx(bar, 2u * 256u * S::kRowBytes);
-            tma_2d_pair(act + q * 256 * S::kRowBytes, map, (row0 + buf * 8 + q) * static_cast<int32_t>(hb::act_map_box(NC)),
+            tma_2d_pair(act + q * 256 * S::kRowBytes, &p.map_acts, (row0 + buf * 8 + q) * static_cast<int32_t>(hb::act_map_box(NC)),
                         map_to_cta(bar, leader));
           }
         }

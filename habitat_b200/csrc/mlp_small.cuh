@@ -27,8 +27,7 @@ struct SmallParams {
   int32_t per_group;          // queries per group
   float* out;
   int32_t* status;
-  uint8_t* acts;              // [groups][2 buffers][2 halves][1024 K rows][row bytes] with parities, and another without
-  uint8_t* sure_acts;         // (mlp_pairs.cu)
+  uint8_t* acts;              // [groups][2 buffers][2 halves][1024 K rows][row bytes] (mlp_pairs.cu)
   unsigned long long* halves; // [groups][64 sets of 16 features][kGroupCols]: fc2 sum, tag
   int32_t* poison;            // set by a launch that gave up; below zero: block ~poison of each group alone heeds it (tests)
   uint32_t tag;               // of this launch
@@ -43,7 +42,7 @@ struct SmallParams {
   uint8_t inline_row[kWideInline];
   CUtensorMap map_slot;       // a ring slot of weight rows
   CUtensorMap map_fc1;        // one K block of the block's rows
-  CUtensorMap map_acts, map_sure;   // 256 rows of acts, of sure_acts
+  CUtensorMap map_acts;       // 256 rows of acts
 };
 
 inline __device__ bool concerns(int32_t poison, uint32_t block) { return poison > 0 || (poison < 0 && ~poison == static_cast<int32_t>(block)); }

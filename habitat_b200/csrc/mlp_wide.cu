@@ -417,8 +417,7 @@ using hb::kMaxCudaDevices;
 // which needs no scratch.
 constexpr int kMaxStreams = 16, kMoreStreams = 16;
 constexpr int kMaxGroups = 34;
-// Activation buffers of mlp_pairs.cu: one for the first runs of each shape (a word's parity counts its own uses), and one that
-// all shapes use for second runs.
+// Activation buffers of mlp_pairs.cu, one for each shape: a word's parity counts its own uses.
 constexpr int kTryShapes = 8;                           // of kShapes, after the first
 constexpr size_t acts_bytes(int groups, int row_bytes) { return static_cast<size_t>(groups) * 4 * kWidth * row_bytes; }
 constexpr int kTryGroups[kTryShapes] = {8, 8, 8, 8, 16, 16, 16, kMaxGroups};
@@ -426,7 +425,7 @@ constexpr int kTryNC[kTryShapes] = {16, 32, 40, 48, 32, 48, 64, 64};
 constexpr size_t try_offset(int shape) {
   return shape ? try_offset(shape - 1) + acts_bytes(kTryGroups[shape - 1], 2 * kTryNC[shape - 1]) : 0;
 }
-constexpr size_t kSureOffset = try_offset(kTryShapes), kActsBytes = kSureOffset + acts_bytes(kMaxGroups, 128);
+constexpr size_t kActsBytes = try_offset(kTryShapes);
 constexpr size_t kHalvesBytes = static_cast<size_t>(kMaxGroups) * 64 * hb::kGroupCols * sizeof(unsigned long long);
 constexpr size_t kScratchBytes = kActsBytes + kHalvesBytes + 256;   // and the mark of a launch that gave up
 struct StreamScratch {
@@ -437,7 +436,7 @@ struct StreamScratch {
   uint32_t tag = 0;
   unsigned long long parity[kTryShapes][2] = {};   // bit g: parity of the next use of group g's buffers
   bool expect_stale = false;                     // at the next launch that could (tests)
-  CUtensorMap map_try[kTryShapes]{}, map_sure[kTryShapes]{};
+  CUtensorMap map_try[kTryShapes]{};
   cudaEvent_t done = nullptr;                    // shared ones: behind the last launch
   uint64_t last_use = 0;
 };
@@ -495,11 +494,9 @@ StreamScratch* scratch_of(GpuScratch& g, cudaStream_t stream, int lane) {
   }
   cudaError_t maps = cudaSuccess;
   uint8_t* const acts = static_cast<uint8_t*>(base);
-  for (int i = 0; i < 2 * kTryShapes && maps == cudaSuccess; ++i) {
-    const int shape = i / 2, NC = kTryNC[shape];
-    maps = hb::encode_rows(i % 2 ? &s.map_sure[shape] : &s.map_try[shape], acts + (i % 2 ? kSureOffset : try_offset(shape)),
-                           hb::act_map_row(NC), acts_bytes(kTryGroups[shape], 2 * NC) / hb::act_map_row(NC), hb::act_map_box(NC));
-  }
+  for (int i = 0; i < kTryShapes && maps == cudaSuccess; ++i)
+    maps = hb::encode_rows(&s.map_try[i], acts + try_offset(i), hb::act_map_row(kTryNC[i]),
+                           acts_bytes(kTryGroups[i], 2 * kTryNC[i]) / hb::act_map_row(kTryNC[i]), hb::act_map_box(kTryNC[i]));
   if (maps != cudaSuccess) {
     cudaGetLastError();
     cudaFree(base);
@@ -704,8 +701,6 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
     while (i < kTryShapes - 1 && (2 * kShapes[i + 1].pairs != w.G || kShapes[i + 1].NC != w.W)) ++i;
     p.acts = s->base + try_offset(i);
     p.map_acts = s->map_try[i];
-    p.sure_acts = s->base + kSureOffset;
-    p.map_sure = s->map_sure[i];
     p.expect_stale = s->expect_stale ? 0x80008000u : 0u;
     s->expect_stale = false;
     // exchange `use` (0 .. layers - 1) takes buffer use & 1; every group of the launch flips with it
