@@ -678,7 +678,8 @@ cudaError_t launch(int P, int NC, const SmallParams& p, int groups, int device, 
     case 448: return launch<4, 48, SPLIT>(p, groups, device, stream, fits);
     case 432: return launch<4, 32, SPLIT>(p, groups, device, stream, fits);
     case 464: return launch<4, 64, SPLIT>(p, groups, device, stream, fits);
-    default: return launch<2, 64, SPLIT>(p, groups, device, stream, fits);
+    case 264: return launch<2, 64, SPLIT>(p, groups, device, stream, fits);
+    default: return cudaErrorInvalidConfiguration;
   }
 }
 }  // namespace

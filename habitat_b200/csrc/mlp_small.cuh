@@ -79,7 +79,10 @@ cudaError_t launch_clusters(Kernel kernel, int ctas, int threads, int smem, cons
   cfg.numAttrs = overlapped_launch_enabled() ? 2 : 1;
   return *fits ? cudaLaunchKernelEx(&cfg, kernel, p) : cudaSuccess;
 }
-// mlp_pairs.cu
+// mlp_pairs.cu: the shapes that it has, P pairs and NC columns per CTA, and a launch of one of them.
+constexpr bool has_pairs_shape(int P, int NC) {
+  return P == 8 ? NC == 16 || NC == 32 || NC == 40 || NC == 48 : (P == 4 ? NC == 32 || NC == 48 || NC == 64 : P == 2 && NC == 64);
+}
 cudaError_t launch_pairs(int P, int NC, bool split, const SmallParams& p, int groups, int device, cudaStream_t stream,
                          bool* fits);
 constexpr int kMaxCudaDevices = 64;

@@ -408,6 +408,21 @@ __global__ void __launch_bounds__(kNearThreads, 1) mlp_near_kernel(const __grid_
 // ---------------------------------------------------------------------------
 namespace {
 using hb::kMaxCudaDevices;
+// The shapes.  pairs: of mlp_pairs.cu, with NC columns per CTA; 0: mlp_near_kernel.  clusters: of the shape that a B200 runs at a
+// time.  us: what a launch takes, full or not (measured, see wide_plan).
+struct Shape { int pairs, NC, clusters, us, us_split; };
+constexpr Shape kShapes[] = {{0, 16, 7, 21, 30}, {8, 16, 7, 25, 32}, {8, 32, 7, 27, 36}, {8, 40, 7, 29, 38}, {8, 48, 7, 32, 42},
+                             {4, 32, 15, 35, 49}, {4, 48, 15, 41, 59},
+                             {4, 64, 15, 45, 62}, {2, 64, 33, 64, 105}};
+constexpr int kNumShapes = static_cast<int>(sizeof(kShapes) / sizeof(kShapes[0]));
+constexpr int kMaxGroups = 33;
+constexpr bool shapes_fit() {
+  for (const Shape& s : kShapes)
+    if (s.clusters > kMaxGroups || (s.pairs != 0 && !hb::has_pairs_shape(s.pairs, s.NC))) return false;
+  return true;
+}
+static_assert(shapes_fit(), "parities are kept for 64 groups, sums for kMaxGroups, and every shape has a kernel");
+
 // Scratch per stream: launches on one stream follow one another, so they can share it (those of one call
 // that run side by side have a lane each).  It is kept between launches and freed with the GPU's last predictor.
 // The first kMaxStreams streams and lanes keep theirs.  Later ones (a program with a stream per request) share
@@ -416,27 +431,24 @@ using hb::kMaxCudaDevices;
 // the first streams go without.  While none of the shared ones is out of use, a launch takes the two-SM kernel,
 // which needs no scratch.
 constexpr int kMaxStreams = 16, kMoreStreams = 16;
-constexpr int kMaxGroups = 34;
-// Activation buffers of mlp_pairs.cu, one for each shape: a word's parity counts its own uses.
-constexpr int kTryShapes = 8;                           // of kShapes, after the first
-constexpr size_t acts_bytes(int groups, int row_bytes) { return static_cast<size_t>(groups) * 4 * kWidth * row_bytes; }
-constexpr int kTryGroups[kTryShapes] = {8, 8, 8, 8, 16, 16, 16, kMaxGroups};
-constexpr int kTryNC[kTryShapes] = {16, 32, 40, 48, 32, 48, 64, 64};
-constexpr size_t try_offset(int shape) {
-  return shape ? try_offset(shape - 1) + acts_bytes(kTryGroups[shape - 1], 2 * kTryNC[shape - 1]) : 0;
-}
-constexpr size_t kActsBytes = try_offset(kTryShapes);
 constexpr size_t kHalvesBytes = static_cast<size_t>(kMaxGroups) * 64 * hb::kGroupCols * sizeof(unsigned long long);
-constexpr size_t kScratchBytes = kActsBytes + kHalvesBytes + 256;   // and the mark of a launch that gave up
+constexpr size_t kBaseBytes = kHalvesBytes + 256;   // and the mark of a launch that gave up
+// Activations of a shape of mlp_pairs.cu, 0.9 to 17 MB: made when the stream first has a batch for the shape.
+constexpr size_t acts_bytes(const Shape& s) { return static_cast<size_t>(s.clusters) * 4 * kWidth * 2 * s.NC; }
+struct Activations {
+  uint8_t* base = nullptr;
+  bool fresh = false;                            // words and parities start over at the next launch
+  unsigned long long parity[2] = {};             // bit g: parity of the next use of group g's buffers
+  CUtensorMap map{};
+};
 struct StreamScratch {
   unsigned long long stream_id = 0;
   int lane = 0;
-  uint8_t* base = nullptr;
-  bool fresh = false;                            // buffers and parities start over at the next launch
+  uint8_t* base = nullptr;                       // sums, mark
+  bool fresh = false;                            // they start over at the next launch
   uint32_t tag = 0;
-  unsigned long long parity[kTryShapes][2] = {};   // bit g: parity of the next use of group g's buffers
+  Activations acts[kNumShapes];                  // (the near shape has none)
   bool expect_stale = false;                     // at the next launch that could (tests)
-  CUtensorMap map_try[kTryShapes]{};
   cudaEvent_t done = nullptr;                    // shared ones: behind the last launch
   uint64_t last_use = 0;
 };
@@ -486,20 +498,8 @@ StreamScratch* scratch_of(GpuScratch& g, cudaStream_t stream, int lane) {
   s = StreamScratch{};
   void* base = nullptr;
   if ((g.used >= kMaxStreams && cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming) != cudaSuccess) ||
-      cudaMalloc(&base, kScratchBytes) != cudaSuccess) {
+      cudaMalloc(&base, kBaseBytes) != cudaSuccess) {
     cudaGetLastError();
-    if (s.done) cudaEventDestroy(s.done);
-    s.done = nullptr;
-    return nullptr;
-  }
-  cudaError_t maps = cudaSuccess;
-  uint8_t* const acts = static_cast<uint8_t*>(base);
-  for (int i = 0; i < kTryShapes && maps == cudaSuccess; ++i)
-    maps = hb::encode_rows(&s.map_try[i], acts + try_offset(i), hb::act_map_row(kTryNC[i]),
-                           acts_bytes(kTryGroups[i], 2 * kTryNC[i]) / hb::act_map_row(kTryNC[i]), hb::act_map_box(kTryNC[i]));
-  if (maps != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(base);
     if (s.done) cudaEventDestroy(s.done);
     s.done = nullptr;
     return nullptr;
@@ -510,6 +510,25 @@ StreamScratch* scratch_of(GpuScratch& g, cudaStream_t stream, int lane) {
   s.fresh = true;
   ++g.used;
   return &s;
+}
+
+// The activations of a shape, or null when there is no memory for them.  Call with the mutex held.
+Activations* acts_of(StreamScratch& s, int shape) {
+  Activations& a = s.acts[shape];
+  if (a.base) return &a;
+  const RelaxedCapture relaxed;
+  const Shape& form = kShapes[shape];
+  void* base = nullptr;
+  if (cudaMalloc(&base, acts_bytes(form)) != cudaSuccess ||
+      hb::encode_rows(&a.map, base, hb::act_map_row(form.NC), acts_bytes(form) / hb::act_map_row(form.NC),
+                      hb::act_map_box(form.NC)) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(base);
+    return nullptr;
+  }
+  a.base = static_cast<uint8_t*>(base);
+  a.fresh = true;
+  return &a;
 }
 
 template <bool SPLIT>
@@ -539,11 +558,6 @@ namespace hb {
 // 28 for 240, 32 for 480, 46 for 960, 48 for 1,056 and 73 for 2,112 queries, split 34 for 56, 46 for 240, 78 for 528 and 126
 // for 1,056: better than these only from 100 to 112 queries, by 3 %.
 namespace {
-// us: what a launch of the shape takes, full or not.  The ones with pairs are in the order of kTryNC.
-struct Shape { int pairs, NC, clusters, us, us_split; };   // pairs 0: mlp_near_kernel
-constexpr Shape kShapes[] = {{0, 16, 7, 21, 30}, {8, 16, 7, 25, 32}, {8, 32, 7, 27, 36}, {8, 40, 7, 29, 38}, {8, 48, 7, 32, 42},
-                             {4, 32, 15, 35, 49}, {4, 48, 15, 41, 59},
-                             {4, 64, 15, 45, 62}, {2, 64, 33, 64, 105}};
 int clusters_of(const Shape& s, int sm_count) { return sm_count >= 148 ? s.clusters : s.clusters * sm_count / 148; }
 int cols_of(const Shape& s, bool split) {
   return s.pairs == 0 ? (split ? kNearQ<true> : kNearQ<false>) : (split ? s.NC : 2 * s.NC);
@@ -551,13 +565,13 @@ int cols_of(const Shape& s, bool split) {
 WidePlan plan_in(const Shape& s, int64_t Q, bool split, int cols = 0) {
   // full groups while they last: fewer groups move the weights fewer times
   if (cols == 0) cols = cols_of(s, split);
-  WidePlan w{s.pairs ? 2 * s.pairs : kNearBlocks, s.NC, static_cast<int>((Q + cols - 1) / cols), 0, s.pairs == 0};
+  WidePlan w{s.pairs ? 2 * s.pairs : kNearBlocks, static_cast<int>((Q + cols - 1) / cols), 0, static_cast<int>(&s - kShapes)};
   w.per_group = static_cast<int>((Q + w.groups - 1) / w.groups);
   w.groups = static_cast<int>((Q + w.per_group - 1) / w.per_group);
   return w;
 }
 // Beside other batches near groups, which hold few queries, cost more of the GPU than they gain.
-bool fits_in_company(const WidePlan& w) { return !w.near || w.groups == 1; }
+bool fits_in_company(const WidePlan& w) { return kShapes[w.shape].pairs != 0 || w.groups == 1; }
 }  // namespace
 
 WidePlan wide_plan(int64_t Q, bool split, int sm_count, bool alone) {
@@ -583,9 +597,7 @@ void wide_plans_together(WidePlan* plans, const int64_t* Q, const bool* split, i
     return clusters ? static_cast<double>(w.groups) / clusters : 2.0;
   };
   int in_turn = 0;
-  for (int b = 0; b < n; ++b)
-    for (const Shape& s : kShapes)
-      if (2 * s.pairs == (plans[b].near ? 0 : plans[b].G) && s.NC == plans[b].W) in_turn += us_of(s, b);
+  for (int b = 0; b < n; ++b) in_turn += us_of(kShapes[plans[b].shape], b);
   for (const Shape& level : kShapes) {
     WidePlan take[kMaxLanes];
     double least[kMaxLanes], all = 0.0;
@@ -629,6 +641,7 @@ void wide_handle_destroyed(int device) {
   if (--g.handles > 0) return;
   for (int i = 0; i < g.used; ++i) {
     cudaFree(g.s[i].base);   // waits for launches that still use it
+    for (Activations& a : g.s[i].acts) cudaFree(a.base);
     if (g.s[i].done) cudaEventDestroy(g.s[i].done);
     g.s[i].done = nullptr;
   }
@@ -639,7 +652,10 @@ void wide_start_over(int device) {
   if (device < 0 || device >= kMaxCudaDevices) return;
   GpuScratch& g = g_wide[device];
   std::lock_guard<std::mutex> lock(g.mu);
-  for (int i = 0; i < g.used; ++i) g.s[i].fresh = true;
+  for (int i = 0; i < g.used; ++i) {
+    g.s[i].fresh = true;
+    for (Activations& a : g.s[i].acts) a.fresh = true;
+  }
 }
 
 hb_status wide_set_mark(int device, int32_t mark) {
@@ -648,7 +664,7 @@ hb_status wide_set_mark(int device, int32_t mark) {
   std::lock_guard<std::mutex> lock(g.mu);
   HB_CUDA_TRY(cudaDeviceSynchronize());
   for (int i = 0; i < g.used; ++i)
-    HB_CUDA_TRY(cudaMemcpy(g.s[i].base + kActsBytes + kHalvesBytes, &mark, sizeof(mark), cudaMemcpyHostToDevice));
+    HB_CUDA_TRY(cudaMemcpy(g.s[i].base + kHalvesBytes, &mark, sizeof(mark), cudaMemcpyHostToDevice));
   HB_CUDA_TRY(cudaDeviceSynchronize());
   return HB_OK;
 }
@@ -672,6 +688,9 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
   GpuScratch& g = g_wide[h->device];
   StreamScratch* s = scratch_of(g, stream, batch.lane);
   if (!s) return HB_OK;
+  const Shape& shape = kShapes[w.shape];
+  Activations* const acts = shape.pairs ? acts_of(*s, w.shape) : nullptr;
+  if (shape.pairs && !acts) return HB_OK;
   s->last_use = ++g.uses;
   const bool split = h->precision == HB_PRECISION_BF16X3;
   SmallParams p{};
@@ -680,7 +699,7 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
   p.feats = batch.feats; p.dev_row = batch.dev_row; p.Q = static_cast<int32_t>(batch.Q);
   p.per_group = w.per_group; p.out = batch.out;
   p.status = h->status;
-  p.beside = batch.beside && !s->fresh ? 1 : 0;   // (a fresh buffer's clearing has to be waited for)
+  p.beside = batch.beside && !s->fresh && !(acts && acts->fresh) ? 1 : 0;   // (a fresh buffer's clearing has to be waited for)
   p.first = batch.first;
   p.grid_n = batch.grid_n;
   if (batch.grid_n) std::memcpy(p.grid_rows, batch.grid_rows, (batch.first + batch.Q) / batch.grid_n);
@@ -689,40 +708,42 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
     std::memcpy(p.inline_feats, batch.feats, sizeof(float) * batch.Q * h->n_op_feat);
     std::memcpy(p.inline_row, batch.dev_row, batch.Q);
   }
-  if (s->fresh) {
-    // all words at parity 0, all tags at 0, no mark
-    HB_CUDA_TRY(cudaMemsetAsync(s->base, 0, kScratchBytes, stream));
-    for (auto& shape : s->parity) shape[0] = shape[1] = ~0ull;
+  if (s->fresh) {   // all tags at 0, no mark
+    HB_CUDA_TRY(cudaMemsetAsync(s->base, 0, kBaseBytes, stream));
     s->tag = 0;
     s->fresh = false;
   }
-  if (!w.near) {
-    int i = 0;   // of the shapes with buffers
-    while (i < kTryShapes - 1 && (2 * kShapes[i + 1].pairs != w.G || kShapes[i + 1].NC != w.W)) ++i;
-    p.acts = s->base + try_offset(i);
-    p.map_acts = s->map_try[i];
+  if (acts) {
+    if (acts->fresh) {   // all words at parity 0
+      HB_CUDA_TRY(cudaMemsetAsync(acts->base, 0, acts_bytes(shape), stream));
+      acts->parity[0] = acts->parity[1] = ~0ull;
+      acts->fresh = false;
+    }
+    p.acts = acts->base;
+    p.map_acts = acts->map;
+    p.parity[0] = acts->parity[0];
+    p.parity[1] = acts->parity[1];
     p.expect_stale = s->expect_stale ? 0x80008000u : 0u;
     s->expect_stale = false;
-    // exchange `use` (0 .. layers - 1) takes buffer use & 1; every group of the launch flips with it
-    const unsigned long long groups = (1ull << w.groups) - 1;
-    for (int b = 0; b < 2; ++b) {
-      p.parity[b] = s->parity[i][b];
-      if (((h->layers + 1 - b) / 2) & 1) s->parity[i][b] ^= groups;
-    }
   }
-  p.halves = reinterpret_cast<unsigned long long*>(s->base + kActsBytes);
-  p.poison = reinterpret_cast<int32_t*>(s->base + kActsBytes + kHalvesBytes);
+  p.halves = reinterpret_cast<unsigned long long*>(s->base);
+  p.poison = reinterpret_cast<int32_t*>(s->base + kHalvesBytes);
   s->tag = s->tag % 0x7FFFFFFFu + 1;   // the high bit is the second run's (mlp_pairs.cu)
   p.tag = s->tag;
-  const bool narrow = w.G == 16 || (w.G == 8 && w.W == 64);   // blocks of 64 weight rows
+  const bool narrow = shape.pairs == 0 || shape.pairs == 8 || (shape.pairs == 4 && shape.NC == 64);   // blocks of 64 weight rows
   p.map_slot = narrow ? h->tmap_slot : h->tmap_tile;
   p.map_fc1 = narrow ? h->tmap_half_tile : h->tmap_tile;
   bool fits = false;
   const cudaError_t e =
-      !w.near ? launch_pairs(w.G / 2, w.W, split, p, w.groups, h->device, stream, &fits)
-              : (split ? launch_near<true>(p, w.groups, h->device, stream, &fits)
-                       : launch_near<false>(p, w.groups, h->device, stream, &fits));
-  s->fresh = e != cudaSuccess || !fits;   // not launched: the parities above did not happen
+      shape.pairs ? launch_pairs(shape.pairs, shape.NC, split, p, w.groups, h->device, stream, &fits)
+                  : (split ? launch_near<true>(p, w.groups, h->device, stream, &fits)
+                           : launch_near<false>(p, w.groups, h->device, stream, &fits));
+  if (acts && e == cudaSuccess && fits) {
+    // exchange `use` (0 .. layers - 1) takes buffer use & 1; every group of the launch flips with it
+    const unsigned long long groups = (1ull << w.groups) - 1;
+    for (int b = 0; b < 2; ++b)
+      if (((h->layers + 1 - b) / 2) & 1) acts->parity[b] ^= groups;
+  }
   if (s->done && cudaEventRecord(s->done, stream) != cudaSuccess) {
     cudaGetLastError();
     cudaEventDestroy(s->done);

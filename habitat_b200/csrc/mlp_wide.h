@@ -14,11 +14,9 @@ namespace hb {
 // `box_images` consecutive 16 KB images of 128-byte rows.
 cudaError_t encode_rows(CUtensorMap* map, void* base, uint32_t row_bytes, uint64_t rows, uint32_t box_rows);
 cudaError_t encode_images(CUtensorMap* map, void* base, uint64_t rows, uint32_t box_rows, uint32_t box_images);
-// G blocks per group (0: not for this batch), W columns (mlp_pairs.cu: per CTA), groups, queries per group; near: the
-// exchange goes through distributed shared memory.
+// G blocks per group (0: not for this batch), groups, queries per group, shape of mlp_wide.cu's table.
 struct WidePlan {
-  int G, W, groups, per_group;
-  bool near;
+  int G, groups, per_group, shape;
 };
 // alone: no other batch that this kernel takes runs beside it (queries beyond full rounds of mlp_chain.cu's tiles are
 // alone in this sense)

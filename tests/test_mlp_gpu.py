@@ -653,6 +653,55 @@ print(want.tobytes().hex()[:200])
     assert outs[0] == outs[1]
 
 
+def test_scratch_of_a_stream_grows_with_the_shapes_it_uses():
+    """What a stream's small batches keep of the GPU's memory: 2.2 MB of sums from the first one on, and each shape's activations
+    (0.9 to 17 MB) from its first batch on; both are given back with the last predictor.  Bounds: those sizes, and 2 MB for each allocation, the
+    driver's unit.  A stream that has had all shapes before leaves what loading the kernels takes out of the count."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch
+from habitat_b200 import batched, workloads
+feats, dev = workloads.make_queries("bmm", 4224, 97)
+mu, sigma = workloads.batch_mu_sigma(feats, dev)
+w = workloads.init_mlp_weights("bmm", seed=2, layers=2, gain=2.0)
+def handle():
+    return batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=workloads.BENCH_DEVICE_FEATURES, **w)
+h = handle()
+f, r, out = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda(), torch.empty(4224, device="cuda")
+sizes = (1, 224, 448, 560, 672, 960, 1440, 1920, 4224)
+streams = [torch.cuda.Stream() for _ in range(2)]
+def run(Q, s):
+    with torch.cuda.stream(s):
+        h.predict(f[:Q], r[:Q], out=out[:Q])
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+for Q in sizes:
+    free = run(Q, streams[0])
+mb = 1 << 20
+took = []
+for Q in sizes:
+    now = run(Q, streams[1])
+    took.append((free - now) / mb)
+    free = now
+    assert run(Q, streams[1]) == now, Q
+print(took)
+need = [2.2] + [clusters * 8192 * columns / mb for clusters, columns in
+                ((7, 16), (7, 32), (7, 40), (7, 48), (15, 32), (15, 48), (15, 64), (33, 64))]
+assert all(t <= n + 2 for t, n in zip(took, need)), (took, need)
+h.check_status()
+h.close()
+h = handle()
+assert torch.cuda.mem_get_info()[0] - free > 2 * 40 * mb
+h.close()
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=root)
+    print(r.stdout)
+    assert r.returncode == 0, r.stderr
+
+
 @pytest.mark.parametrize("precision,edges", [("bf16", (28, 224, 448, 560, 672, 960, 1440, 1920, 4224)),
                                              ("bf16x3", (14, 112, 224, 280, 336, 480, 720, 960, 2112))])
 @pytest.mark.parametrize("layers", [1, 2, 3, 8])
