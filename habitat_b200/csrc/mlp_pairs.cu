@@ -15,21 +15,23 @@
 // Exchange.  Distributed shared memory moves 17 bytes a cycle and SM whatever does it (st.async or bulk copies), L2 about
 // 30 in and 85 out, so it goes through L2: an epilogue warp writes the next layer's rows of its 32 features, as they will
 // lie in shared memory, into the activation buffer where the layer has read it, copies them to global memory (bulk
-// store), waits until they are there and arrives at a barrier of each CTA that wants them; a CTA requests its K quarters (256
-// rows, one tiled load each) when all have arrived.  32 KB are there 730 cycles after the request, 128 KB after 1,540.
+// store), waits until they are there and arrives at a barrier of each CTA that wants them, one per K quarter (256 rows); a
+// CTA requests a quarter, one tiled load, when its rows have arrived (when all had, 112 queries took 24.9 us instead of 24.0, 371 26.6
+// instead of 26.2, 1,200 40.6 instead of 39.9).  32 KB are there 730 cycles after the request, 128 KB after 1,540.
 //
 // The arrival should be a release: one more round trip to L2, 1,300 to 2,300 cycles in each layer.  The network is tried
 // without first.  The arrival is a relaxed one, what has come is used at once, and warps look at it afterwards, while the
-// next layer's is on its way.  An activation is never negative, so the high sign bit of every 32-bit word (two bf16 activations, or the lo and the hi part of one in
-// split precision) carries the parity of the buffer's use; with the parity 1 both halves are negated, and the instruction
-// negates B.  A word of an earlier use with the same parity cannot come: the use in between, n, is ordered before the load of use
-// n + 2, for in every second layer an epilogue warp passes a fence between two arrivals that the loader waits for first, while the
-// MMAs run (371 queries 27.1 us without, 27.4 so, 27.6 with a fence in each layer; 4,224 63.7, 63.9, 64.5).  That
-// a word comes whole, new or old, is what copies of 16 bytes and more do; nothing else is taken for granted.  Where a word does not show the parity (in one launch of 40,000 while other streams kept L2 busy, never
-// alone), all CTAs of the cluster run the network once more, with releases; the words and their parities are those of the first run.  No result is
-// stored before all CTAs have looked at everything.  Two buffers alternate by layer: a CTA writes layer L only after its pair
-// has read all of layer L - 1, which every CTA wrote after reading L - 2.  The host keeps the parity each group's buffers
-// have reached.
+// next layer's is on its way.  An activation is never negative, so the high sign bit of every 32-bit word (two bf16
+// activations, or the lo and the hi part of one in split precision) carries the parity of the buffer's use; with the
+// parity 1 both halves are negated, and the instruction negates B.  A word of an earlier use with the same parity cannot
+// come: the use in between, n, is ordered before the load of use n + 2, for in every second layer an epilogue warp passes
+// a fence between two arrivals that the loader waits for first, while the MMAs run (371 queries 27.1 us without, 27.4 so,
+// 27.6 with a fence in each layer; 4,224 63.7, 63.9, 64.5).  That a word comes whole, new or old, is what copies of 16
+// bytes and more do; nothing else is taken for granted.  Where a word does not show the parity (in one launch of 40,000
+// while other streams kept L2 busy, never alone), all CTAs of the cluster run the network once more, with releases; the
+// words and their parities are those of the first run.  No result is stored before all CTAs have looked at everything.
+// Two buffers alternate by layer: a CTA writes layer L only after its pair has read all of layer L - 1, which every CTA
+// wrote after reading L - 2.  The host keeps the parity each group's buffers have reached.
 // (448 queries: 27.3 us so, 26.5 if nobody looked; with releases 32; by ordinary loads that poll the data in L2, 32 bytes a
 // cycle, 34; bulk copies that are looked at before they are used 30.  1,920 queries 45.6, with releases 49.2; 4,224 65.1 and
 // 68.2.)
@@ -54,10 +56,11 @@
 // have more clusters than fit at a time.
 //
 // Warp roles: 0 TMEM, the mark, activation loads; 1 MMA issuer (the pair's leader); 2-3 weight producers; 4 and more:
-// epilogue; NC = 16 to 48: eight more that look at what has come.  Every wait is bounded, as in mlp_chain.cu; a launch that
-// gave up leaves a mark in the scratch, and launches that find it report an error instead of a result.  After giving up no ring slot is requested again whose
-// copy could be under way: the MMA issuer, whose commits free the slots, waits for the producers of both CTAs to leave
-// before it issues anything past a wait that ran out, and goes no further than the layer's end.
+// epilogue; NC = 16 to 48: eight more that look at what has come.  Every wait is bounded, as in mlp_chain.cu; a launch
+// that gave up leaves a mark in the scratch, and launches that find it report an error instead of a result.  After giving
+// up no ring slot is requested again whose copy could be under way: the MMA issuer, whose commits free the slots, waits
+// for the producers of both CTAs to leave before it issues anything past a wait that ran out, and goes no further than
+// the layer's end.
 #include "mlp_small.cuh"
 
 namespace {
@@ -84,6 +87,7 @@ struct PairShape {
   static constexpr int kImages = kSlotBytes / kUnitBytes;  // per slot
   static constexpr int kParts = SPLIT ? 2 : 1;             // images per packed K block
   static constexpr int kUnits = 4 * kBlocks;               // (block, K quarter) per layer
+  static constexpr int kSignals = kBlocks == 2 ? 2 : 4;    // per exchange: of row blocks, of K quarters
   static constexpr int kUnitSlots = 4 * kParts / kImages;
   // A K quarter of the activations is counted on the barrier of the slot that it is used with.
   static constexpr bool kApart = kBlocks == 1;             // there is room for the rows on their way out
@@ -172,7 +176,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
   const uint32_t bars = stage + S::kStageBytes;
   uint8_t* bars_ptr = base_ptr + (bars - base);
   const uint32_t bar_full = bars, bar_empty = bars + 64;   // [kSlots] full: leader only, both CTAs' boxes landed
-  const uint32_t bar_sig = bars + 128;      // [2 buffers][kBlocks] rows of this CTA's queries are in global memory
+  const uint32_t bar_sig = bars + 264;      // [2 buffers][kSignals] rows of this CTA's queries are in global memory
   const uint32_t bar_actq = bars + 160;     // [4] leader only: K quarter in place in both CTAs
   const uint32_t bar_acc = bars + 192;      // [kBlocks] row block accumulated
   const uint32_t bar_stored = bars + 208;   // [kBlocks] this CTA's rows of the block are in global memory
@@ -181,11 +185,11 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
   const uint32_t bar_seen = bars + 240;     // first run: the layer's input has been looked at
   const uint32_t bar_drain = bars + 248;    // leader only, after giving up: the MMAs have ended
   const uint32_t bar_out = bars + 256;      // kApart: the output of a layer after the first is on its way (kEpiWarps)
-  constexpr int kBars = 33;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_ptr + 288);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + 292);
-  volatile int* stale = reinterpret_cast<volatile int*>(bars_ptr + 296);            // some CTA of the cluster has seen stale words
-  volatile int* producers_left = reinterpret_cast<volatile int*>(bars_ptr + 304);   // [4] leader only
+  constexpr int kBars = 41, kAbort = 340, kStale = 344, kLeft = 352;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars_ptr + 336);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars_ptr + kAbort);
+  volatile int* stale = reinterpret_cast<volatile int*>(bars_ptr + kStale);           // some CTA of the cluster has seen stale words
+  volatile int* producers_left = reinterpret_cast<volatile int*>(bars_ptr + kLeft);   // [4] leader only
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank(), r = cta & 1u, leader = cta & ~1u;
@@ -197,7 +201,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
     for (int i = 0; i < kBars; ++i) mbar_init(bars + 8 * i, 1);
     if (S::kJoint)
       for (int s = 0; s < S::kSlots; ++s) mbar_init(bar_full + 8 * s, 2);
-    for (int i = 0; i < 2 * S::kBlocks; ++i) mbar_init(bar_sig + 8 * i, 32 / S::kBlocks);
+    for (int i = 0; i < 2 * S::kSignals; ++i) mbar_init(bar_sig + 8 * i, 32 / S::kSignals);
     for (int b = 0; b < S::kBlocks; ++b) mbar_init(bar_stored + 8 * b, S::kStores);
     mbar_init(bar_feat, 2);
     mbar_init(bar_seen, S::kApart ? S::kLookWarps : S::kEpiWarps);
@@ -237,7 +241,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
   auto block_feature = [&](int b) { return b * 512 + pair * (2 * S::kRows); };
   auto saw_stale = [&] {
 #pragma unroll 1
-    for (uint32_t c = 0; c < S::kCtas; ++c) st_cluster_u32(map_to_cta(bars + 296, c), 1u);
+    for (uint32_t c = 0; c < S::kCtas; ++c) st_cluster_u32(map_to_cta(bars + kStale, c), 1u);
     __threadfence();
   };
   constexpr uint32_t kSigns = SPLIT ? 0x80000000u : 0x80008000u;   // those that carry the parity
@@ -273,10 +277,12 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
               ok = S::kApart ? pairs_wait(bar_acc, u & 1, abort_flag, p, 0x531)
                              : pairs_wait(bar_stored + 8 * b, u & 1, abort_flag, p, 0x531);
               if (!sure && u > 0 && q == 0) ok = ok && pairs_wait(bar_seen, (u - 1) & 1, abort_flag, p, 0x534);
-              ok = ok && cluster_wait(bar_sig + 8 * (buf * S::kBlocks + b), (u >> 1) & 1, abort_flag, p, 0x532);
-              asm volatile("fence.proxy.async.global;" ::: "memory");
             } else if (S::kBlocks == 2 && q == 1 && u > 0) {
               ok = pairs_wait(bar_q1, (u - 1) & 1, abort_flag, p, 0x533);
+            }
+            if (S::kSignals == 4 || (q & 1) == 0) {
+              ok = ok && cluster_wait(bar_sig + 8 * (buf * S::kSignals + q * S::kSignals / 4), (u >> 1) & 1, abort_flag, p, 0x532);
+              asm volatile("fence.proxy.async.global;" ::: "memory");
             }
             if (!ok) break;
             const uint32_t bar = S::kJoint ? bar_full + 8 * ((S::kBlocks + q) % S::kSlots) : bar_actq + 8 * q;
@@ -315,7 +321,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         // or the shared memory is somebody else's.
         for (uint32_t n = loads + w; n < loads + S::kSlots && *abort_flag == 0; n += 2)
           pairs_wait(bar_empty + 8 * (n % S::kSlots), (n / S::kSlots & 1u) ^ 1u, abort_flag, p, 0x512);
-        st_cluster_u32(map_to_cta(bars + 304 + 4 * (2 * r + w), leader), 1u);
+        st_cluster_u32(map_to_cta(bars + kLeft + 4 * (2 * r + w), leader), 1u);
       }
       __syncwarp();
     } else if (warp == 1) {
@@ -347,7 +353,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         auto wait = [&](uint32_t bar, uint32_t parity, int code) {
           if (!mbar_try_wait(bar, parity) && (*abort_flag || !pairs_wait(bar, parity, abort_flag, p, code))) {
             // (the producers look at their CTA's abort flag when a slot does not come)
-            st_cluster_u32(map_to_cta(bars + 292, leader + 1), 1u);
+            st_cluster_u32(map_to_cta(bars + kAbort, leader + 1), 1u);
             __threadfence();
             const long long t0 = clock64();
             for (int i = 0; i < 4; ++i)
@@ -409,49 +415,29 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         }
       }
       __syncwarp();
-    } else if (S::kApart && warp >= 4 + S::kEpiWarps) {
-      // ------------------------------ looking at what has been used ------------------------------
-      constexpr int kShare = S::kApart ? S::kActBytes / S::kLookWarps : 0, kBatch = NC == 40 ? 10 : 8;
-      static_assert(kShare % (512 * kBatch) == 0, "all of it");
-      const uint8_t* const mine = base_ptr + (warp - 4 - S::kEpiWarps) * kShare + 16 * lane;
-#pragma unroll 1
-      for (int L = 1; L < n_layers && !sure; ++L) {
-        // (not while the epilogue is at it: it took 500 cycles instead of 220)
-        if (!pairs_wait(bar_out, (L - 1) & 1, abort_flag, p, 0x551)) break;
-        const uint32_t want = signs_of(L - 1) ^ p.expect_stale;
-        uint32_t bad = 0;
-#pragma unroll 1
-        for (int i = 0; i < kShare; i += 512 * kBatch) {
-          uint4 x[kBatch];
-#pragma unroll
-          for (int k = 0; k < kBatch; ++k) x[k] = *reinterpret_cast<const uint4*>(mine + i + 512 * k);
-#pragma unroll
-          for (int k = 0; k < kBatch; ++k) bad |= (x[k].x ^ want) | (x[k].y ^ want) | (x[k].z ^ want) | (x[k].w ^ want);
-        }
-        if (bad & kSigns) saw_stale();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_seen);
-      }
-      __syncwarp();
     } else {
-      // ------------------------------ epilogue ------------------------------
-      constexpr int kEpiThreads = 32 * S::kEpiWarps;
+      // ------------------------------ fc1's input ------------------------------
+      // K rows 0..63 hold [hi | lo | hi] of the normalised features, one query per column (split: the second of its two, see
+      // below).  Those that look later help: a thread's two loads in a row and the division take some 1,500 cycles, and the
+      // epilogue's warps alone went round two to five times (112 queries 25.2 -> 24.9 us, 371 27.7 -> 26.6).
+      constexpr int kFeatThreads = S::kThreads - 128;
       const int T = static_cast<int>(threadIdx.x) - 128;
-      // fc1's B operand: K rows 0..63 hold [hi | lo | hi] of the normalised features, one query per column (split: the
-      // second of its two, see below)
-      auto feat_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory"); };
-      const int C_in = p.n_op_feat + 4;
-      for (int i = T; i < 64 * S::kRowBytes / 16; i += kEpiThreads)
+      auto feat_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kFeatThreads) : "memory"); };
+      const int C_in = p.n_op_feat + 4, n_in = n_q * C_in;
+      for (int i = T; i < 64 * S::kRowBytes / 16; i += kFeatThreads)
         *reinterpret_cast<uint4*>(base_ptr + (S::kPanels ? b_chunk<NC>(i & 63, i >> 6) : 16 * i)) = make_uint4(0, 0, 0, 0);
-      feat_sync();
-      for (int i = T; i < n_q * C_in; i += kEpiThreads) {
-        const int q = i / C_in, f = i - q * C_in;
+#pragma unroll 1
+      for (int i0 = 0; i0 == 0 || i0 < n_in; i0 += kFeatThreads) {
+        const int i = i0 + T, q = i / C_in, f = i - q * C_in;
         __nv_bfloat16 hi, lo;
-        load_feature(p, static_cast<int>(q0) + q, f, hi, lo);
-        const uint32_t col = static_cast<uint32_t>(SPLIT ? 2 * q + 1 : q), ch = col >> 3, in = 2u * (col & 7u);
-        *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<NC>(f, ch) + in) = hi;
-        *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<NC>(C_in + f, ch) + in) = lo;
-        *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<NC>(2 * C_in + f, ch) + in) = hi;
+        if (i < n_in) load_feature(p, static_cast<int>(q0) + q, f, hi, lo);
+        if (i0 == 0) feat_sync();   // the zeros are there
+        if (i < n_in) {
+          const uint32_t col = static_cast<uint32_t>(SPLIT ? 2 * q + 1 : q), ch = col >> 3, in = 2u * (col & 7u);
+          *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<NC>(f, ch) + in) = hi;
+          *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<NC>(C_in + f, ch) + in) = lo;
+          *reinterpret_cast<__nv_bfloat16*>(base_ptr + b_chunk<NC>(2 * C_in + f, ch) + in) = hi;
+        }
       }
       fence_proxy_async();
       feat_sync();
@@ -460,157 +446,184 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
         else mbar_arrive_remote(map_to_cta(bar_feat, leader));
       }
       __syncwarp();
-      // A warp drains 32 rows (features) of one half of the columns, or a part of them (kColGroups).  Split precision: a
-      // query has two columns, of the lo and the hi part of its activations: one 32-bit word in a row of B.
-      const int quad = warp & 3, rest = (warp - 4) >> 2;
-      const uint32_t half = S::kNarrow ? quad >> 1 : rest & 1;
-      const int part = S::kNarrow ? rest : rest >> 1;
-      const int row0 = S::kNarrow ? (quad & 1) * 32 : quad * 32;
-      constexpr int kPiece = S::kHalfQ / S::kColGroups;      // queries per warp
-      constexpr int kCols = S::kParts * kPiece;
-      const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (S::kNarrow ? 0u : half * (S::kN / 2)) +
-                              static_cast<uint32_t>(part * kCols);
-      unsigned long long* const group_halves = p.halves + static_cast<size_t>(group) * 64 * hb::kGroupCols;
-      auto rows_sync = [&] {   // the warps of these rows
-        if (S::kColGroups == 2) asm volatile("bar.sync %0, 64;" ::"r"(2 + quad + (S::kNarrow ? 0 : 4 * static_cast<int>(half))) : "memory");
-        else __syncwarp();
-      };
-      // This warp's share of the input, without the first `from` rows of quarters 0 and 2.
-      auto look = [&](uint32_t want, uint32_t from) {
-        constexpr uint32_t kStep = 4096;              // 32 rows
-        uint32_t bad = 0;
+      if (S::kApart && warp >= 4 + S::kEpiWarps) {
+        // ------------------------------ looking at what has been used ------------------------------
+        constexpr int kShare = S::kApart ? S::kActBytes / S::kLookWarps : 0, kBatch = NC == 40 ? 10 : 8;
+        static_assert(kShare % (512 * kBatch) == 0, "all of it");
+        const uint8_t* const mine = base_ptr + (warp - 4 - S::kEpiWarps) * kShare + 16 * lane;
 #pragma unroll 1
-        for (uint32_t at = (warp - 4) * kStep; at < S::kActBytes; at += S::kEpiWarps * kStep) {
-          if ((at / S::kRowBytes & 511u) < from) continue;
-          uint4 x[8];
+        for (int L = 1; L < n_layers && !sure; ++L) {
+          // (not while the epilogue is at it: it took 500 cycles instead of 220)
+          if (!pairs_wait(bar_out, (L - 1) & 1, abort_flag, p, 0x551)) break;
+          const uint32_t want = signs_of(L - 1) ^ p.expect_stale;
+          uint32_t bad = 0;
+#pragma unroll 1
+          for (int i = 0; i < kShare; i += 512 * kBatch) {
+            uint4 x[kBatch];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) x[k] = *reinterpret_cast<const uint4*>(base_ptr + at + 512 * k + 16 * lane);
+            for (int k = 0; k < kBatch; ++k) x[k] = *reinterpret_cast<const uint4*>(mine + i + 512 * k);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) bad |= (x[k].x ^ want) | (x[k].y ^ want) | (x[k].z ^ want) | (x[k].w ^ want);
+            for (int k = 0; k < kBatch; ++k) bad |= (x[k].x ^ want) | (x[k].y ^ want) | (x[k].z ^ want) | (x[k].w ^ want);
+          }
+          if (bad & kSigns) saw_stale();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_seen);
         }
-        if (bad & kSigns) saw_stale();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_seen);
-      };
-      bool ok = true;
-      // a wait that ran out skips the work that is left but none of the barriers
+      } else {
+        // ------------------------------ epilogue ------------------------------
+        // A warp drains 32 rows (features) of one half of the columns, or a part of them (kColGroups).  Split precision: a
+        // query has two columns, of the lo and the hi part of its activations: one 32-bit word in a row of B.
+        const int quad = warp & 3, rest = (warp - 4) >> 2;
+        const uint32_t half = S::kNarrow ? quad >> 1 : rest & 1;
+        const int part = S::kNarrow ? rest : rest >> 1;
+        const int row0 = S::kNarrow ? (quad & 1) * 32 : quad * 32;
+        constexpr int kPiece = S::kHalfQ / S::kColGroups;      // queries per warp
+        constexpr int kCols = S::kParts * kPiece;
+        const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (S::kNarrow ? 0u : half * (S::kN / 2)) +
+                                static_cast<uint32_t>(part * kCols);
+        unsigned long long* const group_halves = p.halves + static_cast<size_t>(group) * 64 * hb::kGroupCols;
+        auto rows_sync = [&] {   // the warps of these rows
+          if (S::kColGroups == 2) asm volatile("bar.sync %0, 64;" ::"r"(2 + quad + (S::kNarrow ? 0 : 4 * static_cast<int>(half))) : "memory");
+          else __syncwarp();
+        };
+        // This warp's share of the input, without the first `from` rows of quarters 0 and 2.
+        auto look = [&](uint32_t want, uint32_t from) {
+          constexpr uint32_t kStep = 4096;              // 32 rows
+          uint32_t bad = 0;
 #pragma unroll 1
-      for (int L = 0; L < n_layers; ++L) {
-        const bool last = L == n_layers - 1;
-        const uint32_t signs = signs_of(L), want = L > 0 ? signs_of(L - 1) ^ p.expect_stale : 0u;
+          for (uint32_t at = (warp - 4) * kStep; at < S::kActBytes; at += S::kEpiWarps * kStep) {
+            if ((at / S::kRowBytes & 511u) < from) continue;
+            uint4 x[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x[k] = *reinterpret_cast<const uint4*>(base_ptr + at + 512 * k + 16 * lane);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) bad |= (x[k].x ^ want) | (x[k].y ^ want) | (x[k].z ^ want) | (x[k].w ^ want);
+          }
+          if (bad & kSigns) saw_stale();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_seen);
+        };
+        bool ok = true;
+        // a wait that ran out skips the work that is left but none of the barriers
 #pragma unroll 1
-        for (int b = 0; b < S::kBlocks; ++b) {
-          const int f0 = block_feature(b) + static_cast<int>(r) * S::kRows + row0, f = f0 + lane;
-          const float bias = __ldg(p.bias + L * kWidth + f);
-          const float w2 = last ? __ldg(p.fc2_w + f) : 0.0f;
-          if (ok) {
-            bool go = true;
-            if (lane == 0) go = pairs_wait(bar_acc + 8 * b, L & 1, abort_flag, p, 0x541);
-            ok = __shfl_sync(0xFFFFFFFFu, go ? 1 : 0, 0) != 0;
-          }
-          // where the rows are kept for the copy: in a place of their own, or the activation buffer, where it has been read
-          // (quarter 2 b) and is loaded over after they have been copied
-          const int at0 = (S::kApart ? 0 : b * 512) + static_cast<int>(half) * S::kRows + row0;
-          const uint32_t rows = S::kApart ? stage : act;
-          if (ok) {
-            tc_fence_after();
-            const uint32_t t_block = t_lane + (S::kBlocks == 2 ? static_cast<uint32_t>(((L & 1) * 2 + b) * S::kDCols) : 0u);
-            float v[kPiece];
-            if constexpr (SPLIT) {
-              float d[kCols];
-              tc_ld_cols<kCols>(t_block, d);
-#pragma unroll
-              for (int i = 0; i < kPiece; ++i) v[i] = d[2 * i + 1] + d[2 * i];
-            } else {
-              tc_ld_cols<kPiece>(t_block, v);
-            }
-            tc_fence_before();
-#pragma unroll
-            for (int i = 0; i < kPiece; ++i) v[i] = fmaxf(v[i] + bias, 0.0f);
-            if (!last) {
-              constexpr int kWords = kCols / 2;
-              uint32_t w[kWords];
-#pragma unroll
-              for (int i = 0; i < kWords; ++i) {
-                if (SPLIT) {
-                  const __nv_bfloat16 hi = __float2bfloat16_rn(v[i % kPiece]);
-                  const __nv_bfloat16 lo = __float2bfloat16_rn(v[i % kPiece] - __bfloat162float(hi));
-                  w[i] = static_cast<uint32_t>(__bfloat16_as_ushort(hi)) << 16 | __bfloat16_as_ushort(lo);
-                } else {
-                  const __nv_bfloat162 pk = __floats2bfloat162_rn(v[(2 * i) % kPiece], v[(2 * i + 1) % kPiece]);
-                  w[i] = *reinterpret_cast<const uint32_t*>(&pk);
-                }
-                w[i] = (w[i] & (SPLIT ? 0x7FFFFFFFu : 0x7FFF7FFFu)) ^ signs;
-              }
-              uint32_t bad = 0;
-#pragma unroll
-              for (int c = 0; c < kWords / 4; ++c) {
-                uint4* const to = reinterpret_cast<uint4*>(
-                    base_ptr + (rows - base) +
-                    b_chunk<NC>(static_cast<uint32_t>(at0 + lane), static_cast<uint32_t>(part * (kWords / 4) + c), 2 * S::kRows));
-                if (!S::kApart && !sure && L > 0) {   // looked at before it goes
-                  const uint4 x = *to;
-                  bad |= (x.x ^ want) | (x.y ^ want) | (x.z ^ want) | (x.w ^ want);
-                }
-                *to = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
-              }
-              fence_proxy_async();
-              if (bad & kSigns) saw_stale();
-            } else {
-              constexpr int kFold = (kPiece + 15) / 16 * 16;
-              float sum[kFold];
-#pragma unroll
-              for (int i = 0; i < kFold; ++i) sum[i] = i < kPiece ? __fmul_rn(w2, v[i % kPiece]) : 0.0f;
-              fold16(sum, lane);
-              const int set = (f0 + (lane & 16)) / 16, col = fold16_col<kFold>(lane);
-              unsigned long long* h = group_halves + set * hb::kGroupCols + half * 64 + part * kPiece + col;
-#pragma unroll
-              for (int i = 0; i < kFold / 16 && (kPiece == kFold || col + i < kPiece); ++i)
-                st_relaxed_u64(h + i, static_cast<unsigned long long>(tag) << 32 | __float_as_uint(sum[i]));
-            }
-          }
-          if (S::kApart && L > 0) {   // (each phase waits for the look of the one before: no parity comes round unseen)
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_out);
-          }
-          if (last) continue;
-          rows_sync();
-          if (part == 0) {
+        for (int L = 0; L < n_layers; ++L) {
+          const bool last = L == n_layers - 1;
+          const uint32_t signs = signs_of(L), want = L > 0 ? signs_of(L - 1) ^ p.expect_stale : 0u;
+#pragma unroll 1
+          for (int b = 0; b < S::kBlocks; ++b) {
+            const int f0 = block_feature(b) + static_cast<int>(r) * S::kRows + row0, f = f0 + lane;
+            const float bias = __ldg(p.bias + L * kWidth + f);
+            const float w2 = last ? __ldg(p.fc2_w + f) : 0.0f;
             if (ok) {
-              uint8_t* const to = group_acts + ((L & 1) * 2 + half) * kHalfBytes;
-              if (S::kPanels) {
-                if (lane < NC / 8)
-                  store_rows(to + (f0 >> 8) * (256 * S::kRowBytes) + b_chunk<NC>(f0 & 255, lane),
-                             rows + b_chunk<NC>(at0, lane, 2 * S::kRows), 32 * 16);
-              } else if (lane == 0) {
-                store_rows(to + static_cast<uint32_t>(f0) * S::kRowBytes, rows + static_cast<uint32_t>(at0) * S::kRowBytes,
-                           32 * S::kRowBytes);
-                if (!S::kApart) mbar_arrive(bar_stored + 8 * b);
+              bool go = true;
+              if (lane == 0) go = pairs_wait(bar_acc + 8 * b, L & 1, abort_flag, p, 0x541);
+              ok = __shfl_sync(0xFFFFFFFFu, go ? 1 : 0, 0) != 0;
+            }
+            // where the rows are kept for the copy: in a place of their own, or the activation buffer, where it has been read
+            // (quarter 2 b) and is loaded over after they have been copied
+            const int at0 = (S::kApart ? 0 : b * 512) + static_cast<int>(half) * S::kRows + row0;
+            const uint32_t rows = S::kApart ? stage : act;
+            if (ok) {
+              tc_fence_after();
+              const uint32_t t_block = t_lane + (S::kBlocks == 2 ? static_cast<uint32_t>(((L & 1) * 2 + b) * S::kDCols) : 0u);
+              float v[kPiece];
+              if constexpr (SPLIT) {
+                float d[kCols];
+                tc_ld_cols<kCols>(t_block, d);
+#pragma unroll
+                for (int i = 0; i < kPiece; ++i) v[i] = d[2 * i + 1] + d[2 * i];
+              } else {
+                tc_ld_cols<kPiece>(t_block, v);
+              }
+              tc_fence_before();
+#pragma unroll
+              for (int i = 0; i < kPiece; ++i) v[i] = fmaxf(v[i] + bias, 0.0f);
+              if (!last) {
+                constexpr int kWords = kCols / 2;
+                uint32_t w[kWords];
+#pragma unroll
+                for (int i = 0; i < kWords; ++i) {
+                  if (SPLIT) {
+                    const __nv_bfloat16 hi = __float2bfloat16_rn(v[i % kPiece]);
+                    const __nv_bfloat16 lo = __float2bfloat16_rn(v[i % kPiece] - __bfloat162float(hi));
+                    w[i] = static_cast<uint32_t>(__bfloat16_as_ushort(hi)) << 16 | __bfloat16_as_ushort(lo);
+                  } else {
+                    const __nv_bfloat162 pk = __floats2bfloat162_rn(v[(2 * i) % kPiece], v[(2 * i + 1) % kPiece]);
+                    w[i] = *reinterpret_cast<const uint32_t*>(&pk);
+                  }
+                  w[i] = (w[i] & (SPLIT ? 0x7FFFFFFFu : 0x7FFF7FFFu)) ^ signs;
+                }
+                uint32_t bad = 0;
+#pragma unroll
+                for (int c = 0; c < kWords / 4; ++c) {
+                  uint4* const to = reinterpret_cast<uint4*>(
+                      base_ptr + (rows - base) +
+                      b_chunk<NC>(static_cast<uint32_t>(at0 + lane), static_cast<uint32_t>(part * (kWords / 4) + c), 2 * S::kRows));
+                  if (!S::kApart && !sure && L > 0) {   // looked at before it goes
+                    const uint4 x = *to;
+                    bad |= (x.x ^ want) | (x.y ^ want) | (x.z ^ want) | (x.w ^ want);
+                  }
+                  *to = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+                }
+                fence_proxy_async();
+                if (bad & kSigns) saw_stale();
+              } else {
+                constexpr int kFold = (kPiece + 15) / 16 * 16;
+                float sum[kFold];
+#pragma unroll
+                for (int i = 0; i < kFold; ++i) sum[i] = i < kPiece ? __fmul_rn(w2, v[i % kPiece]) : 0.0f;
+                fold16(sum, lane);
+                const int set = (f0 + (lane & 16)) / 16, col = fold16_col<kFold>(lane);
+                unsigned long long* h = group_halves + set * hb::kGroupCols + half * 64 + part * kPiece + col;
+#pragma unroll
+                for (int i = 0; i < kFold / 16 && (kPiece == kFold || col + i < kPiece); ++i)
+                  st_relaxed_u64(h + i, static_cast<unsigned long long>(tag) << 32 | __float_as_uint(sum[i]));
+              }
+            }
+            if (S::kApart && L > 0) {   // (each phase waits for the look of the one before: no parity comes round unseen)
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar_out);
+            }
+            if (last) continue;
+            rows_sync();
+            if (part == 0) {
+              if (ok) {
+                uint8_t* const to = group_acts + ((L & 1) * 2 + half) * kHalfBytes;
+                if (S::kPanels) {
+                  if (lane < NC / 8)
+                    store_rows(to + (f0 >> 8) * (256 * S::kRowBytes) + b_chunk<NC>(f0 & 255, lane),
+                               rows + b_chunk<NC>(at0, lane, 2 * S::kRows), 32 * 16);
+                } else if (lane == 0) {
+                  store_rows(to + static_cast<uint32_t>(f0) * S::kRowBytes, rows + static_cast<uint32_t>(at0) * S::kRowBytes,
+                             32 * S::kRowBytes);
+                  if (!S::kApart) mbar_arrive(bar_stored + 8 * b);
+                }
+                __syncwarp();
+                if (lane < P) {
+                  const uint32_t bar = map_to_cta(bar_sig + 8 * ((L & 1) * S::kSignals + (S::kBlocks == 2 ? b : f0 >> 8)), 2 * lane + half);
+                  if (sure) mbar_arrive_remote(bar);
+                  else mbar_arrive_relaxed(bar);
+                }
               }
               __syncwarp();
-              if (lane < P) {
-                const uint32_t bar = map_to_cta(bar_sig + 8 * ((L & 1) * S::kBlocks + b), 2 * lane + half);
-                if (sure) mbar_arrive_remote(bar);
-                else mbar_arrive_relaxed(bar);
-              }
             }
-            __syncwarp();
+            // Block 0 has used all of the layer's input.  What the blocks' rows are not written over is looked at now.
+            if (!S::kApart && b == 0 && L > 0 && ok && !sure) look(want, 2 * S::kRows);
           }
-          // Block 0 has used all of the layer's input.  What the blocks' rows are not written over is looked at now.
-          if (!S::kApart && b == 0 && L > 0 && ok && !sure) look(want, 2 * S::kRows);
+          // With the arrivals after it a release of this layer's and the last one's rows, before those places are read again; while
+          // the next layer's MMAs run.
+          if (!sure && part == 0 && (L & 1) && L + 2 < n_layers) asm volatile("fence.acq_rel.cluster;" ::: "memory");
+          if (!S::kApart && last && ok && !sure) look(want, 0);
         }
-        // With the arrivals after it a release of this layer's and the last one's rows, before those places are read again; while
-        // the next layer's MMAs run.
-        if (!sure && (L & 1) && L + 2 < n_layers) asm volatile("fence.acq_rel.cluster;" ::: "memory");
-        if (!S::kApart && last && ok && !sure) look(want, 0);
-      }
-      if (cta < 2 && warp < 8) {
-        // the first CTA of each half adds the 64 sets of 16 features of its queries
-        const int q = T & 63;
-        float* tots = reinterpret_cast<float*>(bars_ptr + 512);
-        tots[T] = q < n_q && ok ? fc2_sum(p, group_halves + r * 64 + q, T >> 6, tag, abort_flag) : 0.0f;
-        asm volatile("bar.sync 10, 128;" ::: "memory");
-        result = tots[T & 63] + tots[64 + (T & 63)] + p.fc2_b;
+        if (cta < 2 && warp < 8) {
+          // the first CTA of each half adds the 64 sets of 16 features of its queries
+          const int q = T & 63;
+          float* tots = reinterpret_cast<float*>(bars_ptr + 512);
+          tots[T] = q < n_q && ok ? fc2_sum(p, group_halves + r * 64 + q, T >> 6, tag, abort_flag) : 0.0f;
+          asm volatile("bar.sync 10, 128;" ::: "memory");
+          result = tots[T & 63] + tots[64 + (T & 63)] + p.fc2_b;
+        }
       }
     }
     // No CTA leaves while another may still signal to it, all have looked at everything, and all know whether one gave up: what
@@ -620,7 +633,7 @@ mlp_pairs_kernel(const __grid_constant__ SmallParams p) {
     __syncwarp();
     if (lane == 0 && *abort_flag) {
 #pragma unroll 1
-      for (uint32_t c = 0; c < S::kCtas; ++c) st_cluster_u32(map_to_cta(bars + 292, c), 1u);
+      for (uint32_t c = 0; c < S::kCtas; ++c) st_cluster_u32(map_to_cta(bars + kAbort, c), 1u);
       __threadfence();
     }
     __syncwarp();

@@ -6,14 +6,14 @@ phases waits for a third one.  No order may leave the roles waiting, and nothing
 ended: the barriers may start over then, or the shared memory go to another block."""
 import pytest
 
-SLOTS, SLOTS_PER_LAYER = 2, 2
+SLOTS, QUARTERS = 2, 2       # of the ring; of a layer's input, each used with a slot of weights
 
 
 def _roles(layers, looked_from=1, last_slots=True):
     """What each role does, in order: ("wait", barrier, phase), ("arrive", barrier), or ("later", barrier) for an arrival
     that comes when a copy has landed or the MMAs have ended.  looked_from: the first layer whose output is announced
     to the warps that look at what has come.  last_slots: the producer sees every slot freed before it ends."""
-    n_layers, loads = layers + 1, 1 + layers * SLOTS_PER_LAYER
+    n_layers, loads = layers + 1, 1 + layers * QUARTERS
     producer, issuer, loader, epilogue, look = [], [], [], [], []
     for n in range(loads):
         if n >= SLOTS:
@@ -23,9 +23,9 @@ def _roles(layers, looked_from=1, last_slots=True):
         producer.append(("wait", "empty%d" % (n % SLOTS), n // SLOTS - 1))
     n = 0
     for L in range(n_layers):
-        if L > 0:
-            issuer.append(("wait", "act", L - 1))
-        for _ in range(1 if L == 0 else SLOTS_PER_LAYER):
+        for q in range(1 if L == 0 else QUARTERS):
+            if L > 0:
+                issuer.append(("wait", "act%d" % q, L - 1))
             issuer += [("wait", "full%d" % (n % SLOTS), n // SLOTS), ("later", "empty%d" % (n % SLOTS))]
             n += 1
         issuer.append(("later", "acc"))
@@ -36,11 +36,12 @@ def _roles(layers, looked_from=1, last_slots=True):
         if L > 0:
             look.append(("arrive", "seen"))
         if L < layers:
-            epilogue.append(("later", "signal%d" % (L & 1)))
+            epilogue += [("later", "signal%d.%d" % (L & 1, q)) for q in range(QUARTERS)]
             loader.append(("wait", "acc", L))
             if L > 0:
                 loader.append(("wait", "seen", L - 1))
-            loader += [("wait", "signal%d" % (L & 1), L // 2), ("later", "act")]
+            for q in range(QUARTERS):
+                loader += [("wait", "signal%d.%d" % (L & 1, q), L // 2), ("later", "act%d" % q)]
     return producer, issuer, loader, epilogue, look
 
 
