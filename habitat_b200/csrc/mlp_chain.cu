@@ -41,6 +41,7 @@
 // No ring slot is requested again that nobody has waited for: its copy could still be under way, and its barrier would be
 // armed a second time in one phase.  So the MMA issuer, whose commits free the slots of both CTAs, waits for all
 // producers to leave before it issues anything past a wait that ran out, and goes no further than the tile's end.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -1003,6 +1004,22 @@ hb_status queue_tail(ChainLaunch* launch, hb_mlp* h, hb::MlpBatch batch, cudaStr
   return st;
 }
 
+// What the two-SM kernel takes for batches of n predictors as one list of tiles per precision, in us (8 hidden layers, as the
+// times of the small-batch shapes).  Measured for one round: 107, 108 to 112, 113 to 117 and 114 to 120 for one to four predictors; split
+// 171, 195, 215 to 226 and 226 to 229, whose weights (34 MB each) do not stay in L2 together.  Two lists run side by side when they fit.
+int list_us(const int64_t* Q, const bool* split, int n, int sm_count) {
+  const int64_t pairs = sm_count / 2;
+  int64_t tiles[2] = {0, 0};
+  int us[2] = {100, 160};
+  for (int b = 0; b < n; ++b) {
+    const int tile_q = split[b] ? kPairQ / 2 : kPairQ;
+    tiles[split[b]] += (Q[b] + tile_q - 1) / tile_q;
+    us[split[b]] += split[b] ? 16 : 4;
+  }
+  for (int k = 0; k < 2; ++k) us[k] *= static_cast<int>((tiles[k] + pairs - 1) / pairs);
+  return tiles[0] + tiles[1] <= pairs ? std::max(us[0], us[1]) : us[0] + us[1];
+}
+
 // Queues one batch (checked by the callers) on the kernel for its size.  Call under wide_queue.
 hb_status queue_batch(hb_mlp* h, const hb::WidePlan& plan, const hb::MlpBatch& batch, cudaStream_t s) {
   bool launched = false;
@@ -1078,8 +1095,13 @@ extern "C" hb_status hb_mlp_predict_grid(const hb_mlp_grid* items, int32_t n_ite
   }
   if (some == 0) return HB_OK;
   const auto queue = hb::wide_queue(items[order[0]].handle->device);   // the current device, as are the others'
-  if (all_wide && some > 1) {
-    hb::wide_plans_together(plans, sizes, split, some, items[order[0]].handle->sm_count);
+  // Batches that each take most of the GPU follow one another on the small-batch kernels; one list of tiles can be sooner:
+  // 1,956, 582 and 3,972 queries 160 -> 112 us, 498, 684, 1,650 and 492 in split precision 309 -> 220.
+  if (all_wide && some > 1 &&
+      hb::wide_plans_together(plans, sizes, split, some, items[order[0]].handle->sm_count) >
+          list_us(sizes, split, some, items[order[0]].handle->sm_count)) {
+    for (int k = 0; k < some; ++k) plans[k] = hb::WidePlan{};
+  } else if (all_wide && some > 1) {
     // large clusters first: small ones spread over all GPCs and would leave no room for them
     for (int i = 1; i < some; ++i)
       for (int j = i; j > 0 && plans[j].G > plans[j - 1].G; --j) {

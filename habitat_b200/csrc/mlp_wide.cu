@@ -590,14 +590,18 @@ WidePlan wide_plan(int64_t Q, bool split, int sm_count, bool alone) {
 // groups as with many, so the shortest way through is the lowest time at which all batches fit when each takes
 // the narrowest shape of that time or less, unless one after the other is shorter.  What is left of the GPU goes
 // to cheaper shapes for the batches that start last.  Three predictors with 318, 192 and 6 queries take 34 us.
-void wide_plans_together(WidePlan* plans, const int64_t* Q, const bool* split, int n, int sm_count) {
+int wide_plans_together(WidePlan* plans, const int64_t* Q, const bool* split, int n, int sm_count) {
   auto us_of = [&](const Shape& s, int b) { return split[b] ? s.us_split : s.us; };
   auto share_of = [&](const WidePlan& w, const Shape& s) {   // of the clusters that run at a time
     const int clusters = clusters_of(s, sm_count);
     return clusters ? static_cast<double>(w.groups) / clusters : 2.0;
   };
-  int in_turn = 0;
-  for (int b = 0; b < n; ++b) in_turn += us_of(kShapes[plans[b].shape], b);
+  int in_turn = 0;   // (what takes less than half of the GPU mostly runs beside the others all the same)
+  for (int b = 0; b < n; ++b) {
+    const Shape& s = kShapes[plans[b].shape];
+    const double share = share_of(plans[b], s);
+    in_turn += s.pairs == 2 || share >= 0.5 ? us_of(s, b) : static_cast<int>(share * us_of(s, b));
+  }
   for (const Shape& level : kShapes) {
     WidePlan take[kMaxLanes];
     double least[kMaxLanes], all = 0.0;
@@ -625,8 +629,9 @@ void wide_plans_together(WidePlan* plans, const int64_t* Q, const bool* split, i
         break;
       }
     }
-    return;
+    return us;
   }
+  return in_turn;
 }
 
 void wide_handle_created(int device) {

@@ -42,8 +42,9 @@ struct MlpBatch {
   bool beside = false;
 };
 constexpr int kMaxLanes = 4;
-// Replaces the plans of n <= kMaxLanes batches that are launched side by side, where others finish sooner.
-void wide_plans_together(WidePlan* plans, const int64_t* Q, const bool* split, int n, int sm_count);
+// Replaces the plans of n <= kMaxLanes batches that are launched side by side, where others finish sooner; returns the time
+// that they then take, in us.
+int wide_plans_together(WidePlan* plans, const int64_t* Q, const bool* split, int n, int sm_count);
 // One call's launches on `device` follow one another on their stream: the caller holds this from the first to the
 // last of them.  A launch that runs beside the one before it relies on what its own call has queued; another
 // thread's launch in between, on the same stream, could still be using the lane's scratch.

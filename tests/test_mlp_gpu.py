@@ -426,6 +426,35 @@ def test_batches_side_by_side(sizes):
         h.close()
 
 
+@pytest.mark.parametrize("precision,sizes,listed", [("bf16", (662, 326, 97), True), ("bf16", (53, 32), False), ("bf16", (485, 527), True),
+                                                    ("bf16x3", (83, 114, 275, 82), True), ("bf16x3", (9, 38, 33), False)])
+def test_batches_that_would_follow_one_another(precision, sizes, listed):
+    """Batches for six devices that each take most of the GPU on the small-batch kernels go to the two-SM kernel as one list of
+    tiles, which leaves its cycle counters with the first predictor; others run side by side.  The predictions are the same."""
+    import ctypes
+    from habitat_b200 import _native
+    items, keep, want = (_native.MlpGrid * len(sizes))(), [], []
+    rows = bytes(range(6))
+    for i, n in enumerate(sizes):
+        feats, dev = workloads.make_queries("bmm", n, 80 + i)
+        mu, sigma = workloads.batch_mu_sigma(feats, dev)
+        h = batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=DEVF, precision=precision,
+                              **workloads.init_mlp_weights("bmm", seed=i, layers=3, gain=2.0))
+        f, out = torch.from_numpy(feats).cuda(), torch.full((6 * n,), float("nan"), device="cuda")
+        each = torch.tensor(list(rows), dtype=torch.uint8, device="cuda").repeat_interleave(n)
+        want.append(h.predict(f.repeat(6, 1).contiguous(), each))
+        items[i] = _native.MlpGrid(h._handle.value, f.data_ptr(), n, ctypes.cast(ctypes.c_char_p(rows), ctypes.c_void_p), 6,
+                                   out.data_ptr())
+        keep.append((h, f, out))
+    _native.check(_native.load().hb_mlp_predict_grid(items, len(sizes), torch.cuda.current_stream().cuda_stream))
+    first = keep[max(range(len(sizes)), key=sizes.__getitem__)][0]
+    assert (first.phase_cycles()["slots"] > 0) == listed
+    for (h, _, out), ref in zip(keep, want):
+        assert torch.equal(out, ref)
+        h.check_status()
+        h.close()
+
+
 @pytest.mark.parametrize("precision,round_q,most", [("bf16", 9472, 2112), ("bf16x3", 4736, 1056)])
 def test_last_round_of_few_tiles(precision, round_q, most):
     """Queries beyond full rounds of the two-SM kernel (74 tiles) go to the kernel for small batches while they fit
