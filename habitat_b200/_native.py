@@ -119,6 +119,8 @@ EXPORTS = {
     "hb_mlp_inject_mark": (ctypes.c_int32, [ctypes.c_void_p]),
     "hb_mlp_inject_mark_at": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_int32]),
     "hb_mlp_inject_stale": (ctypes.c_int32, [ctypes.c_void_p]),
+    "hb_mlp_inject_stale_at": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32]),
+    "hb_mlp_second_runs": (ctypes.c_int32, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int64)]),
     "hb_mlp_phase_cycles": (ctypes.c_int32, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int64)]),
     "hb_mlp_predict_host": (ctypes.c_int32, [
         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p]),

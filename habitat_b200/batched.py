@@ -316,10 +316,19 @@ class MLPHandle:
         _native.check(lib.hb_mlp_inject_mark(self._handle) if block is None
                       else lib.hb_mlp_inject_mark_at(self._handle, int(block)))
 
-    def inject_stale(self):
-        """Makes the next small-batch launch of each stream on this GPU take what its blocks exchange for stale (tests):
-        it runs the network once more, and the predictions are the same."""
-        _native.check(_native.load().hb_mlp_inject_stale(self._handle))
+    def inject_stale(self, layer=None, feature=0, word=0):
+        """Makes the next launch on clusters of SM pairs (43 to 4,224 queries; split precision 15 to 2,112) of each stream on
+        this GPU take what its blocks exchange for stale (tests), or, in the library with index checks, send one 32-bit
+        word of one feature of a layer's output as if it were.  The network runs once more, and the predictions are the same."""
+        lib = _native.load()
+        _native.check(lib.hb_mlp_inject_stale(self._handle) if layer is None
+                      else lib.hb_mlp_inject_stale_at(self._handle, int(layer), int(feature), int(word)))
+
+    def second_runs(self):
+        """How often a cluster of SM pairs has had to run the network once more (synchronises)."""
+        runs = ctypes.c_int64()
+        _native.check(_native.load().hb_mlp_second_runs(self._handle, ctypes.byref(runs)))
+        return runs.value
 
     def phase_cycles(self):
         """Cycle counters of the first cluster in the last launch of the two-SM kernel (synchronises): epilogue

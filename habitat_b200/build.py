@@ -65,9 +65,9 @@ def build_binding(force=False, verbose=False):
     return BINDING_PATH
 
 
-# Sources that carry index checks under -DHB_BOUNDS_CHECK (the checked library reuses the
+# Sources that carry index checks, or a test hook that costs time, under -DHB_BOUNDS_CHECK (the checked library reuses the
 # ordinary objects of the others).
-CHECKED_SOURCES = ["wave_scale.cu"]
+CHECKED_SOURCES = ["wave_scale.cu", "mlp_pairs.cu"]
 CHECKED_LIB_PATH = os.path.join(LIB_DIR, "libhabitat_b200_checked.so")
 
 

@@ -1208,6 +1208,28 @@ extern "C" hb_status hb_mlp_inject_stale(hb_mlp* h) {
   return HB_OK;
 }
 
+extern "C" hb_status hb_mlp_inject_stale_at(hb_mlp* h, int32_t layer, int32_t feature, int32_t word) {
+  if (!h || layer < 0 || feature < 0 || word < 0) {
+    hb::set_error("hb_mlp_inject_stale_at: bad arguments");
+    return HB_ERR_INVALID_ARGUMENT;
+  }
+  if (!hb::pairs_plant_words()) {
+    hb::set_error("hb_mlp_inject_stale_at: this build plants no words (build with -DHB_BOUNDS_CHECK)");
+    return HB_ERR_UNSUPPORTED;
+  }
+  hb::wide_plant_stale(h->device, layer, feature, word);
+  return HB_OK;
+}
+
+extern "C" hb_status hb_mlp_second_runs(hb_mlp* h, int64_t* runs) {
+  if (!h || !runs) {
+    hb::set_error("hb_mlp_second_runs: NULL argument");
+    return HB_ERR_INVALID_ARGUMENT;
+  }
+  const hb_status st = check_device(h);
+  return st != HB_OK ? st : hb::wide_second_runs(h->device, runs);
+}
+
 extern "C" hb_status hb_mlp_phase_cycles(hb_mlp* h, int64_t out[16]) {
   if (!h || !out) {
     hb::set_error("hb_mlp_phase_cycles: NULL argument");

@@ -29,9 +29,11 @@ struct SmallParams {
   int32_t* status;
   uint8_t* acts;              // [groups][2 buffers][2 halves][1024 K rows][row bytes] (mlp_pairs.cu)
   unsigned long long* halves; // [groups][64 sets of 16 features][kGroupCols]: fc2 sum, tag
-  int32_t* poison;            // set by a launch that gave up; below zero: block ~poison of each group alone heeds it (tests)
+  int32_t* poison;            // [0] set by a launch that gave up, [1] second runs of clusters (mlp_pairs.cu); [0] below zero: block ~poison of each group alone heeds it (tests)
   uint32_t tag;               // of this launch
   uint32_t expect_stale;      // 0x80008000: every word of the first run is taken for stale (tests)
+  int32_t stale_layer, stale_feature, stale_word;   // (checked build) the first run sends one word with the wrong signs: a layer's,
+                              // -1: none; a feature's; 0 .. NC - 1 over both halves of the queries
   unsigned long long parity[2];   // bit g: parity of the next use of group g's buffer 0, 1 (mlp_pairs.cu)
   int32_t beside;             // runs beside the launch before it: nothing to wait for
   int64_t first;              // of feats and dev_row

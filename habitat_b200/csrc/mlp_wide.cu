@@ -449,6 +449,7 @@ struct StreamScratch {
   uint32_t tag = 0;
   Activations acts[kNumShapes];                  // (the near shape has none)
   bool expect_stale = false;                     // at the next launch that could (tests)
+  int32_t stale[3] = {-1, -1, -1};               // then, too: SmallParams::stale_layer ..
   cudaEvent_t done = nullptr;                    // shared ones: behind the last launch
   uint64_t last_use = 0;
 };
@@ -681,6 +682,32 @@ void wide_expect_stale(int device) {
   for (int i = 0; i < g.used; ++i) g.s[i].expect_stale = true;
 }
 
+void wide_plant_stale(int device, int32_t layer, int32_t feature, int32_t word) {
+  if (device < 0 || device >= kMaxCudaDevices) return;
+  GpuScratch& g = g_wide[device];
+  std::lock_guard<std::mutex> lock(g.mu);
+  for (int i = 0; i < g.used; ++i) {
+    g.s[i].stale[0] = layer;
+    g.s[i].stale[1] = feature;
+    g.s[i].stale[2] = word;
+  }
+}
+
+hb_status wide_second_runs(int device, int64_t* runs) {
+  *runs = 0;
+  if (device < 0 || device >= kMaxCudaDevices) return HB_OK;
+  GpuScratch& g = g_wide[device];
+  std::lock_guard<std::mutex> lock(g.mu);
+  HB_CUDA_TRY(cudaDeviceSynchronize());
+  for (int i = 0; i < g.used; ++i) {
+    int32_t n = 0;
+    if (g.s[i].fresh) continue;   // not cleared yet
+    HB_CUDA_TRY(cudaMemcpy(&n, g.s[i].base + kHalvesBytes + sizeof(int32_t), sizeof(n), cudaMemcpyDeviceToHost));
+    *runs += n;
+  }
+  return HB_OK;
+}
+
 std::unique_lock<std::mutex> wide_queue(int device) {
   if (device < 0 || device >= kMaxCudaDevices) return {};   // wide_predict launches nothing there
   return std::unique_lock<std::mutex>(g_wide[device].mu);
@@ -730,6 +757,8 @@ hb_status wide_predict(hb_mlp* h, const WidePlan& w, const MlpBatch& batch, cuda
     p.parity[1] = acts->parity[1];
     p.expect_stale = s->expect_stale ? 0x80008000u : 0u;
     s->expect_stale = false;
+    p.stale_layer = s->stale[0]; p.stale_feature = s->stale[1]; p.stale_word = s->stale[2];
+    s->stale[0] = -1;
   }
   p.halves = reinterpret_cast<unsigned long long*>(s->base);
   p.poison = reinterpret_cast<int32_t*>(s->base + kHalvesBytes);

@@ -56,8 +56,13 @@ void wide_start_over(int device);
 // Leaves the mark of a launch that gave up in the GPU's scratch (tests of the error path): 1, or ~b for block b of each group
 // alone; synchronises.
 hb_status wide_set_mark(int device, int32_t mark);
-// The next launch on each stream of the GPU that tries to do without releases takes what it exchanges for stale (tests).
+// The next launch of mlp_pairs.cu on each stream of the GPU takes what it exchanges for stale (tests).
 void wide_expect_stale(int device);
+// ... sends one word of a layer's output as if it were stale, in builds that can.
+bool pairs_plant_words();
+void wide_plant_stale(int device, int32_t layer, int32_t feature, int32_t word);
+// Second runs of clusters in all streams' launches since their scratch was set up; synchronises.
+hb_status wide_second_runs(int device, int64_t* runs);
 void wide_handle_created(int device);
 void wide_handle_destroyed(int device);
 }  // namespace hb

@@ -265,10 +265,18 @@ hb_status hb_mlp_inject_mark(hb_mlp* handle);
  * had given up by itself. */
 hb_status hb_mlp_inject_mark_at(hb_mlp* handle, int32_t block);
 
-/* The next small-batch launch on each stream that has had one, on the handle's GPU, takes what its
- * blocks exchange for stale and runs the network once more, the slower way (test hook; the
- * predictions are the same).  No reference counterpart. */
+/* The next launch on clusters of SM pairs (batches of 43 to 4,224 queries, 15 to 2,112 in split
+ * precision; smaller and larger ones leave this alone) on each stream of the handle's GPU that has had a
+ * small batch takes what its blocks exchange for stale and runs the network once more, the slower way
+ * (test hook; the predictions are the same).  No reference counterpart. */
 hb_status hb_mlp_inject_stale(hb_mlp* handle);
+/* Builds with -DHB_BOUNDS_CHECK: each cluster of such a launch sends one 32-bit word of one feature of one
+ * layer's output (0: fc1's) as if it were stale.  Words hold two bf16 activations (split precision: the hi
+ * and the lo part of one), those of the first CTAs' half of the queries first. */
+hb_status hb_mlp_inject_stale_at(hb_mlp* handle, int32_t layer, int32_t feature, int32_t word);
+/* How often a cluster of SM pairs has had to run the network once more, over the GPU's streams, since
+ * their scratch was last set up.  Synchronises. */
+hb_status hb_mlp_second_runs(hb_mlp* handle, int64_t* runs);
 
 /* Profiling aid (bf16 kernel): SM cycle counters of the first cluster's leader CTA
  * for the most recent launch.  out[0..3] first epilogue group: waiting for its

@@ -731,6 +731,22 @@ h.close()
     assert r.returncode == 0, r.stderr
 
 
+# Shapes of the kernel for clusters of SM pairs: columns per CTA, clusters at a time.
+PAIR_SHAPES = ((16, 7), (32, 7), (40, 7), (48, 7), (32, 15), (48, 15), (64, 15), (64, 33))
+
+
+def _clusters(Q, precision):
+    """Clusters of SM pairs that a batch alone runs on (0: it runs on another kernel)."""
+    parts = 2 if precision == "bf16" else 1
+    if Q <= (42 if precision == "bf16" else 14):
+        return 0
+    for columns, clusters in PAIR_SHAPES:
+        if Q <= parts * columns * clusters:
+            groups = -(-Q // (parts * columns))
+            return -(-Q // -(-Q // groups))
+    return 0
+
+
 @pytest.mark.parametrize("precision,edges", [("bf16", (28, 224, 448, 560, 672, 960, 1440, 1920, 4224)),
                                              ("bf16x3", (14, 112, 224, 280, 336, 480, 720, 960, 2112))])
 @pytest.mark.parametrize("layers", [1, 2, 3, 8])
@@ -750,9 +766,66 @@ def test_clusters_of_pairs(precision, edges, layers):
         for Q in (e, e + 1, e - 1, e - 13):
             lo = (17 * Q) % (n - Q)
             for turn in range(4):
-                if turn == 1:
+                runs = h.second_runs()
+                if turn == 1 and _clusters(Q, precision):
                     h.inject_stale()
                 got = h.predict(f[lo:lo + Q].contiguous(), r[lo:lo + Q].contiguous())
                 assert torch.equal(got, full[lo:lo + Q]), (Q, turn)
+                assert turn != 1 or h.second_runs() - runs == _clusters(Q, precision), Q
+    h.check_status()
+    h.close()
+
+
+def test_every_word_of_an_exchange_is_looked_at():
+    """In the library built with -DHB_BOUNDS_CHECK (a process of its own): one word with the wrong signs in the output of one
+    layer, in each cluster.  Whichever K quarter, row block, half of the queries or layer it is in, every cluster runs the
+    network once more and the predictions are the usual ones."""
+    import os
+    import subprocess
+    import sys
+    from habitat_b200 import build as hb_build
+    if not os.path.exists(hb_build.CHECKED_LIB_PATH):
+        pytest.fail("libhabitat_b200_checked.so is not built (python -m habitat_b200.build --checked)")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", "from tests.test_mlp_gpu import _plant_words as t\nt('bf16')\nt('bf16x3')"],
+                       env=dict(os.environ, HABITAT_B200_LIB=hb_build.CHECKED_LIB_PATH), capture_output=True, text=True,
+                       timeout=300, cwd=root)
+    assert r.returncode == 0, r.stderr
+    h = batched.MLPHandle(4, mu=np.zeros(8), sigma=np.ones(8), device_features=DEVF,
+                          **workloads.init_mlp_weights("bmm", seed=41, layers=1))
+    with pytest.raises(_native_error(), match="HB_BOUNDS_CHECK"):
+        h.inject_stale(0, 0, 0)
+    h.close()
+
+
+def _plant_words(precision):
+    """All words of a row, every group of eight rows, the rows at the edges of what the warps share out, and random ones, in full
+    batches of each shape."""
+    layers = 3
+    w = workloads.init_mlp_weights("bmm", seed=41, gain=2.0, layers=layers)
+    feats, dev = workloads.make_queries("bmm", 4224, 67)
+    mu, sigma = workloads.batch_mu_sigma(feats, dev)
+    h = batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=DEVF, precision=precision, **w)
+    for columns, clusters in PAIR_SHAPES:
+        Q = clusters * columns * (2 if precision == "bf16" else 1)
+        f, r, out = torch.from_numpy(feats[:Q]).cuda(), torch.from_numpy(dev[:Q]).cuda(), torch.empty(Q, device="cuda")
+        want = h.predict(f, r).clone()
+        assert _clusters(Q, precision) == clusters
+        g = np.random.default_rng(columns + clusters)
+        places = [(k % layers, 331 * k % 1024, k) for k in range(columns)]
+        places += [(k % layers, 8 * k + k % 8, int(g.integers(columns))) for k in range(128)]
+        places += [(L, k, word) for L in range(layers) for k in (0, 127, 128, 255, 256, 511, 512, 639, 640, 767, 768, 1023)
+                   for word in (0, columns - 1)]
+        places += [(int(g.integers(layers)), int(g.integers(1024)), int(g.integers(columns))) for _ in range(100)]
+        runs = h.second_runs()
+        for place in places:
+            h.inject_stale(*place)
+            out.fill_(float("nan"))
+            h.predict(f, r, out=out)
+            now = h.second_runs()
+            # (a word that really was stale: one launch in 40,000, and only while other streams are at work)
+            assert now - runs == clusters, (columns, clusters, place)
+            assert torch.equal(out, want), (columns, clusters, place)
+            runs = now
     h.check_status()
     h.close()
