@@ -41,8 +41,9 @@ def test_bf16_reference_init(op):
     print(op, "bf16 max rel", _rel(got, ref64).max())
 
 
-@pytest.mark.parametrize("Q", [1, 63, 64, 65, 127, 129, 4096 + 17])
+@pytest.mark.parametrize("Q", [1, 63, 64, 65, 127, 129, 4096 + 17, 4224 + 1, 4224 + 17, 4224 + 127])
 def test_tile_tails(Q):
+    """Odd sizes; from 4,225 on on the two-SM kernel, with a last tile of 1, 17 and 127 queries."""
     w = workloads.torch_init_mlp_weights("conv2d")
     feats, dev = workloads.make_queries("conv2d", 8192, 77)
     mu_sigma = workloads.batch_mu_sigma(feats, dev)
@@ -192,10 +193,10 @@ def test_timeout_status_is_reported_once():
     h.close()
 
 
-@pytest.mark.parametrize("precision,sizes", [("bf16", (1, 30, 100, 200, 300, 900, 1000, 2000)),
-                                             ("bf16x3", (1, 15, 50, 100, 200, 500, 1000))])
+@pytest.mark.parametrize("precision,sizes", [("bf16", (1, 30, 100, 200, 300, 500, 600, 900, 1000, 1400, 1700, 2000, 4200)),
+                                             ("bf16x3", (1, 14, 15, 50, 100, 200, 250, 300, 400, 500, 700, 900, 1000, 2100))])
 def test_launches_that_find_the_mark_of_one_that_gave_up(precision, sizes):
-    """Every shape of the small-batch kernel: a launch that finds the mark in its scratch (left by the host here) stores no
+    """Every shape of the small-batch kernels: a launch that finds the mark in its scratch (left by the host here) stores no
     result, reports 0x5ff and ends soon; after the report the scratch starts over and the results are what they were.
     Soon: the roles leave one after the other, up to three of them, when 64 try_waits of at most some 7,800 cycles each
     have brought nothing: 1.5 M cycles, 1.5 ms at 1 GHz."""
@@ -311,13 +312,14 @@ def test_bf16_mode_against_its_own_arithmetic(op, gain, layers, bound):
 
 @pytest.mark.parametrize("precision", ["bf16", "bf16x3"])
 def test_small_batches(precision):
-    """Batches below 2,112 (split: 1,056) queries run on groups of 16, 8 or 4 blocks that exchange their
-    activations; the shapes change at 112, 240, 480, 960, 1,056 (split: 56, 120, 240, 528).  Sizes on both
-    sides of every change: each prediction equals, to the last bit, the one the same query gets inside a
-    batch that runs on the two-SM kernel, and that batch is within the mode's tolerance of the oracle
+    """Batches of up to 4,224 (split: 2,112) queries run on clusters of blocks that exchange their activations; the
+    shapes change at 42, 224, 448, 560, 672, 960, 1,440 and 1,920 (split: 14 and half of the others).  Sizes on both
+    sides of every change: each prediction equals, to the last bit, the one the same query gets in a full round
+    of the two-SM kernel, and that round is within the mode's tolerance of the oracle
     (bf16 on variance-preserving weights: 2e-2 of the output scale, as in the input-sensitive test)."""
+    n = 9472 if precision == "bf16" else 4736
     w = workloads.init_mlp_weights("conv2d", seed=9, gain=2.0)
-    feats, dev = workloads.make_queries("conv2d", 6000, 41)
+    feats, dev = workloads.make_queries("conv2d", n, 41)
     mu, sigma = workloads.batch_mu_sigma(feats, dev)
     h = batched.MLPHandle(feats.shape[1], mu=mu, sigma=sigma, device_features=DEVF, precision=precision, **w)
     f, r = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()
@@ -325,9 +327,11 @@ def test_small_batches(precision):
     ref = omlp.predict(w, feats, dev, DEVF, mu, sigma, np.float64)
     err = np.abs(full.cpu().numpy() - ref).max() / np.abs(ref).max()
     assert err <= (2e-2 if precision == "bf16" else 1e-4), err
-    edges = [112, 240, 480, 960, 1056, 2112] if precision == "bf16" else [56, 120, 240, 528, 1056]
+    edges = [42, 224, 448, 560, 672, 960, 1440, 1920, 4224]
+    if precision == "bf16x3":
+        edges = [14] + [e // 2 for e in edges[1:]]
     for Q in [1, 2, 15, 16, 17, 33] + [e + d for e in edges for d in (0, 1)]:
-        lo = 6000 - Q if Q % 2 else 7
+        lo = n - Q if Q % 2 else 7
         for _ in range(2):
             got = h.predict(f[lo:lo + Q].contiguous(), r[lo:lo + Q].contiguous())
             assert torch.equal(got, full[lo:lo + Q]), Q
@@ -338,11 +342,11 @@ def test_small_batches(precision):
 @pytest.mark.parametrize("precision", ["bf16", "bf16x3"])
 @pytest.mark.parametrize("layers", [1, 2, 3, 8])
 def test_few_queries(precision, layers):
-    """Up to 42 queries (split: 21) run on at most seven groups of up to six (three), which exchange their activations
+    """Up to 42 queries (split: 14) run on at most seven groups of up to six (two), which exchange their activations
     through distributed shared memory, two buffers in turn: odd and even numbers of layers, every size up to the first
-    that runs otherwise, each prediction with the bits it has inside a batch of the two-SM kernel."""
+    ones that run otherwise, each prediction with the bits it has in a full round of the two-SM kernel."""
     w = workloads.init_mlp_weights("lstm", seed=29, gain=2.0, layers=layers)
-    feats, dev = workloads.make_queries("lstm", 3000, 47)
+    feats, dev = workloads.make_queries("lstm", 9472 if precision == "bf16" else 4736, 47)
     mu, sigma = workloads.batch_mu_sigma(feats, dev)
     h = batched.MLPHandle(feats.shape[1], mu=mu, sigma=sigma, device_features=DEVF, precision=precision, **w)
     f, r = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()
@@ -393,7 +397,8 @@ def test_small_batches_on_streams_and_in_a_graph():
 
 @pytest.mark.parametrize("sizes", [[(1, 1), (1, 1), (1, 1), (1, 1)], [(40, 6), (16, 1)], [(264, 4), (250, 4)],
                                    [(1056, 1), (4, 4)], [(352, 6), (1, 1)], [(53, 6), (1, 6), (0, 6), (32, 6)],
-                                   [(2112, 1), (2112, 1)], [(2113, 1), (300, 6), (7, 2)], [(9472, 1), (2500, 4), (9, 3)]])
+                                   [(2112, 1), (2112, 1)], [(2113, 1), (300, 6), (7, 2)], [(9472, 1), (2500, 4), (9, 3)],
+                                   [(4224, 1), (2112, 1)], [(4225, 1), (2113, 1), (7, 2)], [(1408, 3), (37, 6), (64, 1), (3, 2)]])
 def test_batches_side_by_side(sizes):
     """Batches of several predictors in one call take other shapes than alone where they then fit on the GPU
     together, or one list of tiles; each prediction has the bits it has alone.  Sizes around full shapes, an
@@ -455,11 +460,11 @@ def test_batches_that_would_follow_one_another(precision, sizes, listed):
         h.close()
 
 
-@pytest.mark.parametrize("precision,round_q,most", [("bf16", 9472, 2112), ("bf16x3", 4736, 1056)])
+@pytest.mark.parametrize("precision,round_q,most", [("bf16", 9472, 4224), ("bf16x3", 4736, 2112)])
 def test_last_round_of_few_tiles(precision, round_q, most):
     """Queries beyond full rounds of the two-SM kernel (74 tiles) go to the kernel for small batches while they fit
-    there: on both sides of that, one or two rounds, alone and as a grid with a second batch in the list, each
-    prediction has the bits it has in a small batch."""
+    there: on both sides of that and of where the shapes change, one or two rounds, alone and as a grid with a second batch
+    in the list, each prediction has the bits it has in full rounds."""
     import ctypes
     from habitat_b200 import _native
     n = 2 * round_q + 301
@@ -468,8 +473,11 @@ def test_last_round_of_few_tiles(precision, round_q, most):
     h = batched.MLPHandle(4, mu=mu, sigma=sigma, device_features=DEVF, precision=precision,
                           **workloads.init_mlp_weights("bmm", seed=7, layers=3, gain=2.0))
     f, r = torch.from_numpy(feats).cuda(), torch.from_numpy(dev).cuda()
-    want = torch.cat([h.predict(f[i:i + 2000].contiguous(), r[i:i + 2000].contiguous()) for i in range(0, n, 2000)])
-    for q in (round_q, round_q + 1, round_q + most, round_q + most + 1, 2 * round_q, n):
+    want = h.predict(f[:2 * round_q], r[:2 * round_q])
+    want = torch.cat([want, h.predict(f[n - round_q:].contiguous(), r[n - round_q:].contiguous())[round_q - 301:]])
+    shapes = [parts * columns * clusters for parts in (2 if precision == "bf16" else 1,) for columns, clusters in PAIR_SHAPES]
+    assert shapes[-1] == most
+    for q in [round_q, round_q + 1, 2 * round_q, n] + [round_q + e + d for e in shapes for d in (0, 1)]:
         for _ in range(2):
             assert torch.equal(h.predict(f[:q].contiguous(), r[:q].contiguous()), want[:q]), q
     # seven devices x m rows: the cut falls inside a device's rows; the second batch keeps its place in the list
