@@ -987,7 +987,7 @@ hb::WidePlan plan_of(const hb_mlp* h, int64_t Q, bool alone = true) {
 
 // A last round of few tiles takes as long as a full one, and the kernel for small batches is quicker: it takes the
 // queries of that round from the first batch of the list (`batch`), the list follows beside it.  9,572 queries:
-// 220 -> 140 us, 28,916: 435 -> 378; split, 5,792: 376 -> 335.
+// 220 -> 135 us, 28,916: 435 -> 348; split, 5,792: 376 -> 282.
 hb_status queue_tail(ChainLaunch* launch, hb_mlp* h, hb::MlpBatch batch, cudaStream_t s, int* launches) {
   const int64_t n = launch->tail();
   const hb::WidePlan plan = n ? plan_of(h, n) : hb::WidePlan{};
@@ -1006,18 +1006,19 @@ hb_status queue_tail(ChainLaunch* launch, hb_mlp* h, hb::MlpBatch batch, cudaStr
 
 // What the two-SM kernel takes for batches of n predictors as one list of tiles per precision, in us (8 hidden layers, as the
 // times of the small-batch shapes).  Measured for one round: 107, 108 to 112, 113 to 117 and 114 to 120 for one to four predictors; split
-// 171, 195, 215 to 226 and 226 to 229, whose weights (34 MB each) do not stay in L2 together.  Two lists run side by side when they fit.
+// 171, 195, 215 to 226 and 226 to 229, whose weights (34 MB each) do not stay in L2 together.  Two lists run side by side when they fit, some 10 us slower.
 int list_us(const int64_t* Q, const bool* split, int n, int sm_count) {
   const int64_t pairs = sm_count / 2;
   int64_t tiles[2] = {0, 0};
-  int us[2] = {100, 160};
+  int us[2] = {100, 165};
   for (int b = 0; b < n; ++b) {
     const int tile_q = split[b] ? kPairQ / 2 : kPairQ;
     tiles[split[b]] += (Q[b] + tile_q - 1) / tile_q;
     us[split[b]] += split[b] ? 16 : 4;
   }
-  for (int k = 0; k < 2; ++k) us[k] *= static_cast<int>((tiles[k] + pairs - 1) / pairs);
-  return tiles[0] + tiles[1] <= pairs ? std::max(us[0], us[1]) : us[0] + us[1];
+  for (int k = 0; k < 2; ++k) us[k] *= static_cast<int>((tiles[k] + pairs - 1) / pairs);   // rounds, 0 without tiles
+  if (tiles[0] == 0 || tiles[1] == 0) return us[0] + us[1];
+  return tiles[0] + tiles[1] <= pairs ? std::max(us[0], us[1]) + 10 : us[0] + us[1];
 }
 
 // Queues one batch (checked by the callers) on the kernel for its size.  Call under wide_queue.

@@ -268,8 +268,8 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t par
 }
 // The same with cluster scope.  After another role gave up it returns at once (a try_wait lasts 7,800 cycles when
 // nothing comes, 64 of them a quarter of a millisecond): mlp_chain.cu's MMA issuer goes on to the end of its tile
-// whatever the waits say, several hundred of them.  (mbar_wait that looked at the flag first made the small-batch kernel
-// 1 to 2 % slower: 960 queries 45.9 -> 46.6 us, split 528 77.3 -> 79.0.)
+// whatever the waits say, several hundred of them.  (mbar_wait looks at it every 64 tries: the small-batch kernels' waits
+// mostly last less than one, and looking first took 1 to 2 % more.)
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
                                                   volatile int* abort_flag, int32_t* status,
                                                   int code) {

@@ -32,14 +32,14 @@
 // words and their parities are those of the first run.  No result is stored before all CTAs have looked at everything.
 // Two buffers alternate by layer: a CTA writes layer L only after its pair has read all of layer L - 1, which every CTA
 // wrote after reading L - 2.  The host keeps the parity each group's buffers have reached.
-// (448 queries: 27.3 us so, 26.5 if nobody looked; with releases 32; by ordinary loads that poll the data in L2, 32 bytes a
-// cycle, 34; bulk copies that are looked at before they are used 30.  1,920 queries 45.6, with releases 49.2; 4,224 65.1 and
-// 68.2.)
+// (Before the quarters had signals of their own: 448 queries 27.3 us so, 26.5 if nobody looked; with releases 32; by
+// ordinary loads that poll the data in L2, 32 bytes a cycle, 34; bulk copies that are looked at before they are used 30.
+// 1,920 queries 45.6, with releases 49.2; 4,224 65.1 and 68.2.)
 //
 // NC = 40, 48: rows of 80 or 96 bytes fit no swizzle, so B lies in panels of eight columns, 16 bytes a row, and a warp's rows go
 // out as five or six copies of 512 bytes.  N is a multiple of 32, so with 40 the MMAs read a sixth panel per CTA, which is
-// whatever lies behind the fifth; nobody reads the columns of D that come of it.  480 queries: 29.1 us in eight pairs with 40, 34.8 in
-// four with 32; 600: 32.4 in eight with 48; 1,056: 41.1 in four pairs with 48, 45.1 with 64.
+// whatever lies behind the fifth; nobody reads the columns of D that come of it.  480 queries: 28.5 us in eight pairs with 40, 34.3 in
+// four with 32; 600: 31.0 in eight with 48; 1,056: 40.5 in four pairs with 48, 45 with 64.
 //
 // NC = 64: a pair's features are two row blocks, one in K quarters 0 and 1 and one in 2 and 3.  The units (block b, K quarter
 // q) of a layer are issued in the order (0,0) (0,1) (1,0) (0,2) (0,3) | (1,1) (1,2) (1,3): quarters 0 and 1 are

@@ -411,9 +411,9 @@ using hb::kMaxCudaDevices;
 // The shapes.  pairs: of mlp_pairs.cu, with NC columns per CTA; 0: mlp_near_kernel.  clusters: of the shape that a B200 runs at a
 // time.  us: what a launch takes, full or not (measured, see wide_plan).
 struct Shape { int pairs, NC, clusters, us, us_split; };
-constexpr Shape kShapes[] = {{0, 16, 7, 21, 30}, {8, 16, 7, 25, 32}, {8, 32, 7, 27, 36}, {8, 40, 7, 29, 38}, {8, 48, 7, 32, 42},
-                             {4, 32, 15, 35, 49}, {4, 48, 15, 41, 59},
-                             {4, 64, 15, 45, 62}, {2, 64, 33, 64, 105}};
+constexpr Shape kShapes[] = {{0, 16, 7, 21, 30}, {8, 16, 7, 25, 32}, {8, 32, 7, 26, 35}, {8, 40, 7, 29, 38}, {8, 48, 7, 31, 41},
+                             {4, 32, 15, 34, 49}, {4, 48, 15, 40, 58},
+                             {4, 64, 15, 45, 62}, {2, 64, 33, 64, 103}};
 constexpr int kNumShapes = static_cast<int>(sizeof(kShapes) / sizeof(kShapes[0]));
 constexpr int kMaxGroups = 33;
 constexpr bool shapes_fit() {
@@ -546,18 +546,18 @@ namespace hb {
 // 33 of 16, 8 or 4 blocks.  Smaller clusters hold more queries in all but stream more weights per block, wider ones
 // exchange more per layer.  Measured per launch, conv2d predictor, 8 hidden layers (capacity in queries: us), against 103 us
 // (bf16) and 168 us (split) of one tile of mlp_chain.cu's kernel, which is the faster one beyond the last shape:
-//   near               42: 21.5 (one: 17.6)   split    14: 29.5 (one: 27.2)
-//   8 pairs x 16      224: 25.2 (one: 22.5)           112: 32.2 (one: 29.8)
-//   8 pairs x 32      448: 27.2                       224: 35.9
-//   8 pairs x 40      560: 29.2                       280: 38.3   (what 4 pairs x 32 take is 5.6 and 11 more)
-//   8 pairs x 48      672: 32.4                       336: 42.6
-//   4 pairs x 32      960: 34.8                       480: 49.2   (in two row blocks 38.8 and 49.9)
-//   4 pairs x 48    1,440: 41.1                       720: 59.4
-//   4 pairs x 64    1,920: 44.8                       960: 61.5   (in one row block, exchanged at once, 51.5 and 73.6)
-//   2 pairs x 64    4,224: 64.2                     2,112: 105
+//   near               42: 21.6 (one: 17.8)   split    14: 29.6 (one: 27.5)
+//   8 pairs x 16      224: 24.6 (43: 23.1)            112: 32.2 (15: 30.4)
+//   8 pairs x 32      448: 26.3                       224: 35.2
+//   8 pairs x 40      560: 28.6                       280: 37.8   (what 4 pairs x 32 take is 5.7 and 11 more)
+//   8 pairs x 48      672: 31.0                       336: 41.5
+//   4 pairs x 32      960: 34.3                       480: 48.9   (in two row blocks 4.0 and 0.7 more)
+//   4 pairs x 48    1,440: 40.4                       720: 58.3
+//   4 pairs x 64    1,920: 45.3                       960: 61.6   (in one row block, exchanged at once, 51.5 and 73.6)
+//   2 pairs x 64    4,224: 63.6                     2,112: 103
 // Blocks without partners (M = 64 or 128 each, all queries of a group in every block; data polled in L2) took 24 for 112,
 // 28 for 240, 32 for 480, 46 for 960, 48 for 1,056 and 73 for 2,112 queries, split 34 for 56, 46 for 240, 78 for 528 and 126
-// for 1,056: better than these only from 100 to 112 queries, by 3 %.
+// for 1,056: nowhere better than these.
 namespace {
 int clusters_of(const Shape& s, int sm_count) { return sm_count >= 148 ? s.clusters : s.clusters * sm_count / 148; }
 int cols_of(const Shape& s, bool split) {
@@ -590,7 +590,9 @@ WidePlan wide_plan(int64_t Q, bool split, int sm_count, bool alone) {
 // rarely fit on the GPU together: the second then waits for the first.  A shape takes the same time with few
 // groups as with many, so the shortest way through is the lowest time at which all batches fit when each takes
 // the narrowest shape of that time or less, unless one after the other is shorter.  What is left of the GPU goes
-// to cheaper shapes for the batches that start last.  Three predictors with 318, 192 and 6 queries take 34 us.
+// to cheaper shapes for the batches that start last.  Three predictors with 318, 192 and 6 queries take 33 us.
+// (Clusters cannot be cut at will, as the sum of shares has it.  Measured on 108 random calls of two to four batches: with the list
+// of tiles as the other choice, see hb_mlp_predict_grid, none took over 2 % longer than without the shapes for 2,113 to 4,224.)
 int wide_plans_together(WidePlan* plans, const int64_t* Q, const bool* split, int n, int sm_count) {
   auto us_of = [&](const Shape& s, int b) { return split[b] ? s.us_split : s.us; };
   auto share_of = [&](const WidePlan& w, const Shape& s) {   // of the clusters that run at a time
@@ -632,7 +634,7 @@ int wide_plans_together(WidePlan* plans, const int64_t* Q, const bool* split, in
     }
     return us;
   }
-  return in_turn;
+  return in_turn + in_turn / 20;   // (measured: 0 to 9 % more than the sum)
 }
 
 void wide_handle_created(int device) {
