@@ -1005,8 +1005,9 @@ hb_status queue_tail(ChainLaunch* launch, hb_mlp* h, hb::MlpBatch batch, cudaStr
 }
 
 // What the two-SM kernel takes for batches of n predictors as one list of tiles per precision, in us (8 hidden layers, as the
-// times of the small-batch shapes).  Measured for one round: 107, 108 to 112, 113 to 117 and 114 to 120 for one to four predictors; split
-// 171, 195, 215 to 226 and 226 to 229, whose weights (34 MB each) do not stay in L2 together.  Two lists run side by side when they fit, some 10 us slower.
+// times of the small-batch shapes).  Measured for one round: 107, 108 to 112, 113 to 117 and 114 to 120 for one to four
+// predictors; split 171, 195, 215 to 226 and 226 to 229, whose weights (34 MB each) do not stay in L2 together.  Two lists run
+// side by side when they fit, some 10 us slower.
 int list_us(const int64_t* Q, const bool* split, int n, int sm_count) {
   const int64_t pairs = sm_count / 2;
   int64_t tiles[2] = {0, 0};

@@ -29,7 +29,8 @@ struct SmallParams {
   int32_t* status;
   uint8_t* acts;              // [groups][2 buffers][2 halves][1024 K rows][row bytes] (mlp_pairs.cu)
   unsigned long long* halves; // [groups][64 sets of 16 features][kGroupCols]: fc2 sum, tag
-  int32_t* poison;            // [0] set by a launch that gave up, [1] second runs of clusters (mlp_pairs.cu); [0] below zero: block ~poison of each group alone heeds it (tests)
+  int32_t* poison;            // [0] the mark of a launch that gave up (below zero: block ~mark of each group alone heeds it, in
+                              // tests), [1] second runs of clusters (mlp_pairs.cu)
   uint32_t tag;               // of this launch
   uint32_t expect_stale;      // 0x80008000: every word of the first run is taken for stale (tests)
   int32_t stale_layer, stale_feature, stale_word;   // (checked build) the first run sends one word with the wrong signs: a layer's,
@@ -47,7 +48,9 @@ struct SmallParams {
   CUtensorMap map_acts;       // 256 rows of acts
 };
 
-inline __device__ bool concerns(int32_t poison, uint32_t block) { return poison > 0 || (poison < 0 && ~poison == static_cast<int32_t>(block)); }
+inline __device__ bool concerns(int32_t mark, uint32_t block) {
+  return mark > 0 || (mark < 0 && ~mark == static_cast<int32_t>(block));
+}
 
 // Launches `groups` clusters of `ctas` blocks; *fits = false (nothing launched) where the GPU cannot hold one.
 template <typename Kernel>

@@ -692,8 +692,9 @@ print(want.tobytes().hex()[:200])
 
 def test_scratch_of_a_stream_grows_with_the_shapes_it_uses():
     """What a stream's small batches keep of the GPU's memory: 2.2 MB of sums from the first one on, and each shape's activations
-    (0.9 to 17 MB) from its first batch on; both are given back with the last predictor.  Bounds: those sizes, and 2 MB for each allocation, the
-    driver's unit.  A stream that has had all shapes before leaves what loading the kernels takes out of the count."""
+    (0.9 to 17 MB) from its first batch on; both are given back with the last predictor.  Bounds: those sizes, and the 2 MB
+    that memory is handed out in.  A stream that has had all shapes before leaves what loading the kernels takes out of
+    the count."""
     import os
     import subprocess
     import sys
